@@ -14,6 +14,7 @@ SO_PATH = os.environ.get("W4A16_B200_LIB") or os.path.join(HERE, "libw4a16_b200.
 HEADER = os.path.join(os.path.dirname(HERE), "include", "w4a16_b200.h")
 
 _lib = None
+_native = None
 
 _vp, _i, _sz = C.c_void_p, C.c_int, C.c_size_t
 _SIGS = {
@@ -96,3 +97,18 @@ def lib() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = L
     return _lib
+
+
+def native(error_type):
+    """The CPython binding of the forward calls (csrc/native.cpp), bound to the library that :func:`lib` loaded."""
+    global _native
+    if _native is None:
+        import torch  # noqa: F401  (its shared libraries are what the module links against)
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise RuntimeError(f"llm170_b200/_native.so cannot be loaded ({e}): build it with `python -m llm170_b200.build`") from e
+        L = lib()
+        mod.bind(error_type, lambda symbol: C.cast(getattr(L, symbol), C.c_void_p).value)
+        _native = mod
+    return _native

@@ -22,6 +22,10 @@ class W4a16Error(RuntimeError):
     pass
 
 
+# forward entry points that the native binding takes by index (csrc/native.cpp)
+_LIN_FORWARD, _SK_SINGLE, _SK_STATIC, _SK_ALLREDUCE, _LIN_X32 = range(5)
+
+
 def _cur_stream() -> int:
     """torch's current stream as a cudaStream_t.  torch's default stream has the handle 0, which the
     C ABI reads as "use the decoder's own stream"; 1 is cudaStreamLegacy, the explicit name of that
@@ -41,12 +45,15 @@ class W4a16Dec:
         if self._L.w4a16_dec_new(device, C.byref(h)) != 0:
             raise W4a16Error(self._L.w4a16_last_error(None).decode())
         self._h = h
+        self._hp = h.value
+        self._N = _lib.native(W4a16Error)
 
     # -- plumbing ---------------------------------------------------------------------------
     def close(self):
         if getattr(self, "_h", None):
             self._L.w4a16_dec_free(self._h)
             self._h = None
+            self._hp = 0
 
     def __del__(self):
         try:
@@ -165,26 +172,12 @@ class W4a16Dec:
     def lin_forward(self, name: str, x16: torch.Tensor, t: int, dst: torch.Tensor | None = None,
                     out_f16: bool = False) -> torch.Tensor:
         """kernels/mod.rs:121-144: dst[t,n] = x16[t,k] @ W^T; GEMV for t<=8, tensor-core GEMM above."""
-        n, k, _ = self.lin_spec(name)
-        self._tensor_ok(x16, torch.float16, "x16")
-        if x16.numel() != t * k:
-            raise W4a16Error(f"lin_forward {name}: x has {x16.numel()} elements, need {t}x{k}")
-        dst = self._out(t, n, out_f16, dst)
-        self._ck(self._L.w4a16_lin_forward(self._h, name.encode(), x16.data_ptr(), dst.data_ptr(), t,
-                                           OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return dst
+        return self._N.linear(self._hp, self.device, _LIN_FORWARD, name, x16, t, dst, out_f16)
 
     def lin_forward_x32(self, name: str, x32: torch.Tensor, t: int, dst: torch.Tensor | None = None,
                         out_f16: bool = False) -> torch.Tensor:
         """lin_forward on f32 activations (kernels/gemv.rs:4-38 takes x as f32 holding f16 values)."""
-        n, k, _ = self.lin_spec(name)
-        self._tensor_ok(x32, torch.float32, "x32")
-        if x32.numel() != t * k:
-            raise W4a16Error(f"lin_forward_x32 {name}: x has {x32.numel()} elements, need {t}x{k}")
-        dst = self._out(t, n, out_f16, dst)
-        self._ck(self._L.w4a16_lin_forward_x32(self._h, name.encode(), x32.data_ptr(), dst.data_ptr(), t,
-                                               OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return dst
+        return self._N.linear(self._hp, self.device, _LIN_X32, name, x32, t, dst, out_f16)
 
     def lin_forward_lane(self, name: str, x16: torch.Tensor, t: int) -> torch.Tensor:
         """The parity-gate kernel (gptq4.cu:825-951): f32 [t,n] in the CPU lane order, bit-identical to lane.rs."""
@@ -217,25 +210,12 @@ class W4a16Dec:
 
     def head_forward(self, x32: torch.Tensor, t: int = 1, out: torch.Tensor | None = None) -> torch.Tensor:
         """kernels/gemv.rs:64-110 (head_gemv_launch / head_gemv_t_launch): f32 [t,k] -> f32 logits [t,n]."""
-        n, k = self.head_spec()
-        self._tensor_ok(x32, torch.float32, "x32")
-        if x32.numel() != t * k:
-            raise W4a16Error(f"head_forward: x has {x32.numel()} elements, need {t}x{k}")
-        out = self._out(t, n, False, out)
-        self._ck(self._L.w4a16_head_forward(self._h, x32.data_ptr(), out.data_ptr(), t, _cur_stream()))
-        return out
+        return self._N.head(self._hp, self.device, x32, t, out)
 
     def sk_single_dev(self, name: str, x16: torch.Tensor, out: torch.Tensor | None = None, t: int = 1,
                       out_f16: bool = False) -> torch.Tensor:
         """kernels/decode.rs:89-127: split-K decode GEMV on one linear."""
-        n, k, _ = self.lin_spec(name)
-        self._tensor_ok(x16, torch.float16, "x16")
-        if x16.numel() != t * k:
-            raise W4a16Error(f"sk_single_dev {name}: x has {x16.numel()} elements, need {t}x{k}")
-        out = self._out(t, n, out_f16, out)
-        self._ck(self._L.w4a16_sk_single_dev(self._h, name.encode(), x16.data_ptr(), out.data_ptr(), t,
-                                             OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return out
+        return self._N.linear(self._hp, self.device, _SK_SINGLE, name, x16, t, out, out_f16)
 
     def sk_single_static(self, name: str, x16: torch.Tensor, out: torch.Tensor | None = None, t: int = 1,
                          out_f16: bool = False) -> torch.Tensor:
@@ -243,14 +223,7 @@ class W4a16Dec:
         scratch is a fixed 8 MiB array inside the library, shared by all calls (calls that overlap on the
         GPU race on it).  Shapes that need more are rejected.  Pass ``out``: this wrapper allocates the
         output tensor only when it is omitted.  Make the first call on a device outside stream capture."""
-        n, k, _ = self.lin_spec(name)
-        self._tensor_ok(x16, torch.float16, "x16")
-        if x16.numel() != t * k:
-            raise W4a16Error(f"sk_single_static {name}: x has {x16.numel()} elements, need {t}x{k}")
-        out = self._out(t, n, out_f16, out)
-        self._ck(self._L.w4a16_sk_single_static(self._h, name.encode(), x16.data_ptr(), out.data_ptr(), t,
-                                                OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return out
+        return self._N.linear(self._hp, self.device, _SK_STATIC, name, x16, t, out, out_f16)
 
     # -- row-parallel tensor parallelism ---------------------------------------------------------
     def tp_setup(self, rank: int, world: int, max_rows: int, group=None):
@@ -272,29 +245,11 @@ class W4a16Dec:
     def sk_single_allreduce(self, name: str, x16: torch.Tensor, out: torch.Tensor | None = None, t: int = 1,
                             out_f16: bool = False) -> torch.Tensor:
         """Row-parallel GEMV whose kernel also sums the partial outputs over the ranks (peer stores)."""
-        n, k, _ = self.lin_spec(name)
-        self._tensor_ok(x16, torch.float16, "x16")
-        if x16.numel() != t * k:
-            raise W4a16Error(f"sk_single_allreduce {name}: x has {x16.numel()} elements, need {t}x{k}")
-        out = self._out(t, n, out_f16, out)
-        self._ck(self._L.w4a16_sk_single_allreduce(self._h, name.encode(), x16.data_ptr(), out.data_ptr(), t,
-                                                   OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return out
+        return self._N.linear(self._hp, self.device, _SK_ALLREDUCE, name, x16, t, out, out_f16)
 
     def sk_multi_dev(self, names, x16: torch.Tensor, outs=None, t: int = 1, out_f16: bool = False):
         """kernels/decode.rs:23-57: q|k|v or gate|up in one launch (same x, same k)."""
-        specs = [self.lin_spec(nm) for nm in names]
-        self._tensor_ok(x16, torch.float16, "x16")
-        if x16.numel() != t * specs[0][1]:
-            raise W4a16Error("sk_multi_dev: x size does not match t*k")
-        if outs is None:
-            outs = [None] * len(names)
-        outs = [self._out(t, sp[0], out_f16, o) for sp, o in zip(specs, outs)]
-        arr_n = (C.c_char_p * len(names))(*[nm.encode() for nm in names])
-        arr_o = (C.c_void_p * len(names))(*[o.data_ptr() for o in outs])
-        self._ck(self._L.w4a16_sk_multi_dev(self._h, arr_n, len(names), x16.data_ptr(), arr_o, t,
-                                            OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return outs
+        return self._N.multi(self._hp, self.device, names, x16, outs, t, out_f16)
 
     def lin_forward_host(self, name: str, x16: np.ndarray, t: int, out_f16: bool = False,
                          out: np.ndarray | None = None) -> np.ndarray:
@@ -368,15 +323,8 @@ class W4a16Dec:
     def moe_ffn_dev_t(self, il: int, logits: torch.Tensor, x16: torch.Tensor, t: int,
                       out: torch.Tensor | None = None, out_f16: bool = False) -> torch.Tensor:
         """moe/mod.rs:263: y[t,h] over the local experts (sum y over ranks under expert parallelism)."""
-        ne, k, f, h, g, _, _ = self._moe
-        self._tensor_ok(logits, torch.float32, "logits")
-        self._tensor_ok(x16, torch.float16, "x16")
-        if logits.numel() != t * ne or x16.numel() != t * h:
-            raise W4a16Error("moe_ffn_dev_t: logits/x sizes do not match t")
-        out = self._out(t, h, out_f16, out)
-        self._ck(self._L.w4a16_moe_ffn(self._h, il, logits.data_ptr(), x16.data_ptr(), out.data_ptr(), t,
-                                       OUT_F16 if out_f16 else OUT_F32, _cur_stream()))
-        return out
+        ne, h = self._moe[0], self._moe[3]
+        return self._N.moe(self._hp, self.device, il, logits, x16, t, ne, h, out, out_f16)
 
 
 class SafeTensors:
