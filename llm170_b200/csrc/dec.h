@@ -95,6 +95,7 @@ struct Dec {
     int tune_gemm_mt = 0;        // 128-token blocks per GEMM tile: 0 = automatic, 1 or 2
     int tune_gemm_ksplit = 0;    // K splits of the GEMM: 0 = automatic (only when the tiles do not fill the SMs)
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
+    int tune_ts = 1, tune_ts_mt = 0, tune_ts_tok = 0, tune_ts_ks = 0;
     long long* dbg_buf = nullptr;  // device timeline buffer (DBG_SLOTS entries) when the knob is on
     int tune_gemv_ksplit = 0;
     // kernels launched by forward calls since creation
@@ -116,6 +117,7 @@ struct Dec {
     int gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, int t, int out_kind,
              cudaStream_t st, bool allreduce = false);
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
+    int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     int gemm_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b,
                      int max_tiles, int mt, const float* row_w, cudaStream_t st);
     // row-parallel tensor parallelism (fused all-reduce in the GEMV): local exchange block + peer mappings

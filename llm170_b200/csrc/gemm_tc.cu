@@ -26,13 +26,10 @@
 
 #include "../../include/w4a16_b200.h"
 #include "dec.h"
+#include "gemm_common.cuh"
 #include "ptx.cuh"
 
 namespace w4 {
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 namespace {
 
@@ -87,16 +84,6 @@ struct GemmArgs {
     int tma_store;   // 1: whole dense tiles leave through shared memory and TMA stores (tmap_y)
 };
 
-// K-major, 128B-swizzled operand: 8-row groups are 1024 B apart (SBO), LBO unused, descriptor version 1.
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
-    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accum) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -105,10 +92,6 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t 
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accum)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -121,11 +104,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ uint32_t hmul2u(uint32_t a, uint32_t b) {
-    uint32_t r;
-    asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
-    return r;
-}
 template <int GROUP, int MT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_y,
@@ -283,9 +261,9 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     } else {
         // ------------------------------------------------------------------ dequantise, then epilogue
         const int dw = warp - 2;
-        // bank-conflict-free assignment of the 32 (g,t) slots of a tile to lanes (reads and writes)
-        const int ph = lane >> 3, jj = lane & 7;
-        const int t = jj & 3, g = 2 * ((t + ph) & 3) + (jj >> 2);
+        // bank-conflict-free assignment of the 32 (g,t) slots of a tile to lanes: g runs 0 3 4 7 | 1 2 5 6 over the quads, so
+        // that the 16-byte reads of a quarter-warp and the 8-byte swizzled writes of a half-warp hit distinct banks
+        const int t = lane & 3, g = (0x65217430u >> (4 * (lane >> 2))) & 7;
         const int ng = a.k / GROUP;
         bool ok = true;
         // scales of k-block `it` for this lane's two row blocks, fetched one k-block ahead
@@ -325,18 +303,17 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
                     const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
                     const uint32_t row_off = b_addr(sb) + (uint32_t)(rbi * TILE_ROWS + g) * 128u;
 #pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        uint32_t f0[4], f1[4];
-                        dequant_word(rw[2 * p], f0);
-                        dequant_word(rw[2 * p + 1], f1);
-                        const uint32_t s2 = sc[p];
+                    for (int w = 0; w < 4; ++w) {
+                        uint32_t f[4];
+                        dequant_word(rw[w], f);
+                        const uint32_t s2 = sc[w >> 1];
                         const uint32_t s_r0 = __byte_perm(s2, s2, 0x1010);  // (s[r0], s[r0])
                         const uint32_t s_r1 = __byte_perm(s2, s2, 0x3232);  // (s[r1], s[r1])
-                        const uint32_t chunk = (uint32_t)(((4 * p + t) ^ g) << 4);
-                        *reinterpret_cast<uint4*>(base_ptr + (row_off - base) + chunk) =
-                            make_uint4(hmul2u(f0[0], s_r0), hmul2u(f0[2], s_r0), hmul2u(f1[0], s_r0), hmul2u(f1[2], s_r0));
-                        *reinterpret_cast<uint4*>(base_ptr + (row_off - base) + 8u * 128u + chunk) =
-                            make_uint4(hmul2u(f0[1], s_r1), hmul2u(f0[3], s_r1), hmul2u(f1[1], s_r1), hmul2u(f1[3], s_r1));
+                        const uint32_t piece = (uint32_t)(((2 * w + (t >> 1)) ^ g) << 4) + (uint32_t)(t & 1) * 8u;
+                        *reinterpret_cast<uint2*>(base_ptr + (row_off - base) + piece) =
+                            make_uint2(hmul2u(f[0], s_r0), hmul2u(f[2], s_r0));
+                        *reinterpret_cast<uint2*>(base_ptr + (row_off - base) + 8u * 128u + piece) =
+                            make_uint2(hmul2u(f[1], s_r1), hmul2u(f[3], s_r1));
                     }
                 }
             }
@@ -630,6 +607,8 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     }
 }
 
+}  // namespace
+
 EncodeTiledFn encode_fn() {
     static EncodeTiledFn fn = nullptr;
     if (!fn) {
@@ -642,8 +621,6 @@ EncodeTiledFn encode_fn() {
     }
     return fn;
 }
-
-}  // namespace
 
 cudaError_t gemm_init_device() {
     cudaError_t e;
@@ -661,6 +638,9 @@ cudaError_t gemm_init_device() {
 int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st) {
     if (((uintptr_t)x & 15) != 0 || ((uintptr_t)dst & 15) != 0) {
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
+    }
+    if (tune_ts) {
+        return gemm_ts(l, x, dst, t, out_kind, st);
     }
     EncodeTiledFn enc = encode_fn();
     if (!enc) {

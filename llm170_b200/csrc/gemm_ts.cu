@@ -1,0 +1,603 @@
+// W4A16 GEMM with the weights as the TMEM operand:  y[m][n] = sum_k x[m][k] * f16((q[n][k]-8)*s[n][k/g]).
+//
+// Takes the place of the reference's small-batch FFMA family and of its prefill GEMMs
+// (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:44-723, kernels/marlin.rs:94-213) above the decode path's eight rows.
+// Like them it multiplies the dequantised weight ROUNDED ONCE TO F16 and accumulates in f32.
+//
+// The 128 rows of an MMA are WEIGHT rows and its N columns are tokens, so a batch of 9 tokens multiplies a 16-wide tile,
+// not a padded 128-row one.  The expanded weights never touch shared memory: a warp reads a raw int4 tile, expands it in
+// registers and stores it to TMEM (tcgen05.st.16x256b: the T64 layout keeps a lane's nibbles in exactly that register
+// order), where tcgen05.mma reads it as its A operand; the tokens are the shared-memory operand.
+//
+//   warp 0      producer: raw int4 of the CTA's rows (one bulk copy per 64-channel k-block, deep ring: this is what HBM
+//               latency is hidden with) and the token tile of the same k-block (TMA, 128B swizzle, shallow ring: L2)
+//   warp 1      one lane issues MT x 4 tcgen05.mma (M128, N tokens, K16) per k-block; commits hand the TMEM stage and
+//               the token stage back
+//   warps 2-17  raw -> registers -> TMEM, then the epilogue
+//
+// The K splits of a tile form a thread-block cluster and sum their f32 accumulators through distributed shared memory in
+// split order (no global scratch, no tickets).
+// Launched with programmatic stream serialization: raw weights are requested before the dependency wait.
+// Every wait is bounded: on expiry the kernel records a status code and all roles fall through to the common exit.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <string>
+
+#include "../../include/w4a16_b200.h"
+#include "dec.h"
+#include "gemm_common.cuh"
+#include "gemv_common.cuh"
+#include "ptx.cuh"
+
+namespace w4 {
+
+namespace {
+
+constexpr int TS_MROWS = 128;                   // weight rows per MMA
+constexpr int BK = TILE_K;
+constexpr int SK = 2 * BK;                      // channels per stage: two k-blocks, one 128-channel scale group
+constexpr int RAW_PER_MT = TS_MROWS * SK / 2;   // 8 KB per stage and 128-row block
+constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
+__host__ __device__ constexpr int ts_threads(int mt) { return (2 + 8 * mt) * 32; }
+constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
+// Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
+// waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
+// Half the TMEM: two CTAs per SM, never three; all of it: alone, also beside a CTA of the other kind.
+constexpr size_t TS_SMEM_HALF_MIN = 77 * 1024, TS_SMEM_HALF_MAX = 113 * 1024;
+constexpr size_t TS_SMEM_FULL_MIN = 152 * 1024, TS_SMEM_FULL_MAX = 226 * 1024;
+
+struct TsArgs {
+    const uint32_t* qt;
+    const uint32_t* st;
+    void* out;
+    int m, n, k;
+    int out_f16;
+    int m_tiles, n_tiles;
+    int tok;             // tokens per tile = MMA N (multiple of 16)
+    int nrb_w;           // 16-row blocks of the resident matrix (tile pitch)
+    int ksplit;
+    int raw_stages, x_stages, a_stages;
+    int tmem_cols;
+    int off_x, off_bars; // byte offsets in dynamic shared memory (1024-byte aligned base)
+    int pdl;
+    float out_mul;
+    int* status;
+    // grouped (MoE) mode: token tiles come from a device table, one expert's weights per tile
+    int grouped;
+    const int* tile_expert;
+    const int* tile_row0;
+    const int* tile_rows;
+    const int* num_tiles;
+    int expert0;
+    const float* row_w;
+    int glu;
+};
+
+__device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accum)
+        : "memory");
+}
+// 16 TMEM lanes x 32 columns from one warp: register 4i + {0,1} of lane (g, t) -> row g, columns 8i + 2t + {0,1};
+// register 4i + {2,3} -> row g + 8
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned cta_rank) {
+    uint32_t ra;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local_addr), "r"(cta_rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
+    return v;
+}
+
+// MT = 128-row weight blocks per CTA (the token tile is shared by them).
+template <int GROUP, int MT>
+__global__ void __launch_bounds__(ts_threads(MT), MT == 1 ? 2 : 1)
+gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+
+    constexpr int DQ_WARPS = 8 * MT;
+    constexpr int THREADS = ts_threads(MT);
+    constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
+    constexpr uint32_t RAW_BYTES = RAW_PER_MT * MT;
+    const int NR = a.raw_stages, NX = a.x_stages, NA = a.a_stages;
+    const int N = a.tok;
+    const uint32_t x_half = (uint32_t)N * (BK * 2);                  // one k-block of the token tile
+    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_BYTES; };
+    auto x_addr = [&](int s) { return base + (uint32_t)a.off_x + (uint32_t)s * (2 * x_half); };
+    const uint32_t bars = base + (uint32_t)a.off_bars;
+    auto raw_full = [&](int s) { return bars + 8u * s; };
+    auto raw_free = [&](int s) { return bars + 8u * (NR + s); };
+    auto x_full = [&](int s) { return bars + 8u * (2 * NR + s); };
+    auto x_free = [&](int s) { return bars + 8u * (2 * NR + NX + s); };
+    auto a_ready = [&](int s) { return bars + 8u * (2 * NR + 2 * NX + s); };
+    auto a_free = [&](int s) { return bars + 8u * (2 * NR + 2 * NX + NA + s); };
+    const uint32_t accum_bar = bars + 8u * (2 * NR + 2 * NX + 2 * NA);
+
+    // ---- this CTA's tile ----
+    const int tile = (int)blockIdx.x, ks = a.ksplit, split = (int)blockIdx.y;
+    const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
+    const int n0 = ntile * (TS_MROWS * MT);
+    int m0, rows_valid, rb0 = n0 / TILE_ROWS;
+    if (a.grouped) {
+        if (a.pdl) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");       // the segment table is the previous kernels' output
+        }
+        if (mtile >= *a.num_tiles) {
+            return;
+        }
+        m0 = a.tile_row0[mtile];
+        rows_valid = a.tile_rows[mtile];
+        rb0 += (a.tile_expert[mtile] - a.expert0) * (a.n / TILE_ROWS);
+    } else {
+        m0 = mtile * N;
+        rows_valid = min(N, a.m - m0);
+    }
+    const int nrbv = min(TS_MROWS * MT, a.n - n0) / TILE_ROWS;       // valid 16-row blocks
+    const uint32_t kb_bytes = (uint32_t)nrbv * (TILE_WORDS * 4);
+    // K range of this split in stages; the last stage of the matrix may hold one k-block (32-channel groups)
+    const int nkb_all = a.k / BK, st_all = (nkb_all + 1) / 2;
+    const int st0 = (int)((long long)st_all * split / ks);
+    const int nst = (int)((long long)st_all * (split + 1) / ks) - st0;
+    auto stage_kbs = [&](int it) { return min(2, nkb_all - 2 * (st0 + it)); };
+    auto issue_raw = [&](int it, int s) {
+        const int kbs = stage_kbs(it);
+        mbar_expect_tx(raw_full(s), kbs * kb_bytes);
+        const uint32_t* src = a.qt + ((size_t)(2 * (st0 + it)) * a.nrb_w + rb0) * TILE_WORDS;
+        bulk_load(raw_addr(s), src, kb_bytes, raw_full(s));
+        if (kbs == 2) {
+            bulk_load(raw_addr(s) + RAW_BYTES / 2, src + (size_t)a.nrb_w * TILE_WORDS, kb_bytes, raw_full(s));
+        }
+    };
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < NR; ++s) {
+            mbar_init(raw_full(s), 1);
+            mbar_init(raw_free(s), DQ_WARPS);
+        }
+        for (int s = 0; s < NX; ++s) {
+            mbar_init(x_full(s), 1);
+            mbar_init(x_free(s), 1);
+        }
+        for (int s = 0; s < NA; ++s) {
+            mbar_init(a_ready(s), DQ_WARPS);
+            mbar_init(a_free(s), 1);
+        }
+        mbar_init(accum_bar, 1);
+        mbar_init_fence();
+        // the weights do not depend on the previous kernel of the stream
+        for (int it = 0; it < NR && it < nst; ++it) {
+            issue_raw(it, it);
+        }
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                     "r"(a.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (a.pdl) {
+        // only now: a CTA of the next kernel that came earlier could take the TMEM this one still has to allocate, and
+        // then wait for this kernel
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    }
+    const uint32_t tmem = s_tmem_base;
+    const uint32_t tmem_a = tmem + (uint32_t)(MT * N);               // A ring: [stage][MT][64 columns]
+    volatile int* abort_flag = &s_abort;
+
+    bool ok = true;
+    if (warp == 0) {
+        // ------------------------------------------------------------------ producer
+        if (lane == 0) {
+            if (a.pdl) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");
+            }
+            int sx = 0, px = 1, sr = 0, pr = 0;                      // slot / parity of token stage it, of raw stage it + NR
+            for (int it = 0; it < nst; ++it) {
+                if (it >= NX && !mbar_wait(x_free(sx), px, abort_flag, a.status, (31 << 16) | it)) {
+                    break;
+                }
+                const int kbs = stage_kbs(it);
+                mbar_expect_tx(x_full(sx), kbs * x_half);
+                for (int h = 0; h < kbs; ++h) {
+                    tma_load_2d(x_addr(sx) + h * x_half, &tmap_x, (2 * (st0 + it) + h) * BK, m0, x_full(sx));
+                }
+                if (++sx == NX) {
+                    sx = 0;
+                    px ^= 1;
+                }
+                if (it + NR < nst) {
+                    if (!mbar_wait(raw_free(sr), pr, abort_flag, a.status, (32 << 16) | it)) {
+                        break;
+                    }
+                    issue_raw(it + NR, sr);
+                    if (++sr == NR) {
+                        sr = 0;
+                        pr ^= 1;
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        if (lane == 0) {
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
+            int sx = 0, px = 0, sa = 0, pa = 0;
+            for (int it = 0; it < nst; ++it) {
+                if (!mbar_wait(x_full(sx), px, abort_flag, a.status, (33 << 16) | it) ||
+                    !mbar_wait(a_ready(sa), pa, abort_flag, a.status, (34 << 16) | it)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const int kbs = stage_kbs(it);
+                for (int h = 0; h < kbs; ++h) {
+                    const uint64_t db = umma_desc(x_addr(sx) + h * x_half);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) {
+                        const uint32_t ta = tmem_a + (uint32_t)((sa * MT + mt) * A_COLS + h * (BK / 2));
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j) {
+                            umma_ts_f16(tmem + (uint32_t)(mt * N), ta + j * 8, db + 2 * j, idesc, (it > 0 || h > 0 || j > 0) ? 1u : 0u);
+                        }
+                    }
+                }
+                umma_commit(a_free(sa));
+                umma_commit(x_free(sx));
+                if (++sx == NX) {
+                    sx = 0;
+                    px ^= 1;
+                }
+                if (++sa == NA) {
+                    sa = 0;
+                    pa ^= 1;
+                }
+            }
+            if (ok) {
+                umma_commit(accum_bar);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM
+        // One 16-row block per warp.  A warp may touch the TMEM lanes 32 * (warp % 4) .. +31 = two row blocks of each
+        // 128-row block.
+        const int quad = warp & 3, sub = (warp - 2) >> 2;
+        const int half = sub & 1, mt = sub >> 1;
+        const int rb = mt * (TS_MROWS / TILE_ROWS) + quad * 2 + half;
+        const bool live = rb < nrbv;
+        const int rbl = live ? rb : 0;
+        const int ng = a.k / GROUP;
+        // scale words (rows g, g + 8) of this row block, two stages ahead of their use
+        const uint32_t* sp = a.st + ((size_t)(rb0 + rbl) * ng + (size_t)st0 * GPS) * 8 + (lane >> 2);
+        int sleft = ng - st0 * GPS;                                  // groups left in the row block
+        auto load_scales = [&](uint32_t (&sc)[GPS]) {
+#pragma unroll
+            for (int i = 0; i < GPS; ++i) {
+                sc[i] = i < sleft ? __ldg(sp + i * 8) : 0u;
+            }
+            sp += GPS * 8;
+            sleft -= GPS;
+        };
+        uint32_t sc0[GPS], sc1[GPS];
+        load_scales(sc0);
+        load_scales(sc1);
+        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16) + (uint32_t)(mt * A_COLS);
+        const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+        auto expand = [&](const uint4& raw, const uint32_t s_a, const uint32_t s_b, uint32_t (&v)[16]) {
+            const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint32_t f[4];
+                dequant_word(rw[w], f);
+                const uint32_t s2 = w < 2 ? s_a : s_b;
+                const uint32_t s_r0 = __byte_perm(s2, s2, 0x1010), s_r1 = __byte_perm(s2, s2, 0x3232);
+                v[4 * w + 0] = hmul2u(f[0], s_r0);
+                v[4 * w + 1] = hmul2u(f[2], s_r0);
+                v[4 * w + 2] = hmul2u(f[1], s_r1);
+                v[4 * w + 3] = hmul2u(f[3], s_r1);
+            }
+        };
+        int sr = 0, pr = 0, sa = 0, pa = 1;
+        for (int it = 0; it < nst; ++it) {
+            // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
+            if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (35 << 16) | it))) {
+                ok = false;
+                break;
+            }
+            const uint32_t ra = r_ld + (uint32_t)sr * RAW_BYTES;
+            const uint4 raw0 = lds128(ra);
+            const uint4 raw1 = lds128(ra + RAW_BYTES / 2);           // stale bytes when the stage holds one k-block
+            uint32_t sc[GPS];
+#pragma unroll
+            for (int i = 0; i < GPS; ++i) {
+                sc[i] = sc0[i];
+                sc0[i] = sc1[i];
+            }
+            load_scales(sc1);
+            uint32_t v[16];
+            expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
+            if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t td = t_st + (uint32_t)(sa * MT * A_COLS);
+            tmem_st_16x256b_x4(td, v);
+            expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
+            }
+            tmem_st_16x256b_x4(td + BK / 2, v);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(a_ready(sa));
+            }
+            if (++sr == NR) {
+                sr = 0;
+                pr ^= 1;
+            }
+            if (++sa == NA) {
+                sa = 0;
+                pa ^= 1;
+            }
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        ok = ok && mbar_wait(accum_bar, 0, abort_flag, a.status, (37 << 16));
+        ok = __all_sync(0xffffffffu, ok);
+        if (a.pdl && !a.grouped) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");       // outputs may be what the previous kernel still reads
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+
+    // ---------------------------------------------------------------------- epilogue
+    const bool dq_warp = warp >= 2;
+    const int quad = warp & 3, sub = (warp - 2) >> 2;
+    const int emt = sub >> 1;                                        // 128-row block of this warp's accumulator lanes
+    constexpr int EW = 2;                                            // warps that share a (row block, quadrant)
+    const int ei = sub & 1;
+    const int lrow = emt * TS_MROWS + quad * 32 + lane;              // weight row within the tile
+    if (ks == 1) {
+        if (dq_warp && ok) {
+            const bool row_ok = n0 + lrow < a.n;
+            for (int c0 = ei * 16; c0 < rows_valid; c0 += EW * 16) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(emt * N + c0), v);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int tok = c0 + i;
+                    float f = __uint_as_float(v[i]) * a.out_mul;
+                    if (a.glu) {
+                        // lanes 0-15 hold the gate sums, lanes 16-31 the up sums of the same 16 outputs
+                        const float up = __shfl_down_sync(0xffffffffu, f, 16);
+                        if (tok < rows_valid && lane < 16 && row_ok) {
+                            reinterpret_cast<__half*>(a.out)[(size_t)(m0 + tok) * (a.n / 2) + (n0 + emt * TS_MROWS + quad * 32) / 2 + lane] =
+                                silu_mul_f16(f, up);
+                        }
+                    } else if (tok < rows_valid && row_ok) {
+                        if (a.row_w != nullptr) {
+                            f = mul_row_w(f, a.row_w[m0 + tok]);
+                        }
+                        const size_t o = (size_t)(m0 + tok) * a.n + n0 + lrow;
+                        if (a.out_f16) {
+                            reinterpret_cast<__half*>(a.out)[o] = __float2half_rn(f);
+                        } else {
+                            reinterpret_cast<float*>(a.out)[o] = f;
+                        }
+                    }
+                }
+            }
+        }
+    } else {
+        // the splits' accumulators meet in distributed shared memory, RED_TOK tokens at a time: [token][row] f32 over the
+        // (idle) rings; every CTA of the cluster adds an equal share of the elements over all splits, in split order
+        constexpr int ROWS = TS_MROWS * MT;
+        for (int cb = 0; cb < rows_valid; cb += RED_TOK) {
+            const int nt = min(RED_TOK, rows_valid - cb);
+            if (dq_warp && ok) {
+                for (int c0 = ei * 16; c0 < nt; c0 += EW * 16) {
+                    uint32_t v[16];
+                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(emt * N + cb + c0), v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        *reinterpret_cast<float*>(base_ptr + ((c0 + i) * ROWS + lrow) * 4) = __uint_as_float(v[i]);
+                    }
+                }
+            }
+            cluster_sync_all();
+            const int nr4 = min(ROWS, a.n - n0) / 4;
+            const int total = nt * nr4;
+            const int e0 = (int)((long long)total * split / ks), e1 = (int)((long long)total * (split + 1) / ks);
+            for (int e = e0 + (int)threadIdx.x; e < e1; e += THREADS) {
+                const int tok = e / nr4, r = (e - tok * nr4) * 4;
+                float4 pv[8];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    pv[s] = s < ks ? ld_dsmem_f32x4(base + (uint32_t)((tok * ROWS + r) * 4), (unsigned)s) : make_float4(0, 0, 0, 0);
+                }
+                float4 sum = pv[0];
+#pragma unroll
+                for (int s = 1; s < 8; ++s) {
+                    if (s < ks) {
+                        sum.x += pv[s].x;
+                        sum.y += pv[s].y;
+                        sum.z += pv[s].z;
+                        sum.w += pv[s].w;
+                    }
+                }
+                sum.x *= a.out_mul;
+                sum.y *= a.out_mul;
+                sum.z *= a.out_mul;
+                sum.w *= a.out_mul;
+                const size_t o = (size_t)(m0 + cb + tok) * a.n + n0 + r;
+                if (a.out_f16) {
+                    const __half2 h0 = __floats2half2_rn(sum.x, sum.y), h1 = __floats2half2_rn(sum.z, sum.w);
+                    *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(a.out) + o) =
+                        make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+                } else {
+                    *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) = sum;
+                }
+            }
+            cluster_sync_all();   // before the buffer is filled again, and before any CTA of the cluster leaves
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+    }
+}
+
+}  // namespace
+
+
+static size_t ts_smem(int mt, int tok, int nr, int nx, int na, int* off_x, int* off_bars) {
+    size_t off = (size_t)nr * RAW_PER_MT * mt;                      // multiples of 1024
+    *off_x = (int)off;
+    off += (size_t)nx * tok * SK * 2;
+    const size_t red = (size_t)std::min(RED_TOK, tok) * TS_MROWS * mt * 4;   // the cluster's sum reuses the rings
+    off = std::max(off, red);
+    *off_bars = (int)off;
+    return off + (size_t)(2 * nr + 2 * nx + 2 * na + 1) * 8 + 1024;
+}
+
+cudaError_t gemm_ts_init_device() {
+    cudaError_t e = cudaSuccess;
+#define W4_SET(G, MTV) \
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_ts_kernel<G, MTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
+    W4_SET(128, 1)
+    W4_SET(128, 2)
+    W4_SET(32, 1)
+    W4_SET(32, 2)
+#undef W4_SET
+    return e;
+}
+
+int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) {
+        return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
+    }
+    const int mt = tune_ts_mt ? tune_ts_mt : 2;
+    int tok_cap = tune_ts_tok ? tune_ts_tok : 128;
+    TsArgs a{};
+    a.m_tiles = (t + tok_cap - 1) / tok_cap;
+    a.tok = ((t + a.m_tiles - 1) / a.m_tiles + 15) / 16 * 16;
+    a.n_tiles = (l->n + TS_MROWS * mt - 1) / (TS_MROWS * mt);
+    a.ksplit = tune_ts_ks ? tune_ts_ks : 1;
+    a.ksplit = std::min(a.ksplit, (l->k + SK - 1) / SK);
+    // TMEM: accumulators and as many expanded k-blocks as fit in half of it (two CTAs per SM), else in all of it
+    const int acc = mt * a.tok;
+    int na = (256 - acc) / (A_COLS * mt);
+    a.tmem_cols = 256;
+    if (mt == 2 || na < 2) {
+        na = (512 - acc) / (A_COLS * mt);
+        a.tmem_cols = 512;
+    }
+    if (na < 2) return fail("w4a16 gemm: na");
+    na = std::min(na, 4);
+    a.a_stages = na;
+    const size_t limit = a.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
+    int nx = 2, nr = 2;
+    while (nr < 12 && ts_smem(mt, a.tok, nr + 1, nx, na, &a.off_x, &a.off_bars) <= limit) {
+        ++nr;
+        if (nr % 2 == 0 && nx < 4 && ts_smem(mt, a.tok, nr, nx + 1, na, &a.off_x, &a.off_bars) <= limit) {
+            ++nx;
+        }
+    }
+    a.raw_stages = nr;
+    a.x_stages = nx;
+    const size_t smem = ts_smem(mt, a.tok, nr, nx, na, &a.off_x, &a.off_bars);
+    if (smem > limit) {
+        return fail("w4a16 gemm: tile of %d tokens does not fit", a.tok);
+    }
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)l->k, (cuuint64_t)t};
+    const cuuint64_t strides[1] = {(cuuint64_t)l->k * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)a.tok};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) {
+        return fail("w4a16 gemm: cuTensorMapEncodeTiled failed (%d)", (int)cr);
+    }
+    a.qt = l->qt;
+    a.st = (const uint32_t*)l->st;
+    a.out = dst;
+    a.m = t;
+    a.n = l->n;
+    a.k = l->k;
+    a.out_f16 = out_kind == W4A16_OUT_F16;
+    a.nrb_w = l->n / TILE_ROWS;
+    a.pdl = tune_pdl ? 1 : 0;
+    a.out_mul = l->out_mul;
+    a.status = gemm_status;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(a.m_tiles * a.n_tiles, a.ksplit);
+    cfg.blockDim = dim3(ts_threads(mt));
+    cfg.dynamicSmemBytes = std::max(smem, a.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
+    if (a.pdl) {
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
+    }
+    if (a.ksplit > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = 1;
+        attr[n_attr].val.clusterDim.y = a.ksplit;
+        attr[n_attr].val.clusterDim.z = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
+    cudaError_t e;
+    if (l->group == 128) {
+        e = mt == 2 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, 2>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, 1>, map, a);
+    } else {
+        e = mt == 2 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, 2>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, 1>, map, a);
+    }
+    if (e != cudaSuccess) {
+        return cuda_fail("launch gemm", e);
+    }
+    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "," + std::to_string(mt) + "> tok " + std::to_string(a.tok) + " ks " + std::to_string(a.ksplit) + " nr " + std::to_string(nr) + " nx " + std::to_string(nx) + " na " + std::to_string(na);
+    launches++;
+    return 0;
+}
+
+}  // namespace w4

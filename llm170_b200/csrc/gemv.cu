@@ -59,7 +59,7 @@ constexpr int GEMV_SMEM_LIMIT = 112 * 1024;       // two CTAs per SM
 constexpr int SC_STAGE_MAX = 32 * 1024;           // most scale bytes a CTA stages in shared memory
 
 struct SmemPlan {
-    int x_stride;   // halves per token row (byte stride = 64 mod 128: conflict-free 128-bit reads)
+    int x_stride;   // halves per token row (byte stride = 32 mod 128: conflict-free 64-bit reads)
     int x_rows;     // token rows staged (m, plus one all-zero row when m < 8)
     int off_xsum;   // f32 [groups][4 lane columns][4]: the zero-point term of each group as MMA C operands
     int off_sc;     // u32 [16 row blocks][groups][8]: this CTA's scale pairs (when sc_staged)
@@ -75,7 +75,7 @@ __host__ SmemPlan make_plan(int k, int group, int m, int ksplit, int stages) {
     p.stages = stages < 2 ? 2 : (stages > MAX_STAGES ? MAX_STAGES : stages);
     const int halves = max_split_kblocks(k, group, ksplit) * TILE_K;
     const int ngl = halves / group;
-    p.x_stride = halves + 32;
+    p.x_stride = halves + 16;
     p.x_rows = m < GEMV_MAX_M ? m + 1 : m;
     int off = p.x_rows * p.x_stride * 2;
     off = (off + 127) & ~127;
@@ -368,7 +368,7 @@ gemv_w4a16_kernel(const GemvArgs a, const SmemPlan p) {
         }
         // B fragment source: token g (the zero row when g >= m), this lane's 8 k of each half k-block
         const int xrow_i = g < m_loc ? g : m_loc;
-        const unsigned char* xp = smem + (size_t)(xrow_i * p.x_stride + 8 * t) * 2;
+        const unsigned char* xp = smem + (size_t)(xrow_i * p.x_stride + 4 * t) * 2;
         const unsigned char* zp = smem + p.off_xsum + t * 16;
         const unsigned char* wbase = smem + p.off_ring + rbw0 * (TILE_WORDS * 4) + lane * 16;
 
@@ -390,8 +390,8 @@ gemv_w4a16_kernel(const GemvArgs a, const SmemPlan p) {
             for (int r = 0; r < RB_PER_WARP; ++r) {
                 R.w[r] = *reinterpret_cast<const uint4*>(wa + r * (TILE_WORDS * 4));
             }
-            R.x0 = *reinterpret_cast<const uint4*>(xa);
-            R.x1 = *reinterpret_cast<const uint4*>(xa + 64);
+            R.x0 = lds_2x64(xa);
+            R.x1 = lds_2x64(xa + 64);
         };
         auto expand = [&](uint32_t w, uint32_t (&fr)[4]) {
             if (SUBN) {

@@ -36,6 +36,13 @@ __device__ __forceinline__ void mma16816_c(float (&d)[4], const uint32_t (&a)[4]
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
 }
 
+// The token operands of two MMAs of a tile (words w, w+1 of the lane: k = 16w + 4t + {0..3} and 16 further on): two 8-byte
+// shared-memory reads, 32 bytes apart.
+__device__ __forceinline__ uint4 lds_2x64(const unsigned char* p) {
+    const uint2 a = *reinterpret_cast<const uint2*>(p), b = *reinterpret_cast<const uint2*>(p + 32);
+    return make_uint4(a.x, a.y, b.x, b.y);
+}
+
 __device__ __forceinline__ void st_release_sys(unsigned* p, unsigned v) {
     asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }

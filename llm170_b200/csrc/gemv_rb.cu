@@ -51,6 +51,15 @@ constexpr int RB_MAXTOK = 4;
 constexpr int RB_XPAD = 64;       // bytes added to a token's row of x so that the two tokens of a quarter-warp hit distinct banks
 constexpr int RB_GROUP = 128;
 
+// Activations in shared memory: inside every 32 channels the 8-byte pieces are reordered so that lane t's pieces of two
+// consecutive MMAs (channels 4t.. and 16 + 4t..) are adjacent: one 16-byte read per lane and MMA pair.  `c` = index of the
+// 16-byte piece `u` (two of those 8-byte pieces) within the token's row.
+__device__ __forceinline__ void stage_x16(unsigned char* row, int c, const uint4& u) {
+    unsigned char* d = row + (size_t)(c >> 2) * 64 + (c & 1) * 32 + ((c >> 1) & 1) * 8;
+    *reinterpret_cast<uint2*>(d) = make_uint2(u.x, u.y);
+    *reinterpret_cast<uint2*>(d + 16) = make_uint2(u.z, u.w);
+}
+
 // RBW = 16-row blocks per unit (2: a warp multiplies two neighbouring tiles with the same activation fragments, two
 // CTAs per SM;  1: for matrices with fewer row blocks than SMs -- tensor-parallel shards --, so that more CTAs stream,
 // three CTAs per SM).
@@ -219,7 +228,7 @@ __global__ void __launch_bounds__(RB_THREADS, RBW == 2 ? 2 : 3) gemv_rb_kernel(c
                 if (live) {
                     tok = i / per_tok;
                     c = i - tok * per_tok;
-                    *reinterpret_cast<uint4*>(smem + (size_t)tok * xstride + (size_t)c * 16) = u;
+                    stage_x16(smem + (size_t)tok * xstride, c, u);
                 }
                 const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
                 const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
@@ -343,8 +352,8 @@ __global__ void __launch_bounds__(RB_THREADS, RBW == 2 ? 2 : 3) gemv_rb_kernel(c
                         wv[r] = wq[u + h][r];
                     }
                     fetch(wq[u + h]);                                      // refill the slot at once
-                    // word 2p+q of the lane holds rows g, g+8 at channels 32p + 8t + 4q + {0..3}: the activations of
-                    // the same channels are 8 consecutive f16 at 8t (p = 0) and at 32 + 8t (p = 1)
+                    // word w of the lane holds rows g, g+8 at channels 16w + 4t + {0..3}; the activations of words 0, 1 and
+                    // of words 2, 3 are 16 bytes each (stage_x16)
                     const uint4 x0 = *reinterpret_cast<const uint4*>(xl + kb * xk);
                     const uint4 x1 = *reinterpret_cast<const uint4*>(xl + kb * xk + xh);
                     uint32_t af[4];
@@ -516,7 +525,7 @@ __global__ void __launch_bounds__(RU_THREADS, 2) gemv_ru_kernel(const GemvArgs a
                 if (live) {
                     tok = i / per_tok;
                     c = i - tok * per_tok;
-                    *reinterpret_cast<uint4*>(smem + (size_t)tok * xstride + (size_t)c * 16) = u;
+                    stage_x16(smem + (size_t)tok * xstride, c, u);
                 }
                 const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
                 const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));

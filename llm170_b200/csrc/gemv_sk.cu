@@ -63,7 +63,7 @@ SkPlan sk_make_plan(int k, int group, int m, int rows, int sm_count, int max_sta
     for (;;) {
         const int nu = (int)((p.units + ctas - 1) / ctas);
         p.nu_max = nu;
-        p.x_stride = nu * UNIT_K + 32;
+        p.x_stride = nu * UNIT_K + 16;
         int off = p.x_rows * p.x_stride * 2;
         off = (off + 127) & ~127;
         p.off_zc = off;
@@ -381,7 +381,7 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
             tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
         }
         const int xrow_i = g < m ? g : m;
-        const unsigned char* xp = smem + (size_t)(xrow_i * p.x_stride + 8 * t) * 2;
+        const unsigned char* xp = smem + (size_t)(xrow_i * p.x_stride + 4 * t) * 2;
         const unsigned char* zp = smem + p.off_zc + t * 16;
         const unsigned char* scq = smem + p.off_sc + ((size_t)rbw0 * p.nu_max * GPU_ * 8 + g) * 4;
         const size_t sc_rb_stride = (size_t)p.nu_max * GPU_ * 32;
@@ -400,8 +400,8 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
             for (int r = 0; r < RBW; ++r) {
                 R.w[r] = *reinterpret_cast<const uint4*>(wa + r * (TILE_WORDS * 4));
             }
-            R.x0 = *reinterpret_cast<const uint4*>(xa);
-            R.x1 = *reinterpret_cast<const uint4*>(xa + 64);
+            R.x0 = lds_2x64(xa);
+            R.x1 = lds_2x64(xa + 64);
             if (GROUP >= UNIT_K) {
                 // one group per unit: its zero-point term opens k-block 0, its scale closes k-block 1
                 if (hk == 0) {

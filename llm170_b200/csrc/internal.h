@@ -127,7 +127,7 @@ struct SkPlan {
     long long units;    // rows * units_per_row
     int ctas;           // grid size; CTA p owns units [units*p/ctas, units*(p+1)/ctas)
     int nu_max;         // most units one CTA owns
-    int x_stride;       // halves per staged token row (byte stride = 64 mod 128)
+    int x_stride;       // halves per staged token row (byte stride = 32 mod 128)
     int x_rows;         // token rows staged (m, plus one all-zero row when m < 8)
     int off_zc;         // f32 [local group][4 lane columns][4]: zero-point terms as MMA C operands
     int off_sc;         // u32 [16 row blocks][local group][8]: the CTA's scale pairs
@@ -153,6 +153,7 @@ const char* gemv_rb_variant(const GemvArgs& a, int total_units, int rbw, int sm_
 // ---- gemm_tc.cu ------------------------------------------------------------------------------
 // Raises the dynamic shared-memory limit of the tensor-core GEMM kernels on the current device.
 cudaError_t gemm_init_device();
+cudaError_t gemm_ts_init_device();
 cudaError_t head_init_device();
 
 // ---- moe.cu ----------------------------------------------------------------------------------

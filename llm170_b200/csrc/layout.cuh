@@ -10,16 +10,17 @@
 //   st : f16 [N/16][K/group][8][2]                      (pair j = scales of rows j and j+8; group 128 or 32 --
 //                                                        64-channel groups are stored as two groups of 32)
 //
-// Inside a tile, lane = 4*g + t (g = 0..7, t = 0..3) and word w = 2*p + h (p, h in {0,1}) hold
-// rows r0 = 16*rb + g and r1 = r0 + 8 at k = 64*kb + 32*p + 8*t + 4*h + {0,1,2,3}:
+// Inside a tile, lane = 4*g + t (g = 0..7, t = 0..3) and word w = 0..3 hold rows r0 = 16*rb + g and
+// r1 = r0 + 8 at k = 64*kb + 16*w + 4*t + {0,1,2,3}:
 //
 //   nibble position : 0      4      1      5      2      6      3      7
 //   element         : r0,k+0 r0,k+1 r1,k+0 r1,k+1 r0,k+2 r0,k+3 r1,k+2 r1,k+3
 //
 // so that (word & 0x000f000f), (word & 0x00f000f0), and the same two masks of (word >> 8) are,
 // in that order, the four half2 registers a0..a3 of an m16n8k16 A fragment whose 16 rows are the
-// tile's rows -- and, for the GEMM, one lane's 16 bytes expand to four whole 16-byte chunks
-// (8 consecutive k of one row) of a 128B-swizzled K-major shared-memory operand.
+// tile's rows (its k order inside the 16 is 4t..4t+3 per lane, so the token operand of such an MMA is
+// one 8-byte load per lane) -- and, for the GEMM, the expanded registers of a lane are in the order in
+// which tcgen05.st.16x256b spreads them over 16 TMEM lanes x 8 columns, columns in natural k order.
 // A warp reads a tile with one 128-bit load per lane, fully coalesced.  Tiles are ordered k-block
 // major: the tiles of neighbouring row blocks at one k-block are contiguous, so a CTA that owns R
 // row blocks fetches R*512 contiguous bytes per k-block with ONE bulk copy (8 KB for the GEMM's 256-row
@@ -65,12 +66,12 @@ __host__ __device__ inline size_t word_index(int row, int kk, int n_total, int* 
     const int rb = row / TILE_ROWS, rr = row % TILE_ROWS;
     const int g = rr & 7, hi_row = rr >> 3;
     const int kb = kk / TILE_K, kr = kk % TILE_K;
-    const int p = kr >> 5, t = (kr >> 3) & 3, h = (kr >> 2) & 1, e = kr & 3;
+    const int w = kr >> 4, t = (kr >> 2) & 3, e = kr & 3;
     // e: 0 -> pos 0, 1 -> pos 4, 2 -> pos 2, 3 -> pos 6 ; rows r1 shift by one position
     const int base = ((e & 1) << 2) | (e & 2);
     *nib_pos = base + hi_row;
     const size_t tile = (size_t)kb * (size_t)(n_total / TILE_ROWS) + (size_t)rb;
-    return tile * TILE_WORDS + (size_t)(4 * g + t) * 4 + (size_t)(2 * p + h);
+    return tile * TILE_WORDS + (size_t)(4 * g + t) * 4 + (size_t)w;
 }
 
 }  // namespace w4

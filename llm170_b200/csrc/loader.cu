@@ -430,7 +430,7 @@ struct CacheHeader {
     uint64_t source_tag;    // what the tiles were made from (w4a16_st_lin_tag of the source tensors)
     uint64_t q_bytes, s_bytes;
 };
-constexpr uint32_t CACHE_VERSION = 1;
+constexpr uint32_t CACHE_VERSION = 2;   // 2: a lane's word w holds channels 16w + 4t .. of its tile (layout.cuh)
 constexpr size_t IO_CHUNK = 8u << 20;   // 8 MiB, the reference's upload chunk (w4a16_dec/mem.rs)
 
 }  // namespace

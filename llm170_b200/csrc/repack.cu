@@ -35,10 +35,10 @@ __device__ __forceinline__ WordCoord coord_of(size_t widx, int nrb) {
     const size_t tile = widx >> 7;
     const int rb = (int)(tile % (size_t)nrb);
     const int kb = (int)(tile / (size_t)nrb);
-    const int g = lane >> 2, t = lane & 3, p = w >> 1, h = w & 1;
+    const int g = lane >> 2, t = lane & 3;
     WordCoord c;
     c.r0 = rb * TILE_ROWS + g;
-    c.kbase = kb * TILE_K + 32 * p + 8 * t + 4 * h;
+    c.kbase = kb * TILE_K + 16 * w + 4 * t;
     return c;
 }
 
@@ -76,7 +76,7 @@ __global__ void repack_q_rows_kernel(const uint32_t* __restrict__ q, uint32_t* _
 }
 
 __global__ void unpack_q_kernel(const uint32_t* __restrict__ qt, uint32_t* __restrict__ q, int n, int k) {
-    // one thread per ORIGINAL word (8 consecutive k of one row) = two packed words (h = 0, 1)
+    // one thread per ORIGINAL word (8 consecutive k of one row) = the same packed word of two neighbouring lanes
     const size_t total = (size_t)n * (size_t)(k / 8);
     const int k8 = k / 8;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
