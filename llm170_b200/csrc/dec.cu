@@ -480,6 +480,9 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
         if (e == cudaSuccess) {
             e = w4::gemm_ts_init_device();
         }
+        if (e == cudaSuccess) {
+            d.ts_query_clusters();
+        }
     }
     if (e == cudaSuccess) {
         e = w4::head_init_device();
@@ -628,10 +631,18 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         d.tune_gemv_stages = value;
         return 0;
     }
-    if (!strcmp(key, "ts")) { d.tune_ts = value; return 0; }
-    if (!strcmp(key, "ts_mt")) { d.tune_ts_mt = value; return 0; }
-    if (!strcmp(key, "ts_tok")) { d.tune_ts_tok = value; return 0; }
-    if (!strcmp(key, "ts_ks")) { d.tune_ts_ks = value; return 0; }
+    if (!strcmp(key, "gemm_form")) {
+        d.tune_gemm_form = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemm_ts_tok")) {
+        d.tune_ts_tok = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemm_ts_ksplit")) {
+        d.tune_ts_ks = value;
+        return 0;
+    }
     if (!strcmp(key, "gemm_mt")) {
         if (value < 0 || value > 2) {
             return d.fail("w4a16 tuning: gemm_mt must be 0, 1 or 2");

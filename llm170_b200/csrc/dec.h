@@ -52,6 +52,13 @@ struct GemvChoice {
     char name[64] = {0};       // the kernel instantiation, for reports
 };
 
+// Tile and K split of the TMEM-operand GEMM for a call, with the estimated time in microseconds.
+constexpr int TS_MAX_SPLIT = 8;
+struct TsChoice {
+    int tok, ks;
+    double cost;
+};
+
 struct Dec {
     int device = 0;
     int sm_count = 148;
@@ -95,7 +102,10 @@ struct Dec {
     int tune_gemm_mt = 0;        // 128-token blocks per GEMM tile: 0 = automatic, 1 or 2
     int tune_gemm_ksplit = 0;    // K splits of the GEMM: 0 = automatic (only when the tiles do not fill the SMs)
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
-    int tune_ts = 1, tune_ts_mt = 0, tune_ts_tok = 0, tune_ts_ks = 0;
+    int tune_gemm_form = 0;      // above the decode rows: 0 = automatic, 1 = token rows (gemm_tc.cu), 2 = weight rows (gemm_ts.cu)
+    int tune_ts_tok = 0;         // gemm_ts.cu: most tokens per tile (64, 96, 128, 192, 256), 0 = automatic
+    int tune_ts_ks = 0;          // gemm_ts.cu: K splits (1..8), 0 = automatic
+    int ts_clusters[2][TS_MAX_SPLIT + 1] = {};   // resident clusters of 1..8 CTAs, for CTAs with half and all of the TMEM
     long long* dbg_buf = nullptr;  // device timeline buffer (DBG_SLOTS entries) when the knob is on
     int tune_gemv_ksplit = 0;
     // kernels launched by forward calls since creation
@@ -117,7 +127,9 @@ struct Dec {
     int gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, int t, int out_kind,
              cudaStream_t st, bool allreduce = false);
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
-    int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
+    void ts_query_clusters();
+    TsChoice gemm_ts_choose(int n, int k, int t) const;
+    int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
     int gemm_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b,
                      int max_tiles, int mt, const float* row_w, cudaStream_t st);
     // row-parallel tensor parallelism (fused all-reduce in the GEMV): local exchange block + peer mappings

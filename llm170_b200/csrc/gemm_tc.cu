@@ -639,8 +639,78 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     if (((uintptr_t)x & 15) != 0 || ((uintptr_t)dst & 15) != 0) {
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
     }
-    if (tune_ts) {
-        return gemm_ts(l, x, dst, t, out_kind, st);
+    const int n_tiles = (l->n + BN - 1) / BN;
+    // Tile shape and K split are chosen together by a small cost model (times in microseconds, fitted to measurements
+    // on B200): a CTA takes 0.75 us per k-block with one 128-token block and 0.95 us with two (twice the tokens), 5 us
+    // around its loop, and a split CTA another 4 + 6 us per token block for writing, awaiting and adding f32 partial
+    // tiles.  Candidates per tile shape: whole tiles only; whole tiles plus a split last wave; every tile split
+    // 2..16 ways (at least four k-blocks per split, partial tiles within 128 MB of scratch).
+    const int nkb_all = l->k / BK;
+    struct Choice {
+        int mt, n_whole, ks;
+        double cost;
+    };
+    Choice best{1, 0, 1, 1e30};
+    for (int mtc = 1; mtc <= 2; ++mtc) {
+        if ((tune_gemm_mt == 1 || tune_gemm_mt == 2) && mtc != tune_gemm_mt) {
+            continue;
+        }
+        const int m_tiles = (t + BM * mtc - 1) / (BM * mtc);
+        // a second, empty token block is neither fetched nor multiplied: its k-blocks cost what one block costs
+        const bool half_empty = mtc == 2 && t <= BM;
+        const double per_kb = (mtc == 2 && !half_empty) ? 0.95 : 0.75;
+        const long long tiles = (long long)m_tiles * n_tiles;
+        const double tile_bytes = (double)BM * mtc * BN * 4.0;
+        auto cta_cost = [&](int nk, bool split) { return nk * per_kb + 5.0 + (split ? 4.0 + 6.0 * mtc : 0.0); };
+        auto consider = [&](long long n_whole, int ks) {
+            const long long split_tiles = tiles - n_whole;
+            if (ks > 1 && (split_tiles > 4096 || split_tiles * ks * tile_bytes > 128.0 * (1 << 20))) {
+                return;
+            }
+            const int nk_split = (nkb_all + ks - 1) / ks;
+            double c = (double)((n_whole + sm_count - 1) / sm_count) * cta_cost(nkb_all, false);
+            if (split_tiles > 0) {
+                c += (double)((split_tiles * ks + sm_count - 1) / sm_count) * cta_cost(nk_split, ks > 1);
+            }
+            if (c < best.cost) {
+                best = Choice{mtc, (int)n_whole, ks, c};
+            }
+        };
+        if (tune_gemm_ksplit > 0) {
+            consider(0, std::min(tune_gemm_ksplit, std::max(1, nkb_all)));
+            continue;
+        }
+        consider(tiles, 1);
+        if (tune_gemm_ksplit < 0) {
+            continue;
+        }
+        const long long rem = tiles % sm_count;
+        if (rem > 0 && tiles > sm_count) {
+            for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
+                consider(tiles - rem, ks);
+            }
+        }
+        for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
+            consider(0, ks);
+        }
+    }
+    // The weight-row form (gemm_ts.cu) takes the calls that it finishes sooner: up to about 128 tokens all of them (its MMA
+    // tile is as wide as the batch, 30.6 against 52 us for 16 x 34816 x 5120), above that those whose 256-token tiles leave
+    // SMs idle (320 x 5120 x 6144: 24.5 against 48 us); full waves of 256 x 256 tiles run a third faster here (1024 x 34816
+    // x 5120: 274 against 355 us).  This form's time for the comparison: per k-block 0.60 us with one token block and 0.78
+    // with two, 5 us around a wave, 3.5 us and 0.065 us per row for a split tile.
+    if (tune_gemm_form != 1 && (tune_gemm_form == 2 || (tune_gemm_ksplit == 0 && tune_gemm_mt == 0))) {
+        const long long tiles = (long long)((t + BM * best.mt - 1) / (BM * best.mt)) * n_tiles;
+        const double per_kb = best.mt == 2 && t > BM ? 0.78 : 0.60;
+        const int nk_split = (nkb_all + best.ks - 1) / best.ks;
+        const long long whole = best.ks > 1 ? best.n_whole : tiles, split_ctas = (tiles - whole) * best.ks;
+        const double tc_cost = (double)((whole + sm_count - 1) / sm_count) * (nkb_all * per_kb + 5.0) +
+                               (double)((split_ctas + sm_count - 1) / sm_count) *
+                                   (nk_split * per_kb + 8.5 + 0.065 * std::min(t, BM * best.mt));
+        const TsChoice c = gemm_ts_choose(l->n, l->k, t);
+        if (tune_gemm_form == 2 || c.cost < 0.9 * tc_cost) {   // at a tie whole 256 x 256 tiles vary less with the clock
+            return gemm_ts(l, x, dst, t, out_kind, c, st);
+        }
     }
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
@@ -680,61 +750,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     a.n = l->n;
     a.k = l->k;
     a.out_f16 = out16;
-    a.n_tiles = (l->n + BN - 1) / BN;
-    // Tile shape and K split are chosen together by a small cost model (times in microseconds, fitted to measurements
-    // on B200): a CTA takes 0.75 us per k-block with one 128-token block and 0.95 us with two (twice the tokens), 5 us
-    // around its loop, and a split CTA another 4 + 6 us per token block for writing, awaiting and adding f32 partial
-    // tiles.  Candidates per tile shape: whole tiles only; whole tiles plus a split last wave; every tile split
-    // 2..16 ways (at least four k-blocks per split, partial tiles within 128 MB of scratch).
-    const int nkb_all = l->k / BK;
-    struct Choice {
-        int mt, n_whole, ks;
-        double cost;
-    };
-    Choice best{1, 0, 1, 1e30};
-    for (int mtc = 1; mtc <= 2; ++mtc) {
-        if ((tune_gemm_mt == 1 || tune_gemm_mt == 2) && mtc != tune_gemm_mt) {
-            continue;
-        }
-        const int m_tiles = (t + BM * mtc - 1) / (BM * mtc);
-        // a second, empty token block is neither fetched nor multiplied: its k-blocks cost what one block costs
-        const bool half_empty = mtc == 2 && t <= BM;
-        const double per_kb = (mtc == 2 && !half_empty) ? 0.95 : 0.75;
-        const long long tiles = (long long)m_tiles * a.n_tiles;
-        const double tile_bytes = (double)BM * mtc * BN * 4.0;
-        auto cta_cost = [&](int nk, bool split) { return nk * per_kb + 5.0 + (split ? 4.0 + 6.0 * mtc : 0.0); };
-        auto consider = [&](long long n_whole, int ks) {
-            const long long split_tiles = tiles - n_whole;
-            if (ks > 1 && (split_tiles > 4096 || split_tiles * ks * tile_bytes > 128.0 * (1 << 20))) {
-                return;
-            }
-            const int nk_split = (nkb_all + ks - 1) / ks;
-            double c = (double)((n_whole + sm_count - 1) / sm_count) * cta_cost(nkb_all, false);
-            if (split_tiles > 0) {
-                c += (double)((split_tiles * ks + sm_count - 1) / sm_count) * cta_cost(nk_split, ks > 1);
-            }
-            if (c < best.cost) {
-                best = Choice{mtc, (int)n_whole, ks, c};
-            }
-        };
-        if (tune_gemm_ksplit > 0) {
-            consider(0, std::min(tune_gemm_ksplit, std::max(1, nkb_all)));
-            continue;
-        }
-        consider(tiles, 1);
-        if (tune_gemm_ksplit < 0) {
-            continue;
-        }
-        const long long rem = tiles % sm_count;
-        if (rem > 0 && tiles > sm_count) {
-            for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
-                consider(tiles - rem, ks);
-            }
-        }
-        for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
-            consider(0, ks);
-        }
-    }
+    a.n_tiles = n_tiles;
     const int mt = best.mt;
     a.m_tiles = (t + BM * mt - 1) / (BM * mt);
     a.nrb_w = l->n / TILE_ROWS;

@@ -9,11 +9,17 @@
 // registers and stores it to TMEM (tcgen05.st.16x256b: the T64 layout keeps a lane's nibbles in exactly that register
 // order), where tcgen05.mma reads it as its A operand; the tokens are the shared-memory operand.
 //
-//   warp 0      producer: raw int4 of the CTA's rows (one bulk copy per 64-channel k-block, deep ring: this is what HBM
-//               latency is hidden with) and the token tile of the same k-block (TMA, 128B swizzle, shallow ring: L2)
-//   warp 1      one lane issues MT x 4 tcgen05.mma (M128, N tokens, K16) per k-block; commits hand the TMEM stage and
-//               the token stage back
-//   warps 2-17  raw -> registers -> TMEM, then the epilogue
+//   warp 0      tokens: both k-blocks of a 128-channel stage as one TMA box (128B swizzle, shallow ring: L2)
+//   warp 1      issues 8 x tcgen05.mma (M128, N tokens, K16) per stage; commits hand the TMEM stage and the token stage back
+//   warps 2-9   raw -> registers -> TMEM, one 16-row block each, then the epilogue
+//   warp 10     weights: raw int4 of the CTA's rows (one bulk copy per k-block, deep ring: this hides the HBM latency)
+//
+// What bounds it: below about 64 tokens neither HBM nor the tensor pipe but the serial chain of a role per stage (wait,
+// issue, hand over; 34816 x 5120, 16 tokens, two CTAs per SM: 0.69 us per stage of 2 x 8 KB).  So the roles that issue
+// TMA, bulk copies and MMAs each have a warp of their own that stays converged with one elected lane (uniform registers
+// feed these instructions: 36 -> 34 us) and a stage is one token box and two weight copies (34 -> 30.6 us).  The expansion
+// itself, the TMEM stores, loads from HBM and the MMAs each cost under 15 % when taken out alone.  A second set of eight
+// expanding warps (33 us) and 256 rows per CTA (33.5 us) were slower.
 //
 // The K splits of a tile form a thread-block cluster and sum their f32 accumulators through distributed shared memory in
 // split order (no global scratch, no tickets).
@@ -38,9 +44,10 @@ namespace {
 constexpr int TS_MROWS = 128;                   // weight rows per MMA
 constexpr int BK = TILE_K;
 constexpr int SK = 2 * BK;                      // channels per stage: two k-blocks, one 128-channel scale group
-constexpr int RAW_PER_MT = TS_MROWS * SK / 2;   // 8 KB per stage and 128-row block
+constexpr int RAW_BYTES = TS_MROWS * SK / 2;    // 8 KB per stage
 constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
-__host__ __device__ constexpr int ts_threads(int mt) { return (2 + 8 * mt) * 32; }
+constexpr int DQ_WARPS = TS_MROWS / TILE_ROWS;  // a warp per 16-row block
+constexpr int TS_THREADS = (3 + DQ_WARPS) * 32;
 constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
 // Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
 // waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
@@ -64,15 +71,6 @@ struct TsArgs {
     int pdl;
     float out_mul;
     int* status;
-    // grouped (MoE) mode: token tiles come from a device table, one expert's weights per tile
-    int grouped;
-    const int* tile_expert;
-    const int* tile_row0;
-    const int* tile_rows;
-    const int* num_tiles;
-    int expert0;
-    const float* row_w;
-    int glu;
 };
 
 __device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
@@ -108,21 +106,17 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
     return v;
 }
 
-// MT = 128-row weight blocks per CTA (the token tile is shared by them).
-template <int GROUP, int MT>
-__global__ void __launch_bounds__(ts_threads(MT), MT == 1 ? 2 : 1)
+template <int GROUP>
+__global__ void __launch_bounds__(TS_THREADS, 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
 
-    constexpr int DQ_WARPS = 8 * MT;
-    constexpr int THREADS = ts_threads(MT);
     constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be warp-uniform
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
-    constexpr uint32_t RAW_BYTES = RAW_PER_MT * MT;
     const int NR = a.raw_stages, NX = a.x_stages, NA = a.a_stages;
     const int N = a.tok;
     const uint32_t x_half = (uint32_t)N * (BK * 2);                  // one k-block of the token tile
@@ -140,23 +134,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     // ---- this CTA's tile ----
     const int tile = (int)blockIdx.x, ks = a.ksplit, split = (int)blockIdx.y;
     const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
-    const int n0 = ntile * (TS_MROWS * MT);
-    int m0, rows_valid, rb0 = n0 / TILE_ROWS;
-    if (a.grouped) {
-        if (a.pdl) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");       // the segment table is the previous kernels' output
-        }
-        if (mtile >= *a.num_tiles) {
-            return;
-        }
-        m0 = a.tile_row0[mtile];
-        rows_valid = a.tile_rows[mtile];
-        rb0 += (a.tile_expert[mtile] - a.expert0) * (a.n / TILE_ROWS);
-    } else {
-        m0 = mtile * N;
-        rows_valid = min(N, a.m - m0);
-    }
-    const int nrbv = min(TS_MROWS * MT, a.n - n0) / TILE_ROWS;       // valid 16-row blocks
+    const int n0 = ntile * TS_MROWS;
+    const int m0 = mtile * N, rb0 = n0 / TILE_ROWS;
+    const int rows_valid = min(N, a.m - m0);
+    const int nrbv = min(TS_MROWS, a.n - n0) / TILE_ROWS;       // valid 16-row blocks
     const uint32_t kb_bytes = (uint32_t)nrbv * (TILE_WORDS * 4);
     // K range of this split in stages; the last stage of the matrix may hold one k-block (32-channel groups)
     const int nkb_all = a.k / BK, st_all = (nkb_all + 1) / 2;
@@ -208,109 +189,122 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         // then wait for this kernel
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     }
-    const uint32_t tmem = s_tmem_base;
-    const uint32_t tmem_a = tmem + (uint32_t)(MT * N);               // A ring: [stage][MT][64 columns]
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem_base, 0);
+    const uint32_t tmem_a = tmem + (uint32_t)N;                      // A ring: [stage][64 columns]
     volatile int* abort_flag = &s_abort;
 
     bool ok = true;
     if (warp == 0) {
-        // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            if (a.pdl) {
-                asm volatile("griddepcontrol.wait;" ::: "memory");
+        // ------------------------------------------------------------------ tokens
+        if (a.pdl) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        const bool leader = elect_one();
+        int sx = 0, px = 1;
+        for (int it = 0; it < nst; ++it) {
+            if (it >= NX && !__all_sync(0xffffffffu, mbar_wait(x_free(sx), px, abort_flag, a.status, (31 << 16) | it))) {
+                break;
             }
-            int sx = 0, px = 1, sr = 0, pr = 0;                      // slot / parity of token stage it, of raw stage it + NR
-            for (int it = 0; it < nst; ++it) {
-                if (it >= NX && !mbar_wait(x_free(sx), px, abort_flag, a.status, (31 << 16) | it)) {
-                    break;
-                }
-                const int kbs = stage_kbs(it);
-                mbar_expect_tx(x_full(sx), kbs * x_half);
-                for (int h = 0; h < kbs; ++h) {
-                    tma_load_2d(x_addr(sx) + h * x_half, &tmap_x, (2 * (st0 + it) + h) * BK, m0, x_full(sx));
-                }
-                if (++sx == NX) {
-                    sx = 0;
-                    px ^= 1;
-                }
-                if (it + NR < nst) {
-                    if (!mbar_wait(raw_free(sr), pr, abort_flag, a.status, (32 << 16) | it)) {
-                        break;
-                    }
-                    issue_raw(it + NR, sr);
-                    if (++sr == NR) {
-                        sr = 0;
-                        pr ^= 1;
-                    }
-                }
+            if (leader) {
+                // both k-blocks in one box (the second one of the last stage may lie outside: zeros)
+                mbar_expect_tx(x_full(sx), 2 * x_half);
+                tma_load_3d(x_addr(sx), &tmap_x, 0, m0, 2 * (st0 + it), x_full(sx));
+            }
+            __syncwarp();
+            if (++sx == NX) {
+                sx = 0;
+                px ^= 1;
             }
         }
-        __syncwarp();
+    } else if (warp == 2 + DQ_WARPS) {
+        // ------------------------------------------------------------------ weights
+        const bool leader = elect_one();
+        int sr = 0, pr = 0;
+        for (int it = NR; it < nst; ++it) {
+            if (!__all_sync(0xffffffffu, mbar_wait(raw_free(sr), pr, abort_flag, a.status, (32 << 16) | it))) {
+                break;
+            }
+            if (leader) {
+                issue_raw(it, sr);
+            }
+            __syncwarp();
+            if (++sr == NR) {
+                sr = 0;
+                pr ^= 1;
+            }
+        }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
-            int sx = 0, px = 0, sa = 0, pa = 0;
-            for (int it = 0; it < nst; ++it) {
-                if (!mbar_wait(x_full(sx), px, abort_flag, a.status, (33 << 16) | it) ||
-                    !mbar_wait(a_ready(sa), pa, abort_flag, a.status, (34 << 16) | it)) {
-                    ok = false;
-                    break;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
+        const bool leader = elect_one();
+        int sx = 0, px = 0, sa = 0, pa = 0;
+        for (int it = 0; it < nst; ++it) {
+            const bool in = mbar_wait(x_full(sx), px, abort_flag, a.status, (33 << 16) | it) &&
+                            mbar_wait(a_ready(sa), pa, abort_flag, a.status, (34 << 16) | it);
+            if (!__all_sync(0xffffffffu, in)) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t db = umma_desc(x_addr(sx));
+            const uint64_t db1 = db + (x_half >> 4);
+            const uint32_t ta = tmem_a + (uint32_t)(sa * A_COLS);
+            const bool two = stage_kbs(it) == 2;
+            if (leader) {
+#pragma unroll
+                for (int j = 0; j < BK / 16; ++j) {
+                    umma_ts_f16(tmem, ta + j * 8, db + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
                 }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int kbs = stage_kbs(it);
-                for (int h = 0; h < kbs; ++h) {
-                    const uint64_t db = umma_desc(x_addr(sx) + h * x_half);
+                if (two) {
 #pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        const uint32_t ta = tmem_a + (uint32_t)((sa * MT + mt) * A_COLS + h * (BK / 2));
-#pragma unroll
-                        for (int j = 0; j < BK / 16; ++j) {
-                            umma_ts_f16(tmem + (uint32_t)(mt * N), ta + j * 8, db + 2 * j, idesc, (it > 0 || h > 0 || j > 0) ? 1u : 0u);
-                        }
+                    for (int j = 0; j < BK / 16; ++j) {
+                        umma_ts_f16(tmem, ta + BK / 2 + j * 8, db1 + 2 * j, idesc, 1u);
                     }
                 }
                 umma_commit(a_free(sa));
                 umma_commit(x_free(sx));
-                if (++sx == NX) {
-                    sx = 0;
-                    px ^= 1;
-                }
-                if (++sa == NA) {
-                    sa = 0;
-                    pa ^= 1;
-                }
             }
-            if (ok) {
-                umma_commit(accum_bar);
+            __syncwarp();
+            if (++sx == NX) {
+                sx = 0;
+                px ^= 1;
             }
+            if (++sa == NA) {
+                sa = 0;
+                pa ^= 1;
+            }
+        }
+        if (ok && leader) {
+            umma_commit(accum_bar);
         }
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM
-        // One 16-row block per warp.  A warp may touch the TMEM lanes 32 * (warp % 4) .. +31 = two row blocks of each
-        // 128-row block.
-        const int quad = warp & 3, sub = (warp - 2) >> 2;
-        const int half = sub & 1, mt = sub >> 1;
-        const int rb = mt * (TS_MROWS / TILE_ROWS) + quad * 2 + half;
+        // One 16-row block per warp; a warp may touch the TMEM lanes 32 * (warp % 4) .. +31 = two row blocks.
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const int rb = quad * 2 + half;
         const bool live = rb < nrbv;
         const int rbl = live ? rb : 0;
         const int ng = a.k / GROUP;
-        // scale words (rows g, g + 8) of this row block, two stages ahead of their use
-        const uint32_t* sp = a.st + ((size_t)(rb0 + rbl) * ng + (size_t)st0 * GPS) * 8 + (lane >> 2);
-        int sleft = ng - st0 * GPS;                                  // groups left in the row block
-        auto load_scales = [&](uint32_t (&sc)[GPS]) {
-#pragma unroll
-            for (int i = 0; i < GPS; ++i) {
-                sc[i] = i < sleft ? __ldg(sp + i * 8) : 0u;
-            }
-            sp += GPS * 8;
-            sleft -= GPS;
+        // Scale words (rows g, g + 8) of this row block: one coalesced 128-byte load brings four groups (lane 8i + g: group
+        // i), handed out by shuffles.  SCQ loads are in flight, so that a word is requested SCQ stages (32-channel groups)
+        // or 4 * SCQ stages before its use.
+        constexpr int SCQ = 4;
+        const uint32_t* sp = a.st + ((size_t)(rb0 + rbl) * ng + (size_t)st0 * GPS) * 8 + lane;
+        int sleft = (ng - st0 * GPS) * 8 - lane;                     // words left in the row block
+        auto load_scales = [&]() {
+            const uint32_t v = sleft > 0 ? __ldg(sp) : 0u;
+            sp += 32;
+            sleft -= 32;
+            return v;
         };
-        uint32_t sc0[GPS], sc1[GPS];
-        load_scales(sc0);
-        load_scales(sc1);
-        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16) + (uint32_t)(mt * A_COLS);
+        uint32_t scq[SCQ];
+#pragma unroll
+        for (int i = 0; i < SCQ; ++i) {
+            scq[i] = load_scales();
+        }
+        uint32_t sc_cur = 0;
+        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
         const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
         auto expand = [&](const uint4& raw, const uint32_t s_a, const uint32_t s_b, uint32_t (&v)[16]) {
             const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -336,13 +330,19 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
             const uint32_t ra = r_ld + (uint32_t)sr * RAW_BYTES;
             const uint4 raw0 = lds128(ra);
             const uint4 raw1 = lds128(ra + RAW_BYTES / 2);           // stale bytes when the stage holds one k-block
+            if (((it * GPS) & 3) == 0) {
+                sc_cur = scq[0];
+#pragma unroll
+                for (int i = 0; i + 1 < SCQ; ++i) {
+                    scq[i] = scq[i + 1];
+                }
+                scq[SCQ - 1] = load_scales();
+            }
             uint32_t sc[GPS];
 #pragma unroll
             for (int i = 0; i < GPS; ++i) {
-                sc[i] = sc0[i];
-                sc0[i] = sc1[i];
+                sc[i] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + i) & 3) * 8 + (lane >> 2));
             }
-            load_scales(sc1);
             uint32_t v[16];
             expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
             if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
@@ -350,7 +350,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t td = t_st + (uint32_t)(sa * MT * A_COLS);
+            const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
             tmem_st_16x256b_x4(td, v);
             expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
             __syncwarp();
@@ -376,40 +376,28 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         ok = __all_sync(0xffffffffu, ok);
         ok = ok && mbar_wait(accum_bar, 0, abort_flag, a.status, (37 << 16));
         ok = __all_sync(0xffffffffu, ok);
-        if (a.pdl && !a.grouped) {
+        if (a.pdl) {
             asm volatile("griddepcontrol.wait;" ::: "memory");       // outputs may be what the previous kernel still reads
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
 
     // ---------------------------------------------------------------------- epilogue
-    const bool dq_warp = warp >= 2;
+    const bool dq_warp = warp >= 2 && warp < 2 + DQ_WARPS;
     const int quad = warp & 3, sub = (warp - 2) >> 2;
-    const int emt = sub >> 1;                                        // 128-row block of this warp's accumulator lanes
-    constexpr int EW = 2;                                            // warps that share a (row block, quadrant)
-    const int ei = sub & 1;
-    const int lrow = emt * TS_MROWS + quad * 32 + lane;              // weight row within the tile
+    constexpr int EW = DQ_WARPS / 4;                                 // warps that share a TMEM lane quadrant
+    const int lrow = quad * 32 + lane;                               // weight row within the tile
     if (ks == 1) {
         if (dq_warp && ok) {
             const bool row_ok = n0 + lrow < a.n;
-            for (int c0 = ei * 16; c0 < rows_valid; c0 += EW * 16) {
+            for (int c0 = sub * 16; c0 < rows_valid; c0 += EW * 16) {
                 uint32_t v[16];
-                tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(emt * N + c0), v);
+                tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
                     const int tok = c0 + i;
-                    float f = __uint_as_float(v[i]) * a.out_mul;
-                    if (a.glu) {
-                        // lanes 0-15 hold the gate sums, lanes 16-31 the up sums of the same 16 outputs
-                        const float up = __shfl_down_sync(0xffffffffu, f, 16);
-                        if (tok < rows_valid && lane < 16 && row_ok) {
-                            reinterpret_cast<__half*>(a.out)[(size_t)(m0 + tok) * (a.n / 2) + (n0 + emt * TS_MROWS + quad * 32) / 2 + lane] =
-                                silu_mul_f16(f, up);
-                        }
-                    } else if (tok < rows_valid && row_ok) {
-                        if (a.row_w != nullptr) {
-                            f = mul_row_w(f, a.row_w[m0 + tok]);
-                        }
+                    const float f = __uint_as_float(v[i]) * a.out_mul;
+                    if (tok < rows_valid && row_ok) {
                         const size_t o = (size_t)(m0 + tok) * a.n + n0 + lrow;
                         if (a.out_f16) {
                             reinterpret_cast<__half*>(a.out)[o] = __float2half_rn(f);
@@ -423,13 +411,13 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     } else {
         // the splits' accumulators meet in distributed shared memory, RED_TOK tokens at a time: [token][row] f32 over the
         // (idle) rings; every CTA of the cluster adds an equal share of the elements over all splits, in split order
-        constexpr int ROWS = TS_MROWS * MT;
+        constexpr int ROWS = TS_MROWS;
         for (int cb = 0; cb < rows_valid; cb += RED_TOK) {
             const int nt = min(RED_TOK, rows_valid - cb);
             if (dq_warp && ok) {
-                for (int c0 = ei * 16; c0 < nt; c0 += EW * 16) {
+                for (int c0 = sub * 16; c0 < nt; c0 += EW * 16) {
                     uint32_t v[16];
-                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(emt * N + cb + c0), v);
+                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(cb + c0), v);
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         *reinterpret_cast<float*>(base_ptr + ((c0 + i) * ROWS + lrow) * 4) = __uint_as_float(v[i]);
@@ -440,7 +428,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
             const int nr4 = min(ROWS, a.n - n0) / 4;
             const int total = nt * nr4;
             const int e0 = (int)((long long)total * split / ks), e1 = (int)((long long)total * (split + 1) / ks);
-            for (int e = e0 + (int)threadIdx.x; e < e1; e += THREADS) {
+            for (int e = e0 + (int)threadIdx.x; e < e1; e += TS_THREADS) {
                 const int tok = e / nr4, r = (e - tok * nr4) * 4;
                 float4 pv[8];
 #pragma unroll
@@ -483,72 +471,136 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
 }  // namespace
 
 
-static size_t ts_smem(int mt, int tok, int nr, int nx, int na, int* off_x, int* off_bars) {
-    size_t off = (size_t)nr * RAW_PER_MT * mt;                      // multiples of 1024
+static size_t ts_smem(int tok, int nr, int nx, int na, int* off_x, int* off_bars) {
+    size_t off = (size_t)nr * RAW_BYTES;                      // multiples of 1024
     *off_x = (int)off;
     off += (size_t)nx * tok * SK * 2;
-    const size_t red = (size_t)std::min(RED_TOK, tok) * TS_MROWS * mt * 4;   // the cluster's sum reuses the rings
+    const size_t red = (size_t)std::min(RED_TOK, tok) * TS_MROWS * 4;   // the cluster's sum reuses the rings
     off = std::max(off, red);
     *off_bars = (int)off;
     return off + (size_t)(2 * nr + 2 * nx + 2 * na + 1) * 8 + 1024;
 }
 
 cudaError_t gemm_ts_init_device() {
-    cudaError_t e = cudaSuccess;
-#define W4_SET(G, MTV) \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_ts_kernel<G, MTV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
-    W4_SET(128, 1)
-    W4_SET(128, 2)
-    W4_SET(32, 1)
-    W4_SET(32, 2)
-#undef W4_SET
+    cudaError_t e = cudaFuncSetAttribute(gemm_ts_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
+    if (e == cudaSuccess) {
+        e = cudaFuncSetAttribute(gemm_ts_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
+    }
     return e;
 }
 
-int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st) {
+// Shared memory and ring depths of a launch with tiles of `tok` tokens.
+namespace {
+struct TsPlan {
+    int tmem_cols, na, nr, nx, off_x, off_bars;
+    size_t smem;
+};
+TsPlan ts_plan(int tok) {
+    TsPlan p{};
+    // TMEM: the accumulator and as many expanded stages as fit in half of it (two CTAs per SM), else in all of it
+    p.tmem_cols = tok <= 128 ? 256 : 512;
+    p.na = std::min((p.tmem_cols - tok) / A_COLS, 4);
+    const size_t limit = p.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
+    p.nx = p.nr = 2;
+    while (p.nr < 12 && ts_smem(tok, p.nr + 1, p.nx, p.na, &p.off_x, &p.off_bars) <= limit) {
+        ++p.nr;
+        if (p.nr % 2 == 0 && p.nx < 4 && ts_smem(tok, p.nr, p.nx + 1, p.na, &p.off_x, &p.off_bars) <= limit) {
+            ++p.nx;
+        }
+    }
+    p.smem = std::max(ts_smem(tok, p.nr, p.nx, p.na, &p.off_x, &p.off_bars), p.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
+    return p;
+}
+}  // namespace
+
+// Clusters of `ks` CTAs that can be resident at once (a cluster lies within a GPC: of clusters of 7 only two thirds of the
+// SMs' room can be used), for half- and full-TMEM CTAs.
+void Dec::ts_query_clusters() {
+    for (int full = 0; full < 2; ++full) {
+        ts_clusters[full][1] = sm_count * (full ? 1 : 2);
+        for (int ks = 2; ks <= TS_MAX_SPLIT; ++ks) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(1, ks);
+            cfg.blockDim = dim3(TS_THREADS);
+            cfg.dynamicSmemBytes = full ? TS_SMEM_FULL_MAX : TS_SMEM_HALF_MAX;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = 1;
+            attr[0].val.clusterDim.y = ks;
+            attr[0].val.clusterDim.z = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            int n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128>, &cfg) != cudaSuccess) {
+                cudaGetLastError();
+                n = 0;       // then this split is not considered
+            }
+            ts_clusters[full][ks] = n;
+        }
+    }
+}
+
+// Tokens per tile and K split with the least estimated time (microseconds, fitted to measurements on B200): 3 us per launch;
+// a stage of 128 channels takes 0.54 us (16 tokens) to 0.83 us (256) when the CTA has its SM alone and 0.69 to 0.96 us
+// (128) with a second one beside it; a split CTA another 1.2 us plus 0.04 us per token for the sum over the cluster.
+TsChoice Dec::gemm_ts_choose(int n, int k, int t) const {
+    TsChoice best{0, 0, 1e30};
+    const int n_tiles = (n + TS_MROWS - 1) / TS_MROWS, stages = (k + SK - 1) / SK;
+    int last_tok = 0;
+    for (int cap : {256, 192, 128, 96, 64}) {
+        const int m_tiles = (t + cap - 1) / cap;
+        const int tok = ((t + m_tiles - 1) / m_tiles + 15) / 16 * 16;
+        if (tok == last_tok || (tune_ts_tok > 0 && cap != tune_ts_tok)) {
+            continue;
+        }
+        last_tok = tok;
+        const long long tiles = (long long)m_tiles * n_tiles;
+        const int full = tok > 128;
+        for (int ks = 1; ks <= TS_MAX_SPLIT && ks <= stages; ++ks) {
+            const int room = ts_clusters[full][ks];
+            if (room <= 0 || (tune_ts_ks > 0 && ks != std::min(tune_ts_ks, stages))) {
+                continue;
+            }
+            const double alone = 0.52 + 0.0012 * tok, paired = 0.65 + 0.0024 * tok;
+            const double around = ks > 1 ? 1.2 + 0.04 * tok : 0.01 * tok;
+            const int nst = (stages + ks - 1) / ks;
+            const long long waves = tiles / room, rest = tiles - waves * room;
+            const double pair_stage = full ? alone : paired;
+            double c = 3.0 + waves * (nst * pair_stage + around);
+            if (rest > 0) {
+                c += nst * (rest * ks <= sm_count ? alone : pair_stage) + around;
+            }
+            if (c < best.cost) {
+                best = TsChoice{tok, ks, c};
+            }
+        }
+    }
+    return best;
+}
+
+int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
     }
-    const int mt = tune_ts_mt ? tune_ts_mt : 2;
-    int tok_cap = tune_ts_tok ? tune_ts_tok : 128;
+    const TsPlan p = ts_plan(c.tok);
     TsArgs a{};
-    a.m_tiles = (t + tok_cap - 1) / tok_cap;
-    a.tok = ((t + a.m_tiles - 1) / a.m_tiles + 15) / 16 * 16;
-    a.n_tiles = (l->n + TS_MROWS * mt - 1) / (TS_MROWS * mt);
-    a.ksplit = tune_ts_ks ? tune_ts_ks : 1;
-    a.ksplit = std::min(a.ksplit, (l->k + SK - 1) / SK);
-    // TMEM: accumulators and as many expanded k-blocks as fit in half of it (two CTAs per SM), else in all of it
-    const int acc = mt * a.tok;
-    int na = (256 - acc) / (A_COLS * mt);
-    a.tmem_cols = 256;
-    if (mt == 2 || na < 2) {
-        na = (512 - acc) / (A_COLS * mt);
-        a.tmem_cols = 512;
-    }
-    if (na < 2) return fail("w4a16 gemm: na");
-    na = std::min(na, 4);
-    a.a_stages = na;
-    const size_t limit = a.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
-    int nx = 2, nr = 2;
-    while (nr < 12 && ts_smem(mt, a.tok, nr + 1, nx, na, &a.off_x, &a.off_bars) <= limit) {
-        ++nr;
-        if (nr % 2 == 0 && nx < 4 && ts_smem(mt, a.tok, nr, nx + 1, na, &a.off_x, &a.off_bars) <= limit) {
-            ++nx;
-        }
-    }
-    a.raw_stages = nr;
-    a.x_stages = nx;
-    const size_t smem = ts_smem(mt, a.tok, nr, nx, na, &a.off_x, &a.off_bars);
-    if (smem > limit) {
-        return fail("w4a16 gemm: tile of %d tokens does not fit", a.tok);
-    }
+    a.tok = c.tok;
+    a.ksplit = c.ks;
+    a.m_tiles = (t + c.tok - 1) / c.tok;
+    a.n_tiles = (l->n + TS_MROWS - 1) / TS_MROWS;
+    a.tmem_cols = p.tmem_cols;
+    a.a_stages = p.na;
+    a.raw_stages = p.nr;
+    a.x_stages = p.nx;
+    a.off_x = p.off_x;
+    a.off_bars = p.off_bars;
     CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)l->k, (cuuint64_t)t};
-    const cuuint64_t strides[1] = {(cuuint64_t)l->k * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)a.tok};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+    const cuuint64_t dims[3] = {(cuuint64_t)BK, (cuuint64_t)t, (cuuint64_t)(l->k / BK)};
+    const cuuint64_t strides[2] = {(cuuint64_t)l->k * 2, (cuuint64_t)BK * 2};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)a.tok, 2};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) {
@@ -567,8 +619,8 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cu
     a.status = gemm_status;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(a.m_tiles * a.n_tiles, a.ksplit);
-    cfg.blockDim = dim3(ts_threads(mt));
-    cfg.dynamicSmemBytes = std::max(smem, a.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
+    cfg.blockDim = dim3(TS_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     int n_attr = 0;
@@ -587,15 +639,12 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, cu
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cudaError_t e;
-    if (l->group == 128) {
-        e = mt == 2 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, 2>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, 1>, map, a);
-    } else {
-        e = mt == 2 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, 2>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, 1>, map, a);
-    }
+    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32>, map, a);
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
-    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "," + std::to_string(mt) + "> tok " + std::to_string(a.tok) + " ks " + std::to_string(a.ksplit) + " nr " + std::to_string(nr) + " nx " + std::to_string(nx) + " na " + std::to_string(na);
+    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "> " + std::to_string(c.tok) + "-token tiles" +
+                  (c.ks > 1 ? ", clusters of " + std::to_string(c.ks) : std::string());
     launches++;
     return 0;
 }

@@ -241,3 +241,30 @@ def test_last_wave_split_agrees_with_whole_tiles(dec):
     assert torch.equal(y, y2)
     assert (y - y_whole).abs().max().item() <= 1e-5 * y_whole.abs().max().item() + 1e-7
     dec.drop_lin("lw")
+
+
+# the weight-row form (TMEM operand): tiles of 16..256 tokens, ragged last row and token tiles, an odd number of k-blocks, one
+# and several scale groups per stage, every cluster size, more stages than any ring holds
+@pytest.mark.parametrize("t,k,n,group,tok,ks", [
+    (9, 64, 16, 32, 0, 1), (16, 128, 128, 128, 0, 1), (17, 192, 272, 64, 64, 1), (33, 320, 144, 32, 0, 3), (64, 1024, 512, 128, 64, 8),
+    (65, 2048, 256, 128, 64, 5), (100, 640, 1040, 32, 96, 2), (128, 4096, 272, 128, 128, 7), (129, 1024, 144, 128, 192, 4),
+    (200, 832, 400, 32, 256, 6), (256, 2048, 128, 128, 256, 2), (300, 256, 272, 128, 0, 0), (513, 1088, 160, 64, 0, 0)])
+@pytest.mark.parametrize("out_f16", [False, True])
+def test_weight_row_gemm_pow2_exact(dec, t, k, n, group, tok, ks, out_f16):
+    q, s, x, expect = pow2_case(t, k, n, group)
+    dec.upload_lin_g("tsr", q, s, n, k, group)
+    guard = torch.full((t + 16, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    for key, v in (("gemm_form", 2), ("gemm_ts_tok", tok), ("gemm_ts_ksplit", ks)):
+        dec.set_tuning(key, v)
+    try:
+        y = dec.lin_forward("tsr", x_dev(x), t, dst=guard[:t], out_f16=out_f16)
+        name = dec.last_kernel()
+        dec.sync()
+        dec.kernel_status()
+    finally:
+        for key in ("gemm_form", "gemm_ts_tok", "gemm_ts_ksplit"):
+            dec.set_tuning(key, 0)
+    assert name.startswith("gemm_ts_kernel"), name
+    want = expect.astype(np.float16) if out_f16 else expect      # sums of powers of two: exact in f32, one rounding to f16
+    assert np.array_equal(y.cpu().numpy(), want)
+    assert (guard[t:] == 7.0).all()
