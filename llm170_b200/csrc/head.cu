@@ -8,7 +8,8 @@
 //   * the quantiser runs on the device, row chunks at a time, with the reference's arithmetic (f32 absmax / 127,
 //     IEEE division, round half away from zero, clamp to +-127): the stored values are bit-identical to the host recipe;
 //     they are kept offset-binary (q + 128) so that one byte permute puts two of them into the mantissas of two f16;
-//   * a warp owns 16 whole rows at a time (no split along K, no reduction between warps): each lane streams 16 bytes
+//   * a warp owns 16 whole rows at a time while there is a block of 16 rows for every warp of the GPU; the blocks left after
+//     that are spread over all SMs, K split over the warps that would idle.  Each lane streams 16 bytes
 //     of row g and of row g+8 per 64 channels, expands them to exact f16 and feeds them as the 16-row operand of
 //     mma.sync m16n8k16; the tokens (up to 8 per pass) are the columns;
 //   * the activations are f32 in the reference.  They are staged once per CTA as TWO f16 planes, hi = f16(x) and
@@ -90,6 +91,8 @@ struct HeadArgs {
 
 __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const HeadArgs a) {
     extern __shared__ __align__(16) unsigned char hsm[];
+    constexpr int WARPS = HEAD_THREADS / 32;
+    __shared__ float4 s_part[WARPS * 32];
     const int k = a.k, tp = a.tp;
     const int xrow = k * 2 + HEAD_XPAD;                 // bytes of one token's f16 row
     unsigned char* xhi = hsm;
@@ -113,13 +116,14 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
     const unsigned char* xh_l = xhi + (size_t)(tok_live ? g : 0) * xrow + tq * 32;
     const unsigned char* xl_l = xlo + (size_t)(tok_live ? g : 0) * xrow + tq * 32;
     const int nsteps = k / 64;
-    for (int rb = blockIdx.x * (HEAD_THREADS / 32) + warp; rb < nrb; rb += gridDim.x * (HEAD_THREADS / 32)) {
+    // sums of row block rb over steps [s0, s1): .x, .y = row g, tokens 2tq, 2tq + 1;  .z, .w = row g + 8
+    auto multiply = [&](int rb, int s0, int s1) {
         const int r0 = min(rb * 16 + g, a.n - 1), r1 = min(rb * 16 + g + 8, a.n - 1);   // clamped: loads stay in range
         const uint4* p0 = reinterpret_cast<const uint4*>(a.q + (size_t)r0 * k) + tq;
         const uint4* p1 = reinterpret_cast<const uint4*>(a.q + (size_t)r1 * k) + tq;
         float ch[4] = {0.f, 0.f, 0.f, 0.f}, cl[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
-        for (int s = 0; s < nsteps; ++s) {
+        for (int s = s0; s < s1; ++s) {
             // 64 channels: this lane's 16 bytes of row g and of row g+8 (the four lanes of a row cover 64 contiguous bytes)
             const uint4 w0 = __ldg(p0 + s * 4), w1 = __ldg(p1 + s * 4);
             uint4 bh0 = make_uint4(0, 0, 0, 0), bh1 = bh0, bl0 = bh0, bl1 = bh0;
@@ -145,22 +149,65 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
                 mma16816(cl, af, xl[2 * j], xl[2 * j + 1]);
             }
         }
-        // c[0], c[1]: row g, tokens 2tq, 2tq+1;  c[2], c[3]: row g+8
+        return make_float4(ch[0] + cl[0] * (1.0f / 2048.0f), ch[1] + cl[1] * (1.0f / 2048.0f), ch[2] + cl[2] * (1.0f / 2048.0f),
+                           ch[3] + cl[3] * (1.0f / 2048.0f));
+    };
+    auto store = [&](int rb, const float4& c) {
         const int ra = rb * 16 + g, rbb = ra + 8;
         const float sa = ra < a.n ? a.scale[ra] : 0.f, sb = rbb < a.n ? a.scale[rbb] : 0.f;
+        const float ca[2] = {c.x, c.y}, cb[2] = {c.z, c.w};
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int tok = 2 * tq + c;
+        for (int i = 0; i < 2; ++i) {
+            const int tok = 2 * tq + i;
             if (tok < tp) {
                 float* o = a.out + (size_t)(a.t0 + tok) * a.n;
                 if (ra < a.n) {
-                    o[ra] = (ch[c] + cl[c] * (1.0f / 2048.0f)) * sa;
+                    o[ra] = ca[i] * sa;
                 }
                 if (rbb < a.n) {
-                    o[rbb] = (ch[2 + c] + cl[2 + c] * (1.0f / 2048.0f)) * sb;
+                    o[rbb] = cb[i] * sb;
                 }
             }
         }
+    };
+    // Whole rounds: a row block per warp.  The rest of the row blocks is dealt over all SMs and, where it leaves warps idle,
+    // each block's K over several warps of its CTA: 151936 rows are 4.01 rounds, and the fifth one cost as much as the others.
+    const int all_warps = gridDim.x * WARPS, rounds = nrb / all_warps;
+    for (int i = 0; i < rounds; ++i) {
+        const int rb = i * all_warps + blockIdx.x * WARPS + warp;
+        store(rb, multiply(rb, 0, nsteps));
+    }
+    const int rest0 = rounds * all_warps, rest = nrb - rest0;
+    if (rest == 0) {
+        return;
+    }
+    const int per_cta = (rest + (int)gridDim.x - 1) / (int)gridDim.x;            // 1..WARPS
+    int ways = WARPS;
+    while (ways * per_cta > WARPS) {
+        ways >>= 1;
+    }
+    const int sub = warp / ways, part = warp - sub * ways;
+    const int rb = rest0 + sub * (int)gridDim.x + (int)blockIdx.x;
+    const bool live = sub < per_cta && rb < nrb;
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) {
+        c = multiply(rb, nsteps * part / ways, nsteps * (part + 1) / ways);
+    }
+    if (ways > 1) {
+        s_part[threadIdx.x] = c;
+        __syncthreads();
+        if (part == 0) {
+            for (int w = 1; w < ways; ++w) {                                     // in K order
+                const float4 o = s_part[threadIdx.x + w * 32];
+                c.x += o.x;
+                c.y += o.y;
+                c.z += o.z;
+                c.w += o.w;
+            }
+        }
+    }
+    if (live && part == 0) {
+        store(rb, c);
     }
 }
 
@@ -279,7 +326,7 @@ int w4a16_head_forward(w4a16_dec* dec, const float* x32_dev, float* out_dev, int
     const size_t xrow = (size_t)d.head_k * 2 + w4::HEAD_XPAD;
     const int tp_max = (int)std::min<size_t>(w4::HEAD_TOK, ((size_t)200 * 1024) / (2 * xrow));
     const int nrb = (d.head_n + 15) / 16;
-    const int grid = std::min(d.sm_count, (nrb + w4::HEAD_THREADS / 32 - 1) / (w4::HEAD_THREADS / 32));
+    const int grid = std::min(d.sm_count, nrb);
     for (int t0 = 0; t0 < t; t0 += tp_max) {
         w4::HeadArgs a;
         a.q = d.head_q;

@@ -88,6 +88,21 @@ def test_exact_case_matches_integer_arithmetic(dec):
     assert np.array_equal(y.cpu().numpy()[0], (ints.astype(np.float64) @ x[0].astype(np.float64)).astype(np.float32))
 
 
+@pytest.mark.parametrize("n,k,t", [(16, 64, 1), (2400, 192, 3), (7001, 320, 1), (37888, 128, 1), (37904, 192, 2), (45101, 128, 8)])
+def test_row_blocks_left_after_whole_rounds(dec, n, k, t):
+    # a round is one 16-row block per warp of the GPU (37888 rows on 148 SMs); what is left is split over CTAs and along K,
+    # also into more parts than it has 64-channel steps.  Sums of these integers are exact in any order.
+    ints = ((np.arange(n * k, dtype=np.int64).reshape(n, k) * 7) % 255 - 127).astype(np.float32)
+    ints[:, 0] = 127.0
+    dec.upload_head(bf16_of(ints), n, k)
+    x = np.stack([2.0 ** ((np.arange(k) % 5) - 2 + i % 3) for i in range(t)]).astype(np.float32)
+    guard = torch.full((t + 1, n), 7.0, device="cuda", dtype=torch.float32)
+    y = dec.head_forward(torch.from_numpy(x).cuda(), t, out=guard[:t])
+    dec.sync()
+    assert np.array_equal(y.cpu().numpy(), (x.astype(np.float64) @ ints.astype(np.float64).T).astype(np.float32))
+    assert bool((guard[t:] == 7.0).all())
+
+
 def test_contract_errors():
     from llm170_b200.w4a16_dec import W4a16Dec, W4a16Error
     d = W4a16Dec(0)
