@@ -635,6 +635,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         d.tune_gemm_form = value;
         return 0;
     }
+    if (!strcmp(key, "gemm_bn")) {
+        if (value != 0 && (value < 128 || value > 256 || value % 32 != 0)) {
+            return d.fail("w4a16 set_tuning: gemm_bn=%d (a multiple of 32 from 128 to 256, or 0)", value);
+        }
+        d.tune_gemm_bn = value;
+        return 0;
+    }
     if (!strcmp(key, "gemm_ts_tok")) {
         d.tune_ts_tok = value;
         return 0;

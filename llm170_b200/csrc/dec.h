@@ -103,6 +103,7 @@ struct Dec {
     int tune_gemm_ksplit = 0;    // K splits of the GEMM: 0 = automatic (only when the tiles do not fill the SMs)
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
     int tune_gemm_form = 0;      // above the decode rows: 0 = automatic, 1 = token rows (gemm_tc.cu), 2 = weight rows (gemm_ts.cu)
+    int tune_gemm_bn = 0;        // gemm_tc.cu: weight rows per tile (128..256, a multiple of 32), 0 = automatic
     int tune_ts_tok = 0;         // gemm_ts.cu: most tokens per tile (64, 96, 128, 192, 256), 0 = automatic
     int tune_ts_ks = 0;          // gemm_ts.cu: K splits (1..8), 0 = automatic
     int ts_clusters[2][TS_MAX_SPLIT + 1] = {};   // resident clusters of 1..8 CTAs, for CTAs with half and all of the TMEM

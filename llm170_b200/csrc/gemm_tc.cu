@@ -59,6 +59,7 @@ struct GemmArgs {
     int m, n, k;
     int out_f16;
     int m_tiles, n_tiles;
+    int bn;          // weight rows per tile = MMA N: a multiple of 32 up to BN (BN when grouped)
     int nrb_w;       // 16-row blocks of the resident weight matrix (= n/16; experts stacked along n when grouped)
     // grouped (MoE) mode: m-tiles come from a device table, one expert's weights per tile
     int grouped;
@@ -118,7 +119,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     __shared__ int s_abort;
     __shared__ int s_last;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be warp-uniform
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
     // [A ring NT x MT*16K][B ring NB x 32K][raw ring NT x 8K][barriers]; A and B bases are 1024-byte aligned
@@ -148,7 +149,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
         }
         m0 = a.tile_row0[mt];
         rows_valid = a.tile_rows[mt];
-        n0 = n_tile * BN;
+        n0 = n_tile * a.bn;
         rb0 = ((a.tile_expert[mt] - a.expert0) * a.n + n0) / TILE_ROWS;
     } else {
         // groups of GROUP_M m-tiles walk the n-tiles together
@@ -159,14 +160,14 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
         const int gsz = min(GROUP_M, a.m_tiles - first_m);
         const int rem = tile - grp * per_group;
         m0 = (first_m + rem % gsz) * BMT;
-        n0 = (rem / gsz) * BN;
+        n0 = (rem / gsz) * a.bn;
         rb0 = n0 / TILE_ROWS;
         rows_valid = min(BMT, a.m - m0);
     }
     const int nkb_all = a.k / BK;
     const int kb0 = (int)((long long)nkb_all * split / ks);                 // this split's k-blocks: [kb0, kb0 + nkb)
     const int nkb = (int)((long long)nkb_all * (split + 1) / ks) - kb0;
-    const int nrbv = min(BN, a.n - n0) / TILE_ROWS;  // valid 16-row blocks in this tile
+    const int nrbv = min(a.bn, a.n - n0) / TILE_ROWS;  // valid 16-row blocks in this tile
     // 128-token blocks of this tile that hold rows: an empty second block is neither fetched nor multiplied
     const int mt_live = (MT == 2 && rows_valid <= BM) ? 1 : MT;
 
@@ -196,17 +197,19 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem_base;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem_base, 0);
     volatile int* abort_flag = &s_abort;
 
     if (warp == 0) {
         // ------------------------------------------------------------------ producer
-        if (lane == 0) {
-            for (int it = 0; it < nkb; ++it) {
-                const int s = it % NT, r = it / NT;
-                if (!mbar_wait(empty_bar(s), (r & 1) ^ 1, abort_flag, a.status, (1 << 16) | it)) {
-                    break;
-                }
+        // (both issuing roles run converged with one elected lane: elect_one)
+        const bool leader = elect_one();
+        for (int it = 0; it < nkb; ++it) {
+            const int s = it % NT, r = it / NT;
+            if (!__all_sync(0xffffffffu, mbar_wait(empty_bar(s), (r & 1) ^ 1, abort_flag, a.status, (1 << 16) | it))) {
+                break;
+            }
+            if (leader) {
                 if (stamp && it < 1000) {
                     a.dbg[it] = clock64();
                 }
@@ -221,41 +224,45 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
                 bulk_load(raw_addr(s), a.qt + ((size_t)(kb0 + it) * a.nrb_w + rb0) * TILE_WORDS,
                           nrbv * (TILE_WORDS * 4), full_bar(s));
             }
+            __syncwarp();
         }
-        __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
-            bool ok = true;
-            for (int it = 0; it < nkb && ok; ++it) {
-                const int s = it % NT, r = it / NT, sb = it % NB, rb_ = it / NB;
-                ok = mbar_wait(full_bar(s), r & 1, abort_flag, a.status, (2 << 16) | it) &&
-                     mbar_wait(bready_bar(sb), rb_ & 1, abort_flag, a.status, (3 << 16) | it);
-                if (!ok) {
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(a.bn >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+        const bool leader = elect_one();
+        bool ok = true;
+        for (int it = 0; it < nkb; ++it) {
+            const int s = it % NT, r = it / NT, sb = it % NB, rb_ = it / NB;
+            const bool in = mbar_wait(full_bar(s), r & 1, abort_flag, a.status, (2 << 16) | it) &&
+                            mbar_wait(bready_bar(sb), rb_ & 1, abort_flag, a.status, (3 << 16) | it);
+            ok = __all_sync(0xffffffffu, in);
+            if (!ok) {
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t db = umma_desc(b_addr(sb));
+            const uint64_t da0 = umma_desc(a_addr(s));
+            if (leader) {
                 if (stamp && it < 1000) {
                     a.dbg[3000 + it] = clock64();
                 }
-                const uint64_t db = umma_desc(b_addr(sb));
 #pragma unroll
                 for (int mt = 0; mt < MT; ++mt) {
                     if (mt < mt_live) {
-                        const uint64_t da = umma_desc(a_addr(s) + mt * A_BYTES);
+                        const uint64_t da = da0 + (uint64_t)(mt * A_BYTES >> 4);
 #pragma unroll
                         for (int j = 0; j < BK / 16; ++j) {
-                            umma_f16(tmem + mt * 256, da + 2 * j, db + 2 * j, IDESC, (it > 0 || j > 0) ? 1u : 0u);
+                            umma_f16(tmem + mt * 256, da + 2 * j, db + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
                         }
                     }
                 }
                 umma_commit(empty_bar(s));
                 umma_commit(bfree_bar(sb));
             }
-            if (ok) {
-                umma_commit(accum_bar);
-            }
+            __syncwarp();
+        }
+        if (ok && leader) {
+            umma_commit(accum_bar);
         }
         __syncwarp();
     } else {
@@ -339,7 +346,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int quad = warp & 3;
-                const int ncols = min(BN, a.n - n0);
+                const int ncols = min(a.bn, a.n - n0);
                 int n_staged = 0;
                 for (int mc = 0; mc < mt_live * (BN / 32); ++mc) {
                     const int mt = mc / (BN / 32), c0 = (mc % (BN / 32)) * 32;
@@ -553,7 +560,7 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
         }
         __syncthreads();
         if (s_last) {
-            const int ncols = min(BN, a.n - n0), c4n = ncols / 4;
+            const int ncols = min(a.bn, a.n - n0), c4n = ncols / 4;
             const float* base_p = a.part + (size_t)sidx * ks * (size_t)(BMT * BN);
             const int r_begin = (int)((long long)rows_valid * split / ks), r_end = (int)((long long)rows_valid * (split + 1) / ks);
             for (int idx = threadIdx.x; idx < (r_end - r_begin) * c4n; idx += NUM_THREADS) {
@@ -639,79 +646,86 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     if (((uintptr_t)x & 15) != 0 || ((uintptr_t)dst & 15) != 0) {
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
     }
-    const int n_tiles = (l->n + BN - 1) / BN;
-    // Tile shape and K split are chosen together by a small cost model (times in microseconds, fitted to measurements
-    // on B200): a CTA takes 0.75 us per k-block with one 128-token block and 0.95 us with two (twice the tokens), 5 us
-    // around its loop, and a split CTA another 4 + 6 us per token block for writing, awaiting and adding f32 partial
-    // tiles.  Candidates per tile shape: whole tiles only; whole tiles plus a split last wave; every tile split
-    // 2..16 ways (at least four k-blocks per split, partial tiles within 128 MB of scratch).
+    // Tile shape and K split are chosen together by a small cost model (microseconds, fitted to measurements on B200).  A
+    // k-block takes 0.30 + 0.00105 bn with one 128-token block; with two, 0.295 + 0.00133 bn while at most 100 CTAs run and
+    // 0.163 + 0.0024 bn (0.78 at 256) when the GPU is full; 5 us around a wave; a split tile another 3.5 us and, at 256 rows,
+    // 0.065 us per token for writing, awaiting and adding f32 partial tiles.  Candidates per tile shape: whole tiles only;
+    // whole tiles plus a split last wave; every tile split 2..16 ways (at least four k-blocks per split, partial tiles within
+    // 128 MB of scratch).  Tiles narrower than 256 rows multiply less per expanded k-block and are taken where they fill SMs
+    // that 256 leaves idle, by a tenth at least (1024 tokens, 5120 x 17408: 128 tiles of 160 rows 149 us, 80 of 256 178 us;
+    // 5120 x 6144: 57 against 67 us).
     const int nkb_all = l->k / BK;
     struct Choice {
-        int mt, n_whole, ks;
+        int mt, bn, n_whole, ks;
         double cost;
     };
-    Choice best{1, 0, 1, 1e30};
-    for (int mtc = 1; mtc <= 2; ++mtc) {
-        if ((tune_gemm_mt == 1 || tune_gemm_mt == 2) && mtc != tune_gemm_mt) {
+    Choice best{1, BN, 0, 1, 1e30};
+    for (int bnc : {256, 224, 192, 160, 128}) {
+        if (tune_gemm_bn > 0 ? bnc != tune_gemm_bn : (bnc != BN && tune_gemm_ksplit > 0)) {
             continue;
         }
-        const int m_tiles = (t + BM * mtc - 1) / (BM * mtc);
-        // a second, empty token block is neither fetched nor multiplied: its k-blocks cost what one block costs
-        const bool half_empty = mtc == 2 && t <= BM;
-        const double per_kb = (mtc == 2 && !half_empty) ? 0.95 : 0.75;
-        const long long tiles = (long long)m_tiles * n_tiles;
-        const double tile_bytes = (double)BM * mtc * BN * 4.0;
-        auto cta_cost = [&](int nk, bool split) { return nk * per_kb + 5.0 + (split ? 4.0 + 6.0 * mtc : 0.0); };
-        auto consider = [&](long long n_whole, int ks) {
-            const long long split_tiles = tiles - n_whole;
-            if (ks > 1 && (split_tiles > 4096 || split_tiles * ks * tile_bytes > 128.0 * (1 << 20))) {
-                return;
+        const int n_tiles = (l->n + bnc - 1) / bnc;
+        const double bar = bnc == BN || tune_gemm_bn > 0 ? 1.0 : 1.0 / 0.9;     // what a narrow tile's estimate is weighed with
+        for (int mtc = 1; mtc <= 2; ++mtc) {
+            if ((tune_gemm_mt == 1 || tune_gemm_mt == 2) && mtc != tune_gemm_mt) {
+                continue;
             }
-            const int nk_split = (nkb_all + ks - 1) / ks;
-            double c = (double)((n_whole + sm_count - 1) / sm_count) * cta_cost(nkb_all, false);
-            if (split_tiles > 0) {
-                c += (double)((split_tiles * ks + sm_count - 1) / sm_count) * cta_cost(nk_split, ks > 1);
+            const int m_tiles = (t + BM * mtc - 1) / (BM * mtc);
+            // a second, empty token block is neither fetched nor multiplied: its k-blocks cost what one block costs
+            const bool two = mtc == 2 && t > BM;
+            const long long tiles = (long long)m_tiles * n_tiles;
+            const double tile_bytes = (double)BM * mtc * BN * 4.0;
+            auto ctas_cost = [&](long long ctas, int nk, bool split) {
+                const long long waves = ctas / sm_count, rest = ctas - waves * sm_count;
+                const double around = 5.0 + (split ? 3.5 + 0.065 * std::min(t, BM * mtc) * bnc / BN : 0.0);
+                const double full = two ? 0.163 + 0.0024 * bnc : 0.30 + 0.00105 * bnc;
+                const double light = two ? 0.295 + 0.00133 * bnc : full;
+                return waves * (nk * full + around) + (rest > 0 ? nk * (rest <= 100 ? light : full) + around : 0.0);
+            };
+            auto consider = [&](long long n_whole, int ks) {
+                const long long split_tiles = tiles - n_whole;
+                if (ks > 1 && (split_tiles > 4096 || split_tiles * ks * tile_bytes > 128.0 * (1 << 20))) {
+                    return;
+                }
+                double c = ctas_cost(n_whole, nkb_all, false);
+                if (split_tiles > 0) {
+                    c += ctas_cost(split_tiles * ks, (nkb_all + ks - 1) / ks, ks > 1);
+                }
+                if (c * bar < best.cost) {
+                    best = Choice{mtc, bnc, (int)n_whole, ks, c * bar};
+                }
+            };
+            if (tune_gemm_ksplit > 0) {
+                consider(0, std::min(tune_gemm_ksplit, std::max(1, nkb_all)));
+                continue;
             }
-            if (c < best.cost) {
-                best = Choice{mtc, (int)n_whole, ks, c};
+            consider(tiles, 1);
+            if (tune_gemm_ksplit < 0) {
+                continue;
             }
-        };
-        if (tune_gemm_ksplit > 0) {
-            consider(0, std::min(tune_gemm_ksplit, std::max(1, nkb_all)));
-            continue;
-        }
-        consider(tiles, 1);
-        if (tune_gemm_ksplit < 0) {
-            continue;
-        }
-        const long long rem = tiles % sm_count;
-        if (rem > 0 && tiles > sm_count) {
+            const long long rem = tiles % sm_count;
+            if (rem > 0 && tiles > sm_count) {
+                for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
+                    consider(tiles - rem, ks);
+                }
+            }
             for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
-                consider(tiles - rem, ks);
+                consider(0, ks);
             }
-        }
-        for (int ks = 2; ks <= 16 && nkb_all / ks >= 4; ++ks) {
-            consider(0, ks);
         }
     }
-    // The weight-row form (gemm_ts.cu) takes the calls that it finishes sooner: up to about 128 tokens all of them (its MMA
-    // tile is as wide as the batch, 30.6 against 52 us for 16 x 34816 x 5120), above that those whose 256-token tiles leave
-    // SMs idle (320 x 5120 x 6144: 24.5 against 48 us); full waves of 256 x 256 tiles run a third faster here (1024 x 34816
-    // x 5120: 274 against 355 us).  This form's time for the comparison: per k-block 0.60 us with one token block and 0.78
-    // with two, 5 us around a wave, 3.5 us and 0.065 us per row for a split tile.
-    if (tune_gemm_form != 1 && (tune_gemm_form == 2 || (tune_gemm_ksplit == 0 && tune_gemm_mt == 0))) {
-        const long long tiles = (long long)((t + BM * best.mt - 1) / (BM * best.mt)) * n_tiles;
-        const double per_kb = best.mt == 2 && t > BM ? 0.78 : 0.60;
-        const int nk_split = (nkb_all + best.ks - 1) / best.ks;
-        const long long whole = best.ks > 1 ? best.n_whole : tiles, split_ctas = (tiles - whole) * best.ks;
-        const double tc_cost = (double)((whole + sm_count - 1) / sm_count) * (nkb_all * per_kb + 5.0) +
-                               (double)((split_ctas + sm_count - 1) / sm_count) *
-                                   (nk_split * per_kb + 8.5 + 0.065 * std::min(t, BM * best.mt));
+    // The weight-row form (gemm_ts.cu) takes the calls that it finishes sooner: up to about 128 tokens nearly all of them (its
+    // MMA tile is as wide as the batch: 27 x 34816 x 5120 in 31 us against 52), above that those whose tiles here leave SMs
+    // idle (512 x 7168 x 5120: 32 against 59 us); in full waves the 256 x 256 tiles are up to a fifth faster (256 x 34816 x
+    // 5120: 67 against 72 us).  At a tie, within a tenth, this form; above 1024 tokens within a fifth: over several full
+    // waves the clock sinks and the two measured alike (4096 x 5120 x 6144: 196..237 against 201 us).
+    if (tune_gemm_form == 2 || (tune_gemm_form == 0 && tune_gemm_ksplit == 0 && tune_gemm_mt == 0 && tune_gemm_bn == 0)) {
         const TsChoice c = gemm_ts_choose(l->n, l->k, t);
-        if (tune_gemm_form == 2 || c.cost < 0.9 * tc_cost) {   // at a tie whole 256 x 256 tiles vary less with the clock
+        if (tune_gemm_form == 2 || c.cost < (t <= 1024 ? 0.9 : 0.8) * best.cost) {
             return gemm_ts(l, x, dst, t, out_kind, c, st);
         }
     }
+    const int bn = best.bn, n_tiles = (l->n + bn - 1) / bn;
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
@@ -751,6 +765,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     a.k = l->k;
     a.out_f16 = out16;
     a.n_tiles = n_tiles;
+    a.bn = bn;
     const int mt = best.mt;
     a.m_tiles = (t + BM * mt - 1) / (BM * mt);
     a.nrb_w = l->n / TILE_ROWS;
@@ -834,6 +849,7 @@ int Dec::gemm_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int 
     a.out_f16 = 1;
     a.m_tiles = max_tiles;
     a.n_tiles = (n_per_expert + BN - 1) / BN;
+    a.bn = BN;
     a.nrb_w = l->n / TILE_ROWS;
     a.grouped = 1;
     a.tile_expert = b.tile_expert;

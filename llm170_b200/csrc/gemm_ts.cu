@@ -52,7 +52,7 @@ constexpr int RED_TOK = 64;                     // tokens per round of the clust
 // Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
 // waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
 // Half the TMEM: two CTAs per SM, never three; all of it: alone, also beside a CTA of the other kind.
-constexpr size_t TS_SMEM_HALF_MIN = 77 * 1024, TS_SMEM_HALF_MAX = 113 * 1024;
+constexpr size_t TS_SMEM_HALF_MIN = 77 * 1024, TS_SMEM_HALF_MAX = 112 * 1024;
 constexpr size_t TS_SMEM_FULL_MIN = 152 * 1024, TS_SMEM_FULL_MAX = 226 * 1024;
 
 struct TsArgs {
@@ -541,8 +541,9 @@ void Dec::ts_query_clusters() {
 }
 
 // Tokens per tile and K split with the least estimated time (microseconds, fitted to measurements on B200): 3 us per launch;
-// a stage of 128 channels takes 0.54 us (16 tokens) to 0.83 us (256) when the CTA has its SM alone and 0.69 to 0.96 us
-// (128) with a second one beside it; a split CTA another 1.2 us plus 0.04 us per token for the sum over the cluster.
+// a stage of 128 channels takes 0.48 us and 0.0006 per token when the CTA has its SM alone (wide tiles more when all SMs run:
+// 0.82 at 256 tokens) and 0.65 us and 0.0018 per token with a second one beside it; a split CTA another 1.2 us and 0.04 us per
+// token for the sum over the cluster.
 TsChoice Dec::gemm_ts_choose(int n, int k, int t) const {
     TsChoice best{0, 0, 1e30};
     const int n_tiles = (n + TS_MROWS - 1) / TS_MROWS, stages = (k + SK - 1) / SK;
@@ -561,14 +562,18 @@ TsChoice Dec::gemm_ts_choose(int n, int k, int t) const {
             if (room <= 0 || (tune_ts_ks > 0 && ks != std::min(tune_ts_ks, stages))) {
                 continue;
             }
-            const double alone = 0.52 + 0.0012 * tok, paired = 0.65 + 0.0024 * tok;
             const double around = ks > 1 ? 1.2 + 0.04 * tok : 0.01 * tok;
             const int nst = (stages + ks - 1) / ks;
+            auto stage = [&](long long ctas) {
+                if (!full && ctas > sm_count) {
+                    return 0.65 + 0.0018 * tok;
+                }
+                return 0.48 + 0.0006 * tok + (full && ctas > 128 ? 0.06 + 0.0020 * std::max(0, tok - 192) : 0.0);
+            };
             const long long waves = tiles / room, rest = tiles - waves * room;
-            const double pair_stage = full ? alone : paired;
-            double c = 3.0 + waves * (nst * pair_stage + around);
+            double c = 3.0 + waves * (nst * stage((long long)room * ks) + around);
             if (rest > 0) {
-                c += nst * (rest * ks <= sm_count ? alone : pair_stage) + around;
+                c += nst * stage(rest * ks) + around;
             }
             if (c < best.cost) {
                 best = TsChoice{tok, ks, c};

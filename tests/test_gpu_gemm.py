@@ -268,3 +268,24 @@ def test_weight_row_gemm_pow2_exact(dec, t, k, n, group, tok, ks, out_f16):
     want = expect.astype(np.float16) if out_f16 else expect      # sums of powers of two: exact in f32, one rounding to f16
     assert np.array_equal(y.cpu().numpy(), want)
     assert (guard[t:] == 7.0).all()
+
+
+@pytest.mark.parametrize("bn", [128, 160, 192, 224])
+@pytest.mark.parametrize("t,k,n,group,mt,ks", [(130, 256, 272, 128, 2, -1), (300, 768, 496, 32, 2, -1), (200, 512, 448, 64, 1, -1),
+                                               (300, 1024, 624, 128, 2, 3)])
+def test_narrow_weight_tiles_pow2_exact(dec, t, k, n, group, mt, ks, bn):
+    # tiles of fewer than 256 weight rows: ragged last row tile (also by 16 rows), ragged token tile, split K
+    q, s, x, expect = pow2_case(t, k, n, group)
+    dec.upload_lin_g("nwt", q, s, n, k, group)
+    for out_f16 in (False, True):
+        guard = torch.full((t + 64, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+        for key, v in (("gemm_form", 1), ("gemm_bn", bn), ("gemm_mt", mt), ("gemm_ksplit", ks)):
+            dec.set_tuning(key, v)
+        try:
+            y = dec.lin_forward("nwt", x_dev(x), t, dst=guard[:t], out_f16=out_f16)
+            dec.sync()
+        finally:
+            for key in ("gemm_form", "gemm_bn", "gemm_mt", "gemm_ksplit"):
+                dec.set_tuning(key, 0)
+        assert np.array_equal(y.cpu().numpy(), expect.astype(np.float16) if out_f16 else expect)
+        assert (guard[t:] == 7.0).all()
