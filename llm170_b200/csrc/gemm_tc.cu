@@ -7,7 +7,8 @@
 // the f16 scale; the reference's own model of this is crates/server/src/probes/w4a16/gpu/bench.rs:240)
 // and accumulates in f32.
 //
-// One CTA computes a 128 (tokens) x 256 (weight rows) tile:
+// One CTA computes a tile of 128 or 256 tokens x 256 weight rows (128..224 where that fills SMs which 256 leaves idle).  The
+// issuing warps stay converged with one elected lane (4096 tokens, four linears of a 27B-class layer: 2390 -> 2338 us).
 //   warp 0      producer: TMA-loads the f16 activation tile (128 x 64, 128B swizzle) and bulk-copies the
 //               raw int4 tiles (16 x 512 B of the T64 layout) of each 64-wide k-block into a 6-stage ring
 //   warps 2-17  expand int4 -> f16 into a 2-stage ring of K-major 128B-swizzled B operands (one 16-byte
