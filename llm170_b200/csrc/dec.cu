@@ -632,6 +632,9 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         return 0;
     }
     if (!strcmp(key, "gemm_form")) {
+        if (value < 0 || value > 2) {
+            return d.fail("w4a16 set_tuning: gemm_form=%d (0..2)", value);
+        }
         d.tune_gemm_form = value;
         return 0;
     }
@@ -643,10 +646,16 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         return 0;
     }
     if (!strcmp(key, "gemm_ts_tok")) {
+        if (value != 0 && value != 64 && value != 96 && value != 128 && value != 192 && value != 256) {
+            return d.fail("w4a16 set_tuning: gemm_ts_tok=%d (64, 96, 128, 192, 256, or 0)", value);
+        }
         d.tune_ts_tok = value;
         return 0;
     }
     if (!strcmp(key, "gemm_ts_ksplit")) {
+        if (value < 0 || value > w4::TS_MAX_SPLIT) {
+            return d.fail("w4a16 set_tuning: gemm_ts_ksplit=%d (1..%d, or 0)", value, w4::TS_MAX_SPLIT);
+        }
         d.tune_ts_ks = value;
         return 0;
     }

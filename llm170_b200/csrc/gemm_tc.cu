@@ -722,6 +722,10 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     // waves the clock sinks and the two measured alike (4096 x 5120 x 6144: 196..237 against 201 us).
     if (tune_gemm_form == 2 || (tune_gemm_form == 0 && tune_gemm_ksplit == 0 && tune_gemm_mt == 0 && tune_gemm_bn == 0)) {
         const TsChoice c = gemm_ts_choose(l->n, l->k, t);
+        if (tune_gemm_form == 2 && c.tok == 0) {
+            return fail("w4a16 gemm: no weight-row tile for %d x %d x %d (gemm_ts_ksplit=%d: no such cluster on this device)", t, l->n,
+                        l->k, tune_ts_ks);
+        }
         if (tune_gemm_form == 2 || c.cost < (t <= 1024 ? 0.9 : 0.8) * best.cost) {
             return gemm_ts(l, x, dst, t, out_kind, c, st);
         }

@@ -545,7 +545,8 @@ void Dec::ts_query_clusters() {
 // Tokens per tile and K split with the least estimated time (microseconds, fitted to measurements on B200): 3 us per launch;
 // a stage of 128 channels takes 0.48 us and 0.0006 per token when the CTA has its SM alone (wide tiles more when all SMs run:
 // 0.82 at 256 tokens) and 0.65 us and 0.0018 per token with a second one beside it; a split CTA another 1.2 us and 0.04 us per
-// token for the sum over the cluster.
+// token for the sum over the cluster.  Without a candidate (a cluster size that is asked for and cannot be resident) the result
+// has tok = 0 and a cost above every other form's.
 TsChoice Dec::gemm_ts_choose(int n, int k, int t) const {
     TsChoice best{0, 0, 1e30};
     const int n_tiles = (n + TS_MROWS - 1) / TS_MROWS, stages = (k + SK - 1) / SK;

@@ -289,3 +289,22 @@ def test_narrow_weight_tiles_pow2_exact(dec, t, k, n, group, mt, ks, bn):
                 dec.set_tuning(key, 0)
         assert np.array_equal(y.cpu().numpy(), expect.astype(np.float16) if out_f16 else expect)
         assert (guard[t:] == 7.0).all()
+
+
+@pytest.mark.parametrize("key,bad", [("gemm_form", -1), ("gemm_form", 3), ("gemm_ts_tok", 32), ("gemm_ts_tok", 100),
+                                     ("gemm_ts_tok", -64), ("gemm_ts_ksplit", -1), ("gemm_ts_ksplit", 9)])
+def test_weight_row_tuning_refuses_values_without_a_tile(dec, key, bad):
+    # a value that matches no tile left the weight-row form without a candidate and divided by its token count of zero
+    from llm170_b200.w4a16_dec import W4a16Error
+    q, s, x, expect = pow2_case(16, 2048, 64, 128)          # more 128-channel stages than the largest split
+    dec.upload_lin_g("tun", q, s, 64, 2048, 128)
+    try:
+        with pytest.raises(W4a16Error, match=key):
+            dec.set_tuning(key, bad)
+        dec.set_tuning("gemm_form", 2)
+        y = dec.lin_forward("tun", x_dev(x), 16)
+        dec.sync()
+        assert np.array_equal(y.cpu().numpy(), expect)
+    finally:
+        for k in ("gemm_form", "gemm_ts_tok", "gemm_ts_ksplit"):
+            dec.set_tuning(k, 0)
