@@ -3,7 +3,7 @@
 //
 // Why: a decode linear runs 4 to 20 us on the GPU, and a host that drives a layer call by call (no captured graph) spent
 // 13 us in Python and ctypes around each of them: 4 us for torch.cuda.current_stream(), 2.5 for torch.empty, 1.3 for a
-// ctypes lin_spec, 1 for the ctypes call itself.  Here the same steps take about 1.5 us (at::detail::empty_cuda, the raw
+// ctypes lin_spec, 1 for the ctypes call itself.  Here the same steps take about 1.5 us (at::empty, the raw
 // stream, direct C calls), so eager decode is bound by the launches again.
 //
 // The library itself keeps its plain C ABI; this module reaches it through the addresses that the ctypes loader resolved
@@ -12,7 +12,6 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
-#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -65,7 +64,8 @@ const at::Tensor* checked(PyObject* o, at::ScalarType st, int device, const char
 bool output(PyObject* dst, int64_t t, int64_t n, bool f16, int device, at::Tensor* out) {
     const at::ScalarType st = f16 ? at::kHalf : at::kFloat;
     if (dst == Py_None) {
-        *out = at::detail::empty_cuda({t, n}, st, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt);
+        // (through the dispatcher, as torch.empty: dispatch modes see it, deterministic mode fills it)
+        *out = at::empty({t, n}, at::TensorOptions().dtype(st).device(at::kCUDA, (c10::DeviceIndex)device));
         return true;
     }
     const at::Tensor* d = checked(dst, st, device, "dst");
@@ -173,17 +173,18 @@ PyObject* multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             return nullptr;
         }
         constexpr Py_ssize_t MAXSEG = 64;   // the library refuses more than it supports with its own message
-        PyObject* names = PySequence_Fast(a[2], "names must be a sequence");
+        // tuples of their own: the library reads the names without the interpreter lock, while the caller's lists may change
+        PyObject* names = PySequence_Tuple(a[2]);
         if (!names) {
             return nullptr;
         }
-        PyObject* outs = a[4] == Py_None ? nullptr : PySequence_Fast(a[4], "outs must be a sequence");
+        PyObject* outs = a[4] == Py_None ? nullptr : PySequence_Tuple(a[4]);
         PyObject* result = nullptr;
         [&] {
             if (a[4] != Py_None && !outs) {
                 return;
             }
-            const Py_ssize_t ns = PySequence_Fast_GET_SIZE(names);
+            const Py_ssize_t ns = PyTuple_GET_SIZE(names);
             const long long t = PyLong_AsLongLong(a[5]);
             const int f16 = PyObject_IsTrue(a[6]);
             if (PyErr_Occurred()) {
@@ -196,7 +197,7 @@ PyObject* multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
             const char* nm[MAXSEG];
             int n[MAXSEG], k = 0;
             for (Py_ssize_t i = 0; i < ns; ++i) {
-                nm[i] = PyUnicode_AsUTF8(PySequence_Fast_GET_ITEM(names, i));
+                nm[i] = PyUnicode_AsUTF8(PyTuple_GET_ITEM(names, i));
                 if (!nm[i]) {
                     return;
                 }
@@ -215,16 +216,16 @@ PyObject* multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
                 PyErr_SetString(error_type, "sk_multi_dev: x size does not match t*k");
                 return;
             }
-            // as zip() does, a list of outputs of another length than the names pairs up with the shorter of the two
-            const Py_ssize_t no = outs ? std::min(ns, PySequence_Fast_GET_SIZE(outs)) : ns;
-            if (no != ns) {
+            // outputs beyond the names are left alone, a name without an output is refused
+            const Py_ssize_t no = outs ? PyTuple_GET_SIZE(outs) : ns;
+            if (no < ns) {
                 PyErr_Format(error_type, "sk_multi_dev: %zd outputs for %zd names", no, ns);
                 return;
             }
             at::Tensor y[MAXSEG];
             void* yp[MAXSEG];
             for (Py_ssize_t i = 0; i < ns; ++i) {
-                if (!output(outs ? PySequence_Fast_GET_ITEM(outs, i) : Py_None, t, n[i], f16, r.device, &y[i])) {
+                if (!output(outs ? PyTuple_GET_ITEM(outs, i) : Py_None, t, n[i], f16, r.device, &y[i])) {
                     return;
                 }
                 yp[i] = y[i].data_ptr();
