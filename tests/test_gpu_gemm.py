@@ -38,25 +38,50 @@ def pow2_case(t, k, n, group):
     return q, s, x, (x.view(np.float16).astype(np.float64) @ w.T).astype(np.float32)
 
 
+FORMS = {1: "gemm_w4a16_tc_kernel", 2: "gemm_ts_kernel"}      # "gemm_form": token rows, weight rows
+
+
+class forced:
+    """A tuning key at a value, and back at its default."""
+
+    def __init__(self, dec, key, value, default=0):
+        self.args = dec, key, value, default
+
+    def __enter__(self):
+        dec, key, value, _ = self.args
+        dec.set_tuning(key, value)
+
+    def __exit__(self, *_):
+        dec, key, _, default = self.args
+        dec.set_tuning(key, default)
+
+
+@pytest.mark.parametrize("form", [1, 2])
 @pytest.mark.parametrize("t,k,n,group", [(16, 256, 128, 128), (64, 512, 256, 128), (300, 256, 272, 128),
                                          (33, 128, 64, 32), (129, 768, 512, 32)])
-def test_pow2_kat_exact(dec, t, k, n, group):
+def test_pow2_kat_exact(dec, t, k, n, group, form):
     # crates/server/src/probes/w4a16/gpu/bench.rs:77-166: power-of-two scales/activations -> exact sums
     q, s, x, expect = pow2_case(t, k, n, group)
     dec.upload_lin_g("p2", q, s, n, k, group)
-    y = dec.lin_forward("p2", x_dev(x), t)
+    with forced(dec, "gemm_form", form):
+        y = dec.lin_forward("p2", x_dev(x), t)
+    assert dec.last_kernel().startswith(FORMS[form])
     dec.sync()
     assert np.array_equal(y.cpu().numpy().view(np.uint32), expect.view(np.uint32))
 
 
+@pytest.mark.parametrize("form", [1, 2])
 @pytest.mark.parametrize("n,k,group,t", [(256, 128, 128, 9), (512, 1024, 128, 130), (1536, 2048, 32, 257),
                                          (2048, 768, 32, 64), (4096, 4096, 128, 16), (7168, 5120, 128, 512)])
-def test_gemm_vs_f16_dequant_model_and_lane_oracle(dec, orc, n, k, group, t):
+def test_gemm_vs_f16_dequant_model_and_lane_oracle(dec, orc, n, k, group, t, form):
     q, s = synth.make_linear(n, k, group, seed=300 + t)
     x = synth.make_acts(t, k, seed=400 + t, scale=1.0 / np.sqrt(k))
     dec.upload_lin_g("g", q, s, n, k, group)
     xd = x_dev(x)
-    y = dec.lin_forward("g", xd, t)
+    with forced(dec, "gemm_form", form):
+        y = dec.lin_forward("g", xd, t)
+        y16 = dec.lin_forward("g", xd, t, out_f16=True)
+    assert dec.last_kernel().startswith(FORMS[form])
     dec.sync()
     w16 = dec.dequant_lin("g", f16=True)
     ref = xd.float() @ w16.float().T                       # plain torch fp32 reference of the specified op
@@ -66,8 +91,6 @@ def test_gemm_vs_f16_dequant_model_and_lane_oracle(dec, orc, n, k, group, t):
     want = orc.linear_lane(q, s, x, t, n, k, group, rows=rows)
     got = y.cpu().numpy()[:, rows[0]:rows[1]]
     assert np.abs(got - want[:, rows[0]:rows[1]]).max() <= TOL
-    y16 = dec.lin_forward("g", xd, t, out_f16=True)
-    dec.sync()
     assert torch.equal(y16, y.to(torch.float16))
     dec.drop_lin("g")
 
@@ -104,21 +127,23 @@ def test_tile_variants_agree_bitwise(dec):
 
 @pytest.mark.parametrize("n,k,group,t,out_f16", [(512, 1024, 128, 512, 0), (1024, 2048, 128, 700, 0),
                                                   (784, 512, 32, 1300, 0), (2048, 2048, 32, 1024, 1),
-                                                  (272, 128, 128, 130, 1), (256, 256, 128, 9, 1), (4864, 4096, 128, 512, 1)])
+                                                  (272, 128, 128, 130, 1), (256, 256, 128, 9, 1), (4864, 4096, 128, 512, 1),
+                                                  (6144, 4096, 128, 2048, 1)])
 def test_tma_store_epilogue_agrees_bitwise_with_per_lane_stores(dec, n, k, group, t, out_f16):
     # the staged TMA-store epilogue writes the same values as the per-lane stores: ragged last token tile, a last
     # column chunk cut at n, both output types, and a launch whose last wave is split (those tiles keep their own path)
     q, s = synth.make_linear(n, k, group, seed=71 + t)
     dec.upload_lin_g("epi", q, s, n, k, group)
     x = x_dev(synth.make_acts(t, k, seed=72 + t, scale=1 / np.sqrt(k)))
-    try:
-        dec.set_tuning("gemm_tma_store", 0)
-        lanes = dec.lin_forward("epi", x, t, out_f16=bool(out_f16)).clone()
-        dec.set_tuning("gemm_tma_store", 1)
-        guard = torch.full((t + 64, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    guard = torch.full((t + 64, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    with forced(dec, "gemm_form", 1):
+        with forced(dec, "gemm_tma_store", 0, default=1):
+            lanes = dec.lin_forward("epi", x, t, out_f16=bool(out_f16)).clone()
+            kernels = [dec.last_kernel()]
         staged = dec.lin_forward("epi", x, t, dst=guard[:t], out_f16=bool(out_f16))
-    finally:
-        dec.set_tuning("gemm_tma_store", 1)
+        kernels.append(dec.last_kernel())
+    assert all(nm.startswith(FORMS[1]) for nm in kernels), kernels
+    assert "last wave" in kernels[1] or n != 6144, kernels
     dec.sync()
     assert torch.equal(lanes, staged)
     assert bool((guard[t:] == 7.0).all())        # nothing is written past the batch
@@ -308,3 +333,44 @@ def test_weight_row_tuning_refuses_values_without_a_tile(dec, key, bad):
     finally:
         for k in ("gemm_form", "gemm_ts_tok", "gemm_ts_ksplit"):
             dec.set_tuning(k, 0)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("t,form,ks", [(27, 2, 1), (27, 2, 4), (150, 2, 1), (150, 2, 2), (300, 0, 0)])
+def test_launches_that_feed_one_another(dec, t, form, ks, graph):
+    # A launch reads its weights before the previous one of the stream is complete.  Here each reads what the one before wrote
+    # and overwrites what that one read: two buffers in turn, against the same chain with a wait after every launch.
+    n, links = 1024, 12
+    for i in range(links):
+        q, s = synth.make_linear(n, n, 128, seed=90 + i)
+        dec.upload_lin_g(f"chain{i}", q, s, n, n, 128)
+    start = x_dev(synth.make_acts(t, n, seed=91))
+    bufs = [torch.empty_like(start), torch.empty_like(start)]
+    stream = torch.cuda.ExternalStream(dec.stream_ptr())
+
+    def chain(wait):
+        bufs[0].copy_(start)
+        for i in range(links):
+            dec.lin_forward(f"chain{i}", bufs[i % 2], t, dst=bufs[(i + 1) % 2], out_f16=True)
+            if wait:
+                stream.synchronize()
+
+    with forced(dec, "gemm_form", form), forced(dec, "gemm_ts_ksplit", ks), torch.cuda.stream(stream):
+        chain(wait=True)
+        assert dec.last_kernel().startswith(FORMS[2]), dec.last_kernel()
+        want = bufs[links % 2].clone()
+        assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+        if graph:
+            dec.capture_begin()
+            chain(wait=False)
+            g = dec.capture_end()
+        for _ in range(20):
+            if graph:
+                dec.graph_launch(g)
+            else:
+                chain(wait=False)
+            stream.synchronize()
+            assert torch.equal(bufs[links % 2], want)
+        if graph:
+            dec.graph_destroy(g)
+    dec.kernel_status()
