@@ -718,15 +718,20 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     // The weight-row form (gemm_ts.cu) takes the calls that it finishes sooner: up to about 128 tokens nearly all of them (its
     // MMA tile is as wide as the batch: 27 x 34816 x 5120 in 31 us against 52), above that those whose tiles here leave SMs
     // idle (512 x 7168 x 5120: 32 against 59 us); in full waves the 256 x 256 tiles are up to a fifth faster (256 x 34816 x
-    // 5120: 67 against 72 us).  At a tie, within a tenth, this form; above 1024 tokens within a fifth: over several full
-    // waves the clock sinks and the two measured alike (4096 x 5120 x 6144: 196..237 against 201 us).
+    // 5120: 67 against 72 us).  At a tie, within a tenth, this form; above 1024 tokens with K below 3072 within a fifth: there the
+    // estimates leave out part of what the weight-row form's many short tiles cost.  Where its estimate is 0.8..0.9 of this
+    // form's, at 1025..4096 tokens, it took 0.65..0.97 of the time on 24 shapes with K >= 3072 and 1.01 on two (1281 tokens, 7168
+    // x 5120: 80 against 99 us, 5120 x 17408: 180 against 234), and 0.77..1.30 on 24 with a shorter K (1391 tokens, 15824 x 512:
+    // 41 against 37 us; 2332 tokens, 22768 x 1216: 162 against 150); up to 1024 tokens 0.61..0.99 at any K (16 shapes).  More
+    // than 4096 tokens were not compared: a fifth, too.
+    const double bar_ts = t <= 1024 || (l->k >= 3072 && t <= 4096) ? 0.9 : 0.8;
     if (tune_gemm_form == 2 || (tune_gemm_form == 0 && tune_gemm_ksplit == 0 && tune_gemm_mt == 0 && tune_gemm_bn == 0)) {
         const TsChoice c = gemm_ts_choose(l->n, l->k, t);
         if (tune_gemm_form == 2 && c.tok == 0) {
             return fail("w4a16 gemm: no weight-row tile for %d x %d x %d (gemm_ts_ksplit=%d: no such cluster on this device)", t, l->n,
                         l->k, tune_ts_ks);
         }
-        if (tune_gemm_form == 2 || c.cost < (t <= 1024 ? 0.9 : 0.8) * best.cost) {
+        if (tune_gemm_form == 2 || c.cost < bar_ts * best.cost) {
             return gemm_ts(l, x, dst, t, out_kind, c, st);
         }
     }

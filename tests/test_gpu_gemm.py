@@ -374,3 +374,20 @@ def test_launches_that_feed_one_another(dec, t, form, ks, graph):
         if graph:
             dec.graph_destroy(g)
     dec.kernel_status()
+
+
+@pytest.mark.parametrize("n,k,t,form", [(784, 512, 1300, 2), (2048, 2048, 1024, 2), (7168, 5120, 27, 2), (2048, 8192, 1300, 2),
+                                        (5120, 6144, 1281, 2), (5120, 6144, 4096, 1), (15824, 512, 1391, 1)])
+def test_automatic_form(dec, n, k, t, form):
+    # narrow linears stay on the weight-row form at any batch; full waves of 256 x 256 tiles, and many tokens over a short K, do not
+    # (the two agree to the order of their f32 sums: the bound of the f16-model test)
+    q, s = synth.make_linear_cuda(n, k, 128, 95, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("auto", q, s, n, k, 128)
+    x = x_dev(synth.make_acts(t, k, seed=96, scale=1 / np.sqrt(k)))
+    y = dec.lin_forward("auto", x, t)
+    assert dec.last_kernel().startswith(FORMS[form]), dec.last_kernel()
+    with forced(dec, "gemm_form", 3 - form):
+        other = dec.lin_forward("auto", x, t)
+    dec.sync()
+    assert (y - other).abs().max().item() <= 1e-4 * y.abs().max().item() + 1e-6
+    dec.drop_lin("auto")
