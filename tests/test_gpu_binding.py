@@ -116,9 +116,44 @@ def test_calls_run_on_torchs_current_stream(dec, t):
     assert torch.equal(y, want)
 
 
+class library_call:
+    """One entry point of the library replaced by a host function."""
+
+    def __init__(self, symbol, stand_in):
+        self.symbol, self.stand_in = symbol, stand_in
+
+    def _bind(self, stand_in):
+        from llm170_b200.w4a16_dec import W4a16Error
+        L = _lib.lib()
+        own = lambda s: C.cast(getattr(L, s), C.c_void_p).value  # noqa: E731
+        at = lambda s: C.cast(stand_in, C.c_void_p).value if stand_in and s == self.symbol else own(s)  # noqa: E731
+        _lib.native(W4a16Error).bind(W4a16Error, at)
+
+    def __enter__(self):
+        self._bind(self.stand_in)
+
+    def __exit__(self, *_):
+        self._bind(None)
+
+
+def test_new_outputs_are_filled_in_deterministic_mode(dec):
+    x = x_of(2)
+
+    @C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_char_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p)
+    def writes_nothing(*_):
+        return 0
+
+    torch.use_deterministic_algorithms(True)
+    try:
+        with library_call("w4a16_lin_forward", writes_nothing):
+            y = dec.lin_forward("a", x, 2)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert bool(torch.isnan(y).all())
+
+
 def test_names_outlive_the_callers_list(dec):
     # the library runs without the interpreter lock: another thread may change the list of names meanwhile
-    from llm170_b200.w4a16_dec import W4a16Error
     seen = []
     names = ["".join(["lin", str(i)]) for i in (900, 901)]
     for nm in names:
@@ -135,12 +170,7 @@ def test_names_outlive_the_callers_list(dec):
         seen.extend(nm[i] for i in range(ns))
         return len(keep) - 64
 
-    L, native = _lib.lib(), _lib.native(W4a16Error)
-    address = lambda symbol: C.cast(getattr(L, symbol), C.c_void_p).value  # noqa: E731
     x = x_of(1)
-    native.bind(W4a16Error, lambda symbol: C.cast(in_the_library, C.c_void_p).value if symbol == "w4a16_sk_multi_dev" else address(symbol))
-    try:
+    with library_call("w4a16_sk_multi_dev", in_the_library):
         dec.sk_multi_dev(names, x)
-    finally:
-        native.bind(W4a16Error, address)
     assert seen == want
