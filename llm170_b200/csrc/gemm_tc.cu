@@ -11,10 +11,10 @@
 // issuing warps stay converged with one elected lane (4096 tokens, four linears of a 27B-class layer: 2390 -> 2338 us).
 //   warp 0      producer: TMA-loads the f16 activation tile (128 x 64, 128B swizzle) and bulk-copies the
 //               raw int4 tiles (16 x 512 B of the T64 layout) of each 64-wide k-block into a 6-stage ring
-//   warps 2-17  expand int4 -> f16 into a 2-stage ring of K-major 128B-swizzled B operands (one 16-byte
-//               chunk = 8 consecutive k of one weight row), then signal the MMA warp
-//   warp 1      one lane issues 4 x tcgen05.mma (M128 N256 K16, f16 x f16 -> f32 in TMEM) per k-block and
-//               commits the stage back to the producer
+//   warps 2-17  expand int4 -> f16 into a 2-stage ring of K-major 128B-swizzled B operands (a lane's word holds 4
+//               consecutive k of two weight rows: 8-byte pieces, half a swizzled chunk), then signal the MMA warp
+//   warp 1      issues 4 x tcgen05.mma (M128, N = weight rows of the tile, K16, f16 x f16 -> f32 in TMEM) per k-block
+//               and 128-token block and commits the stage back to the producer
 //   warps 2-17  epilogue: tcgen05.ld the f32 accumulators (each warp its TMEM lane quadrant, every fourth
 //               32-column chunk), convert, store y
 // Every mbarrier wait is bounded: on expiry the kernel records a status code, all roles fall through to
@@ -75,8 +75,9 @@ struct GemmArgs {
                           // f16(silu(f16 gate) * f16 up), n/2 values per row
     // split-K: the first `n_whole` tiles (in launch order) are one CTA each; every later tile is `ksplit` CTAs, each
     // multiplying k-blocks [nkb*s/ksplit, nkb*(s+1)/ksplit).  Their f32 partial tiles go to `part`, and the last
-    // split to arrive (ticket per tile, left at zero) adds them in split order, converts and stores.  Used for all
-    // tiles when they are few (small token counts), and for the tiles of an incomplete last wave otherwise.
+    // splits of a tile add a slice each, in split order (ticket per tile, left at zero), convert and store.  Used for the
+    // tiles of an incomplete last wave, and for all tiles where there are too few of them and the weight-row form
+    // (gemm_ts.cu) is not estimated faster.
     int n_whole;
     int ksplit;
     float* part;          // [split tiles][ksplit][BM*MT][BN] f32
@@ -539,9 +540,11 @@ gemm_w4a16_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_co
     if (ks > 1) {
         // Every split of the tile adds a slice of its rows over all partial tiles, in split order (the same bits whatever
         // the arrival order), converts and stores.  One CTA adding all of them would read ksplit x 256 KB alone and take
-        // longer than the wave it saves.  The splits of a tile are consecutive CTAs of the launch's last wave (their
-        // number never exceeds the SM count), so they run at the same time; the wait for the siblings is bounded all
-        // the same.  The ticket counts arrivals up to ksplit and departures up to 2 x ksplit, then returns to zero.
+        // longer than the wave it saves.  The splits of a tile are consecutive CTAs, at most 16 of them.  When every tile is
+        // split there can be more CTAs than SMs; blocks start in the order of their index, so the earliest unfinished tile
+        // has all of its splits on the GPU or next in line behind tiles that need nothing from it.  The wait for the
+        // siblings is bounded all the same.  The ticket counts arrivals up to ksplit and departures up to 2 x ksplit, then
+        // returns to zero.
         if (threadIdx.x == 0) {
             int ready = 0;
             if (!*abort_flag) {
@@ -654,7 +657,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     // whole tiles plus a split last wave; every tile split 2..16 ways (at least four k-blocks per split, partial tiles within
     // 128 MB of scratch).  Tiles narrower than 256 rows multiply less per expanded k-block and are taken where they fill SMs
     // that 256 leaves idle, by a tenth at least (1024 tokens, 5120 x 17408: 128 tiles of 160 rows 149 us, 80 of 256 178 us;
-    // 5120 x 6144: 57 against 67 us).
+    // 5120 x 6144: 57 against 67 us).  224 rows never won the estimate over 20000 shapes and are there for the tuning key.
     const int nkb_all = l->k / BK;
     struct Choice {
         int mt, bn, n_whole, ks;

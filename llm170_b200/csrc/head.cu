@@ -172,8 +172,9 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
     };
     // Whole rounds: a row block per warp.  The rest of the row blocks is dealt over all SMs and, where it leaves warps idle,
     // each block's K over several warps of its CTA: 151936 rows are 4.01 rounds, and the fifth one cost as much as the others.
-    // (One token, before and after: 151936 x 2048 67 -> 62 us, 151936 x 5120 148 -> 135, 50000 x 4096 51 -> 43.  Bound by HBM
-    // latency: fetching four steps ahead in two register sets keeps fewer loads in flight and took 72 us.)
+    // (One token, calls back to back into one output, before and after: 151936 x 2048 66.9 -> 61.6 us, 151936 x 5120 147 -> 134,
+    // 50000 x 4096 50.2 -> 43.1.  Bound by HBM latency: fetching four steps ahead in two register sets keeps fewer loads in
+    // flight and took 72 us on the first.)
     const int all_warps = gridDim.x * WARPS, rounds = nrb / all_warps;
     for (int i = 0; i < rounds; ++i) {
         const int rb = i * all_warps + blockIdx.x * WARPS + warp;

@@ -3,7 +3,7 @@
 //
 // Why: a decode linear runs 4 to 20 us on the GPU, and a host that drives a layer call by call (no captured graph) spent
 // 13 us in Python and ctypes around each of them (10 with the caller's output): 4 us for torch.cuda.current_stream(), 2.5 for
-// torch.empty, 1.3 for a ctypes lin_spec, 1 for the ctypes call itself.  Here the same steps and the launch take 3.7 us (2.7
+// torch.empty, 1.3 for a ctypes lin_spec, 1 for the ctypes call itself.  Here the same steps and the launch take 3.4 us (2.4
 // with the caller's output), so eager decode is bound by the launches again.
 //
 // The library itself keeps its plain C ABI; this module reaches it through the addresses that the ctypes loader resolved
@@ -64,7 +64,7 @@ const at::Tensor* checked(PyObject* o, at::ScalarType st, int device, const char
 }
 
 // Nothing stands between torch.empty and its allocator: no dispatch mode or function transform, no profiler, no deterministic
-// fill.  Then the allocator may be called directly (3.7 us of host time per call against 4.4 through the dispatcher).
+// fill.  Then the allocator may be called directly (3.4 us of host time per call against 4.4 through the dispatcher).
 bool plain_empty() {
     const at::Context& ctx = at::globalContext();
     return c10::impl::tls_local_dispatch_key_set().included_ == c10::default_included_set && !at::hasCallbacks() &&
