@@ -131,8 +131,10 @@ struct Dec {
     void ts_query_clusters();
     TsChoice gemm_ts_choose(int n, int k, int t) const;
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
+    int gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
+                        int tok, const float* row_w, cudaStream_t st, bool tables_fresh);
     int gemm_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b,
-                     int max_tiles, int mt, const float* row_w, cudaStream_t st);
+                     int max_tiles, const float* row_w, cudaStream_t st);
     // row-parallel tensor parallelism (fused all-reduce in the GEMV): local exchange block + peer mappings
     TpComm tp{};
     void* tp_block = nullptr;

@@ -48,6 +48,7 @@ constexpr int RAW_BYTES = TS_MROWS * SK / 2;    // 8 KB per stage
 constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
 constexpr int DQ_WARPS = TS_MROWS / TILE_ROWS;  // a warp per 16-row block
 constexpr int TS_THREADS = (3 + DQ_WARPS) * 32;
+constexpr int TS_XBOX = 64;                     // grouped mode: rows of a token box
 constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
 // Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
 // waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
@@ -71,6 +72,16 @@ struct TsArgs {
     int pdl;
     float out_mul;
     int* status;
+    // grouped (MoE) mode: token tiles come from a device table, one expert's weights (n rows) per tile; tok is then the most
+    // rows that a tile holds
+    const int* tile_expert;
+    const int* tile_row0;
+    const int* tile_rows;
+    const int* num_tiles;
+    int expert0;
+    const float* row_w;  // optional factor per sorted row
+    int glu;             // 1: interleaved gate / up row blocks; stores f16(silu(f16 gate) * f16 up), n / 2 values per row
+    int tables_fresh;    // 1: a launch that may not be complete yet wrote the table: read it only after the dependency wait
 };
 
 __device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accum) {
@@ -106,7 +117,7 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
     return v;
 }
 
-template <int GROUP>
+template <int GROUP, bool GROUPED>
 __global__ void __launch_bounds__(TS_THREADS, 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
@@ -132,11 +143,28 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     const uint32_t accum_bar = bars + 8u * (2 * NR + 2 * NX + 2 * NA);
 
     // ---- this CTA's tile ----
-    const int tile = (int)blockIdx.x, ks = a.ksplit, split = (int)blockIdx.y;
-    const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
-    const int n0 = ntile * TS_MROWS;
-    const int m0 = mtile * N, rb0 = n0 / TILE_ROWS;
-    const int rows_valid = min(N, a.m - m0);
+    const int tile = (int)blockIdx.x, ks = GROUPED ? 1 : a.ksplit, split = GROUPED ? 0 : (int)blockIdx.y;
+    int m0, n0, rb0, rows_valid;
+    if (GROUPED) {
+        if (a.tables_fresh) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+        }
+        // neighbours share the token rows, then the expert's weights
+        const int mt = tile / a.n_tiles, ntile = tile - mt * a.n_tiles;
+        if (mt >= *a.num_tiles) {
+            return;      // the grid is sized for the worst case
+        }
+        n0 = ntile * TS_MROWS;
+        m0 = a.tile_row0[mt];
+        rows_valid = a.tile_rows[mt];
+        rb0 = ((a.tile_expert[mt] - a.expert0) * a.n + n0) / TILE_ROWS;
+    } else {
+        const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
+        n0 = ntile * TS_MROWS;
+        m0 = mtile * N;
+        rb0 = n0 / TILE_ROWS;
+        rows_valid = min(N, a.m - m0);
+    }
     const int nrbv = min(TS_MROWS, a.n - n0) / TILE_ROWS;       // valid 16-row blocks
     const uint32_t kb_bytes = (uint32_t)nrbv * (TILE_WORDS * 4);
     // K range of this split in stages; the last stage of the matrix may hold one k-block (32-channel groups)
@@ -206,9 +234,21 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 break;
             }
             if (leader) {
-                // both k-blocks in one box (the second one of the last stage may lie outside: zeros)
-                mbar_expect_tx(x_full(sx), 2 * x_half);
-                tma_load_3d(x_addr(sx), &tmap_x, 0, m0, 2 * (st0 + it), x_full(sx));
+                if (GROUPED) {
+                    // the rows of the tile in boxes of 64 (rows of the next expert, or zeros, fill the last one up)
+                    const int kbs = stage_kbs(it), boxes = (rows_valid + TS_XBOX - 1) / TS_XBOX;
+                    mbar_expect_tx(x_full(sx), (uint32_t)(kbs * boxes) * (TS_XBOX * BK * 2));
+                    for (int h = 0; h < kbs; ++h) {
+                        for (int c = 0; c < boxes; ++c) {
+                            tma_load_2d(x_addr(sx) + h * x_half + (uint32_t)c * (TS_XBOX * BK * 2), &tmap_x, (2 * (st0 + it) + h) * BK,
+                                        m0 + c * TS_XBOX, x_full(sx));
+                        }
+                    }
+                } else {
+                    // both k-blocks in one box (the second one of the last stage may lie outside: zeros)
+                    mbar_expect_tx(x_full(sx), 2 * x_half);
+                    tma_load_3d(x_addr(sx), &tmap_x, 0, m0, 2 * (st0 + it), x_full(sx));
+                }
             }
             __syncwarp();
             if (++sx == NX) {
@@ -235,7 +275,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
+        const int n_mma = GROUPED ? (rows_valid + 15) & ~15 : N;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(n_mma >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
         const bool leader = elect_one();
         int sx = 0, px = 0, sa = 0, pa = 0;
         for (int it = 0; it < nst; ++it) {
@@ -387,28 +428,46 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     const int quad = warp & 3, sub = (warp - 2) >> 2;
     constexpr int EW = DQ_WARPS / 4;                                 // warps that share a TMEM lane quadrant
     const int lrow = quad * 32 + lane;                               // weight row within the tile
-    if (ks == 1 && a.out_f16) {
+    if (ks == 1 && (GROUPED || a.out_f16)) {
         // f16 results meet in shared memory ([token][row], the rings are idle) and leave as whole 16-byte pieces of a token's
         // row: a lane holds one weight row, so from registers it would store 2 bytes at a time (197 x 34816 x 5120: 62.9 -> 60.7
         // us; 64 tokens 32.2 -> 31.8)
-        constexpr int PER_TOK = TS_MROWS * 2;
+        const bool glu = GROUPED && a.glu;
+        const int per_tok = glu ? TS_MROWS : TS_MROWS * 2, n_out = glu ? a.n / 2 : a.n;      // bytes; values per row of the result
         if (dq_warp && ok) {
             for (int c0 = sub * 16; c0 < rows_valid; c0 += EW * 16) {
                 uint32_t v[16];
                 tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+                if (glu) {
+                    // lanes 0-15 hold gate sums, lanes 16-31 the up sums of the same outputs: the former take tokens 0-7 of
+                    // the chunk, the latter 8-15
+                    const bool hi = lane >= 16;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    *reinterpret_cast<__half*>(base_ptr + (c0 + i) * PER_TOK + lrow * 2) = __float2half_rn(__uint_as_float(v[i]) * a.out_mul);
+                    for (int i = 0; i < 8; ++i) {
+                        const float mine = __uint_as_float(hi ? v[i + 8] : v[i]) * a.out_mul;
+                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(hi ? v[i] : v[i + 8]), 16) * a.out_mul;
+                        *reinterpret_cast<__half*>(base_ptr + (c0 + i + (hi ? 8 : 0)) * per_tok + (quad * 16 + (lane & 15)) * 2) =
+                            silu_mul_f16(hi ? other : mine, hi ? mine : other);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        float f = __uint_as_float(v[i]) * a.out_mul;
+                        if (GROUPED && a.row_w != nullptr) {
+                            f = mul_row_w(f, c0 + i < rows_valid ? a.row_w[m0 + c0 + i] : 0.f);
+                        }
+                        *reinterpret_cast<__half*>(base_ptr + (c0 + i) * per_tok + lrow * 2) = __float2half_rn(f);
+                    }
                 }
             }
         }
         __syncthreads();
         if (!*abort_flag) {
-            const int pieces = min(TS_MROWS, a.n - n0) / 8;
-            __half* out = reinterpret_cast<__half*>(a.out) + (size_t)m0 * a.n + n0;
+            const int pieces = min(TS_MROWS, a.n - n0) / (glu ? 16 : 8);
+            __half* out = reinterpret_cast<__half*>(a.out) + (size_t)m0 * n_out + (glu ? n0 / 2 : n0);
             for (int e = (int)threadIdx.x; e < rows_valid * pieces; e += TS_THREADS) {
                 const int tok = e / pieces, c = e - tok * pieces;
-                *reinterpret_cast<uint4*>(out + (size_t)tok * a.n + c * 8) = *reinterpret_cast<const uint4*>(base_ptr + tok * PER_TOK + c * 16);
+                *reinterpret_cast<uint4*>(out + (size_t)tok * n_out + c * 8) = *reinterpret_cast<const uint4*>(base_ptr + tok * per_tok + c * 16);
             }
         }
     } else if (ks == 1) {
@@ -500,9 +559,12 @@ static size_t ts_smem(int tok, int nr, int nx, int na, int* off_x, int* off_bars
 }
 
 cudaError_t gemm_ts_init_device() {
-    cudaError_t e = cudaFuncSetAttribute(gemm_ts_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
-    if (e == cudaSuccess) {
-        e = cudaFuncSetAttribute(gemm_ts_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
+    cudaError_t e = cudaSuccess;
+    for (const void* f : {(const void*)gemm_ts_kernel<128, false>, (const void*)gemm_ts_kernel<32, false>,
+                          (const void*)gemm_ts_kernel<128, true>, (const void*)gemm_ts_kernel<32, true>}) {
+        if (e == cudaSuccess) {
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
+        }
     }
     return e;
 }
@@ -550,7 +612,7 @@ void Dec::ts_query_clusters() {
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128, false>, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 n = 0;       // then this split is not considered
             }
@@ -665,12 +727,85 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cudaError_t e;
-    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128>, map, a) : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32>, map, a);
+    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, a)
+                        : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, a);
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
     last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "> " + std::to_string(c.tok) + "-token tiles" +
                   (c.ks > 1 ? ", clusters of " + std::to_string(c.ks) : std::string());
+    launches++;
+    return 0;
+}
+
+// Grouped form over expert segments: `l` stacks the local experts along n (n_per_expert rows each); xs holds the gathered rows
+// (sorted by expert), the token-tile table (at most `tok` rows each) lives on the device (moe.cu).
+int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
+                         int tok, const float* row_w, cudaStream_t st, bool tables_fresh) {
+    EncodeTiledFn enc = encode_fn();
+    if (!enc) {
+        return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
+    }
+    const TsPlan p = ts_plan(tok);
+    TsArgs a{};
+    a.tok = tok;
+    a.ksplit = 1;
+    a.m_tiles = max_tiles;
+    a.n_tiles = (n_per_expert + TS_MROWS - 1) / TS_MROWS;
+    a.tmem_cols = p.tmem_cols;
+    a.a_stages = p.na;
+    a.raw_stages = p.nr;
+    a.x_stages = p.nx;
+    a.off_x = p.off_x;
+    a.off_bars = p.off_bars;
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)l->k, (cuuint64_t)xs_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)l->k * 2};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)TS_XBOX};
+    const cuuint32_t estr[2] = {1, 1};
+    CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs), dims, strides, box, estr,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) {
+        return fail("w4a16 gemm: cuTensorMapEncodeTiled failed (%d)", (int)cr);
+    }
+    a.qt = l->qt;
+    a.st = (const uint32_t*)l->st;
+    a.out = out;
+    a.m = xs_rows;
+    a.n = n_per_expert;
+    a.k = l->k;
+    a.out_f16 = 1;
+    a.nrb_w = l->n / TILE_ROWS;
+    a.pdl = tune_pdl ? 1 : 0;
+    a.out_mul = l->out_mul;
+    a.status = gemm_status;
+    a.tile_expert = b.tile_expert;
+    a.tile_row0 = b.tile_row0;
+    a.tile_rows = b.tile_rows;
+    a.num_tiles = b.n_tiles;
+    a.expert0 = moe.e0;
+    a.row_w = row_w;
+    a.glu = l->glu_f > 0 ? 1 : 0;
+    a.tables_fresh = tables_fresh ? 1 : 0;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(a.m_tiles * a.n_tiles);
+    cfg.blockDim = dim3(TS_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (a.pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    const cudaError_t e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, a)
+                                          : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, true>, map, a);
+    if (e != cudaSuccess) {
+        return cuda_fail("launch grouped gemm", e);
+    }
+    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "> (grouped)";
     launches++;
     return 0;
 }

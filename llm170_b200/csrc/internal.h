@@ -159,8 +159,9 @@ cudaError_t head_init_device();
 // ---- moe.cu ----------------------------------------------------------------------------------
 struct MoeBufs;
 void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, cudaStream_t st);
-// histogram -> offsets + m-tile table (tiles of `bm` rows) -> placement of the local experts' slots
-void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, cudaStream_t st);
+// histogram -> offsets + m-tile table (tiles of `bm` rows; `even`: of equal shares of at most bm rows) -> placement of the local
+// experts' slots
+void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, int even, cudaStream_t st);
 // the same tables as topk + align for at most 1024 slots, in one launch of one block
 int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm,
                             cudaStream_t st);

@@ -132,6 +132,15 @@ __device__ __forceinline__ void topk_of_token(const float* __restrict__ l, int* 
     }
 }
 
+// Rows per tile of an expert with c rows: `bm` of them, or (`even`) equal shares of at most bm, in multiples of 16 rows.
+__device__ __forceinline__ int tile_step(int c, int bm, int even) {
+    if (!even || c <= 0) {
+        return bm;
+    }
+    const int nt = (c + bm - 1) / bm;
+    return ((c + nt - 1) / nt + 15) & ~15;
+}
+
 __global__ void moe_topk_kernel(const float* __restrict__ lg, int* __restrict__ idx, float* __restrict__ wt, int t,
                                 int n, int k, int stage_rows) {
     extern __shared__ float s_stage[];   // [warps][n] when the launch provides it
@@ -251,12 +260,13 @@ __global__ void moe_count_kernel(const int* __restrict__ idx, int* __restrict__ 
 __global__ void moe_offsets_kernel(const int* __restrict__ cnt, int* __restrict__ off, int* __restrict__ cursor,
                                    int* __restrict__ tile_expert, int* __restrict__ tile_row0,
                                    int* __restrict__ tile_rows, int* __restrict__ n_tiles, int* __restrict__ n_rows,
-                                   int n_exp, int e0, int e1, int bm) {
+                                   int n_exp, int e0, int e1, int bm, int even) {
     __shared__ int s_rows[1024], s_tiles[1024];
     const int e = threadIdx.x;
     const int c = (e >= e0 && e < e1) ? cnt[e] : 0;
+    const int step = tile_step(c, bm, even);
     s_rows[e] = c;
-    s_tiles[e] = (c + bm - 1) / bm;
+    s_tiles[e] = (c + step - 1) / step;
     __syncthreads();
     for (int d = 1; d < 1024; d <<= 1) {   // inclusive Hillis-Steele scan of both arrays
         const int r = e >= d ? s_rows[e - d] : 0, t = e >= d ? s_tiles[e - d] : 0;
@@ -265,15 +275,15 @@ __global__ void moe_offsets_kernel(const int* __restrict__ cnt, int* __restrict_
         s_tiles[e] += t;
         __syncthreads();
     }
-    const int row0 = s_rows[e] - c, tile0 = s_tiles[e] - (c + bm - 1) / bm;
+    const int row0 = s_rows[e] - c, tile0 = s_tiles[e] - (c + step - 1) / step;
     if (e < n_exp) {
         off[e] = row0;
         cursor[e] = 0;
     }
-    for (int r = 0, i = tile0; r < c; r += bm, ++i) {
+    for (int r = 0, i = tile0; r < c; r += step, ++i) {
         tile_expert[i] = e;
         tile_row0[i] = row0 + r;
-        tile_rows[i] = min(bm, c - r);
+        tile_rows[i] = min(step, c - r);
     }
     if (e == 1023) {
         *n_tiles = s_tiles[e];
@@ -424,11 +434,11 @@ int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_e
     return own_topk ? 1 : 2;
 }
 
-void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, cudaStream_t st) {
+void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, int even, cudaStream_t st) {
     cudaMemsetAsync(b.cnt, 0, (size_t)n_exp * sizeof(int), st);
     moe_count_kernel<<<blocks_for(ns, 256), 256, 0, st>>>(b.idx, b.cnt, ns, e0, e1);
     moe_offsets_kernel<<<1, 1024, 0, st>>>(b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles,
-                                          b.n_rows, n_exp, e0, e1, bm);
+                                          b.n_rows, n_exp, e0, e1, bm, even);
     moe_place_kernel<<<blocks_for(ns, 256), 256, 0, st>>>(b.idx, b.wt, b.off, b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w,
                                                           ns, e0, e1);
 }

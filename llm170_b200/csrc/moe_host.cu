@@ -2,6 +2,7 @@
 // Mirrors W4a16Dec::set_moe / upload_experts_resident_streamed / build_marlin_moe_arenas
 // (crates/backend-gpu/src/rawcuda/w4a16_dec/upload.rs:795-812,1021-1235) and moe_ffn_dev_t
 // (crates/backend-gpu/src/rawcuda/w4a16_dec/moe/mod.rs:263-447).
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -12,8 +13,6 @@
 namespace w4 {
 
 namespace {
-constexpr int MOE_BM = 128;  // rows per m-tile of the grouped GEMM (256 when experts get enough rows)
-
 std::string w13_name(int layer) { return "\x01moe." + std::to_string(layer) + ".w13"; }
 std::string w2_name(int layer) { return "\x01moe." + std::to_string(layer) + ".w2"; }
 
@@ -121,7 +120,7 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             }
         } else {
             launch_moe_topk(logits, mb.idx, mb.wt, t, moe.n_experts, moe.top_k, st);
-            launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, 8, st);
+            launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, 8, 0, st);
             launch_moe_gather(x16, mb, ns, moe.top_k, moe.hidden, st);
             launches += 5;
             if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, nullptr, st)) {
@@ -133,18 +132,32 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             return rc;
         }
     } else {
-        // 256-row tiles (two accumulators per CTA) once the average expert segment fills most of one
-        const int bm = ((long long)ns * 4 >= (long long)moe.n_experts * 3 * 256) ? 256 : MOE_BM;
-        const int max_tiles = (ns + bm - 1) / bm + n_local;
+        // Experts with fewer than 192 rows on average: weight-row tiles of up to 128 rows, an expert's rows in equal shares, padded
+        // to 16; above that 256-row token tiles.  128 experts, top-8, 2048 x 768, groups of 32, us per layer, weight-row / token
+        // tiles: 192 tokens (12 rows per expert) 179 / 275, 1024 tokens 226 / 291, 2000 tokens 327 / 388, 3000 tokens (188 rows)
+        // 452 / 530, 4096 tokens (256 rows) 574 / 505; 64 experts, top-6, 2048 x 1024: 2000 tokens (188 rows) 284 / 337, 3000
+        // tokens (281 rows) 408 / 394.
+        const bool weight_rows = (long long)ns < 192LL * moe.n_experts;
+        const int bm = weight_rows ? 128 : 256;
+        const int max_tiles = (ns + bm - 1) / bm + std::min(ns, n_local);
         launch_moe_topk(logits, mb.idx, mb.wt, t, moe.n_experts, moe.top_k, st);
         launches += 5;
-        launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, bm, st);
+        launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, bm, weight_rows, st);
         launch_moe_gather(x16, mb, ns, moe.top_k, moe.hidden, st);
-        if (int rc = gemm_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, bm / 128, nullptr, st)) {
-            return rc;
-        }
-        if (int rc = gemm_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, bm / 128, mb.row_w, st)) {
-            return rc;
+        if (weight_rows) {
+            if (int rc = gemm_ts_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, bm, nullptr, st, true)) {
+                return rc;
+            }
+            if (int rc = gemm_ts_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, bm, mb.row_w, st, false)) {
+                return rc;
+            }
+        } else {
+            if (int rc = gemm_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, nullptr, st)) {
+                return rc;
+            }
+            if (int rc = gemm_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, mb.row_w, st)) {
+                return rc;
+            }
         }
     }
     launch_moe_combine(mb, y, t, moe.hidden, moe.top_k, out_kind == W4A16_OUT_F16, st);

@@ -178,3 +178,30 @@ def test_topk_near_ties_order_on_normalised_probabilities(dec, orc):
         want = orc.select_topk(lg[i], k)
         assert [e for e, _ in want] == idx[i].tolist(), i
         assert np.allclose([w for _, w in want], wt[i], rtol=0, atol=2e-7)
+
+
+# prefill-sized batches below 192 rows per expert: weight-row tiles (gemm_ts.cu) over equal shares of an expert's rows
+@pytest.mark.parametrize("t,n_exp,k,f,h,group,local,kernel", [
+    (65, 16, 2, 64, 64, 32, 16, "gemm_ts"),        # just above the GEMV's rows; one 64-channel block, one stage, a half tile
+    (520, 8, 2, 320, 576, 32, 8, "gemm_ts"),       # odd numbers of k-blocks, last tiles of 64 rows, two shares per expert
+    (300, 4, 2, 192, 448, 64, 2, "gemm_ts"),       # half of the experts elsewhere; groups of 64
+    (767, 8, 2, 128, 256, 128, 8, "gemm_ts"),      # the last batch below the line ...
+    (768, 8, 2, 128, 256, 128, 8, "gemm_w4a16_tc"),   # ... and the first above it
+])
+def test_expert_tiles_at_the_edges(dec, orc, t, n_exp, k, f, h, group, local, kernel):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=7 + t)
+    x, lg = synth.make_acts(t, h, seed=11 + t), synth.make_router_logits(t, n_exp, seed=13 + t)
+    lg[: t // 2, 0] += 4.0                          # one expert with far more rows than the others
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    total = 0
+    for e0 in range(0, n_exp, local):
+        dec.set_moe(n_exp, k, f, h, group, e0, local)
+        mine = slice(e0, e0 + local)
+        dec.upload_experts(0, w13_q[mine], w13_s[mine], w2_q[mine], w2_s[mine])
+        y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+        assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        assert dec.last_kernel().startswith(kernel)
+        total = total + y.cpu().numpy()
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
+    err = np.abs(total - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the test above
