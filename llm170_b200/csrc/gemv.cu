@@ -219,7 +219,7 @@ gemv_w4a16_kernel(const GemvArgs a, const SmemPlan p) {
     };
     const bool is_producer = warp == CONS_WARPS;
     if (is_producer) {
-        if (p.sc_staged) {
+        if (p.sc_staged && a.grouped) {
             // this CTA's scale pairs, [row block][group][8]: one bulk copy per row block (contiguous along K), requested
             // first so that nothing queues in front of them; like the weights they do not depend on the previous kernel
             const int ng_all = a.k / GROUP;
@@ -236,6 +236,23 @@ gemv_w4a16_kernel(const GemvArgs a, const SmemPlan p) {
         if (lane == 0) {
             for (int c = 0; c < S && c < nchunks; ++c) {
                 issue_chunk(c, c);
+            }
+        }
+    } else if (p.sc_staged && !a.grouped) {
+        // This warp's scale pairs, [row block][group][8], contiguous along K; like the weights they do not depend on the
+        // previous kernel.  Asynchronous 16-byte copies of the consumers, and not a bulk copy per row block: the copy engine
+        // takes about 60 ns for each, however small, and the weights queue behind them.
+        const int ng_all = a.k / GROUP;
+        const size_t grp_first = (size_t)kb0 * GROUPS_PER_KB / KB_PER_GROUP;
+#pragma unroll
+        for (int r = 0; r < RB_PER_WARP; ++r) {
+            const int rb = warp * RB_PER_WARP + r;
+            if (rb < nrbv) {
+                const uint32_t* src = sg.st + ((size_t)(rb_w0 + rb) * ng_all + grp_first) * 8;
+                const uint32_t dst = sbase + p.off_sc + (uint32_t)(rb * ngl * 32);
+                for (int i = lane; i < 2 * ngl; i += 32) {
+                    cp_async_16(dst + (uint32_t)i * 16u, src + i * 4);
+                }
             }
         }
     }
@@ -290,9 +307,10 @@ gemv_w4a16_kernel(const GemvArgs a, const SmemPlan p) {
     bool ok = true;
     if (!is_producer) {
         ok = mbar_wait(xbar, 0, abort_flag, a.status, (10 << 16));
-        if (ok && p.sc_staged) {
+        if (ok && p.sc_staged && a.grouped) {
             ok = mbar_wait(scbar, 0, abort_flag, a.status, (14 << 16));
         }
+        cp_async_wait_all();      // the scales of a dense call
         if (stamp && threadIdx.x == 0) {
             stamp_now(2);   // x and scales in shared memory
         }

@@ -72,7 +72,7 @@ SkPlan sk_make_plan(int k, int group, int m, int rows, int sm_count, int max_sta
         off += nu * gpu * CTA_RB * 32;
         off = (off + 1023) & ~1023;
         p.off_ring = off;
-        const int room = SK_SMEM_MAX - off - (2 + 2 * SK_MAX_STAGES) * 8;
+        const int room = SK_SMEM_MAX - off - (1 + 2 * SK_MAX_STAGES) * 8;
         int stages = room / STAGE_BYTES;
         if (stages >= 2 || nu == 1) {
             if (stages > max_stages) {
@@ -83,7 +83,7 @@ SkPlan sk_make_plan(int k, int group, int m, int rows, int sm_count, int max_sta
             }
             p.stages = stages;
             p.off_bars = off + stages * STAGE_BYTES;
-            p.total = p.off_bars + (2 + 2 * stages) * 8;
+            p.total = p.off_bars + (1 + 2 * stages) * 8;
             break;
         }
         // too long a range for the staging area: more, shorter ranges (more CTAs than SM slots)
@@ -170,7 +170,6 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
         s_abort = 0;
         s_last[0] = s_last[1] = 0;
         mbar_init(xbar, 1);
-        mbar_init(xbar + 8u + 16u * S, 1);   // scbar
         for (int s = 0; s < S; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), SK_CONS_WARPS);
@@ -225,42 +224,34 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
         }
     };
     const bool is_producer = warp == SK_CONS_WARPS;
-    const uint32_t scbar = xbar + 8u + 16u * S;
     Cursor pq;
     int pj = 0;   // next unit to issue
-    if (is_producer) {
-        // This CTA's scale pairs, [row block][local group][8 words]: one bulk copy per row block and run of
-        // units inside a row of row blocks, requested first so that nothing queues in front of them.  Like the
-        // weights they do not depend on the previous kernel of the stream.
-        if (lane == 0) {
-            uint32_t total = 0;
-            for (int j = 0, c = c0, rg = rg0; j < nu; ++rg) {
-                const int run = min(nu - j, C - c);
-                GemvSeg sg;
-                int r, nrbv;
-                row_info(rg, sg, r, nrbv);
-                total += (uint32_t)(min(run * GPU_, ng - c * GPU_) * 32 * nrbv);
-                j += run;
-                c = 0;
-            }
-            mbar_expect_tx(scbar, total);
-        }
-        __syncwarp();
-        if (lane < CTA_RB) {
-            for (int j = 0, c = c0, rg = rg0; j < nu; ++rg) {
-                const int run = min(nu - j, C - c);
-                GemvSeg sg;
-                int r, nrbv;
-                row_info(rg, sg, r, nrbv);
-                if (lane < nrbv) {
-                    bulk_load(sbase + p.off_sc + (uint32_t)(lane * p.nu_max + j) * (GPU_ * 32),
-                              sg.st + ((size_t)(r * CTA_RB + lane) * ng + (size_t)c * GPU_) * 8,
-                              (uint32_t)min(run * GPU_, ng - c * GPU_) * 32u, scbar);
+    if (!is_producer) {
+        // This warp's scale pairs, [row block][local group][8 words]; like the weights they do not depend on the previous kernel
+        // of the stream.  Asynchronous 16-byte copies of the consumers, and not a bulk copy per row block and run: the copy engine
+        // takes about 60 ns for each, however small, and the weights of both CTAs of the SM queue behind them (a CTA that came late
+        // needed 2.7 us from its entry to its x).
+        for (int j = 0, c = c0, rg = rg0; j < nu; ++rg) {
+            const int run = min(nu - j, C - c);
+            GemvSeg sg;
+            int r, nrbv;
+            row_info(rg, sg, r, nrbv);
+            const int pieces = 2 * min(run * GPU_, ng - c * GPU_);
+#pragma unroll
+            for (int b = 0; b < RBW; ++b) {
+                const int rb = warp * RBW + b;
+                if (rb < nrbv) {
+                    const uint32_t* src = sg.st + ((size_t)(r * CTA_RB + rb) * ng + (size_t)c * GPU_) * 8;
+                    const uint32_t dst = sbase + p.off_sc + (uint32_t)(rb * p.nu_max + j) * (GPU_ * 32);
+                    for (int i = lane; i < pieces; i += 32) {
+                        cp_async_16(dst + (uint32_t)i * 16u, src + i * 4);
+                    }
                 }
-                j += run;
-                c = 0;
             }
+            j += run;
+            c = 0;
         }
+    } else {
         if (lane == 0) {
             cursor_init(pq);
             // before the previous kernel of the stream is complete only `prefetch` stages are requested: its last
@@ -325,7 +316,7 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
     } else {
         // ------------------------------------------------------------------ consumers
         bool ok = mbar_wait(xbar, 0, abort_flag, a.status, (10 << 16));
-        ok = ok && mbar_wait(scbar, 0, abort_flag, a.status, (14 << 16));
+        cp_async_wait_all();
         if (stamp && threadIdx.x == 0) {
             stamp_now(2);
         }
@@ -591,21 +582,22 @@ gemv_sk_kernel(const GemvArgs a, const SkPlan p) {
     int prow[2];
     prow[0] = (c0 == 0 && u1 >= (rg0 + 1) * C) ? -1 : rg0;
     prow[1] = (rg_last != rg0 && u1 != (rg_last + 1) * C) ? rg_last : -1;
-    __threadfence();
     __syncthreads();
     if (stamp && threadIdx.x == 0) {
-        stamp_now(8);   // partial sums visible
+        stamp_now(8);   // partial sums written
     }
-    if (threadIdx.x == 0 && !*abort_flag) {
-        for (int sl = 0; sl < 2; ++sl) {
-            if (prow[sl] >= 0) {
-                const unsigned ub = (unsigned)(prow[sl] * C);
-                const int ncontrib = sk_owner(U, P, ub + C - 1) - sk_owner(U, P, ub) + 1;
-                const unsigned ticket = atomicAdd(a.counters + prow[sl], 1u);
-                s_last[sl] = ticket == (unsigned)ncontrib - 1u;
-            }
+    if ((threadIdx.x == 0 || threadIdx.x == 32) && !*abort_flag) {
+        // Both tickets at once, each taken by one thread with release and acquire order at GPU scope: the barriers around carry
+        // the order to the sums of the other threads, so no thread needs a fence of its own.
+        const int sl = (int)threadIdx.x >> 5;
+        const int rg = sl ? prow[1] : prow[0];
+        if (rg >= 0) {
+            const unsigned ub = (unsigned)(rg * C);
+            const int ncontrib = sk_owner(U, P, ub + C - 1) - sk_owner(U, P, ub) + 1;
+            unsigned ticket;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(a.counters + rg) : "memory");
+            s_last[sl] = ticket == (unsigned)ncontrib - 1u;
         }
-        __threadfence();   // the parked sums of the earlier contributors, ordered after the tickets
     }
     __syncthreads();
     if (stamp && threadIdx.x == 0) {
