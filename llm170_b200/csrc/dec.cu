@@ -337,14 +337,11 @@ int Dec::gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, 
 // w4a16_gemv_experts_* kernels (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:317-374,
 // crates/backend-gpu/src/rawcuda/w4a16_dec/moe/moe_gemv.rs:92-114).
 int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
-                      int est_tiles, const float* row_w, cudaStream_t st, const int* x_slot_of_pos,
+                      int est_tiles, int est_segments, const float* row_w, cudaStream_t st, const int* x_slot_of_pos,
                       int x_slots_per_token, bool tables_fresh) {
     if (l->glu_f > 0 && tune_gemv_warps != 8) {
         return fail("w4a16 grouped gemv: the fused gate|up form needs gemv_warps = 8");
     }
-    // eight staged token rows leave little room: with a two-stage ring the scales still fit in shared memory
-    // and three CTAs share an SM (measured: 177 -> 147 us for 64 tokens of the 128-expert layer)
-    const int grouped_stages = 2;
     GemvArgs a{};
     a.nseg = 1;
     a.k = l->k;
@@ -357,6 +354,39 @@ int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert,
     a.m = GEMV_MAX_M;            // sizes the staging area; each segment brings its own row count
     a.out_f16 = 1;
     a.x = (const uint16_t*)xs;
+    a.subnormal = tune_gemv_subnormal;
+    a.pdl = tune_pdl;
+    a.glu = l->glu_f > 0 ? 1 : 0;
+    a.status = gemm_status;
+    a.grouped = 1;
+    a.expert0 = moe.e0;
+    a.tile_expert = b.tile_expert;
+    a.tile_row0 = b.tile_row0;
+    a.tile_rows = b.tile_rows;
+    a.num_tiles = b.n_tiles;
+    a.row_w = row_w;
+    a.x_slot_of_pos = x_slot_of_pos;
+    a.x_slots_per_token = x_slots_per_token;
+    a.tables_fresh = tables_fresh ? 1 : 0;
+    a.nrb_w = l->n / TILE_ROWS;
+    a.tp = TpComm{};
+    cudaError_t e;
+    // The form with four row blocks per warp (gemv_moe.cu) wherever eight rows of x fit beside its rings (K up to about 10000);
+    // the (row block, K split) form stages K / ksplit of them and takes any K.
+    MoeGemvPlan gp{};
+    if (tune_moe_gemv != 1 && tune_gemv_subnormal && tune_gemv_ksplit == 0 &&
+        moe_gemv_plan(n_per_expert, a.k, a.group, sm_count, est_segments, tune_moe_gemv, gp)) {
+        e = launch_gemv_moe(a, gp, st);
+        if (e != cudaSuccess) {
+            return cuda_fail("launch grouped gemv", e);
+        }
+        last_kernel = "gemv_moe_kernel<" + std::to_string(a.group) + "," + std::to_string(gp.kw) + ">";
+        launches++;
+        return 0;
+    }
+    // eight staged token rows leave little room: with a two-stage ring the scales still fit in shared memory
+    // and three CTAs share an SM (measured: 177 -> 147 us for 64 tokens of the 128-expert layer)
+    const int grouped_stages = 2;
     const int cps = gemv_plan_ctas(a);  // CTAs per segment (256 rows each)
     const int grid_x = cps * max_tiles;
     int ks = tune_gemv_ksplit > 0 ? tune_gemv_ksplit
@@ -372,31 +402,15 @@ int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert,
         return fail("w4a16 grouped gemv: k=%d too large", a.k);
     }
     a.ksplit = ks;
-    a.subnormal = tune_gemv_subnormal;
-    a.pdl = tune_pdl;
-    a.glu = l->glu_f > 0 ? 1 : 0;
     a.ring_stages = grouped_stages;
     a.cons_warps = tune_gemv_warps;
     a.cluster = ks >= 2 ? 1 : 0;
-    a.status = gemm_status;
     a.dbg = dbg_buf;
     a.dbg_seq = (int)(launches % DBG_LAUNCHES);
-    a.grouped = 1;
     a.ctas_per_seg = cps;
-    a.expert0 = moe.e0;
-    a.tile_expert = b.tile_expert;
-    a.tile_row0 = b.tile_row0;
-    a.tile_rows = b.tile_rows;
-    a.num_tiles = b.n_tiles;
-    a.row_w = row_w;
-    a.x_slot_of_pos = x_slot_of_pos;
-    a.x_slots_per_token = x_slots_per_token;
-    a.tables_fresh = tables_fresh ? 1 : 0;
-    a.nrb_w = l->n / TILE_ROWS;
-    a.tp = TpComm{};
     a.part = part;
     a.counters = counters;
-    cudaError_t e = launch_gemv(a, grid_x, st);
+    e = launch_gemv(a, grid_x, st);
     if (e != cudaSuccess) {
         return cuda_fail("launch grouped gemv", e);
     }
@@ -473,6 +487,9 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
         }
         if (e == cudaSuccess) {
             e = w4::gemv_rb_init_device();
+        }
+        if (e == cudaSuccess) {
+            e = w4::gemv_moe_init_device();
         }
     }
     if (e == cudaSuccess) {
@@ -622,6 +639,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
     Dec& d = dec->d;
     if (!strcmp(key, "gemv_rowblock_units")) {
         d.tune_gemv_rowblock_units = value ? 1 : 0;
+        return 0;
+    }
+    if (!strcmp(key, "moe_gemv")) {
+        if (value != 0 && value != 1 && value != 2 && value != 4 && value != 8) {
+            return d.fail("w4a16 set_tuning: moe_gemv=%d (0, 1, 2, 4 or 8)", value);
+        }
+        d.tune_moe_gemv = value;
         return 0;
     }
     if (!strcmp(key, "gemv_stages")) {

@@ -97,6 +97,7 @@ struct Dec {
     int tune_gemv_persistent = 1;  // dense decode GEMV as two persistent CTAs per SM with equal unit ranges (gemv_sk.cu)
     int tune_gemv_cluster = 1;   // K splits of a row block as a thread-block cluster (DSMEM reduce) when 2 <= ksplit <= 8
     int tune_gemv_subnormal = 1;
+    int tune_moe_gemv = 0;       // MoE decode: 0 = automatic, 1 = (row block, K split) form, 2 / 4 / 8 = warps along K of gemv_moe.cu
     int tune_pdl = 1;
     int tune_tp_wait_log2 = 31;  // the fused all-reduce gives up on its peers after 2^this cycles
     int tune_gemm_mt = 0;        // 128-token blocks per GEMM tile: 0 = automatic, 1 or 2
@@ -141,7 +142,7 @@ struct Dec {
     void* tp_peer[TP_MAX_WORLD] = {};
     int tp_max_rows = 0;
     int gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
-                     int est_tiles, const float* row_w, cudaStream_t st, const int* x_slot_of_pos = nullptr,
+                     int est_tiles, int est_segments, const float* row_w, cudaStream_t st, const int* x_slot_of_pos = nullptr,
                      int x_slots_per_token = 1, bool tables_fresh = false);
     MoeCfg moe;
     MoeBufs mb;

@@ -1,0 +1,398 @@
+// Decode-time grouped GEMV of the MoE path: every segment of at most eight sorted rows is multiplied with its expert's rows.
+//
+// Takes the place of the reference's w4a16_gemv_experts_* kernels (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:317-374,
+// crates/backend-gpu/src/rawcuda/w4a16_dec/moe/moe_gemv.rs:92-114).  Same arithmetic as the other decode forms: mma.sync m16n8k16
+// with the weight tile as the 16-row operand, raw nibbles as exact f16 subnormals, f32 sums, the f32 group scale on a group's sum.
+//
+// Bound by issued instructions: 32-channel groups leave two scale folds per 512-byte tile, and the (row block, K split) form
+// spent 84 warp instructions per tile (22 us per 256-row CTA of 128 experts x 1536 x 2048, 17.5 of them in its loop).  Here
+//   * a warp multiplies four row blocks with the same activations, so their loads and the zero-point term are shared by four
+//     tiles, and four independent chains hide the latency of the MMAs;
+//   * the zero-point term of a group, -8 * sum(x), is the sum of two MMAs whose A operand is the constant -8 in the nibbles' own
+//     scalings, and opens the chains of the four row blocks as their C operand: no pass over x, no table of sums, no add;
+//   * the CTAs are persistent (two per SM) and take equal contiguous runs of (segment, 128 or 256 rows) units: the weights of the
+//     next unit are on the way while the last one is summed, and the activations stay in shared memory for a segment's units;
+//   * every warp streams its own tiles into its own ring with asynchronous copies: no producer, no barrier in the loop.
+#include <cuda_fp16.h>
+
+#include "gemv_common.cuh"
+
+namespace w4 {
+
+namespace {
+
+constexpr int GM_WARPS = 8;
+constexpr int GM_THREADS = GM_WARPS * 32;
+constexpr int GM_NR = 4;                                      // row blocks per warp
+constexpr int D = 2;                                          // ring slots per warp (3 and 4 measured the same)
+constexpr int GM_W_BYTES = GM_NR * TILE_WORDS * 4;            // weights of a slot: one k-block
+constexpr int GM_SMEM_MAX = 224 * 1024;
+__host__ __device__ constexpr int gm_slot(int group) { return GM_W_BYTES + GM_NR * 32 * (group == 32 ? 2 : 1); }
+
+// KW = warps along K; the other warps of a CTA take further row blocks.
+template <int GROUP, int KW>
+__global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs a, const MoeGemvPlan p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_xbar;
+    __shared__ int s_abort;
+    constexpr int RW = GM_WARPS / KW, UR = RW * GM_NR;        // row blocks of a unit
+    constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
+    constexpr uint32_t SLOT = gm_slot(GROUP);
+    if (a.tables_fresh) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int kw = warp % KW, rw = warp / KW;
+    const int nrb = a.seg[0].n / TILE_ROWS, upe = (nrb + UR - 1) / UR;
+    const int units = *a.num_tiles * upe;
+    const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+    if (u0 >= u1) {
+        return;
+    }
+    const int ku = a.k / (TILE_K * KPU), ng = a.k / GROUP;
+    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks
+    const size_t pitch = (size_t)a.nrb_w * 32;                // uint4 between k-blocks
+
+    // ---- weights and scales: slots of one k-block of the warp's row blocks, requested in the order of use.  Row blocks past the
+    // expert's last one read that one again.
+    const uint32_t ring = smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * SLOT);
+    int fu = u0, fi = 0;
+    int fexp = a.tile_expert[u0 / upe];                       // expert of unit fu
+    const uint4* fq = nullptr;
+    const uint32_t* fs = nullptr;
+    int fstep[GM_NR];                                         // offset of the warp's r-th row block
+    auto fetch_unit = [&]() {
+        const int sub = fu % upe, rb = sub * UR + rw * GM_NR, base = (fexp - a.expert0) * nrb;
+#pragma unroll
+        for (int r = 0; r < GM_NR; ++r) {
+            fstep[r] = (base + min(rb + r, nrb - 1)) * 32;
+        }
+        fq = a.seg[0].qt + (size_t)kb0 * pitch + lane;
+        // scale words: 16 bytes per lane; row block lane / (pieces per slot)
+        constexpr int SP = GROUP == 32 ? 4 : 2;
+        fs = a.seg[0].st + (size_t)(base + min(rb + lane / SP % GM_NR, nrb - 1)) * ng * 8 + (size_t)kb0 * TILE_K / GROUP * 8 + (lane % SP) * 4;
+        fi = 0;
+        if (fu + 1 < u1) {
+            fexp = a.tile_expert[(fu + 1) / upe];
+        }
+    };
+    uint32_t fdst = 0;
+    auto fetch = [&]() {
+        if (fu < u1) {
+            const uint32_t dst = ring + fdst;
+#pragma unroll
+            for (int r = 0; r < GM_NR; ++r) {
+                cp_async_16(dst + (uint32_t)r * 512u + (uint32_t)lane * 16u, fq + fstep[r]);
+            }
+            if (GROUP == 32) {
+                if (lane < 4 * GM_NR) {
+                    cp_async_16(dst + GM_W_BYTES + (uint32_t)lane * 16u, fs);
+                }
+                fs += 16;
+            } else if (fi & 1) {                              // with a group's second k-block, after which it is needed
+                if (lane < 2 * GM_NR) {
+                    cp_async_16(dst + GM_W_BYTES + (uint32_t)lane * 16u, fs);
+                }
+                fs += 8;
+            }
+            fq += pitch;
+            if (++fi == nk) {
+                if (++fu < u1) {
+                    fetch_unit();
+                }
+            }
+        }
+        cp_async_commit();
+        if ((fdst += SLOT) == D * SLOT) {
+            fdst = 0;
+        }
+    };
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        mbar_init(smem_u32(&s_xbar), 1);
+        mbar_init_fence();
+    }
+    if (nk > 0) {
+        fetch_unit();
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            fetch();
+        }
+    }
+    if (!a.tables_fresh) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    // the next kernel may come: what it reads before its own wait was complete before this launch
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    const int xstride = a.k * 2 + 32;                         // bytes; 32 mod 128: conflict-free 8-byte reads of eight rows
+    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][8 tokens]
+    const uint32_t wl = ring + (uint32_t)lane * 16u;
+    const uint32_t zA[4] = {0x80088008u, 0x80808080u, 0x80088008u, 0x80808080u};   // -8 in the nibbles' two scalings
+    uint32_t rslot = 0, xphase = 0;
+    int seg = -1, row0 = 0, m = 0;
+    uint32_t xl = 0;
+    for (int u = u0; u < u1; ++u) {
+        if (u / upe != seg) {
+            // ---- another segment: its rows' activations
+            seg = u / upe;
+            row0 = a.tile_row0[seg];
+            m = a.tile_rows[seg];
+            __syncthreads();                                  // (and the barrier word is initialised)
+            if (warp == 0) {
+                if (lane == 0) {
+                    mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * a.k * 2));
+                }
+                __syncwarp();
+                if (lane < m) {
+                    const int row = a.x_slot_of_pos != nullptr ? a.x_slot_of_pos[row0 + lane] / a.x_slots_per_token : row0 + lane;
+                    bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)row * a.k, (uint32_t)(a.k * 2), smem_u32(&s_xbar));
+                }
+            }
+            mbar_wait(smem_u32(&s_xbar), xphase, &s_abort, a.status, (42 << 16) | (seg & 0xffff));
+            xphase ^= 1;
+            __syncwarp();
+            // lanes without a token read token 0: their columns are never stored
+            xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
+        }
+        float tot[GM_NR][4], acc[GM_NR][4];
+#pragma unroll
+        for (int r = 0; r < GM_NR; ++r) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                tot[r][j] = acc[r][j] = 0.f;
+            }
+        }
+        uint32_t xa = xl;
+        auto fold = [&](int r, uint32_t s2) {
+            const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&s2));
+            tot[r][0] = fmaf(acc[r][0], sf.x, tot[r][0]);
+            tot[r][1] = fmaf(acc[r][1], sf.x, tot[r][1]);
+            tot[r][2] = fmaf(acc[r][2], sf.y, tot[r][2]);
+            tot[r][3] = fmaf(acc[r][3], sf.y, tot[r][3]);
+        };
+        if (GROUP == 32) {
+            for (int i = 0; i < nk; ++i) {
+                uint2 x[4];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    x[w] = lds64(xa + (uint32_t)w * 32u);
+                }
+                xa += TILE_K * 2;
+                cp_async_wait_group<D - 1>();
+                __syncwarp();                                 // the scale words are other lanes' copies
+                uint4 wv[GM_NR];
+                uint32_t sc[GM_NR][2];
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
+                    sc[r][0] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 64u + (uint32_t)g * 4u);
+                    sc[r][1] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 64u + 32u + (uint32_t)g * 4u);
+                }
+                __syncwarp();
+                fetch();
+                if ((rslot += SLOT) == D * SLOT) {
+                    rslot = 0;
+                }
+                float z0[4], z1[4];
+                mma16816_z(z0, zA, x[0].x, x[0].y);
+                mma16816_z(z1, zA, x[2].x, x[2].y);
+                mma16816(z0, zA, x[1].x, x[1].y);
+                mma16816(z1, zA, x[3].x, x[3].y);
+                const float4 c0 = make_float4(z0[0], z0[1], z0[2], z0[3]), c1 = make_float4(z1[0], z1[1], z1[2], z1[3]);
+                uint32_t af[4];
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    nibbles_as_subnormals(wv[r].x, af);
+                    mma16816_c(acc[r], af, x[0].x, x[0].y, c0);
+                }
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    nibbles_as_subnormals(wv[r].y, af);
+                    mma16816(acc[r], af, x[1].x, x[1].y);
+                }
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    fold(r, sc[r][0]);
+                    nibbles_as_subnormals(wv[r].z, af);
+                    mma16816_c(acc[r], af, x[2].x, x[2].y, c1);
+                }
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    nibbles_as_subnormals(wv[r].w, af);
+                    mma16816(acc[r], af, x[3].x, x[3].y);
+                }
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+                    fold(r, sc[r][1]);
+                }
+            }
+        } else {
+            for (int i = 0; i < nk; i += 2) {
+                float z[4];
+                uint32_t sc[GM_NR];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint2 x[4];
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        x[w] = lds64(xa + (uint32_t)w * 32u);
+                    }
+                    xa += TILE_K * 2;
+                    cp_async_wait_group<D - 1>();
+                    __syncwarp();
+                    uint4 wv[GM_NR];
+#pragma unroll
+                    for (int r = 0; r < GM_NR; ++r) {
+                        wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
+                        if (h == 1) {
+                            sc[r] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 32u + (uint32_t)g * 4u);
+                        }
+                    }
+                    __syncwarp();
+                    fetch();
+                    if ((rslot += SLOT) == D * SLOT) {
+                        rslot = 0;
+                    }
+                    uint32_t af[4];
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) {
+                        const bool open = h == 0 && w == 0;
+                        if (open) {
+                            mma16816_z(z, zA, x[w].x, x[w].y);
+                        } else {
+                            mma16816(z, zA, x[w].x, x[w].y);
+                        }
+#pragma unroll
+                        for (int r = 0; r < GM_NR; ++r) {
+                            nibbles_as_subnormals(w == 0 ? wv[r].x : w == 1 ? wv[r].y : w == 2 ? wv[r].z : wv[r].w, af);
+                            if (open) {
+                                mma16816_z(acc[r], af, x[w].x, x[w].y);
+                            } else {
+                                mma16816(acc[r], af, x[w].x, x[w].y);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < GM_NR; ++r) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[r][j] += z[j];
+                    }
+                    fold(r, sc[r]);
+                }
+            }
+        }
+        // ---- the K warps' sums meet in shared memory
+        const int rb0 = u % upe * UR, rows = min(UR, nrb - rb0) * TILE_ROWS;
+        if (u > u0) {
+            __syncthreads();
+        }
+        const float m0 = 16777216.f * a.seg[0].out_mul, m1 = 1048576.f * a.seg[0].out_mul;
+#pragma unroll
+        for (int r = 0; r < GM_NR; ++r) {
+            float* d = red + ((size_t)kw * (UR * TILE_ROWS) + (rw * GM_NR + r) * TILE_ROWS + g) * GEMV_MAX_M + 2 * t;
+            *reinterpret_cast<float2*>(d) = make_float2(tot[r][0] * m0, tot[r][1] * m0);
+            *reinterpret_cast<float2*>(d + 8 * GEMV_MAX_M) = make_float2(tot[r][2] * m1, tot[r][3] * m1);
+        }
+        __syncthreads();
+        auto sum_of = [&](int row, int tok) {
+            float v = red[row * GEMV_MAX_M + tok];
+#pragma unroll
+            for (int w = 1; w < KW; ++w) {
+                v += red[(w * (UR * TILE_ROWS) + row) * GEMV_MAX_M + tok];      // fixed order: the same bits every run
+            }
+            return v;
+        };
+        if (a.glu) {
+            // interleaved gate / up row blocks: output o of the unit has its gate sum in row 32 (o / 16) + o % 16, its up sum 16
+            // rows further
+            const int nout = rows / 2, nh = a.seg[0].n / 2;
+            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * nh + (size_t)rb0 * (TILE_ROWS / 2);
+            for (int e = threadIdx.x; e < nout * m; e += GM_THREADS) {
+                const int tok = e / nout, o = e - tok * nout;
+                const int lg = (o / TILE_ROWS) * 2 * TILE_ROWS + (o % TILE_ROWS);
+                ob[(size_t)tok * nh + o] = silu_mul_f16(sum_of(lg, tok), sum_of(lg + TILE_ROWS, tok));
+            }
+        } else {
+            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * a.seg[0].n + (size_t)rb0 * TILE_ROWS;
+            for (int e = threadIdx.x; e < rows * m; e += GM_THREADS) {
+                const int tok = e / rows, row = e - tok * rows;
+                float v = sum_of(row, tok);
+                if (a.row_w != nullptr) {
+                    v = mul_row_w(v, a.row_w[row0 + tok]);
+                }
+                ob[(size_t)tok * a.seg[0].n + row] = __float2half_rn(v);
+            }
+        }
+    }
+}
+
+const void* gm_kernel(int group, int kw) {
+    if (group == 128) {
+        return kw == 2 ? (const void*)gemv_moe_kernel<128, 2> : kw == 4 ? (const void*)gemv_moe_kernel<128, 4> : (const void*)gemv_moe_kernel<128, 8>;
+    }
+    return kw == 2 ? (const void*)gemv_moe_kernel<32, 2> : kw == 4 ? (const void*)gemv_moe_kernel<32, 4> : (const void*)gemv_moe_kernel<32, 8>;
+}
+
+}  // namespace
+
+// Plan of a call with about `segments` segments of `rows` rows per expert; false: eight rows of x do not fit in shared memory.
+// The fewer warps share K, the more rows has a unit and the fewer sums and barriers there are, but the fewer units; a unit costs about
+// as much as five k-blocks beside its own.  Both matmuls, us per layer with 2 / 4 / 8 warps along K, and in the (row block, K split)
+// form: 128 experts x 2048 x 768, groups of 32: 64 tokens 97 / 102 / 118, 125; 8 tokens 61 / 55 / 57, 71; 1 token 38 / 29 / 26, 32;
+// 64 experts x 1024 x 384: 64 tokens 32.8 / 35.9 / 38.6, 39.1; 128 experts x 1536 x 896: 4 tokens 28.9 / 25.8 / 28.8, 34.1.
+bool moe_gemv_plan(int rows, int k, int group, int sm_count, int segments, int force_kw, MoeGemvPlan& p) {
+    const int x = GEMV_MAX_M * (k * 2 + 32), red = GM_WARPS * GM_NR * TILE_ROWS * GEMV_MAX_M * 4;
+    p.off_red = (x + 127) & ~127;
+    p.off_ring = p.off_red + red;
+    p.smem = p.off_ring + D * GM_WARPS * gm_slot(group);
+    if (p.smem > GM_SMEM_MAX) {
+        return false;
+    }
+    p.ctas = (p.smem <= GM_SMEM_MAX / 2 ? 2 : 1) * sm_count;
+    long long best = -1;
+    for (int kw = 2; kw <= 8; kw *= 2) {
+        const int unit_rows = GM_WARPS / kw * GM_NR * TILE_ROWS;
+        const long long units = (long long)segments * ((rows + unit_rows - 1) / unit_rows);
+        const long long cost = (units + p.ctas - 1) / p.ctas * ((k / TILE_K + kw - 1) / kw + 5);
+        if (force_kw > 1 ? kw == force_kw : (best < 0 || cost < best)) {
+            best = cost;
+            p.kw = kw;
+        }
+    }
+    return true;
+}
+
+cudaError_t gemv_moe_init_device() {
+    for (int group : {128, 32}) {
+        for (int kw : {2, 4, 8}) {
+            const cudaError_t e = cudaFuncSetAttribute(gm_kernel(group, kw), cudaFuncAttributeMaxDynamicSharedMemorySize, GM_SMEM_MAX);
+            if (e != cudaSuccess) {
+                return e;
+            }
+        }
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_gemv_moe(const GemvArgs& a, const MoeGemvPlan& p, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.ctas);
+    cfg.blockDim = dim3(GM_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (a.pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    void* args[] = {const_cast<GemvArgs*>(&a), const_cast<MoeGemvPlan*>(&p)};
+    return cudaLaunchKernelExC(&cfg, gm_kernel(a.group, p.kw), args);
+}
+
+}  // namespace w4

@@ -142,6 +142,16 @@ size_t sk_part_floats(const SkPlan& p);   // scratch for parked partial sums; co
 cudaError_t launch_gemv_sk(const GemvArgs& a, const SkPlan& p, cudaStream_t st);
 cudaError_t gemv_sk_init_device();
 cudaError_t gemv_rb_init_device();
+// ---- gemv_moe.cu: grouped GEMV of the MoE decode path ----
+struct MoeGemvPlan {
+    int kw;                  // warps along K: 2, 4 or 8
+    int ctas;                // two per SM (one, where the activations leave no room)
+    int off_red, off_ring;   // byte offsets in dynamic shared memory: activations first
+    int smem;
+};
+bool moe_gemv_plan(int rows, int k, int group, int sm_count, int segments, int force_kw, MoeGemvPlan& p);
+cudaError_t launch_gemv_moe(const GemvArgs& a, const MoeGemvPlan& p, cudaStream_t st);
+cudaError_t gemv_moe_init_device();
 bool gemv_rb_fits(const GemvArgs& a);
 int gemv_rb_plan(GemvArgs& a, int sm_count, int& rbw);
 cudaError_t launch_gemv_rb(const GemvArgs& a, int total_units, int rbw, int sm_count, cudaStream_t st);

@@ -3,6 +3,7 @@
 // (crates/backend-gpu/src/rawcuda/w4a16_dec/upload.rs:795-812,1021-1235) and moe_ffn_dev_t
 // (crates/backend-gpu/src/rawcuda/w4a16_dec/moe/mod.rs:263-447).
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
@@ -108,13 +109,15 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         // this bound, and CTAs beyond the actual count leave at once
         const int est_tiles = ns < n_local ? ns : n_local;   // segments expected to be non-empty (split-K sizing)
         const int max_tiles = est_tiles + ns / 8;
+        // local experts that a batch of t tokens reaches on average
+        const int est_segments = (int)(n_local * (1.0 - pow(1.0 - (double)moe.top_k / moe.n_experts, t)) + 0.5);
         if (max_tiles > mb.max_tiles) {
             return fail("w4a16 moe_ffn: tile table too small");
         }
         if (ns <= 1024) {
             // routing and all dispatch tables in one launch; the first grouped GEMV fetches each row's token itself
             launches += launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, st);
-            if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, nullptr, st,
+            if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st,
                                       mb.slot_of_pos, moe.top_k, /*tables_fresh=*/true)) {
                 return rc;
             }
@@ -123,12 +126,12 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, 8, 0, st);
             launch_moe_gather(x16, mb, ns, moe.top_k, moe.hidden, st);
             launches += 5;
-            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, nullptr, st)) {
+            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st)) {
                 return rc;
             }
         }
         // silu(gate)*up is applied by the first grouped matmul (interleaved gate / up rows): no activation pass
-        if (int rc = gemv_grouped(&i2->second, mb.act, mb.c2, moe.hidden, mb, max_tiles, est_tiles, mb.row_w, st)) {
+        if (int rc = gemv_grouped(&i2->second, mb.act, mb.c2, moe.hidden, mb, max_tiles, est_tiles, est_segments, mb.row_w, st)) {
             return rc;
         }
     } else {

@@ -205,3 +205,28 @@ def test_expert_tiles_at_the_edges(dec, orc, t, n_exp, k, f, h, group, local, ke
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
     err = np.abs(total - want).max()
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the test above
+
+
+# the grouped GEMV: segments of up to eight rows, K of one to many ring rounds (and too short for all warps), row blocks that do not
+# fill a unit, every way of sharing K, and the form for activations that do not fit
+@pytest.mark.parametrize("way", [0, 1, 2, 4, 8])
+@pytest.mark.parametrize("t,n_exp,k,f,h,group", [(1, 8, 2, 64, 64, 32), (3, 4, 3, 320, 576, 32), (16, 16, 4, 192, 448, 64),
+                                                (20, 8, 2, 128, 640, 128), (140, 40, 2, 64, 320, 32)])
+def test_grouped_gemv_forms(dec, orc, t, n_exp, k, f, h, group, way):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=31 + t)
+    x, lg = synth.make_acts(t, h, seed=32 + t), synth.make_router_logits(t, n_exp, seed=33 + t)
+    if t > 8:
+        lg[:11, 1] += 6.0                               # one expert with more rows than a segment holds
+    dec.set_moe(n_exp, k, f, h, group)
+    dec.upload_experts(0, w13_q, w13_s, w2_q, w2_s)
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    dec.set_tuning("moe_gemv", way)
+    try:
+        y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+        assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+    finally:
+        dec.set_tuning("moe_gemv", 0)
+    assert dec.last_kernel().startswith("gemv_w4a16_kernel" if way == 1 else "gemv_moe_kernel")
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
+    err = np.abs(y.cpu().numpy() - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # as above
