@@ -168,15 +168,14 @@ cudaError_t head_init_device();
 
 // ---- moe.cu ----------------------------------------------------------------------------------
 struct MoeBufs;
-void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, cudaStream_t st);
-// histogram -> offsets + m-tile table (tiles of `bm` rows; `even`: of equal shares of at most bm rows) -> placement of the local
-// experts' slots
-void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, int even, cudaStream_t st);
-// the same tables as topk + align for at most 1024 slots, in one launch of one block
-int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm,
-                            cudaStream_t st);
-void launch_moe_gather(const void* x, const MoeBufs& b, int ns, int k, int h, cudaStream_t st);
-void launch_moe_act(const MoeBufs& b, int rows_upper, int ffn, cudaStream_t st);
-void launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, cudaStream_t st);
+// `pdl`: programmatic stream serialization.  `cnt` (optional): counts the rows of local experts [e0, e1) as well.
+void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl, cudaStream_t st);
+// routing and sorting of any batch: top-k and histogram -> offsets and m-tile table (tiles of `bm` rows; `even`: of equal shares of at
+// most bm rows) -> placement of the local experts' slots and gather of their token rows.  Returns the number of launches.
+int launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm, int even,
+                    int pdl, cudaStream_t st);
+// the same tables for at most 1024 slots, from one block, without the gather
+int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm, int pdl, cudaStream_t st);
+void launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, int pdl, cudaStream_t st);
 
 }  // namespace w4

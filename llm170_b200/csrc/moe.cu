@@ -19,6 +19,14 @@ namespace w4 {
 
 namespace {
 
+// Start of every kernel here.  They are small, and between two calls' matmuls their launches cost as much as their work: so they are
+// launched with programmatic stream serialization, let the next kernel come as soon as they run, and touch nothing before the kernel
+// before them is complete.  (In an ordinary launch both instructions do nothing.)
+__device__ __forceinline__ void pdl_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 constexpr int TOPK_WARPS = 8;
 
 // One warp per token, experts dealt to lanes round-robin (expert e lives in lane e % 32, slot e / 32).
@@ -34,7 +42,7 @@ constexpr int TOPK_WARPS = 8;
 // SLOTS = experts per lane the instantiation can hold (n <= 32 * SLOTS): a compile-time bound keeps the lane's values in
 // registers.
 template <int SLOTS>
-__device__ __forceinline__ void topk_of_token_n(const float* __restrict__ l, int* __restrict__ idx, float* __restrict__ wt,
+__device__ __forceinline__ void topk_of_token_n(const float* l, int* idx, float* wt,
                                                 int n, int k, int lane, float* stage) {
     float mx = -INFINITY;
     for (int i = lane; i < n; i += 32) {
@@ -121,7 +129,7 @@ __device__ __forceinline__ void topk_of_token_n(const float* __restrict__ l, int
     }
 }
 
-__device__ __forceinline__ void topk_of_token(const float* __restrict__ l, int* __restrict__ idx, float* __restrict__ wt,
+__device__ __forceinline__ void topk_of_token(const float* l, int* idx, float* wt,
                                               int n, int k, int lane, float* stage = nullptr) {
     if (n <= 128) {
         topk_of_token_n<4>(l, idx, wt, n, k, lane, stage);
@@ -141,9 +149,10 @@ __device__ __forceinline__ int tile_step(int c, int bm, int even) {
     return ((c + nt - 1) / nt + 15) & ~15;
 }
 
-__global__ void moe_topk_kernel(const float* __restrict__ lg, int* __restrict__ idx, float* __restrict__ wt, int t,
-                                int n, int k, int stage_rows) {
+// `cnt` (optional): rows per local expert; zero on entry, moe_offsets_kernel leaves it so.
+__global__ void moe_topk_kernel(const float* lg, int* idx, float* wt, int t, int n, int k, int stage_rows, int* cnt, int e0, int e1) {
     extern __shared__ float s_stage[];   // [warps][n] when the launch provides it
+    pdl_begin();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ti = blockIdx.x * TOPK_WARPS + w;
     if (ti >= t) {
@@ -151,22 +160,70 @@ __global__ void moe_topk_kernel(const float* __restrict__ lg, int* __restrict__ 
     }
     topk_of_token(lg + (size_t)ti * n, idx + (size_t)ti * k, wt + (size_t)ti * k, n, k, lane,
                   stage_rows ? s_stage + (size_t)w * n : nullptr);
+    if (cnt != nullptr) {
+        __syncwarp();
+        if (lane < k) {                                                  // k <= 32
+            const int e = idx[(size_t)ti * k + lane];
+            if (e >= e0 && e < e1) {
+                atomicAdd(cnt + e, 1);
+            }
+        }
+    }
+}
+
+// Inclusive scan of (rows, tiles) over the block's 1024 threads: shuffles inside a warp, then the 32 warp totals.
+__device__ __forceinline__ void scan_rows_tiles(int& vr, int& vt, int& total_rows, int& total_tiles, int* s_r, int* s_t) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int r = __shfl_up_sync(0xffffffffu, vr, d), tt = __shfl_up_sync(0xffffffffu, vt, d);
+        if (lane >= d) {
+            vr += r;
+            vt += tt;
+        }
+    }
+    if (lane == 31) {
+        s_r[w] = vr;
+        s_t[w] = vt;
+    }
+    __syncthreads();
+    if (w == 0) {
+        int tr = s_r[lane], tl = s_t[lane];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int r = __shfl_up_sync(0xffffffffu, tr, d), tt = __shfl_up_sync(0xffffffffu, tl, d);
+            if (lane >= d) {
+                tr += r;
+                tl += tt;
+            }
+        }
+        s_r[lane] = tr;    // inclusive totals of warps 0..lane
+        s_t[lane] = tl;
+    }
+    __syncthreads();
+    if (w > 0) {
+        vr += s_r[w - 1];
+        vt += s_t[w - 1];
+    }
+    total_rows = s_r[31];
+    total_tiles = s_t[31];
 }
 
 // Decode-sized batches (at most 1024 (token, expert) slots): routing, histogram, offsets, tile table, placement
 // and sorted routing weights in ONE block of 1024 threads -- the six launches they take otherwise cost more
 // than the expert matmuls of a single token.  Same tables as the separate kernels below.
 __global__ void __launch_bounds__(1024)
-moe_route_small_kernel(const float* __restrict__ lg, int* __restrict__ idx, float* __restrict__ wt,
-                       int* __restrict__ off, int* __restrict__ pos_of_slot, int* __restrict__ slot_of_pos,
-                       int* __restrict__ tile_expert, int* __restrict__ tile_row0, int* __restrict__ tile_rows,
-                       int* __restrict__ n_tiles, int* __restrict__ n_rows, float* __restrict__ row_w, int t, int n_exp,
+moe_route_small_kernel(const float* lg, int* idx, float* wt,
+                       int* off, int* pos_of_slot, int* slot_of_pos,
+                       int* tile_expert, int* tile_row0, int* tile_rows,
+                       int* n_tiles, int* n_rows, float* row_w, int t, int n_exp,
                        int k, int e0, int e1, int bm, int stage_rows, int do_topk) {
-    __shared__ int s_rows[1024], s_tiles[1024], s_off[1024], s_cursor[1024];
+    __shared__ int s_rows[1024], s_off[1024], s_cursor[1024], s_wr[32], s_wt[32];
     extern __shared__ float s_stage[];   // [32 warps][n_exp] when the launch provides it
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     s_rows[tid] = 0;
     s_cursor[tid] = 0;
+    pdl_begin();
     if (do_topk) {   // a handful of tokens: routed here; more: routed by moe_topk_kernel on many SMs just before
         for (int ti = w; ti < t; ti += 32) {
             topk_of_token(lg + (size_t)ti * n_exp, idx + (size_t)ti * k, wt + (size_t)ti * k, n_exp, k, lane,
@@ -185,41 +242,11 @@ moe_route_small_kernel(const float* __restrict__ lg, int* __restrict__ idx, floa
         }
     }
     __syncthreads();
-    // inclusive scan of (rows, tiles) over the 1024 experts slots: shuffles inside a warp, then the 32 warp totals
     const int c = s_rows[tid];
     const int ct = (c + bm - 1) / bm;
-    int vr = c, vt = ct;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int r = __shfl_up_sync(0xffffffffu, vr, d), tt = __shfl_up_sync(0xffffffffu, vt, d);
-        if (lane >= d) {
-            vr += r;
-            vt += tt;
-        }
-    }
-    __syncthreads();          // every thread has read its s_rows entry
-    if (lane == 31) {
-        s_rows[w] = vr;       // warp totals reuse the first 32 entries
-        s_tiles[w] = vt;
-    }
-    __syncthreads();
-    if (w == 0) {
-        int tr = s_rows[lane], tl = s_tiles[lane];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int r = __shfl_up_sync(0xffffffffu, tr, d), tt = __shfl_up_sync(0xffffffffu, tl, d);
-            if (lane >= d) {
-                tr += r;
-                tl += tt;
-            }
-        }
-        s_rows[lane] = tr;    // inclusive totals of warps 0..lane
-        s_tiles[lane] = tl;
-    }
-    __syncthreads();
-    const int base_r = w > 0 ? s_rows[w - 1] : 0, base_t = w > 0 ? s_tiles[w - 1] : 0;
-    const int row0 = base_r + vr - c, tile0 = base_t + vt - ct;
-    const int total_rows = s_rows[31], total_tiles = s_tiles[31];
+    int vr = c, vt = ct, total_rows, total_tiles;
+    scan_rows_tiles(vr, vt, total_rows, total_tiles, s_wr, s_wt);
+    const int row0 = vr - c, tile0 = vt - ct;
     s_off[tid] = row0;
     if (tid < n_exp) {
         off[tid] = row0;
@@ -245,40 +272,24 @@ moe_route_small_kernel(const float* __restrict__ lg, int* __restrict__ idx, floa
     }
 }
 
-__global__ void moe_count_kernel(const int* __restrict__ idx, int* __restrict__ cnt, int ns, int e0, int e1) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += gridDim.x * blockDim.x) {
-        const int e = idx[i];
-        if (e >= e0 && e < e1) {
-            atomicAdd(cnt + e, 1);
-        }
-    }
-}
-
 // One block of 1024 threads (n_exp <= 1024): exclusive offsets of the local experts' segments and the m-tile
-// table of the grouped GEMM, tile i -> (expert, first sorted row, valid rows), both by a shared-memory scan.
-// Also clears the placement cursors.
-__global__ void moe_offsets_kernel(const int* __restrict__ cnt, int* __restrict__ off, int* __restrict__ cursor,
-                                   int* __restrict__ tile_expert, int* __restrict__ tile_row0,
-                                   int* __restrict__ tile_rows, int* __restrict__ n_tiles, int* __restrict__ n_rows,
-                                   int n_exp, int e0, int e1, int bm, int even) {
-    __shared__ int s_rows[1024], s_tiles[1024];
+// table of the grouped GEMM, tile i -> (expert, first sorted row, valid rows).  Also clears the placement cursors and the counts.
+__global__ void __launch_bounds__(1024)
+moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_row0, int* tile_rows, int* n_tiles, int* n_rows,
+                   int n_exp, int e0, int e1, int bm, int even) {
+    __shared__ int s_r[32], s_t[32];
     const int e = threadIdx.x;
+    pdl_begin();
     const int c = (e >= e0 && e < e1) ? cnt[e] : 0;
     const int step = tile_step(c, bm, even);
-    s_rows[e] = c;
-    s_tiles[e] = (c + step - 1) / step;
-    __syncthreads();
-    for (int d = 1; d < 1024; d <<= 1) {   // inclusive Hillis-Steele scan of both arrays
-        const int r = e >= d ? s_rows[e - d] : 0, t = e >= d ? s_tiles[e - d] : 0;
-        __syncthreads();
-        s_rows[e] += r;
-        s_tiles[e] += t;
-        __syncthreads();
-    }
-    const int row0 = s_rows[e] - c, tile0 = s_tiles[e] - (c + step - 1) / step;
+    const int ct = (c + step - 1) / step;
+    int vr = c, vt = ct, total_rows, total_tiles;
+    scan_rows_tiles(vr, vt, total_rows, total_tiles, s_r, s_t);
+    const int row0 = vr - c, tile0 = vt - ct;
     if (e < n_exp) {
         off[e] = row0;
         cursor[e] = 0;
+        cnt[e] = 0;
     }
     for (int r = 0, i = tile0; r < c; r += step, ++i) {
         tile_expert[i] = e;
@@ -286,54 +297,48 @@ __global__ void moe_offsets_kernel(const int* __restrict__ cnt, int* __restrict_
         tile_rows[i] = min(step, c - r);
     }
     if (e == 1023) {
-        *n_tiles = s_tiles[e];
-        *n_rows = s_rows[e];
+        *n_tiles = total_tiles;
+        *n_rows = total_rows;
     }
 }
 
-// placement of the local experts' slots in sorted order, with the routing weight of each sorted row
-// (grouped matmul 2 multiplies by it)
-__global__ void moe_place_kernel(const int* __restrict__ idx, const float* __restrict__ wt, const int* __restrict__ off,
-                                 int* __restrict__ cursor, int* __restrict__ pos_of_slot, int* __restrict__ slot_of_pos,
-                                 float* __restrict__ row_w, int ns, int e0, int e1) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += gridDim.x * blockDim.x) {
-        const int e = idx[i];
-        int pos = -1;
-        if (e >= e0 && e < e1) {
-            pos = off[e] + atomicAdd(cursor + e, 1);
-            slot_of_pos[pos] = i;
-            row_w[pos] = wt[i];
-        }
-        pos_of_slot[i] = pos;  // -1: the expert lives on another rank
-    }
-}
-
-// xs[pos][:] = x[token][:] for the token's k slots (f16 rows of h).  A warp reads 2 KB of a token's row once and writes it to
-// all of the token's places: bound by the writes.  (One thread per 16 bytes of a slot read every row k times and spent its
-// instructions on two 64-bit divisions: 39 us for 4096 tokens x 8 slots x 4 KB, serialised with cold caches; now 23.)
+// Placement of the local experts' slots in sorted order, with the routing weight of each sorted row (grouped matmul 2 multiplies by
+// it), and xs[pos][:] = x[token][:] for the token's k slots (f16 rows of h).  A warp takes a token: its lanes place the slots, then it
+// reads the token's row once, 2 KB at a time, and writes it to all of the token's places: bound by the writes.  (One thread per 16 bytes
+// of a slot read every row k times and spent its instructions on two 64-bit divisions: 39 us for 4096 tokens x 8 slots x 4 KB,
+// serialised with cold caches; 23 with a warp per 2 KB.)
 constexpr int GATHER_VEC = 4;   // 16-byte words per lane
-__global__ void moe_gather_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const int* __restrict__ pos_of_slot,
-                                  int t, int k, int h8) {
+__global__ void moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* wt, const int* off, int* cursor,
+                                        int* pos_of_slot, int* slot_of_pos, float* row_w, int t, int k, int h8, int e0, int e1) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
-    const int chunks = (h8 + 32 * GATHER_VEC - 1) / (32 * GATHER_VEC);
-    const long long units = (long long)t * chunks, step = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long u = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < units; u += step) {
-        const int tok = (int)(u / chunks), c0 = (int)(u - (long long)tok * chunks) * (32 * GATHER_VEC) + lane;
-        const int my_pos = lane < k ? pos_of_slot[(size_t)tok * k + lane] : -1;      // k <= 32
-        uint4 v[GATHER_VEC];
-#pragma unroll
-        for (int i = 0; i < GATHER_VEC; ++i) {
-            if (c0 + 32 * i < h8) {
-                v[i] = x[(size_t)tok * h8 + c0 + 32 * i];
+    for (int tok = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); tok < t; tok += (int)(gridDim.x * (blockDim.x >> 5))) {
+        int my_pos = -1;                                                             // -1: the expert lives on another rank
+        if (lane < k) {                                                              // k <= 32
+            const int slot = tok * k + lane, e = idx[slot];
+            if (e >= e0 && e < e1) {
+                my_pos = off[e] + atomicAdd(cursor + e, 1);
+                slot_of_pos[my_pos] = slot;
+                row_w[my_pos] = wt[slot];
             }
+            pos_of_slot[slot] = my_pos;
         }
-        for (int j = 0; j < k; ++j) {
-            const int pos = __shfl_sync(0xffffffffu, my_pos, j);
-            if (pos >= 0) {                                                          // else the expert lives on another rank
+        for (int c0 = lane; c0 - lane < h8; c0 += 32 * GATHER_VEC) {
+            uint4 v[GATHER_VEC];
 #pragma unroll
-                for (int i = 0; i < GATHER_VEC; ++i) {
-                    if (c0 + 32 * i < h8) {
-                        xs[(size_t)pos * h8 + c0 + 32 * i] = v[i];
+            for (int i = 0; i < GATHER_VEC; ++i) {
+                if (c0 + 32 * i < h8) {
+                    v[i] = x[(size_t)tok * h8 + c0 + 32 * i];
+                }
+            }
+            for (int j = 0; j < k; ++j) {
+                const int pos = __shfl_sync(0xffffffffu, my_pos, j);
+                if (pos >= 0) {
+#pragma unroll
+                    for (int i = 0; i < GATHER_VEC; ++i) {
+                        if (c0 + 32 * i < h8) {
+                            xs[(size_t)pos * h8 + c0 + 32 * i] = v[i];
+                        }
                     }
                 }
             }
@@ -341,33 +346,12 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ x, uint4* __restrict
     }
 }
 
-// act[pos][c] = f16( silu(gate) * up ),  c13 = [rows][2*ffn] with gate in the first half; 8 outputs per thread
-__global__ void moe_act_silu_kernel(const __half* __restrict__ c13, __half* __restrict__ act, const int* __restrict__ n_rows,
-                                    int ffn) {
-    const int f8 = ffn / 8;
-    const size_t total = (size_t)(*n_rows) * f8;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / f8, c = (i % f8) * 8;
-        const uint4 gv = *reinterpret_cast<const uint4*>(c13 + r * 2 * ffn + c);
-        const uint4 uv = *reinterpret_cast<const uint4*>(c13 + r * 2 * ffn + ffn + c);
-        const __half2* gh = reinterpret_cast<const __half2*>(&gv);
-        const __half2* uh = reinterpret_cast<const __half2*>(&uv);
-        uint4 ov;
-        __half2* oh = reinterpret_cast<__half2*>(&ov);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 g = __half22float2(gh[j]), u = __half22float2(uh[j]);
-            oh[j] = __floats2half2_rn((g.x / (1.0f + expf(-g.x))) * u.x, (g.y / (1.0f + expf(-g.y))) * u.y);
-        }
-        *reinterpret_cast<uint4*>(act + r * ffn + c) = ov;
-    }
-}
-
 // out[t][c] = sum_j c2[pos(t*k+j)][c]  (routing weights were applied in GEMM-2's epilogue); slots whose
 // expert is not local contribute nothing
 template <bool OUT_F16>
-__global__ void moe_combine_kernel(const __half* __restrict__ c2, void* __restrict__ out, const int* __restrict__ pos_of_slot,
+__global__ void moe_combine_kernel(const __half* c2, void* out, const int* pos_of_slot,
                                    int t, int h, int k) {
+    pdl_begin();
     const int h8 = h / 8;
     const size_t total = (size_t)t * h8;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -412,55 +396,64 @@ inline int blocks_for(size_t total, int threads) {
 
 }  // namespace
 
-void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, cudaStream_t st) {
+namespace {
+
+template <class... P, class... A>
+void launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, int pdl, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+}  // namespace
+
+void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl,
+                     cudaStream_t st) {
     const int stage = n_exp <= 512;   // 8 warps x 512 floats = 16 KB of shared memory at most
-    moe_topk_kernel<<<(t + TOPK_WARPS - 1) / TOPK_WARPS, TOPK_WARPS * 32, stage ? TOPK_WARPS * n_exp * sizeof(float) : 0, st>>>(
-        logits, idx, wt, t, n_exp, k, stage);
+    launch(moe_topk_kernel, (t + TOPK_WARPS - 1) / TOPK_WARPS, TOPK_WARPS * 32, stage ? TOPK_WARPS * n_exp * sizeof(float) : 0, st, pdl,
+           logits, idx, wt, t, n_exp, k, stage, cnt, e0, e1);
 }
 
 // Returns the number of launches.  Up to eight tokens are routed by the table block itself (one launch); above that
 // one block's 32 warps would route two or more tokens each in turn (27 us at 64 tokens), so the routing runs on
 // many SMs first and the block only builds the tables.
-int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm,
+int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm, int pdl,
                            cudaStream_t st) {
-    const int stage = n_exp <= 256;   // 32 warps x 256 floats = 32 KB beside the 16 KB of tables
+    const int stage = n_exp <= 256;   // 32 warps x 256 floats = 32 KB beside the 12 KB of tables
     const int own_topk = t <= 8;
     if (!own_topk) {
-        launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, st);
+        launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, nullptr, 0, 0, pdl, st);
     }
-    moe_route_small_kernel<<<1, 1024, (stage && own_topk) ? 32 * n_exp * sizeof(float) : 0, st>>>(
-        logits, b.idx, b.wt, b.off, b.pos_of_slot, b.slot_of_pos, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
-        b.row_w, t, n_exp, k, e0, e1, bm, stage, own_topk);
+    launch(moe_route_small_kernel, 1, 1024, (stage && own_topk) ? 32 * n_exp * sizeof(float) : 0, st, pdl, logits, b.idx, b.wt, b.off,
+           b.pos_of_slot, b.slot_of_pos, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows, b.row_w, t, n_exp, k, e0, e1, bm,
+           stage, own_topk);
     return own_topk ? 1 : 2;
 }
 
-void launch_moe_align(const MoeBufs& b, int ns, int n_exp, int e0, int e1, int bm, int even, cudaStream_t st) {
-    cudaMemsetAsync(b.cnt, 0, (size_t)n_exp * sizeof(int), st);
-    moe_count_kernel<<<blocks_for(ns, 256), 256, 0, st>>>(b.idx, b.cnt, ns, e0, e1);
-    moe_offsets_kernel<<<1, 1024, 0, st>>>(b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles,
-                                          b.n_rows, n_exp, e0, e1, bm, even);
-    moe_place_kernel<<<blocks_for(ns, 256), 256, 0, st>>>(b.idx, b.wt, b.off, b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w,
-                                                          ns, e0, e1);
+int launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
+                    int even, int pdl, cudaStream_t st) {
+    launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
+    launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
+           n_exp, e0, e1, bm, even);
+    launch(moe_place_gather_kernel, blocks_for((size_t)t * 32, 256), 256, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt, b.off,
+           b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
+    return 3;
 }
 
-void launch_moe_gather(const void* x, const MoeBufs& b, int ns, int k, int h, cudaStream_t st) {
-    const int h8 = h / 8, t = ns / k, chunks = (h8 + 32 * GATHER_VEC - 1) / (32 * GATHER_VEC);
-    moe_gather_kernel<<<blocks_for((size_t)t * chunks * 32, 256), 256, 0, st>>>((const uint4*)x, (uint4*)b.xs, b.pos_of_slot, t, k,
-                                                                               h8);
-}
-
-void launch_moe_act(const MoeBufs& b, int rows_upper, int ffn, cudaStream_t st) {
-    moe_act_silu_kernel<<<blocks_for((size_t)rows_upper * (ffn / 8), 256), 256, 0, st>>>((const __half*)b.c13, (__half*)b.act,
-                                                                                 b.n_rows, ffn);
-}
-
-void launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, cudaStream_t st) {
+void launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, int pdl, cudaStream_t st) {
     const int g = blocks_for((size_t)t * (h / 8), 256);
-    if (out_f16) {
-        moe_combine_kernel<true><<<g, 256, 0, st>>>((const __half*)b.c2, out, b.pos_of_slot, t, h, k);
-    } else {
-        moe_combine_kernel<false><<<g, 256, 0, st>>>((const __half*)b.c2, out, b.pos_of_slot, t, h, k);
-    }
+    launch(out_f16 ? moe_combine_kernel<true> : moe_combine_kernel<false>, g, 256, 0, st, pdl, (const __half*)b.c2, out, b.pos_of_slot, t,
+           h, k);
 }
 
 }  // namespace w4

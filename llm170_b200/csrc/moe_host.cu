@@ -74,6 +74,7 @@ int Dec::ensure_moe(int t, cudaStream_t st) {
     ok(cudaMalloc(&mb.c13, slots * 2 * moe.ffn * 2));
     ok(cudaMalloc(&mb.act, slots * moe.ffn * 2));
     ok(cudaMalloc(&mb.c2, slots * moe.hidden * 2));
+    ok(cudaMemset(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int)));   // the counts of a call are left at zero by it
     if (e != cudaSuccess) {
         free_moe();
         return cuda_fail("alloc moe scratch", e);
@@ -116,17 +117,15 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         }
         if (ns <= 1024) {
             // routing and all dispatch tables in one launch; the first grouped GEMV fetches each row's token itself
-            launches += launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, st);
+            launches += launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, tune_pdl, st);
             if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st,
                                       mb.slot_of_pos, moe.top_k, /*tables_fresh=*/true)) {
                 return rc;
             }
         } else {
-            launch_moe_topk(logits, mb.idx, mb.wt, t, moe.n_experts, moe.top_k, st);
-            launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, 8, 0, st);
-            launch_moe_gather(x16, mb, ns, moe.top_k, moe.hidden, st);
-            launches += 5;
-            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st)) {
+            launches += launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, 8, 0, tune_pdl, st);
+            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, nullptr,
+                                      1, /*tables_fresh=*/true)) {
                 return rc;
             }
         }
@@ -143,10 +142,7 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         const bool weight_rows = (long long)ns < 192LL * moe.n_experts;
         const int bm = weight_rows ? 128 : 256;
         const int max_tiles = (ns + bm - 1) / bm + std::min(ns, n_local);
-        launch_moe_topk(logits, mb.idx, mb.wt, t, moe.n_experts, moe.top_k, st);
-        launches += 5;
-        launch_moe_align(mb, ns, moe.n_experts, moe.e0, moe.e1, bm, weight_rows, st);
-        launch_moe_gather(x16, mb, ns, moe.top_k, moe.hidden, st);
+        launches += launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, weight_rows, tune_pdl, st);
         if (weight_rows) {
             if (int rc = gemm_ts_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, bm, nullptr, st, true)) {
                 return rc;
@@ -163,7 +159,7 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             }
         }
     }
-    launch_moe_combine(mb, y, t, moe.hidden, moe.top_k, out_kind == W4A16_OUT_F16, st);
+    launch_moe_combine(mb, y, t, moe.hidden, moe.top_k, out_kind == W4A16_OUT_F16, tune_pdl, st);
     launches += 1;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : cuda_fail("moe_ffn launch", e);
@@ -256,7 +252,7 @@ int w4a16_moe_topk(w4a16_dec* dec, const float* logits_dev, int* idx_dev, float*
     if (!d.moe.set) {
         return d.fail("w4a16 moe_topk: set_moe was not called");
     }
-    w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, moe_stream(dec, stream));
+    w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, nullptr, 0, 0, d.tune_pdl, moe_stream(dec, stream));
     d.launches++;
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : d.cuda_fail("moe_topk", e);
