@@ -69,7 +69,16 @@ __device__ __forceinline__ void topk_of_token_n(const float* l, int* idx, float*
         }
         __syncwarp();
         if (lane == 0) {
-            for (int e = 0; e < n; ++e) {
+            int e = 0;
+            for (; e + 4 <= n; e += 4) {        // (rows of n floats: 16-byte aligned where n is a multiple of 4)
+                if ((n & 3) == 0) {
+                    const float4 q = *reinterpret_cast<const float4*>(stage + e);
+                    sum = (((sum + q.x) + q.y) + q.z) + q.w;
+                } else {
+                    sum = (((sum + stage[e]) + stage[e + 1]) + stage[e + 2]) + stage[e + 3];
+                }
+            }
+            for (; e < n; ++e) {
                 sum += stage[e];
             }
         }
@@ -151,7 +160,7 @@ __device__ __forceinline__ int tile_step(int c, int bm, int even) {
 
 // `cnt` (optional): rows per local expert; zero on entry, moe_offsets_kernel leaves it so.
 __global__ void moe_topk_kernel(const float* lg, int* idx, float* wt, int t, int n, int k, int stage_rows, int* cnt, int e0, int e1) {
-    extern __shared__ float s_stage[];   // [warps][n] when the launch provides it
+    extern __shared__ __align__(16) float s_stage[];   // [warps][n] when the launch provides it
     pdl_begin();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ti = blockIdx.x * TOPK_WARPS + w;
@@ -219,7 +228,7 @@ moe_route_small_kernel(const float* lg, int* idx, float* wt,
                        int* n_tiles, int* n_rows, float* row_w, int t, int n_exp,
                        int k, int e0, int e1, int bm, int stage_rows, int do_topk) {
     __shared__ int s_rows[1024], s_off[1024], s_cursor[1024], s_wr[32], s_wt[32];
-    extern __shared__ float s_stage[];   // [32 warps][n_exp] when the launch provides it
+    extern __shared__ __align__(16) float s_stage[];   // [32 warps][n_exp] when the launch provides it
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     s_rows[tid] = 0;
     s_cursor[tid] = 0;
@@ -303,46 +312,42 @@ moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_
 }
 
 // Placement of the local experts' slots in sorted order, with the routing weight of each sorted row (grouped matmul 2 multiplies by
-// it), and xs[pos][:] = x[token][:] for the token's k slots (f16 rows of h).  A warp takes a token: its lanes place the slots, then it
-// reads the token's row once, 2 KB at a time, and writes it to all of the token's places: bound by the writes.  (One thread per 16 bytes
-// of a slot read every row k times and spent its instructions on two 64-bit divisions: 39 us for 4096 tokens x 8 slots x 4 KB,
-// serialised with cold caches; 23 with a warp per 2 KB.)
-constexpr int GATHER_VEC = 4;   // 16-byte words per lane
-__global__ void moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* wt, const int* off, int* cursor,
-                                        int* pos_of_slot, int* slot_of_pos, float* row_w, int t, int k, int h8, int e0, int e1) {
+// it), and xs[pos][:] = x[token][:] for the token's k slots (f16 rows of h).  A block takes a token: its first warp places the slots, then
+// every thread reads 16 bytes of the row once and writes them to all of the token's places: bound by the writes (4096 tokens x 8 slots x
+// 4 KB, cold: 39 us with a thread per 16 bytes of a slot, 33 with a warp per token, 31 so).
+constexpr int GATHER_THREADS = 128;
+__global__ void __launch_bounds__(GATHER_THREADS)
+moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* wt, const int* off, int* cursor, int* pos_of_slot,
+                        int* slot_of_pos, float* row_w, int t, int k, int h8, int e0, int e1) {
+    __shared__ int s_pos[32];                                                        // k <= 32
     pdl_begin();
-    const int lane = threadIdx.x & 31;
-    for (int tok = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); tok < t; tok += (int)(gridDim.x * (blockDim.x >> 5))) {
-        int my_pos = -1;                                                             // -1: the expert lives on another rank
-        if (lane < k) {                                                              // k <= 32
-            const int slot = tok * k + lane, e = idx[slot];
+    for (int tok = (int)blockIdx.x; tok < t; tok += (int)gridDim.x) {
+        if ((int)threadIdx.x < k) {
+            const int slot = tok * k + (int)threadIdx.x, e = idx[slot];
+            int pos = -1;                                                            // the expert lives on another rank
             if (e >= e0 && e < e1) {
-                my_pos = off[e] + atomicAdd(cursor + e, 1);
-                slot_of_pos[my_pos] = slot;
-                row_w[my_pos] = wt[slot];
+                pos = off[e] + atomicAdd(cursor + e, 1);
+                slot_of_pos[pos] = slot;
+                row_w[pos] = wt[slot];
             }
-            pos_of_slot[slot] = my_pos;
+            pos_of_slot[slot] = pos;
+            s_pos[threadIdx.x] = pos;
         }
-        for (int c0 = lane; c0 - lane < h8; c0 += 32 * GATHER_VEC) {
-            uint4 v[GATHER_VEC];
-#pragma unroll
-            for (int i = 0; i < GATHER_VEC; ++i) {
-                if (c0 + 32 * i < h8) {
-                    v[i] = x[(size_t)tok * h8 + c0 + 32 * i];
-                }
-            }
+        __syncthreads();
+        for (int c = (int)threadIdx.x; c < h8; c += 2 * GATHER_THREADS) {
+            const bool two = c + GATHER_THREADS < h8;
+            const uint4 v0 = x[(size_t)tok * h8 + c], v1 = two ? x[(size_t)tok * h8 + c + GATHER_THREADS] : make_uint4(0, 0, 0, 0);
             for (int j = 0; j < k; ++j) {
-                const int pos = __shfl_sync(0xffffffffu, my_pos, j);
+                const int pos = s_pos[j];
                 if (pos >= 0) {
-#pragma unroll
-                    for (int i = 0; i < GATHER_VEC; ++i) {
-                        if (c0 + 32 * i < h8) {
-                            xs[(size_t)pos * h8 + c0 + 32 * i] = v[i];
-                        }
+                    xs[(size_t)pos * h8 + c] = v0;
+                    if (two) {
+                        xs[(size_t)pos * h8 + c + GATHER_THREADS] = v1;
                     }
                 }
             }
         }
+        __syncthreads();                                                             // s_pos is for the next token
     }
 }
 
@@ -445,7 +450,7 @@ int launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t,
     launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
     launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
            n_exp, e0, e1, bm, even);
-    launch(moe_place_gather_kernel, blocks_for((size_t)t * 32, 256), 256, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt, b.off,
+    launch(moe_place_gather_kernel, blocks_for((size_t)t, 1), GATHER_THREADS, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt, b.off,
            b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
     return 3;
 }
