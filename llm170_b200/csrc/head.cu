@@ -19,7 +19,9 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <new>
 #include <string>
+#include <vector>
 
 #include "../../include/w4a16_b200.h"
 #include "dec.h"
@@ -35,13 +37,29 @@ constexpr int HEAD_XPAD = 16;           // bytes added to a token's row of f16 s
 
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
 
-// One block per row: absmax, scale, quantise.  w: bf16 [rows][k] (device staging), q: offset-binary bytes [rows][k].
+// Resident layout: [16 rows][64 channels][rows g / g + 8][32 lanes][16 bytes].  Lane 4g + t of the GEMV multiplies row g and row g + 8 at
+// channels 16t..16t+15 of a 64-channel step; its 16 bytes of either lie beside those of the other lanes, so that a warp reads two whole
+// 512-byte lines per step and 16 rows of the matrix are one contiguous piece.
+__host__ __device__ __forceinline__ size_t head_at(size_t row, int ch, int k) {
+    const size_t tile = row / 16 * (size_t)(k / 64) + (size_t)(ch / 64);
+    const int r = (int)(row % 16);
+    return tile * 1024 + (size_t)((r >> 3) * 512 + ((r & 7) * 4 + ch % 64 / 16) * 16 + ch % 16);
+}
+
+// One block per row, row0 + blockIdx.x: absmax, scale, quantise.  w: bf16 [rows][k] (device staging), q: offset-binary bytes (head_at).
+// Rows from `n` on fill the last 16: zeros.
 __global__ void __launch_bounds__(256) head_quant_kernel(const uint16_t* __restrict__ w, uint8_t* __restrict__ q,
-                                                         float* __restrict__ scale, int k) {
+                                                         float* __restrict__ scale, int row0, int n, int k) {
     __shared__ float red[8];
     __shared__ float s_scale;
-    const size_t row = blockIdx.x;
-    const uint16_t* wr = w + row * (size_t)k;
+    const size_t row = (size_t)row0 + blockIdx.x;
+    if (row >= (size_t)n) {
+        for (int i = threadIdx.x; i < k; i += blockDim.x) {
+            q[head_at(row, i, k)] = 128;
+        }
+        return;
+    }
+    const uint16_t* wr = w + (size_t)blockIdx.x * (size_t)k;
     float amax = 0.0f;
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
         amax = fmaxf(amax, fabsf(bf16_bits_to_f32(wr[i])));
@@ -65,11 +83,10 @@ __global__ void __launch_bounds__(256) head_quant_kernel(const uint16_t* __restr
     }
     __syncthreads();
     const float s = s_scale;
-    uint8_t* qr = q + row * (size_t)k;
     for (int i = threadIdx.x; i < k; i += blockDim.x) {
         float v = roundf(__fdiv_rn(bf16_bits_to_f32(wr[i]), s));   // half away from zero, as f32::round
         v = fminf(fmaxf(v, -127.0f), 127.0f);
-        qr[i] = (uint8_t)((int)v + 128);
+        q[head_at(row, i, k)] = (uint8_t)((int)v + 128);
     }
 }
 
@@ -89,14 +106,65 @@ struct HeadArgs {
     int n, k, t0, tp;
 };
 
-__global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const HeadArgs a) {
-    extern __shared__ __align__(16) unsigned char hsm[];
+// D = 64-channel steps that a warp has on the way.
+template <int D>
+__global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const HeadArgs a) {
+    extern __shared__ __align__(128) unsigned char hsm[];
     constexpr int WARPS = HEAD_THREADS / 32;
     __shared__ float4 s_part[WARPS * 32];
     const int k = a.k, tp = a.tp;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int g = lane >> 2, tq = lane & 3;
+    const int nrb = (a.n + 15) / 16, nsteps = k / 64;
+    // Whole rounds: a row block per warp.  The rest of the row blocks is dealt over all SMs and, where it leaves warps idle,
+    // each block's K over several warps of its CTA: 151936 rows are 4.01 rounds, and the fifth one cost as much as the others.
+    const int all_warps = gridDim.x * WARPS, rounds = nrb / all_warps;
+    const int rest0 = rounds * all_warps, rest = nrb - rest0;
+    const int per_cta = (rest + (int)gridDim.x - 1) / (int)gridDim.x;            // 0..WARPS
+    int ways = WARPS;
+    while (ways > 1 && ways * per_cta > WARPS) {
+        ways >>= 1;
+    }
+    const int sub = warp / ways, part = warp - sub * ways;
+    const int rb_rest = rest0 + sub * (int)gridDim.x + (int)blockIdx.x;
+    const bool live = sub < per_cta && rb_rest < nrb;
+    const int s0_rest = nsteps * part / ways, n_rest = live ? nsteps * (part + 1) / ways - s0_rest : 0;
+
+    // ---- weights: a private ring of D steps of 1 KB, filled by asynchronous copies in the order of use, across row blocks.  Every lane
+    // reads back what it copied itself, so the loop has no barrier.  (One token, calls back to back: 151936 x 2048 47.8 us, 151936 x 5120 114; with
+    // loads to registers, eight steps unrolled, 61.7 and 134: a warp had nothing on the way while it multiplied.)
+    const uint32_t ring = smem_u32(hsm) + (uint32_t)warp * (D * 1024u) + (uint32_t)lane * 16u;
+    const unsigned char* fp = nullptr;
+    int fr = -1, fleft = 0;                                                      // round being requested, steps left in it
+    uint32_t fdst = 0;
+    auto fetch = [&]() {
+        if (fleft == 0 && fr < rounds) {
+            ++fr;
+            const int rb = fr < rounds ? fr * all_warps + (int)blockIdx.x * WARPS + warp : rb_rest;
+            fleft = fr < rounds ? nsteps : n_rest;
+            fp = a.q + ((size_t)rb * nsteps + (fr < rounds ? 0 : s0_rest)) * 1024 + lane * 16;
+        }
+        if (fleft > 0) {
+            cp_async_16(ring + fdst, fp);
+            cp_async_16(ring + fdst + 512u, fp + 512);
+            fp += 1024;
+            --fleft;
+        }
+        cp_async_commit();
+        if ((fdst += 1024u) == D * 1024u) {
+            fdst = 0;
+        }
+    };
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        fetch();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");                           // the weights do not depend on the kernel before, x may
+
     const int xrow = k * 2 + HEAD_XPAD;                 // bytes of one token's f16 row
-    unsigned char* xhi = hsm;
-    unsigned char* xlo = hsm + (size_t)tp * xrow;
+    unsigned char* xhi = hsm + WARPS * D * 1024;
+    unsigned char* xlo = xhi + (size_t)tp * xrow;
     // stage the activations: hi = f16(x), lo = f16((x - hi) * 2^11)
     for (int i = threadIdx.x; i < tp * (k / 2); i += HEAD_THREADS) {
         const int tok = i / (k / 2), c = (i - tok * (k / 2)) * 2;
@@ -109,44 +177,36 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
     }
     __syncthreads();
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int g = lane >> 2, tq = lane & 3;
-    const int nrb = (a.n + 15) / 16;
-    const bool tok_live = g < tp;                        // this lane's column of the MMA holds a token
-    const unsigned char* xh_l = xhi + (size_t)(tok_live ? g : 0) * xrow + tq * 32;
-    const unsigned char* xl_l = xlo + (size_t)(tok_live ? g : 0) * xrow + tq * 32;
-    const int nsteps = k / 64;
-    // sums of row block rb over steps [s0, s1): .x, .y = row g, tokens 2tq, 2tq + 1;  .z, .w = row g + 8
-    auto multiply = [&](int rb, int s0, int s1) {
-        const int r0 = min(rb * 16 + g, a.n - 1), r1 = min(rb * 16 + g + 8, a.n - 1);   // clamped: loads stay in range
-        const uint4* p0 = reinterpret_cast<const uint4*>(a.q + (size_t)r0 * k) + tq;
-        const uint4* p1 = reinterpret_cast<const uint4*>(a.q + (size_t)r1 * k) + tq;
+    // lanes whose column of the MMA holds no token read token 0: their sums are never stored
+    const uint32_t xh_l = smem_u32(xhi) + (uint32_t)((g < tp ? g : 0) * xrow + tq * 32), xl_l = xh_l + (uint32_t)(tp * xrow);
+    uint32_t rsrc = 0;
+    // sums of the next row block in the ring, steps [s0, s1): .x, .y = row g, tokens 2tq, 2tq + 1;  .z, .w = row g + 8
+    auto multiply = [&](int s0, int s1) {
         float ch[4] = {0.f, 0.f, 0.f, 0.f}, cl[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
         for (int s = s0; s < s1; ++s) {
-            // 64 channels: this lane's 16 bytes of row g and of row g+8 (the four lanes of a row cover 64 contiguous bytes)
-            const uint4 w0 = __ldg(p0 + s * 4), w1 = __ldg(p1 + s * 4);
-            uint4 bh0 = make_uint4(0, 0, 0, 0), bh1 = bh0, bl0 = bh0, bl1 = bh0;
-            if (tok_live) {
-                bh0 = *reinterpret_cast<const uint4*>(xh_l + s * 128);
-                bh1 = *reinterpret_cast<const uint4*>(xh_l + s * 128 + 16);
-                bl0 = *reinterpret_cast<const uint4*>(xl_l + s * 128);
-                bl1 = *reinterpret_cast<const uint4*>(xl_l + s * 128 + 16);
+            cp_async_wait_group<D - 1>();
+            const uint4 w0 = lds128(ring + rsrc), w1 = lds128(ring + rsrc + 512u);
+            fetch();
+            if ((rsrc += 1024u) == D * 1024u) {
+                rsrc = 0;
             }
             const uint32_t ww0[4] = {w0.x, w0.y, w0.z, w0.w}, ww1[4] = {w1.x, w1.y, w1.z, w1.w};
-            const uint32_t xh[8] = {bh0.x, bh0.y, bh0.z, bh0.w, bh1.x, bh1.y, bh1.z, bh1.w};
-            const uint32_t xl[8] = {bl0.x, bl0.y, bl0.z, bl0.w, bl1.x, bl1.y, bl1.z, bl1.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                // MMA j multiplies the lane's channels 4j..4j+3: the k order inside the MMA is permuted the same way
-                // for the weights and for the activations, which leaves every product in place
-                uint32_t af[4];
-                af[0] = ob_pair_to_half2(ww0[j], 0x4140u);
-                af[1] = ob_pair_to_half2(ww1[j], 0x4140u);
-                af[2] = ob_pair_to_half2(ww0[j], 0x4342u);
-                af[3] = ob_pair_to_half2(ww1[j], 0x4342u);
-                mma16816(ch, af, xh[2 * j], xh[2 * j + 1]);
-                mma16816(cl, af, xl[2 * j], xl[2 * j + 1]);
+            for (int h = 0; h < 2; ++h) {
+                const uint4 bh = lds128(xh_l + (uint32_t)(s * 128 + h * 16)), bl = lds128(xl_l + (uint32_t)(s * 128 + h * 16));
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    // MMA j multiplies the lane's channels 4j..4j+3: the k order inside the MMA is permuted the same way
+                    // for the weights and for the activations, which leaves every product in place
+                    const int j = 2 * h + i;
+                    uint32_t af[4];
+                    af[0] = ob_pair_to_half2(ww0[j], 0x4140u);
+                    af[1] = ob_pair_to_half2(ww1[j], 0x4140u);
+                    af[2] = ob_pair_to_half2(ww0[j], 0x4342u);
+                    af[3] = ob_pair_to_half2(ww1[j], 0x4342u);
+                    mma16816(ch, af, i ? bh.z : bh.x, i ? bh.w : bh.y);
+                    mma16816(cl, af, i ? bl.z : bl.x, i ? bl.w : bl.y);
+                }
             }
         }
         return make_float4(ch[0] + cl[0] * (1.0f / 2048.0f), ch[1] + cl[1] * (1.0f / 2048.0f), ch[2] + cl[2] * (1.0f / 2048.0f),
@@ -170,32 +230,14 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
             }
         }
     };
-    // Whole rounds: a row block per warp.  The rest of the row blocks is dealt over all SMs and, where it leaves warps idle,
-    // each block's K over several warps of its CTA: 151936 rows are 4.01 rounds, and the fifth one cost as much as the others.
-    // (One token, calls back to back into one output, before and after: 151936 x 2048 66.9 -> 61.6 us, 151936 x 5120 147 -> 134,
-    // 50000 x 4096 50.2 -> 43.1.  Bound by HBM latency: fetching four steps ahead in two register sets keeps fewer loads in
-    // flight and took 72 us on the first.)
-    const int all_warps = gridDim.x * WARPS, rounds = nrb / all_warps;
     for (int i = 0; i < rounds; ++i) {
-        const int rb = i * all_warps + blockIdx.x * WARPS + warp;
-        store(rb, multiply(rb, 0, nsteps));
+        const float4 c = multiply(0, nsteps);
+        store(i * all_warps + (int)blockIdx.x * WARPS + warp, c);
     }
-    const int rest0 = rounds * all_warps, rest = nrb - rest0;
     if (rest == 0) {
         return;
     }
-    const int per_cta = (rest + (int)gridDim.x - 1) / (int)gridDim.x;            // 1..WARPS
-    int ways = WARPS;
-    while (ways * per_cta > WARPS) {
-        ways >>= 1;
-    }
-    const int sub = warp / ways, part = warp - sub * ways;
-    const int rb = rest0 + sub * (int)gridDim.x + (int)blockIdx.x;
-    const bool live = sub < per_cta && rb < nrb;
-    float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live) {
-        c = multiply(rb, nsteps * part / ways, nsteps * (part + 1) / ways);
-    }
+    float4 c = multiply(s0_rest, s0_rest + n_rest);
     if (ways > 1) {
         s_part[threadIdx.x] = c;
         __syncthreads();
@@ -210,14 +252,47 @@ __global__ void __launch_bounds__(HEAD_THREADS, 1) head_gemv_i8_kernel(const Hea
         }
     }
     if (live && part == 0) {
-        store(rb, c);
+        store(rb_rest, c);
+    }
+}
+
+constexpr int HEAD_DEPTHS[] = {8, 6, 5, 4, 3, 2, 1};
+constexpr size_t HEAD_SMEM_MAX = 218 * 1024;            // beside 8 KB for the sums
+// Steps on the way per warp beside `x_bytes` of activations: five where that leaves room for a second CTA (the next call's, whose weights
+// are then on the way before this one ends), else what fits beside them.
+int head_depth(size_t x_bytes) {
+    if (x_bytes + 5 * (HEAD_THREADS / 32 * 1024) <= (size_t)104 * 1024) {
+        return 5;
+    }
+    for (int d : HEAD_DEPTHS) {
+        if (x_bytes + (size_t)d * (HEAD_THREADS / 32 * 1024) <= HEAD_SMEM_MAX) {
+            return d;
+        }
+    }
+    return 1;
+}
+const void* head_kernel(int depth) {
+    switch (depth) {
+    case 8: return (const void*)head_gemv_i8_kernel<8>;
+    case 6: return (const void*)head_gemv_i8_kernel<6>;
+    case 5: return (const void*)head_gemv_i8_kernel<5>;
+    case 4: return (const void*)head_gemv_i8_kernel<4>;
+    case 3: return (const void*)head_gemv_i8_kernel<3>;
+    case 2: return (const void*)head_gemv_i8_kernel<2>;
+    default: return (const void*)head_gemv_i8_kernel<1>;
     }
 }
 
 }  // namespace
 
 cudaError_t head_init_device() {
-    return cudaFuncSetAttribute(head_gemv_i8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    for (int d : HEAD_DEPTHS) {
+        const cudaError_t e = cudaFuncSetAttribute(head_kernel(d), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HEAD_SMEM_MAX);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    return cudaSuccess;
 }
 
 }  // namespace w4
@@ -248,7 +323,8 @@ int w4a16_upload_head(w4a16_dec* dec, const void* w_bf16_host, size_t bytes, int
     float* sc = nullptr;
     uint16_t* stage = nullptr;
     const int rows_chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)32 << 20) / ((size_t)k * 2)));
-    cudaError_t e = cudaMalloc(&q, (size_t)n * k);
+    const int n16 = (n + 15) / 16 * 16;
+    cudaError_t e = cudaMalloc(&q, (size_t)n16 * k);
     if (e == cudaSuccess) e = cudaMalloc(&sc, (size_t)n * 4);
     if (e == cudaSuccess) e = cudaMalloc(&stage, (size_t)rows_chunk * k * 2);
     if (e != cudaSuccess) {
@@ -262,7 +338,7 @@ int w4a16_upload_head(w4a16_dec* dec, const void* w_bf16_host, size_t bytes, int
         e = cudaMemcpyAsync(stage, (const unsigned char*)w_bf16_host + (size_t)r0 * k * 2, (size_t)rows * k * 2,
                             cudaMemcpyHostToDevice, d.stream);
         if (e == cudaSuccess) {
-            w4::head_quant_kernel<<<rows, 256, 0, d.stream>>>(stage, q + (size_t)r0 * k, sc + r0, k);
+            w4::head_quant_kernel<<<r0 + rows == n ? n16 - r0 : rows, 256, 0, d.stream>>>(stage, q, sc, r0, n, k);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
@@ -299,17 +375,33 @@ int w4a16_head_unpack(w4a16_dec* dec, void* q_host, void* scale_host) {
         return d.fail("w4a16 head: no lm-head uploaded");
     }
     cudaSetDevice(d.device);
-    const size_t nb = (size_t)d.head_n * d.head_k;
-    cudaError_t e = cudaMemcpy(q_host, d.head_q, nb, cudaMemcpyDeviceToHost);
+    // 32 MB of whole row blocks at a time, from the resident order to rows, offset-binary -> two's complement
+    const int k = d.head_k, rows_chunk = (int)std::max<size_t>(16, ((size_t)32 << 20) / k / 16 * 16);
+    std::vector<unsigned char> tiles;
+    cudaError_t e = cudaSuccess;
+    try {
+        tiles.resize((size_t)std::min(rows_chunk, (d.head_n + 15) / 16 * 16) * k);
+    } catch (const std::bad_alloc&) {
+        return d.fail("w4a16 head_unpack: out of host memory");
+    }
+    for (int r0 = 0; r0 < d.head_n && e == cudaSuccess; r0 += rows_chunk) {
+        const int rows = std::min(rows_chunk, d.head_n - r0);
+        e = cudaMemcpy(tiles.data(), d.head_q + (size_t)r0 * k, (size_t)((rows + 15) / 16 * 16) * k, cudaMemcpyDeviceToHost);
+        for (int r = 0; r < rows && e == cudaSuccess; ++r) {
+            unsigned char* dst = (unsigned char*)q_host + (size_t)(r0 + r) * k;
+            for (int c = 0; c < k; c += 16) {
+                const unsigned char* src = tiles.data() + w4::head_at((size_t)r, c, k);
+                for (int i = 0; i < 16; ++i) {
+                    dst[c + i] = src[i] ^ 0x80;
+                }
+            }
+        }
+    }
     if (e == cudaSuccess && scale_host) {
         e = cudaMemcpy(scale_host, d.head_scale, (size_t)d.head_n * 4, cudaMemcpyDeviceToHost);
     }
     if (e != cudaSuccess) {
         return d.cuda_fail("read lm-head", e);
-    }
-    unsigned char* b = (unsigned char*)q_host;   // offset-binary -> two's complement
-    for (size_t i = 0; i < nb; ++i) {
-        b[i] ^= 0x80;
     }
     return 0;
 }
@@ -340,8 +432,21 @@ int w4a16_head_forward(w4a16_dec* dec, const float* x32_dev, float* out_dev, int
         a.k = d.head_k;
         a.t0 = t0;
         a.tp = std::min(tp_max, t - t0);
-        w4::head_gemv_i8_kernel<<<grid, w4::HEAD_THREADS, 2 * (size_t)a.tp * xrow, st>>>(a);
-        cudaError_t e = cudaGetLastError();
+        const int depth = w4::head_depth(2 * (size_t)a.tp * xrow);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(w4::HEAD_THREADS);
+        cfg.dynamicSmemBytes = 2 * (size_t)a.tp * xrow + (size_t)depth * (w4::HEAD_THREADS / 32 * 1024);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        if (d.tune_pdl) {
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+        }
+        void* args[] = {&a};
+        cudaError_t e = cudaLaunchKernelExC(&cfg, w4::head_kernel(depth), args);
         if (e != cudaSuccess) {
             return d.cuda_fail("launch lm-head gemv", e);
         }
