@@ -179,7 +179,8 @@ int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, i
 
 // Which form of the decode GEMV serves a call, with its plan and the scratch it needs.  Shared by Dec::gemv and
 // the allocation-free entry point, so that both launch the same kernel with the same plan.
-int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, GemvChoice& c) {
+// `single`: a call through the single-linear entry points (w4a16_sk_single_dev and its twin with its own scratch).
+int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single, GemvChoice& c) {
     const int t = a.m;
     c = GemvChoice{};
     c.grid_x = gemv_plan_ctas(a);   // 256-row blocks over all segments
@@ -198,6 +199,26 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, GemvChoice& 
             return fail("w4a16 allreduce gemv: n=%d exceeds the exchange buffer (%d rows)", a.seg[0].n, tp_max_rows);
         }
         a.tp = tp;
+    }
+    // The row-group form (gemv_rg.cu) takes every call whose activations fit in shared memory beside its rings (t x K up to about 95000)
+    // unless a tuning key asks for another form, or the sums go on to other GPUs.  Single-linear calls of up to four tokens that the
+    // row-block form takes stay with it (below): that entry point and its allocation-free twin are where the form of a call is pinned,
+    // and replay to the same bits is what they are used for; the row-group form is 1.1 to 1.5 times as fast there, too, and
+    // w4a16_lin_forward runs it.
+    const bool stock = tune_gemv_rowblock == 1 && tune_gemv_rowblock_units && tune_gemv_persistent == 1 && tune_gemv_cluster &&
+                       tune_gemv_subnormal && tune_gemv_ksplit == 0;
+    const bool rowgroup = tune_gemv_rowgroup > 0 && stock && !allreduce;
+    auto choose_rowgroup = [&]() {
+        const int forced = tune_gemv_rowgroup - 1;
+        if (!rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg)) {
+            return false;
+        }
+        c.form = GemvChoice::ROWGROUP;
+        a.ksplit = 1;
+        return true;
+    };
+    if (rowgroup && !single && choose_rowgroup()) {
+        return 0;
     }
     // Up to four tokens of a g128 linear with K <= 6144 and at most 48 MB of weights: CTAs that own whole rows, no
     // scratch, no ticket (gemv_rb.cu).  At its 16 warps per SM it streams at 4 to 4.7 TB/s, the persistent form's bulk
@@ -221,6 +242,9 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, GemvChoice& 
         c.grid_x = gemv_rb_plan(a, sm_count, c.rbw);
         a.ksplit = 1;
         snprintf(c.name, sizeof(c.name), "%s", gemv_rb_variant(a, c.grid_x, c.rbw, sm_count));
+        return 0;
+    }
+    if (rowgroup && single && choose_rowgroup()) {
         return 0;
     }
     const bool prefer_split = rb_ok && rb_shape && !rb_tokens && tune_gemv_persistent < 2;
@@ -268,6 +292,9 @@ int Dec::gemv_run(GemvArgs& a, const GemvChoice& c, cudaStream_t st) {
     case GemvChoice::PERSISTENT:
         e = launch_gemv_sk(a, c.sk, st);
         break;
+    case GemvChoice::ROWGROUP:
+        e = launch_gemv_rg(a, c.rg, st);
+        break;
     case GemvChoice::ROWBLOCK:
         e = launch_gemv_rb(a, c.grid_x, c.rbw, sm_count, st);
         break;
@@ -278,13 +305,13 @@ int Dec::gemv_run(GemvArgs& a, const GemvChoice& c, cudaStream_t st) {
     if (e != cudaSuccess) {
         return cuda_fail("launch gemv", e);
     }
-    last_kernel = c.name;
+    last_kernel = c.form == GemvChoice::ROWGROUP ? gemv_rg_name(a.group, c.rg) : c.name;
     launches++;
     return 0;
 }
 
 int Dec::gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, int t, int out_kind,
-              cudaStream_t st, bool allreduce) {
+              cudaStream_t st, bool allreduce, bool single) {
     if (t < 1 || t > GEMV_MAX_M) {
         return fail("w4a16 gemv: t=%d outside 1..%d", t, GEMV_MAX_M);
     }
@@ -318,7 +345,7 @@ int Dec::gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, 
         }
     }
     GemvChoice c;
-    if (int rc = gemv_select(a, allreduce, false, c)) {
+    if (int rc = gemv_select(a, allreduce, false, single, c)) {
         return rc;
     }
     if (int rc = ensure_scratch(c.part_floats, (int)c.tickets, st)) {
@@ -489,6 +516,9 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
             e = w4::gemv_rb_init_device();
         }
         if (e == cudaSuccess) {
+            e = w4::gemv_rg_init_device();
+        }
+        if (e == cudaSuccess) {
             e = w4::gemv_moe_init_device();
         }
     }
@@ -646,6 +676,14 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
             return d.fail("w4a16 set_tuning: moe_gemv=%d (0, 1, 2, 4 or 8)", value);
         }
         d.tune_moe_gemv = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemv_rowgroup")) {
+        const int nr = (value - 1) & 15, kw = (value - 1) >> 4;
+        if (value != 0 && value != 1 && ((nr != 2 && nr != 3 && nr != 4) || (kw != 4 && kw != 8))) {
+            return d.fail("w4a16 set_tuning: gemv_rowgroup=%d (0, 1, or 1 + row blocks per warp (2..4) + 16 * warps along K (4, 8))", value);
+        }
+        d.tune_gemv_rowgroup = value;
         return 0;
     }
     if (!strcmp(key, "gemv_stages")) {
@@ -921,7 +959,7 @@ int w4a16_sk_single_dev(w4a16_dec* dec, const char* name, const void* x16_dev, v
     }
     const Lin* ls[1] = {l};
     void* outs[1] = {out_dev};
-    return d.gemv(ls, 1, x16_dev, outs, t, out_kind, pick_stream(dec, stream));
+    return d.gemv(ls, 1, x16_dev, outs, t, out_kind, pick_stream(dec, stream), false, /*single=*/true);
 }
 
 // ---- row-parallel tensor parallelism ----------------------------------------------------------------

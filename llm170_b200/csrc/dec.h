@@ -43,8 +43,9 @@ struct MoeBufs {
 
 // The form of the decode GEMV chosen for a call (Dec::gemv_select).
 struct GemvChoice {
-    enum Form { PERSISTENT, SPLIT, ROWBLOCK } form = SPLIT;
+    enum Form { PERSISTENT, SPLIT, ROWBLOCK, ROWGROUP } form = SPLIT;
     SkPlan sk{};
+    RgPlan rg{};
     int grid_x = 0;            // 256-row blocks over all segments (16-row blocks in the row-block form)
     size_t part_floats = 0;    // partial-sum scratch the launch needs
     size_t tickets = 0;        // arrival tickets the launch needs
@@ -98,6 +99,7 @@ struct Dec {
     int tune_gemv_cluster = 1;   // K splits of a row block as a thread-block cluster (DSMEM reduce) when 2 <= ksplit <= 8
     int tune_gemv_subnormal = 1;
     int tune_moe_gemv = 0;       // MoE decode: 0 = automatic, 1 = (row block, K split) form, 2 / 4 / 8 = warps along K of gemv_moe.cu
+    int tune_gemv_rowgroup = 1;  // the row-group form: 0 = never, 1 = where it fits, else 1 + row blocks per warp + 16 * warps along K
     int tune_pdl = 1;
     int tune_tp_wait_log2 = 31;  // the fused all-reduce gives up on its peers after 2^this cycles
     int tune_gemm_mt = 0;        // 128-token blocks per GEMM tile: 0 = automatic, 1 or 2
@@ -124,10 +126,10 @@ struct Dec {
     int upload_common(const char* name, const void* q_dev, const void* s_dev, int n, int k, int group,
                       int scale_bf16, int glu_f = 0);
     std::string last_kernel;   // instantiation launched by the last forward call
-    int gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, GemvChoice& c);
+    int gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single, GemvChoice& c);
     int gemv_run(GemvArgs& a, const GemvChoice& c, cudaStream_t st);
     int gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, int t, int out_kind,
-             cudaStream_t st, bool allreduce = false);
+             cudaStream_t st, bool allreduce = false, bool single = false);
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     void ts_query_clusters();
     TsChoice gemm_ts_choose(int n, int k, int t) const;

@@ -8,36 +8,32 @@
 // spent 84 warp instructions per tile (22 us per 256-row CTA of 128 experts x 1536 x 2048, 17.5 of them in its loop).  Here
 //   * a warp multiplies four row blocks with the same activations, so their loads and the zero-point term are shared by four
 //     tiles, and four independent chains hide the latency of the MMAs;
-//   * the zero-point term of a group, -8 * sum(x), is the sum of two MMAs whose A operand is the constant -8 in the nibbles' own
-//     scalings, and opens the chains of the four row blocks as their C operand: no pass over x, no table of sums, no add;
+//   * the zero-point term of a group is the sum of two MMAs with a constant operand and opens the chains of the four row blocks
+//     (gemv_rg.cuh): no pass over x, no table of sums, no add;
 //   * the CTAs are persistent (two per SM) and take equal contiguous runs of (segment, 128 or 256 rows) units: the weights of the
 //     next unit are on the way while the last one is summed, and the activations stay in shared memory for a segment's units;
 //   * every warp streams its own tiles into its own ring with asynchronous copies: no producer, no barrier in the loop.
 #include <cuda_fp16.h>
 
-#include "gemv_common.cuh"
+#include "gemv_rg.cuh"
 
 namespace w4 {
 
 namespace {
 
-constexpr int GM_WARPS = 8;
-constexpr int GM_THREADS = GM_WARPS * 32;
 constexpr int GM_NR = 4;                                      // row blocks per warp
 constexpr int D = 2;                                          // ring slots per warp (3 and 4 measured the same)
-constexpr int GM_W_BYTES = GM_NR * TILE_WORDS * 4;            // weights of a slot: one k-block
 constexpr int GM_SMEM_MAX = 224 * 1024;
-__host__ __device__ constexpr int gm_slot(int group) { return GM_W_BYTES + GM_NR * 32 * (group == 32 ? 2 : 1); }
 
 // KW = warps along K; the other warps of a CTA take further row blocks.
 template <int GROUP, int KW>
-__global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs a, const MoeGemvPlan p) {
+__global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs a, const MoeGemvPlan p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long s_xbar;
     __shared__ int s_abort;
-    constexpr int RW = GM_WARPS / KW, UR = RW * GM_NR;        // row blocks of a unit
+    constexpr int RW = RG_WARPS / KW, UR = RW * GM_NR;        // row blocks of a unit
     constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
-    constexpr uint32_t SLOT = gm_slot(GROUP);
+    constexpr uint32_t SLOT = rg_slot_bytes(GROUP, GM_NR);
     if (a.tables_fresh) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
@@ -52,55 +48,25 @@ __global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     }
     const int ku = a.k / (TILE_K * KPU), ng = a.k / GROUP;
     const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks
-    const size_t pitch = (size_t)a.nrb_w * 32;                // uint4 between k-blocks
 
-    // ---- weights and scales: slots of one k-block of the warp's row blocks, requested in the order of use.  Row blocks past the
-    // expert's last one read that one again.
+    // ---- weights and scales, in the order of use.  Row blocks past the expert's last one read that one again.
     const uint32_t ring = smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * SLOT);
     int fu = u0, fi = 0;
     int fexp = a.tile_expert[u0 / upe];                       // expert of unit fu
-    const uint4* fq = nullptr;
-    const uint32_t* fs = nullptr;
-    int fstep[GM_NR];                                         // offset of the warp's r-th row block
+    uint32_t fdst = 0;
+    RgCursor<GROUP, GM_NR> cur;
     auto fetch_unit = [&]() {
-        const int sub = fu % upe, rb = sub * UR + rw * GM_NR, base = (fexp - a.expert0) * nrb;
-#pragma unroll
-        for (int r = 0; r < GM_NR; ++r) {
-            fstep[r] = (base + min(rb + r, nrb - 1)) * 32;
-        }
-        fq = a.seg[0].qt + (size_t)kb0 * pitch + lane;
-        // scale words: 16 bytes per lane; row block lane / (pieces per slot)
-        constexpr int SP = GROUP == 32 ? 4 : 2;
-        fs = a.seg[0].st + (size_t)(base + min(rb + lane / SP % GM_NR, nrb - 1)) * ng * 8 + (size_t)kb0 * TILE_K / GROUP * 8 + (lane % SP) * 4;
+        cur.init(a.seg[0].qt, a.seg[0].st, (fexp - a.expert0) * nrb, fu % upe * UR + rw * GM_NR, nrb, a.nrb_w, ng, kb0, lane);
         fi = 0;
         if (fu + 1 < u1) {
             fexp = a.tile_expert[(fu + 1) / upe];
         }
     };
-    uint32_t fdst = 0;
     auto fetch = [&]() {
         if (fu < u1) {
-            const uint32_t dst = ring + fdst;
-#pragma unroll
-            for (int r = 0; r < GM_NR; ++r) {
-                cp_async_16(dst + (uint32_t)r * 512u + (uint32_t)lane * 16u, fq + fstep[r]);
-            }
-            if (GROUP == 32) {
-                if (lane < 4 * GM_NR) {
-                    cp_async_16(dst + GM_W_BYTES + (uint32_t)lane * 16u, fs);
-                }
-                fs += 16;
-            } else if (fi & 1) {                              // with a group's second k-block, after which it is needed
-                if (lane < 2 * GM_NR) {
-                    cp_async_16(dst + GM_W_BYTES + (uint32_t)lane * 16u, fs);
-                }
-                fs += 8;
-            }
-            fq += pitch;
-            if (++fi == nk) {
-                if (++fu < u1) {
-                    fetch_unit();
-                }
+            cur.fetch(ring + fdst, lane, (fi & 1) != 0);
+            if (++fi == nk && ++fu < u1) {
+                fetch_unit();
             }
         }
         cp_async_commit();
@@ -126,10 +92,8 @@ __global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     // the next kernel may come: what it reads before its own wait was complete before this launch
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    const int xstride = a.k * 2 + 32;                         // bytes; 32 mod 128: conflict-free 8-byte reads of eight rows
+    const int xstride = a.k * 2 + RG_XPAD;
     float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][8 tokens]
-    const uint32_t wl = ring + (uint32_t)lane * 16u;
-    const uint32_t zA[4] = {0x80088008u, 0x80808080u, 0x80088008u, 0x80808080u};   // -8 in the nibbles' two scalings
     uint32_t rslot = 0, xphase = 0;
     int seg = -1, row0 = 0, m = 0;
     uint32_t xl = 0;
@@ -156,135 +120,12 @@ __global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs 
             // lanes without a token read token 0: their columns are never stored
             xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
         }
-        float tot[GM_NR][4], acc[GM_NR][4];
+        float tot[GM_NR][4];
 #pragma unroll
         for (int r = 0; r < GM_NR; ++r) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                tot[r][j] = acc[r][j] = 0.f;
-            }
+            tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
         }
-        uint32_t xa = xl;
-        auto fold = [&](int r, uint32_t s2) {
-            const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&s2));
-            tot[r][0] = fmaf(acc[r][0], sf.x, tot[r][0]);
-            tot[r][1] = fmaf(acc[r][1], sf.x, tot[r][1]);
-            tot[r][2] = fmaf(acc[r][2], sf.y, tot[r][2]);
-            tot[r][3] = fmaf(acc[r][3], sf.y, tot[r][3]);
-        };
-        if (GROUP == 32) {
-            for (int i = 0; i < nk; ++i) {
-                uint2 x[4];
-#pragma unroll
-                for (int w = 0; w < 4; ++w) {
-                    x[w] = lds64(xa + (uint32_t)w * 32u);
-                }
-                xa += TILE_K * 2;
-                cp_async_wait_group<D - 1>();
-                __syncwarp();                                 // the scale words are other lanes' copies
-                uint4 wv[GM_NR];
-                uint32_t sc[GM_NR][2];
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
-                    sc[r][0] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 64u + (uint32_t)g * 4u);
-                    sc[r][1] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 64u + 32u + (uint32_t)g * 4u);
-                }
-                __syncwarp();
-                fetch();
-                if ((rslot += SLOT) == D * SLOT) {
-                    rslot = 0;
-                }
-                float z0[4], z1[4];
-                mma16816_z(z0, zA, x[0].x, x[0].y);
-                mma16816_z(z1, zA, x[2].x, x[2].y);
-                mma16816(z0, zA, x[1].x, x[1].y);
-                mma16816(z1, zA, x[3].x, x[3].y);
-                const float4 c0 = make_float4(z0[0], z0[1], z0[2], z0[3]), c1 = make_float4(z1[0], z1[1], z1[2], z1[3]);
-                uint32_t af[4];
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    nibbles_as_subnormals(wv[r].x, af);
-                    mma16816_c(acc[r], af, x[0].x, x[0].y, c0);
-                }
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    nibbles_as_subnormals(wv[r].y, af);
-                    mma16816(acc[r], af, x[1].x, x[1].y);
-                }
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    fold(r, sc[r][0]);
-                    nibbles_as_subnormals(wv[r].z, af);
-                    mma16816_c(acc[r], af, x[2].x, x[2].y, c1);
-                }
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    nibbles_as_subnormals(wv[r].w, af);
-                    mma16816(acc[r], af, x[3].x, x[3].y);
-                }
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-                    fold(r, sc[r][1]);
-                }
-            }
-        } else {
-            for (int i = 0; i < nk; i += 2) {
-                float z[4];
-                uint32_t sc[GM_NR];
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    uint2 x[4];
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        x[w] = lds64(xa + (uint32_t)w * 32u);
-                    }
-                    xa += TILE_K * 2;
-                    cp_async_wait_group<D - 1>();
-                    __syncwarp();
-                    uint4 wv[GM_NR];
-#pragma unroll
-                    for (int r = 0; r < GM_NR; ++r) {
-                        wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
-                        if (h == 1) {
-                            sc[r] = lds32(ring + rslot + GM_W_BYTES + (uint32_t)r * 32u + (uint32_t)g * 4u);
-                        }
-                    }
-                    __syncwarp();
-                    fetch();
-                    if ((rslot += SLOT) == D * SLOT) {
-                        rslot = 0;
-                    }
-                    uint32_t af[4];
-#pragma unroll
-                    for (int w = 0; w < 4; ++w) {
-                        const bool open = h == 0 && w == 0;
-                        if (open) {
-                            mma16816_z(z, zA, x[w].x, x[w].y);
-                        } else {
-                            mma16816(z, zA, x[w].x, x[w].y);
-                        }
-#pragma unroll
-                        for (int r = 0; r < GM_NR; ++r) {
-                            nibbles_as_subnormals(w == 0 ? wv[r].x : w == 1 ? wv[r].y : w == 2 ? wv[r].z : wv[r].w, af);
-                            if (open) {
-                                mma16816_z(acc[r], af, x[w].x, x[w].y);
-                            } else {
-                                mma16816(acc[r], af, x[w].x, x[w].y);
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < GM_NR; ++r) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        acc[r][j] += z[j];
-                    }
-                    fold(r, sc[r]);
-                }
-            }
-        }
+        rg_multiply<GROUP, GM_NR, D>(tot, xl, nk, ring, rslot, lane, fetch);
         // ---- the K warps' sums meet in shared memory
         const int rb0 = u % upe * UR, rows = min(UR, nrb - rb0) * TILE_ROWS;
         if (u > u0) {
@@ -311,14 +152,14 @@ __global__ void __launch_bounds__(GM_THREADS, 2) gemv_moe_kernel(const GemvArgs 
             // rows further
             const int nout = rows / 2, nh = a.seg[0].n / 2;
             __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * nh + (size_t)rb0 * (TILE_ROWS / 2);
-            for (int e = threadIdx.x; e < nout * m; e += GM_THREADS) {
+            for (int e = threadIdx.x; e < nout * m; e += RG_THREADS) {
                 const int tok = e / nout, o = e - tok * nout;
                 const int lg = (o / TILE_ROWS) * 2 * TILE_ROWS + (o % TILE_ROWS);
                 ob[(size_t)tok * nh + o] = silu_mul_f16(sum_of(lg, tok), sum_of(lg + TILE_ROWS, tok));
             }
         } else {
             __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * a.seg[0].n + (size_t)rb0 * TILE_ROWS;
-            for (int e = threadIdx.x; e < rows * m; e += GM_THREADS) {
+            for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
                 const int tok = e / rows, row = e - tok * rows;
                 float v = sum_of(row, tok);
                 if (a.row_w != nullptr) {
@@ -345,17 +186,17 @@ const void* gm_kernel(int group, int kw) {
 // form: 128 experts x 2048 x 768, groups of 32: 64 tokens 97 / 102 / 118, 125; 8 tokens 61 / 55 / 57, 71; 1 token 38 / 29 / 26, 32;
 // 64 experts x 1024 x 384: 64 tokens 32.8 / 35.9 / 38.6, 39.1; 128 experts x 1536 x 896: 4 tokens 28.9 / 25.8 / 28.8, 34.1.
 bool moe_gemv_plan(int rows, int k, int group, int sm_count, int segments, int force_kw, MoeGemvPlan& p) {
-    const int x = GEMV_MAX_M * (k * 2 + 32), red = GM_WARPS * GM_NR * TILE_ROWS * GEMV_MAX_M * 4;
+    const int x = GEMV_MAX_M * (k * 2 + RG_XPAD), red = RG_WARPS * GM_NR * TILE_ROWS * GEMV_MAX_M * 4;
     p.off_red = (x + 127) & ~127;
     p.off_ring = p.off_red + red;
-    p.smem = p.off_ring + D * GM_WARPS * gm_slot(group);
+    p.smem = p.off_ring + D * RG_WARPS * rg_slot_bytes(group, GM_NR);
     if (p.smem > GM_SMEM_MAX) {
         return false;
     }
     p.ctas = (p.smem <= GM_SMEM_MAX / 2 ? 2 : 1) * sm_count;
     long long best = -1;
     for (int kw = 2; kw <= 8; kw *= 2) {
-        const int unit_rows = GM_WARPS / kw * GM_NR * TILE_ROWS;
+        const int unit_rows = RG_WARPS / kw * GM_NR * TILE_ROWS;
         const long long units = (long long)segments * ((rows + unit_rows - 1) / unit_rows);
         const long long cost = (units + p.ctas - 1) / p.ctas * ((k / TILE_K + kw - 1) / kw + 5);
         if (force_kw > 1 ? kw == force_kw : (best < 0 || cost < best)) {
@@ -381,7 +222,7 @@ cudaError_t gemv_moe_init_device() {
 cudaError_t launch_gemv_moe(const GemvArgs& a, const MoeGemvPlan& p, cudaStream_t st) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.ctas);
-    cfg.blockDim = dim3(GM_THREADS);
+    cfg.blockDim = dim3(RG_THREADS);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

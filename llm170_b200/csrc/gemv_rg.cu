@@ -1,0 +1,281 @@
+// Decode GEMV for 1..8 tokens, row-group form: a warp multiplies two to four 16-row blocks with the same activations, the eight warps of a
+// CTA share K (or K and the rows), and a CTA holds all of K for its rows.
+//
+// Takes the place of the reference's split-K GEMV pair and small-batch family
+// (crates/backend-gpu/src/rawcuda/assets/decode.cu:46-267, crates/backend-gpu/src/rawcuda/assets/gptq4.cu:44-723).  Same arithmetic as the
+// other decode forms: mma.sync m16n8k16 with the weight tile as the 16-row operand, raw nibbles as exact f16 subnormals, f32 sums, the f32
+// group scale on a group's sum.
+//
+// What bounded the forms before it were issued instructions -- 56 per 512-byte tile in the persistent form, most of them loads of
+// activations, zero-point terms and scales for two row blocks at a time -- and what surrounds the stream: tickets and sums across CTAs, a
+// pass over x for the zero points, a producer's barriers.  Here
+//   * the loads of x and the zero-point MMAs are shared by NR row blocks, whose chains hide the latency of the MMAs (gemv_rg.cuh);
+//   * every warp streams its own tiles and scales into its own ring with asynchronous copies, requested before the dependency wait and
+//     refilled across units: no producer, no barrier in the loop, nothing of the copy engine, which takes 60 ns for each copy;
+//   * the warps' sums meet in shared memory once per unit; nothing is shared between CTAs.
+// One token, us per launch, this form against the best of the others: 7168 x 5120 6.6 / 7.2, 5120 x 6144 6.2 / 7.5, 34816 x 5120
+// 17.3 / 21.6 (5.3 TB/s), 5120 x 17408 13.0 / 13.8, 24576 x 4096 12.0 / 15.9; eight tokens: 7.4 / 10.3, 6.6 / 10.2, 20.5 / 26.2;
+// 34816 x 5120 in groups of 32, eight tokens: 21.7 / 48.9.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "gemv_rg.cuh"
+
+namespace w4 {
+
+namespace {
+
+// KW = warps along K; the other warps of a CTA take further row blocks.  NR = row blocks per warp, D = ring slots per warp.
+template <int GROUP, int KW, int NR, int D>
+__global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a, const RgPlan p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_xbar;
+    __shared__ int s_abort;
+    constexpr int RW = RG_WARPS / KW, UR = RW * NR;           // row blocks of a unit
+    constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
+    constexpr uint32_t SLOT = rg_slot_bytes(GROUP, NR);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // optional timeline (diagnostic; a.dbg is null in normal runs): wall-clock stamps of thread 0 in the slots of the other forms
+    auto stamp_now = [&](int j) {
+        if (a.dbg != nullptr && threadIdx.x == 0 && (int)blockIdx.x < DBG_CTAS) {
+            unsigned long long ns;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(ns));
+            a.dbg[((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS + j] = (long long)ns;
+        }
+    };
+    stamp_now(0);
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int kw = warp % KW, rw = warp / KW;
+    // equal contiguous runs of units (row groups over all segments)
+    const int u0 = (int)((long long)p.units * blockIdx.x / gridDim.x), u1 = (int)((long long)p.units * (blockIdx.x + 1) / gridDim.x);
+    const int ku = a.k / (TILE_K * KPU), ng = a.k / GROUP;
+    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks
+    auto seg_of = [&](int u) {
+        int si = 0;
+#pragma unroll
+        for (int i = 1; i < GEMV_MAX_SEG; ++i) {
+            if (i < a.nseg && u >= a.seg[i].cta0) {
+                si = i;
+            }
+        }
+        return si;
+    };
+
+    // ---- weights and scales, in the order of use
+    const uint32_t ring = smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * SLOT);
+    int fu = u0, fi = 0;
+    uint32_t fdst = 0;
+    RgCursor<GROUP, NR> cur;
+    auto fetch_unit = [&]() {
+        const int si = seg_of(fu), nrb = a.seg[si].n / TILE_ROWS;
+        cur.init(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, kb0, lane);
+        fi = 0;
+    };
+    auto fetch = [&]() {
+        if (fu < u1) {
+            cur.fetch(ring + fdst, lane, (fi & 1) != 0);
+            if (++fi == nk && ++fu < u1) {
+                fetch_unit();
+            }
+        }
+        cp_async_commit();
+        if ((fdst += SLOT) == D * SLOT) {
+            fdst = 0;
+        }
+    };
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        mbar_init(smem_u32(&s_xbar), 1);
+        mbar_init_fence();
+        if (a.dbg != nullptr && (int)blockIdx.x < DBG_CTAS) {
+            unsigned smid;
+            asm volatile("mov.u32 %0, %smid;" : "=r"(smid));
+            long long* d = a.dbg + ((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS;
+            d[6] = smid;
+            d[7] = u1 - u0;
+        }
+    }
+    if (nk > 0) {
+        fetch_unit();
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            fetch();
+        }
+    }
+    stamp_now(8);   // first tiles requested
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // x and the outputs may be the previous kernel's
+    stamp_now(1);
+
+    // ---- activations: one bulk copy per token
+    const int m = a.m, xstride = a.k * 2 + RG_XPAD;
+    if (warp == 0) {
+        if (lane == 0) {
+            mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * a.k * 2));
+        }
+        __syncwarp();
+        if (lane < m) {
+            bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k, (uint32_t)(a.k * 2), smem_u32(&s_xbar));
+        }
+    }
+    mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16));
+    __syncwarp();
+    stamp_now(2);   // x staged
+    stamp_now(3);
+    // lanes without a token read token 0: their columns are never stored
+    const uint32_t xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
+    const int mp = (m + 1) & ~1;
+    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][mp]
+    uint32_t rslot = 0;
+    for (int u = u0; u < u1; ++u) {
+        float tot[NR][4];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
+        }
+        rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, rslot, lane, fetch);
+        stamp_now(4);   // (of the last unit)
+        // ---- the K warps' sums meet in shared memory
+        const GemvSeg& sg = a.seg[seg_of(u)];
+        const int rb0 = (u - sg.cta0) * UR, rows = min(UR, sg.n / TILE_ROWS - rb0) * TILE_ROWS;
+        if (u > u0) {
+            __syncthreads();
+        }
+        if (2 * t < mp) {
+            const float m0 = 16777216.f * sg.out_mul, m1 = 1048576.f * sg.out_mul;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                float* d = red + ((size_t)kw * (UR * TILE_ROWS) + (rw * NR + r) * TILE_ROWS + g) * mp + 2 * t;
+                *reinterpret_cast<float2*>(d) = make_float2(tot[r][0] * m0, tot[r][1] * m0);
+                *reinterpret_cast<float2*>(d + 8 * mp) = make_float2(tot[r][2] * m1, tot[r][3] * m1);
+            }
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
+            const int tok = e / rows, row = e - tok * rows;
+            float v = red[row * mp + tok];
+#pragma unroll
+            for (int w = 1; w < KW; ++w) {
+                v += red[(w * (UR * TILE_ROWS) + row) * mp + tok];      // fixed order: the same bits every run
+            }
+            const size_t o = (size_t)tok * sg.n + (size_t)rb0 * TILE_ROWS + row;
+            if (a.out_f16) {
+                reinterpret_cast<__half*>(sg.out)[o] = __float2half_rn(v);
+            } else {
+                reinterpret_cast<float*>(sg.out)[o] = v;
+            }
+        }
+    }
+    stamp_now(5);   // sums stored
+}
+
+struct RgKernel {
+    int group, kw, nr, depth;
+    const void* f;
+    const char* name;
+};
+#define W4_RG(G, K, N, D) {G, K, N, D, (const void*)gemv_rg_kernel<G, K, N, D>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
+#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2), W4_RG(G, K, N, 4), W4_RG(G, K, N, 6)
+#define W4_RG_N(G, K) W4_RG_D(G, K, 2), W4_RG_D(G, K, 3), W4_RG_D(G, K, 4)
+const RgKernel rg_kernels[] = {W4_RG_N(128, 4), W4_RG_N(128, 8), W4_RG_N(32, 4), W4_RG_N(32, 8)};
+#undef W4_RG_N
+#undef W4_RG_D
+#undef W4_RG
+const RgKernel& rg_kernel(int group, const RgPlan& p) {
+    return rg_kernels[(group == 128 ? 0 : 18) + (p.kw == 4 ? 0 : 9) + (p.nr - 2) * 3 + p.depth / 2 - 1];
+}
+
+constexpr int RG_SMEM_MAX = 224 * 1024, RG_SMEM_TWO = 112 * 1024;
+
+}  // namespace
+
+// Row blocks per warp, warps along K and CTAs per SM with the least estimated time, in tiles of work on the fullest SM; fills seg[].cta0.
+// A CTA alone on its SM has eight warps to hide latency, two have sixteen: half as much again per tile alone.  Fewer row blocks per warp
+// share less (two: 1.3, three: 1.05 per tile).  A unit costs about twenty tiles beside its own for its sums.  Best of the twelve ways
+// measured, and the choice: 7168 x 5120 (448 row blocks) 6.6: 4 row blocks, 8 warps, alone; 5120 x 6144 6.2: 3, 8, alone; 12544 x 4224
+// 7.6: 3, 8, two (alone 8.5); 24576 x 4096 12.0: 3, 4, two (4, 8, alone 12.9); 34816 x 5120 17.3: 4, 4, two (4, 8, two 17.7).
+// false: x does not fit in shared memory beside two slots per warp.
+bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& best) {
+    const int unit_k = a.group > TILE_K ? a.group : TILE_K, ku = a.k / unit_k, mp = (a.m + 1) & ~1;
+    const int x_bytes = (a.m * (a.k * 2 + RG_XPAD) + 127) & ~127;
+    double cost = -1.0;
+    for (int kw : {4, 8}) {
+        for (int nr : {4, 3, 2}) {
+            if ((force_nr > 0 && nr != force_nr) || (force_kw > 0 && kw != force_kw)) {
+                continue;
+            }
+            const int ur = RG_WARPS / kw * nr, slot = rg_slot_bytes(a.group, nr);
+            RgPlan p{};
+            p.nr = nr;
+            p.kw = kw;
+            for (int i = 0; i < a.nseg; ++i) {
+                p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
+            }
+            p.off_red = x_bytes;
+            p.off_ring = (x_bytes + kw * ur * TILE_ROWS * mp * 4 + 127) & ~127;
+            const double tiles = (double)((ku + kw - 1) / kw * (unit_k / TILE_K) * nr) * (nr == 2 ? 1.3 : nr == 3 ? 1.05 : 1.0);
+            for (int per_sm = 1; per_sm <= 2; ++per_sm) {
+                const int room = per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX;
+                if (p.off_ring + 2 * RG_WARPS * slot > room || (per_sm == 2 && p.units <= sm_count)) {
+                    continue;
+                }
+                p.ctas = std::min(p.units, per_sm * sm_count);
+                const int rounds = (p.units + p.ctas - 1) / p.ctas;
+                const double c = rounds * (per_sm == 1 ? 1.5 * tiles + 20.0 : 2.0 * (tiles + 20.0));
+                if (cost < 0.0 || c < cost) {
+                    cost = c;
+                    best = p;
+                    // alone: as deep a ring as fits; two: two slots (four measured the same)
+                    best.depth = per_sm == 2 ? 2 : p.off_ring + 6 * RG_WARPS * slot <= room ? 6 : p.off_ring + 4 * RG_WARPS * slot <= room ? 4 : 2;
+                    best.smem = p.off_ring + best.depth * RG_WARPS * slot;
+                    if (per_sm == 1) {
+                        best.smem = std::max(best.smem, RG_SMEM_TWO + 2048);      // no second CTA of this launch on the SM
+                    }
+                }
+            }
+        }
+    }
+    if (cost < 0.0) {
+        return false;
+    }
+    int units = 0;
+    for (int i = 0; i < a.nseg; ++i) {
+        const int ur = RG_WARPS / best.kw * best.nr;
+        a.seg[i].cta0 = units;
+        units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
+    }
+    return true;
+}
+
+const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(group, p).name; }
+
+cudaError_t gemv_rg_init_device() {
+    for (const RgKernel& k : rg_kernels) {
+        const cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM_MAX);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(p.ctas);
+    cfg.blockDim = dim3(RG_THREADS);
+    cfg.dynamicSmemBytes = p.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (a.pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    void* args[] = {const_cast<GemvArgs*>(&a), const_cast<RgPlan*>(&p)};
+    return cudaLaunchKernelExC(&cfg, rg_kernel(a.group, p).f, args);
+}
+
+}  // namespace w4

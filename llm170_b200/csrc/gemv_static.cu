@@ -89,7 +89,7 @@ extern "C" int w4a16_sk_single_static(w4a16_dec* dec, const char* name, const vo
     cudaStream_t st = stream ? (cudaStream_t)stream : d.stream;
     // the same kernel form and plan as w4a16_sk_single_dev (shared selection), so the two give identical results
     GemvChoice c;
-    if (int rc = d.gemv_select(a, false, true, c)) {
+    if (int rc = d.gemv_select(a, false, true, true, c)) {
         return rc;
     }
     const size_t need = c.part_floats * sizeof(float);

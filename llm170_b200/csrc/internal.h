@@ -142,6 +142,19 @@ size_t sk_part_floats(const SkPlan& p);   // scratch for parked partial sums; co
 cudaError_t launch_gemv_sk(const GemvArgs& a, const SkPlan& p, cudaStream_t st);
 cudaError_t gemv_sk_init_device();
 cudaError_t gemv_rb_init_device();
+// ---- gemv_rg.cu: the row-group form of the decode GEMV ----
+struct RgPlan {
+    int nr, kw;              // row blocks per warp, warps along K
+    int units;               // row groups over all segments (seg[].cta0 = first of the segment)
+    int ctas;                // CTA c takes units [units c / ctas, units (c + 1) / ctas)
+    int depth;               // ring slots per warp
+    int off_red, off_ring;   // byte offsets in dynamic shared memory: activations first
+    int smem;
+};
+bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& p);
+cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st);
+cudaError_t gemv_rg_init_device();
+const char* gemv_rg_name(int group, const RgPlan& p);
 // ---- gemv_moe.cu: grouped GEMV of the MoE decode path ----
 struct MoeGemvPlan {
     int kw;                  // warps along K: 2, 4 or 8

@@ -547,3 +547,58 @@ def test_row_block_form_units_and_edges(dec, orc, n, k, t):
     dec.sync()
     assert torch.equal(y16, y.to(torch.float16))
     dec.drop_lin("rbu")
+
+
+# The row-group form: units that the last rows do not fill, more units than CTAs, fewer k-blocks than warps, an odd number of k-blocks,
+# every group size and scale type, one to eight tokens, every way of dealing rows and K to the warps (0: chosen).
+@pytest.mark.parametrize("way", [0, (2, 8), (3, 8), (4, 8), (2, 4), (3, 4), (4, 4)])
+@pytest.mark.parametrize("n,k,group,t,bf16", [(16, 128, 128, 1, False), (48, 192, 32, 5, False), (272, 576, 64, 3, False), (1040, 1152, 128, 8, False),
+                                             (2064, 320, 32, 8, True), (20000, 256, 128, 2, True), (38000, 128, 64, 4, False), (512, 4096, 128, 7, False)])
+def test_row_group_form(dec, orc, n, k, group, t, bf16, way):
+    q, s = synth.make_linear(n, k, group, seed=900 + n % 97)
+    if bf16:
+        s = np.ascontiguousarray((s.view(np.float16).astype(np.float32).view(np.uint32) >> 16).astype(np.uint16))
+        want_s = (s.astype(np.uint32) << 16).view(np.float32).astype(np.float16).view(np.uint16)   # exact: 8 bits of mantissa
+    else:
+        want_s = s
+    dec.upload_lin_g("rg", q, s, n, k, group, scale_bf16=bf16)
+    xs = synth.make_acts(t, k, seed=910 + t)
+    guard = torch.full((t + 1, n), 7.0, device="cuda", dtype=torch.float32)
+    dec.set_tuning("gemv_rowgroup", 1 if way == 0 else 1 + way[0] + 16 * way[1])
+    try:
+        dec.lin_forward("rg", x_dev(xs), t, dst=guard[:t])
+        dec.sync()
+        name = dec.last_kernel()
+        assert name.startswith("gemv_rg_kernel") and (way == 0 or f",{way[1]},{way[0]}," in name), name
+        y = guard[:t].clone()
+        assert torch.equal(dec.lin_forward("rg", x_dev(xs), t, out_f16=True), y.to(torch.float16))
+        outs = dec.sk_multi_dev(["rg", "rg"], x_dev(xs), t=t)
+        assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], y)      # a row's sum does not depend on what is beside it
+        dec.set_tuning("gemv_rowgroup", 0)
+        other = dec.lin_forward("rg", x_dev(xs), t)
+        assert not dec.last_kernel().startswith("gemv_rg_kernel")
+    finally:
+        dec.set_tuning("gemv_rowgroup", 1)
+    rows = (0, n) if n < 4096 else (n - 1024, n)
+    expect = orc.linear_lane(q, want_s, xs, t, n, k, group, rows=rows)
+    assert np.abs(y.cpu().numpy()[:, rows[0]:rows[1]] - expect[:, rows[0]:rows[1]]).max() <= TOL
+    # the general path over all rows: the same f32 terms in another order (at most k of them, 2^-24 each, sum of their sizes as bound)
+    size = (x_dev(xs).float().abs() @ dec.dequant_lin("rg").abs().T).max().item()
+    assert (y - other).abs().max().item() <= 2.0 ** -20 * size
+    assert bool((guard[t:] == 7.0).all())
+    dec.drop_lin("rg")
+
+
+def test_row_group_form_leaves_what_does_not_fit(dec, orc):
+    # eight tokens of 17408 channels are 278 KB: the call keeps the form that stages a part of K at a time
+    n, k, t = 256, 17408, 8
+    q, s = synth.make_linear(n, k, 128, seed=950)
+    dec.upload_lin_g("rgx", q, s, n, k, 128)
+    xs = synth.make_acts(t, k, seed=951)
+    y = dec.lin_forward("rgx", x_dev(xs), t)
+    dec.sync()
+    assert not dec.last_kernel().startswith("gemv_rg_kernel")
+    assert np.abs(y.cpu().numpy() - orc.linear_lane(q, s, xs, t, n, k, 128)).max() <= TOL
+    dec.lin_forward("rgx", x_dev(xs[:1]), 1)
+    assert dec.last_kernel().startswith("gemv_rg_kernel")
+    dec.drop_lin("rgx")
