@@ -48,7 +48,8 @@ constexpr int RAW_BYTES = TS_MROWS * SK / 2;    // 8 KB per stage
 constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
 constexpr int DQ_WARPS = TS_MROWS / TILE_ROWS;  // a warp per 16-row block
 constexpr int TS_THREADS = (3 + DQ_WARPS) * 32;
-constexpr int TS_XBOX = 64;                     // grouped mode: rows of a token box
+constexpr int TS_XBOX = 64;                     // grouped form: rows of a token box
+constexpr int TS_STAGE_BYTES = 16 * 1024;       // grouped form: results on their way out
 constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
 // Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
 // waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
@@ -69,6 +70,7 @@ struct TsArgs {
     int raw_stages, x_stages, a_stages;
     int tmem_cols;
     int off_x, off_bars; // byte offsets in dynamic shared memory (1024-byte aligned base)
+    int off_stage;       // grouped: results of a tile on their way out
     int pdl;
     float out_mul;
     int* status;
@@ -117,7 +119,24 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
     return v;
 }
 
-template <int GROUP, bool GROUPED>
+// A lane's 16 raw bytes of a tile -> its 16 registers of tcgen05.st.16x256b.x4, f16((q - 8) * s): s_a / s_b = scale pair (rows g, g + 8)
+// of the first / second 32 channels.
+__device__ __forceinline__ void ts_expand(const uint4& raw, const uint32_t s_a, const uint32_t s_b, uint32_t (&v)[16]) {
+    const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        uint32_t f[4];
+        dequant_word(rw[w], f);
+        const uint32_t s2 = w < 2 ? s_a : s_b;
+        const uint32_t s_r0 = __byte_perm(s2, s2, 0x1010), s_r1 = __byte_perm(s2, s2, 0x3232);
+        v[4 * w + 0] = hmul2u(f[0], s_r0);
+        v[4 * w + 1] = hmul2u(f[2], s_r0);
+        v[4 * w + 2] = hmul2u(f[1], s_r1);
+        v[4 * w + 3] = hmul2u(f[3], s_r1);
+    }
+}
+
+template <int GROUP>
 __global__ void __launch_bounds__(TS_THREADS, 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
@@ -143,28 +162,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     const uint32_t accum_bar = bars + 8u * (2 * NR + 2 * NX + 2 * NA);
 
     // ---- this CTA's tile ----
-    const int tile = (int)blockIdx.x, ks = GROUPED ? 1 : a.ksplit, split = GROUPED ? 0 : (int)blockIdx.y;
-    int m0, n0, rb0, rows_valid;
-    if (GROUPED) {
-        if (a.tables_fresh) {
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-        }
-        // neighbours share the token rows, then the expert's weights
-        const int mt = tile / a.n_tiles, ntile = tile - mt * a.n_tiles;
-        if (mt >= *a.num_tiles) {
-            return;      // the grid is sized for the worst case
-        }
-        n0 = ntile * TS_MROWS;
-        m0 = a.tile_row0[mt];
-        rows_valid = a.tile_rows[mt];
-        rb0 = ((a.tile_expert[mt] - a.expert0) * a.n + n0) / TILE_ROWS;
-    } else {
-        const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
-        n0 = ntile * TS_MROWS;
-        m0 = mtile * N;
-        rb0 = n0 / TILE_ROWS;
-        rows_valid = min(N, a.m - m0);
-    }
+    const int tile = (int)blockIdx.x, ks = a.ksplit, split = (int)blockIdx.y;
+    const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
+    const int n0 = ntile * TS_MROWS;
+    const int m0 = mtile * N, rb0 = n0 / TILE_ROWS;
+    const int rows_valid = min(N, a.m - m0);
     const int nrbv = min(TS_MROWS, a.n - n0) / TILE_ROWS;       // valid 16-row blocks
     const uint32_t kb_bytes = (uint32_t)nrbv * (TILE_WORDS * 4);
     // K range of this split in stages; the last stage of the matrix may hold one k-block (32-channel groups)
@@ -234,21 +236,9 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 break;
             }
             if (leader) {
-                if (GROUPED) {
-                    // the rows of the tile in boxes of 64 (rows of the next expert, or zeros, fill the last one up)
-                    const int kbs = stage_kbs(it), boxes = (rows_valid + TS_XBOX - 1) / TS_XBOX;
-                    mbar_expect_tx(x_full(sx), (uint32_t)(kbs * boxes) * (TS_XBOX * BK * 2));
-                    for (int h = 0; h < kbs; ++h) {
-                        for (int c = 0; c < boxes; ++c) {
-                            tma_load_2d(x_addr(sx) + h * x_half + (uint32_t)c * (TS_XBOX * BK * 2), &tmap_x, (2 * (st0 + it) + h) * BK,
-                                        m0 + c * TS_XBOX, x_full(sx));
-                        }
-                    }
-                } else {
-                    // both k-blocks in one box (the second one of the last stage may lie outside: zeros)
-                    mbar_expect_tx(x_full(sx), 2 * x_half);
-                    tma_load_3d(x_addr(sx), &tmap_x, 0, m0, 2 * (st0 + it), x_full(sx));
-                }
+                // both k-blocks in one box (the second one of the last stage may lie outside: zeros)
+                mbar_expect_tx(x_full(sx), 2 * x_half);
+                tma_load_3d(x_addr(sx), &tmap_x, 0, m0, 2 * (st0 + it), x_full(sx));
             }
             __syncwarp();
             if (++sx == NX) {
@@ -275,8 +265,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer
-        const int n_mma = GROUPED ? (rows_valid + 15) & ~15 : N;
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(n_mma >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
         const bool leader = elect_one();
         int sx = 0, px = 0, sa = 0, pa = 0;
         for (int it = 0; it < nst; ++it) {
@@ -347,20 +336,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         uint32_t sc_cur = 0;
         const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
         const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
-        auto expand = [&](const uint4& raw, const uint32_t s_a, const uint32_t s_b, uint32_t (&v)[16]) {
-            const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-            for (int w = 0; w < 4; ++w) {
-                uint32_t f[4];
-                dequant_word(rw[w], f);
-                const uint32_t s2 = w < 2 ? s_a : s_b;
-                const uint32_t s_r0 = __byte_perm(s2, s2, 0x1010), s_r1 = __byte_perm(s2, s2, 0x3232);
-                v[4 * w + 0] = hmul2u(f[0], s_r0);
-                v[4 * w + 1] = hmul2u(f[2], s_r0);
-                v[4 * w + 2] = hmul2u(f[1], s_r1);
-                v[4 * w + 3] = hmul2u(f[3], s_r1);
-            }
-        };
         int sr = 0, pr = 0, sa = 0, pa = 1;
         for (int it = 0; it < nst; ++it) {
             // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
@@ -385,7 +360,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 sc[i] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + i) & 3) * 8 + (lane >> 2));
             }
             uint32_t v[16];
-            expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
+            ts_expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
             if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
                 ok = false;
                 break;
@@ -393,7 +368,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
             tmem_st_16x256b_x4(td, v);
-            expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
+            ts_expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
@@ -428,46 +403,28 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     const int quad = warp & 3, sub = (warp - 2) >> 2;
     constexpr int EW = DQ_WARPS / 4;                                 // warps that share a TMEM lane quadrant
     const int lrow = quad * 32 + lane;                               // weight row within the tile
-    if (ks == 1 && (GROUPED || a.out_f16)) {
+    if (ks == 1 && a.out_f16) {
         // f16 results meet in shared memory ([token][row], the rings are idle) and leave as whole 16-byte pieces of a token's
         // row: a lane holds one weight row, so from registers it would store 2 bytes at a time (197 x 34816 x 5120: 62.9 -> 60.7
         // us; 64 tokens 32.2 -> 31.8)
-        const bool glu = GROUPED && a.glu;
-        const int per_tok = glu ? TS_MROWS : TS_MROWS * 2, n_out = glu ? a.n / 2 : a.n;      // bytes; values per row of the result
+        constexpr int PER_TOK = TS_MROWS * 2;
         if (dq_warp && ok) {
             for (int c0 = sub * 16; c0 < rows_valid; c0 += EW * 16) {
                 uint32_t v[16];
                 tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
-                if (glu) {
-                    // lanes 0-15 hold gate sums, lanes 16-31 the up sums of the same outputs: the former take tokens 0-7 of
-                    // the chunk, the latter 8-15
-                    const bool hi = lane >= 16;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float mine = __uint_as_float(hi ? v[i + 8] : v[i]) * a.out_mul;
-                        const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(hi ? v[i] : v[i + 8]), 16) * a.out_mul;
-                        *reinterpret_cast<__half*>(base_ptr + (c0 + i + (hi ? 8 : 0)) * per_tok + (quad * 16 + (lane & 15)) * 2) =
-                            silu_mul_f16(hi ? other : mine, hi ? mine : other);
-                    }
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        float f = __uint_as_float(v[i]) * a.out_mul;
-                        if (GROUPED && a.row_w != nullptr) {
-                            f = mul_row_w(f, c0 + i < rows_valid ? a.row_w[m0 + c0 + i] : 0.f);
-                        }
-                        *reinterpret_cast<__half*>(base_ptr + (c0 + i) * per_tok + lrow * 2) = __float2half_rn(f);
-                    }
+                for (int i = 0; i < 16; ++i) {
+                    *reinterpret_cast<__half*>(base_ptr + (c0 + i) * PER_TOK + lrow * 2) = __float2half_rn(__uint_as_float(v[i]) * a.out_mul);
                 }
             }
         }
         __syncthreads();
         if (!*abort_flag) {
-            const int pieces = min(TS_MROWS, a.n - n0) / (glu ? 16 : 8);
-            __half* out = reinterpret_cast<__half*>(a.out) + (size_t)m0 * n_out + (glu ? n0 / 2 : n0);
+            const int pieces = min(TS_MROWS, a.n - n0) / 8;
+            __half* out = reinterpret_cast<__half*>(a.out) + (size_t)m0 * a.n + n0;
             for (int e = (int)threadIdx.x; e < rows_valid * pieces; e += TS_THREADS) {
                 const int tok = e / pieces, c = e - tok * pieces;
-                *reinterpret_cast<uint4*>(out + (size_t)tok * n_out + c * 8) = *reinterpret_cast<const uint4*>(base_ptr + tok * per_tok + c * 16);
+                *reinterpret_cast<uint4*>(out + (size_t)tok * a.n + c * 8) = *reinterpret_cast<const uint4*>(base_ptr + tok * PER_TOK + c * 16);
             }
         }
     } else if (ks == 1) {
@@ -545,6 +502,368 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     }
 }
 
+
+// Grouped (MoE) form: token tiles from a device table, one expert's weights per tile, persistent CTAs.  The roles are those of the dense
+// kernel, but run on from tile to tile: with a CTA per tile, entry, table, TMEM, barriers and the first loads took about 4 us of the 14
+// (K = 2048) or 8 (K = 768) that a tile of 128 experts x 2048 x 768 took.  Now the rings run ahead into the next tile while the last one is
+// converted, and the two CTAs of an SM fill each other's epilogues.  (Layer of 128 experts, top-8: 256 tokens 165 ->
+// 141 us, 1024 tokens 209 -> 186.)
+template <int GROUP>
+__global__ void __launch_bounds__(TS_THREADS, 2)
+gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
+    extern __shared__ unsigned char smem_dyn[];
+    __shared__ uint32_t s_tmem_base;
+    __shared__ int s_abort;
+    constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    if (a.tables_fresh) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
+    unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
+    const int NR = a.raw_stages, NX = a.x_stages, NA = a.a_stages;
+    const uint32_t x_half = (uint32_t)a.tok * (BK * 2);
+    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_BYTES; };
+    auto x_addr = [&](int s) { return base + (uint32_t)a.off_x + (uint32_t)s * (2 * x_half); };
+    const uint32_t bars = base + (uint32_t)a.off_bars;
+    auto raw_full = [&](int s) { return bars + 8u * s; };
+    auto raw_free = [&](int s) { return bars + 8u * (NR + s); };
+    auto x_full = [&](int s) { return bars + 8u * (2 * NR + s); };
+    auto x_free = [&](int s) { return bars + 8u * (2 * NR + NX + s); };
+    auto a_ready = [&](int s) { return bars + 8u * (2 * NR + 2 * NX + s); };
+    auto a_free = [&](int s) { return bars + 8u * (2 * NR + 2 * NX + NA + s); };
+    const uint32_t accum_bar = bars + 8u * (2 * NR + 2 * NX + 2 * NA), acc_free = accum_bar + 8u;
+
+    const int nkb = a.k / BK, nst = (nkb + 1) / 2;                   // the last stage may hold one k-block (32-channel groups)
+    const int tiles = *a.num_tiles * a.n_tiles;
+    // neighbours share the token rows, then the expert's weights
+    struct Tile {
+        int m0, rows, n0, rb0, nrbv;
+    };
+    auto tile_at = [&](int i) {
+        const int mt = i / a.n_tiles;
+        Tile r;
+        r.n0 = (i - mt * a.n_tiles) * TS_MROWS;
+        r.m0 = a.tile_row0[mt];
+        r.rows = a.tile_rows[mt];
+        r.rb0 = ((a.tile_expert[mt] - a.expert0) * a.n + r.n0) / TILE_ROWS;
+        r.nrbv = min(TS_MROWS, a.n - r.n0) / TILE_ROWS;
+        return r;
+    };
+
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        for (int s = 0; s < NR; ++s) {
+            mbar_init(raw_full(s), 1);
+            mbar_init(raw_free(s), DQ_WARPS);
+        }
+        for (int s = 0; s < NX; ++s) {
+            mbar_init(x_full(s), 1);
+            mbar_init(x_free(s), 1);
+        }
+        for (int s = 0; s < NA; ++s) {
+            mbar_init(a_ready(s), DQ_WARPS);
+            mbar_init(a_free(s), 1);
+        }
+        mbar_init(accum_bar, 1);
+        mbar_init(acc_free, DQ_WARPS);
+        mbar_init_fence();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
+                     "r"(a.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // only now: a CTA of the next kernel that came earlier could take the TMEM this one still has to allocate
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem_base, 0);
+    const uint32_t tmem_a = tmem + (uint32_t)a.tok;                  // A ring: [stage][64 columns]
+    volatile int* abort_flag = &s_abort;
+
+    // After a wait that ran out a role goes on through its loops without waiting, loading or multiplying, so that the barrier of the
+    // converting warps stays matched.
+    bool ok = true;
+    if (warp == 0) {
+        // ------------------------------------------------------------------ tokens
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const bool leader = elect_one();
+        int sx = 0;
+        uint32_t px = 1, cnt = 0;
+        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+            const Tile tl = tile_at(i);
+            const int boxes = (tl.rows + TS_XBOX - 1) / TS_XBOX;     // rows of the next expert, or zeros, fill the last box up
+            for (int it = 0; it < nst; ++it, ++cnt) {
+                if (cnt >= (uint32_t)NX && !__all_sync(0xffffffffu, mbar_wait(x_free(sx), px, abort_flag, a.status, (51 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                if (leader) {
+                    const int kbs = min(2, nkb - 2 * it);
+                    mbar_expect_tx(x_full(sx), (uint32_t)(kbs * boxes) * (TS_XBOX * BK * 2));
+                    for (int h = 0; h < kbs; ++h) {
+                        for (int c = 0; c < boxes; ++c) {
+                            tma_load_2d(x_addr(sx) + h * x_half + (uint32_t)c * (TS_XBOX * BK * 2), &tmap_x, (2 * it + h) * BK,
+                                        tl.m0 + c * TS_XBOX, x_full(sx));
+                        }
+                    }
+                }
+                __syncwarp();
+                if (++sx == NX) {
+                    sx = 0;
+                    px ^= 1;
+                }
+            }
+        }
+    } else if (warp == 2 + DQ_WARPS) {
+        // ------------------------------------------------------------------ weights (they do not depend on the previous kernel)
+        const bool leader = elect_one();
+        int sr = 0;
+        uint32_t pr = 1, cnt = 0;
+        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+            const Tile tl = tile_at(i);
+            const uint32_t kb_bytes = (uint32_t)tl.nrbv * (TILE_WORDS * 4);
+            for (int it = 0; it < nst; ++it, ++cnt) {
+                if (cnt >= (uint32_t)NR && !__all_sync(0xffffffffu, mbar_wait(raw_free(sr), pr, abort_flag, a.status, (52 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                if (leader) {
+                    const int kbs = min(2, nkb - 2 * it);
+                    mbar_expect_tx(raw_full(sr), kbs * kb_bytes);
+                    const uint32_t* src = a.qt + ((size_t)(2 * it) * a.nrb_w + tl.rb0) * TILE_WORDS;
+                    bulk_load(raw_addr(sr), src, kb_bytes, raw_full(sr));
+                    if (kbs == 2) {
+                        bulk_load(raw_addr(sr) + RAW_BYTES / 2, src + (size_t)a.nrb_w * TILE_WORDS, kb_bytes, raw_full(sr));
+                    }
+                }
+                __syncwarp();
+                if (++sr == NR) {
+                    sr = 0;
+                    pr ^= 1;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------------ MMA issuer
+        const bool leader = elect_one();
+        int sx = 0, sa = 0;
+        uint32_t px = 0, pa = 0, done = 0;
+        for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++done) {
+            const int rows = a.tile_rows[i / a.n_tiles];
+            const uint32_t idesc = (1u << 4) | ((uint32_t)((rows + 15) / 16 * 2) << 17) | ((uint32_t)(TS_MROWS >> 4) << 24);
+            // the accumulator is read before it is written again
+            if (done > 0 && !__all_sync(0xffffffffu, mbar_wait(acc_free, (done - 1) & 1, abort_flag, a.status, (53 << 16)))) {
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int it = 0; it < nst; ++it) {
+                const bool in = mbar_wait(x_full(sx), px, abort_flag, a.status, (54 << 16) | it) &&
+                                mbar_wait(a_ready(sa), pa, abort_flag, a.status, (55 << 16) | it);
+                if (!__all_sync(0xffffffffu, in)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t db = umma_desc(x_addr(sx));
+                const uint64_t db1 = db + (x_half >> 4);
+                const uint32_t ta = tmem_a + (uint32_t)(sa * A_COLS);
+                const bool two = 2 * it + 1 < nkb;
+                if (leader) {
+#pragma unroll
+                    for (int j = 0; j < BK / 16; ++j) {
+                        umma_ts_f16(tmem, ta + j * 8, db + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
+                    }
+                    if (two) {
+#pragma unroll
+                        for (int j = 0; j < BK / 16; ++j) {
+                            umma_ts_f16(tmem, ta + BK / 2 + j * 8, db1 + 2 * j, idesc, 1u);
+                        }
+                    }
+                    umma_commit(a_free(sa));
+                    umma_commit(x_free(sx));
+                    if (it + 1 == nst) {
+                        umma_commit(accum_bar);
+                    }
+                }
+                __syncwarp();
+                if (++sx == NX) {
+                    sx = 0;
+                    px ^= 1;
+                }
+                if (++sa == NA) {
+                    sa = 0;
+                    pa ^= 1;
+                }
+            }
+        }
+    } else {
+        // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM; then convert and store
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const int rb = quad * 2 + half;                              // a warp may touch the TMEM lanes 32 * (warp % 4) .. +31
+        const int ng = a.k / GROUP;
+        const int lrow = quad * 32 + lane;
+        const int et = (int)threadIdx.x - 64;                        // thread among the converting warps
+        const bool glu = a.glu != 0;
+        const int per_tok = glu ? TS_MROWS : TS_MROWS * 2, n_out = glu ? a.n / 2 : a.n;      // bytes; values per row of the result
+        unsigned char* stage_ptr = base_ptr + a.off_stage;
+        constexpr int SCQ = 4;                                       // scale loads in flight, as in the dense kernel
+        const uint32_t* sp = nullptr;
+        int sleft = 0;
+        uint32_t scq[SCQ];
+        auto load_scales = [&]() {
+            const uint32_t v = sleft > 0 ? __ldg(sp) : 0u;
+            sp += 32;
+            sleft -= 32;
+            return v;
+        };
+        auto open_scales = [&](const Tile& tl) {
+            sp = a.st + (size_t)(tl.rb0 + (rb < tl.nrbv ? rb : 0)) * ng * 8 + lane;
+            sleft = ng * 8 - lane;
+#pragma unroll
+            for (int i = 0; i < SCQ; ++i) {
+                scq[i] = load_scales();
+            }
+        };
+        uint32_t sc_cur = 0;
+        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
+        int sr = 0, sa = 0;
+        uint32_t pr = 0, pa = 1, cnt = 0, done = 0;
+        Tile tl{}, next{};
+        if ((int)blockIdx.x < tiles) {
+            next = tile_at(blockIdx.x);
+            open_scales(next);
+        }
+        for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++done) {
+            tl = next;
+            const bool more = i + (int)gridDim.x < tiles;
+            if (more) {
+                next = tile_at(i + (int)gridDim.x);
+            }
+            const uint32_t r_ld = base + (uint32_t)(rb < tl.nrbv ? rb : 0) * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+            for (int it = 0; it < nst && ok; ++it, ++cnt) {
+                if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (56 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t ra = r_ld + (uint32_t)sr * RAW_BYTES;
+                const uint4 raw0 = lds128(ra);
+                const uint4 raw1 = lds128(ra + RAW_BYTES / 2);       // stale bytes when the stage holds one k-block
+                if (((it * GPS) & 3) == 0) {
+                    sc_cur = scq[0];
+#pragma unroll
+                    for (int q = 0; q + 1 < SCQ; ++q) {
+                        scq[q] = scq[q + 1];
+                    }
+                    scq[SCQ - 1] = load_scales();
+                }
+                uint32_t sc[GPS];
+#pragma unroll
+                for (int q = 0; q < GPS; ++q) {
+                    sc[q] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + q) & 3) * 8 + (lane >> 2));
+                }
+                uint32_t v[16];
+                ts_expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
+                if (cnt >= (uint32_t)NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (57 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
+                tmem_st_16x256b_x4(td, v);
+                ts_expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(raw_free(sr));                       // both k-blocks are in registers
+                }
+                tmem_st_16x256b_x4(td + BK / 2, v);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(a_ready(sa));
+                }
+                if (++sr == NR) {
+                    sr = 0;
+                    pr ^= 1;
+                }
+                if (++sa == NA) {
+                    sa = 0;
+                    pa ^= 1;
+                }
+            }
+            if (more) {
+                open_scales(next);                                   // on the way while this tile is converted
+            }
+            ok = ok && mbar_wait(accum_bar, done & 1, abort_flag, a.status, (58 << 16));
+            ok = __all_sync(0xffffffffu, ok);
+            if (done == 0) {
+                asm volatile("griddepcontrol.wait;" ::: "memory");   // outputs may be what the previous kernel still reads
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // f16 results through shared memory, [token][row], a stage of 16 KB at a time
+            const int stage_tok = TS_STAGE_BYTES / per_tok;
+            for (int t0 = 0; t0 < tl.rows; t0 += stage_tok) {
+                const int nt = min(stage_tok, tl.rows - t0);
+                if (ok) {
+                    for (int c0 = half * 16; c0 < nt; c0 += 32) {
+                        uint32_t v[16];
+                        tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(t0 + c0), v);
+                        if (glu) {
+                            // lanes 0-15 hold gate sums, lanes 16-31 the up sums of the same outputs: the former take tokens 0-7 of
+                            // the chunk, the latter 8-15
+                            const bool hi = lane >= 16;
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) {
+                                const float mine = __uint_as_float(hi ? v[q + 8] : v[q]) * a.out_mul;
+                                const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(hi ? v[q] : v[q + 8]), 16) * a.out_mul;
+                                *reinterpret_cast<__half*>(stage_ptr + (c0 + q + (hi ? 8 : 0)) * per_tok + (quad * 16 + (lane & 15)) * 2) =
+                                    silu_mul_f16(hi ? other : mine, hi ? mine : other);
+                            }
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 16; ++q) {
+                                float f = __uint_as_float(v[q]) * a.out_mul;
+                                if (a.row_w != nullptr) {
+                                    f = mul_row_w(f, c0 + q < nt ? a.row_w[tl.m0 + t0 + c0 + q] : 0.f);
+                                }
+                                *reinterpret_cast<__half*>(stage_ptr + (c0 + q) * per_tok + lrow * 2) = __float2half_rn(f);
+                            }
+                        }
+                    }
+                }
+                if (t0 + stage_tok >= tl.rows) {
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+                        mbar_arrive(acc_free);
+                    }
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(DQ_WARPS * 32) : "memory");
+                if (ok) {
+                    const int pieces = min(TS_MROWS, a.n - tl.n0) / (glu ? 16 : 8);
+                    __half* out = reinterpret_cast<__half*>(a.out) + (size_t)(tl.m0 + t0) * n_out + (glu ? tl.n0 / 2 : tl.n0);
+                    for (int e = et; e < nt * pieces; e += DQ_WARPS * 32) {
+                        const int tok = e / pieces, c = e - tok * pieces;
+                        *reinterpret_cast<uint4*>(out + (size_t)tok * n_out + c * 8) =
+                            *reinterpret_cast<const uint4*>(stage_ptr + tok * per_tok + c * 16);
+                    }
+                }
+                asm volatile("bar.sync 1, %0;" ::"n"(DQ_WARPS * 32) : "memory");     // the stage is free again
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols) : "memory");
+    }
+}
+
 }  // namespace
 
 
@@ -560,8 +879,8 @@ static size_t ts_smem(int tok, int nr, int nx, int na, int* off_x, int* off_bars
 
 cudaError_t gemm_ts_init_device() {
     cudaError_t e = cudaSuccess;
-    for (const void* f : {(const void*)gemm_ts_kernel<128, false>, (const void*)gemm_ts_kernel<32, false>,
-                          (const void*)gemm_ts_kernel<128, true>, (const void*)gemm_ts_kernel<32, true>}) {
+    for (const void* f : {(const void*)gemm_ts_kernel<128>, (const void*)gemm_ts_kernel<32>, (const void*)gemm_ts_grouped_kernel<128>,
+                          (const void*)gemm_ts_grouped_kernel<32>}) {
         if (e == cudaSuccess) {
             e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
         }
@@ -612,7 +931,7 @@ void Dec::ts_query_clusters() {
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128, false>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128>, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 n = 0;       // then this split is not considered
             }
@@ -727,8 +1046,8 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cudaError_t e;
-    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, a)
-                        : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, a);
+    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128>, map, a)
+                        : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32>, map, a);
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
@@ -746,18 +1065,26 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
     }
-    const TsPlan p = ts_plan(tok);
+    // half of the TMEM: the accumulator and as many expanded stages as fit; two CTAs per SM
+    const int tmem_cols = 256, na = std::min((tmem_cols - tok) / A_COLS, 4), nx = tok <= 64 ? 3 : 2;
     TsArgs a{};
+    int nr = 2;
+    auto bars_at = [&](int raw) { return raw * RAW_BYTES + nx * tok * SK * 2 + TS_STAGE_BYTES; };
+    auto smem_of = [&](int raw) { return (size_t)bars_at(raw) + (size_t)(2 * raw + 2 * nx + 2 * na + 2) * 8 + 1024; };
+    while (nr < 8 && smem_of(nr + 1) <= TS_SMEM_HALF_MAX) {
+        ++nr;
+    }
     a.tok = tok;
     a.ksplit = 1;
     a.m_tiles = max_tiles;
     a.n_tiles = (n_per_expert + TS_MROWS - 1) / TS_MROWS;
-    a.tmem_cols = p.tmem_cols;
-    a.a_stages = p.na;
-    a.raw_stages = p.nr;
-    a.x_stages = p.nx;
-    a.off_x = p.off_x;
-    a.off_bars = p.off_bars;
+    a.tmem_cols = tmem_cols;
+    a.a_stages = na;
+    a.raw_stages = nr;
+    a.x_stages = nx;
+    a.off_x = nr * RAW_BYTES;
+    a.off_stage = a.off_x + nx * tok * SK * 2;
+    a.off_bars = bars_at(nr);
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)l->k, (cuuint64_t)xs_rows};
     const cuuint64_t strides[1] = {(cuuint64_t)l->k * 2};
@@ -789,9 +1116,9 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     a.glu = l->glu_f > 0 ? 1 : 0;
     a.tables_fresh = tables_fresh ? 1 : 0;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(a.m_tiles * a.n_tiles);
+    cfg.gridDim = dim3(std::min(a.m_tiles * a.n_tiles, 2 * sm_count));
     cfg.blockDim = dim3(TS_THREADS);
-    cfg.dynamicSmemBytes = p.smem;
+    cfg.dynamicSmemBytes = std::max(smem_of(nr), TS_SMEM_HALF_MIN);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     if (a.pdl) {
@@ -800,12 +1127,12 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    const cudaError_t e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, a)
-                                          : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, true>, map, a);
+    const cudaError_t e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<128>, map, a)
+                                          : cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<32>, map, a);
     if (e != cudaSuccess) {
         return cuda_fail("launch grouped gemm", e);
     }
-    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "> (grouped)";
+    last_kernel = "gemm_ts_grouped_kernel<" + std::to_string(l->group) + "> " + std::to_string(tok) + "-row tiles";
     launches++;
     return 0;
 }
