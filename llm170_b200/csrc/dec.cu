@@ -98,6 +98,32 @@ void Dec::free_lin(Lin& l) {
     l = Lin{};
 }
 
+// Whether the weight-row GEMM may form f16((q - 8) * s) * 2^-E with one f16 multiply-add per pair of weights, and with which E.  The raw
+// nibble is an exact f16 subnormal, q * 2^-24 (rows g of a tile) or q * 2^-20 (rows g + 8), so q * 2^-24 * (s * 2^(24 - E)) - 8 * s * 2^-E is
+// that weight with a single rounding -- the same one -- while every scaled scale is a finite f16 value and every weight, from s * 2^-E up,
+// a normal one: exponent fields e of all scales with e + 24 - E <= 30 and e - E >= 1.  Scales that span more than five binades, zeros,
+// subnormals, infinities and NaN keep the general expansion (fma_e = -1).
+int Dec::scan_scales(Lin& l) {
+    if (l.group != 128) {
+        return 0;      // four scale words per stage leave nothing to win (27 x 34816 x 5120, groups of 32: 30.5 / 30.2 us)
+    }
+    int range[2] = {31, 0};
+    cudaError_t e = cudaMemcpyAsync(err_flag + 1, range, sizeof(range), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) {
+        launch_scale_range_f16(l.st, (size_t)l.n * (size_t)(l.k / l.group), err_flag + 1, stream);
+        e = cudaMemcpyAsync(range, err_flag + 1, sizeof(range), cudaMemcpyDeviceToHost, stream);
+    }
+    if (e == cudaSuccess) {
+        e = cudaStreamSynchronize(stream);
+    }
+    if (e != cudaSuccess) {
+        return cuda_fail("scale range", e);
+    }
+    const int shift = range[1] > 6 ? range[1] - 6 : 0;
+    l.fma_e = shift <= 20 && range[0] - shift >= 1 ? shift : -1;
+    return 0;
+}
+
 int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, int n, int k, int group,
                        int scale_bf16, int glu_f) {
     // q_dev/s_dev: boundary format already on the device.  Groups of 64 channels (accepted by the reference's loader,
@@ -165,6 +191,11 @@ int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, i
             return cuda_fail("repack", e);
         }
         return fail("w4a16 upload %s: a bf16 scale is not representable in f16 even after shifting", name);
+    }
+    if (int rc = scan_scales(l)) {
+        cudaFree(l.qt);
+        cudaFree(l.st);
+        return rc;
     }
     l.bytes = qb + sb;
     auto it = lins.find(name);

@@ -29,6 +29,8 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstring>
 #include <string>
 
 #include "../../include/w4a16_b200.h"
@@ -73,6 +75,7 @@ struct TsArgs {
     int off_stage;       // grouped: results of a tile on their way out
     int pdl;
     float out_mul;
+    uint32_t fma_add, fma_mul;   // (20 - E) << 26 | (24 - E) << 10 and the pair (-8 * 2^-E, -8 * 2^-E) (Dec::scan_scales)
     int* status;
     // grouped (MoE) mode: token tiles come from a device table, one expert's weights (n rows) per tile; tok is then the most
     // rows that a tile holds
@@ -119,24 +122,47 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
     return v;
 }
 
-// A lane's 16 raw bytes of a tile -> its 16 registers of tcgen05.st.16x256b.x4, f16((q - 8) * s): s_a / s_b = scale pair (rows g, g + 8)
-// of the first / second 32 channels.
-__device__ __forceinline__ void ts_expand(const uint4& raw, const uint32_t s_a, const uint32_t s_b, uint32_t (&v)[16]) {
+// Scale pair (rows g, g + 8) of a tile's 32 or more channels, ready for ts_expand: f16((q - 8) * s) as (q - 8) times s, or (FMA) as a
+// multiply-add of the raw nibble with s scaled by powers of two and -8 s 2^-E (Dec::scan_scales).
+template <bool FMA>
+struct TsScale {
+    uint32_t s0, s1, c0, c1;
+    __device__ __forceinline__ TsScale(uint32_t s2, uint32_t add, uint32_t mul) {
+        const uint32_t sp = FMA ? s2 + add : s2;           // exponents up by 24 - E (rows g) and 20 - E (rows g + 8): no field overflows
+        s0 = __byte_perm(sp, sp, 0x1010);
+        s1 = __byte_perm(sp, sp, 0x3232);
+        if (FMA) {
+            const uint32_t c = hmul2u(s2, mul);
+            c0 = __byte_perm(c, c, 0x1010);
+            c1 = __byte_perm(c, c, 0x3232);
+        }
+    }
+};
+// A lane's 16 raw bytes of a tile -> its 16 registers of tcgen05.st.16x256b.x4: sa / sb = scales of the first / second 32 channels.
+template <bool FMA>
+__device__ __forceinline__ void ts_expand(const uint4& raw, const TsScale<FMA>& sa, const TsScale<FMA>& sb, uint32_t (&v)[16]) {
     const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
+        const TsScale<FMA>& s = w < 2 ? sa : sb;
         uint32_t f[4];
-        dequant_word(rw[w], f);
-        const uint32_t s2 = w < 2 ? s_a : s_b;
-        const uint32_t s_r0 = __byte_perm(s2, s2, 0x1010), s_r1 = __byte_perm(s2, s2, 0x3232);
-        v[4 * w + 0] = hmul2u(f[0], s_r0);
-        v[4 * w + 1] = hmul2u(f[2], s_r0);
-        v[4 * w + 2] = hmul2u(f[1], s_r1);
-        v[4 * w + 3] = hmul2u(f[3], s_r1);
+        if (FMA) {
+            nibbles_as_subnormals(rw[w], f);
+            v[4 * w + 0] = hfma2u(f[0], s.s0, s.c0);
+            v[4 * w + 1] = hfma2u(f[2], s.s0, s.c0);
+            v[4 * w + 2] = hfma2u(f[1], s.s1, s.c1);
+            v[4 * w + 3] = hfma2u(f[3], s.s1, s.c1);
+        } else {
+            dequant_word(rw[w], f);
+            v[4 * w + 0] = hmul2u(f[0], s.s0);
+            v[4 * w + 1] = hmul2u(f[2], s.s0);
+            v[4 * w + 2] = hmul2u(f[1], s.s1);
+            v[4 * w + 3] = hmul2u(f[3], s.s1);
+        }
     }
 }
 
-template <int GROUP>
+template <int GROUP, bool FMA>
 __global__ void __launch_bounds__(TS_THREADS, 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
@@ -360,7 +386,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 sc[i] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + i) & 3) * 8 + (lane >> 2));
             }
             uint32_t v[16];
-            ts_expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
+            const TsScale<FMA> sc0(sc[0], a.fma_add, a.fma_mul), sc1(sc[GPS > 1 ? 1 : 0], a.fma_add, a.fma_mul);
+            ts_expand<FMA>(raw0, sc0, sc1, v);
             if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
                 ok = false;
                 break;
@@ -368,7 +395,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
             tmem_st_16x256b_x4(td, v);
-            ts_expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
+            if (GPS > 1) {
+                ts_expand<FMA>(raw1, TsScale<FMA>(sc[GPS > 2 ? 2 : 0], a.fma_add, a.fma_mul), TsScale<FMA>(sc[GPS > 2 ? 3 : 0], a.fma_add, a.fma_mul), v);
+            } else {
+                ts_expand<FMA>(raw1, sc0, sc1, v);
+            }
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
@@ -767,7 +798,7 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
                     sc[q] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + q) & 3) * 8 + (lane >> 2));
                 }
                 uint32_t v[16];
-                ts_expand(raw0, sc[0], sc[GPS > 1 ? 1 : 0], v);
+                ts_expand<false>(raw0, TsScale<false>(sc[0], 0, 0), TsScale<false>(sc[GPS > 1 ? 1 : 0], 0, 0), v);
                 if (cnt >= (uint32_t)NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (57 << 16) | it))) {
                     ok = false;
                     break;
@@ -775,7 +806,7 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
                 tmem_st_16x256b_x4(td, v);
-                ts_expand(raw1, sc[GPS > 2 ? 2 : 0], sc[GPS > 2 ? 3 : 0], v);
+                ts_expand<false>(raw1, TsScale<false>(sc[GPS > 2 ? 2 : 0], 0, 0), TsScale<false>(sc[GPS > 2 ? 3 : 0], 0, 0), v);
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive(raw_free(sr));                       // both k-blocks are in registers
@@ -879,7 +910,7 @@ static size_t ts_smem(int tok, int nr, int nx, int na, int* off_x, int* off_bars
 
 cudaError_t gemm_ts_init_device() {
     cudaError_t e = cudaSuccess;
-    for (const void* f : {(const void*)gemm_ts_kernel<128>, (const void*)gemm_ts_kernel<32>, (const void*)gemm_ts_grouped_kernel<128>,
+    for (const void* f : {(const void*)gemm_ts_kernel<128, false>, (const void*)gemm_ts_kernel<128, true>, (const void*)gemm_ts_kernel<32, false>, (const void*)gemm_ts_grouped_kernel<128>,
                           (const void*)gemm_ts_grouped_kernel<32>}) {
         if (e == cudaSuccess) {
             e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
@@ -931,7 +962,7 @@ void Dec::ts_query_clusters() {
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128, false>, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 n = 0;       // then this split is not considered
             }
@@ -1046,8 +1077,19 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     cudaError_t e;
-    e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128>, map, a)
-                        : cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32>, map, a);
+    if (l->group != 128) {
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, a);
+    } else if (l->fma_e < 0) {
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, a);
+    } else {
+        // one f16 operation per pair of weights where two do it otherwise, in the expansion that a small batch waits for (27 x 34816 x
+        // 5120: 29.8 -> 26.5 us, 27 x 5120 x 17408: 21.3 -> 19.3); the weights come out 2^-E smaller
+        const __half2 mul = __float2half2_rn(ldexpf(-8.0f, -l->fma_e));
+        memcpy(&a.fma_mul, &mul, sizeof(mul));
+        a.fma_add = ((uint32_t)(20 - l->fma_e) << 26) + ((uint32_t)(24 - l->fma_e) << 10);
+        a.out_mul = ldexpf(l->out_mul, l->fma_e);
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, a);
+    }
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }

@@ -13,6 +13,8 @@ namespace w4 {
 void launch_repack_q(const uint32_t* q_orig, uint32_t* qt, int n, int k, int glu_f, cudaStream_t st);
 // Biased-exponent range of the non-zero bf16 scales: range2[0] = min (preset 255), range2[1] = max (preset 0).
 void launch_scale_range(const uint16_t* s_orig, size_t total, int* range2, cudaStream_t st);
+// Exponent fields of resident f16 scales (a multiple of 8 of them): range2[0] = min (preset 31), range2[1] = max (preset 0).
+void launch_scale_range_f16(const uint16_t* stl, size_t total, int* range2, cudaStream_t st);
 // `group` is the group size of the TILED array; a source group covers `src_div` tiled groups.  bf16 scales are
 // multiplied by 2^shift and stored as f16; err_flag (device int, may be null) is set to 1 if one of them is not
 // exactly representable.

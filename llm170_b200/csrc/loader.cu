@@ -563,6 +563,10 @@ int Dec::upload_stream(const char* name, int n, int k, int group, int scale_bf16
         }
         return fail("w4a16 upload %s: a bf16 scale is not representable in f16 even after shifting", name);
     }
+    if (int rc = scan_scales(l)) {
+        drop();
+        return rc;
+    }
     l.bytes = qb + sb;
     auto it = lins.find(name);
     if (it != lins.end()) {
@@ -848,6 +852,11 @@ int w4a16_load_lin_cache(w4a16_dec* dec, const char* name, const char* path, uin
         cudaFree(l.qt);
         cudaFree(l.st);
         return d.fail("w4a16 load_lin_cache: reading %s failed", path);
+    }
+    if (int rc = d.scan_scales(l)) {
+        cudaFree(l.qt);
+        cudaFree(l.st);
+        return rc;
     }
     l.bytes = qb + sb;
     auto it = d.lins.find(name);

@@ -120,6 +120,27 @@ __global__ void scale_range_kernel(const uint16_t* __restrict__ s, size_t total,
     }
 }
 
+// The same for resident f16 scales (range[0] starts at 31, range[1] at 0); zeros and subnormals count as exponent 0.
+__global__ void scale_range_f16_kernel(const uint4* __restrict__ s, size_t total8, int* __restrict__ range) {
+    int lo = 31, hi = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
+        const uint4 v = s[i];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int e0 = (int)(w[j] >> 10) & 31, e1 = (int)(w[j] >> 26) & 31;
+            lo = min(lo, min(e0, e1));
+            hi = max(hi, max(e0, e1));
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(range, lo);
+        atomicMax(range + 1, hi);
+    }
+}
+
 // `ng`: groups per row of the TILED array; a source group covers `src_div` of them (2 when 64-channel groups are
 // stored as two 32-channel groups with the same scale, else 1).
 __global__ void repack_s_kernel(const uint16_t* __restrict__ s, uint16_t* __restrict__ stl, int n, int ng, int src_div,
@@ -288,6 +309,9 @@ void launch_cast_f16(const float* x, void* y16, size_t total, cudaStream_t st) {
 }
 void launch_scale_range(const uint16_t* s, size_t total, int* range2, cudaStream_t st) {
     scale_range_kernel<<<grid_for(total), 256, 0, st>>>(s, total, range2);
+}
+void launch_scale_range_f16(const uint16_t* stl, size_t total, int* range2, cudaStream_t st) {
+    scale_range_f16_kernel<<<grid_for(total / 8), 256, 0, st>>>((const uint4*)stl, total / 8, range2);
 }
 void launch_repack_s(const uint16_t* s, uint16_t* stl, int n, int k, int group, int src_div, int scale_bf16, int shift,
                      int* err, int glu_f, cudaStream_t st) {

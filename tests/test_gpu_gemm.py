@@ -391,3 +391,41 @@ def test_automatic_form(dec, n, k, t, form):
     dec.sync()
     assert (y - other).abs().max().item() <= 1e-4 * y.abs().max().item() + 1e-6
     dec.drop_lin("auto")
+
+
+# The weight-row form expands groups of 128 with one multiply-add per pair where the scales allow it; either way every weight is the
+# exact product rounded once to f16, so with activations that pick out single channels the outputs are those weights bit for bit.
+@pytest.mark.parametrize("scales", ["plain", "widest", "one binade more", "zero", "subnormal", "tiny", "huge", "negative"])
+def test_weight_row_expansion_rounds_once(dec, scales):
+    n, k, t = 144, 384, 128
+    rng = np.random.default_rng(5)
+    q = rng.integers(0, 2 ** 32, (n, k // 8), dtype=np.uint32)
+    q[:16, :2] = 0x76543210
+    q[:16, 2:4] = 0xFEDCBA98                                 # every nibble in every row of a tile
+    e = {"plain": (5, 8), "widest": (4, 9), "one binade more": (3, 9), "zero": (5, 8), "subnormal": (5, 8), "tiny": (1, 6), "huge": (21, 26),
+         "negative": (5, 8)}[scales]
+    s = (rng.integers(e[0], e[1] + 1, (n, k // 128)) << 10 | rng.integers(0, 1024, (n, k // 128))).astype(np.uint16)
+    s[0, 0], s[1, 0] = e[0] << 10, e[1] << 10 | 1023         # both ends of the range
+    if scales == "zero":
+        s[2, 1] = 0
+    elif scales == "subnormal":
+        s[2, 1] = 5
+    elif scales == "negative":
+        s[::3] |= 0x8000
+    dec.upload_lin_g("exp", q, s, n, k, 128)
+    nib = (q[:, :, None] >> (4 * np.arange(8, dtype=np.uint32)) & 15).reshape(n, k).astype(np.float64) - 8
+    with np.errstate(over="ignore"):
+        w = (nib * np.repeat(s.view(np.float16).astype(np.float64), 128, axis=1)).astype(np.float16)
+    for c0 in range(0, k, t):
+        x = torch.zeros((t, k), device="cuda", dtype=torch.float16)
+        x[torch.arange(t), c0 + torch.arange(t)] = 1
+        with forced(dec, "gemm_form", 2):
+            y = dec.lin_forward("exp", x, t).cpu().numpy()
+        dec.sync()
+        want = w[:, c0:c0 + t].T.astype(np.float32)
+        if scales != "huge":                                 # (a weight beyond f16 is an infinity, and infinity times 0 is NaN)
+            assert np.array_equal(y, want)
+        else:
+            fine = np.isfinite(w).all(axis=1)
+            assert fine.any() and np.array_equal(y[:, fine], want[:, fine])
+    dec.drop_lin("exp")
