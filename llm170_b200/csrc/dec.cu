@@ -559,6 +559,9 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
             e = w4::gemm_ts_init_device();
         }
         if (e == cudaSuccess) {
+            e = w4::gemm_ts2_init_device();
+        }
+        if (e == cudaSuccess) {
             d.ts_query_clusters();
         }
     }
@@ -722,6 +725,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
             return d.fail("w4a16 tuning: gemv_stages must be 2..8");
         }
         d.tune_gemv_stages = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemm_pair")) {
+        if (value != 0 && value != 1 && (value < 32 || value > 256 || value % 32 != 0)) {
+            return d.fail("w4a16 set_tuning: gemm_pair=%d (0, 1 or a multiple of 32 up to 256)", value);
+        }
+        d.tune_gemm_pair = value;
         return 0;
     }
     if (!strcmp(key, "gemm_form")) {

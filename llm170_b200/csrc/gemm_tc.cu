@@ -652,6 +652,9 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     if (((uintptr_t)x & 15) != 0 || ((uintptr_t)dst & 15) != 0) {
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
     }
+    if (tune_gemm_pair > 1) {
+        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, st);
+    }
     // Tile shape and K split are chosen together by a small cost model (microseconds, fitted to measurements on B200).  A
     // k-block takes 0.30 + 0.00105 bn with one 128-token block; with two, 0.295 + 0.00133 bn while at most 100 CTAs run and
     // 0.163 + 0.0024 bn (0.78 at 256) when the GPU is full; 5 us around a wave; a split tile another 3.5 us and, at 256 rows,
@@ -736,7 +739,18 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             return fail("w4a16 gemm: no weight-row tile for %d x %d x %d (gemm_ts_ksplit=%d: no such cluster on this device)", t, l->n,
                         l->k, tune_ts_ks);
         }
-        if (tune_gemm_form == 2 || c.cost < bar_ts * best.cost) {
+        const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
+        if (t <= 4096 && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
+            // The pairs (gemm_ts2.cu) take what they are estimated to finish sooner by at least 2 %.  Over 140 drawn shapes (66..4096 tokens) the
+            // choice took 6.4 % less time than the better of the two other forms' rule, the best choice of each 7.1 %; the worst case was
+            // 551 x 20752 x 16128, 301 against 294 us, the best 3418 x 24592 x 1408, 185 against 266.  Calls of few tiles (526 x 2144 x 16384: 52 against 38 us)
+            // stay with the weight-row form, which splits K over clusters.  More than 4096 tokens were not compared.
+            const TsChoice p = gemm_ts2_choose(l, t);
+            if (p.cost < 0.98 * (ts ? c.cost : best.cost)) {
+                return gemm_ts2(l, x, dst, t, out_kind, p.tok, st);
+            }
+        }
+        if (ts) {
             return gemm_ts(l, x, dst, t, out_kind, c, st);
         }
     }

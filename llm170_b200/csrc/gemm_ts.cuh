@@ -1,0 +1,75 @@
+// Pieces shared by the weight-row GEMM kernels (gemm_ts.cu, gemm_ts2.cu): weights expanded in registers and stored to TMEM.
+#pragma once
+#include <cstdint>
+
+#include "gemm_common.cuh"
+#include "gemv_common.cuh"
+#include "ptx.cuh"
+
+namespace w4 {
+
+constexpr int TS_MROWS = 128;                   // weight rows per MMA
+constexpr int BK = TILE_K;
+constexpr int SK = 2 * BK;                      // channels per stage: two k-blocks, one 128-channel scale group
+constexpr int RAW_BYTES = TS_MROWS * SK / 2;    // 8 KB per stage
+constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
+constexpr int DQ_WARPS = TS_MROWS / TILE_ROWS;  // a warp per 16-row block
+
+// 16 TMEM lanes x 32 columns from one warp: register 4i + {0,1} of lane (g, t) -> row g, columns 8i + 2t + {0,1};
+// register 4i + {2,3} -> row g + 8
+__device__ __forceinline__ void tmem_st_16x256b_x4(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// Scale pair (rows g, g + 8) of a tile's 32 or more channels, ready for ts_expand: f16((q - 8) * s) as (q - 8) times s, or (FMA) as a
+// multiply-add of the raw nibble with s scaled by powers of two and -8 s 2^-E (Dec::scan_scales).
+template <bool FMA>
+struct TsScale {
+    uint32_t s0, s1, c0, c1;
+    __device__ __forceinline__ TsScale(uint32_t s2, uint32_t add, uint32_t mul) {
+        const uint32_t sp = FMA ? s2 + add : s2;           // exponents up by 24 - E (rows g) and 20 - E (rows g + 8): no field overflows
+        s0 = __byte_perm(sp, sp, 0x1010);
+        s1 = __byte_perm(sp, sp, 0x3232);
+        if (FMA) {
+            const uint32_t c = hmul2u(s2, mul);
+            c0 = __byte_perm(c, c, 0x1010);
+            c1 = __byte_perm(c, c, 0x3232);
+        }
+    }
+};
+// A lane's 16 raw bytes of a tile -> its 16 registers of tcgen05.st.16x256b.x4: sa / sb = scales of the first / second 32 channels.
+template <bool FMA>
+__device__ __forceinline__ void ts_expand(const uint4& raw, const TsScale<FMA>& sa, const TsScale<FMA>& sb, uint32_t (&v)[16]) {
+    const uint32_t rw[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const TsScale<FMA>& s = w < 2 ? sa : sb;
+        uint32_t f[4];
+        if (FMA) {
+            nibbles_as_subnormals(rw[w], f);
+            v[4 * w + 0] = hfma2u(f[0], s.s0, s.c0);
+            v[4 * w + 1] = hfma2u(f[2], s.s0, s.c0);
+            v[4 * w + 2] = hfma2u(f[1], s.s1, s.c1);
+            v[4 * w + 3] = hfma2u(f[3], s.s1, s.c1);
+        } else {
+            dequant_word(rw[w], f);
+            v[4 * w + 0] = hmul2u(f[0], s.s0);
+            v[4 * w + 1] = hmul2u(f[2], s.s0);
+            v[4 * w + 2] = hmul2u(f[1], s.s1);
+            v[4 * w + 3] = hmul2u(f[3], s.s1);
+        }
+    }
+}
+
+}  // namespace w4

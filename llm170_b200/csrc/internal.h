@@ -179,6 +179,7 @@ const char* gemv_rb_variant(const GemvArgs& a, int total_units, int rbw, int sm_
 // Raises the dynamic shared-memory limit of the tensor-core GEMM kernels on the current device.
 cudaError_t gemm_init_device();
 cudaError_t gemm_ts_init_device();
+cudaError_t gemm_ts2_init_device();
 cudaError_t head_init_device();
 
 // ---- moe.cu ----------------------------------------------------------------------------------

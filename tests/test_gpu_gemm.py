@@ -429,3 +429,57 @@ def test_weight_row_expansion_rounds_once(dec, scales):
             fine = np.isfinite(w).all(axis=1)
             assert fine.any() and np.array_equal(y[:, fine], want[:, fine])
     dec.drop_lin("exp")
+
+
+# CTA pairs: a pair's tile is 256 weight rows x the given tokens; ragged last tiles in both directions, rows that only the first CTA of
+# the last pair has, odd numbers of k-blocks, more tiles than pairs (the rings and both TMEM parts are used again), fewer tokens than
+# half a tile.
+@pytest.mark.parametrize("t,k,n,group,tok", [
+    (9, 128, 16, 128, 32), (33, 192, 144, 32, 32), (65, 320, 272, 64, 64), (197, 256, 496, 128, 96), (256, 640, 384, 32, 128),
+    (300, 1024, 400, 128, 160), (511, 1280, 656, 128, 192), (449, 448, 768, 64, 224), (256, 512, 256, 128, 256), (257, 128, 528, 32, 256),
+    (1500, 384, 4112, 128, 96)])
+@pytest.mark.parametrize("out_f16", [False, True])
+def test_cta_pairs_pow2_exact(dec, t, k, n, group, tok, out_f16):
+    q, s, x, expect = pow2_case(t, k, n, group)
+    dec.upload_lin_g("pair", q, s, n, k, group)
+    guard = torch.full((t + 256, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    with forced(dec, "gemm_pair", tok):
+        y = dec.lin_forward("pair", x_dev(x), t, dst=guard[:t], out_f16=out_f16)
+        assert dec.last_kernel().startswith("gemm_ts2_kernel")
+        dec.sync()
+        dec.kernel_status()
+    assert np.array_equal(y.cpu().numpy(), expect.astype(np.float16) if out_f16 else expect)
+    assert (guard[t:] == 7.0).all()
+    dec.drop_lin("pair")
+
+
+@pytest.mark.parametrize("t,k,n,group,bf16", [(700, 2048, 2560, 128, False), (1000, 1984, 2064, 32, False), (600, 3072, 2576, 64, True)])
+def test_cta_pairs_equal_the_weight_row_form(dec, t, k, n, group, bf16):
+    # the same weights in the same order of accumulation: the same bits, also out of a graph that replays the call twice over new rows
+    q, s = synth.make_linear_cuda(n, k, group, 7, "cuda")
+    dec.upload_lin_g_dev("pairf", q, s.to(torch.bfloat16) if bf16 else s, n, k, group, bf16)
+    x = torch.randn((t, k), device="cuda").half()
+    y = torch.zeros((t, n), device="cuda", dtype=torch.float16)
+    with forced(dec, "gemm_pair", 192):
+        dec.capture_begin()
+        dec.lin_forward("pairf", x, t, dst=y, out_f16=True)
+        dec.lin_forward("pairf", x, t, dst=y, out_f16=True)
+        g = dec.capture_end()
+    for seed in range(2):
+        x.copy_(torch.randn((t, k), device="cuda", generator=torch.Generator("cuda").manual_seed(seed)).half())
+        torch.cuda.synchronize()
+        dec.graph_launch(g)
+        dec.sync()
+        with forced(dec, "gemm_form", 2), forced(dec, "gemm_ts_ksplit", 1):
+            want = dec.lin_forward("pairf", x, t, out_f16=True)
+        dec.sync()
+        assert torch.equal(y, want)
+    dec.graph_destroy(g)
+    dec.drop_lin("pairf")
+
+
+@pytest.mark.parametrize("bad", [-1, 2, 16, 48, 288])
+def test_cta_pair_tuning_refuses_values_without_a_tile(dec, bad):
+    from llm170_b200.w4a16_dec import W4a16Error
+    with pytest.raises(W4a16Error, match="gemm_pair"):
+        dec.set_tuning("gemm_pair", bad)
