@@ -740,11 +740,12 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                         l->k, tune_ts_ks);
         }
         const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
-        if (t <= 4096 && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
+        if (t <= 4096 && out_kind == W4A16_OUT_F16 && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
             // The pairs (gemm_ts2.cu) take what they are estimated to finish sooner by at least 2 %.  Over 140 drawn shapes (66..4096 tokens) the
             // choice took 6.4 % less time than the better of the two other forms' rule, the best choice of each 7.1 %; the worst case was
             // 551 x 20752 x 16128, 301 against 294 us, the best 3418 x 24592 x 1408, 185 against 266.  Calls of few tiles (526 x 2144 x 16384: 52 against 38 us)
-            // stay with the weight-row form, which splits K over clusters.  More than 4096 tokens were not compared.
+            // stay with the weight-row form, which splits K over clusters.  More than 4096 tokens, and f32 results, were not compared:
+            // they keep their forms.
             const TsChoice p = gemm_ts2_choose(l, t);
             if (p.cost < 0.98 * (ts ? c.cost : best.cost)) {
                 return gemm_ts2(l, x, dst, t, out_kind, p.tok, st);

@@ -460,7 +460,8 @@ def test_cta_pairs_equal_the_weight_row_form(dec, t, k, n, group, bf16):
     dec.upload_lin_g_dev("pairf", q, s.to(torch.bfloat16) if bf16 else s, n, k, group, bf16)
     x = torch.randn((t, k), device="cuda").half()
     y = torch.zeros((t, n), device="cuda", dtype=torch.float16)
-    with forced(dec, "gemm_pair", 192):
+    torch.cuda.synchronize()
+    with forced(dec, "gemm_pair", 192), torch.cuda.stream(torch.cuda.ExternalStream(dec.stream_ptr())):
         dec.capture_begin()
         dec.lin_forward("pairf", x, t, dst=y, out_f16=True)
         dec.lin_forward("pairf", x, t, dst=y, out_f16=True)
