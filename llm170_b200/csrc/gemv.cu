@@ -1,6 +1,6 @@
 // Decode-time W4A16 split-K GEMV for 1..8 tokens:  y[m][n] = sum_k x[m][k] * (q[n][k]-8) * s[n][k/group],
-// (row block, K split) form: grid (256-row blocks, K splits).  Dec::gemv uses it for 5..8 tokens, the MoE decode
-// path uses its table-driven "grouped" mode; up to 4 tokens run the persistent form in gemv_sk.cu.
+// (row block, K split) form: grid (256-row blocks, K splits).  It takes what the row-group form (gemv_rg.cu) and the grouped one
+// (gemv_moe.cu) have no room for, and the tuned calls.
 //
 // Takes the place of the reference's split-K GEMV pair (crates/backend-gpu/src/rawcuda/assets/decode.cu:46-267,
 // launched from crates/backend-gpu/src/rawcuda/w4a16_dec/kernels/decode.rs:23-127) and of its FFMA
