@@ -135,7 +135,7 @@ struct Dec {
              cudaStream_t st, bool allreduce = false, bool single = false);
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     void ts_query_clusters();
-    TsChoice gemm_ts_choose(int n, int k, int t, int split) const;   // split: 0 = any, else this many K splits
+    TsChoice gemm_ts_choose(int n, int k, int t) const;
     TsChoice gemm_ts2_choose(const Lin* l, int t) const;
     int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, cudaStream_t st);
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);

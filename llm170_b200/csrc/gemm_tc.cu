@@ -737,25 +737,27 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     // than 4096 tokens were not compared: a fifth, too.
     const double bar_ts = t <= 1024 || (l->k >= 3072 && t <= 4096) ? 0.9 : 0.8;
     if (tune_gemm_form == 2 || (tune_gemm_form == 0 && tune_gemm_ksplit == 0 && tune_gemm_mt == 0 && tune_gemm_bn == 0)) {
-        TsChoice c = gemm_ts_choose(l->n, l->k, t, tune_ts_ks);
+        const TsChoice c = gemm_ts_choose(l->n, l->k, t);
         if (tune_gemm_form == 2 && c.tok == 0) {
             return fail("w4a16 gemm: no weight-row tile for %d x %d x %d (gemm_ts_ksplit=%d: no such cluster on this device)", t, l->n,
                         l->k, tune_ts_ks);
         }
         const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
-        if (t > 64 && t <= 4096 && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
+        if (t > 64 && t <= 4096 && !(ts && c.ks > 1) && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
             // The pairs (gemm_ts2.cu) take what they are estimated to finish sooner by at least 2 %.  Over 140 drawn shapes (66..4096 tokens) the
             // choice took 6.4 % less time than the better of the two other forms' rule, the best choice of each 7.1 %; the worst case was
             // 551 x 20752 x 16128, 301 against 294 us, the best 3418 x 24592 x 1408, 185 against 266.  Calls of few tiles (526 x 2144 x 16384: 52 against 38 us)
             // stay with the weight-row form, which splits K over clusters.  Below 65 and above 4096 tokens
             // they were not compared, nor were f32 results: those keep their form.  It runs without a K split then, so that a call's f32 sums
             // are the ones that its f16 results are rounded from; each of the three forms adds the channels of a sum in the same order.
+            // (4096 tokens with f32 results: 7168 x 5120 239 -> 257 us, 5120 x 17408 535 -> 566, two other shapes of the layer the same.)
+            // Where the weight-row form would split K, both kinds of result stay with it: unsplit, f32 lost more than f16 gained (300 x
+            // 5120 x 17408 58 -> 84 us).
             const TsChoice p = gemm_ts2_choose(l, t);
             if (p.cost < 0.98 * (ts ? c.cost : best.cost)) {
                 if (out_kind == W4A16_OUT_F16) {
                     return gemm_ts2(l, x, dst, t, out_kind, p.tok, st);
                 }
-                c = gemm_ts_choose(l->n, l->k, t, 1);
                 best = whole;
             }
         }

@@ -912,7 +912,7 @@ void Dec::ts_query_clusters() {
 // 0.82 at 256 tokens) and 0.65 us and 0.0018 per token with a second one beside it; a split CTA another 1.2 us and 0.04 us per
 // token for the sum over the cluster.  Without a candidate (a cluster size that is asked for and cannot be resident) the result
 // has tok = 0 and a cost above every other form's.
-TsChoice Dec::gemm_ts_choose(int n, int k, int t, int split) const {
+TsChoice Dec::gemm_ts_choose(int n, int k, int t) const {
     TsChoice best{0, 0, 1e30};
     const int n_tiles = (n + TS_MROWS - 1) / TS_MROWS, stages = (k + SK - 1) / SK;
     int last_tok = 0;
@@ -927,7 +927,7 @@ TsChoice Dec::gemm_ts_choose(int n, int k, int t, int split) const {
         const int full = tok > 128;
         for (int ks = 1; ks <= TS_MAX_SPLIT && ks <= stages; ++ks) {
             const int room = ts_clusters[full][ks];
-            if (room <= 0 || (split > 0 && ks != std::min(split, stages))) {
+            if (room <= 0 || (tune_ts_ks > 0 && ks != std::min(tune_ts_ks, stages))) {
                 continue;
             }
             const double around = ks > 1 ? 1.2 + 0.04 * tok : 0.01 * tok;
