@@ -44,6 +44,13 @@ bool Dec::capturing(cudaStream_t st) {
     return cs != cudaStreamCaptureStatusNone;
 }
 
+// Device memory that later launches count on, filled before this returns.  (cudaMemset returns before the default stream has run it, and
+// nothing orders that stream and the non-blocking ones that the kernels run on.)
+cudaError_t Dec::fill_now(void* p, int byte, size_t bytes, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(p, byte, bytes, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
 // Grow-only scratch. Never grows while `st` is capturing (allocation is illegal there).
 int Dec::ensure_scratch(size_t part_floats, int grid_x, cudaStream_t st) {
     if (part_floats <= part_cap && (size_t)grid_x <= counters_cap) {

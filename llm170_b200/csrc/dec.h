@@ -121,6 +121,7 @@ struct Dec {
     int fail(const char* fmt, ...);
     int cuda_fail(const char* what, cudaError_t e);
     static bool capturing(cudaStream_t st);
+    static cudaError_t fill_now(void* p, int byte, size_t bytes, cudaStream_t st);
     int ensure_scratch(size_t part_floats, int grid_x, cudaStream_t st);
     void free_lin(Lin& l);
     int scan_scales(Lin& l);

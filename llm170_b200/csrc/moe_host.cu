@@ -74,7 +74,9 @@ int Dec::ensure_moe(int t, cudaStream_t st) {
     ok(cudaMalloc(&mb.c13, slots * 2 * moe.ffn * 2));
     ok(cudaMalloc(&mb.act, slots * moe.ffn * 2));
     ok(cudaMalloc(&mb.c2, slots * moe.hidden * 2));
-    ok(cudaMemset(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int)));   // the counts of a call are left at zero by it
+    if (e == cudaSuccess) {
+        e = fill_now(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int), st);   // the counts of a call are left at zero by it
+    }
     if (e != cudaSuccess) {
         free_moe();
         return cuda_fail("alloc moe scratch", e);

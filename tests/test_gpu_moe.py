@@ -230,3 +230,22 @@ def test_grouped_gemv_forms(dec, orc, t, n_exp, k, f, h, group, way):
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
     err = np.abs(y.cpu().numpy() - want).max()
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # as above
+
+
+# the first call of a scratch counts rows into memory that nothing has written before: on a stream of the caller's, and again after growth
+def test_first_calls_of_a_scratch_on_a_side_stream(dec):
+    n_exp, k, f, h, group = 16, 4, 128, 192, 32
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=41)
+    dec.set_moe(n_exp, k, f, h, group)
+    dec.upload_experts(0, w13_q, w13_s, w2_q, w2_s)
+    side = torch.cuda.Stream()
+    for t in (300, 1100):
+        x = torch.from_numpy(synth.make_acts(t, h, seed=42 + t).view(np.float16).copy()).cuda()
+        lg = torch.from_numpy(synth.make_router_logits(t, n_exp, seed=43 + t)).cuda()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            first = dec.moe_ffn_dev_t(0, lg, x, t)
+            again = dec.moe_ffn_dev_t(0, lg, x, t)
+        side.synchronize()
+        assert torch.equal(first, again)
+        assert torch.equal(first, dec.moe_ffn_dev_t(0, lg, x, t))

@@ -1,0 +1,50 @@
+"""The host code between the entry points and the kernels, on a stand-in for the CUDA runtime (fake_cudart.cpp): what is launched, cleared
+and awaited, in which order and on which stream."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from llm170_b200 import build
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SOURCES = ["dec.cu", "moe.cu", "moe_host.cu", "repack.cu"]      # the rest is not called
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("host")
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    jobs = [(["-c", os.path.join(build.CSRC, s)], str(tmp / (s + ".o"))) for s in SOURCES]
+    flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1"]
+    commands = [[nvcc, *flags, *args, "-o", out] for args, out in jobs]
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(nvcc) or nvcc))), "include")
+    jobs.append((None, str(tmp / "fake.o")))
+    commands.append(["g++", "-std=c++17", "-O1", "-I" + include, "-c", os.path.join(HERE, "fake_cudart.cpp"), "-o", jobs[-1][1]])
+    running = [subprocess.Popen(c, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True) for c in commands]
+    for p in running:
+        text = p.communicate()[0]
+        assert p.returncode == 0, text
+    exe = str(tmp / "host")
+    subprocess.run(["g++", "-no-pie", "-Wl,--unresolved-symbols=ignore-all", "-z", "lazy", *[out for _, out in jobs], "-o", exe], check=True)
+
+    def run(*args):
+        out = subprocess.run([exe, *map(str, args)], capture_output=True, text=True, timeout=60)
+        assert out.returncode == 0, (out.returncode, out.stdout, out.stderr)
+        return out.stdout.splitlines()
+
+    return run
+
+
+def _kernels(lines):
+    return [ln.split()[1] for ln in lines if ln.startswith("kernel ")]
+
+
+def test_expert_counts_are_clear_before_the_first_call_counts(host):
+    lines = host("moe")
+    assert lines.count("returned 0") == 2
+    assert not [ln for ln in lines if ln.startswith("UNORDERED")], lines
+    first_clear = next(i for i, ln in enumerate(lines) if ln.startswith("clear counts"))
+    first_count = next(i for i, ln in enumerate(lines) if "moe_topk" in ln)
+    assert first_clear < first_count
