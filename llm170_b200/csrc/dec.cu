@@ -32,6 +32,7 @@ int Dec::fail(const char* fmt, ...) {
 }
 
 int Dec::cuda_fail(const char* what, cudaError_t e) {
+    cudaGetLastError();      // reported here, and not once more by the check behind some later launch
     return fail("w4a16: %s: %s", what, cudaGetErrorString(e));
 }
 

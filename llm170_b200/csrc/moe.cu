@@ -404,7 +404,7 @@ inline int blocks_for(size_t total, int threads) {
 namespace {
 
 template <class... P, class... A>
-void launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, int pdl, A... args) {
+cudaError_t launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t st, int pdl, A... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -417,48 +417,61 @@ void launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
 }  // namespace
 
-void launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl,
-                     cudaStream_t st) {
+cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl,
+                            cudaStream_t st) {
     const int stage = n_exp <= 512;   // 8 warps x 512 floats = 16 KB of shared memory at most
-    launch(moe_topk_kernel, (t + TOPK_WARPS - 1) / TOPK_WARPS, TOPK_WARPS * 32, stage ? TOPK_WARPS * n_exp * sizeof(float) : 0, st, pdl,
-           logits, idx, wt, t, n_exp, k, stage, cnt, e0, e1);
+    return launch(moe_topk_kernel, (t + TOPK_WARPS - 1) / TOPK_WARPS, TOPK_WARPS * 32, stage ? TOPK_WARPS * n_exp * sizeof(float) : 0, st,
+                  pdl, logits, idx, wt, t, n_exp, k, stage, cnt, e0, e1);
 }
 
-// Returns the number of launches.  Up to eight tokens are routed by the table block itself (one launch); above that
-// one block's 32 warps would route two or more tokens each in turn (27 us at 64 tokens), so the routing runs on
-// many SMs first and the block only builds the tables.
-int launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm, int pdl,
-                           cudaStream_t st) {
+// Up to eight tokens are routed by the table block itself (one launch); above that one block's 32 warps would route two or more tokens
+// each in turn (27 us at 64 tokens), so the routing runs on many SMs first and the block only builds the tables.
+cudaError_t launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm, int pdl,
+                                   cudaStream_t st, unsigned long long& launched) {
     const int stage = n_exp <= 256;   // 32 warps x 256 floats = 32 KB beside the 12 KB of tables
     const int own_topk = t <= 8;
+    cudaError_t e = cudaSuccess;
     if (!own_topk) {
-        launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, nullptr, 0, 0, pdl, st);
+        e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, nullptr, 0, 0, pdl, st);
+        launched += e == cudaSuccess;
     }
-    launch(moe_route_small_kernel, 1, 1024, (stage && own_topk) ? 32 * n_exp * sizeof(float) : 0, st, pdl, logits, b.idx, b.wt, b.off,
-           b.pos_of_slot, b.slot_of_pos, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows, b.row_w, t, n_exp, k, e0, e1, bm,
-           stage, own_topk);
-    return own_topk ? 1 : 2;
+    if (e == cudaSuccess) {
+        e = launch(moe_route_small_kernel, 1, 1024, (stage && own_topk) ? 32 * n_exp * sizeof(float) : 0, st, pdl, logits, b.idx, b.wt,
+                   b.off, b.pos_of_slot, b.slot_of_pos, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows, b.row_w, t, n_exp, k,
+                   e0, e1, bm, stage, own_topk);
+        launched += e == cudaSuccess;
+    }
+    return e;
 }
 
-int launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
-                    int even, int pdl, cudaStream_t st) {
-    launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
-    launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
-           n_exp, e0, e1, bm, even);
-    launch(moe_place_gather_kernel, blocks_for((size_t)t, 1), GATHER_THREADS, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt, b.off,
-           b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
-    return 3;
+cudaError_t launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
+                            int even, int pdl, cudaStream_t st, unsigned long long& launched) {
+    cudaError_t e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    ++launched;
+    e = launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
+               n_exp, e0, e1, bm, even);
+    if (e != cudaSuccess) {
+        return e;
+    }
+    ++launched;
+    e = launch(moe_place_gather_kernel, blocks_for((size_t)t, 1), GATHER_THREADS, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt,
+               b.off, b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
+    launched += e == cudaSuccess;
+    return e;
 }
 
-void launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, int pdl, cudaStream_t st) {
+cudaError_t launch_moe_combine(const MoeBufs& b, void* out, int t, int h, int k, int out_f16, int pdl, cudaStream_t st) {
     const int g = blocks_for((size_t)t * (h / 8), 256);
-    launch(out_f16 ? moe_combine_kernel<true> : moe_combine_kernel<false>, g, 256, 0, st, pdl, (const __half*)b.c2, out, b.pos_of_slot, t,
-           h, k);
+    return launch(out_f16 ? moe_combine_kernel<true> : moe_combine_kernel<false>, g, 256, 0, st, pdl, (const __half*)b.c2, out,
+                  b.pos_of_slot, t, h, k);
 }
 
 }  // namespace w4

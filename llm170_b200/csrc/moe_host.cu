@@ -105,6 +105,16 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
     }
     const int ns = t * moe.top_k;
     const int n_local = moe.e1 - moe.e0;
+    cudaError_t e = cudaSuccess;
+    auto sort = [&](int bm, bool even) {
+        e = launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, even, tune_pdl, st, launches);
+        // The top-k may have counted, with nothing after it that clears the counts for the next call; where they cannot be cleared, that
+        // call makes its scratch anew.
+        if (e != cudaSuccess && cudaMemsetAsync(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int), st) != cudaSuccess) {
+            mb.cap_tokens = 0;
+        }
+        return e == cudaSuccess ? 0 : cuda_fail("moe_ffn launch", e);
+    };
     if ((long long)ns <= 8LL * moe.n_experts) {
         // decode-sized batches (on average at most 8 rows per expert): the op is weight streaming, so every
         // <=8-row segment of an expert runs through the GEMV kernel instead of a padded 128-row MMA tile
@@ -119,13 +129,18 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         }
         if (ns <= 1024) {
             // routing and all dispatch tables in one launch; the first grouped GEMV fetches each row's token itself
-            launches += launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, tune_pdl, st);
+            e = launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, tune_pdl, st, launches);
+            if (e != cudaSuccess) {
+                return cuda_fail("moe_ffn launch", e);
+            }
             if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st,
                                       mb.slot_of_pos, moe.top_k, /*tables_fresh=*/true)) {
                 return rc;
             }
         } else {
-            launches += launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, 8, 0, tune_pdl, st);
+            if (int rc = sort(8, false)) {
+                return rc;
+            }
             if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, nullptr,
                                       1, /*tables_fresh=*/true)) {
                 return rc;
@@ -144,7 +159,9 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         const bool weight_rows = (long long)ns < 192LL * moe.n_experts;
         const int bm = weight_rows ? 128 : 256;
         const int max_tiles = (ns + bm - 1) / bm + std::min(ns, n_local);
-        launches += launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, weight_rows, tune_pdl, st);
+        if (int rc = sort(bm, weight_rows)) {
+            return rc;
+        }
         if (weight_rows) {
             if (int rc = gemm_ts_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, bm, nullptr, st, true)) {
                 return rc;
@@ -161,10 +178,12 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             }
         }
     }
-    launch_moe_combine(mb, y, t, moe.hidden, moe.top_k, out_kind == W4A16_OUT_F16, tune_pdl, st);
+    e = launch_moe_combine(mb, y, t, moe.hidden, moe.top_k, out_kind == W4A16_OUT_F16, tune_pdl, st);
+    if (e != cudaSuccess) {
+        return cuda_fail("moe_ffn launch", e);
+    }
     launches += 1;
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : cuda_fail("moe_ffn launch", e);
+    return 0;
 }
 
 }  // namespace w4
@@ -254,10 +273,13 @@ int w4a16_moe_topk(w4a16_dec* dec, const float* logits_dev, int* idx_dev, float*
     if (!d.moe.set) {
         return d.fail("w4a16 moe_topk: set_moe was not called");
     }
-    w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, nullptr, 0, 0, d.tune_pdl, moe_stream(dec, stream));
+    const cudaError_t e =
+        w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, nullptr, 0, 0, d.tune_pdl, moe_stream(dec, stream));
+    if (e != cudaSuccess) {
+        return d.cuda_fail("moe_topk", e);
+    }
     d.launches++;
-    cudaError_t e = cudaGetLastError();
-    return e == cudaSuccess ? 0 : d.cuda_fail("moe_topk", e);
+    return 0;
 }
 
 int w4a16_moe_ffn(w4a16_dec* dec, int layer, const float* router_logits_dev, const void* x16_dev, void* y_dev, int t,

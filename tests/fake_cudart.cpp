@@ -140,6 +140,8 @@ cudaError_t cudaIpcGetMemHandle(cudaIpcMemHandle_t* h, void*) {
 
 namespace w4 {
 // the grouped matmuls: only that they are asked for
+bool moe_gemv_plan(int, int, int, int, int, int, MoeGemvPlan&) { return true; }
+cudaError_t launch_gemv_moe(const GemvArgs&, const MoeGemvPlan&, cudaStream_t st) { return start(matmul, st); }
 int Dec::gemm_ts_grouped(const Lin*, const void*, int, void*, int, const MoeBufs&, int, int, const float*, cudaStream_t st, bool) { return start(matmul, st); }
 int Dec::gemm_grouped(const Lin*, const void*, int, void*, int, const MoeBufs&, int, const float*, cudaStream_t st) { return start(matmul, st); }
 }  // namespace w4

@@ -48,3 +48,24 @@ def test_expert_counts_are_clear_before_the_first_call_counts(host):
     first_clear = next(i for i, ln in enumerate(lines) if ln.startswith("clear counts"))
     first_count = next(i for i, ln in enumerate(lines) if "moe_topk" in ln)
     assert first_clear < first_count
+
+
+# a launch that fails ends the call with an error: nothing that would read its tables is launched, and no count is left for the next call
+SORT = ["moe_topk", "moe_offsets", "moe_place_gather", "matmul", "matmul", "moe_combine"]
+SMALL = ["moe_topk", "moe_route_small", "matmul", "matmul", "moe_combine"]
+
+
+@pytest.mark.parametrize("tokens,chain,bad", [(256, SORT, i) for i in range(6)] + [(9, SMALL, i) for i in range(5)])
+def test_a_failed_launch_ends_the_call(host, tokens, chain, bad):
+    lines = host("moe", bad, tokens)
+    at = next(i for i, ln in enumerate(lines) if ln.startswith("returned"))
+    first, second = lines[:at], lines[at + 1:]
+    assert lines[at] != "returned 0" and second[-1] == "returned 0"
+    ran = _kernels(first)
+    assert len(ran) == bad and all(c in k for c, k in zip(chain, ran)), ran
+    ran = _kernels(second)
+    assert len(ran) == len(chain) and all(c in k for c, k in zip(chain, ran)), ran
+    if chain is SORT and bad < 2:
+        refused = next(i for i, ln in enumerate(lines) if ln.startswith("refused"))
+        assert lines[refused + 1] == "clear counts stream2"
+    assert not [ln for ln in lines if ln.startswith("UNORDERED")]
