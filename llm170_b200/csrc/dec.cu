@@ -89,7 +89,12 @@ int Dec::ensure_scratch(size_t part_floats, int grid_x, cudaStream_t st) {
         if (e != cudaSuccess) {
             return cuda_fail("alloc split-K tickets", e);
         }
-        cudaMemset(counters, 0, cap * sizeof(unsigned));
+        e = fill_now(counters, 0, cap * sizeof(unsigned), st);
+        if (e != cudaSuccess) {
+            cudaFree(counters);
+            counters = nullptr;
+            return cuda_fail("clear split-K tickets", e);
+        }
         counters_cap = cap;
     }
     return 0;
@@ -544,7 +549,7 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
         e = cudaMalloc(&d.gemm_status, sizeof(int));
     }
     if (e == cudaSuccess) {
-        e = cudaMemset(d.gemm_status, 0, sizeof(int));
+        e = w4::Dec::fill_now(d.gemm_status, 0, sizeof(int), d.stream);
     }
     if (e == cudaSuccess) {
         e = w4::gemv_init_device();
@@ -689,10 +694,17 @@ int w4a16_kernel_status(w4a16_dec* dec) {
         return d.cuda_fail("read kernel status", e);
     }
     if (st != 0) {
-        cudaMemset(d.gemm_status, 0, sizeof(int));
+        cudaSetDevice(d.device);
+        e = cudaDeviceSynchronize();       // launches that are under way still use them
+        if (e == cudaSuccess) {
+            e = Dec::fill_now(d.gemm_status, 0, sizeof(int), d.stream);
+        }
         // an abandoned launch may have left tickets taken and peers' sums unread
-        if (d.counters) {
-            cudaMemset(d.counters, 0, d.counters_cap * sizeof(unsigned));
+        if (e == cudaSuccess && d.counters) {
+            e = Dec::fill_now(d.counters, 0, d.counters_cap * sizeof(unsigned), d.stream);
+        }
+        if (e != cudaSuccess) {
+            return d.cuda_fail("clear kernel status", e);
         }
         // the exchange block of the fused all-reduce is NOT re-armed here: the peers may still be pushing into
         // it, and all ranks must restart from the same launch number (w4a16_tp_rearm, between two host barriers)
@@ -830,7 +842,12 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
             if (e != cudaSuccess) {
                 return d.cuda_fail("alloc timeline buffer", e);
             }
-            cudaMemset(d.dbg_buf, 0, w4::DBG_SLOTS * sizeof(long long));
+            e = Dec::fill_now(d.dbg_buf, 0, w4::DBG_SLOTS * sizeof(long long), d.stream);
+            if (e != cudaSuccess) {
+                cudaFree(d.dbg_buf);
+                d.dbg_buf = nullptr;
+                return d.cuda_fail("clear timeline buffer", e);
+            }
         } else if (!value && d.dbg_buf) {
             cudaDeviceSynchronize();
             cudaFree(d.dbg_buf);
@@ -1031,8 +1048,8 @@ int w4a16_tp_create(w4a16_dec* dec, int rank, int world, int max_rows, void* han
     }
     const size_t bytes = TP_HEADER + 2 * (size_t)world * area * sizeof(float);
     cudaError_t e = cudaMalloc(&d.tp_block, bytes);
-    if (e == cudaSuccess) e = cudaMemset(d.tp_block, 0, TP_HEADER);
-    if (e == cudaSuccess) e = cudaMemset((char*)d.tp_block + TP_HEADER, 0xff, bytes - TP_HEADER);   // the sentinel
+    if (e == cudaSuccess) e = Dec::fill_now(d.tp_block, 0, TP_HEADER, d.stream);
+    if (e == cudaSuccess) e = Dec::fill_now((char*)d.tp_block + TP_HEADER, 0xff, bytes - TP_HEADER, d.stream);   // the sentinel
     cudaIpcMemHandle_t h;
     if (e == cudaSuccess) e = cudaIpcGetMemHandle(&h, d.tp_block);
     if (e != cudaSuccess) {
@@ -1084,11 +1101,10 @@ int w4a16_tp_rearm(w4a16_dec* dec) {
     cudaSetDevice(d.device);
     cudaError_t e = cudaDeviceSynchronize();
     const size_t data = 2 * (size_t)d.tp.world * d.tp.area_floats * sizeof(float);
-    if (e == cudaSuccess) e = cudaMemset(d.tp_block, 0, TP_HEADER);                      // launch number and done count
-    if (e == cudaSuccess) e = cudaMemset((char*)d.tp_block + TP_HEADER, 0xff, data);     // every word: not arrived
-    if (e == cudaSuccess && d.counters) e = cudaMemset(d.counters, 0, d.counters_cap * sizeof(unsigned));
-    if (e == cudaSuccess) e = cudaMemset(d.gemm_status, 0, sizeof(int));
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = Dec::fill_now(d.tp_block, 0, TP_HEADER, d.stream);                      // launch number and done count
+    if (e == cudaSuccess) e = Dec::fill_now((char*)d.tp_block + TP_HEADER, 0xff, data, d.stream);     // every word: not arrived
+    if (e == cudaSuccess && d.counters) e = Dec::fill_now(d.counters, 0, d.counters_cap * sizeof(unsigned), d.stream);
+    if (e == cudaSuccess) e = Dec::fill_now(d.gemm_status, 0, sizeof(int), d.stream);
     return e == cudaSuccess ? 0 : d.cuda_fail("tp_rearm", e);
 }
 

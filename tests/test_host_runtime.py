@@ -69,3 +69,12 @@ def test_a_failed_launch_ends_the_call(host, tokens, chain, bad):
         refused = next(i for i, ln in enumerate(lines) if ln.startswith("refused"))
         assert lines[refused + 1] == "clear counts stream2"
     assert not [ln for ln in lines if ln.startswith("UNORDERED")]
+
+
+@pytest.mark.parametrize("what,cleared", [("scratch", ["tickets stream2"]), ("status", ["status stream1", "tickets stream1"]),
+                                          ("exchange", ["exchange stream1", "block stream1"]), ("timeline", ["block stream1"])])
+def test_what_launches_count_on_is_clear_before_them(host, what, cleared):
+    lines = host(what)
+    assert [ln[len("clear "):] for ln in lines if ln.startswith("clear ")] == cleared
+    assert not [ln for ln in lines if ln.startswith("UNORDERED")], lines
+    assert _kernels(lines) == ["matmul"]
