@@ -116,25 +116,11 @@ void Dec::free_lin(Lin& l) {
 // that weight with a single rounding -- the same one -- while every scaled scale is a finite f16 value and every weight, from s * 2^-E up,
 // a normal one: exponent fields e of all scales with e + 24 - E <= 30 and e - E >= 1.  Scales that span more than five binades, zeros,
 // subnormals, infinities and NaN keep the general expansion (fma_e = -1).
-int Dec::scan_scales(Lin& l) {
-    if (l.group != 128) {
-        return 0;      // four scale words per stage leave nothing to win (27 x 34816 x 5120, groups of 32: 30.5 / 30.2 us)
-    }
-    int range[2] = {31, 0};
-    cudaError_t e = cudaMemcpyAsync(err_flag + 1, range, sizeof(range), cudaMemcpyHostToDevice, stream);
-    if (e == cudaSuccess) {
-        launch_scale_range_f16(l.st, (size_t)l.n * (size_t)(l.k / l.group), err_flag + 1, stream);
-        e = cudaMemcpyAsync(range, err_flag + 1, sizeof(range), cudaMemcpyDeviceToHost, stream);
-    }
-    if (e == cudaSuccess) {
-        e = cudaStreamSynchronize(stream);
-    }
-    if (e != cudaSuccess) {
-        return cuda_fail("scale range", e);
-    }
-    const int shift = range[1] > 6 ? range[1] - 6 : 0;
-    l.fma_e = shift <= 20 && range[0] - shift >= 1 ? shift : -1;
-    return 0;
+// `flags`: as the repack of the scales left them.
+int Dec::fma_shift(int group, const int (&flags)[3]) {
+    const int lo = 31 - flags[1], hi = flags[2], shift = hi > 6 ? hi - 6 : 0;
+    // (groups of 32: four scale words per stage leave nothing to win; 27 x 34816 x 5120: 30.5 / 30.2 us)
+    return group == 128 && shift <= 20 && lo - shift >= 1 ? shift : -1;
 }
 
 int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, int n, int k, int group,
@@ -189,15 +175,15 @@ int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, i
         }
     }
     l.out_mul = ldexpf(1.0f, -shift);
-    cudaMemsetAsync(err_flag, 0, sizeof(int), stream);
+    int flags[3] = {};
+    cudaMemsetAsync(err_flag, 0, sizeof(flags), stream);
     launch_repack_q((const uint32_t*)q_dev, l.qt, n, k, glu_f, stream);
     launch_repack_s((const uint16_t*)s_dev, l.st, n, k, l.group, src_div, scale_bf16, shift, err_flag, glu_f, stream);
-    int bad = 0;
-    e = cudaMemcpyAsync(&bad, err_flag, sizeof(int), cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(flags, err_flag, sizeof(flags), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) {
         e = cudaStreamSynchronize(stream);
     }
-    if (e != cudaSuccess || bad) {
+    if (e != cudaSuccess || flags[0]) {
         cudaFree(l.qt);
         cudaFree(l.st);
         if (e != cudaSuccess) {
@@ -205,11 +191,7 @@ int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, i
         }
         return fail("w4a16 upload %s: a bf16 scale is not representable in f16 even after shifting", name);
     }
-    if (int rc = scan_scales(l)) {
-        cudaFree(l.qt);
-        cudaFree(l.st);
-        return rc;
-    }
+    l.fma_e = fma_shift(l.group, flags);
     l.bytes = qb + sb;
     auto it = lins.find(name);
     if (it != lins.end()) {

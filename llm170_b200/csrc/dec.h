@@ -17,7 +17,7 @@ struct Lin {
     int n = 0, k = 0, group = 0;   // group: of the resident scale tiles (128 or 32)
     int group_src = 0;             // group of the uploaded scales (64 is stored as two groups of 32)
     float out_mul = 1.0f;          // 2^-shift when bf16 scales had to be shifted into the f16 range (else 1)
-    int fma_e = -1;                // >= 0: f16((q - 8) * s) * 2^-fma_e comes from one multiply-add per pair (Dec::scan_scales)
+    int fma_e = -1;                // >= 0: f16((q - 8) * s) * 2^-fma_e comes from one multiply-add per pair (Dec::fma_shift)
     int glu_f = 0;                 // > 0: gate / up row blocks of every expert interleaved (layout.cuh), = ffn / 16
     size_t bytes = 0;
 };
@@ -73,7 +73,7 @@ struct Dec {
     unsigned* counters = nullptr;
     size_t counters_cap = 0;
     std::vector<void*> retired;   // scratch blocks superseded by larger ones: freed with the decoder (graphs may hold them)
-    int* err_flag = nullptr;       // device int[4]: repack error flag, bf16 exponent range (min, max)
+    int* err_flag = nullptr;       // device int[4]: what a repack of scales reports (internal.h); bf16 exponent range (min, max) from [1] on
     int* gemm_status = nullptr;  // device word: first bounded wait that expired in any kernel (0 = none)
     // device staging for the host-buffer entry points
     void* xh = nullptr;
@@ -124,7 +124,7 @@ struct Dec {
     static cudaError_t fill_now(void* p, int byte, size_t bytes, cudaStream_t st);
     int ensure_scratch(size_t part_floats, int grid_x, cudaStream_t st);
     void free_lin(Lin& l);
-    int scan_scales(Lin& l);
+    static int fma_shift(int group, const int (&flags)[3]);
     int upload_stream(const char* name, int n, int k, int group, int scale_bf16, w4a16_fill_fn fill, void* user,
                       int glu_f = 0);
     int upload_common(const char* name, const void* q_dev, const void* s_dev, int n, int k, int group,

@@ -67,7 +67,7 @@ struct TsArgs {
     int off_stage;       // grouped: results of a tile on their way out
     int pdl;
     float out_mul;
-    uint32_t fma_add, fma_mul;   // (20 - E) << 26 | (24 - E) << 10 and the pair (-8 * 2^-E, -8 * 2^-E) (Dec::scan_scales)
+    uint32_t fma_add, fma_mul;   // (20 - E) << 26 | (24 - E) << 10 and the pair (-8 * 2^-E, -8 * 2^-E) (Dec::fma_shift)
     int* status;
     // grouped (MoE) mode: token tiles come from a device table, one expert's weights (n rows) per tile; tok is then the most
     // rows that a tile holds
@@ -1028,7 +1028,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
-    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + "> " + std::to_string(c.tok) + "-token tiles" +
+    last_kernel = "gemm_ts_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(c.tok) + "-token tiles" +
                   (c.ks > 1 ? ", clusters of " + std::to_string(c.ks) : std::string());
     launches++;
     return 0;

@@ -33,7 +33,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 // Scale pair (rows g, g + 8) of a tile's 32 or more channels, ready for ts_expand: f16((q - 8) * s) as (q - 8) times s, or (FMA) as a
-// multiply-add of the raw nibble with s scaled by powers of two and -8 s 2^-E (Dec::scan_scales).
+// multiply-add of the raw nibble with s scaled by powers of two and -8 s 2^-E (Dec::fma_shift).
 template <bool FMA>
 struct TsScale {
     uint32_t s0, s1, c0, c1;

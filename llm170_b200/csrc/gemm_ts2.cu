@@ -604,7 +604,7 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
-    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + "> " + std::to_string(tok) + "-token tiles";
+    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(tok) + "-token tiles";
     launches++;
     return 0;
 }

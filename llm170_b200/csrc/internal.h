@@ -13,18 +13,18 @@ namespace w4 {
 void launch_repack_q(const uint32_t* q_orig, uint32_t* qt, int n, int k, int glu_f, cudaStream_t st);
 // Biased-exponent range of the non-zero bf16 scales: range2[0] = min (preset 255), range2[1] = max (preset 0).
 void launch_scale_range(const uint16_t* s_orig, size_t total, int* range2, cudaStream_t st);
-// Exponent fields of resident f16 scales (a multiple of 8 of them): range2[0] = min (preset 31), range2[1] = max (preset 0).
+// Exponent fields of resident f16 scales (a multiple of 8 of them): range2[0] = 31 - min, range2[1] = max (both preset to 0).
 void launch_scale_range_f16(const uint16_t* stl, size_t total, int* range2, cudaStream_t st);
 // `group` is the group size of the TILED array; a source group covers `src_div` tiled groups.  bf16 scales are
-// multiplied by 2^shift and stored as f16; err_flag (device int, may be null) is set to 1 if one of them is not
-// exactly representable.
+// multiplied by 2^shift and stored as f16; flags (three device ints, preset to 0): [0] is set to 1 if one of them is not
+// exactly representable, [1] and [2] become the exponent range of the stored scales as above.
 void launch_repack_s(const uint16_t* s_orig, uint16_t* stl, int n, int k, int group, int src_div, int scale_bf16,
-                     int shift, int* err_flag, int glu_f, cudaStream_t st);
+                     int shift, int* flags, int glu_f, cudaStream_t st);
 // the same for a chunk of source rows [16*rb0, 16*(rb0+nrbc)) (streamed uploads)
 void launch_repack_q_rows(const uint32_t* q_chunk, uint32_t* qt, int n, int k, int rb0, int nrbc, int glu_f,
                           cudaStream_t st);
 void launch_repack_s_rows(const uint16_t* s_chunk, uint16_t* stl, int n, int k, int group, int src_div, int scale_bf16,
-                          int shift, int* err_flag, int rb0, int nrbc, int glu_f, cudaStream_t st);
+                          int shift, int* flags, int rb0, int nrbc, int glu_f, cudaStream_t st);
 void launch_unpack_q(const uint32_t* qt, uint32_t* q_orig, int n, int k, cudaStream_t st);
 void launch_unpack_s(const uint16_t* stl, uint16_t* s_orig, int n, int k, int group, int src_div, cudaStream_t st);
 // out: f32 [n][k] (out_f16 == 0) or f16 [n][k] (out_f16 == 1, round-to-nearest-even of the f32 value);

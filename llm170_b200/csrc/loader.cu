@@ -530,7 +530,8 @@ int Dec::upload_stream(const char* name, int n, int k, int group, int scale_bf16
         }
     }
     l.out_mul = ldexpf(1.0f, -shift);
-    cudaMemsetAsync(err_flag, 0, sizeof(int), stream);
+    int flags[3] = {};
+    cudaMemsetAsync(err_flag, 0, sizeof(flags), stream);
     for (int r0 = 0, i = 0; r0 < n; r0 += rows_c, ++i) {
         const int rows = std::min(rows_c, n - r0);
         unsigned char* hp = (unsigned char*)pin + (i & 1) * slot;
@@ -546,8 +547,7 @@ int Dec::upload_stream(const char* name, int n, int k, int group, int scale_bf16
                              r0 / TILE_ROWS, rows / TILE_ROWS, glu_f, stream);
         cudaEventRecord(done[i & 1], stream);
     }
-    int bad = 0;
-    e = cudaMemcpyAsync(&bad, err_flag, sizeof(int), cudaMemcpyDeviceToHost, stream);
+    e = cudaMemcpyAsync(flags, err_flag, sizeof(flags), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) {
         e = cudaStreamSynchronize(stream);
     }
@@ -556,17 +556,14 @@ int Dec::upload_stream(const char* name, int n, int k, int group, int scale_bf16
     if (e == cudaSuccess) {
         e = cudaGetLastError();
     }
-    if (e != cudaSuccess || bad) {
+    if (e != cudaSuccess || flags[0]) {
         drop();
         if (e != cudaSuccess) {
             return cuda_fail("streamed upload", e);
         }
         return fail("w4a16 upload %s: a bf16 scale is not representable in f16 even after shifting", name);
     }
-    if (int rc = scan_scales(l)) {
-        drop();
-        return rc;
-    }
+    l.fma_e = fma_shift(l.group, flags);
     l.bytes = qb + sb;
     auto it = lins.find(name);
     if (it != lins.end()) {
@@ -845,6 +842,12 @@ int w4a16_load_lin_cache(w4a16_dec* dec, const char* name, const char* path, uin
         }
     }
     fclose(f);
+    int flags[3] = {};
+    if (ok && l.group == 128) {
+        cudaMemsetAsync(d.err_flag, 0, sizeof(flags), d.stream);
+        w4::launch_scale_range_f16(l.st, sb / 2, d.err_flag + 1, d.stream);
+        ok = cudaMemcpyAsync(flags, d.err_flag, sizeof(flags), cudaMemcpyDeviceToHost, d.stream) == cudaSuccess;
+    }
     e = cudaStreamSynchronize(d.stream);
     cudaEventDestroy(done[0]);
     cudaEventDestroy(done[1]);
@@ -853,11 +856,7 @@ int w4a16_load_lin_cache(w4a16_dec* dec, const char* name, const char* path, uin
         cudaFree(l.st);
         return d.fail("w4a16 load_lin_cache: reading %s failed", path);
     }
-    if (int rc = d.scan_scales(l)) {
-        cudaFree(l.qt);
-        cudaFree(l.st);
-        return rc;
-    }
+    l.fma_e = w4::Dec::fma_shift(l.group, flags);
     l.bytes = qb + sb;
     auto it = d.lins.find(name);
     if (it != d.lins.end()) {

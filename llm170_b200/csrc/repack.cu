@@ -120,7 +120,22 @@ __global__ void scale_range_kernel(const uint16_t* __restrict__ s, size_t total,
     }
 }
 
-// The same for resident f16 scales (range[0] starts at 31, range[1] at 0); zeros and subnormals count as exponent 0.
+// Exponent fields of f16 scales that a warp saw, lowest and highest: range[0] = most of 31 - field, range[1] = most of field, both from
+// zero on; zeros and subnormals count as field 0.  Nearly every warp finds the range already there and spares the atomics.
+__device__ __forceinline__ void note_scale_range(int lo, int hi, int* range) {
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    if ((threadIdx.x & 31) == 0) {
+        if (31 - lo > *(volatile int*)range) {
+            atomicMax(range, 31 - lo);
+        }
+        if (hi > *(volatile int*)(range + 1)) {
+            atomicMax(range + 1, hi);
+        }
+    }
+}
+
+// for scales that come without a repack (tile cache files)
 __global__ void scale_range_f16_kernel(const uint4* __restrict__ s, size_t total8, int* __restrict__ range) {
     int lo = 31, hi = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total8; i += (size_t)gridDim.x * blockDim.x) {
@@ -133,20 +148,16 @@ __global__ void scale_range_f16_kernel(const uint4* __restrict__ s, size_t total
             hi = max(hi, max(e0, e1));
         }
     }
-    lo = __reduce_min_sync(0xffffffffu, lo);
-    hi = __reduce_max_sync(0xffffffffu, hi);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(range, lo);
-        atomicMax(range + 1, hi);
-    }
+    note_scale_range(lo, hi, range);
 }
 
 // `ng`: groups per row of the TILED array; a source group covers `src_div` of them (2 when 64-channel groups are
 // stored as two 32-channel groups with the same scale, else 1).
 __global__ void repack_s_kernel(const uint16_t* __restrict__ s, uint16_t* __restrict__ stl, int n, int ng, int src_div,
-                                int scale_bf16, int shift, int* __restrict__ err, int glu_f) {
+                                int scale_bf16, int shift, int* __restrict__ flags, int glu_f) {
     const size_t total = (size_t)n * (size_t)ng;
     const int ng_src = ng / src_div;
+    int lo = 31, top = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
          i += (size_t)gridDim.x * blockDim.x) {
         // i indexes the tiled array: [rb][grp][j][hi]
@@ -157,20 +168,24 @@ __global__ void repack_s_kernel(const uint16_t* __restrict__ s, uint16_t* __rest
         if (scale_bf16) {
             int bad = 0;
             v = bf16_to_f16_exact(v, shift, &bad);
-            if (bad && err) {
-                *err = 1;
+            if (bad) {
+                flags[0] = 1;
             }
         }
+        lo = min(lo, v >> 10 & 31);
+        top = max(top, v >> 10 & 31);
         stl[i] = v;
     }
+    note_scale_range(lo, top, flags + 1);
 }
 
 // Scales of a chunk of source rows: the tiled array keeps a row block's groups together, so the chunk's tiles are the
 // contiguous range starting at row block rb0.
 __global__ void repack_s_rows_kernel(const uint16_t* __restrict__ s, uint16_t* __restrict__ stl, int ng, int src_div,
-                                     int scale_bf16, int shift, int* __restrict__ err, int rb0, int nrbc, int glu_f) {
+                                     int scale_bf16, int shift, int* __restrict__ flags, int rb0, int nrbc, int glu_f) {
     const size_t total = (size_t)nrbc * TILE_ROWS * (size_t)ng;
     const int ng_src = ng / src_div;
+    int lo = 31, top = 0;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total;
          i += (size_t)gridDim.x * blockDim.x) {
         const int hi = (int)(i & 1), j = (int)((i >> 1) & 7);
@@ -180,12 +195,15 @@ __global__ void repack_s_rows_kernel(const uint16_t* __restrict__ s, uint16_t* _
         if (scale_bf16) {
             int bad = 0;
             v = bf16_to_f16_exact(v, shift, &bad);
-            if (bad && err) {
-                *err = 1;
+            if (bad) {
+                flags[0] = 1;
             }
         }
+        lo = min(lo, v >> 10 & 31);
+        top = max(top, v >> 10 & 31);
         stl[(size_t)glu_dest_rb(rb0 + rb, glu_f) * ng * 16 + (i - (size_t)rb * ng * 16)] = v;
     }
+    note_scale_range(lo, top, flags + 1);
 }
 
 __global__ void unpack_s_kernel(const uint16_t* __restrict__ stl, uint16_t* __restrict__ s, int n, int ng, int src_div) {
@@ -314,8 +332,8 @@ void launch_scale_range_f16(const uint16_t* stl, size_t total, int* range2, cuda
     scale_range_f16_kernel<<<grid_for(total / 8), 256, 0, st>>>((const uint4*)stl, total / 8, range2);
 }
 void launch_repack_s(const uint16_t* s, uint16_t* stl, int n, int k, int group, int src_div, int scale_bf16, int shift,
-                     int* err, int glu_f, cudaStream_t st) {
-    repack_s_kernel<<<grid_for((size_t)n * (k / group)), 256, 0, st>>>(s, stl, n, k / group, src_div, scale_bf16, shift, err,
+                     int* flags, int glu_f, cudaStream_t st) {
+    repack_s_kernel<<<grid_for((size_t)n * (k / group)), 256, 0, st>>>(s, stl, n, k / group, src_div, scale_bf16, shift, flags,
                                                                        glu_f);
 }
 void launch_repack_q_rows(const uint32_t* q_chunk, uint32_t* qt, int n, int k, int rb0, int nrbc, int glu_f,
@@ -323,10 +341,10 @@ void launch_repack_q_rows(const uint32_t* q_chunk, uint32_t* qt, int n, int k, i
     repack_q_rows_kernel<<<grid_for((size_t)nrbc * TILE_ROWS * (k / 8)), 256, 0, st>>>(q_chunk, qt, n, k, rb0, nrbc, glu_f);
 }
 void launch_repack_s_rows(const uint16_t* s_chunk, uint16_t* stl, int n, int k, int group, int src_div, int scale_bf16,
-                          int shift, int* err, int rb0, int nrbc, int glu_f, cudaStream_t st) {
+                          int shift, int* flags, int rb0, int nrbc, int glu_f, cudaStream_t st) {
     (void)n;
     repack_s_rows_kernel<<<grid_for((size_t)nrbc * TILE_ROWS * (k / group)), 256, 0, st>>>(
-        s_chunk, stl, k / group, src_div, scale_bf16, shift, err, rb0, nrbc, glu_f);
+        s_chunk, stl, k / group, src_div, scale_bf16, shift, flags, rb0, nrbc, glu_f);
 }
 void launch_unpack_q(const uint32_t* qt, uint32_t* q, int n, int k, cudaStream_t st) {
     unpack_q_kernel<<<grid_for((size_t)n * (k / 8)), 256, 0, st>>>(qt, q, n, k);

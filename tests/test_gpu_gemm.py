@@ -484,3 +484,35 @@ def test_cta_pair_tuning_refuses_values_without_a_tile(dec, bad):
     from llm170_b200.w4a16_dec import W4a16Error
     with pytest.raises(W4a16Error, match="gemm_pair"):
         dec.set_tuning("gemm_pair", bad)
+
+
+# Which expansion a linear takes follows from its scales, whichever way they came: one multiply-add per pair of weights while all of them are
+# normal and within six exponents, the general one otherwise.  n and k leave the last scale to a chunk and a warp of its own.
+@pytest.mark.parametrize("path", ["host", "device", "stream", "cache"])
+@pytest.mark.parametrize("odd,fma", [(None, True), (9 << 10, True), (10 << 10, False), (3 << 10, True), (2 << 10, False), (0, False), (5, False), (31 << 10, False),
+                                     (0x8000 | 4 << 10, True)])
+def test_expansion_follows_the_scales(dec, tmp_path, path, odd, fma):
+    n, k = 4112, 1152
+    rng = np.random.default_rng(8)
+    q = rng.integers(0, 2 ** 32, (n, k // 8), dtype=np.uint32)
+    s = (rng.integers(4, 9, (n, k // 128)) << 10 | rng.integers(0, 1024, (n, k // 128))).astype(np.uint16)
+    if odd is not None:
+        s[-1, -1] = odd
+    if path == "device":
+        dec.upload_lin_g_dev("ef", torch.from_numpy(q.view(np.int32)).cuda(), torch.from_numpy(s.view(np.int16)).cuda(), n, k, 128)
+    elif path == "stream":
+        parts = (q.tobytes(), s.tobytes())
+
+        def fill(which, off, buf):
+            buf[:] = parts[which][off:off + len(buf)]
+
+        dec.upload_lin_g_stream("ef", n, k, 128, False, fill)
+    else:
+        dec.upload_lin_g("ef", q, s, n, k, 128)
+    if path == "cache":
+        dec.save_lin_cache("ef", str(tmp_path / "ef"), 1)
+        dec.drop_lin("ef")
+        dec.load_lin_cache("ef", str(tmp_path / "ef"), 1)
+    dec.lin_forward("ef", torch.zeros((16, k), device="cuda", dtype=torch.float16), 16)
+    assert dec.last_kernel().startswith("gemm_ts_kernel<128,fma>" if fma else "gemm_ts_kernel<128>"), dec.last_kernel()
+    dec.drop_lin("ef")

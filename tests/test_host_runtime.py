@@ -78,3 +78,11 @@ def test_what_launches_count_on_is_clear_before_them(host, what, cleared):
     assert [ln[len("clear "):] for ln in lines if ln.startswith("clear ")] == cleared
     assert not [ln for ln in lines if ln.startswith("UNORDERED")], lines
     assert _kernels(lines) == ["matmul"]
+
+
+# what an upload learns about its scales comes with the repack: no pass, copy or wait of its own in groups of 128
+@pytest.mark.parametrize("bf16", [0, 1])
+def test_upload_of_128_channel_groups_waits_no_more_than_of_32(host, bf16):
+    want = host("upload", -1, 32, bf16)
+    assert want[-1] == "returned 0" and sum("repack_q_kernel" in k or "repack_s_kernel" in k for k in _kernels(want)) == 2
+    assert host("upload", -1, 128, bf16) == want
