@@ -232,7 +232,8 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
     // and replay to the same bits is what they are used for; the row-group form is 1.1 to 1.5 times as fast there, too, and
     // w4a16_lin_forward runs it.
     const bool stock = tune_gemv_rowblock == 1 && tune_gemv_rowblock_units && tune_gemv_persistent == 1 && tune_gemv_cluster &&
-                       tune_gemv_subnormal && tune_gemv_ksplit == 0;
+                       tune_gemv_subnormal && tune_gemv_ksplit == 0 && tune_gemv_stages == GEMV_STAGES && tune_gemv_warps == GEMV_WARPS &&
+                       tune_gemv_sk_stages == GEMV_SK_STAGES && tune_gemv_sk_prefetch == GEMV_SK_PREFETCH;
     const bool rowgroup = tune_gemv_rowgroup > 0 && stock && !allreduce;
     auto choose_rowgroup = [&]() {
         const int forced = tune_gemv_rowgroup - 1;

@@ -90,11 +90,12 @@ struct Dec {
     float* head_scale = nullptr;
     int head_n = 0, head_k = 0;
     // knobs
-    int tune_gemv_stages = 4;
+    static constexpr int GEMV_STAGES = 4, GEMV_WARPS = 8, GEMV_SK_STAGES = 4, GEMV_SK_PREFETCH = 2;
+    int tune_gemv_stages = GEMV_STAGES;
     int tune_gemv_rowblock_units = 1;  // 1: launches whose 32-row units are all resident at once run the 16-warp variant
-    int tune_gemv_warps = 8;
-    int tune_gemv_sk_stages = 4;   // most 16 KB ring stages of the persistent GEMV (2..6; fewer when x needs the room)
-    int tune_gemv_sk_prefetch = 2; // ring stages the persistent GEMV requests before the previous kernel is complete
+    int tune_gemv_warps = GEMV_WARPS;
+    int tune_gemv_sk_stages = GEMV_SK_STAGES;   // most 16 KB ring stages of the persistent GEMV (2..6; fewer when x needs the room)
+    int tune_gemv_sk_prefetch = GEMV_SK_PREFETCH; // ring stages the persistent GEMV requests before the previous kernel is complete
     int tune_gemv_rowblock = 1;    // up to four tokens of a g128 linear run one small CTA per 16-row block (gemv_rb.cu)
     int tune_gemv_persistent = 1;  // dense decode GEMV as two persistent CTAs per SM with equal unit ranges (gemv_sk.cu)
     int tune_gemv_cluster = 1;   // K splits of a row block as a thread-block cluster (DSMEM reduce) when 2 <= ksplit <= 8

@@ -743,7 +743,8 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                         l->k, tune_ts_ks);
         }
         const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
-        if (t > 64 && t <= 4096 && !(ts && c.ks > 1) && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0) {
+        if (t > 64 && t <= 4096 && !(ts && c.ks > 1) && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0 &&
+            tune_gemm_tma_store == 1) {
             // The pairs (gemm_ts2.cu) take what they are estimated to finish sooner by at least 2 %.  Over 140 drawn shapes (66..4096 tokens) the
             // choice took 6.4 % less time than the better of the two other forms' rule, the best choice of each 7.1 %; the worst case was
             // 551 x 20752 x 16128, 301 against 294 us, the best 3418 x 24592 x 1408, 185 against 266.  Calls of few tiles (526 x 2144 x 16384: 52 against 38 us)

@@ -602,3 +602,28 @@ def test_row_group_form_leaves_what_does_not_fit(dec, orc):
     dec.lin_forward("rgx", x_dev(xs[:1]), 1)
     assert dec.last_kernel().startswith("gemv_rg_kernel")
     dec.drop_lin("rgx")
+
+
+# a tuning key moves a call to the form that it tunes, also where the row-group form would run
+@pytest.mark.parametrize("key,value,default,k,t,form", [
+    ("gemv_stages", 3, 4, 2048, 8, "gemv_w4a16_kernel"), ("gemv_warps", 16, 8, 2048, 8, "gemv_w4a16_kernel"), ("gemv_sk_stages", 3, 4, 6272, 2, "gemv_sk_kernel"),
+    ("gemv_sk_prefetch", 4, 2, 6272, 2, "gemv_sk_kernel"), ("gemv_cluster", 0, 1, 2048, 8, "gemv_w4a16_kernel"), ("gemv_ksplit", 2, 0, 2048, 8, "gemv_w4a16_kernel"),
+    ("gemv_persistent", 2, 1, 2048, 8, "gemv_sk_kernel"), ("gemv_rowblock", 2, 1, 2048, 2, "gemv_rb_kernel"), ("gemm_tma_store", 0, 1, 2048, 2048, "gemm_w4a16_tc_kernel")])
+def test_tuning_keys_reach_their_form(dec, orc, key, value, default, k, t, form):
+    n = 20000
+    q, s = synth.make_linear(n, k, 128, seed=960)
+    dec.upload_lin_g("key", q, s, n, k, 128)
+    xs = synth.make_acts(t, k, seed=961)
+    y = dec.lin_forward("key", x_dev(xs), t, out_f16=t > 8)
+    assert dec.last_kernel().startswith("gemv_rg_kernel" if t <= 8 else "gemm_ts2_kernel"), dec.last_kernel()
+    dec.set_tuning(key, value)
+    try:
+        tuned = dec.lin_forward("key", x_dev(xs), t, out_f16=t > 8)
+        assert dec.last_kernel().startswith(form), dec.last_kernel()
+        dec.sync()
+    finally:
+        dec.set_tuning(key, default)
+    bound = 2.0 ** -20 if t <= 8 else 2.0 ** -9                     # f32 terms in another order; f16 results: their rounding
+    size = (x_dev(xs).float().abs() @ dec.dequant_lin("key").abs().T).max().item()
+    assert (y.float() - tuned.float()).abs().max().item() <= bound * size
+    dec.drop_lin("key")
