@@ -19,9 +19,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <new>
 #include <string>
-#include <vector>
 
 #include "../../include/w4a16_b200.h"
 #include "dec.h"
@@ -98,6 +96,20 @@ __device__ __forceinline__ uint32_t ob_pair_to_half2(uint32_t w, uint32_t sel) {
     return r;
 }
 
+// Rows of whole row blocks out of the resident order, offset-binary -> two's complement.  A block takes a row at a time.
+__global__ void __launch_bounds__(256) head_untile_kernel(const uint8_t* __restrict__ q, uint4* __restrict__ rows, int n, int k) {
+    for (int r = blockIdx.x; r < n; r += gridDim.x) {
+        for (int c = threadIdx.x; c < k / 16; c += blockDim.x) {
+            uint4 v = *reinterpret_cast<const uint4*>(q + head_at((size_t)r, c * 16, k));
+            v.x ^= 0x80808080u;
+            v.y ^= 0x80808080u;
+            v.z ^= 0x80808080u;
+            v.w ^= 0x80808080u;
+            rows[(size_t)r * (k / 16) + c] = v;
+        }
+    }
+}
+
 struct HeadArgs {
     const uint8_t* q;
     const float* scale;
@@ -106,9 +118,10 @@ struct HeadArgs {
     int n, k, t0, tp;
 };
 
-// D = 64-channel steps that a warp has on the way.
+// D = 64-channel steps that a warp has on the way in its ring; 0: loads to registers, eight steps unrolled, for activations that leave no room
+// for a ring of three (head_depth).
 template <int D>
-__global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const HeadArgs a) {
+__global__ void __launch_bounds__(HEAD_THREADS, D > 0 ? 2 : 1) head_gemv_i8_kernel(const HeadArgs a) {
     extern __shared__ __align__(128) unsigned char hsm[];
     constexpr int WARPS = HEAD_THREADS / 32;
     __shared__ float4 s_part[WARPS * 32];
@@ -139,6 +152,9 @@ __global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const Hea
     int fr = -1, fleft = 0;                                                      // round being requested, steps left in it
     uint32_t fdst = 0;
     auto fetch = [&]() {
+        if (D == 0) {
+            return;
+        }
         if (fleft == 0 && fr < rounds) {
             ++fr;
             const int rb = fr < rounds ? fr * all_warps + (int)blockIdx.x * WARPS + warp : rb_rest;
@@ -180,15 +196,24 @@ __global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const Hea
     // lanes whose column of the MMA holds no token read token 0: their sums are never stored
     const uint32_t xh_l = smem_u32(xhi) + (uint32_t)((g < tp ? g : 0) * xrow + tq * 32), xl_l = xh_l + (uint32_t)(tp * xrow);
     uint32_t rsrc = 0;
-    // sums of the next row block in the ring, steps [s0, s1): .x, .y = row g, tokens 2tq, 2tq + 1;  .z, .w = row g + 8
-    auto multiply = [&](int s0, int s1) {
+    // sums of row block rb (with a ring: of the next one in it), steps [s0, s1): .x, .y = row g, tokens 2tq, 2tq + 1;  .z, .w = row g + 8
+    auto multiply = [&](int rb, int s0, int s1) {
         float ch[4] = {0.f, 0.f, 0.f, 0.f}, cl[4] = {0.f, 0.f, 0.f, 0.f};
+        const uint4* wp = reinterpret_cast<const uint4*>(a.q + (size_t)rb * nsteps * 1024) + lane;
+#pragma unroll(D > 0 ? 1 : 8)
         for (int s = s0; s < s1; ++s) {
-            cp_async_wait_group<D - 1>();
-            const uint4 w0 = lds128(ring + rsrc), w1 = lds128(ring + rsrc + 512u);
-            fetch();
-            if ((rsrc += 1024u) == D * 1024u) {
-                rsrc = 0;
+            uint4 w0, w1;
+            if (D > 0) {
+                cp_async_wait_group<(D > 0 ? D - 1 : 0)>();
+                w0 = lds128(ring + rsrc);
+                w1 = lds128(ring + rsrc + 512u);
+                fetch();
+                if ((rsrc += 1024u) == D * 1024u) {
+                    rsrc = 0;
+                }
+            } else {
+                w0 = __ldg(wp + s * 64);
+                w1 = __ldg(wp + s * 64 + 32);
             }
             const uint32_t ww0[4] = {w0.x, w0.y, w0.z, w0.w}, ww1[4] = {w1.x, w1.y, w1.z, w1.w};
 #pragma unroll
@@ -231,13 +256,13 @@ __global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const Hea
         }
     };
     for (int i = 0; i < rounds; ++i) {
-        const float4 c = multiply(0, nsteps);
-        store(i * all_warps + (int)blockIdx.x * WARPS + warp, c);
+        const int rb = i * all_warps + (int)blockIdx.x * WARPS + warp;
+        store(rb, multiply(rb, 0, nsteps));
     }
     if (rest == 0) {
         return;
     }
-    float4 c = multiply(s0_rest, s0_rest + n_rest);
+    float4 c = multiply(rb_rest, s0_rest, s0_rest + n_rest);
     if (ways > 1) {
         s_part[threadIdx.x] = c;
         __syncthreads();
@@ -256,7 +281,7 @@ __global__ void __launch_bounds__(HEAD_THREADS, 2) head_gemv_i8_kernel(const Hea
     }
 }
 
-constexpr int HEAD_DEPTHS[] = {8, 6, 5, 4, 3, 2, 1};
+constexpr int HEAD_DEPTHS[] = {8, 6, 5, 4, 3, 0};
 constexpr size_t HEAD_SMEM_MAX = 218 * 1024;            // beside 8 KB for the sums
 // Steps on the way per warp beside `x_bytes` of activations: five where that leaves room for a second CTA (the next call's, whose weights
 // are then on the way before this one ends), else what fits beside them.
@@ -269,7 +294,7 @@ int head_depth(size_t x_bytes) {
             return d;
         }
     }
-    return 1;
+    return 0;
 }
 const void* head_kernel(int depth) {
     switch (depth) {
@@ -278,8 +303,7 @@ const void* head_kernel(int depth) {
     case 5: return (const void*)head_gemv_i8_kernel<5>;
     case 4: return (const void*)head_gemv_i8_kernel<4>;
     case 3: return (const void*)head_gemv_i8_kernel<3>;
-    case 2: return (const void*)head_gemv_i8_kernel<2>;
-    default: return (const void*)head_gemv_i8_kernel<1>;
+    default: return (const void*)head_gemv_i8_kernel<0>;
     }
 }
 
@@ -375,28 +399,28 @@ int w4a16_head_unpack(w4a16_dec* dec, void* q_host, void* scale_host) {
         return d.fail("w4a16 head: no lm-head uploaded");
     }
     cudaSetDevice(d.device);
-    // 32 MB of whole row blocks at a time, from the resident order to rows, offset-binary -> two's complement
-    const int k = d.head_k, rows_chunk = (int)std::max<size_t>(16, ((size_t)32 << 20) / k / 16 * 16);
-    std::vector<unsigned char> tiles;
-    cudaError_t e = cudaSuccess;
-    try {
-        tiles.resize((size_t)std::min(rows_chunk, (d.head_n + 15) / 16 * 16) * k);
-    } catch (const std::bad_alloc&) {
-        return d.fail("w4a16 head_unpack: out of host memory");
+    // 32 MB of whole row blocks at a time (less where the device has no room), from the resident order to rows on the device
+    const int k = d.head_k;
+    int rows_chunk = (int)std::min<size_t>(std::max<size_t>(16, ((size_t)32 << 20) / k / 16 * 16), (size_t)(d.head_n + 15) / 16 * 16);
+    uint4* rows_dev = nullptr;
+    cudaError_t e = cudaMalloc(&rows_dev, (size_t)rows_chunk * k);
+    while (e != cudaSuccess && rows_chunk > 16) {
+        cudaGetLastError();
+        rows_chunk = std::max(16, rows_chunk / 2 / 16 * 16);
+        e = cudaMalloc(&rows_dev, (size_t)rows_chunk * k);
     }
     for (int r0 = 0; r0 < d.head_n && e == cudaSuccess; r0 += rows_chunk) {
         const int rows = std::min(rows_chunk, d.head_n - r0);
-        e = cudaMemcpy(tiles.data(), d.head_q + (size_t)r0 * k, (size_t)((rows + 15) / 16 * 16) * k, cudaMemcpyDeviceToHost);
-        for (int r = 0; r < rows && e == cudaSuccess; ++r) {
-            unsigned char* dst = (unsigned char*)q_host + (size_t)(r0 + r) * k;
-            for (int c = 0; c < k; c += 16) {
-                const unsigned char* src = tiles.data() + w4::head_at((size_t)r, c, k);
-                for (int i = 0; i < 16; ++i) {
-                    dst[c + i] = src[i] ^ 0x80;
-                }
-            }
+        w4::head_untile_kernel<<<std::min(rows, 148 * 16), 256, 0, d.stream>>>(d.head_q + (size_t)r0 * k, rows_dev, rows, k);
+        e = cudaGetLastError();
+        if (e == cudaSuccess) {
+            e = cudaMemcpyAsync((unsigned char*)q_host + (size_t)r0 * k, rows_dev, (size_t)rows * k, cudaMemcpyDeviceToHost, d.stream);
+        }
+        if (e == cudaSuccess) {
+            e = cudaStreamSynchronize(d.stream);
         }
     }
+    cudaFree(rows_dev);
     if (e == cudaSuccess && scale_host) {
         e = cudaMemcpy(scale_host, d.head_scale, (size_t)d.head_n * 4, cudaMemcpyDeviceToHost);
     }

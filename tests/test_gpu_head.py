@@ -116,3 +116,25 @@ def test_contract_errors():
             d.head_forward(torch.zeros(17 * 128, device="cuda"), 17)
     finally:
         d.close()
+
+
+# Activations that leave no room for a ring of three steps (the weights then come through registers): whole rounds and a rest of one row block,
+# rests that are split along K over two to sixteen warps, seven and eight tokens, several launches, and the last size that has a ring.
+@pytest.mark.parametrize("n,k,t", [(37904, 6144, 8), (1000, 6144, 8), (40, 6144, 7), (5000, 8192, 14), (2370, 16384, 3), (777, 49984, 1),
+                                   (1000, 5312, 8)])
+def test_head_gemv_without_a_ring(dec, n, k, t):
+    gen = torch.Generator("cuda").manual_seed(n + t)
+    w = (torch.randn((n, k), device="cuda", generator=gen) * 0.02).to(torch.bfloat16)
+    dec.upload_head(w.view(torch.int16).cpu().numpy().view(np.uint16), n, k)
+    q, sc = dec.head_unpack()
+    x = torch.randn((t, k), device="cuda", generator=gen)
+    guard = torch.full((t + 1, n), 7.0, device="cuda")
+    y = dec.head_forward(x, t, out=guard[:t])
+    torch.cuda.synchronize()
+    for r0 in range(0, n, 4096):
+        qd = torch.from_numpy(q[r0:r0 + 4096]).cuda().double()
+        s = torch.from_numpy(sc[r0:r0 + 4096]).cuda().double()
+        bound = REL * (x.double().abs() @ qd.abs().T) * s
+        assert ((y[:, r0:r0 + 4096].double() - (x.double() @ qd.T) * s).abs() <= bound).all()
+    assert (guard[t:] == 7.0).all()
+    assert torch.equal(y, dec.head_forward(x, t))
