@@ -122,8 +122,8 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         // this bound, and CTAs beyond the actual count leave at once
         const int est_tiles = ns < n_local ? ns : n_local;   // segments expected to be non-empty (split-K sizing)
         const int max_tiles = est_tiles + ns / 8;
-        // local experts that a batch of t tokens reaches on average
-        const int est_segments = (int)(n_local * (1.0 - pow(1.0 - (double)moe.top_k / moe.n_experts, t)) + 0.5);
+        // local experts that a batch of t tokens reaches on average; where it is less than one, of the calls that reach one
+        const int est_segments = std::max(1, (int)(n_local * (1.0 - pow(1.0 - (double)moe.top_k / moe.n_experts, t)) + 0.5));
         if (max_tiles > mb.max_tiles) {
             return fail("w4a16 moe_ffn: tile table too small");
         }

@@ -249,3 +249,22 @@ def test_first_calls_of_a_scratch_on_a_side_stream(dec):
         side.synchronize()
         assert torch.equal(first, again)
         assert torch.equal(first, dec.moe_ffn_dev_t(0, lg, x, t))
+
+
+# where a call reaches less than half an expert of this rank on average, the plan is the one for a call that reaches one
+@pytest.mark.parametrize("n_exp,k,f,h", [(8, 2, 512, 256), (128, 4, 1024, 320)])
+def test_plan_of_a_rank_that_is_hardly_reached(dec, orc, n_exp, k, f, h):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, 32, seed=51)
+    x = synth.make_acts(1, h, seed=52)
+    lg = synth.make_router_logits(1, n_exp, seed=53)
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    total, names = 0, set()
+    for e0 in range(n_exp):
+        dec.set_moe(n_exp, k, f, h, 32, e0, 1)
+        dec.upload_experts(0, w13_q[e0:e0 + 1], w13_s[e0:e0 + 1], w2_q[e0:e0 + 1], w2_s[e0:e0 + 1])
+        total = total + dec.moe_ffn_dev_t(0, lgd, xd, 1).cpu().numpy()
+        names.add(dec.last_kernel())
+    assert names == {"gemv_moe_kernel<32,8>"}
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, 32)
+    err = np.abs(total - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())
