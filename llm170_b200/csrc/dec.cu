@@ -391,7 +391,7 @@ int Dec::gemv(const Lin* const* ls, int nseg, const void* x, void* const* outs, 
 // w4a16_gemv_experts_* kernels (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:317-374,
 // crates/backend-gpu/src/rawcuda/w4a16_dec/moe/moe_gemv.rs:92-114).
 int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
-                      int est_tiles, int est_segments, const float* row_w, cudaStream_t st, const int* x_slot_of_pos,
+                      int est_tiles, int est_segments, const float* row_w, cudaStream_t st, bool& uneven, const int* x_slot_of_pos,
                       int x_slots_per_token, bool tables_fresh) {
     if (l->glu_f > 0 && tune_gemv_warps != 8) {
         return fail("w4a16 grouped gemv: the fused gate|up form needs gemv_warps = 8");
@@ -425,6 +425,8 @@ int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert,
     a.nrb_w = l->n / TILE_ROWS;
     a.tp = TpComm{};
     cudaError_t e;
+    const bool after_uneven = uneven;
+    uneven = false;
     // The form with four row blocks per warp (gemv_moe.cu) wherever eight rows of x fit beside its rings (K up to about 10000);
     // the (row block, K split) form stages K / ksplit of them and takes any K.
     MoeGemvPlan gp{};
@@ -434,6 +436,7 @@ int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert,
         if (e != cudaSuccess) {
             return cuda_fail("launch grouped gemv", e);
         }
+        uneven = gp.uneven;
         last_kernel = "gemv_moe_kernel<" + std::to_string(a.group) + "," + std::to_string(gp.kw) + ">";
         launches++;
         return 0;
@@ -456,6 +459,12 @@ int Dec::gemv_grouped(const Lin* l, const void* xs, void* out, int n_per_expert,
         return fail("w4a16 grouped gemv: k=%d too large", a.k);
     }
     a.ksplit = ks;
+    // Behind a row-group matmul whose CTAs end unevenly this one starts when that is complete: programmatically launched, its clusters fill the
+    // SMs that end first two by two and leave the others one (8 experts, top-2, 4096 x 14336 in groups of 128, one token: 76.5 us per layer
+    // so, with this form for both matmuls 68, now 64.8; 4096 x 12288 70.2, 67, 60.5).
+    if (after_uneven) {
+        a.pdl = 0;
+    }
     a.ring_stages = grouped_stages;
     a.cons_warps = tune_gemv_warps;
     a.cluster = ks >= 2 ? 1 : 0;

@@ -202,6 +202,7 @@ bool moe_gemv_plan(int rows, int k, int group, int sm_count, int segments, int f
         if (force_kw > 1 ? kw == force_kw : (best < 0 || cost < best)) {
             best = cost;
             p.kw = kw;
+            p.uneven = units > p.ctas && units < 4 * p.ctas && units % p.ctas != 0;
         }
     }
     return true;

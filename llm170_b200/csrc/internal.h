@@ -161,6 +161,7 @@ const char* gemv_rg_name(int group, const RgPlan& p);
 struct MoeGemvPlan {
     int kw;                  // warps along K: 2, 4 or 8
     int ctas;                // two per SM (one, where the activations leave no room)
+    bool uneven;             // some CTAs are expected to take one to three units and others one more
     int off_red, off_ring;   // byte offsets in dynamic shared memory: activations first
     int smem;
 };

@@ -127,13 +127,14 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         if (max_tiles > mb.max_tiles) {
             return fail("w4a16 moe_ffn: tile table too small");
         }
+        bool uneven = false;                         // whether the CTAs of the matmul before end far apart
         if (ns <= 1024) {
             // routing and all dispatch tables in one launch; the first grouped GEMV fetches each row's token itself
             e = launch_moe_route_small(logits, mb, t, moe.n_experts, moe.top_k, moe.e0, moe.e1, 8, tune_pdl, st, launches);
             if (e != cudaSuccess) {
                 return cuda_fail("moe_ffn launch", e);
             }
-            if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st,
+            if (int rc = gemv_grouped(&i13->second, x16, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, uneven,
                                       mb.slot_of_pos, moe.top_k, /*tables_fresh=*/true)) {
                 return rc;
             }
@@ -141,13 +142,13 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             if (int rc = sort(8, false)) {
                 return rc;
             }
-            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, nullptr,
+            if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, uneven, nullptr,
                                       1, /*tables_fresh=*/true)) {
                 return rc;
             }
         }
         // silu(gate)*up is applied by the first grouped matmul (interleaved gate / up rows): no activation pass
-        if (int rc = gemv_grouped(&i2->second, mb.act, mb.c2, moe.hidden, mb, max_tiles, est_tiles, est_segments, mb.row_w, st)) {
+        if (int rc = gemv_grouped(&i2->second, mb.act, mb.c2, moe.hidden, mb, max_tiles, est_tiles, est_segments, mb.row_w, st, uneven)) {
             return rc;
         }
     } else {
