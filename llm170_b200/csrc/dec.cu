@@ -226,8 +226,8 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
         }
         a.tp = tp;
     }
-    // The row-group form (gemv_rg.cu) takes every call whose activations fit in shared memory beside its rings (t x K up to about 95000)
-    // unless a tuning key asks for another form, or the sums go on to other GPUs.  Single-linear calls of up to four tokens that the
+    // The row-group form (gemv_rg.cu) takes every call whose activations fit in shared memory beside its rings, but for the corners where
+    // another form is the sooner one (rg_leaves), unless a tuning key asks for another form, or the sums go on to other GPUs.  Single-linear calls of up to four tokens that the
     // row-block form takes stay with it (below): that entry point and its allocation-free twin are where the form of a call is pinned,
     // and replay to the same bits is what they are used for; the row-group form is 1.1 to 1.5 times as fast there, too, and
     // w4a16_lin_forward runs it.
@@ -238,6 +238,11 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
     auto choose_rowgroup = [&]() {
         const int forced = tune_gemv_rowgroup - 1;
         if (!rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg)) {
+            return false;
+        }
+        if (tune_gemv_rowgroup == 1 &&
+            rg_leaves(a, c.rg, sk_make_plan(a.k, a.group, t, c.grid_x, sm_count, tune_gemv_sk_stages, tune_gemv_sk_prefetch), sm_count)) {
+            c.grid_x = gemv_plan_ctas(a);       // the segments' first blocks, which the plan counted in its own units
             return false;
         }
         c.form = GemvChoice::ROWGROUP;
@@ -578,7 +583,8 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
         delete dec;
         return 1;
     }
-    if (d.ensure_scratch(1 << 20, 4096, d.stream)) {
+    // what any plan of the persistent form needs, so that none of its calls has to grow the scratch (which a capture may not)
+    if (d.ensure_scratch((size_t)2 * d.sm_count * 2 * w4::GEMV_MAX_M * 256, 4096, d.stream)) {
         g_create_error = d.err;
         delete dec;
         return 1;

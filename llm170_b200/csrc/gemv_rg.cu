@@ -249,6 +249,42 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
     return true;
 }
 
+// Three corners where the row-group form is not the best one.  All figures on B200, us per launch, this form / the other.
+//   * Long K: a warp walks its part of K serially (0.25 us per k-block of two row blocks), and where few units are left or x leaves room for
+//     two slots of two row blocks only, the persistent form, which deals K to all SMs, is sooner: 1024 x 28672 15.0 / 10.4, 1024 x 17408
+//     9.6 / 8.9, 5120 x 16384 at six tokens 24.0 / 18.1; the other way 4096 x 17408 13.2 / 15.0, 5120 x 17408 at four tokens 0.89 of it.
+//     Both times are estimated from the plans; over 2869 shapes of K >= 8192 the choice takes 0.4 % more than the best of both.
+//   * One or two tokens of a small linear in groups of 128: the 16-warp row-block kernel has all of its weights on the way at once, a step
+//     per 2048 channels, this one six k-blocks per warp: 512 x 6144 4.35 / 3.89, 512 x 4096 3.39 / 3.21, 512 x 5120 3.87 / 3.84, 512 x 3072
+//     2.87 / 3.12.  Fitted to 260 shapes of up to 4096 rows.
+//   * Hardly any K under many rows, five tokens and more: a unit's sums cost as much as its tiles.  128 channels, eight tokens: 16384 rows
+//     3.4 / 3.0, 34816 rows 4.0 / 3.2, 12288 rows 2.9 / 2.8; 256 channels, 34816 rows 4.8 / 4.3, 24576 rows 0.96.
+bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_count) {
+    const bool g32 = a.group == 32, two = p.smem <= RG_SMEM_TWO;
+    const int unit_k = a.group > TILE_K ? a.group : TILE_K, chain = (a.k / unit_k + p.kw - 1) / p.kw * (unit_k / TILE_K);
+    const int rounds = (p.units + p.ctas - 1) / p.ctas;
+    long long rows = 0;
+    for (int i = 0; i < a.nseg; ++i) {
+        rows += a.seg[i].n;
+    }
+    if (a.k >= 8192) {
+        static const double tau[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.437}}, {{0.44, 0.53, 0.64}, {0.49, 0.60, 0.742}}};
+        const double step = tau[two][g32][p.nr - 2] + (!two && p.depth == 2 ? (p.nr == 2 ? 0.085 : 0.04) : 0.0);
+        double us = 2.0 + rounds * (1.0 + step * chain);
+        if (rounds == 1 && 2 * p.units <= sm_count) {
+            us -= 0.95 + (g32 ? 0.0 : 0.012 * chain);        // no two CTAs on neighbouring SMs
+        }
+        return us > sk_estimate_us(sk, a.group, a.m, sm_count);
+    }
+    if (a.m <= 2 && rows <= 4096 && p.nr == 2 && p.kw == RG_WARPS && rounds == 1 && gemv_ru_fits(a, sm_count)) {
+        const double mb = 0.5e-6 * (double)rows * a.k, over = mb > 4.0 ? mb - 4.0 : 0.0;
+        const int steps = (a.k / 128 + 15) / 16;
+        const double ru = a.m == 1 ? 1.86 + 0.575 * steps + 0.092 * mb + 0.116 * over : 1.61 + 0.832 * steps + 0.088 * mb + 0.145 * over;
+        return 1.49 + 0.22 * chain + (2 * p.units > sm_count ? 0.33 : 0.0) + 0.058 * mb > ru;
+    }
+    return a.m >= 5 && rows * 8 > (long long)a.k * (a.m >= 7 ? 880 : 2667) * (g32 ? 2 : 1);
+}
+
 const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(group, p).name; }
 
 cudaError_t gemv_rg_init_device() {

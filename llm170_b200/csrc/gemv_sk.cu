@@ -101,6 +101,19 @@ SkPlan sk_make_plan(int k, int group, int m, int rows, int sm_count, int max_sta
     return p;
 }
 
+// Microseconds of a launch with K >= 8192, fitted with rg_leaves (gemv_rg.cu) to 2800 shapes on B200: units of a CTA, the CTAs that meet in a
+// row block, and for five tokens and more their one-CTA sum (with more than sixteen contributors it takes half of the launch).  A plan
+// of more CTAs than fit at once takes a second round.
+double sk_estimate_us(const SkPlan& p, int group, int m, int sm_count) {
+    const bool g128 = group == 128;
+    const double met = (double)p.units_per_row / p.nu_max;
+    if (p.ctas < 1 || p.ctas > 2 * sm_count || (m > 4 && met > 16.0)) {
+        return 1e9;
+    }
+    const double us = (g128 ? 5.6 : 5.0) + 0.2 * (m < 4 ? m : 4) + p.nu_max * ((g128 ? 0.87 : 1.23) + 0.03 * m) + met * (g128 ? 0.0245 : 0.030);
+    return us * (p.stages > 2 ? 1.0 : m > 4 ? 1.4 : 1.15) + (m > 4 ? 1.5 + 0.2 * met : 0.0);
+}
+
 size_t sk_part_floats(const SkPlan& p) {
     return (size_t)p.ctas * 2 * PART_FLOATS;
 }

@@ -140,6 +140,7 @@ struct SkPlan {
     int total;          // dynamic shared memory requested (at least 77 KB: never three CTAs on an SM)
 };
 SkPlan sk_make_plan(int k, int group, int m, int rows, int sm_count, int max_stages, int prefetch);
+double sk_estimate_us(const SkPlan& p, int group, int m, int sm_count);
 size_t sk_part_floats(const SkPlan& p);   // scratch for parked partial sums; counters: one per row block
 cudaError_t launch_gemv_sk(const GemvArgs& a, const SkPlan& p, cudaStream_t st);
 cudaError_t gemv_sk_init_device();
@@ -154,6 +155,8 @@ struct RgPlan {
     int smem;
 };
 bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& p);
+// Whether another form is estimated to finish the call sooner than this plan; `sk`: the persistent form's plan.
+bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_count);
 cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st);
 cudaError_t gemv_rg_init_device();
 const char* gemv_rg_name(int group, const RgPlan& p);

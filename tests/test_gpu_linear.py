@@ -627,3 +627,76 @@ def test_tuning_keys_reach_their_form(dec, orc, key, value, default, k, t, form)
     size = (x_dev(xs).float().abs() @ dec.dequant_lin("key").abs().T).max().item()
     assert (y.float() - tuned.float()).abs().max().item() <= bound * size
     dec.drop_lin("key")
+
+
+# The corners that the row-group form leaves to another one: long K under few rows, x that leaves room for two slots of two row blocks, one token
+# of a small linear, hardly any K under many rows -- and their neighbours on the other side of each line.
+CORNERS = [([1024], 28672, 128, 1, "gemv_sk"), ([512], 10240, 128, 1, "gemv_rg"), ([1024, 1024], 32768, 32, 2, "gemv_sk"), ([528, 16], 32768, 64, 3, "gemv_sk"),
+           ([5120], 16384, 128, 6, "gemv_sk"), ([5120], 14336, 128, 5, "gemv_rg"), ([5136], 16384, 32, 6, "gemv_sk"), ([304], 6144, 128, 1, "gemv_ru"),
+           ([304], 6144, 128, 2, "gemv_rg"), ([304], 3072, 128, 1, "gemv_rg"), ([304, 16], 6144, 128, 1, "gemv_rg"), ([304], 6144, 64, 1, "gemv_rg"),
+           ([16400], 128, 128, 8, "gemv_w4a16"), ([16400], 128, 128, 4, "gemv_rg"), ([8192, 8208], 128, 128, 7, "gemv_w4a16"), ([35008], 128, 32, 8, "gemv_w4a16")]
+
+
+@pytest.mark.parametrize("ns,k,group,t,form", CORNERS)
+def test_corners_the_row_group_form_leaves(dec, orc, ns, k, group, t, form):
+    xs = synth.make_acts(t, k, seed=970 + t)
+    x, names, wants, sizes = x_dev(xs), [], [], []
+    for i, n in enumerate(ns):
+        q, s = synth.make_linear(n, k, group, seed=971 + i)
+        dec.upload_lin_g(f"cor{i}", q, s, n, k, group)
+        names.append(f"cor{i}")
+        rows = (max(0, n - 300), n)
+        wants.append((rows, orc.linear_lane(q, s, xs, t, n, k, group, rows=rows)))
+        sizes.append((x.float().abs() @ dec.dequant_lin(names[-1]).abs().T).max().item())
+
+    def run(f16=False):
+        if len(ns) > 1:
+            return dec.sk_multi_dev(names, x, t=t, out_f16=f16)
+        guard = torch.full((t + 1, ns[0]), 7.0, device="cuda", dtype=torch.float16 if f16 else torch.float32)
+        dec.lin_forward(names[0], x, t, dst=guard[:t], out_f16=f16)
+        assert (guard[t:] == 7.0).all()
+        return [guard[:t].clone()]
+
+    ys = run()
+    assert dec.last_kernel().startswith(form), dec.last_kernel()
+    for y, y16, again, (rows, want), size in zip(ys, run(True), run(), wants, sizes):
+        assert torch.equal(y, again) and torch.equal(y16, y.half())
+        # f32 sums in another order, 2^-24 for each addition along a chain; what is added are nibbles of up to 15 and eights, together up to
+        # five times the weights' own sizes
+        assert np.abs(y.cpu().numpy()[:, rows[0]:rows[1]] - want[:, rows[0]:rows[1]]).max() <= 2.0 ** -18 * size
+    dec.set_tuning("gemv_rowgroup", 1 + 2 + 16 * 8)        # the row-group form, whatever the estimate
+    try:
+        for y, other, size in zip(ys, run(), sizes):
+            assert (y - other).abs().max().item() <= 2.0 ** -18 * size
+        assert dec.last_kernel().startswith("gemv_rg_kernel")
+    finally:
+        dec.set_tuning("gemv_rowgroup", 1)
+    if len(ns) == 1:
+        assert torch.equal(dec.sk_single_dev(names[0], x, t=t), dec.sk_single_static(names[0], x, t=t))
+    for nm in names:
+        dec.drop_lin(nm)
+
+
+def test_corner_calls_are_captured_without_a_call_before(orc):
+    # the persistent form needs scratch, which a capture may not make: a decoder comes with as much as any plan of one round takes
+    from llm170_b200.w4a16_dec import W4a16Dec
+    d = W4a16Dec(0)
+    n, k, t = 5120, 16384, 6
+    q, s = synth.make_linear(n, k, 128, seed=980)
+    d.upload_lin_g("cc", q, s, n, k, 128)
+    x = x_dev(synth.make_acts(t, k, seed=981))
+    y = torch.zeros((t, n), device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(d.stream_ptr())):
+        d.capture_begin()
+        d.lin_forward("cc", x, t, dst=y)
+        g = d.capture_end()
+    assert d.last_kernel().startswith("gemv_sk_kernel")
+    for _ in range(2):
+        y.zero_()
+        torch.cuda.synchronize()
+        d.graph_launch(g)
+        d.sync()
+        assert torch.equal(y, d.lin_forward("cc", x, t))
+    d.graph_destroy(g)
+    d.close()
