@@ -138,7 +138,7 @@ struct Dec {
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     void ts_query_clusters();
     TsChoice gemm_ts_choose(int n, int k, int t) const;
-    TsChoice gemm_ts2_choose(const Lin* l, int t) const;
+    TsChoice gemm_ts2_choose(const Lin* l, int t, int out_kind) const;
     int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, cudaStream_t st);
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
     int gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,

@@ -527,8 +527,9 @@ cudaError_t gemm_ts2_init_device() {
 // Tokens per tile with the least estimated time (microseconds, fitted to 700 measurements on B200: 140 shapes of 66..4096 tokens, 1024..34816
 // rows, K 512..17408, five tile widths each): 5.4 us per launch and 1.7 per further tile of a pair; a stage of 128 channels takes 0.00224 us per
 // token of the tile, the rate of the MMAs, but not less than the expansion (0.317 us, groups of 32: 0.445), and with all pairs busy, when
-// power holds the clock down, 0.082 + 0.00254 per token and at least 0.439 (0.470).
-TsChoice Dec::gemm_ts2_choose(const Lin* l, int t) const {
+// power holds the clock down, 0.082 + 0.00254 per token and at least 0.439 (0.470).  f32 results, stored from registers while the MMAs wait for
+// the accumulators, take another 0.0263 per token less 3.23 with each tile (202 measurements: 0.84..1.09 of them, nine tenths 0.94..1.06).
+TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind) const {
     TsChoice best{0, 1, 1e30};
     const int n_tiles = (l->n + P_ROWS - 1) / P_ROWS, stages = (l->k + SK - 1) / SK, pairs = sm_count / 2;
     for (int cap = P_TOK_MAX; cap >= 96; cap -= 32) {
@@ -538,7 +539,8 @@ TsChoice Dec::gemm_ts2_choose(const Lin* l, int t) const {
         const double full = std::min(1.0, std::max(0.0, ((double)tiles / (waves * pairs) - 0.41) / 0.52));
         const double light = std::max(l->group == 128 ? 0.317 : 0.445, 0.00224 * tok);
         const double heavy = std::max(l->group == 128 ? 0.439 : 0.470, 0.082 + 0.00254 * tok);
-        const double c = 5.4 + waves * (stages * (light + std::max(0.0, heavy - light) * full)) + (waves - 1) * 1.7;
+        const double f32 = out_kind == W4A16_OUT_F16 ? 0.0 : 0.0263 * tok - 3.23;
+        const double c = 5.4 + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * 1.7;
         if (c < best.cost) {
             best = TsChoice{tok, 1, c};
         }

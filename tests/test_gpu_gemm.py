@@ -516,3 +516,31 @@ def test_expansion_follows_the_scales(dec, tmp_path, path, odd, fma):
     dec.lin_forward("ef", torch.zeros((16, k), device="cuda", dtype=torch.float16), 16)
     assert dec.last_kernel().startswith("gemm_ts_kernel<128,fma>" if fma else "gemm_ts_kernel<128>"), dec.last_kernel()
     dec.drop_lin("ef")
+
+
+# Which form stock tuning takes for f16 and for f32 results, on both sides of each line: 64 and 65, 4096 and 4097 tokens, calls that the
+# weight-row form splits along K, token rows that a nearly empty and a nearly full last wave leave without a split.  Whatever the forms, the f16
+# results are the f32 results rounded.
+TC, TS, PAIR = "gemm_w4a16_tc_kernel", "gemm_ts_kernel", "gemm_ts2_kernel"
+
+
+@pytest.mark.parametrize("n,k,group,t,form16,form32", [
+    (34816, 1024, 128, 64, TS, TS), (34816, 1024, 128, 65, TS, TS), (12288, 2048, 128, 197, TS, TS), (7168, 5120, 128, 256, PAIR, TS),
+    (5120, 17408, 128, 300, TS, TS), (2144, 16384, 128, 526, TS, TS), (2048, 2048, 128, 1024, PAIR, TS), (7168, 5120, 128, 1500, PAIR, PAIR),
+    (7168, 5120, 32, 3000, PAIR, PAIR), (7168, 5120, 128, 4096, PAIR, PAIR), (5120, 6144, 128, 4096, PAIR, TC), (5120, 6144, 128, 4097, TC, TC),
+    (12288, 2048, 64, 2048, PAIR, TC), (8704, 5120, 32, 512, PAIR, TS)])
+def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form32):
+    q, s = synth.make_linear_cuda(n, k, group, 97, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("both", q, s, n, k, group)
+    x = x_dev(synth.make_acts(t, k, seed=98, scale=1 / np.sqrt(k)))
+    y32 = dec.lin_forward("both", x, t)
+    name32 = dec.last_kernel()
+    y16 = dec.lin_forward("both", x, t, out_f16=True)
+    name16 = dec.last_kernel()
+    dec.sync()
+    assert torch.equal(y16, y32.half())
+    assert name16.startswith(form16) and name32.startswith(form32), (name16, name32)
+    if n * k <= 1 << 24:
+        want = x.float() @ dec.dequant_lin("both", f16=True).float().T
+        assert (y32 - want).abs().max().item() <= 1e-4 * want.abs().max().item() + 1e-6
+    dec.drop_lin("both")
