@@ -256,7 +256,8 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
 //     Both times are estimated from the plans; over 2869 shapes of K >= 8192 the choice takes 0.4 % more than the best of both.
 //   * One or two tokens of a small linear in groups of 128: the 16-warp row-block kernel has all of its weights on the way at once, a step
 //     per 2048 channels, this one six k-blocks per warp: 512 x 6144 4.35 / 3.89, 512 x 4096 3.39 / 3.21, 512 x 5120 3.87 / 3.84, 512 x 3072
-//     2.87 / 3.12.  Fitted to 260 shapes of up to 4096 rows.
+//     2.87 / 3.12.  Fitted to 260 shapes of up to 4096 rows; less than a
+//     tenth of a microsecond is a tie.
 //   * Hardly any K under many rows, five tokens and more: a unit's sums cost as much as its tiles.  128 channels, eight tokens: 16384 rows
 //     3.4 / 3.0, 34816 rows 4.0 / 3.2, 12288 rows 2.9 / 2.8; 256 channels, 34816 rows 4.8 / 4.3, 24576 rows 0.96.
 bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_count) {
@@ -280,7 +281,7 @@ bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_coun
         const double mb = 0.5e-6 * (double)rows * a.k, over = mb > 4.0 ? mb - 4.0 : 0.0;
         const int steps = (a.k / 128 + 15) / 16;
         const double ru = a.m == 1 ? 1.86 + 0.575 * steps + 0.092 * mb + 0.116 * over : 1.61 + 0.832 * steps + 0.088 * mb + 0.145 * over;
-        return 1.49 + 0.22 * chain + (2 * p.units > sm_count ? 0.33 : 0.0) + 0.058 * mb > ru;
+        return 1.49 + 0.22 * chain + (2 * p.units > sm_count ? 0.33 : 0.0) + 0.058 * mb > ru + 0.1;
     }
     return a.m >= 5 && rows * 8 > (long long)a.k * (a.m >= 7 ? 880 : 2667) * (g32 ? 2 : 1);
 }
