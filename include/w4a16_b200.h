@@ -80,17 +80,33 @@ W4A16_API unsigned long long w4a16_launch_count(w4a16_dec* dec);
  * (crates/backend-gpu/src/rawcuda/gptq4.rs:60-70). Valid until the next forward call. */
 W4A16_API const char* w4a16_last_kernel(w4a16_dec* dec);
 /* Kernel-selection knobs, the analogue of the reference's LLM170_* environment flags
- * (crates/diag/src/flag.rs:3-27). Keys: "gemv_persistent" (which form of the decode GEMV runs: 1 = default,
- * two persistent CTAs per SM with equal ranges of work for up to 4 tokens and the (row block, K split) grid
- * above that; 2 = always persistent; 0 = never), "tp_wait_log2" (16..40, default 31: the fused all-reduce gives up
- * on its peers after 2^n cycles), "gemv_sk_stages" (2..6) and "gemv_sk_prefetch" (0..6): ring
- * stages of the persistent form and how many of them are requested before the previous kernel of the stream is
- * complete; "gemv_rowblock" (1 = default: up to four tokens of a 128-channel-group linear of at most 48 MB and K <= 6144 run on CTAs that own whole rows, without scratch or tickets -- a 16-warp kernel when all 32-row units are resident at once and x fits beside the weights in shared memory, else an 8-warp kernel up to tokens x K <= 11264 and the (row block, K split) form beyond; 2 = whatever the size; 0 = never), "gemv_rowblock_units" (1 = default; 0 = never the 16-warp kernel); the remaining gemv_* keys tune the (row block, K split) form: "gemv_ksplit" (0 = automatic),
- * "gemv_stages" (16 KB weight stages in flight per CTA, 2..8), "gemv_warps" (consumer warps per CTA, 8 or 16), "gemv_cluster" (1 = default: 2..8 K splits of a row
- * block run as a thread-block cluster and reduce through distributed shared memory),
- * "gemv_subnormal" (1 = default arithmetic, 0 = exact nibble-8 operands), "gemm_form" (above eight rows: 0 = automatic, 1 = token rows, 2 = weight rows as the MMA's rows), "gemm_bn" (weight rows per prefill GEMM tile: 0 = automatic, 128..256 in steps of 32), "gemm_ts_tok" (weight-row form, most tokens per tile: 0 = automatic, 64, 96, 128, 192, 256), "gemm_ts_ksplit" (weight-row form, K splits: 0 = automatic, 1..8), "gemm_mt" (128-token blocks per prefill GEMM tile: 0 = automatic, 1, 2), "gemm_ksplit" (K splits of the GEMM tiles: 0 = automatic -- all tiles when they are few, the tiles of an incomplete last wave otherwise; -1 = never; 1..16 = every tile), "gemm_tma_store" (1 = default: whole dense tiles leave through shared memory and TMA stores; 0 = per-lane stores), "debug_timeline" (0/1, see w4a16_debug_timeline), "pdl" (1 = default: kernels are
- * launched with programmatic stream serialization and prefetch weights while the previous kernel of
- * the stream drains; 2 = the next kernel may start as soon as this one is resident; 0 = ordinary launches). */
+ * (crates/diag/src/flag.rs:3-27). Keys of the decode GEMV; one that is not at its default moves a call to the form it tunes:
+ *   "gemv_rowgroup"  the row-group form: 1 = default, wherever x fits beside its rings and no other form is estimated to be
+ *       sooner; 0 = never; 1 + row blocks per warp (2..4) + 16 * warps along K (4, 8) = with that plan, whatever the estimate
+ *   "gemv_rowblock"  CTAs that own whole rows: 1 = default, up to four tokens of a 128-channel-group linear of at most 48 MB and
+ *       K <= 6144 through w4a16_sk_single_dev and w4a16_sk_single_static (a 16-warp kernel when all 32-row units are resident at
+ *       once and x fits beside the weights, else an 8-warp kernel up to tokens x K <= 11264), and small one- and two-token calls of
+ *       w4a16_lin_forward; 2 = whatever the size; 0 = never.  "gemv_rowblock_units" (1 = default; 0 = never the 16-warp kernel)
+ *   "gemv_persistent"  two persistent CTAs per SM with equal ranges of work: 1 = default, what the forms above leave of up to four
+ *       tokens or K >= 8192; 2 = always; 0 = never.  "gemv_sk_stages" (2..6, default 4) and "gemv_sk_prefetch" (0..6, default 2): its
+ *       ring stages and how many of them are requested before the previous kernel of the stream is complete
+ *   the (row block, K split) form takes the rest: "gemv_ksplit" (0 = automatic), "gemv_stages" (16 KB weight stages in flight per
+ *       CTA, 2..8, default 4), "gemv_warps" (consumer warps per CTA, 8 or 16), "gemv_cluster" (1 = default: 2..8 K splits of a row
+ *       block run as a thread-block cluster and reduce through distributed shared memory)
+ *   "gemv_subnormal" (1 = default arithmetic, 0 = exact nibble-8 operands), "moe_gemv" (MoE decode: 0 = automatic, 1 = the (row
+ *       block, K split) form, 2, 4 or 8 = the row-group form with that many warps along K), "tp_wait_log2" (16..40, default 31:
+ *       the fused all-reduce gives up on its peers after 2^n cycles)
+ * Keys of the GEMM above eight rows:
+ *   "gemm_form" (0 = automatic, 1 = token rows, 2 = weight rows as the MMA's rows), "gemm_pair" (CTA pairs: 0 = automatic, 1 =
+ *       never, 32..256 in steps of 32 = always, with tiles of that many tokens), "gemm_ts_tok" (weight rows, most tokens per tile:
+ *       0 = automatic, 64, 96, 128, 192, 256), "gemm_ts_ksplit" (weight rows, K splits: 0 = automatic, 1..8), "gemm_bn" (token
+ *       rows, weight rows per tile: 0 = automatic, 128..256 in steps of 32), "gemm_mt" (token rows, 128-token blocks per tile: 0 =
+ *       automatic, 1, 2), "gemm_ksplit" (token rows, K splits: 0 = automatic -- all tiles when they are few, the tiles of an
+ *       incomplete last wave otherwise; -1 = never; 1..16 = every tile), "gemm_tma_store" (token rows, 1 = default: whole dense
+ *       tiles leave through shared memory and TMA stores; 0 = per-lane stores)
+ * "debug_timeline" (0/1, see w4a16_debug_timeline), "pdl" (1 = default: kernels are launched with programmatic stream
+ * serialization and prefetch weights while the previous kernel of the stream drains; 2 = the next kernel may start as soon as
+ * this one is resident; 0 = ordinary launches). */
 W4A16_API int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value);
 
 /* ---- weights ----------------------------------------------------------------------------- */
@@ -203,7 +219,8 @@ W4A16_API int w4a16_head_unpack(w4a16_dec* dec, void* q_host, void* scale_host);
  * it agrees with the reference's f32 lane sum within 1e-5 of sum_k |q x| * scale (both are f32 sums in different orders). */
 W4A16_API int w4a16_head_forward(w4a16_dec* dec, const float* x32_dev, float* out_dev, int t, void* stream);
 /* W4a16Dec::sk_single_dev (crates/backend-gpu/src/rawcuda/w4a16_dec/kernels/decode.rs:89-127):
- * the decode GEMV on one linear, t in 1..8. */
+ * the decode GEMV on one linear, t in 1..8. A call replays to the same bits, also through w4a16_sk_single_static;
+ * w4a16_lin_forward may add the same f32 terms in another order (up to four tokens of 128-channel groups). */
 W4A16_API int w4a16_sk_single_dev(w4a16_dec* dec, const char* name, const void* x16_dev, void* out_dev, int t,
                         int out_kind, void* stream);
 /* W4a16Dec::sk_multi_dev (crates/backend-gpu/src/rawcuda/w4a16_dec/kernels/decode.rs:23-57): up to

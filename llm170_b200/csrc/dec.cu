@@ -227,10 +227,10 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
         a.tp = tp;
     }
     // The row-group form (gemv_rg.cu) takes every call whose activations fit in shared memory beside its rings, but for the corners where
-    // another form is the sooner one (rg_leaves), unless a tuning key asks for another form, or the sums go on to other GPUs.  Single-linear calls of up to four tokens that the
-    // row-block form takes stay with it (below): that entry point and its allocation-free twin are where the form of a call is pinned,
-    // and replay to the same bits is what they are used for; the row-group form is 1.1 to 1.5 times as fast there, too, and
-    // w4a16_lin_forward runs it.
+    // another form is the sooner one (rg_leaves), unless a tuning key asks for another form, or the sums go on to other GPUs.
+    // Single-linear calls of up to four tokens that the row-block form takes stay with it (below): that entry point and its allocation-free
+    // twin are where the form of a call is pinned, and replay to the same bits is what they are used for; w4a16_lin_forward runs the
+    // row-group form there, mostly 1.1 to 1.5 times as fast.
     const bool stock = tune_gemv_rowblock == 1 && tune_gemv_rowblock_units && tune_gemv_persistent == 1 && tune_gemv_cluster &&
                        tune_gemv_subnormal && tune_gemv_ksplit == 0 && tune_gemv_stages == GEMV_STAGES && tune_gemv_warps == GEMV_WARPS &&
                        tune_gemv_sk_stages == GEMV_SK_STAGES && tune_gemv_sk_prefetch == GEMV_SK_PREFETCH;

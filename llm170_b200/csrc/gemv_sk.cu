@@ -9,7 +9,8 @@
 // none on others, clusters confined to one GPC), and the next kernel of the stream cannot pass its
 // griddepcontrol.wait before the slowest CTA has left.  Here every SM slot gets one CTA of the same length.
 //
-// It takes what has no room in the row-group form (gemv_rg.cu), which multiplies with fewer instructions and needs no tickets.
+// It takes what has no room in the row-group form (gemv_rg.cu), which multiplies with fewer instructions and needs no tickets, and
+// long K that leaves that form a serial walk (rg_leaves).
 //
 // Same arithmetic as gemv.cu (mma.sync m16n8k16 with weight rows as the 16-row operand, raw nibbles as f16
 // subnormals, zero point through the per-group sum of x fed in as the MMA's C operand, f32 scales applied per

@@ -6,8 +6,8 @@
 //   SiLU(gate)*up -> grouped GEMM-2 over down, scaled by the routing weight -> sum over k.
 // Kernels here: top-k (crates/backend-gpu/src/rawcuda/assets/moe.cu:686-759), the expert histogram / offsets /
 // placement that replace the single-block counting sort (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:376-413,
-// crates/backend-gpu/src/rawcuda/assets/moe.cu:1599-1633), the row gather, the activation
-// (crates/backend-gpu/src/rawcuda/assets/moe.cu:1649-1660) and the top-k sum (:1662-1674).
+// crates/backend-gpu/src/rawcuda/assets/moe.cu:1599-1633), the row gather and the top-k sum
+// (crates/backend-gpu/src/rawcuda/assets/moe.cu:1662-1674); the activation (:1649-1660) is in the first matmul's epilogue.
 // Slots of one expert are placed with an atomic cursor, so their order inside an expert's segment is
 // not fixed; every output row is computed independently and the final sum runs over k in index order,
 // so results do not depend on that order.
@@ -219,7 +219,7 @@ __device__ __forceinline__ void scan_rows_tiles(int& vr, int& vt, int& total_row
 }
 
 // Decode-sized batches (at most 1024 (token, expert) slots): routing, histogram, offsets, tile table, placement
-// and sorted routing weights in ONE block of 1024 threads -- the six launches they take otherwise cost more
+// and sorted routing weights in ONE block of 1024 threads -- the launches they take otherwise cost more
 // than the expert matmuls of a single token.  Same tables as the separate kernels below.
 __global__ void __launch_bounds__(1024)
 moe_route_small_kernel(const float* lg, int* idx, float* wt,

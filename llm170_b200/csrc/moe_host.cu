@@ -156,7 +156,9 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         // to 16; above that 256-row token tiles.  128 experts, top-8, 2048 x 768, groups of 32, us per layer, weight-row / token
         // tiles: 200 tokens (12 rows per expert) 139 / 254, 1024 tokens 186 / 272, 2000 tokens 279 / 311, 3000 tokens (188 rows)
         // 386 / 374, 4096 tokens (256 rows) 510 / 493; 64 experts, top-6, 2048 x 1024: 2000 tokens (188 rows) 247 / 246, 3000 tokens
-        // (281 rows) 354 / 382, 4096 tokens 456 / 424.  Tiles of up to 64 rows: the same below 64 rows per expert, slower above.
+        // (281 rows) 354 / 382, 4096 tokens 456 / 424.  The line lies where the two met with a CTA per weight-row tile; with persistent
+        // CTAs they are within 8 % of each other, either way, from 188 to 281 rows.  Tiles of up to 64 rows: the same below 64 rows per
+        // expert, slower above.
         const bool weight_rows = (long long)ns < 192LL * moe.n_experts;
         const int bm = weight_rows ? 128 : 256;
         const int max_tiles = (ns + bm - 1) / bm + std::min(ns, n_local);
