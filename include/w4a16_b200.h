@@ -11,7 +11,8 @@
  *     (crates/backend-gpu/src/rawcuda/ffi.rs:18-40);
  *   - a decoder is bound to one device and is not thread-safe (the reference's W4a16Dec is Send
  *     but not Sync: crates/backend-gpu/src/rawcuda/w4a16_dec/mod.rs:626);
- *   - weights and scratch are owned by the decoder; activations and outputs by the caller;
+ *   - weights and scratch are owned by the decoder; activations and outputs by the caller.  The scratch (split-K sums and
+ *     tickets, the tables of a MoE call) is one set: calls that may overlap on the GPU belong on one stream;
  *   - forward calls launch asynchronously, allocate nothing once warmed, and may be captured in a
  *     CUDA graph (crates/backend-gpu/src/rawcuda/ctx/graph.rs:4-65).
  * Weight format at the boundary (compressed-tensors pack-quantized, crates/core/src/w4a16.rs:124-175):

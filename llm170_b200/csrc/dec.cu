@@ -240,7 +240,8 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
         if (!rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg)) {
             return false;
         }
-        if (tune_gemv_rowgroup == 1 &&
+        // (up to the tickets that a decoder and the array of the allocation-free entry come with)
+        if (tune_gemv_rowgroup == 1 && c.grid_x <= 4096 &&
             rg_leaves(a, c.rg, sk_make_plan(a.k, a.group, t, c.grid_x, sm_count, tune_gemv_sk_stages, tune_gemv_sk_prefetch), sm_count)) {
             c.grid_x = gemv_plan_ctas(a);       // the segments' first blocks, which the plan counted in its own units
             return false;
