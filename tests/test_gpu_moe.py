@@ -268,3 +268,39 @@ def test_plan_of_a_rank_that_is_hardly_reached(dec, orc, n_exp, k, f, h):
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, 32)
     err = np.abs(total - want).max()
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())
+
+
+# the second matmul in the (row block, K split) form behind a first one in the row-group form: behind CTAs that end evenly (programmatic start) and
+# unevenly (ordinary start), eagerly and out of a graph that replays the layer over new rows
+@pytest.mark.parametrize("t,f,h,group", [(1, 12288, 64, 64), (4, 12288, 64, 32), (3, 12800, 128, 128)])
+def test_second_matmul_in_the_other_form(dec, orc, t, f, h, group):
+    n_exp, k = 4, 2
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=61)
+    dec.set_moe(n_exp, k, f, h, group)
+    dec.upload_experts(0, w13_q, w13_s, w2_q, w2_s)
+    x, lg = synth.make_acts(t, h, seed=62 + t), synth.make_router_logits(t, n_exp, seed=63 + t)
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+    assert dec.last_kernel().startswith("gemv_w4a16_kernel")
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
+    err = np.abs(y.cpu().numpy() - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())
+    out = torch.zeros_like(y)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(dec.stream_ptr())):
+        dec.capture_begin()
+        for _ in range(3):
+            dec.moe_ffn_dev_t(0, lgd, xd, t, out=out)
+        g = dec.capture_end()
+    for seed in range(3):
+        xd.copy_(torch.from_numpy(synth.make_acts(t, h, seed=70 + seed).view(np.float16).copy()))
+        torch.cuda.synchronize()
+        dec.graph_launch(g)
+        dec.sync()
+        assert torch.equal(out, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        dec.set_tuning("pdl", 0)
+        try:
+            assert torch.equal(out, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        finally:
+            dec.set_tuning("pdl", 1)
+    dec.graph_destroy(g)
