@@ -114,7 +114,9 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
                     bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)row * a.k, (uint32_t)(a.k * 2), smem_u32(&s_xbar));
                 }
             }
-            mbar_wait(smem_u32(&s_xbar), xphase, &s_abort, a.status, (42 << 16) | (seg & 0xffff));
+            if (!mbar_wait(smem_u32(&s_xbar), xphase, &s_abort, a.status, (42 << 16) | (seg & 0xffff))) {
+                mbar_drain(smem_u32(&s_xbar), xphase);
+            }
             xphase ^= 1;
             __syncwarp();
             // lanes without a token read token 0: their columns are never stored

@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
             bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k, (uint32_t)(a.k * 2), smem_u32(&s_xbar));
         }
     }
-    mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16));
+    if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
+        mbar_drain(smem_u32(&s_xbar), 0);
+    }
     __syncwarp();
     stamp_now(2);   // x staged
     stamp_now(3);

@@ -59,6 +59,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     return true;
 }
 
+// After a wait that ran out: a quarter as long again for the copies that the barrier counts, which would otherwise land in shared memory that
+// the block has given back.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity) && clock64() - t0 <= (1ll << 29)) {
+    }
+}
+
 // 1-D bulk copy global -> shared, completion counted in bytes on an mbarrier.
 // Both addresses 16-byte aligned, size a multiple of 16.
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
