@@ -99,19 +99,20 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
 
 template <int GROUP, bool FMA>
 __global__ void __launch_bounds__(TS_THREADS, 2)
-gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
+gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
 
     constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    constexpr uint32_t RAW_STAGE = RAW_BYTES + ts_scale_bytes(GROUP);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be warp-uniform
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
     unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
     const int NR = a.raw_stages, NX = a.x_stages, NA = a.a_stages;
     const int N = a.tok;
     const uint32_t x_half = (uint32_t)N * (BK * 2);                  // one k-block of the token tile
-    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_BYTES; };
+    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_STAGE; };
     auto x_addr = [&](int s) { return base + (uint32_t)a.off_x + (uint32_t)s * (2 * x_half); };
     const uint32_t bars = base + (uint32_t)a.off_bars;
     auto raw_full = [&](int s) { return bars + 8u * s; };
@@ -137,7 +138,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
     auto stage_kbs = [&](int it) { return min(2, nkb_all - 2 * (st0 + it)); };
     auto issue_raw = [&](int it, int s) {
         const int kbs = stage_kbs(it);
-        mbar_expect_tx(raw_full(s), kbs * kb_bytes);
+        mbar_expect_tx(raw_full(s), kbs * kb_bytes + ts_scale_bytes(GROUP));         // (scales past the end: zeros)
+        tma_load_2d(raw_addr(s) + RAW_BYTES, &tmap_s, (st0 + it) * GPS * 8, rb0, raw_full(s));
         const uint32_t* src = a.qt + ((size_t)(2 * (st0 + it)) * a.nrb_w + rb0) * TILE_WORDS;
         bulk_load(raw_addr(s), src, kb_bytes, raw_full(s));
         if (kbs == 2) {
@@ -276,27 +278,9 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
         const int rb = quad * 2 + half;
         const bool live = rb < nrbv;
         const int rbl = live ? rb : 0;
-        const int ng = a.k / GROUP;
-        // Scale words (rows g, g + 8) of this row block: one coalesced 128-byte load brings four groups (lane 8i + g: group
-        // i), handed out by shuffles.  SCQ loads are in flight, so that a word is requested SCQ stages (32-channel groups)
-        // or 4 * SCQ stages before its use.
-        constexpr int SCQ = 4;
-        const uint32_t* sp = a.st + ((size_t)(rb0 + rbl) * ng + (size_t)st0 * GPS) * 8 + lane;
-        int sleft = (ng - st0 * GPS) * 8 - lane;                     // words left in the row block
-        auto load_scales = [&]() {
-            const uint32_t v = sleft > 0 ? __ldg(sp) : 0u;
-            sp += 32;
-            sleft -= 32;
-            return v;
-        };
-        uint32_t scq[SCQ];
-#pragma unroll
-        for (int i = 0; i < SCQ; ++i) {
-            scq[i] = load_scales();
-        }
-        uint32_t sc_cur = 0;
         const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
         const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+        const uint32_t s_ld = base + (uint32_t)(RAW_BYTES + rbl * (GPS * 32)) + (uint32_t)(lane >> 2) * 4u;   // scale pairs of the lane's rows
         int sr = 0, pr = 0, sa = 0, pa = 1;
         for (int it = 0; it < nst; ++it) {
             // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
@@ -304,21 +288,13 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
                 ok = false;
                 break;
             }
-            const uint32_t ra = r_ld + (uint32_t)sr * RAW_BYTES;
+            const uint32_t ra = r_ld + (uint32_t)sr * RAW_STAGE;
             const uint4 raw0 = lds128(ra);
             const uint4 raw1 = lds128(ra + RAW_BYTES / 2);           // stale bytes when the stage holds one k-block
-            if (((it * GPS) & 3) == 0) {
-                sc_cur = scq[0];
-#pragma unroll
-                for (int i = 0; i + 1 < SCQ; ++i) {
-                    scq[i] = scq[i + 1];
-                }
-                scq[SCQ - 1] = load_scales();
-            }
             uint32_t sc[GPS];
 #pragma unroll
             for (int i = 0; i < GPS; ++i) {
-                sc[i] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + i) & 3) * 8 + (lane >> 2));
+                sc[i] = lds32(s_ld + (uint32_t)sr * RAW_STAGE + (uint32_t)i * 32u);
             }
             uint32_t v[16];
             const TsScale<FMA> sc0(sc[0], a.fma_add, a.fma_mul), sc1(sc[GPS > 1 ? 1 : 0], a.fma_add, a.fma_mul);
@@ -476,11 +452,12 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
 // 141 us, 1024 tokens 209 -> 186.)
 template <int GROUP>
 __global__ void __launch_bounds__(TS_THREADS, 2)
-gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs a) {
+gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
     constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    constexpr uint32_t RAW_STAGE = RAW_BYTES + ts_scale_bytes(GROUP);
     if (a.tables_fresh) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
@@ -489,7 +466,7 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
     unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
     const int NR = a.raw_stages, NX = a.x_stages, NA = a.a_stages;
     const uint32_t x_half = (uint32_t)a.tok * (BK * 2);
-    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_BYTES; };
+    auto raw_addr = [&](int s) { return base + (uint32_t)s * RAW_STAGE; };
     auto x_addr = [&](int s) { return base + (uint32_t)a.off_x + (uint32_t)s * (2 * x_half); };
     const uint32_t bars = base + (uint32_t)a.off_bars;
     auto raw_full = [&](int s) { return bars + 8u * s; };
@@ -599,7 +576,8 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
                 }
                 if (leader) {
                     const int kbs = min(2, nkb - 2 * it);
-                    mbar_expect_tx(raw_full(sr), kbs * kb_bytes);
+                    mbar_expect_tx(raw_full(sr), kbs * kb_bytes + ts_scale_bytes(GROUP));
+                    tma_load_2d(raw_addr(sr) + RAW_BYTES, &tmap_s, it * GPS * 8, tl.rb0, raw_full(sr));
                     const uint32_t* src = a.qt + ((size_t)(2 * it) * a.nrb_w + tl.rb0) * TILE_WORDS;
                     bulk_load(raw_addr(sr), src, kb_bytes, raw_full(sr));
                     if (kbs == 2) {
@@ -671,38 +649,17 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
         // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM; then convert and store
         const int quad = warp & 3, half = (warp - 2) >> 2;
         const int rb = quad * 2 + half;                              // a warp may touch the TMEM lanes 32 * (warp % 4) .. +31
-        const int ng = a.k / GROUP;
         const int lrow = quad * 32 + lane;
         const int et = (int)threadIdx.x - 64;                        // thread among the converting warps
         const bool glu = a.glu != 0;
         const int per_tok = glu ? TS_MROWS : TS_MROWS * 2, n_out = glu ? a.n / 2 : a.n;      // bytes; values per row of the result
         unsigned char* stage_ptr = base_ptr + a.off_stage;
-        constexpr int SCQ = 4;                                       // scale loads in flight, as in the dense kernel
-        const uint32_t* sp = nullptr;
-        int sleft = 0;
-        uint32_t scq[SCQ];
-        auto load_scales = [&]() {
-            const uint32_t v = sleft > 0 ? __ldg(sp) : 0u;
-            sp += 32;
-            sleft -= 32;
-            return v;
-        };
-        auto open_scales = [&](const Tile& tl) {
-            sp = a.st + (size_t)(tl.rb0 + (rb < tl.nrbv ? rb : 0)) * ng * 8 + lane;
-            sleft = ng * 8 - lane;
-#pragma unroll
-            for (int i = 0; i < SCQ; ++i) {
-                scq[i] = load_scales();
-            }
-        };
-        uint32_t sc_cur = 0;
         const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
         int sr = 0, sa = 0;
         uint32_t pr = 0, pa = 1, cnt = 0, done = 0;
         Tile tl{}, next{};
         if ((int)blockIdx.x < tiles) {
             next = tile_at(blockIdx.x);
-            open_scales(next);
         }
         for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++done) {
             tl = next;
@@ -710,27 +667,21 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
             if (more) {
                 next = tile_at(i + (int)gridDim.x);
             }
-            const uint32_t r_ld = base + (uint32_t)(rb < tl.nrbv ? rb : 0) * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+            const int rbl = rb < tl.nrbv ? rb : 0;
+            const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+            const uint32_t s_ld = base + (uint32_t)(RAW_BYTES + rbl * (GPS * 32)) + (uint32_t)(lane >> 2) * 4u;
             for (int it = 0; it < nst && ok; ++it, ++cnt) {
                 if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (56 << 16) | it))) {
                     ok = false;
                     break;
                 }
-                const uint32_t ra = r_ld + (uint32_t)sr * RAW_BYTES;
+                const uint32_t ra = r_ld + (uint32_t)sr * RAW_STAGE;
                 const uint4 raw0 = lds128(ra);
                 const uint4 raw1 = lds128(ra + RAW_BYTES / 2);       // stale bytes when the stage holds one k-block
-                if (((it * GPS) & 3) == 0) {
-                    sc_cur = scq[0];
-#pragma unroll
-                    for (int q = 0; q + 1 < SCQ; ++q) {
-                        scq[q] = scq[q + 1];
-                    }
-                    scq[SCQ - 1] = load_scales();
-                }
                 uint32_t sc[GPS];
 #pragma unroll
                 for (int q = 0; q < GPS; ++q) {
-                    sc[q] = __shfl_sync(0xffffffffu, sc_cur, ((it * GPS + q) & 3) * 8 + (lane >> 2));
+                    sc[q] = lds32(s_ld + (uint32_t)sr * RAW_STAGE + (uint32_t)q * 32u);
                 }
                 uint32_t v[16];
                 ts_expand<false>(raw0, TsScale<false>(sc[0], 0, 0), TsScale<false>(sc[GPS > 1 ? 1 : 0], 0, 0), v);
@@ -761,9 +712,6 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
                     sa = 0;
                     pa ^= 1;
                 }
-            }
-            if (more) {
-                open_scales(next);                                   // on the way while this tile is converted
             }
             ok = ok && mbar_wait(accum_bar, done & 1, abort_flag, a.status, (58 << 16));
             ok = __all_sync(0xffffffffu, ok);
@@ -833,8 +781,11 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const TsArgs 
 }  // namespace
 
 
-static size_t ts_smem(int tok, int nr, int nx, int na, int* off_x, int* off_bars) {
-    size_t off = (size_t)nr * RAW_BYTES;                      // multiples of 1024
+// bytes of `nr` raw stages; what follows is 1024-byte aligned
+static size_t ts_raw_bytes(int group, int nr) { return ((size_t)nr * (RAW_BYTES + ts_scale_bytes(group)) + 1023) & ~(size_t)1023; }
+
+static size_t ts_smem(int group, int tok, int nr, int nx, int na, int* off_x, int* off_bars) {
+    size_t off = ts_raw_bytes(group, nr);
     *off_x = (int)off;
     off += (size_t)nx * tok * SK * 2;
     const size_t red = (size_t)std::min(RED_TOK, tok) * TS_MROWS * 4;   // the cluster's sum reuses the rings
@@ -860,20 +811,20 @@ struct TsPlan {
     int tmem_cols, na, nr, nx, off_x, off_bars;
     size_t smem;
 };
-TsPlan ts_plan(int tok) {
+TsPlan ts_plan(int group, int tok) {
     TsPlan p{};
     // TMEM: the accumulator and as many expanded stages as fit in half of it (two CTAs per SM), else in all of it
     p.tmem_cols = tok <= 128 ? 256 : 512;
     p.na = std::min((p.tmem_cols - tok) / A_COLS, 4);
     const size_t limit = p.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
-    p.nx = p.nr = 2;
-    while (p.nr < 12 && ts_smem(tok, p.nr + 1, p.nx, p.na, &p.off_x, &p.off_bars) <= limit) {
+    p.nx = p.nr = ts_smem(group, tok, 3, 3, p.na, &p.off_x, &p.off_bars) <= limit ? 3 : 2;
+    while (p.nr < 12 && ts_smem(group, tok, p.nr + 1, p.nx, p.na, &p.off_x, &p.off_bars) <= limit) {
         ++p.nr;
-        if (p.nr % 2 == 0 && p.nx < 4 && ts_smem(tok, p.nr, p.nx + 1, p.na, &p.off_x, &p.off_bars) <= limit) {
+        if (p.nr % 2 == 0 && p.nx < 4 && ts_smem(group, tok, p.nr, p.nx + 1, p.na, &p.off_x, &p.off_bars) <= limit) {
             ++p.nx;
         }
     }
-    p.smem = std::max(ts_smem(tok, p.nr, p.nx, p.na, &p.off_x, &p.off_bars), p.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
+    p.smem = std::max(ts_smem(group, tok, p.nr, p.nx, p.na, &p.off_x, &p.off_bars), p.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
     return p;
 }
 }  // namespace
@@ -956,7 +907,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
     }
-    const TsPlan p = ts_plan(c.tok);
+    const TsPlan p = ts_plan(l->group, c.tok);
     TsArgs a{};
     a.tok = c.tok;
     a.ksplit = c.ks;
@@ -976,6 +927,10 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(x), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUtensorMap smap;
+    if (cr == CUDA_SUCCESS) {
+        cr = ts_scale_map(enc, &smap, l->st, l->n, l->k, l->group);
+    }
     if (cr != CUDA_SUCCESS) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled failed (%d)", (int)cr);
     }
@@ -1013,9 +968,9 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     cfg.numAttrs = n_attr;
     cudaError_t e;
     if (l->group != 128) {
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, a);
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, smap, a);
     } else if (l->fma_e < 0) {
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, a);
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, smap, a);
     } else {
         // one f16 operation per pair of weights where two do it otherwise, in the expansion that a small batch waits for (27 x 34816 x
         // 5120: 29.8 -> 26.5 us, 27 x 5120 x 17408: 21.3 -> 19.3); the weights come out 2^-E smaller
@@ -1023,7 +978,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
         memcpy(&a.fma_mul, &mul, sizeof(mul));
         a.fma_add = ((uint32_t)(20 - l->fma_e) << 26) + ((uint32_t)(24 - l->fma_e) << 10);
         a.out_mul = ldexpf(l->out_mul, l->fma_e);
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, a);
+        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, smap, a);
     }
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
@@ -1046,7 +1001,7 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     const int tmem_cols = 256, na = std::min((tmem_cols - tok) / A_COLS, 4), nx = tok <= 64 ? 3 : 2;
     TsArgs a{};
     int nr = 2;
-    auto bars_at = [&](int raw) { return raw * RAW_BYTES + nx * tok * SK * 2 + TS_STAGE_BYTES; };
+    auto bars_at = [&](int raw) { return (int)ts_raw_bytes(l->group, raw) + nx * tok * SK * 2 + TS_STAGE_BYTES; };
     auto smem_of = [&](int raw) { return (size_t)bars_at(raw) + (size_t)(2 * raw + 2 * nx + 2 * na + 2) * 8 + 1024; };
     while (nr < 8 && smem_of(nr + 1) <= TS_SMEM_HALF_MAX) {
         ++nr;
@@ -1059,7 +1014,7 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     a.a_stages = na;
     a.raw_stages = nr;
     a.x_stages = nx;
-    a.off_x = nr * RAW_BYTES;
+    a.off_x = (int)ts_raw_bytes(l->group, nr);
     a.off_stage = a.off_x + nx * tok * SK * 2;
     a.off_bars = bars_at(nr);
     CUtensorMap map;
@@ -1070,6 +1025,10 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     CUresult cr = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUtensorMap smap;
+    if (cr == CUDA_SUCCESS) {
+        cr = ts_scale_map(enc, &smap, l->st, l->n, l->k, l->group);
+    }
     if (cr != CUDA_SUCCESS) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled failed (%d)", (int)cr);
     }
@@ -1104,8 +1063,8 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    const cudaError_t e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<128>, map, a)
-                                          : cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<32>, map, a);
+    const cudaError_t e = l->group == 128 ? cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<128>, map, smap, a)
+                                          : cudaLaunchKernelEx(&cfg, gemm_ts_grouped_kernel<32>, map, smap, a);
     if (e != cudaSuccess) {
         return cuda_fail("launch grouped gemm", e);
     }

@@ -14,6 +14,21 @@ constexpr int SK = 2 * BK;                      // channels per stage: two k-blo
 constexpr int RAW_BYTES = TS_MROWS * SK / 2;    // 8 KB per stage
 constexpr int A_COLS = SK / 2;                  // TMEM columns of one expanded stage (two f16 per column)
 constexpr int DQ_WARPS = TS_MROWS / TILE_ROWS;  // a warp per 16-row block
+// Scales of a raw stage, behind its weights: [row block][group][8] words, one TMA box.  Read by the lanes from global memory instead, four
+// loads ahead, they held up every stage: the wait for the stores to TMEM took those reads along.  us per launch before / now: 27 tokens of
+// 34816 x 5120 29.2 / 27.2, of 5120 x 17408 19.7 / 18.7; groups of 32: 27 tokens 33.8 / 31.0, 197 tokens of 34816 x 5120 64.8 / 56.6.
+__host__ __device__ constexpr int ts_scale_bytes(int group) { return DQ_WARPS * (SK / group) * 32; }
+
+// Scale words [16-row blocks][groups][8] of a matrix: boxes of a stage's groups by the row blocks of a CTA.
+inline CUresult ts_scale_map(EncodeTiledFn enc, CUtensorMap* map, void* st, int n, int k, int group) {
+    const int ng = k / group;
+    const cuuint64_t dims[2] = {(cuuint64_t)ng * 8, (cuuint64_t)(n / TILE_ROWS)};
+    const cuuint64_t strides[1] = {(cuuint64_t)ng * 32};
+    const cuuint32_t box[2] = {(cuuint32_t)(SK / group * 8), (cuuint32_t)DQ_WARPS};
+    const cuuint32_t estr[2] = {1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, st, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
 
 // 16 TMEM lanes x 32 columns from one warp: register 4i + {0,1} of lane (g, t) -> row g, columns 8i + 2t + {0,1};
 // register 4i + {2,3} -> row g + 8
