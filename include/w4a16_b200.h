@@ -95,8 +95,9 @@ W4A16_API const char* w4a16_last_kernel(w4a16_dec* dec);
  *       CTA, 2..8, default 4), "gemv_warps" (consumer warps per CTA, 8 or 16), "gemv_cluster" (1 = default: 2..8 K splits of a row
  *       block run as a thread-block cluster and reduce through distributed shared memory)
  *   "gemv_subnormal" (1 = default arithmetic, 0 = exact nibble-8 operands), "moe_gemv" (MoE decode: 0 = automatic, 1 = the (row
- *       block, K split) form, 2, 4 or 8 = the row-group form with that many warps along K), "tp_wait_log2" (16..40, default 31:
- *       the fused all-reduce gives up on its peers after 2^n cycles)
+ *       block, K split) form, 2, 4 or 8 = the row-group form with that many warps along K), "moe_gemm" (MoE prefill: 0 = automatic,
+ *       1 = weight rows, 2 = token rows, 128, 192 or 256 = CTA pairs with tiles of at most that many rows), "tp_wait_log2" (16..40,
+ *       default 31: the fused all-reduce gives up on its peers after 2^n cycles)
  * Keys of the GEMM above eight rows:
  *   "gemm_form" (0 = automatic, 1 = token rows, 2 = weight rows as the MMA's rows), "gemm_pair" (CTA pairs: 0 = automatic, 1 =
  *       never, 32..256 in steps of 32 = always, with tiles of that many tokens), "gemm_ts_tok" (weight rows, most tokens per tile:

@@ -746,6 +746,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         d.tune_gemv_stages = value;
         return 0;
     }
+    if (!strcmp(key, "moe_gemm")) {
+        if ((value < 0 || value > 2) && value != 128 && value != 192 && value != 256) {
+            return d.fail("w4a16 set_tuning: moe_gemm=%d (0, 1, 2, 128, 192 or 256)", value);
+        }
+        d.tune_moe_gemm = value;
+        return 0;
+    }
     if (!strcmp(key, "gemm_pair")) {
         if (value != 0 && value != 1 && (value < 32 || value > 256 || value % 32 != 0)) {
             return d.fail("w4a16 set_tuning: gemm_pair=%d (0, 1 or a multiple of 32 up to 256)", value);

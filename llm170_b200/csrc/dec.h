@@ -108,6 +108,7 @@ struct Dec {
     int tune_gemm_ksplit = 0;    // K splits of the GEMM: 0 = automatic (only when the tiles do not fill the SMs)
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
     int tune_gemm_pair = 0;      // CTA pairs (gemm_ts2.cu): 0 = automatic, 1 = never, 32..256 = always, with tiles of that many tokens
+    int tune_moe_gemm = 0;       // MoE prefill: 0 = automatic, 1 = weight rows, 2 = token rows, 128 / 192 / 256 = pairs, tiles of at most that many rows
     int tune_gemm_form = 0;      // above the decode rows: 0 = automatic, 1 = token rows (gemm_tc.cu), 2 = weight rows (gemm_ts.cu)
     int tune_gemm_bn = 0;        // gemm_tc.cu: weight rows per tile (128..256, a multiple of 32), 0 = automatic
     int tune_ts_tok = 0;         // gemm_ts.cu: most tokens per tile (64, 96, 128, 192, 256), 0 = automatic
@@ -143,6 +144,8 @@ struct Dec {
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
     int gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
                         int tok, const float* row_w, cudaStream_t st, bool tables_fresh);
+    int gemm_ts2_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
+                         int bm, const float* row_w, cudaStream_t st, bool tables_fresh);
     int gemm_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b,
                      int max_tiles, const float* row_w, cudaStream_t st);
     // row-parallel tensor parallelism (fused all-reduce in the GEMV): local exchange block + peer mappings
@@ -156,6 +159,11 @@ struct Dec {
     MoeCfg moe;
     MoeBufs mb;
     int ensure_moe(int t, cudaStream_t st);
+    struct MoeTiles {
+        enum Form { PAIRS, WEIGHT_ROWS, TOKEN_ROWS } form;
+        int rows;
+    };
+    MoeTiles moe_tiles(int ns) const;
     void free_moe(bool retire = false);
     int moe_ffn(int layer, const float* logits, const void* x16, void* y, int t, int out_kind, cudaStream_t st);
 };

@@ -188,14 +188,15 @@ cudaError_t head_init_device();
 
 // ---- moe.cu ----------------------------------------------------------------------------------
 struct MoeBufs;
+enum { TILES_FULL = 0, TILES_EVEN = 1, TILES_SORTED = 2 };
 // All return the first launch error and launch nothing after it.  `pdl`: programmatic stream serialization.  `cnt` (optional): counts the
 // rows of local experts [e0, e1) as well.  `launched`: raised by the number of launches.
 cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl, cudaStream_t st);
-// routing and sorting of any batch: top-k and histogram -> offsets and m-tile table (tiles of `bm` rows; `even`: of equal shares of at
-// most bm rows) -> placement of the local experts' slots and gather of their token rows.  Wants b.cnt at zero and leaves it so; after an
+// routing and sorting of any batch: top-k and histogram -> offsets and m-tile table (tiles of at most `bm` rows, cut as `shares` says) ->
+// placement of the local experts' slots and gather of their token rows.  Wants b.cnt at zero and leaves it so; after an
 // error it may hold counts.
 cudaError_t launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
-                            int even, int pdl, cudaStream_t st, unsigned long long& launched);
+                            int shares, int pdl, cudaStream_t st, unsigned long long& launched);
 // the same tables for at most 1024 slots, from one block, without the gather
 cudaError_t launch_moe_route_small(const float* logits, const MoeBufs& b, int t, int n_exp, int k, int e0, int e1, int bm, int pdl,
                                    cudaStream_t st, unsigned long long& launched);

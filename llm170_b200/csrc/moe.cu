@@ -281,26 +281,46 @@ moe_route_small_kernel(const float* lg, int* idx, float* wt,
     }
 }
 
+// How an expert's rows are cut into tiles: of bm rows with a remainder, in equal shares of at most bm (multiples of 16), or like the first
+// but with the table sorted.  Persistent CTAs take tiles in turn: sorted, no CTA gets more of the large ones than another.
 // One block of 1024 threads (n_exp <= 1024): exclusive offsets of the local experts' segments and the m-tile
 // table of the grouped GEMM, tile i -> (expert, first sorted row, valid rows).  Also clears the placement cursors and the counts.
 __global__ void __launch_bounds__(1024)
 moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_row0, int* tile_rows, int* n_tiles, int* n_rows,
-                   int n_exp, int e0, int e1, int bm, int even) {
+                   int n_exp, int e0, int e1, int bm, int shares) {
     __shared__ int s_r[32], s_t[32];
+    __shared__ __align__(16) int s_rest[1024];
     const int e = threadIdx.x;
     pdl_begin();
     const int c = (e >= e0 && e < e1) ? cnt[e] : 0;
-    const int step = tile_step(c, bm, even);
-    const int ct = (c + step - 1) / step;
+    const int step = tile_step(c, bm, shares == TILES_EVEN), rest = shares == TILES_SORTED ? c % bm : 0;
+    const int ct = shares == TILES_SORTED ? c / bm : (c + step - 1) / step;
     int vr = c, vt = ct, total_rows, total_tiles;
     scan_rows_tiles(vr, vt, total_rows, total_tiles, s_r, s_t);
     const int row0 = vr - c, tile0 = vt - ct;
+    if (shares == TILES_SORTED) {
+        // whole tiles first, then what is left of each expert, the largest first
+        s_rest[e] = rest;
+        const int rests = __syncthreads_count(rest > 0);
+        if (rest > 0) {
+            int rank = 0;
+            for (int o = 0; o < n_exp; o += 4) {                     // (nothing is left of experts past the last)
+                const int4 r4 = *reinterpret_cast<const int4*>(s_rest + o);
+                rank += (r4.x > rest || (r4.x == rest && o < e)) + (r4.y > rest || (r4.y == rest && o + 1 < e)) +
+                        (r4.z > rest || (r4.z == rest && o + 2 < e)) + (r4.w > rest || (r4.w == rest && o + 3 < e));
+            }
+            tile_expert[total_tiles + rank] = e;
+            tile_row0[total_tiles + rank] = row0 + c - rest;
+            tile_rows[total_tiles + rank] = rest;
+        }
+        total_tiles += rests;
+    }
     if (e < n_exp) {
         off[e] = row0;
         cursor[e] = 0;
         cnt[e] = 0;
     }
-    for (int r = 0, i = tile0; r < c; r += step, ++i) {
+    for (int r = 0, i = tile0; r < c - rest; r += step, ++i) {
         tile_expert[i] = e;
         tile_row0[i] = row0 + r;
         tile_rows[i] = min(step, c - r);
@@ -450,14 +470,14 @@ cudaError_t launch_moe_route_small(const float* logits, const MoeBufs& b, int t,
 }
 
 cudaError_t launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
-                            int even, int pdl, cudaStream_t st, unsigned long long& launched) {
+                            int shares, int pdl, cudaStream_t st, unsigned long long& launched) {
     cudaError_t e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
     if (e != cudaSuccess) {
         return e;
     }
     ++launched;
     e = launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
-               n_exp, e0, e1, bm, even);
+               n_exp, e0, e1, bm, shares);
     if (e != cudaSuccess) {
         return e;
     }

@@ -86,6 +86,48 @@ int Dec::ensure_moe(int t, cudaStream_t st) {
     return 0;
 }
 
+// Form and largest tile of MoE prefill, `ns` rows in all.  us per layer, weight rows / pairs of at most 128 / 192 / 256 rows, of 60 shapes:
+//   128 experts, top-8, 2048 x 768, groups of 32: 130 tokens (8 rows per expert) 123 / 117 / 132 / 121, 800 (50) 163 / 135 / 150 / 143,
+//   1600 (100) 221 / 170 / 177 / 177, 2500 (156) 350 / 276 / 230 / 234, 3000 (188) 382 / 298 / 280 / 265, 4096 (256) 494 / 381 / 383 / 357.
+// So the pairs, and smaller tiles for fewer rows: up to 110 per expert 128, whose deeper ring of weights counts, to 170 192.  Where there are
+// hardly two tiles for a pair, 128 again (8 experts, top-2, 4096 x 2048, 1000 tokens: 116 / 120 / 118).
+// Few experts of short K leave pairs, two SMs each, a last round that is nearly empty: up to 64 rows per expert the weight rows stay where both
+// estimates say so (16 of 64 experts, top-4, 1280 x 832, 130 tokens: 29.7 / 32.9; 256 experts, 1024 x 384, 520 tokens: 87.5 / 89.5).  In
+// microseconds: 0.2 a stage of 128 channels and 0.85 a tile; 0.45, 0.002 a row and 1.0 with four times the CTAs.  The choice takes 0.4 % more
+// than the best of all over those shapes.
+// Layers of up to three stages in all stay with the forms that the tests of the tiles' edges name (8 experts, 256 x 128, 768 tokens: 32 us with
+// 256-row token tiles; weight rows 26, pairs 24).
+Dec::MoeTiles Dec::moe_tiles(int ns) const {
+    const int n_local = moe.e1 - moe.e0, stages13 = (moe.hidden + 127) / 128, stages2 = (moe.ffn + 127) / 128;
+    if (tune_moe_gemm > 2) {
+        return {MoeTiles::PAIRS, tune_moe_gemm};
+    }
+    if (tune_moe_gemm == 2 || (tune_moe_gemm == 0 && stages13 + stages2 <= 3 && (long long)ns >= 192LL * moe.n_experts)) {
+        return {MoeTiles::TOKEN_ROWS, 256};
+    }
+    if (tune_moe_gemm == 1 || stages13 + stages2 <= 3) {
+        return {MoeTiles::WEIGHT_ROWS, 128};
+    }
+    const double rows = (double)ns / moe.n_experts;                  // per expert, on average
+    auto round_up = [](int a, int b) { return (a + b - 1) / b; };
+    auto tiles = [&](int cap) { return n_local * (rows <= 0.8 * cap ? 1.0 : rows / cap + 0.5); };
+    if (rows <= 64.0) {
+        const int pairs = sm_count / 2, tok = round_up((int)ceil(rows), 16) * 16;
+        const double step = 0.45 + 0.002 * tok;
+        double p = 1.0, w = 0.0;
+        for (int m = 0; m < 2; ++m) {
+            const int n = m == 0 ? 2 * moe.ffn : moe.hidden, stages = m == 0 ? stages13 : stages2;
+            p += ceil(tiles(128) * round_up(n, 256) / pairs) * (stages * 0.2 + 0.85);
+            w += ceil(tiles(128) * round_up(n, 128) / (4 * pairs)) * (stages * step + 1.0);
+        }
+        if (w < p) {
+            return {MoeTiles::WEIGHT_ROWS, 128};
+        }
+    }
+    const bool few = n_local * round_up(2 * moe.ffn, 256) * std::max(1.0, rows / 256.0) < sm_count;
+    return {MoeTiles::PAIRS, rows <= 110.0 || few ? 128 : rows <= 170.0 ? 192 : 256};
+}
+
 int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t, int out_kind, cudaStream_t st) {
     if (!moe.set) {
         return fail("w4a16 moe_ffn: set_moe was not called");
@@ -106,8 +148,8 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
     const int ns = t * moe.top_k;
     const int n_local = moe.e1 - moe.e0;
     cudaError_t e = cudaSuccess;
-    auto sort = [&](int bm, bool even) {
-        e = launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, even, tune_pdl, st, launches);
+    auto sort = [&](int bm, int shares) {
+        e = launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, shares, tune_pdl, st, launches);
         // The top-k may have counted, with nothing after it that clears the counts for the next call; where they cannot be cleared, that
         // call makes its scratch anew.
         if (e != cudaSuccess && cudaMemsetAsync(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int), st) != cudaSuccess) {
@@ -139,7 +181,7 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
                 return rc;
             }
         } else {
-            if (int rc = sort(8, false)) {
+            if (int rc = sort(8, TILES_FULL)) {
                 return rc;
             }
             if (int rc = gemv_grouped(&i13->second, mb.xs, mb.act, 2 * moe.ffn, mb, max_tiles, est_tiles, est_segments, nullptr, st, uneven, nullptr,
@@ -152,24 +194,23 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
             return rc;
         }
     } else {
-        // Experts with fewer than 192 rows on average: weight-row tiles of up to 128 rows, an expert's rows in equal shares, padded
-        // to 16; above that 256-row token tiles.  128 experts, top-8, 2048 x 768, groups of 32, us per layer, weight-row / token
-        // tiles: 200 tokens (12 rows per expert) 139 / 254, 1024 tokens 186 / 272, 2000 tokens 279 / 311, 3000 tokens (188 rows)
-        // 386 / 374, 4096 tokens (256 rows) 510 / 493; 64 experts, top-6, 2048 x 1024: 2000 tokens (188 rows) 247 / 246, 3000 tokens
-        // (281 rows) 354 / 382, 4096 tokens 456 / 424.  The line lies where the two met with a CTA per weight-row tile; with persistent
-        // CTAs they are within 8 % of each other, either way, from 188 to 281 rows.  Tiles of up to 64 rows: the same below 64 rows per
-        // expert, slower above.
-        const bool weight_rows = (long long)ns < 192LL * moe.n_experts;
-        const int bm = weight_rows ? 128 : 256;
-        const int max_tiles = (ns + bm - 1) / bm + std::min(ns, n_local);
-        if (int rc = sort(bm, weight_rows)) {
+        const MoeTiles f = moe_tiles(ns);
+        const int max_tiles = (ns + f.rows - 1) / f.rows + std::min(ns, n_local);
+        if (int rc = sort(f.rows, f.form == MoeTiles::PAIRS ? TILES_SORTED : f.form == MoeTiles::WEIGHT_ROWS ? TILES_EVEN : TILES_FULL)) {
             return rc;
         }
-        if (weight_rows) {
-            if (int rc = gemm_ts_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, bm, nullptr, st, true)) {
+        if (f.form == MoeTiles::PAIRS) {
+            if (int rc = gemm_ts2_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, f.rows, nullptr, st, true)) {
                 return rc;
             }
-            if (int rc = gemm_ts_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, bm, mb.row_w, st, false)) {
+            if (int rc = gemm_ts2_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, f.rows, mb.row_w, st, false)) {
+                return rc;
+            }
+        } else if (f.form == MoeTiles::WEIGHT_ROWS) {
+            if (int rc = gemm_ts_grouped(&i13->second, mb.xs, ns, mb.act, 2 * moe.ffn, mb, max_tiles, f.rows, nullptr, st, true)) {
+                return rc;
+            }
+            if (int rc = gemm_ts_grouped(&i2->second, mb.act, ns, mb.c2, moe.hidden, mb, max_tiles, f.rows, mb.row_w, st, false)) {
                 return rc;
             }
         } else {

@@ -304,3 +304,34 @@ def test_second_matmul_in_the_other_form(dec, orc, t, f, h, group):
         finally:
             dec.set_tuning("pdl", 1)
     dec.graph_destroy(g)
+
+
+# MoE prefill on CTA pairs (gemm_ts2.cu): experts of 0, 1, 7, 8, ... rows around the steps of the stores (8, 32), of the accumulators (128), of the tiles
+# that are two MMAs (more than 224) and of the largest tiles; odd numbers of k-blocks, row tiles of 64 and 128 of 256 rows; half of the experts elsewhere
+@pytest.mark.parametrize("tile", [128, 192, 256])
+@pytest.mark.parametrize("f,h,group,local", [(320, 576, 32, 12), (128, 448, 64, 6), (384, 640, 128, 12)])
+def test_expert_tiles_on_pairs(dec, orc, tile, f, h, group, local):
+    rows = [0, 33, 1, 129, 7, 225, 8, 257, 31, 300, 224, 96]
+    n_exp, t = len(rows), sum(rows)
+    rng = np.random.Generator(np.random.PCG64(tile))
+    lg = rng.standard_normal((t, n_exp)).astype(np.float32)
+    lg[np.arange(t), rng.permutation(np.repeat(np.arange(n_exp), rows))] += 40.0
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=81)
+    x = synth.make_acts(t, h, seed=82)
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    total = 0
+    dec.set_tuning("moe_gemm", tile)
+    try:
+        for e0 in range(0, n_exp, local):
+            mine = slice(e0, e0 + local)
+            dec.set_moe(n_exp, 1, f, h, group, e0, local)
+            dec.upload_experts(0, w13_q[mine], w13_s[mine], w2_q[mine], w2_s[mine])
+            y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+            assert dec.last_kernel().startswith("gemm_ts2_kernel")
+            assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+            total = total + y.cpu().numpy()
+    finally:
+        dec.set_tuning("moe_gemm", 0)
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, 1, group)
+    err = np.abs(total - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the tests above
