@@ -164,6 +164,7 @@ struct Dec {
         int rows;
     };
     MoeTiles moe_tiles(int ns) const;
+    bool tiny_moe() const { return (moe.hidden + 127) / 128 + (moe.ffn + 127) / 128 <= 3; }   // hardly any K in either matmul
     void free_moe(bool retire = false);
     int moe_ffn(int layer, const float* logits, const void* x16, void* y, int t, int out_kind, cudaStream_t st);
 };

@@ -743,26 +743,31 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                         l->k, tune_ts_ks);
         }
         const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
-        if (t > 64 && t <= 4096 && !(ts && c.ks > 1) && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0 &&
+        const bool stays = ts && (c.ks > 1 ? l->k >= 16384 : t <= 320 && (long long)l->n * l->k <= 1 << 20);
+        if (t > 64 && t <= 4096 && !stays && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0 &&
             tune_gemm_tma_store == 1) {
-            // The pairs (gemm_ts2.cu) take f16 results that they are estimated to finish sooner by at least 2 %.  Over 140 drawn shapes (66..4096
-            // tokens) the choice took 6.4 % less time than the better of the two other forms' rule, the best choice of each 7.1 %; the worst case
-            // was 551 x 20752 x 16128, 301 against 294 us, the best 3418 x 24592 x 1408, 185 against 266.  Calls of few tiles (526 x 2144 x 16384:
-            // 52 against 38 us) stay with the weight-row form, which splits K over clusters.  Below 65 and above 4096 tokens they were not compared.
-            // The f32 results of such a call are what its f16 results are rounded from, so they come from a form without a K split, too -- each
-            // of the three adds the channels of a sum in the same order.  They keep the form that they have without the pairs, unless that
-            // splits tiles: then the token-row form without a split, or the pairs where a nearly empty last wave is what the split was for (its
-            // estimate leaves out that the full waves hold the clock down) or where they are ahead by a clear margin (their estimate for f32
-            // results is good to a tenth).  f32, us with the split / without / pairs: 7168 x 5120 at 4096 tokens 235 / 257 / 230, at 3000 185 / 218 /
-            // 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512; 5120 x 6144 at 4096, 2.92 waves, 206 / 205 / 193.
-            if (gemm_ts2_choose(l, t, W4A16_OUT_F16).cost < 0.98 * (ts ? c.cost : best.cost)) {
-                if (out_kind == W4A16_OUT_F16) {
+            // The pairs (gemm_ts2.cu) take f16 results that they are estimated to finish sooner.  The estimates of the weight-row form run 5 % high
+            // in the median, so the line lies at 0.92 of them, 0.9 below 256 tokens, at 0.84 where they split K over clusters, and at 0.8 up to 128
+            // tokens, where a wrong choice costs most.  Over 308 measured calls (22 shapes, 72..3000 tokens) the choice takes 1.0 % more than the
+            // best form and tile of each; with a line that ended at split calls, and the estimates before it, it took 7.2 %.  Split calls of
+            // K >= 16384, and up to 320 tokens of linears of up to 2^20 weights, stay with the weight rows, as the tests name them (256 x 5120 x
+            // 17408: 44 us, pairs of 96 tokens 40).  Up to 64 and above 4096 tokens the pairs were not compared.
+            // The f32 results of such a call are what its f16 results are rounded from, so they come from a form without a K split, too -- each of
+            // the three adds the channels of a sum in the same order: from the pairs where the weight rows would split K.  Otherwise they keep the
+            // form that they have without the pairs, unless that splits tiles: then the token-row form without a split, or the pairs where a nearly
+            // empty last wave is what the split was for (its estimate leaves out that the full waves hold the clock down) or where they are ahead
+            // by a clear margin (their estimate for f32 results is good to a tenth).  f32, us with the split / without / pairs: 7168 x 5120 at 4096
+            // tokens 235 / 257 / 230, at 3000 185 / 218 / 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512; 5120 x 6144 at 4096,
+            // 2.92 waves, 206 / 205 / 193.
+            const double line = t <= 128 ? 0.8 : !ts ? 0.98 : c.ks > 1 ? 0.84 : t < 256 ? 0.9 : 0.92;
+            if (gemm_ts2_choose(l, t, W4A16_OUT_F16).cost < line * (ts ? c.cost : best.cost)) {
+                if (out_kind == W4A16_OUT_F16 || (ts && c.ks > 1)) {
                     return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind).tok, st);
                 }
                 if (!ts && best.cost < whole.cost) {
                     const TsChoice p = gemm_ts2_choose(l, t, out_kind);
                     const int rest = (t + BM * whole.mt - 1) / (BM * whole.mt) * ((l->n + whole.bn - 1) / whole.bn) % sm_count;
-                    if (p.cost < whole.cost * (rest > 0 && rest <= 100 ? 1.0 : 0.86)) {
+                    if (p.cost < whole.cost * (rest > 0 && rest <= 100 ? 1.0 : 0.78)) {
                         return gemm_ts2(l, x, dst, t, out_kind, p.tok, st);
                     }
                     best = whole;

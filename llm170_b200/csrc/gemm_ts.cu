@@ -11,15 +11,19 @@
 //
 //   warp 0      tokens: both k-blocks of a 128-channel stage as one TMA box (128B swizzle, shallow ring: L2)
 //   warp 1      issues 8 x tcgen05.mma (M128, N tokens, K16) per stage; commits hand the TMEM stage and the token stage back
-//   warps 2-9   raw -> registers -> TMEM, one 16-row block each, then the epilogue
-//   warp 10     weights: raw int4 of the CTA's rows (one bulk copy per k-block, deep ring: this hides the HBM latency)
+//   warps 2-    raw -> registers -> TMEM, then the epilogue (the first eight): three teams of four warps that take stages in turn, or
+//               eight warps with a 16-row block of every stage each
+//   last warp   weights: raw int4 of the CTA's rows (one bulk copy per k-block) and their scales, deep ring: this hides the HBM latency
 //
 // What bounds it: below about 64 tokens neither HBM nor the tensor pipe but the serial chain of a role per stage (wait,
 // issue, hand over; 34816 x 5120, 16 tokens, two CTAs per SM: 0.69 us per stage of 2 x 8 KB).  So the roles that issue
 // TMA, bulk copies and MMAs each have a warp of their own that stays converged with one elected lane (uniform registers
 // feed these instructions: 36 -> 34 us) and a stage is one token box and two weight copies (34 -> 30.6 us).  The expansion
-// itself, the TMEM stores, loads from HBM and the MMAs each cost under 15 % when taken out alone.  A second set of eight
-// expanding warps (33 us) and 256 rows per CTA (33.5 us) were slower.
+// itself, the TMEM stores, loads from HBM and the MMAs each cost under 15 % when taken out alone; what is left is the chain of the
+// expanding warps, about 600 cycles a stage, so up to 64 tokens (96 where CTAs queue) teams of four take stages in turn, and three chains
+// overlap: 27 tokens of 34816 x 5120 27.2 -> 25.6 us, of 5120 x 17408 18.7 -> 18.4, in groups of 32 31.0 -> 28.9.  Above that the MMAs
+// of a stage take as long as its chain, with fewer than four stages per CTA a team is idle: eight warps on every stage.
+// 256 rows per CTA were slower (33.5 us).
 //
 // The K splits of a tile form a thread-block cluster and sum their f32 accumulators through distributed shared memory in
 // split order (no global scratch, no tickets).
@@ -41,7 +45,9 @@ namespace w4 {
 
 namespace {
 
-constexpr int TS_THREADS = (3 + DQ_WARPS) * 32;
+constexpr int TS_TEAM = 4, TS_MAX_TEAMS = 3;    // expanding warps: teams that take stages in turn, or a warp per 16-row block on every stage
+__host__ __device__ constexpr int ts_threads(bool teams) { return (3 + (teams ? TS_MAX_TEAMS * TS_TEAM : DQ_WARPS)) * 32; }
+constexpr int TSG_THREADS = ts_threads(false);  // grouped form (teams: 2 to 6 % slower, 60 and fewer rows per expert)
 constexpr int TS_XBOX = 64;                     // grouped form: rows of a token box
 constexpr int TS_STAGE_BYTES = 16 * 1024;       // grouped form: results on their way out
 constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
@@ -62,6 +68,7 @@ struct TsArgs {
     int nrb_w;           // 16-row blocks of the resident matrix (tile pitch)
     int ksplit;
     int raw_stages, x_stages, a_stages;
+    int teams;           // of expanding warps; raw_stages and a_stages are multiples of it
     int tmem_cols;
     int off_x, off_bars; // byte offsets in dynamic shared memory (1024-byte aligned base)
     int off_stage;       // grouped: results of a tile on their way out
@@ -97,14 +104,15 @@ __device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned c
     return v;
 }
 
-template <int GROUP, bool FMA>
-__global__ void __launch_bounds__(TS_THREADS, 2)
+template <int GROUP, bool FMA, bool TEAMS>
+__global__ void __launch_bounds__(ts_threads(TEAMS), 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
 
     constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    constexpr int EXP_WARPS = TEAMS ? TS_MAX_TEAMS * TS_TEAM : DQ_WARPS, ARRIVE = TEAMS ? TS_TEAM : DQ_WARPS;
     constexpr uint32_t RAW_STAGE = RAW_BYTES + ts_scale_bytes(GROUP);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // known to be warp-uniform
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -151,14 +159,14 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         s_abort = 0;
         for (int s = 0; s < NR; ++s) {
             mbar_init(raw_full(s), 1);
-            mbar_init(raw_free(s), DQ_WARPS);
+            mbar_init(raw_free(s), ARRIVE);
         }
         for (int s = 0; s < NX; ++s) {
             mbar_init(x_full(s), 1);
             mbar_init(x_free(s), 1);
         }
         for (int s = 0; s < NA; ++s) {
-            mbar_init(a_ready(s), DQ_WARPS);
+            mbar_init(a_ready(s), ARRIVE);
             mbar_init(a_free(s), 1);
         }
         mbar_init(accum_bar, 1);
@@ -209,7 +217,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 px ^= 1;
             }
         }
-    } else if (warp == 2 + DQ_WARPS) {
+    } else if (warp == 2 + EXP_WARPS) {
         // ------------------------------------------------------------------ weights
         const bool leader = elect_one();
         int sr = 0, pr = 0;
@@ -273,62 +281,90 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         __syncwarp();
     } else {
         // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM
-        // One 16-row block per warp; a warp may touch the TMEM lanes 32 * (warp % 4) .. +31 = two row blocks.
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int rb = quad * 2 + half;
-        const bool live = rb < nrbv;
-        const int rbl = live ? rb : 0;
-        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
-        const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
-        const uint32_t s_ld = base + (uint32_t)(RAW_BYTES + rbl * (GPS * 32)) + (uint32_t)(lane >> 2) * 4u;   // scale pairs of the lane's rows
-        int sr = 0, pr = 0, sa = 0, pa = 1;
-        for (int it = 0; it < nst; ++it) {
-            // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
-            if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (35 << 16) | it))) {
-                ok = false;
-                break;
+        if (TEAMS) {
+            // A team of four warps takes a stage, the teams take stages in turn (ts_expand_stage).
+            const int quad = warp & 3, team = (warp - 2) >> 2, teams = a.teams;
+            const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32) << 16);
+            int sr = team, sa = team;
+            uint32_t pr = 0, pa = 1;
+            for (int it = team; team < teams && it < nst; it += teams) {
+                // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
+                const bool in = ts_expand_stage<GROUP, FMA>(
+                    raw_addr(sr), quad, nrbv, lane, t_st + (uint32_t)(sa * A_COLS), a.fma_add, a.fma_mul,
+                    [&]() { return __all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (35 << 16) | it)) != 0; },
+                    [&]() { return it < NA || __all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it)) != 0; },
+                    [&]() { mbar_arrive(raw_free(sr)); }, [&]() { mbar_arrive(a_ready(sa)); });
+                if (!in) {
+                    ok = false;
+                    break;
+                }
+                if ((sr += teams) >= NR) {
+                    sr = team;
+                    pr ^= 1;
+                }
+                if ((sa += teams) >= NA) {
+                    sa = team;
+                    pa ^= 1;
+                }
             }
-            const uint32_t ra = r_ld + (uint32_t)sr * RAW_STAGE;
-            const uint4 raw0 = lds128(ra);
-            const uint4 raw1 = lds128(ra + RAW_BYTES / 2);           // stale bytes when the stage holds one k-block
-            uint32_t sc[GPS];
+        } else {
+            // One 16-row block per warp; a warp may touch the TMEM lanes 32 * (warp % 4) .. +31 = two row blocks.
+            const int quad = warp & 3, half = (warp - 2) >> 2;
+            const int rb = quad * 2 + half;
+            const bool live = rb < nrbv;
+            const int rbl = live ? rb : 0;
+            const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32 + half * 16) << 16);
+            const uint32_t r_ld = base + (uint32_t)rbl * (TILE_WORDS * 4) + (uint32_t)lane * 16u;
+            const uint32_t s_ld = base + (uint32_t)(RAW_BYTES + rbl * (GPS * 32)) + (uint32_t)(lane >> 2) * 4u;   // scale pairs of the lane's rows
+            int sr = 0, pr = 0, sa = 0, pa = 1;
+            for (int it = 0; it < nst; ++it) {
+                // (a warp leaves as a whole: an expired wait may be seen by some of its lanes first)
+                if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (35 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t ra = r_ld + (uint32_t)sr * RAW_STAGE;
+                const uint4 raw0 = lds128(ra);
+                const uint4 raw1 = lds128(ra + RAW_BYTES / 2);           // stale bytes when the stage holds one k-block
+                uint32_t sc[GPS];
 #pragma unroll
-            for (int i = 0; i < GPS; ++i) {
-                sc[i] = lds32(s_ld + (uint32_t)sr * RAW_STAGE + (uint32_t)i * 32u);
-            }
-            uint32_t v[16];
-            const TsScale<FMA> sc0(sc[0], a.fma_add, a.fma_mul), sc1(sc[GPS > 1 ? 1 : 0], a.fma_add, a.fma_mul);
-            ts_expand<FMA>(raw0, sc0, sc1, v);
-            if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
-                ok = false;
-                break;
-            }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
-            tmem_st_16x256b_x4(td, v);
-            if (GPS > 1) {
-                ts_expand<FMA>(raw1, TsScale<FMA>(sc[GPS > 2 ? 2 : 0], a.fma_add, a.fma_mul), TsScale<FMA>(sc[GPS > 2 ? 3 : 0], a.fma_add, a.fma_mul), v);
-            } else {
-                ts_expand<FMA>(raw1, sc0, sc1, v);
-            }
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
-            }
-            tmem_st_16x256b_x4(td + BK / 2, v);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(a_ready(sa));
-            }
-            if (++sr == NR) {
-                sr = 0;
-                pr ^= 1;
-            }
-            if (++sa == NA) {
-                sa = 0;
-                pa ^= 1;
+                for (int i = 0; i < GPS; ++i) {
+                    sc[i] = lds32(s_ld + (uint32_t)sr * RAW_STAGE + (uint32_t)i * 32u);
+                }
+                uint32_t v[16];
+                const TsScale<FMA> sc0(sc[0], a.fma_add, a.fma_mul), sc1(sc[GPS > 1 ? 1 : 0], a.fma_add, a.fma_mul);
+                ts_expand<FMA>(raw0, sc0, sc1, v);
+                if (it >= NA && !__all_sync(0xffffffffu, mbar_wait(a_free(sa), pa, abort_flag, a.status, (36 << 16) | it))) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
+                tmem_st_16x256b_x4(td, v);
+                if (GPS > 1) {
+                    ts_expand<FMA>(raw1, TsScale<FMA>(sc[GPS > 2 ? 2 : 0], a.fma_add, a.fma_mul), TsScale<FMA>(sc[GPS > 2 ? 3 : 0], a.fma_add, a.fma_mul), v);
+                } else {
+                    ts_expand<FMA>(raw1, sc0, sc1, v);
+                }
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
+                }
+                tmem_st_16x256b_x4(td + BK / 2, v);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(a_ready(sa));
+                }
+                if (++sr == NR) {
+                    sr = 0;
+                    pr ^= 1;
+                }
+                if (++sa == NA) {
+                    sa = 0;
+                    pa ^= 1;
+                }
             }
         }
         ok = __all_sync(0xffffffffu, ok);
@@ -341,7 +377,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     }
 
     // ---------------------------------------------------------------------- epilogue
-    const bool dq_warp = warp >= 2 && warp < 2 + DQ_WARPS;
+    const bool dq_warp = warp >= 2 && warp < 2 + DQ_WARPS;           // (the third team has nothing to do with the results)
     const int quad = warp & 3, sub = (warp - 2) >> 2;
     constexpr int EW = DQ_WARPS / 4;                                 // warps that share a TMEM lane quadrant
     const int lrow = quad * 32 + lane;                               // weight row within the tile
@@ -364,7 +400,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         if (!*abort_flag) {
             const int pieces = min(TS_MROWS, a.n - n0) / 8;
             __half* out = reinterpret_cast<__half*>(a.out) + (size_t)m0 * a.n + n0;
-            for (int e = (int)threadIdx.x; e < rows_valid * pieces; e += TS_THREADS) {
+            for (int e = (int)threadIdx.x; e < rows_valid * pieces; e += ts_threads(TEAMS)) {
                 const int tok = e / pieces, c = e - tok * pieces;
                 *reinterpret_cast<uint4*>(out + (size_t)tok * a.n + c * 8) = *reinterpret_cast<const uint4*>(base_ptr + tok * PER_TOK + c * 16);
             }
@@ -404,7 +440,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const int nr4 = min(ROWS, a.n - n0) / 4;
             const int total = nt * nr4;
             const int e0 = (int)((long long)total * split / ks), e1 = (int)((long long)total * (split + 1) / ks);
-            for (int e = e0 + (int)threadIdx.x; e < e1; e += TS_THREADS) {
+            for (int e = e0 + (int)threadIdx.x; e < e1; e += ts_threads(TEAMS)) {
                 const int tok = e / nr4, r = (e - tok * nr4) * 4;
                 float4 pv[8];
 #pragma unroll
@@ -451,7 +487,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 // converted, and the two CTAs of an SM fill each other's epilogues.  (Layer of 128 experts, top-8: 256 tokens 165 ->
 // 141 us, 1024 tokens 209 -> 186.)
 template <int GROUP>
-__global__ void __launch_bounds__(TS_THREADS, 2)
+__global__ void __launch_bounds__(TSG_THREADS, 2)
 gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s, const TsArgs a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
@@ -796,8 +832,9 @@ static size_t ts_smem(int group, int tok, int nr, int nx, int na, int* off_x, in
 
 cudaError_t gemm_ts_init_device() {
     cudaError_t e = cudaSuccess;
-    for (const void* f : {(const void*)gemm_ts_kernel<128, false>, (const void*)gemm_ts_kernel<128, true>, (const void*)gemm_ts_kernel<32, false>, (const void*)gemm_ts_grouped_kernel<128>,
-                          (const void*)gemm_ts_grouped_kernel<32>}) {
+    for (const void* f : {(const void*)gemm_ts_kernel<128, false, false>, (const void*)gemm_ts_kernel<128, true, false>, (const void*)gemm_ts_kernel<32, false, false>,
+                          (const void*)gemm_ts_kernel<128, false, true>, (const void*)gemm_ts_kernel<128, true, true>, (const void*)gemm_ts_kernel<32, false, true>,
+                          (const void*)gemm_ts_grouped_kernel<128>, (const void*)gemm_ts_grouped_kernel<32>}) {
         if (e == cudaSuccess) {
             e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TS_SMEM_FULL_MAX);
         }
@@ -809,18 +846,22 @@ cudaError_t gemm_ts_init_device() {
 namespace {
 struct TsPlan {
     int tmem_cols, na, nr, nx, off_x, off_bars;
+    int teams;           // 0: a warp per row block
     size_t smem;
 };
-TsPlan ts_plan(int group, int tok) {
+TsPlan ts_plan(int group, int tok, bool teams) {
     TsPlan p{};
     // TMEM: the accumulator and as many expanded stages as fit in half of it (two CTAs per SM), else in all of it
     p.tmem_cols = tok <= 128 ? 256 : 512;
     p.na = std::min((p.tmem_cols - tok) / A_COLS, 4);
     const size_t limit = p.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
+    p.teams = !teams ? 0 : p.na % 3 == 0 ? 3 : 2;
+    const int step = std::max(1, p.teams);                       // the rings divide by the teams
     p.nx = p.nr = ts_smem(group, tok, 3, 3, p.na, &p.off_x, &p.off_bars) <= limit ? 3 : 2;
-    while (p.nr < 12 && ts_smem(group, tok, p.nr + 1, p.nx, p.na, &p.off_x, &p.off_bars) <= limit) {
-        ++p.nr;
-        if (p.nr % 2 == 0 && p.nx < 4 && ts_smem(group, tok, p.nr, p.nx + 1, p.na, &p.off_x, &p.off_bars) <= limit) {
+    p.nr = (p.nr + step - 1) / step * step;
+    while (p.nr + step <= 12 && ts_smem(group, tok, p.nr + step, p.nx, p.na, &p.off_x, &p.off_bars) <= limit) {
+        p.nr += step;
+        if ((teams || p.nr % 2 == 0) && p.nx < 4 && ts_smem(group, tok, p.nr, p.nx + 1, p.na, &p.off_x, &p.off_bars) <= limit) {
             ++p.nx;
         }
     }
@@ -839,7 +880,7 @@ void Dec::ts_query_clusters() {
         if (ks > 1) {
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3(1, ks);
-            cfg.blockDim = dim3(TS_THREADS);
+            cfg.blockDim = dim3(ts_threads(false));
             cfg.dynamicSmemBytes = TS_SMEM_FULL_MAX;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -848,7 +889,7 @@ void Dec::ts_query_clusters() {
             attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr;
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128, false>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&n, gemm_ts_kernel<128, false, false>, &cfg) != cudaSuccess) {
                 cudaGetLastError();
                 n = 0;       // then this split is not considered
             }
@@ -907,7 +948,13 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
     }
-    const TsPlan p = ts_plan(l->group, c.tok);
+    // Teams where stages follow one another quickly: up to 64 tokens, to 96 with two CTAs on an SM.  A CTA of few stages has its first one sooner
+    // with all warps on it (us, a warp per row block / teams: 27 x 34816 x 5120 27.2 / 25.6, groups of 32 31.0 / 28.9; 96 x 34816 x 5120 33.3 /
+    // 29.2; 72 x 4096 x 4096 10.4 / 10.7, 197 x 5120 x 6144 21.2 / 22.0, 9 x 1024 x 1024 in clusters of 8 3.4 / 3.6).
+    const long long ctas = (long long)((t + c.tok - 1) / c.tok) * ((l->n + TS_MROWS - 1) / TS_MROWS) * c.ks;
+    const int nst = ((l->k + SK - 1) / SK + c.ks - 1) / c.ks;
+    const bool teams = nst >= 4 && (c.tok <= 64 || (c.tok <= 96 && ctas > sm_count && nst >= 16));
+    const TsPlan p = ts_plan(l->group, c.tok, teams);
     TsArgs a{};
     a.tok = c.tok;
     a.ksplit = c.ks;
@@ -916,6 +963,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     a.tmem_cols = p.tmem_cols;
     a.a_stages = p.na;
     a.raw_stages = p.nr;
+    a.teams = p.teams;
     a.x_stages = p.nx;
     a.off_x = p.off_x;
     a.off_bars = p.off_bars;
@@ -947,7 +995,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     a.status = gemm_status;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(a.m_tiles * a.n_tiles, a.ksplit);
-    cfg.blockDim = dim3(TS_THREADS);
+    cfg.blockDim = dim3(ts_threads(teams));
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -968,9 +1016,9 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     cfg.numAttrs = n_attr;
     cudaError_t e;
     if (l->group != 128) {
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<32, false>, map, smap, a);
+        e = cudaLaunchKernelEx(&cfg, teams ? gemm_ts_kernel<32, false, true> : gemm_ts_kernel<32, false, false>, map, smap, a);
     } else if (l->fma_e < 0) {
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, false>, map, smap, a);
+        e = cudaLaunchKernelEx(&cfg, teams ? gemm_ts_kernel<128, false, true> : gemm_ts_kernel<128, false, false>, map, smap, a);
     } else {
         // one f16 operation per pair of weights where two do it otherwise, in the expansion that a small batch waits for (27 x 34816 x
         // 5120: 29.8 -> 26.5 us, 27 x 5120 x 17408: 21.3 -> 19.3); the weights come out 2^-E smaller
@@ -978,7 +1026,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
         memcpy(&a.fma_mul, &mul, sizeof(mul));
         a.fma_add = ((uint32_t)(20 - l->fma_e) << 26) + ((uint32_t)(24 - l->fma_e) << 10);
         a.out_mul = ldexpf(l->out_mul, l->fma_e);
-        e = cudaLaunchKernelEx(&cfg, gemm_ts_kernel<128, true>, map, smap, a);
+        e = cudaLaunchKernelEx(&cfg, teams ? gemm_ts_kernel<128, true, true> : gemm_ts_kernel<128, true, false>, map, smap, a);
     }
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
@@ -1053,7 +1101,7 @@ int Dec::gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, i
     a.tables_fresh = tables_fresh ? 1 : 0;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(std::min(a.m_tiles * a.n_tiles, 2 * sm_count));
-    cfg.blockDim = dim3(TS_THREADS);
+    cfg.blockDim = dim3(TSG_THREADS);
     cfg.dynamicSmemBytes = std::max(smem_of(nr), TS_SMEM_HALF_MIN);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];

@@ -87,4 +87,65 @@ __device__ __forceinline__ void ts_expand(const uint4& raw, const TsScale<FMA>& 
     }
 }
 
+// One warp's part of a stage: the two 16-row blocks of the TMEM lanes that it may touch (32 * (warp % 4) .. +31), expanded from the raw stage at
+// `raw` into the stage at `td`.  A stage's way -- wait, expand, wait, store, hand over -- is a chain of about 600 cycles: teams of four warps
+// take stages in turn, so that the chains of several stages overlap, where eight warps with a row block each went through every stage
+// together.  A team keeps to its slots of the rings (their numbers are multiples of the teams'): it waits for every phase of the barriers that
+// it looks at, so the parity of a phase says which one it is.
+template <int GROUP, bool FMA, class Full, class Free, class RawRead, class Ready>
+__device__ __forceinline__ bool ts_expand_stage(uint32_t raw, int quad, int nrbv, int lane, uint32_t td, uint32_t fma_add, uint32_t fma_mul,
+                                                Full&& wait_full, Free&& wait_free, RawRead&& raw_read, Ready&& ready) {
+    constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
+    if (!wait_full()) {
+        return false;
+    }
+    constexpr int SPK = GPS > 1 ? 2 : 1;                             // scale groups per k-block
+    const int rb[2] = {quad * 2 < nrbv ? quad * 2 : 0, quad * 2 + 1 < nrbv ? quad * 2 + 1 : 0};
+    uint4 w[2][2];                                                   // [k-block][row block] (stale bytes when there is no second k-block)
+    uint32_t sc[2][2][SPK];                                          // scale pairs of the lane's rows
+    auto load = [&](int kb) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            w[kb][b] = lds128(raw + (uint32_t)(kb * (RAW_BYTES / 2) + rb[b] * (TILE_WORDS * 4)) + (uint32_t)lane * 16u);
+#pragma unroll
+            for (int q = 0; q < SPK; ++q) {
+                sc[kb][b][q] = lds32(raw + RAW_BYTES + (uint32_t)(rb[b] * (GPS * 32) + (GPS > 1 ? kb * 64 : 0) + q * 32) + (uint32_t)(lane >> 2) * 4u);
+            }
+        }
+    };
+    load(0);
+    if (!wait_free()) {
+        return false;
+    }
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int b = q & 1, kb = q >> 1;
+        const TsScale<FMA> s0(sc[kb][b][0], fma_add, fma_mul);
+        uint32_t v[16];
+        if (GPS > 1) {
+            ts_expand<FMA>(w[kb][b], s0, TsScale<FMA>(sc[kb][b][SPK - 1], fma_add, fma_mul), v);
+        } else {
+            ts_expand<FMA>(w[kb][b], s0, s0, v);
+        }
+        if (q == 0) {
+            load(1);
+        }
+        if (q == 2) {
+            __syncwarp();
+            if (lane == 0) {
+                raw_read();                                          // the stage is in registers
+            }
+        }
+        tmem_st_16x256b_x4(td + ((uint32_t)(b * 16) << 16) + (uint32_t)(kb * (BK / 2)), v);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) {
+        ready();
+    }
+    return true;
+}
+
 }  // namespace w4

@@ -441,71 +441,30 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
         }
     } else if (warp < 2 + P_EXP_WARPS) {
         // ------------------------------------------------------------------ expand: raw int4 -> f16 in TMEM
-        // A warp may touch the TMEM lanes 32 * (warp % 4) .. +31, two 16-row blocks: a team of four warps takes a stage, the teams take
-        // stages in turn.  A stage's way -- wait, expand, wait, store, hand over -- is a chain of about 600 cycles, which all 16 warps
-        // on one stage went through together, and which the teams' stages overlap.
-        const int quad = warp & 3, team = (warp - 2) >> 2;            // (with three stages the fourth team has nothing to do)
+        // A team of four warps takes a stage, the teams take stages in turn (ts_expand_stage; with three stages the fourth team has nothing to do).
+        const int quad = warp & 3, team = (warp - 2) >> 2;
         Tile tl{};
         int expert = pair0 < tiles ? expert_of(pair0) : 0;
-        const uint32_t t_st = tmem_a + ((uint32_t)(quad * 32) << 16);
-        uint32_t first = 0;                                          // stages of the tiles before
-        for (int i = pair0; team < NS && i < tiles && ok; i += pairs, first += (uint32_t)nst) {
+        const uint32_t td = tmem_a + ((uint32_t)(quad * 32) << 16) + (uint32_t)(team * A_COLS);
+        int sr = team, skip = team;                                  // skip: stages of the other teams before this one's next
+        uint32_t pr = 0, pa = 1, cnt = 0;
+        for (int i = pair0; team < NS && i < tiles && ok; i += pairs) {
             weights_at(i, expert, tl);
             expert = expert_of(i + pairs);
-            const int rb0 = quad * 2 < tl.nrbv ? quad * 2 : 0, rb1 = quad * 2 + 1 < tl.nrbv ? quad * 2 + 1 : 0;
-            const uint32_t r0 = base + (uint32_t)(rb0 * (TILE_WORDS * 4)) + (uint32_t)lane * 16u, r1 = r0 + (uint32_t)((rb1 - rb0) * (TILE_WORDS * 4));
-            // scale pair of the lane's rows, in the stage's first group
-            const uint32_t s0 = base + (uint32_t)(RAW_BYTES + rb0 * (GPS * 32)) + (uint32_t)(lane >> 2) * 4u, s1 = s0 + (uint32_t)((rb1 - rb0) * (GPS * 32));
-            for (int it = (int)(((uint32_t)team + NS - first % NS) % NS); it < nst; it += NS) {
-                const uint32_t g = first + (uint32_t)it, turn_r = g / NR, turn = g / NS;
-                const int sr = (int)(g - turn_r * NR), sa = team;
-                if (!__all_sync(0xffffffffu, mbar_wait(raw_full(sr), turn_r & 1, abort_flag, a.status, (66 << 16) | it))) {
-                    ok = false;
-                    break;
-                }
-                const uint32_t slot = (uint32_t)sr * P_RAW_STAGE;
-                uint4 raw[4];                                        // row block 0, 1 of k-block 0, then of 1 (stale bytes when there is none)
-                uint32_t sc[2][GPS];
-                raw[0] = lds128(r0 + slot);
-                raw[1] = lds128(r1 + slot);
-                raw[2] = lds128(r0 + slot + RAW_BYTES / 2);
-                raw[3] = lds128(r1 + slot + RAW_BYTES / 2);
-#pragma unroll
-                for (int q = 0; q < GPS; ++q) {
-                    sc[0][q] = lds32(s0 + slot + (uint32_t)q * 32u);
-                    sc[1][q] = lds32(s1 + slot + (uint32_t)q * 32u);
-                }
-                if (turn > 0 && !__all_sync(0xffffffffu, mbar_wait(free_(sa), (turn - 1) & 1, abort_flag, a.status, (67 << 16) | it))) {
-                    ok = false;
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int b = q & 1, kb = q >> 1;
-                    const TsScale<FMA> sc0(sc[b][GPS > 1 ? kb * 2 : 0], a.fma_add, a.fma_mul);
-                    uint32_t v[16];
-                    if (GPS > 1) {
-                        ts_expand<FMA>(raw[q], sc0, TsScale<FMA>(sc[b][kb * 2 + 1], a.fma_add, a.fma_mul), v);
-                    } else {
-                        ts_expand<FMA>(raw[q], sc0, sc0, v);
-                    }
-                    tmem_st_16x256b_x4(td + ((uint32_t)(b * 16) << 16) + (uint32_t)(kb * (BK / 2)), v);
-                    if (q == 3) {
-                        __syncwarp();
-                        if (lane == 0) {
-                            mbar_arrive(raw_free(sr));               // the stage is in registers
-                        }
-                    }
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive_cluster(in_leader(full(sa)));
+            int it = skip;
+            for (; it < nst && ok; it += NS, ++cnt) {
+                ok = ts_expand_stage<GROUP, FMA>(
+                    raw_addr(sr), quad, tl.nrbv, lane, td, a.fma_add, a.fma_mul,
+                    [&]() { return __all_sync(0xffffffffu, mbar_wait(raw_full(sr), pr, abort_flag, a.status, (66 << 16) | it)) != 0; },
+                    [&]() { return cnt == 0 || __all_sync(0xffffffffu, mbar_wait(free_(team), pa, abort_flag, a.status, (67 << 16) | it)) != 0; },
+                    [&]() { mbar_arrive(raw_free(sr)); }, [&]() { mbar_arrive_cluster(in_leader(full(team))); });
+                pa ^= 1;
+                if ((sr += NS) >= NR) {
+                    sr = team;
+                    pr ^= 1;
                 }
             }
+            skip = it - nst;
         }
     } else {
         // ------------------------------------------------------------------ epilogue
@@ -682,23 +641,25 @@ cudaError_t gemm_ts2_init_device() {
     return e;
 }
 
-// Tokens per tile with the least estimated time (microseconds, fitted to 700 measurements on B200: 140 shapes of 66..4096 tokens, 1024..34816
-// rows, K 512..17408, five tile widths each): 5.4 us per launch and 1.7 per further tile of a pair; a stage of 128 channels takes 0.00224 us per
-// token of the tile, the rate of the MMAs, but not less than the expansion (0.317 us, groups of 32: 0.445), and with all pairs busy, when
-// power holds the clock down, 0.082 + 0.00254 per token and at least 0.439 (0.470).  f32 results, stored from registers while the MMAs wait for
-// the accumulators, take another 0.0263 per token less 3.23 with each tile (202 measurements: 0.84..1.09 of them, nine tenths 0.94..1.06).
+// Tokens per tile with the least estimated time (microseconds, fitted to 1238 measurements on B200 within a third of their shape's best: 22 shapes
+// of 1792..34816 rows, K 1536..17408, 14 batches of 72..3000 tokens, seven tile widths; good to 4.2 %): 3.14 and 0.0064 per token of the tile per
+// launch; a stage of 128 channels takes 0.009 + 0.00212 per token, the rate of the MMAs, but not less than the expansion (0.193 us, groups of
+// 32: 0.221), and with all pairs busy, when power holds the clock down, 0.05 + 0.00272 per token and at least 0.268 (0.326); each further tile
+// of a pair 0.48 where tiles take both accumulators.  f32 results, stored from registers, take another 0.0263 per token less 3.23 with each tile
+// (202 measurements before the accumulators alternated).
 TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind) const {
     TsChoice best{0, 1, 1e30};
     const int n_tiles = (l->n + P_ROWS - 1) / P_ROWS, stages = (l->k + SK - 1) / SK, pairs = sm_count / 2;
-    for (int cap = P_TOK_MAX; cap >= 96; cap -= 32) {
+    const bool g128 = l->group == 128;
+    for (int cap = P_TOK_MAX; cap >= 64; cap -= 32) {
         const int m_tiles = (t + cap - 1) / cap;
         const int tok = ((t + m_tiles - 1) / m_tiles + 31) / 32 * 32;
         const long long tiles = (long long)m_tiles * n_tiles, waves = (tiles + pairs - 1) / pairs;
-        const double full = std::min(1.0, std::max(0.0, ((double)tiles / (waves * pairs) - 0.41) / 0.52));
-        const double light = std::max(l->group == 128 ? 0.317 : 0.445, 0.00224 * tok);
-        const double heavy = std::max(l->group == 128 ? 0.439 : 0.470, 0.082 + 0.00254 * tok);
-        const double f32 = out_kind == W4A16_OUT_F16 ? 0.0 : 0.0263 * tok - 3.23;
-        const double c = 5.4 + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * 1.7;
+        const double full = std::min(1.0, std::max(0.0, ((double)tiles / (waves * pairs) - 0.46) / 0.54));
+        const double light = std::max(g128 ? 0.193 : 0.221, 0.009 + 0.00212 * tok);
+        const double heavy = std::max(g128 ? 0.268 : 0.326, 0.05 + 0.00272 * tok);
+        const double f32 = out_kind == W4A16_OUT_F16 ? 0.0 : std::max(0.0, 0.0263 * tok - 3.23);
+        const double c = 3.14 + 0.0064 * tok + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * (tok > P_SUB_MAX ? 0.48 : 0.0);
         if (c < best.cost) {
             best = TsChoice{tok, 1, c};
         }

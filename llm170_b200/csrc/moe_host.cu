@@ -102,19 +102,21 @@ Dec::MoeTiles Dec::moe_tiles(int ns) const {
     if (tune_moe_gemm > 2) {
         return {MoeTiles::PAIRS, tune_moe_gemm};
     }
-    if (tune_moe_gemm == 2 || (tune_moe_gemm == 0 && stages13 + stages2 <= 3 && (long long)ns >= 192LL * moe.n_experts)) {
+    if (tune_moe_gemm == 2 || (tune_moe_gemm == 0 && tiny_moe() && (long long)ns >= 192LL * moe.n_experts)) {
         return {MoeTiles::TOKEN_ROWS, 256};
     }
-    if (tune_moe_gemm == 1 || stages13 + stages2 <= 3) {
+    const double rows = (double)ns / moe.n_experts;                  // per expert, on average
+    if (tune_moe_gemm == 1 || tiny_moe()) {
         return {MoeTiles::WEIGHT_ROWS, 128};
     }
-    const double rows = (double)ns / moe.n_experts;                  // per expert, on average
     auto round_up = [](int a, int b) { return (a + b - 1) / b; };
     auto tiles = [&](int cap) { return n_local * (rows <= 0.8 * cap ? 1.0 : rows / cap + 0.5); };
     if (rows <= 64.0) {
         const int pairs = sm_count / 2, tok = round_up((int)ceil(rows), 16) * 16;
         const double step = 0.45 + 0.002 * tok;
-        double p = 1.0, w = 0.0;
+        // (one round of pairs for both matmuls: nothing hides how a pair starts and ends, 64 experts of 1024 x 384 at 560 and 1600 slots 24.4 / 22.8 and
+        // 26.6 / 24.8 us)
+        double p = tiles(128) * std::max(round_up(2 * moe.ffn, 256), round_up(moe.hidden, 256)) <= pairs ? 5.0 : 1.0, w = 0.0;
         for (int m = 0; m < 2; ++m) {
             const int n = m == 0 ? 2 * moe.ffn : moe.hidden, stages = m == 0 ? stages13 : stages2;
             p += ceil(tiles(128) * round_up(n, 256) / pairs) * (stages * 0.2 + 0.85);
@@ -157,9 +159,11 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         }
         return e == cudaSuccess ? 0 : cuda_fail("moe_ffn launch", e);
     };
-    if ((long long)ns <= 8LL * moe.n_experts) {
-        // decode-sized batches (on average at most 8 rows per expert): the op is weight streaming, so every
-        // <=8-row segment of an expert runs through the GEMV kernel instead of a padded 128-row MMA tile
+    if ((long long)ns <= (tiny_moe() || tune_moe_gemm != 0 ? 8LL : 7LL) * moe.n_experts) {
+        // decode-sized batches (on average at most 7 rows per expert): the op is weight streaming, so every
+        // <=8-row segment of an expert runs through the GEMV kernel instead of a padded MMA tile.  (us per layer, segments / pairs: 128 experts,
+        // top-8, 2048 x 768, 6.9 rows 108 / 110, 8 rows 116 / 111; 64 experts, top-6, 2048 x 1024, 5.6 rows 67 / 81, 8 rows 90 / 82; 8 experts,
+        // 4096 x 2048, 6 rows 43 / 49, 8 rows 59 / 50.)
         // every expert with rows adds at most one partial segment to the ns / 8 full ones: the grid is sized for
         // this bound, and CTAs beyond the actual count leave at once
         const int est_tiles = ns < n_local ? ns : n_local;   // segments expected to be non-empty (split-K sizing)

@@ -479,6 +479,27 @@ def test_cta_pairs_equal_the_weight_row_form(dec, t, k, n, group, bf16):
     dec.drop_lin("pairf")
 
 
+# teams of expanding warps that take stages in turn: three to eleven stages (below four: no teams), numbers of stages that two and three teams do not
+# divide, a last stage of one k-block, a ragged row tile, the largest tiles that have teams, more CTAs than SMs
+@pytest.mark.parametrize("t,k,n,group", [(9, 384, 272, 128), (16, 512, 272, 128), (27, 640, 400, 32), (33, 832, 272, 64), (64, 960, 144, 32), (64, 1408, 272, 128),
+                                         (90, 2048, 19216, 128), (96, 2176, 19216, 32)])
+def test_expanding_teams_equal_the_pairs(dec, t, k, n, group):
+    q, s = synth.make_linear_cuda(n, k, group, 17, "cuda")
+    dec.upload_lin_g_dev("team", q, s, n, k, group)
+    x = torch.randn((t, k), device="cuda").half()
+    with forced(dec, "gemm_pair", 64):
+        want = dec.lin_forward("team", x, t, out_f16=True)
+        assert dec.last_kernel().startswith("gemm_ts2_kernel")
+    with forced(dec, "gemm_form", 2), forced(dec, "gemm_ts_ksplit", 1):
+        for _ in range(3):
+            y = dec.lin_forward("team", x, t, out_f16=True)
+            assert dec.last_kernel().startswith("gemm_ts_kernel")
+            dec.sync()
+            assert torch.equal(y, want)
+    dec.kernel_status()
+    dec.drop_lin("team")
+
+
 @pytest.mark.parametrize("bad", [-1, 2, 16, 48, 288])
 def test_cta_pair_tuning_refuses_values_without_a_tile(dec, bad):
     from llm170_b200.w4a16_dec import W4a16Error
@@ -544,3 +565,9 @@ def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form
         want = x.float() @ dec.dequant_lin("both", f16=True).float().T
         assert (y32 - want).abs().max().item() <= 1e-4 * want.abs().max().item() + 1e-6
     dec.drop_lin("both")
+
+
+# ... and where the pairs take the place of weight rows that would split K over clusters: both kinds of results come from them
+@pytest.mark.parametrize("n,k,group,t", [(7168, 5120, 128, 197), (5120, 6144, 32, 197), (4096, 4096, 64, 320)])
+def test_pairs_in_place_of_split_weight_rows(dec, n, k, group, t):
+    test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, PAIR, PAIR)
