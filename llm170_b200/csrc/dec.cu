@@ -237,12 +237,22 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
     const bool rowgroup = tune_gemv_rowgroup > 0 && stock && !allreduce;
     auto choose_rowgroup = [&]() {
         const int forced = tune_gemv_rowgroup - 1;
-        if (!rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg)) {
-            return false;
+        const bool fits = rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg);
+        long long rows = 0;
+        for (int i = 0; i < a.nseg; ++i) {
+            rows += a.seg[i].n;
         }
-        // (up to the tickets that a decoder and the array of the allocation-free entry come with)
-        if (tune_gemv_rowgroup == 1 && c.grid_x <= 4096 &&
-            rg_leaves(a, c.rg, sk_make_plan(a.k, a.group, t, c.grid_x, sm_count, tune_gemv_sk_stages, tune_gemv_sk_prefetch), sm_count)) {
+        // (the persistent form: up to the tickets that a decoder and the array of the allocation-free entry come with)
+        const SkPlan sk = sk_make_plan(a.k, a.group, t, c.grid_x, sm_count, tune_gemv_sk_stages, tune_gemv_sk_prefetch);
+        const bool leaves = fits && tune_gemv_rowgroup == 1 && c.grid_x <= 4096 && rg_leaves(a, c.rg, sk, sm_count);
+        // x that does not fit, under rows enough: clusters (fewer rows leave them idle, and the persistent form deals K to all SMs)
+        bool clusters = false;
+        if (tune_gemv_rg_cluster > 1) {
+            clusters = rg_cluster_plan(a, ts_clusters[1], tune_gemv_rg_cluster, c.rg, 1e30);
+        } else if (!fits && tune_gemv_rowgroup == 1 && tune_gemv_rg_cluster == 0 && rows >= 3072) {
+            clusters = rg_cluster_plan(a, ts_clusters[1], 0, c.rg, sk.ctas > 0 && c.grid_x <= 4096 ? 0.95 * sk_estimate_us(sk, a.group, t, sm_count) : 1e30);
+        }
+        if (!clusters && (!fits || leaves)) {
             c.grid_x = gemv_plan_ctas(a);       // the segments' first blocks, which the plan counted in its own units
             return false;
         }
@@ -338,7 +348,7 @@ int Dec::gemv_run(GemvArgs& a, const GemvChoice& c, cudaStream_t st) {
     if (e != cudaSuccess) {
         return cuda_fail("launch gemv", e);
     }
-    last_kernel = c.form == GemvChoice::ROWGROUP ? gemv_rg_name(a.group, c.rg) : c.name;
+    last_kernel = c.form == GemvChoice::ROWGROUP ? gemv_rg_name(a.group, c.rg) + std::string(c.rg.split > 1 ? ", clusters of " + std::to_string(c.rg.split) : "") : c.name;
     launches++;
     return 0;
 }
@@ -744,6 +754,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
             return d.fail("w4a16 tuning: gemv_stages must be 2..8");
         }
         d.tune_gemv_stages = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemv_rg_cluster")) {
+        if (value < 0 || value > 8) {
+            return d.fail("w4a16 set_tuning: gemv_rg_cluster=%d (0..8)", value);
+        }
+        d.tune_gemv_rg_cluster = value;
         return 0;
     }
     if (!strcmp(key, "moe_gemm")) {

@@ -12,7 +12,8 @@
 //   * the loads of x and the zero-point MMAs are shared by NR row blocks, whose chains hide the latency of the MMAs (gemv_rg.cuh);
 //   * every warp streams its own tiles and scales into its own ring with asynchronous copies, requested before the dependency wait and
 //     refilled across units: no producer, no barrier in the loop, nothing of the copy engine, which takes 60 ns for each copy;
-//   * the warps' sums meet in shared memory once per unit; nothing is shared between CTAs.
+//   * the warps' sums meet in shared memory once per unit; nothing is shared between CTAs, but where x does not fit beside the rings (five to
+//     eight tokens of long K): there the CTAs of a cluster share K and add up in each other's shared memory (rg_cluster_plan).
 // One token, us per launch, this form against the best of the others: 7168 x 5120 6.6 / 7.2, 5120 x 6144 6.2 / 7.5, 34816 x 5120
 // 17.3 / 21.6 (5.3 TB/s), 5120 x 17408 13.0 / 13.8, 24576 x 4096 12.0 / 15.9; eight tokens: 7.4 / 10.3, 6.6 / 10.2, 20.5 / 26.2;
 // 34816 x 5120 in groups of 32, eight tokens: 21.7 / 48.9.
@@ -27,7 +28,9 @@ namespace w4 {
 namespace {
 
 // KW = warps along K; the other warps of a CTA take further row blocks.  NR = row blocks per warp, D = ring slots per warp.
-template <int GROUP, int KW, int NR, int D>
+// CL: the CTAs of a cluster share K as well, so that a unit's rows are spread over several SMs and each stages its part of x only; their sums
+// meet in distributed shared memory, in the order of their ranks.
+template <int GROUP, int KW, int NR, int D, bool CL>
 __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a, const RgPlan p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long s_xbar;
@@ -48,10 +51,12 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int g = lane >> 2, t = lane & 3;
     const int kw = warp % KW, rw = warp / KW;
+    const int cl = CL ? p.split : 1, rank = CL ? (int)blockIdx.x % cl : 0, cta = (int)blockIdx.x / cl, ctas = (int)gridDim.x / cl;
     // equal contiguous runs of units (row groups over all segments)
-    const int u0 = (int)((long long)p.units * blockIdx.x / gridDim.x), u1 = (int)((long long)p.units * (blockIdx.x + 1) / gridDim.x);
-    const int ku = a.k / (TILE_K * KPU), ng = a.k / GROUP;
-    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks
+    const int u0 = (int)((long long)p.units * cta / ctas), u1 = (int)((long long)p.units * (cta + 1) / ctas);
+    const int ku_all = a.k / (TILE_K * KPU), ng = a.k / GROUP;
+    const int ku0 = ku_all * rank / cl, ku = ku_all * (rank + 1) / cl - ku0;   // this CTA's part of K
+    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks, from there
     auto seg_of = [&](int u) {
         int si = 0;
 #pragma unroll
@@ -70,7 +75,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     RgCursor<GROUP, NR> cur;
     auto fetch_unit = [&]() {
         const int si = seg_of(fu), nrb = a.seg[si].n / TILE_ROWS;
-        cur.init(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, kb0, lane);
+        cur.init(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, ku0 * KPU + kb0, lane);
         fi = 0;
     };
     auto fetch = [&]() {
@@ -110,14 +115,14 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     stamp_now(1);
 
     // ---- activations: one bulk copy per token
-    const int m = a.m, xstride = a.k * 2 + RG_XPAD;
+    const int m = a.m, xbytes = ku * (KPU * TILE_K * 2), xstride = CL ? (ku_all + cl - 1) / cl * (KPU * TILE_K * 2) + RG_XPAD : a.k * 2 + RG_XPAD;
     if (warp == 0) {
         if (lane == 0) {
-            mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * a.k * 2));
+            mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * xbytes));
         }
         __syncwarp();
         if (lane < m) {
-            bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k, (uint32_t)(a.k * 2), smem_u32(&s_xbar));
+            bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k + ku0 * (KPU * TILE_K), (uint32_t)xbytes, smem_u32(&s_xbar));
         }
     }
     if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
@@ -155,12 +160,36 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
             }
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
-            const int tok = e / rows, row = e - tok * rows;
+        auto local_sum = [&](int tok, int row) {
             float v = red[row * mp + tok];
 #pragma unroll
             for (int w = 1; w < KW; ++w) {
                 v += red[(w * (UR * TILE_ROWS) + row) * mp + tok];      // fixed order: the same bits every run
+            }
+            return v;
+        };
+        int e0 = 0, e1 = rows * m;
+        // a CTA's sums for the others of its cluster, two units in turn: those of the unit before may still be read
+        const uint32_t part = smem_u32(smem) + (uint32_t)p.off_part + (uint32_t)((u - u0) & 1) * (UR * TILE_ROWS * GEMV_MAX_M * 4);
+        if (CL) {
+            for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
+                const int tok = e / rows;
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (uint32_t)e * 4u), "f"(local_sum(tok, e - tok * rows)) : "memory");
+            }
+            cluster_sync_all();
+            e0 = rows * m * rank / cl;
+            e1 = rows * m * (rank + 1) / cl;
+        }
+        for (int e = e0 + (int)threadIdx.x; e < e1; e += RG_THREADS) {
+            const int tok = e / rows, row = e - tok * rows;
+            float v;
+            if (CL) {
+                v = ld_dsmem_f32(part + (uint32_t)e * 4u, 0);
+                for (int c = 1; c < cl; ++c) {
+                    v += ld_dsmem_f32(part + (uint32_t)e * 4u, (unsigned)c);
+                }
+            } else {
+                v = local_sum(tok, row);
             }
             const size_t o = (size_t)tok * sg.n + (size_t)rb0 * TILE_ROWS + row;
             if (a.out_f16) {
@@ -170,26 +199,32 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
             }
         }
     }
+    if (CL) {
+        cluster_sync_all();                                   // nothing of this CTA's shared memory is still read
+    }
     stamp_now(5);   // sums stored
 }
 
 struct RgKernel {
     int group, kw, nr, depth;
+    bool cluster;
     const void* f;
     const char* name;
 };
-#define W4_RG(G, K, N, D) {G, K, N, D, (const void*)gemv_rg_kernel<G, K, N, D>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
-#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2), W4_RG(G, K, N, 4), W4_RG(G, K, N, 6)
+#define W4_RG(G, K, N, D, C) {G, K, N, D, C, (const void*)gemv_rg_kernel<G, K, N, D, C>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
+#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2, false), W4_RG(G, K, N, 4, false), W4_RG(G, K, N, 6, false), W4_RG(G, K, N, 2, true)
 #define W4_RG_N(G, K) W4_RG_D(G, K, 2), W4_RG_D(G, K, 3), W4_RG_D(G, K, 4)
 const RgKernel rg_kernels[] = {W4_RG_N(128, 4), W4_RG_N(128, 8), W4_RG_N(32, 4), W4_RG_N(32, 8)};
 #undef W4_RG_N
 #undef W4_RG_D
 #undef W4_RG
 const RgKernel& rg_kernel(int group, const RgPlan& p) {
-    return rg_kernels[(group == 128 ? 0 : 18) + (p.kw == 4 ? 0 : 9) + (p.nr - 2) * 3 + p.depth / 2 - 1];
+    return rg_kernels[(group == 128 ? 0 : 24) + (p.kw == 4 ? 0 : 12) + (p.nr - 2) * 4 + (p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
 }
 
 constexpr int RG_SMEM_MAX = 224 * 1024, RG_SMEM_TWO = 112 * 1024;
+// us per k-block of two, three, four row blocks: a CTA alone on its SM, two; groups of 128, of 32
+constexpr double RG_STEP_US[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.437}}, {{0.44, 0.53, 0.64}, {0.49, 0.60, 0.742}}};
 
 }  // namespace
 
@@ -212,6 +247,7 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
             RgPlan p{};
             p.nr = nr;
             p.kw = kw;
+            p.split = 1;
             for (int i = 0; i < a.nseg; ++i) {
                 p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
             }
@@ -251,6 +287,19 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
     return true;
 }
 
+// Estimated time of a plan, K from 8192 on.
+static double rg_us(const GemvArgs& a, const RgPlan& p, int sm_count) {
+    const bool g32 = a.group == 32, two = p.smem <= RG_SMEM_TWO;
+    const int unit_k = a.group > TILE_K ? a.group : TILE_K, chain = (a.k / unit_k + p.kw - 1) / p.kw * (unit_k / TILE_K);
+    const int rounds = (p.units + p.ctas - 1) / p.ctas;
+    const double step = RG_STEP_US[two][g32][p.nr - 2] + (!two && p.depth == 2 ? (p.nr == 2 ? 0.085 : 0.04) : 0.0);
+    double us = 2.0 + rounds * (1.0 + step * chain);
+    if (rounds == 1 && 2 * p.units <= sm_count) {
+        us -= 0.95 + (g32 ? 0.0 : 0.012 * chain);            // no two CTAs on neighbouring SMs
+    }
+    return us;
+}
+
 // Three corners where the row-group form is not the best one.  All figures on B200, us per launch, this form / the other.
 //   * Long K: a warp walks its part of K serially (0.25 us per k-block of two row blocks), and where few units are left or x leaves room for
 //     two slots of two row blocks only, the persistent form, which deals K to all SMs, is sooner: 1024 x 28672 15.0 / 10.4, 1024 x 17408
@@ -263,7 +312,7 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
 //   * Hardly any K under many rows, five tokens and more: a unit's sums cost as much as its tiles.  128 channels, eight tokens: 16384 rows
 //     3.4 / 3.0, 34816 rows 4.0 / 3.2, 12288 rows 2.9 / 2.8; 256 channels, 34816 rows 4.8 / 4.3, 24576 rows 0.96.
 bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_count) {
-    const bool g32 = a.group == 32, two = p.smem <= RG_SMEM_TWO;
+    const bool g32 = a.group == 32;
     const int unit_k = a.group > TILE_K ? a.group : TILE_K, chain = (a.k / unit_k + p.kw - 1) / p.kw * (unit_k / TILE_K);
     const int rounds = (p.units + p.ctas - 1) / p.ctas;
     long long rows = 0;
@@ -271,13 +320,7 @@ bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_coun
         rows += a.seg[i].n;
     }
     if (a.k >= 8192) {
-        static const double tau[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.437}}, {{0.44, 0.53, 0.64}, {0.49, 0.60, 0.742}}};
-        const double step = tau[two][g32][p.nr - 2] + (!two && p.depth == 2 ? (p.nr == 2 ? 0.085 : 0.04) : 0.0);
-        double us = 2.0 + rounds * (1.0 + step * chain);
-        if (rounds == 1 && 2 * p.units <= sm_count) {
-            us -= 0.95 + (g32 ? 0.0 : 0.012 * chain);        // no two CTAs on neighbouring SMs
-        }
-        return us > sk_estimate_us(sk, a.group, a.m, sm_count);
+        return rg_us(a, p, sm_count) > sk_estimate_us(sk, a.group, a.m, sm_count);
     }
     if (a.m <= 2 && rows <= 4096 && p.nr == 2 && p.kw == RG_WARPS && rounds == 1 && gemv_ru_fits(a, sm_count)) {
         const double mb = 0.5e-6 * (double)rows * a.k, over = mb > 4.0 ? mb - 4.0 : 0.0;
@@ -286,6 +329,63 @@ bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_coun
         return 1.49 + 0.22 * chain + (2 * p.units > sm_count ? 0.33 : 0.0) + 0.058 * mb > ru + 0.1;
     }
     return a.m >= 5 && rows * 8 > (long long)a.k * (a.m >= 7 ? 880 : 2667) * (g32 ? 2 : 1);
+}
+
+// The row-group form over clusters, two CTAs per SM, for activations that do not fit beside a ring: every CTA stages its part of K.  us per
+// launch, the persistent form / clusters of the size chosen: 4096 x 14336 at eight tokens 18.4 / 11.4 (groups of 32 20.2 / 12.3), 5120 x 17408 at
+// six to eight 18.0 / 14.8, 18.6 / 15.2, 18.9 / 15.4 (21.4 / 16.2), 5632 x 20224 at five 20.8 / 16.8, 8192 x 28672 at eight 38.2 / 36.1 (52.2 /
+// 39.6).  Where the activations fit, a CTA alone on its SM with all of K is as fast or faster (5120 x 17408, one token: 13.6 / 14.0; 5120 x 8704
+// 8.1 / 8.8): what the barriers of a cluster take, about 1.2 us, is what the better balance brings.  `clusters`: how many of 1..8 whole-SM CTAs
+// can be resident; of half-SM CTAs at least twice as many.  `us`: the time to beat, estimated as in rg_us.
+bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& best, double us) {
+    const int unit_k = a.group > TILE_K ? a.group : TILE_K, ku = a.k / unit_k, mp = (a.m + 1) & ~1;
+    bool found = false;
+    for (int cl = 2; cl <= 8 && cl <= ku; ++cl) {
+        if (force_split > 0 && cl != force_split) {
+            continue;
+        }
+        const int x_bytes = (a.m * ((ku + cl - 1) / cl * unit_k * 2 + RG_XPAD) + 127) & ~127;
+        for (int kw : {4, 8}) {
+            for (int nr : {4, 3, 2}) {
+                const int ur = RG_WARPS / kw * nr, slot = rg_slot_bytes(a.group, nr);
+                RgPlan p{};
+                p.nr = nr;
+                p.kw = kw;
+                p.split = cl;
+                for (int i = 0; i < a.nseg; ++i) {
+                    p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
+                }
+                p.off_red = x_bytes;
+                p.off_part = (x_bytes + kw * ur * TILE_ROWS * mp * 4 + 127) & ~127;
+                p.off_ring = (p.off_part + 2 * ur * TILE_ROWS * GEMV_MAX_M * 4 + 127) & ~127;
+                const int room = 2 * clusters[cl];
+                if (room <= 0 || p.off_ring + 2 * RG_WARPS * slot > RG_SMEM_TWO) {
+                    continue;
+                }
+                p.depth = 2;                                  // (four slots, where they fit, were not faster: 4096 x 14336 11.9 / 11.4 us)
+                p.smem = p.off_ring + p.depth * RG_WARPS * slot;
+                const int at_once = std::min(p.units, room), rounds = (p.units + at_once - 1) / at_once;
+                p.ctas = at_once * cl;
+                // (fitted to 28 launches of 3072 to 24576 rows, 4 % on average: the sums of eight warps take longer)
+                const double step = RG_STEP_US[1][a.group == 32][nr - 2] * 1.25;
+                const double c = 3.3 + rounds * ((kw == 8 ? 2.2 : 1.4) + step * (((ku + cl - 1) / cl + kw - 1) / kw * (unit_k / TILE_K)));
+                if (c < us) {
+                    us = c;
+                    best = p;
+                    found = true;
+                }
+            }
+        }
+    }
+    if (found) {
+        const int ur = RG_WARPS / best.kw * best.nr;
+        int units = 0;
+        for (int i = 0; i < a.nseg; ++i) {
+            a.seg[i].cta0 = units;
+            units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
+        }
+    }
+    return found;
 }
 
 const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(group, p).name; }
@@ -306,13 +406,22 @@ cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st) 
     cfg.blockDim = dim3(RG_THREADS);
     cfg.dynamicSmemBytes = p.smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    int n_attr = 0;
     if (a.pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
+        ++n_attr;
     }
+    if (p.split > 1) {
+        attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+        attr[n_attr].val.clusterDim.x = p.split;
+        attr[n_attr].val.clusterDim.y = 1;
+        attr[n_attr].val.clusterDim.z = 1;
+        ++n_attr;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n_attr;
     void* args[] = {const_cast<GemvArgs*>(&a), const_cast<RgPlan*>(&p)};
     return cudaLaunchKernelExC(&cfg, rg_kernel(a.group, p).f, args);
 }

@@ -151,10 +151,13 @@ struct RgPlan {
     int units;               // row groups over all segments (seg[].cta0 = first of the segment)
     int ctas;                // CTA c takes units [units c / ctas, units (c + 1) / ctas)
     int depth;               // ring slots per warp
-    int off_red, off_ring;   // byte offsets in dynamic shared memory: activations first
+    int split;               // CTAs of a cluster that share K (1: none)
+    int off_red, off_part, off_ring;   // byte offsets in dynamic shared memory: activations first
     int smem;
 };
 bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& p);
+// A plan over clusters that is estimated to take less than `us` (false: none); fills seg[].cta0.
+bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& p, double us);
 // Whether another form is estimated to finish the call sooner than this plan; `sk`: the persistent form's plan.
 bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_count);
 cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st);

@@ -604,6 +604,42 @@ def test_row_group_form_leaves_what_does_not_fit(dec, orc):
     dec.drop_lin("rgx")
 
 
+# The row-group form over clusters: K that does not divide by the CTAs or their warps (one has no k-blocks), odd numbers of k-blocks, units that the last
+# rows do not fill, more units than clusters, several linears at once, one to eight tokens, every group size -- and x that does not fit, by itself
+@pytest.mark.parametrize("n,k,group,t,cl", [(16, 256, 128, 1, 2), (272, 704, 32, 3, 5), (1040, 1152, 64, 8, 8), (528, 4992, 128, 5, 7), (20000, 512, 128, 2, 3),
+                                            (2064, 2048, 32, 8, 6), (3200, 14336, 128, 8, 0), (3088, 14400, 64, 8, 0)])
+def test_row_group_form_over_clusters(dec, orc, n, k, group, t, cl):
+    q, s = synth.make_linear(n, k, group, seed=990 + n % 97)
+    dec.upload_lin_g("rgc", q, s, n, k, group)
+    xs = synth.make_acts(t, k, seed=991 + t)
+    guard = torch.full((t + 1, n), 7.0, device="cuda", dtype=torch.float32)
+    dec.set_tuning("gemv_rg_cluster", cl)
+    try:
+        for _ in range(2):
+            dec.lin_forward("rgc", x_dev(xs), t, dst=guard[:t])
+            assert dec.last_kernel().startswith("gemv_rg_kernel") and "clusters of" in dec.last_kernel()
+            dec.sync()
+            y = guard[:t].clone()
+        assert torch.equal(dec.lin_forward("rgc", x_dev(xs), t, out_f16=True), y.to(torch.float16))
+        outs = dec.sk_multi_dev(["rgc", "rgc"], x_dev(xs), t=t)
+        assert "clusters of" in dec.last_kernel()
+        assert torch.equal(outs[0], outs[1])
+        dec.set_tuning("gemv_rg_cluster", 1)
+        other = dec.lin_forward("rgc", x_dev(xs), t)
+        assert "clusters of" not in dec.last_kernel()
+    finally:
+        dec.set_tuning("gemv_rg_cluster", 0)
+    rows = (0, n) if n < 1024 else (n - 512, n)
+    expect = orc.linear_lane(q, s, xs, t, n, k, group, rows=rows)
+    size = (x_dev(xs).float().abs() @ dec.dequant_lin("rgc").abs().T).max().item()
+    # f32 sums in another order, as in the tests of the corners
+    assert np.abs(y.cpu().numpy()[:, rows[0]:rows[1]] - expect[:, rows[0]:rows[1]]).max() <= 2.0 ** -18 * size
+    # (several linears at once have more units, and with them another split of K over the warps)
+    assert max((y - v).abs().max().item() for v in (other, outs[0])) <= 2.0 ** -18 * size
+    assert bool((guard[t:] == 7.0).all())
+    dec.drop_lin("rgc")
+
+
 # a tuning key moves a call to the form that it tunes, also where the row-group form would run
 @pytest.mark.parametrize("key,value,default,k,t,form", [
     ("gemv_stages", 3, 4, 2048, 8, "gemv_w4a16_kernel"), ("gemv_warps", 16, 8, 2048, 8, "gemv_w4a16_kernel"), ("gemv_sk_stages", 3, 4, 6272, 2, "gemv_sk_kernel"),
