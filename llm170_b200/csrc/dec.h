@@ -29,10 +29,13 @@ struct MoeCfg {
     int e0 = 0, e1 = 0;  // experts [e0, e1) are resident on this decoder (expert parallelism)
 };
 
+constexpr int MOE_CNT_STRIDE = 8;   // ints between the counters of two experts: a sector of L2 each
+
 struct MoeBufs {
     int* idx = nullptr;          // [slots] expert of each (token, j) slot
     float* wt = nullptr;         // [slots] routing weight
-    int *cnt = nullptr, *off = nullptr, *cursor = nullptr;  // [n_experts]
+    int* cnt = nullptr;          // [n_experts][MOE_CNT_STRIDE]
+    int* off = nullptr;          // [n_experts]
     int *pos_of_slot = nullptr, *slot_of_pos = nullptr;     // [slots]
     int *tile_expert = nullptr, *tile_row0 = nullptr, *tile_rows = nullptr;  // [max_tiles]
     int *n_tiles = nullptr, *n_rows = nullptr;

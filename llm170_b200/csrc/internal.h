@@ -194,7 +194,8 @@ struct MoeBufs;
 enum { TILES_FULL = 0, TILES_EVEN = 1, TILES_SORTED = 2 };
 // All return the first launch error and launch nothing after it.  `pdl`: programmatic stream serialization.  `cnt` (optional): counts the
 // rows of local experts [e0, e1) as well.  `launched`: raised by the number of launches.
-cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl, cudaStream_t st);
+cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int* rank, int e0, int e1, int pdl,
+                            cudaStream_t st);
 // routing and sorting of any batch: top-k and histogram -> offsets and m-tile table (tiles of at most `bm` rows, cut as `shares` says) ->
 // placement of the local experts' slots and gather of their token rows.  Wants b.cnt at zero and leaves it so; after an
 // error it may hold counts.

@@ -8,7 +8,7 @@
 // placement that replace the single-block counting sort (crates/backend-gpu/src/rawcuda/assets/gptq4.cu:376-413,
 // crates/backend-gpu/src/rawcuda/assets/moe.cu:1599-1633), the row gather and the top-k sum
 // (crates/backend-gpu/src/rawcuda/assets/moe.cu:1662-1674); the activation (:1649-1660) is in the first matmul's epilogue.
-// Slots of one expert are placed with an atomic cursor, so their order inside an expert's segment is
+// Slots of one expert are placed in the order in which they were counted, so their order inside an expert's segment is
 // not fixed; every output row is computed independently and the final sum runs over k in index order,
 // so results do not depend on that order.
 #include <cuda_fp16.h>
@@ -41,22 +41,27 @@ constexpr int TOPK_WARPS = 8;
 // lane (independent loads, one dependent add each) instead of travelling through n dependent shuffles.
 // SLOTS = experts per lane the instantiation can hold (n <= 32 * SLOTS): a compile-time bound keeps the lane's values in
 // registers.
+// Returns the lane's pick: lane r < k has the r-th one.
 template <int SLOTS>
-__device__ __forceinline__ void topk_of_token_n(const float* l, int* idx, float* wt,
-                                                int n, int k, int lane, float* stage) {
-    float mx = -INFINITY;
-    for (int i = lane; i < n; i += 32) {
-        mx = fmaxf(mx, l[i]);
+__device__ __forceinline__ int topk_of_token_n(const float* l, int* idx, float* wt,
+                                               int n, int k, int lane, float* stage) {
+    float mx = -INFINITY, pv[SLOTS];
+    const int cnt = (n - lane + 31) >> 5;   // experts lane, lane + 32, ... below n
+#pragma unroll
+    for (int j = 0; j < SLOTS; ++j) {
+        pv[j] = j < cnt ? l[lane + 32 * j] : -INFINITY;
+    }
+#pragma unroll
+    for (int j = 0; j < SLOTS; ++j) {
+        mx = fmaxf(mx, pv[j]);
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
     }
-    float pv[SLOTS];
-    const int cnt = (n - lane + 31) >> 5;   // experts lane, lane + 32, ... below n
 #pragma unroll
     for (int j = 0; j < SLOTS; ++j) {
-        pv[j] = j < cnt ? (float)exp((double)(l[lane + 32 * j] - mx)) : 0.f;
+        pv[j] = j < cnt ? (float)exp((double)(pv[j] - mx)) : 0.f;
     }
     // sum in index order, the same on every lane: element e = 32*j + src comes from lane src, slot j
     float sum = 0.f;
@@ -103,7 +108,8 @@ __device__ __forceinline__ void topk_of_token_n(const float* l, int* idx, float*
     }
     unsigned used = 0u;
     float wsum = 0.f;
-    float mine = 0.f;  // lane r keeps the r-th picked p
+    float mine = 0.f;  // lane r keeps the r-th picked p and its expert
+    int mine_e = 0;
     for (int r = 0; r < k; ++r) {
         unsigned best = 0u;   // bit pattern of the lane's largest remaining p (p >= 0: patterns order like values)
 #pragma unroll
@@ -124,29 +130,28 @@ __device__ __forceinline__ void topk_of_token_n(const float* l, int* idx, float*
         if ((bi & 31) == lane) {
             used |= 1u << (bi >> 5);
         }
-        if (lane == 0) {
-            idx[r] = bi;
-        }
         const float bv = __uint_as_float(top);
         if (lane == (r & 31)) {
             mine = bv;
+            mine_e = bi;
         }
         wsum += bv;
     }
     if (lane < k) {
         wt[lane] = mine / wsum;
+        idx[lane] = mine_e;
     }
+    return mine_e;
 }
 
-__device__ __forceinline__ void topk_of_token(const float* l, int* idx, float* wt,
-                                              int n, int k, int lane, float* stage = nullptr) {
+__device__ __forceinline__ int topk_of_token(const float* l, int* idx, float* wt,
+                                             int n, int k, int lane, float* stage = nullptr) {
     if (n <= 128) {
-        topk_of_token_n<4>(l, idx, wt, n, k, lane, stage);
+        return topk_of_token_n<4>(l, idx, wt, n, k, lane, stage);
     } else if (n <= 256) {
-        topk_of_token_n<8>(l, idx, wt, n, k, lane, stage);
-    } else {
-        topk_of_token_n<32>(l, idx, wt, n, k, lane, stage);
+        return topk_of_token_n<8>(l, idx, wt, n, k, lane, stage);
     }
+    return topk_of_token_n<32>(l, idx, wt, n, k, lane, stage);
 }
 
 // Rows per tile of an expert with c rows: `bm` of them, or (`even`) equal shares of at most bm, in multiples of 16 rows.
@@ -158,8 +163,11 @@ __device__ __forceinline__ int tile_step(int c, int bm, int even) {
     return ((c + nt - 1) / nt + 15) & ~15;
 }
 
-// `cnt` (optional): rows per local expert; zero on entry, moe_offsets_kernel leaves it so.
-__global__ void moe_topk_kernel(const float* lg, int* idx, float* wt, int t, int n, int k, int stage_rows, int* cnt, int e0, int e1) {
+// `cnt` (optional): rows per local expert, MOE_CNT_STRIDE apart; zero on entry, moe_offsets_kernel leaves it so.  What a slot's count was before
+// it is its place in the expert's segment (`rank`): the gather asks for no place of its own.
+// What bounds it at a prefill's sizes is the counting: 32768 atomics on 128 neighbouring words queued up in four lines of L2.  A sector for every
+// counter and no second pass of atomics: layers of 512 tokens 124.9 -> 120.8 us, of 4096 354 -> 347 (with the sums below).
+__global__ void moe_topk_kernel(const float* lg, int* idx, float* wt, int t, int n, int k, int stage_rows, int* cnt, int* rank, int e0, int e1) {
     extern __shared__ __align__(16) float s_stage[];   // [warps][n] when the launch provides it
     pdl_begin();
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -167,16 +175,10 @@ __global__ void moe_topk_kernel(const float* lg, int* idx, float* wt, int t, int
     if (ti >= t) {
         return;
     }
-    topk_of_token(lg + (size_t)ti * n, idx + (size_t)ti * k, wt + (size_t)ti * k, n, k, lane,
-                  stage_rows ? s_stage + (size_t)w * n : nullptr);
-    if (cnt != nullptr) {
-        __syncwarp();
-        if (lane < k) {                                                  // k <= 32
-            const int e = idx[(size_t)ti * k + lane];
-            if (e >= e0 && e < e1) {
-                atomicAdd(cnt + e, 1);
-            }
-        }
+    const int e = topk_of_token(lg + (size_t)ti * n, idx + (size_t)ti * k, wt + (size_t)ti * k, n, k, lane,
+                                stage_rows ? s_stage + (size_t)w * n : nullptr);
+    if (cnt != nullptr && lane < k && e >= e0 && e < e1) {               // k <= 32
+        rank[(size_t)ti * k + lane] = atomicAdd(cnt + e * MOE_CNT_STRIDE, 1);
     }
 }
 
@@ -227,7 +229,7 @@ moe_route_small_kernel(const float* lg, int* idx, float* wt,
                        int* tile_expert, int* tile_row0, int* tile_rows,
                        int* n_tiles, int* n_rows, float* row_w, int t, int n_exp,
                        int k, int e0, int e1, int bm, int stage_rows, int do_topk) {
-    __shared__ int s_rows[1024], s_off[1024], s_cursor[1024], s_wr[32], s_wt[32];
+    __shared__ int s_rows[1024], s_off[1024], s_cursor[1024], s_wr[32], s_wt[32], s_idx[8 * 32];
     extern __shared__ __align__(16) float s_stage[];   // [32 warps][n_exp] when the launch provides it
     const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     s_rows[tid] = 0;
@@ -235,15 +237,18 @@ moe_route_small_kernel(const float* lg, int* idx, float* wt,
     pdl_begin();
     if (do_topk) {   // a handful of tokens: routed here; more: routed by moe_topk_kernel on many SMs just before
         for (int ti = w; ti < t; ti += 32) {
-            topk_of_token(lg + (size_t)ti * n_exp, idx + (size_t)ti * k, wt + (size_t)ti * k, n_exp, k, lane,
-                          stage_rows ? s_stage + (size_t)w * n_exp : nullptr);
+            const int e = topk_of_token(lg + (size_t)ti * n_exp, idx + (size_t)ti * k, wt + (size_t)ti * k, n_exp, k, lane,
+                                        stage_rows ? s_stage + (size_t)w * n_exp : nullptr);
+            if (lane < k) {
+                s_idx[ti * k + lane] = e;                                // t <= 8, k <= 32
+            }
         }
     }
     __syncthreads();   // idx / wt of every token are visible to the block
     const int ns = t * k;
     int my_e = -1;
     if (tid < ns) {
-        my_e = idx[tid];
+        my_e = do_topk ? s_idx[tid] : idx[tid];
         if (my_e >= e0 && my_e < e1) {
             atomicAdd(&s_rows[my_e], 1);
         } else {
@@ -284,15 +289,15 @@ moe_route_small_kernel(const float* lg, int* idx, float* wt,
 // How an expert's rows are cut into tiles: of bm rows with a remainder, in equal shares of at most bm (multiples of 16), or like the first
 // but with the table sorted.  Persistent CTAs take tiles in turn: sorted, no CTA gets more of the large ones than another.
 // One block of 1024 threads (n_exp <= 1024): exclusive offsets of the local experts' segments and the m-tile
-// table of the grouped GEMM, tile i -> (expert, first sorted row, valid rows).  Also clears the placement cursors and the counts.
+// table of the grouped GEMM, tile i -> (expert, first sorted row, valid rows).  Also clears the counts.
 __global__ void __launch_bounds__(1024)
-moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_row0, int* tile_rows, int* n_tiles, int* n_rows,
+moe_offsets_kernel(int* cnt, int* off, int* tile_expert, int* tile_row0, int* tile_rows, int* n_tiles, int* n_rows,
                    int n_exp, int e0, int e1, int bm, int shares) {
     __shared__ int s_r[32], s_t[32];
     __shared__ __align__(16) int s_rest[1024];
     const int e = threadIdx.x;
     pdl_begin();
-    const int c = (e >= e0 && e < e1) ? cnt[e] : 0;
+    const int c = (e >= e0 && e < e1) ? cnt[e * MOE_CNT_STRIDE] : 0;
     const int step = tile_step(c, bm, shares == TILES_EVEN), rest = shares == TILES_SORTED ? c % bm : 0;
     const int ct = shares == TILES_SORTED ? c / bm : (c + step - 1) / step;
     int vr = c, vt = ct, total_rows, total_tiles;
@@ -317,8 +322,7 @@ moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_
     }
     if (e < n_exp) {
         off[e] = row0;
-        cursor[e] = 0;
-        cnt[e] = 0;
+        cnt[e * MOE_CNT_STRIDE] = 0;
     }
     for (int r = 0, i = tile0; r < c - rest; r += step, ++i) {
         tile_expert[i] = e;
@@ -337,7 +341,7 @@ moe_offsets_kernel(int* cnt, int* off, int* cursor, int* tile_expert, int* tile_
 // 4 KB, cold: 39 us with a thread per 16 bytes of a slot, 33 with a warp per token, 31 so).
 constexpr int GATHER_THREADS = 128;
 __global__ void __launch_bounds__(GATHER_THREADS)
-moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* wt, const int* off, int* cursor, int* pos_of_slot,
+moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* wt, const int* off, int* pos_of_slot,
                         int* slot_of_pos, float* row_w, int t, int k, int h8, int e0, int e1) {
     __shared__ int s_pos[32];                                                        // k <= 32
     pdl_begin();
@@ -346,7 +350,7 @@ moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* 
             const int slot = tok * k + (int)threadIdx.x, e = idx[slot];
             int pos = -1;                                                            // the expert lives on another rank
             if (e >= e0 && e < e1) {
-                pos = off[e] + atomicAdd(cursor + e, 1);
+                pos = off[e] + pos_of_slot[slot];                                     // (its rank so far)
                 slot_of_pos[pos] = slot;
                 row_w[pos] = wt[slot];
             }
@@ -372,7 +376,9 @@ moe_place_gather_kernel(const uint4* x, uint4* xs, const int* idx, const float* 
 }
 
 // out[t][c] = sum_j c2[pos(t*k+j)][c]  (routing weights were applied in GEMM-2's epilogue); slots whose
-// expert is not local contribute nothing
+// expert is not local contribute nothing.  The rows of eight slots are on their way at once:
+// a slot after the other, each took two trips to memory, about 2 us of a decode call (a layer of one token 22.8 -> 20.7 us, of eight 50.1 -> 47.3).
+constexpr int COMBINE_AHEAD = 8;
 template <bool OUT_F16>
 __global__ void moe_combine_kernel(const __half* c2, void* out, const int* pos_of_slot,
                                    int t, int h, int k) {
@@ -382,16 +388,29 @@ __global__ void moe_combine_kernel(const __half* c2, void* out, const int* pos_o
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const int r = (int)(i / h8), c = (int)(i % h8) * 8;
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int j = 0; j < k; ++j) {
-            const int pos = pos_of_slot[r * k + j];
-            if (pos >= 0) {
-                const uint4 v = *reinterpret_cast<const uint4*>(c2 + (size_t)pos * h + c);
-                const __half2* vh = reinterpret_cast<const __half2*>(&v);
+        for (int j0 = 0; j0 < k; j0 += COMBINE_AHEAD) {
+            int pos[COMBINE_AHEAD];
+            uint4 v[COMBINE_AHEAD];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const float2 f = __half22float2(vh[q]);
-                    acc[2 * q] += f.x;
-                    acc[2 * q + 1] += f.y;
+            for (int j = 0; j < COMBINE_AHEAD; ++j) {
+                pos[j] = j0 + j < k ? pos_of_slot[r * k + j0 + j] : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < COMBINE_AHEAD; ++j) {
+                if (pos[j] >= 0) {
+                    v[j] = *reinterpret_cast<const uint4*>(c2 + (size_t)pos[j] * h + c);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < COMBINE_AHEAD; ++j) {
+                if (pos[j] >= 0) {
+                    const __half2* vh = reinterpret_cast<const __half2*>(&v[j]);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float2 f = __half22float2(vh[q]);
+                        acc[2 * q] += f.x;
+                        acc[2 * q + 1] += f.y;
+                    }
                 }
             }
         }
@@ -442,11 +461,11 @@ cudaError_t launch(void (*kernel)(P...), int grid, int block, size_t smem, cudaS
 
 }  // namespace
 
-cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int e0, int e1, int pdl,
-                            cudaStream_t st) {
+cudaError_t launch_moe_topk(const float* logits, int* idx, float* wt, int t, int n_exp, int k, int* cnt, int* rank, int e0, int e1,
+                            int pdl, cudaStream_t st) {
     const int stage = n_exp <= 512;   // 8 warps x 512 floats = 16 KB of shared memory at most
     return launch(moe_topk_kernel, (t + TOPK_WARPS - 1) / TOPK_WARPS, TOPK_WARPS * 32, stage ? TOPK_WARPS * n_exp * sizeof(float) : 0, st,
-                  pdl, logits, idx, wt, t, n_exp, k, stage, cnt, e0, e1);
+                  pdl, logits, idx, wt, t, n_exp, k, stage, cnt, rank, e0, e1);
 }
 
 // Up to eight tokens are routed by the table block itself (one launch); above that one block's 32 warps would route two or more tokens
@@ -457,7 +476,7 @@ cudaError_t launch_moe_route_small(const float* logits, const MoeBufs& b, int t,
     const int own_topk = t <= 8;
     cudaError_t e = cudaSuccess;
     if (!own_topk) {
-        e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, nullptr, 0, 0, pdl, st);
+        e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, nullptr, nullptr, 0, 0, pdl, st);
         launched += e == cudaSuccess;
     }
     if (e == cudaSuccess) {
@@ -471,19 +490,19 @@ cudaError_t launch_moe_route_small(const float* logits, const MoeBufs& b, int t,
 
 cudaError_t launch_moe_sort(const float* logits, const void* x, const MoeBufs& b, int t, int n_exp, int k, int h, int e0, int e1, int bm,
                             int shares, int pdl, cudaStream_t st, unsigned long long& launched) {
-    cudaError_t e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, e0, e1, pdl, st);
+    cudaError_t e = launch_moe_topk(logits, b.idx, b.wt, t, n_exp, k, b.cnt, b.pos_of_slot, e0, e1, pdl, st);
     if (e != cudaSuccess) {
         return e;
     }
     ++launched;
-    e = launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.cursor, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
+    e = launch(moe_offsets_kernel, 1, 1024, 0, st, pdl, b.cnt, b.off, b.tile_expert, b.tile_row0, b.tile_rows, b.n_tiles, b.n_rows,
                n_exp, e0, e1, bm, shares);
     if (e != cudaSuccess) {
         return e;
     }
     ++launched;
     e = launch(moe_place_gather_kernel, blocks_for((size_t)t, 1), GATHER_THREADS, 0, st, pdl, (const uint4*)x, (uint4*)b.xs, b.idx, b.wt,
-               b.off, b.cursor, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
+               b.off, b.pos_of_slot, b.slot_of_pos, b.row_w, t, k, h / 8, e0, e1);
     launched += e == cudaSuccess;
     return e;
 }

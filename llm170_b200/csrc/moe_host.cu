@@ -25,7 +25,7 @@ cudaError_t dalloc(T** p, size_t count) {
 
 // `retire`: keep the blocks until the decoder is freed (a captured graph may still name them)
 void Dec::free_moe(bool retire) {
-    void* ptrs[] = {mb.idx, mb.wt, mb.cnt, mb.off, mb.cursor, mb.pos_of_slot, mb.slot_of_pos, mb.tile_expert, mb.tile_row0,
+    void* ptrs[] = {mb.idx, mb.wt, mb.cnt, mb.off, mb.pos_of_slot, mb.slot_of_pos, mb.tile_expert, mb.tile_row0,
                     mb.tile_rows, mb.n_tiles, mb.n_rows, mb.row_w, mb.xs, mb.c13, mb.act, mb.c2};
     for (void* p : ptrs) {
         if (p) {
@@ -59,9 +59,8 @@ int Dec::ensure_moe(int t, cudaStream_t st) {
     };
     ok(dalloc(&mb.idx, slots));
     ok(dalloc(&mb.wt, slots));
-    ok(dalloc(&mb.cnt, (size_t)moe.n_experts));
+    ok(dalloc(&mb.cnt, (size_t)moe.n_experts * MOE_CNT_STRIDE));
     ok(dalloc(&mb.off, (size_t)moe.n_experts));
-    ok(dalloc(&mb.cursor, (size_t)moe.n_experts));
     ok(dalloc(&mb.pos_of_slot, slots));
     ok(dalloc(&mb.slot_of_pos, slots));
     ok(dalloc(&mb.tile_expert, (size_t)max_tiles));
@@ -75,7 +74,7 @@ int Dec::ensure_moe(int t, cudaStream_t st) {
     ok(cudaMalloc(&mb.act, slots * moe.ffn * 2));
     ok(cudaMalloc(&mb.c2, slots * moe.hidden * 2));
     if (e == cudaSuccess) {
-        e = fill_now(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int), st);   // the counts of a call are left at zero by it
+        e = fill_now(mb.cnt, 0, (size_t)moe.n_experts * MOE_CNT_STRIDE * sizeof(int), st);   // the counts of a call are left at zero by it
     }
     if (e != cudaSuccess) {
         free_moe();
@@ -154,7 +153,7 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         e = launch_moe_sort(logits, x16, mb, t, moe.n_experts, moe.top_k, moe.hidden, moe.e0, moe.e1, bm, shares, tune_pdl, st, launches);
         // The top-k may have counted, with nothing after it that clears the counts for the next call; where they cannot be cleared, that
         // call makes its scratch anew.
-        if (e != cudaSuccess && cudaMemsetAsync(mb.cnt, 0, (size_t)moe.n_experts * sizeof(int), st) != cudaSuccess) {
+        if (e != cudaSuccess && cudaMemsetAsync(mb.cnt, 0, (size_t)moe.n_experts * MOE_CNT_STRIDE * sizeof(int), st) != cudaSuccess) {
             mb.cap_tokens = 0;
         }
         return e == cudaSuccess ? 0 : cuda_fail("moe_ffn launch", e);
@@ -322,7 +321,7 @@ int w4a16_moe_topk(w4a16_dec* dec, const float* logits_dev, int* idx_dev, float*
         return d.fail("w4a16 moe_topk: set_moe was not called");
     }
     const cudaError_t e =
-        w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, nullptr, 0, 0, d.tune_pdl, moe_stream(dec, stream));
+        w4::launch_moe_topk(logits_dev, idx_dev, wt_dev, t, d.moe.n_experts, d.moe.top_k, nullptr, nullptr, 0, 0, d.tune_pdl, moe_stream(dec, stream));
     if (e != cudaSuccess) {
         return d.cuda_fail("moe_topk", e);
     }

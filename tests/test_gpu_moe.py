@@ -335,3 +335,26 @@ def test_expert_tiles_on_pairs(dec, orc, tile, f, h, group, local):
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, 1, group)
     err = np.abs(total - want).max()
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the tests above
+
+
+# The small kernels around the matmuls: numbers of picks below, at and past the eight rows that the sum has on the way, with counts by the block of the
+# small tables (3 and 40 tokens) and by the routing itself (300 tokens), all experts or the second half of them here; twice, as each call counts from zero
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 17, 32])
+@pytest.mark.parametrize("t", [3, 40, 300])
+@pytest.mark.parametrize("e0", [0, 20])
+def test_any_number_of_picks(dec, orc, k, t, e0):
+    n_exp, f, h, group = 40, 64, 128, 32
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=83)
+    if e0:                                                       # an expert elsewhere adds nothing: the oracle gets zeros for it
+        w2_s = w2_s.copy()
+        w2_s.reshape(n_exp, -1)[:e0] = 0
+    x = synth.make_acts(t, h, seed=84)
+    lg = np.random.Generator(np.random.PCG64(85)).standard_normal((t, n_exp)).astype(np.float32)
+    dec.set_moe(n_exp, k, f, h, group, e0, n_exp - e0)
+    dec.upload_experts(0, w13_q[e0:], w13_s[e0:], w2_q[e0:], w2_s[e0:])
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+    assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
+    err = np.abs(y.cpu().numpy() - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the tests above
