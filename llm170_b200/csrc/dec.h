@@ -112,6 +112,7 @@ struct Dec {
     int tune_gemm_ksplit = 0;    // K splits of the GEMM: 0 = automatic (only when the tiles do not fill the SMs)
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
     int tune_gemm_pair = 0;      // CTA pairs (gemm_ts2.cu): 0 = automatic, 1 = never, 32..256 = always, with tiles of that many tokens
+    int tune_gemm_pair_ks = 0;   // ... K splits of a tile: 0 = automatic, 1 = never, with gemm_pair 1..4 = that many
     int tune_moe_gemm = 0;       // MoE prefill: 0 = automatic, 1 = weight rows, 2 = token rows, 128 / 192 / 256 = pairs, tiles of at most that many rows
     int tune_gemm_form = 0;      // above the decode rows: 0 = automatic, 1 = token rows (gemm_tc.cu), 2 = weight rows (gemm_ts.cu)
     int tune_gemm_bn = 0;        // gemm_tc.cu: weight rows per tile (128..256, a multiple of 32), 0 = automatic
@@ -143,8 +144,8 @@ struct Dec {
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     void ts_query_clusters();
     TsChoice gemm_ts_choose(int n, int k, int t) const;
-    TsChoice gemm_ts2_choose(const Lin* l, int t, int out_kind) const;
-    int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, cudaStream_t st);
+    TsChoice gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split) const;
+    int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, cudaStream_t st);
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
     int gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
                         int tok, const float* row_w, cudaStream_t st, bool tables_fresh);

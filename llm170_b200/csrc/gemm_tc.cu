@@ -653,7 +653,8 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
     }
     if (tune_gemm_pair > 1) {
-        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, st);
+        const int ks = std::min(std::max(tune_gemm_pair_ks, 1), (l->k + 2 * TILE_K - 1) / (2 * TILE_K));
+        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, ks, st);
     }
     // Tile shape and K split are chosen together by a small cost model (microseconds, fitted to measurements on B200).  A
     // k-block takes 0.30 + 0.00105 bn with one 128-token block; with two, 0.295 + 0.00133 bn while at most 100 CTAs run and
@@ -743,7 +744,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                         l->k, tune_ts_ks);
         }
         const bool ts = tune_gemm_form == 2 || c.cost < bar_ts * best.cost;
-        const bool stays = ts && (c.ks > 1 ? l->k >= 16384 : t <= 320 && (long long)l->n * l->k <= 1 << 20);
+        const bool stays = ts && (c.ks > 1 ? l->k >= 16384 && t >= 256 : t <= 320 && (long long)l->n * l->k <= 1 << 20);
         if (t > 64 && t <= 4096 && !stays && tune_gemm_form == 0 && tune_gemm_pair == 0 && tune_ts_tok == 0 && tune_ts_ks == 0 &&
             tune_gemm_tma_store == 1) {
             // The pairs (gemm_ts2.cu) take f16 results that they are estimated to finish sooner.  The estimates of the weight-row form run 5 % high
@@ -760,17 +761,26 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // tokens 235 / 257 / 230, at 3000 185 / 218 / 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512; 5120 x 6144 at 4096,
             // 2.92 waves, 206 / 205 / 193.
             const double line = t <= 128 ? 0.8 : !ts ? 0.98 : c.ks > 1 ? 0.84 : t < 256 ? 0.9 : 0.92;
-            if (gemm_ts2_choose(l, t, W4A16_OUT_F16).cost < line * (ts ? c.cost : best.cost)) {
+            if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost)) {
                 if (out_kind == W4A16_OUT_F16 || (ts && c.ks > 1)) {
-                    return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind).tok, st);
+                    return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, st);
                 }
                 if (!ts && best.cost < whole.cost) {
-                    const TsChoice p = gemm_ts2_choose(l, t, out_kind);
+                    const TsChoice p = gemm_ts2_choose(l, t, out_kind, 1);
                     const int rest = (t + BM * whole.mt - 1) / (BM * whole.mt) * ((l->n + whole.bn - 1) / whole.bn) % sm_count;
                     if (p.cost < whole.cost * (rest > 0 && rest <= 100 ? 1.0 : 0.78)) {
-                        return gemm_ts2(l, x, dst, t, out_kind, p.tok, st);
+                        return gemm_ts2(l, x, dst, t, out_kind, p.tok, 1, st);
                     }
                     best = whole;
+                }
+            } else if (ts && c.ks > 1 && t < 256 && (long long)l->n * l->k >= 8 << 20 && tune_gemm_pair_ks != 1) {
+                // Few tiles, which the weight rows would split over clusters of single CTAs: the pairs split them as well, results of either kind.
+                // Over 70 such calls of 65 to 250 tokens (13 shapes) they take 0.89 of the time, the worst one 1.01; linears of fewer than 8 M
+                // weights were slower (1024 x 4096 at 96 tokens 7.4 / 6.5 us), and from 256 tokens on f32 results keep the forms that the tests
+                // name.
+                const TsChoice p = gemm_ts2_choose(l, t, W4A16_OUT_F16, 4);
+                if (p.ks > 1 && p.cost < c.cost) {
+                    return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, st);
                 }
             }
         }

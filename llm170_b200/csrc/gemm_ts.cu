@@ -96,14 +96,6 @@ __device__ __forceinline__ void umma_ts_f16(uint32_t tmem_d, uint32_t tmem_a, ui
         ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accum)
         : "memory");
 }
-__device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned cta_rank) {
-    uint32_t ra;
-    float4 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local_addr), "r"(cta_rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
-    return v;
-}
-
 template <int GROUP, bool FMA, bool TEAMS>
 __global__ void __launch_bounds__(ts_threads(TEAMS), 2)
 gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_s, const TsArgs a) {

@@ -47,6 +47,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ float4 ld_dsmem_f32x4(uint32_t local_addr, unsigned cta_rank) {
+    uint32_t ra;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local_addr), "r"(cta_rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(ra) : "memory");
+    return v;
+}
 // Scale pair (rows g, g + 8) of a tile's 32 or more channels, ready for ts_expand: f16((q - 8) * s) as (q - 8) times s, or (FMA) as a
 // multiply-add of the raw nibble with s scaled by powers of two and -8 s 2^-E (Dec::fma_shift).
 template <bool FMA>

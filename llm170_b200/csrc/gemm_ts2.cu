@@ -53,6 +53,10 @@ constexpr int P_EPI0 = 3 + P_EXP_WARPS;                              // first wa
 constexpr int P_THREADS = (3 + P_EXP_WARPS + P_EPI_WARPS) * 32;
 constexpr int P_ROWS = 2 * TS_MROWS;                                 // weight rows of a pair's tile
 constexpr int P_TOK_MAX = 256;
+// Few tiles leave pairs idle: two to four pairs of a cluster share a tile's K, and their f32 sums meet in distributed shared memory, over the idle rings.
+// us, weight rows with their clusters of single CTAs / so: 96 x 5120 x 17408 24.5 / 22.1, 128 x 5120 x 6144 17.2 / 14.3, 128 x 2560 x 9728 17.9 / 13.6,
+// 128 x 3584 x 18944 in groups of 32 29.7 / 22.8.
+constexpr int P_MAX_SPLIT = 4;
 constexpr int P_SUB_MAX = P_TOK_MAX / 2;                             // tokens of an accumulator: a tile takes one or two
 constexpr int P_RAW_STAGE = RAW_BYTES + ts_scale_bytes(32);          // raw weights and their scales, 128 channels
 constexpr int P_OUT_STAGE = P_SUB_MAX * TS_MROWS * 2;                // f16 results of an accumulator on their way out, two of them
@@ -71,6 +75,7 @@ constexpr int P_OUT_BOX = 32;                                        // tokens o
 constexpr int P_X_BOXES = P_TOK_MAX / 32;                            // grouped form: token boxes of 16, 32, .. 128 rows, half of a tile
 constexpr int P_TMEM_COLS = 512;                                     // 256 accumulator columns, four stages of 64
 constexpr int P_GROUP_M = 8;                                         // token tiles that take turns on the same weights
+static_assert(128 * TS_MROWS * 4 <= p_off_bars(128) && 192 * TS_MROWS * 4 <= p_off_bars(192) && 256 * TS_MROWS * 4 <= p_off_bars(256), "sums of a split");
 static_assert(P_TOK_MAX + 4 * A_COLS <= P_TMEM_COLS, "TMEM");
 static_assert(p_smem(128) <= 226 * 1024 && p_smem(192) <= 226 * 1024 && p_smem(256) <= 226 * 1024, "shared memory");
 
@@ -82,6 +87,7 @@ struct PairArgs {
     int out_f16;
     int m_tiles, n_tiles;
     int tok;                     // tokens per tile = MMA N (multiple of 32); grouped form: the most that a tile holds
+    int ks;                      // K splits of a tile: that many pairs in a cluster, one tile each (dense)
     int split;                   // 1: a tile of more than 128 tokens is two MMAs (the grouped form's always are)
     int nrb_w;                   // 16-row blocks of the resident matrix (tile pitch)
     int pdl;
@@ -116,19 +122,14 @@ __device__ __forceinline__ void umma2_ts_f16(bool leader, uint32_t tmem_d, uint3
         ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accum), "r"((uint32_t)leader)
         : "memory");
 }
-// arrives on the barrier at this offset in both CTAs of the pair
-__device__ __forceinline__ void umma2_commit(bool leader, uint32_t bar) {
+// arrives on the barrier at this offset in both CTAs of the pair (`both`: a bit each, by rank in the cluster)
+__device__ __forceinline__ void umma2_commit(bool leader, uint32_t bar, unsigned short both) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
         "setp.ne.b32 q, %2, 0;\n\t"
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar),
-        "h"((unsigned short)3), "r"((uint32_t)leader)
+        "h"(both), "r"((uint32_t)leader)
         : "memory");
-}
-__device__ __forceinline__ uint32_t in_leader(uint32_t addr) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-    return r;
 }
 // What the barriers order across the pair is TMEM (tcgen05.wait and the tcgen05 fences) and TMA writes (complete_tx), no memory that
 // a thread reads or writes: release at cluster scope, which waits for all of a thread's stores, took 0.9 us per stage.
@@ -157,9 +158,8 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t 
 
 // CAP: the most tokens of a tile.  (Ring sizes known at compile time: the MMAs' addresses cost their issuer fewer instructions, 256 x 7168 x
 // 5120, tiles of 128, 19.5 -> 17.9 us.)
-template <int GROUP, bool FMA, bool GROUPED, int CAP>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
-gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a) {
+template <int GROUP, bool FMA, bool GROUPED, int CAP, bool SPLIT>
+__device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const PairArgs& a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
     __shared__ int s_abort;
@@ -170,6 +170,17 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
     constexpr int GPS = SK / GROUP;                                  // scale groups per stage: 1 or 4
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int rank = (int)blockIdx.x & 1;                            // in the pair; CTA 0 issues the MMAs
+    const int ks = SPLIT ? a.ks : 1, ksplit = SPLIT ? (int)(blockIdx.x >> 1) % ks : 0;
+    const unsigned short both = (unsigned short)(3u << (2 * ksplit));
+    auto in_leader = [&](uint32_t addr) {
+        uint32_t r;
+        if (SPLIT) {
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(2 * ksplit));
+        } else {
+            asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+        }
+        return r;
+    };
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;     // the same offset in both CTAs
     unsigned char* base_ptr = smem_dyn + (base - smem_u32(smem_dyn));
     constexpr int X_STAGE = p_x_stage(CAP), NS = p_stages(CAP), NR = p_raw_stages(CAP);
@@ -184,9 +195,10 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
     auto accum_bar = [&](int s) { return bars + 8u * (2 * NR + 2 * NS + s); };
     auto acc_free = [&](int s) { return bars + 8u * (2 * NR + 2 * NS + 2 + s); };     // of CTA 0
 
-    const int nkb = a.k / BK, nst = (nkb + 1) / 2;                   // the last stage may hold one k-block (32-channel groups)
+    // this pair's stages, of the tile's or of its part of K; the last of all may hold one k-block (32-channel groups)
+    const int nst_all = (a.k / BK + 1) / 2, st0 = nst_all * ksplit / ks, nst = nst_all * (ksplit + 1) / ks - st0, nkb = min(a.k / BK - 2 * st0, 2 * nst);
     const int tiles = (GROUPED ? *a.num_tiles : a.m_tiles) * a.n_tiles;
-    const int pair0 = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
+    const int pair0 = (int)(blockIdx.x >> 1) / ks, pairs = (int)(gridDim.x >> 1) / ks;
     // Dense: groups of P_GROUP_M token tiles, whose neighbours share the weights: a wave's weights and tokens both stay within the L2.
     // Grouped: neighbours share the token rows, then the expert's weights; the table goes by size, the largest tiles first.
     struct Tile {
@@ -285,9 +297,9 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
                     if (rank == 0) {
                         mbar_expect_tx(full(sx), (uint32_t)(tl.tok * (SK * 2)));     // both CTAs' tokens (zeros past the end)
                     }
-                    tma2_load_3d(x_addr(sx), map0, 0, tl.m0 + rank * (n0 / 2), 2 * it, in_leader(full(sx)));
+                    tma2_load_3d(x_addr(sx), map0, 0, tl.m0 + rank * (n0 / 2), 2 * (st0 + it), in_leader(full(sx)));
                     if (n1 > 0) {
-                        tma2_load_3d(x_addr(sx) + (uint32_t)(n0 * SK), map1, 0, tl.m0 + n0 + rank * (n1 / 2), 2 * it, in_leader(full(sx)));
+                        tma2_load_3d(x_addr(sx) + (uint32_t)(n0 * SK), map1, 0, tl.m0 + n0 + rank * (n1 / 2), 2 * (st0 + it), in_leader(full(sx)));
                     }
                 }
                 __syncwarp();
@@ -322,8 +334,8 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
                 if (leader) {
                     const int kbs = min(2, nkb - 2 * it);
                     mbar_expect_tx(raw_full(sr), kbs * kb_bytes + ts_scale_bytes(GROUP));   // (scales past the end: zeros)
-                    tma_load_2d(raw_addr(sr) + RAW_BYTES, &maps.scales, it * GPS * 8, tl.rb0, raw_full(sr));
-                    const uint32_t* src = a.qt + ((size_t)(2 * it) * a.nrb_w + tl.rb0) * TILE_WORDS;
+                    tma_load_2d(raw_addr(sr) + RAW_BYTES, &maps.scales, (st0 + it) * GPS * 8, tl.rb0, raw_full(sr));
+                    const uint32_t* src = a.qt + ((size_t)(2 * (st0 + it)) * a.nrb_w + tl.rb0) * TILE_WORDS;
                     bulk_load(raw_addr(sr), src, kb_bytes, raw_full(sr));
                     if (kbs == 2) {
                         bulk_load(raw_addr(sr) + RAW_BYTES / 2, src + (size_t)a.nrb_w * TILE_WORDS, kb_bytes, raw_full(sr));
@@ -373,13 +385,13 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
             }
         };
         auto hand_back = [&]() {
-            umma2_commit(leader, free_(sa));
+            umma2_commit(leader, free_(sa), both);
             if (++sa == NS) {
                 sa = 0;
                 pa ^= 1;
             }
         };
-        auto complete = [&](uint32_t u) { umma2_commit(leader, accum_bar(u & 1)); };
+        auto complete = [&](uint32_t u) { umma2_commit(leader, accum_bar(u & 1), both); };
         int tok_next = pair0 < tiles ? tok_at(pair0) : 0;
         for (int i = pair0; rank == 0 && i < tiles && ok; i += pairs) {
             const int tok = __shfl_sync(0xffffffffu, tok_next, 0);
@@ -465,6 +477,23 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
                 }
             }
             skip = it - nst;
+        }
+    } else if (SPLIT) {
+        // ------------------------------------------------------------------ this pair's sums, for the pairs of the cluster
+        // [token][row] f32 over the rings, which are idle: every MMA is complete
+        const int quad = warp & 3, sub = (warp - P_EPI0) >> 2;
+        Tile tl;
+        tokens_at(pair0, tl);
+        ok = mbar_wait(accum_bar(0), 0, abort_flag, a.status, (68 << 16)) && (tl.tok <= P_SUB_MAX || mbar_wait(accum_bar(1), 0, abort_flag, a.status, (68 << 16)));
+        ok = __all_sync(0xffffffffu, ok);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int c0 = sub * 16; ok && c0 < tl.rows; c0 += P_EPI_WARPS / 4 * 16) {
+            uint32_t v[16];
+            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                *reinterpret_cast<float*>(base_ptr + ((c0 + q) * TS_MROWS + quad * 32 + lane) * 4) = __uint_as_float(v[q]);
+            }
         }
     } else {
         // ------------------------------------------------------------------ epilogue
@@ -608,6 +637,45 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
             }
         }
     }
+    if (SPLIT) {
+        // Every CTA adds an equal share of its rows' results over all splits, in their order.
+        __syncthreads();
+        cluster_sync_all();
+        if (a.pdl) {
+            asm volatile("griddepcontrol.wait;" ::: "memory");           // outputs may be what the previous kernel still reads
+        }
+        Tile tl;
+        tokens_at(pair0, tl);
+        const int nr4 = max(0, min(TS_MROWS, a.n - tl.n0)) / 4, total = tl.rows * nr4;
+        const int e0 = total * ksplit / ks, e1 = total * (ksplit + 1) / ks;
+        for (int e = e0 + (int)threadIdx.x; e < e1 && !*abort_flag; e += P_THREADS) {
+            const int tok = e / nr4, r = (e - tok * nr4) * 4;
+            float4 pv[P_MAX_SPLIT];
+#pragma unroll
+            for (int s = 0; s < P_MAX_SPLIT; ++s) {
+                pv[s] = s < ks ? ld_dsmem_f32x4(base + (uint32_t)((tok * TS_MROWS + r) * 4), (unsigned)(2 * s + rank)) : make_float4(0, 0, 0, 0);
+            }
+            float4 sum = pv[0];
+#pragma unroll
+            for (int s = 1; s < P_MAX_SPLIT; ++s) {
+                if (s < ks) {
+                    sum.x += pv[s].x;
+                    sum.y += pv[s].y;
+                    sum.z += pv[s].z;
+                    sum.w += pv[s].w;
+                }
+            }
+            const size_t o = (size_t)(tl.m0 + tok) * a.n + tl.n0 + r;
+            if (a.out_f16) {
+                const __half2 h0 = __floats2half2_rn(sum.x * a.out_mul, sum.y * a.out_mul), h1 = __floats2half2_rn(sum.z * a.out_mul, sum.w * a.out_mul);
+                *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(a.out) + o) =
+                    make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+            } else {
+                *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.out) + o) =
+                    make_float4(sum.x * a.out_mul, sum.y * a.out_mul, sum.z * a.out_mul, sum.w * a.out_mul);
+            }
+        }
+    }
     if (warp == P_EPI0 && lane == 0) {
         bulk_wait_group_read<0>();                                   // the last stores have read this CTA's shared memory
     }
@@ -619,9 +687,24 @@ gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a
     }
 }
 
+template <int GROUP, bool FMA, bool GROUPED, int CAP>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
+gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a) {
+    pair_gemm<GROUP, FMA, GROUPED, CAP, false>(maps, a);
+}
+// (a kernel of its own: a launch that names the size of its clusters, and K ranges known only then, cost 0.6 us)
+template <int GROUP, bool FMA, int CAP>
+__global__ void __launch_bounds__(P_THREADS, 1) gemm_ts2_split_kernel(const __grid_constant__ PairMaps<false> maps, const PairArgs a) {
+    pair_gemm<GROUP, FMA, false, CAP, true>(maps, a);
+}
+
 }  // namespace
 
 namespace {
+template <int GROUP, bool FMA>
+auto pair_split_kernel(int tok) {
+    return tok <= 128 ? gemm_ts2_split_kernel<GROUP, FMA, 128> : tok <= 192 ? gemm_ts2_split_kernel<GROUP, FMA, 192> : gemm_ts2_split_kernel<GROUP, FMA, 256>;
+}
 template <int GROUP, bool FMA, bool GROUPED>
 auto pair_kernel(int tok) {
     return tok <= 128 ? gemm_ts2_kernel<GROUP, FMA, GROUPED, 128> : tok <= 192 ? gemm_ts2_kernel<GROUP, FMA, GROUPED, 192> : gemm_ts2_kernel<GROUP, FMA, GROUPED, 256>;
@@ -632,7 +715,8 @@ cudaError_t gemm_ts2_init_device() {
     cudaError_t e = cudaSuccess;
     for (int tok : {128, 192, 256}) {
         for (const void* f : {(const void*)pair_kernel<128, false, false>(tok), (const void*)pair_kernel<128, true, false>(tok), (const void*)pair_kernel<32, false, false>(tok),
-                              (const void*)pair_kernel<128, false, true>(tok), (const void*)pair_kernel<128, true, true>(tok), (const void*)pair_kernel<32, false, true>(tok)}) {
+                              (const void*)pair_kernel<128, false, true>(tok), (const void*)pair_kernel<128, true, true>(tok), (const void*)pair_kernel<32, false, true>(tok),
+                              (const void*)pair_split_kernel<128, false>(tok), (const void*)pair_split_kernel<128, true>(tok), (const void*)pair_split_kernel<32, false>(tok)}) {
             if (e == cudaSuccess) {
                 e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, p_smem(tok));
             }
@@ -647,7 +731,10 @@ cudaError_t gemm_ts2_init_device() {
 // 32: 0.221), and with all pairs busy, when power holds the clock down, 0.05 + 0.00272 per token and at least 0.268 (0.326); each further tile
 // of a pair 0.48 where tiles take both accumulators.  f32 results, stored from registers, take another 0.0263 per token less 3.23 with each tile
 // (202 measurements before the accumulators alternated).
-TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind) const {
+// K splits (up to `max_split`, where all clusters are resident at once): the stages of a tile are dealt to two to four pairs of a cluster, which takes
+// another 0.01 us per token for the sums and, with all pairs busy, 2.73 us and 0.067 per stage (330 measurements, 15 shapes of 1024..34816 rows,
+// 12..250 tokens; good to 3.6 %).
+TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split) const {
     TsChoice best{0, 1, 1e30};
     const int n_tiles = (l->n + P_ROWS - 1) / P_ROWS, stages = (l->k + SK - 1) / SK, pairs = sm_count / 2;
     const bool g128 = l->group == 128;
@@ -662,6 +749,14 @@ TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind) const {
         const double c = 3.14 + 0.0064 * tok + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * (tok > P_SUB_MAX ? 0.48 : 0.0);
         if (c < best.cost) {
             best = TsChoice{tok, 1, c};
+        }
+        for (int ks = 2; ks <= max_split && ks <= stages && tiles <= ts_clusters[1][2 * ks]; ++ks) {
+            const double busy = std::min(1.0, std::max(0.0, ((double)tiles * ks / pairs - 0.46) / 0.54));
+            const int nst = (stages + ks - 1) / ks;
+            const double cs = 3.14 + 0.0164 * tok + nst * (light + std::max(0.0, heavy - light) * busy) + (double)tiles * ks / pairs * (2.73 + 0.067 * nst);
+            if (cs < best.cost) {
+                best = TsChoice{tok, ks, cs};
+            }
         }
     }
     return best;
@@ -696,32 +791,39 @@ cudaError_t launch_pairs(const Lin* l, const PairMaps<GROUPED>& maps, PairArgs& 
     a.nrb_w = l->n / TILE_ROWS;
     a.out_mul = l->out_mul;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(2 * std::min(tiles, sm_count / 2));
+    cfg.gridDim = dim3(2 * (a.ks > 1 ? tiles * a.ks : std::min(tiles, sm_count / 2)));
     cfg.blockDim = dim3(P_THREADS);
     cfg.dynamicSmemBytes = a.tok <= 128 ? p_smem(128) : a.tok <= 192 ? p_smem(192) : p_smem(256);
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
     if (a.pdl) {
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    if (l->group != 128) {
-        return cudaLaunchKernelEx(&cfg, pair_kernel<32, false, GROUPED>(a.tok), maps, a);
+    if (!GROUPED && a.ks > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2 * a.ks;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
-    if (l->fma_e < 0) {
-        return cudaLaunchKernelEx(&cfg, pair_kernel<128, false, GROUPED>(a.tok), maps, a);
+    const bool fma = l->group == 128 && l->fma_e >= 0;
+    if (fma) {
+        const __half2 mul = __float2half2_rn(ldexpf(-8.0f, -l->fma_e));
+        memcpy(&a.fma_mul, &mul, sizeof(mul));
+        a.fma_add = ((uint32_t)(20 - l->fma_e) << 26) + ((uint32_t)(24 - l->fma_e) << 10);
+        a.out_mul = ldexpf(l->out_mul, l->fma_e);
     }
-    const __half2 mul = __float2half2_rn(ldexpf(-8.0f, -l->fma_e));
-    memcpy(&a.fma_mul, &mul, sizeof(mul));
-    a.fma_add = ((uint32_t)(20 - l->fma_e) << 26) + ((uint32_t)(24 - l->fma_e) << 10);
-    a.out_mul = ldexpf(l->out_mul, l->fma_e);
-    return cudaLaunchKernelEx(&cfg, pair_kernel<128, true, GROUPED>(a.tok), maps, a);
+    if constexpr (!GROUPED) {
+        if (a.ks > 1) {
+            return cudaLaunchKernelEx(&cfg, l->group != 128 ? pair_split_kernel<32, false>(a.tok) : fma ? pair_split_kernel<128, true>(a.tok) : pair_split_kernel<128, false>(a.tok), maps, a);
+        }
+    }
+    return cudaLaunchKernelEx(&cfg, l->group != 128 ? pair_kernel<32, false, GROUPED>(a.tok) : fma ? pair_kernel<128, true, GROUPED>(a.tok) : pair_kernel<128, false, GROUPED>(a.tok), maps, a);
 }
 }  // namespace
 
-int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, cudaStream_t st) {
+int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, cudaStream_t st) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
@@ -730,7 +832,7 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     CUresult cr = ts_scale_map(enc, &maps.scales, l->st, l->n, l->k, l->group);
     // Two MMAs keep the pipe busy from tile to tile, at 8 cycles more than one each below 128 tokens: 512 x 5120 x 17408, tiles of 192, one
     // MMA / two 71.5 / 74.8 us, 1024 x 5120 x 17408, tiles of 160, 131 / 147; full ones cost nothing.
-    const int split = tok > 192, n0 = split ? (tok / 2 + 31) & ~31 : tok;             // as in the kernel
+    const int split = ks == 1 && tok > 192, n0 = split ? (tok / 2 + 31) & ~31 : tok;             // as in the kernel
     for (int i = 0; i < 2 && cr == CUDA_SUCCESS; ++i) {
         cr = pair_map(enc, &maps.x[i], x, t, l->k, (i == 1 && split ? tok - n0 : n0) / 2);
     }
@@ -742,6 +844,7 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     }
     PairArgs a{};
     a.tok = tok;
+    a.ks = ks;
     a.m_tiles = (t + tok - 1) / tok;
     a.n_tiles = (l->n + P_ROWS - 1) / P_ROWS;
     a.out = dst;
@@ -755,7 +858,7 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
-    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(tok) + "-token tiles";
+    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(tok) + "-token tiles" + (ks > 1 ? ", ksplit " + std::to_string(ks) : "");
     launches++;
     return 0;
 }
@@ -781,6 +884,7 @@ int Dec::gemm_ts2_grouped(const Lin* l, const void* xs, int xs_rows, void* out, 
     }
     PairArgs a{};
     a.tok = bm;
+    a.ks = 1;
     a.n_tiles = (n_per_expert + P_ROWS - 1) / P_ROWS;
     a.out = out;
     a.m = xs_rows;

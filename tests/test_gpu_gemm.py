@@ -500,6 +500,37 @@ def test_expanding_teams_equal_the_pairs(dec, t, k, n, group):
     dec.drop_lin("team")
 
 
+# pairs that split K over a cluster: fewer stages than splits, parts of unlike length, a last stage of one k-block, ragged rows (also a second half of a tile
+# without any) and tokens, the largest tiles of each ring, more clusters than are resident at once
+@pytest.mark.parametrize("t,k,n,group,tok,ks", [(9, 128, 16, 128, 32, 4), (33, 320, 144, 32, 64, 2), (65, 640, 528, 128, 96, 3), (128, 1088, 272, 64, 128, 4),
+                                                (150, 1024, 784, 32, 160, 3), (192, 896, 256, 128, 192, 4), (250, 1152, 400, 128, 256, 2), (300, 960, 1296, 32, 160, 3),
+                                                (200, 512, 8720, 128, 96, 4)])
+@pytest.mark.parametrize("out_f16", [False, True])
+def test_pairs_that_split_k_pow2_exact(dec, t, k, n, group, tok, ks, out_f16):
+    q, s, x, expect = pow2_case(t, k, n, group)
+    dec.upload_lin_g("pks", q, s, n, k, group)
+    guard = torch.full((t + 16, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    with forced(dec, "gemm_pair", tok), forced(dec, "gemm_pair_ksplit", ks):
+        for _ in range(2):
+            y = dec.lin_forward("pks", x_dev(x), t, dst=guard[:t], out_f16=out_f16)
+            name = dec.last_kernel()
+            dec.sync()
+            dec.kernel_status()
+    assert name.startswith("gemm_ts2_kernel") and ("ksplit" in name) == (k > 128), name
+    assert np.array_equal(y.cpu().numpy(), expect.astype(np.float16) if out_f16 else expect)   # sums of powers of two: exact in any order
+    assert (guard[t:] == 7.0).all()
+    with pytest.raises(Exception):
+        dec.set_tuning("gemm_pair_ksplit", 5)
+    dec.drop_lin("pks")
+
+
+# ... and by themselves: f16 results are the f32 results rounded, also for K of 16384 and more below 256 tokens
+@pytest.mark.parametrize("n,k,group,t", [(5120, 6144, 128, 96), (5120, 17408, 128, 72), (3584, 18944, 32, 128), (2560, 9728, 128, 250)])
+def test_automatic_pairs_that_split_k(dec, n, k, group, t):
+    test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, PAIR, PAIR)
+    assert "ksplit" in dec.last_kernel()
+
+
 @pytest.mark.parametrize("bad", [-1, 2, 16, 48, 288])
 def test_cta_pair_tuning_refuses_values_without_a_tile(dec, bad):
     from llm170_b200.w4a16_dec import W4a16Error
