@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     constexpr int RW = RG_WARPS / KW, UR = RW * NR;           // row blocks of a unit
     constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
     constexpr uint32_t SLOT = rg_slot_bytes(GROUP, NR);
+    constexpr int PITCH = rg_red_pitch(UR);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // optional timeline (diagnostic; a.dbg is null in normal runs): wall-clock stamps of thread 0 in the slots of the other forms
     auto stamp_now = [&](int j) {
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     // lanes without a token read token 0: their columns are never stored
     const uint32_t xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
     const int mp = (m + 1) & ~1;
-    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][mp]
+    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][mp][PITCH]
     uint32_t rslot = 0;
     for (int u = u0; u < u1; ++u) {
         float tot[NR][4];
@@ -152,19 +153,15 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
         }
         if (2 * t < mp) {
             const float m0 = 16777216.f * sg.out_mul, m1 = 1048576.f * sg.out_mul;
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                float* d = red + ((size_t)kw * (UR * TILE_ROWS) + (rw * NR + r) * TILE_ROWS + g) * mp + 2 * t;
-                *reinterpret_cast<float2*>(d) = make_float2(tot[r][0] * m0, tot[r][1] * m0);
-                *reinterpret_cast<float2*>(d + 8 * mp) = make_float2(tot[r][2] * m1, tot[r][3] * m1);
-            }
+            rg_store_sums(red + (kw * mp + 2 * t) * PITCH + rw * NR * TILE_ROWS + g, PITCH, tot, m0, m1);
         }
         __syncthreads();
         auto local_sum = [&](int tok, int row) {
-            float v = red[row * mp + tok];
+            const float* d = red + tok * PITCH + row;
+            float v = d[0];
 #pragma unroll
             for (int w = 1; w < KW; ++w) {
-                v += red[(w * (UR * TILE_ROWS) + row) * mp + tok];      // fixed order: the same bits every run
+                v += d[w * mp * PITCH];                                  // fixed order: the same bits every run
             }
             return v;
         };
@@ -252,7 +249,7 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
                 p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
             }
             p.off_red = x_bytes;
-            p.off_ring = (x_bytes + kw * ur * TILE_ROWS * mp * 4 + 127) & ~127;
+            p.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
             const double tiles = (double)((ku + kw - 1) / kw * (unit_k / TILE_K) * nr) * (nr == 2 ? 1.3 : nr == 3 ? 1.05 : 1.0);
             for (int per_sm = 1; per_sm <= 2; ++per_sm) {
                 const int room = per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX;
@@ -356,7 +353,7 @@ bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& 
                     p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
                 }
                 p.off_red = x_bytes;
-                p.off_part = (x_bytes + kw * ur * TILE_ROWS * mp * 4 + 127) & ~127;
+                p.off_part = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
                 p.off_ring = (p.off_part + 2 * ur * TILE_ROWS * GEMV_MAX_M * 4 + 127) & ~127;
                 const int room = 2 * clusters[cl];
                 if (room <= 0 || p.off_ring + 2 * RG_WARPS * slot > RG_SMEM_TWO) {
