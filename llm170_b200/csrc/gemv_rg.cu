@@ -15,7 +15,7 @@
 //   * the warps' sums meet in shared memory once per unit; nothing is shared between CTAs, but where x does not fit beside the rings (five to
 //     eight tokens of long K): there the CTAs of a cluster share K and add up in each other's shared memory (rg_cluster_plan).
 // One token, us per launch, this form against the best of the others: 7168 x 5120 6.6 / 7.2, 5120 x 6144 6.2 / 7.5, 34816 x 5120
-// 17.3 / 21.6 (5.3 TB/s), 5120 x 17408 13.0 / 13.8, 24576 x 4096 12.0 / 15.9; eight tokens: 7.4 / 10.3, 6.6 / 10.2, 20.5 / 26.2;
+// 17.3 / 21.6 (5.3 TB/s), 5120 x 17408 13.0 / 13.8, 24576 x 4096 12.0 / 15.9; eight tokens: 7.1 / 10.3, 6.6 / 10.2, 20.5 / 26.2;
 // 34816 x 5120 in groups of 32, eight tokens: 21.7 / 48.9.
 #include <cuda_fp16.h>
 
@@ -329,9 +329,8 @@ bool rg_leaves(const GemvArgs& a, const RgPlan& p, const SkPlan& sk, int sm_coun
 }
 
 // The row-group form over clusters, two CTAs per SM, for activations that do not fit beside a ring: every CTA stages its part of K.  us per
-// launch, the persistent form / clusters of the size chosen: 4096 x 14336 at eight tokens 18.4 / 11.4 (groups of 32 20.2 / 12.3), 5120 x 17408 at
-// six to eight 18.0 / 14.8, 18.6 / 15.2, 18.9 / 15.4 (21.4 / 16.2), 5632 x 20224 at five 20.8 / 16.8, 8192 x 28672 at eight 38.2 / 36.1 (52.2 /
-// 39.6).  Where the activations fit, a CTA alone on its SM with all of K is as fast or faster (5120 x 17408, one token: 13.6 / 14.0; 5120 x 8704
+// launch, the persistent form / clusters of the size chosen: 4096 x 14336 at eight tokens 18.4 / 11.2 (groups of 32 20.2 / 12.1), 5120 x 17408 at
+// six to eight 18.0 / 14.5, 18.6 / 14.5, 18.9 / 14.6 (21.4 / 15.7), 5632 x 20224 at five 20.8 / 16.8, 8192 x 28672 at eight 38.2 / 36.1.  Where the activations fit, a CTA alone on its SM with all of K is as fast or faster (5120 x 17408, one token: 13.6 / 14.0; 5120 x 8704
 // 8.1 / 8.8): what the barriers of a cluster take, about 1.2 us, is what the better balance brings.  `clusters`: how many of 1..8 whole-SM CTAs
 // can be resident; of half-SM CTAs at least twice as many.  `us`: the time to beat, estimated as in rg_us.
 bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& best, double us) {
