@@ -144,8 +144,8 @@ struct Dec {
     int gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st);
     void ts_query_clusters();
     TsChoice gemm_ts_choose(int n, int k, int t) const;
-    TsChoice gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split) const;
-    int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, cudaStream_t st);
+    TsChoice gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split, int min_parts = 1) const;
+    int gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, bool short_sums, cudaStream_t st);
     int gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, const TsChoice& c, cudaStream_t st);
     int gemm_ts_grouped(const Lin* l, const void* xs, int xs_rows, void* out, int n_per_expert, const MoeBufs& b, int max_tiles,
                         int tok, const float* row_w, cudaStream_t st, bool tables_fresh);

@@ -654,7 +654,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     }
     if (tune_gemm_pair > 1) {
         const int ks = std::min(std::max(tune_gemm_pair_ks, 1), (l->k + 2 * TILE_K - 1) / (2 * TILE_K));
-        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, ks, st);
+        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, ks, ks > 1, st);
     }
     // Tile shape and K split are chosen together by a small cost model (microseconds, fitted to measurements on B200).  A
     // k-block takes 0.30 + 0.00105 bn with one 128-token block; with two, 0.295 + 0.00133 bn while at most 100 CTAs run and
@@ -761,26 +761,27 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // tokens 235 / 257 / 230, at 3000 185 / 218 / 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512; 5120 x 6144 at 4096,
             // 2.92 waves, 206 / 205 / 193.
             const double line = t <= 128 ? 0.8 : !ts ? 0.98 : c.ks > 1 ? 0.84 : t < 256 ? 0.9 : 0.92;
-            if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost)) {
-                if (out_kind == W4A16_OUT_F16 || (ts && c.ks > 1)) {
-                    return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, st);
+            // In place of weight rows that split K: pairs whose accumulators take no more stages each (gemm_ts2), results of either kind from the
+            // same tiles.  Below 256 tokens of more than 2^24 weights these may split K, too: few tiles (101 calls of both kinds take 0.89 of the time).
+            // Smaller linears gain little or lose: 1792 x 5120 at 100 tokens 9.4 / 9.2 us, 4096 x 4096 11.1 / 10.8, 1024 x 4096 7.4 / 6.5; from 256
+            // tokens on f32 results keep the forms that the tests name.
+            if (ts && c.ks > 1) {
+                const bool may_split = t < 256 && (long long)l->n * l->k > 16 << 20 && tune_gemm_pair_ks != 1;
+                const TsChoice p = gemm_ts2_choose(l, t, W4A16_OUT_F16, may_split ? 4 : 1, c.ks);
+                if (p.ks > 0 && p.cost < (p.ks > 1 ? 1.0 : line) * c.cost) {
+                    return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, true, st);
+                }
+            } else if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost)) {
+                if (out_kind == W4A16_OUT_F16) {
+                    return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, false, st);
                 }
                 if (!ts && best.cost < whole.cost) {
                     const TsChoice p = gemm_ts2_choose(l, t, out_kind, 1);
                     const int rest = (t + BM * whole.mt - 1) / (BM * whole.mt) * ((l->n + whole.bn - 1) / whole.bn) % sm_count;
                     if (p.cost < whole.cost * (rest > 0 && rest <= 100 ? 1.0 : 0.78)) {
-                        return gemm_ts2(l, x, dst, t, out_kind, p.tok, 1, st);
+                        return gemm_ts2(l, x, dst, t, out_kind, p.tok, 1, false, st);
                     }
                     best = whole;
-                }
-            } else if (ts && c.ks > 1 && t < 256 && (long long)l->n * l->k >= 8 << 20 && tune_gemm_pair_ks != 1) {
-                // Few tiles, which the weight rows would split over clusters of single CTAs: the pairs split them as well, results of either kind.
-                // Over 70 such calls of 65 to 250 tokens (13 shapes) they take 0.89 of the time, the worst one 1.01; linears of fewer than 8 M
-                // weights were slower (1024 x 4096 at 96 tokens 7.4 / 6.5 us), and from 256 tokens on f32 results keep the forms that the tests
-                // name.
-                const TsChoice p = gemm_ts2_choose(l, t, W4A16_OUT_F16, 4);
-                if (p.ks > 1 && p.cost < c.cost) {
-                    return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, st);
                 }
             }
         }

@@ -88,6 +88,7 @@ struct PairArgs {
     int m_tiles, n_tiles;
     int tok;                     // tokens per tile = MMA N (multiple of 32); grouped form: the most that a tile holds
     int ks;                      // K splits of a tile: that many pairs in a cluster, one tile each (dense)
+    int halves;                  // 1: the second half of a tile's stages goes to an accumulator of its own (one tile of at most 128 tokens per pair)
     int split;                   // 1: a tile of more than 128 tokens is two MMAs (the grouped form's always are)
     int nrb_w;                   // 16-row blocks of the resident matrix (tile pitch)
     int pdl;
@@ -151,6 +152,15 @@ __device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t* v) 
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
+// v += 16 columns of another accumulator
+__device__ __forceinline__ void add_tmem16(uint32_t (&v)[16], uint32_t taddr) {
+    uint32_t w[16];
+    tmem_ld16(taddr, w);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+        v[q] = __float_as_uint(__uint_as_float(v[q]) + __uint_as_float(w[q]));
+    }
+}
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&h)[4]) {
     asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(h[0]), "r"(h[1]), "r"(h[2]), "r"(h[3])
                  : "memory");
@@ -199,6 +209,7 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
     const int nst_all = (a.k / BK + 1) / 2, st0 = nst_all * ksplit / ks, nst = nst_all * (ksplit + 1) / ks - st0, nkb = min(a.k / BK - 2 * st0, 2 * nst);
     const int tiles = (GROUPED ? *a.num_tiles : a.m_tiles) * a.n_tiles;
     const int pair0 = (int)(blockIdx.x >> 1) / ks, pairs = (int)(gridDim.x >> 1) / ks;
+    const bool halves = !GROUPED && a.halves != 0 && nst > 1;
     // Dense: groups of P_GROUP_M token tiles, whose neighbours share the weights: a wave's weights and tokens both stay within the L2.
     // Grouped: neighbours share the token rows, then the expert's weights; the table goes by size, the largest tiles first.
     struct Tile {
@@ -366,7 +377,7 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
         };
         auto stage_ready = [&](int ba, uint32_t qa, int it) { return in_time(mbar_wait(full(ba), qa, abort_flag, a.status, (64 << 16) | it)); };
         // one stage into one accumulator: `n` of the tile's tokens, `off` bytes into the stage's tokens
-        auto multiply = [&](int ba, int it, uint32_t acc, int n, uint32_t off) {
+        auto multiply = [&](int ba, int it, uint32_t acc, int n, uint32_t off, bool first) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t idesc = (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(P_ROWS >> 4) << 24);
             const uint64_t db = umma_desc(x_addr(ba) + off);
@@ -375,7 +386,7 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
             const bool two = 2 * it + 1 < nkb;
 #pragma unroll
             for (int j = 0; j < BK / 16; ++j) {
-                umma2_ts_f16(leader, acc, ta + j * 8, db + 2 * j, idesc, (it > 0 || j > 0) ? 1u : 0u);
+                umma2_ts_f16(leader, acc, ta + j * 8, db + 2 * j, idesc, (!first || j > 0) ? 1u : 0u);
             }
             if (two) {
 #pragma unroll
@@ -401,11 +412,13 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
             if (!split(tok)) {
                 const bool two = tok > P_SUB_MAX;                    // (tiles that take both come first, so `used` is even here)
                 const uint32_t acc = tmem + (used & 1) * P_SUB_MAX;
+                const int half = (nst + 1) / 2;
                 ok = acc_ready(used) && (!two || acc_ready(used + 1));
                 for (int it = 0; it < nst && ok; ++it) {
                     ok = stage_ready(sa, pa, it);
                     if (ok) {
-                        multiply(sa, it, acc, tok, 0);
+                        const int it0 = halves && it >= half ? half : 0;
+                        multiply(sa, it, it0 > 0 ? acc + P_SUB_MAX : acc, tok, 0, it == it0);
                         hand_back();
                     }
                 }
@@ -426,11 +439,11 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
                 const int next = both ? it + 2 : it + 1;
                 ok = stage_ready(sa, pa, it);
                 if (ok) {
-                    multiply(sa, it, acc0, n0, 0);
+                    multiply(sa, it, acc0, n0, 0, it == 0);
                     if (both) {
                         ok = stage_ready(ba, qa, it + 1);
                         if (ok) {
-                            multiply(ba, it + 1, acc0, n0, 0);
+                            multiply(ba, it + 1, acc0, n0, 0, false);
                         }
                     }
                 }
@@ -439,10 +452,10 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
                 }
                 ok = ok && (it > 0 || acc_ready(used + 1));
                 if (ok) {
-                    multiply(sa, it, acc1, n1, off1);
+                    multiply(sa, it, acc1, n1, off1, it == 0);
                     hand_back();
                     if (both) {
-                        multiply(sa, it + 1, acc1, n1, off1);
+                        multiply(sa, it + 1, acc1, n1, off1, false);
                         hand_back();
                     }
                 }
@@ -490,6 +503,9 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
         for (int c0 = sub * 16; ok && c0 < tl.rows; c0 += P_EPI_WARPS / 4 * 16) {
             uint32_t v[16];
             tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+            if (halves) {
+                add_tmem16(v, tmem + P_SUB_MAX + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0);
+            }
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 *reinterpret_cast<float*>(base_ptr + ((c0 + q) * TS_MROWS + quad * 32 + lane) * 4) = __uint_as_float(v[q]);
@@ -547,6 +563,20 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
                             tmem_ld_16x256b_x4(t_ld + acc + (uint32_t)c0 + 32u, v + 16);
                         }
                         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (halves) {
+#pragma unroll
+                            for (int hh = 0; hh < 2; ++hh) {
+                                if (c0 + 32 * hh < n) {
+                                    uint32_t w[16];
+                                    tmem_ld_16x256b_x4(t_ld + P_SUB_MAX + (uint32_t)(c0 + 32 * hh), w);
+                                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                                    for (int q = 0; q < 16; ++q) {
+                                        v[16 * hh + q] = __float_as_uint(__uint_as_float(v[16 * hh + q]) + __uint_as_float(w[q]));
+                                    }
+                                }
+                            }
+                        }
 #pragma unroll
                         for (int q = 0; q < 4; ++q) {
                             uint32_t h[4];
@@ -567,6 +597,9 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
                     for (int c0 = sub * 16; c0 < rows; c0 += P_EPI_WARPS / 4 * 16) {
                         uint32_t v[16];
                         tmem_ld16(tmem + acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+                        if (halves) {
+                            add_tmem16(v, tmem + P_SUB_MAX + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0);
+                        }
 #pragma unroll
                         for (int q = 0; q < 16; ++q) {
                             if (c0 + q < rows && lrow < rows_out) {
@@ -733,9 +766,9 @@ cudaError_t gemm_ts2_init_device() {
 // (202 measurements before the accumulators alternated).
 // K splits (up to `max_split`, where all clusters are resident at once): the stages of a tile are dealt to two to four pairs of a cluster, which takes
 // another 0.01 us per token for the sums and, with all pairs busy, 2.73 us and 0.067 per stage (330 measurements, 15 shapes of 1024..34816 rows,
-// 12..250 tokens; good to 3.6 %).
-TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split) const {
-    TsChoice best{0, 1, 1e30};
+// 12..250 tokens; good to 3.6 %).  `min_parts`: in place of weight rows that split K in so many parts -- no accumulator takes more stages than there.
+TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split, int min_parts) const {
+    TsChoice best{0, 0, 1e30};
     const int n_tiles = (l->n + P_ROWS - 1) / P_ROWS, stages = (l->k + SK - 1) / SK, pairs = sm_count / 2;
     const bool g128 = l->group == 128;
     for (int cap = P_TOK_MAX; cap >= 64; cap -= 32) {
@@ -747,14 +780,15 @@ TsChoice Dec::gemm_ts2_choose(const Lin* l, int t, int out_kind, int max_split) 
         const double heavy = std::max(g128 ? 0.268 : 0.326, 0.05 + 0.00272 * tok);
         const double f32 = out_kind == W4A16_OUT_F16 ? 0.0 : std::max(0.0, 0.0263 * tok - 3.23);
         const double c = 3.14 + 0.0064 * tok + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * (tok > P_SUB_MAX ? 0.48 : 0.0);
-        if (c < best.cost) {
+        const int halves = tok <= P_SUB_MAX ? 2 : 1;                 // (as in gemm_ts2)
+        if (c < best.cost && (min_parts <= 1 || (min_parts <= halves && tiles <= pairs))) {
             best = TsChoice{tok, 1, c};
         }
         for (int ks = 2; ks <= max_split && ks <= stages && tiles <= ts_clusters[1][2 * ks]; ++ks) {
             const double busy = std::min(1.0, std::max(0.0, ((double)tiles * ks / pairs - 0.46) / 0.54));
             const int nst = (stages + ks - 1) / ks;
             const double cs = 3.14 + 0.0164 * tok + nst * (light + std::max(0.0, heavy - light) * busy) + (double)tiles * ks / pairs * (2.73 + 0.067 * nst);
-            if (cs < best.cost) {
+            if (cs < best.cost && min_parts <= ks * halves) {
                 best = TsChoice{tok, ks, cs};
             }
         }
@@ -823,7 +857,10 @@ cudaError_t launch_pairs(const Lin* l, const PairMaps<GROUPED>& maps, PairArgs& 
 }
 }  // namespace
 
-int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, cudaStream_t st) {
+// `short_sums`: in place of weight rows that would split K.  An MMA's sum drops what lies below the accumulator's last bit, so the error of a result grows
+// with the stages that go through one accumulator (6144 channels in three parts 2.4e-6 of the results' size, in one 7.2e-6).  A pair with one tile of
+// at most 128 tokens has a second accumulator to spare: half of its stages go there, and both are added at the end.
+int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, int tok, int ks, bool short_sums, cudaStream_t st) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) {
         return fail("w4a16 gemm: cuTensorMapEncodeTiled is not available from the driver");
@@ -852,6 +889,7 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     a.n = l->n;
     a.out_f16 = out_kind == W4A16_OUT_F16;
     a.split = split;
+    a.halves = short_sums && tok <= P_SUB_MAX && (ks > 1 || a.m_tiles * a.n_tiles <= sm_count / 2);
     a.pdl = tune_pdl ? 1 : 0;
     a.status = gemm_status;
     const cudaError_t e = launch_pairs<false>(l, maps, a, a.m_tiles * a.n_tiles, sm_count, st);
