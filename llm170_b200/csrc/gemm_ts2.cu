@@ -54,8 +54,8 @@ constexpr int P_THREADS = (3 + P_EXP_WARPS + P_EPI_WARPS) * 32;
 constexpr int P_ROWS = 2 * TS_MROWS;                                 // weight rows of a pair's tile
 constexpr int P_TOK_MAX = 256;
 // Few tiles leave pairs idle: two to four pairs of a cluster share a tile's K, and their f32 sums meet in distributed shared memory, over the idle rings.
-// us, weight rows with their clusters of single CTAs / so: 96 x 5120 x 17408 24.5 / 22.1, 128 x 5120 x 6144 17.2 / 14.3, 128 x 2560 x 9728 17.9 / 13.6,
-// 128 x 3584 x 18944 in groups of 32 29.7 / 22.8.
+// us, weight rows with their clusters of single CTAs / so: 100 x 5120 x 17408 25.9 / 24.8, 128 x 5120 x 6144 17.1 / 14.2, 128 x 2560 x 9728 17.6 / 13.8,
+// 128 x 3584 x 18944 in groups of 32 30.1 / 22.1.
 constexpr int P_MAX_SPLIT = 4;
 constexpr int P_SUB_MAX = P_TOK_MAX / 2;                             // tokens of an accumulator: a tile takes one or two
 constexpr int P_RAW_STAGE = RAW_BYTES + ts_scale_bytes(32);          // raw weights and their scales, 128 channels
