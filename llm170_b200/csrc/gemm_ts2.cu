@@ -168,7 +168,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t 
 
 // CAP: the most tokens of a tile.  (Ring sizes known at compile time: the MMAs' addresses cost their issuer fewer instructions, 256 x 7168 x
 // 5120, tiles of 128, 19.5 -> 17.9 us.)
-template <int GROUP, bool FMA, bool GROUPED, int CAP, bool SPLIT>
+template <int GROUP, bool FMA, bool GROUPED, int CAP, bool SPLIT, bool HALVES>
 __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const PairArgs& a) {
     extern __shared__ unsigned char smem_dyn[];
     __shared__ uint32_t s_tmem_base;
@@ -209,7 +209,7 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
     const int nst_all = (a.k / BK + 1) / 2, st0 = nst_all * ksplit / ks, nst = nst_all * (ksplit + 1) / ks - st0, nkb = min(a.k / BK - 2 * st0, 2 * nst);
     const int tiles = (GROUPED ? *a.num_tiles : a.m_tiles) * a.n_tiles;
     const int pair0 = (int)(blockIdx.x >> 1) / ks, pairs = (int)(gridDim.x >> 1) / ks;
-    const bool halves = !GROUPED && a.halves != 0 && nst > 1;
+    const bool halves = HALVES && a.halves != 0 && nst > 1;
     // Dense: groups of P_GROUP_M token tiles, whose neighbours share the weights: a wave's weights and tokens both stay within the L2.
     // Grouped: neighbours share the token rows, then the expert's weights; the table goes by size, the largest tiles first.
     struct Tile {
@@ -723,12 +723,17 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
 template <int GROUP, bool FMA, bool GROUPED, int CAP>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_ts2_kernel(const __grid_constant__ PairMaps<GROUPED> maps, const PairArgs a) {
-    pair_gemm<GROUP, FMA, GROUPED, CAP, false>(maps, a);
+    pair_gemm<GROUP, FMA, GROUPED, CAP, false, false>(maps, a);
+}
+// Sums in two halves (one tile of at most 128 tokens per pair).
+template <int GROUP, bool FMA>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1) gemm_ts2_halves_kernel(const __grid_constant__ PairMaps<false> maps, const PairArgs a) {
+    pair_gemm<GROUP, FMA, false, P_SUB_MAX, false, true>(maps, a);
 }
 // (a kernel of its own: a launch that names the size of its clusters, and K ranges known only then, cost 0.6 us)
 template <int GROUP, bool FMA, int CAP>
 __global__ void __launch_bounds__(P_THREADS, 1) gemm_ts2_split_kernel(const __grid_constant__ PairMaps<false> maps, const PairArgs a) {
-    pair_gemm<GROUP, FMA, false, CAP, true>(maps, a);
+    pair_gemm<GROUP, FMA, false, CAP, true, (CAP <= P_SUB_MAX)>(maps, a);
 }
 
 }  // namespace
@@ -753,6 +758,11 @@ cudaError_t gemm_ts2_init_device() {
             if (e == cudaSuccess) {
                 e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, p_smem(tok));
             }
+        }
+    }
+    for (const void* f : {(const void*)gemm_ts2_halves_kernel<128, false>, (const void*)gemm_ts2_halves_kernel<128, true>, (const void*)gemm_ts2_halves_kernel<32, false>}) {
+        if (e == cudaSuccess) {
+            e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, p_smem(P_SUB_MAX));
         }
     }
     return e;
@@ -849,6 +859,9 @@ cudaError_t launch_pairs(const Lin* l, const PairMaps<GROUPED>& maps, PairArgs& 
         a.out_mul = ldexpf(l->out_mul, l->fma_e);
     }
     if constexpr (!GROUPED) {
+        if (a.ks == 1 && a.halves) {
+            return cudaLaunchKernelEx(&cfg, l->group != 128 ? gemm_ts2_halves_kernel<32, false> : fma ? gemm_ts2_halves_kernel<128, true> : gemm_ts2_halves_kernel<128, false>, maps, a);
+        }
         if (a.ks > 1) {
             return cudaLaunchKernelEx(&cfg, l->group != 128 ? pair_split_kernel<32, false>(a.tok) : fma ? pair_split_kernel<128, true>(a.tok) : pair_split_kernel<128, false>(a.tok), maps, a);
         }
