@@ -358,3 +358,28 @@ def test_any_number_of_picks(dec, orc, k, t, e0):
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
     err = np.abs(y.cpu().numpy() - want).max()
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the tests above
+
+
+# Up to eight rows per expert on average, the last of them here, a batch takes the decode form, whose weights are exact nibbles and f32 scales; whichever
+# prefill form a key names.  The halves of the batch take it anyway, so both give the same rows but for the order of f32 sums: roundings to f16 that
+# fall the other way now and then, about 1e-4 in the 2-norm.  Weights rounded to f16 are 3e-4 off each, 6e-4 in the two matmuls.
+@pytest.mark.parametrize("moe_gemm", [0, 1, 128])
+@pytest.mark.parametrize("t,n_exp,k,f,h,group,local", [(30, 16, 4, 320, 576, 32, 16), (32, 16, 4, 320, 576, 64, 8), (58, 8, 1, 384, 640, 128, 8),
+                                                      (170, 128, 6, 448, 1024, 32, 128), (156, 160, 8, 192, 256, 32, 160)])
+def test_eight_rows_per_expert_keep_exact_weights(dec, t, n_exp, k, f, h, group, local, moe_gemm):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=91)
+    dec.set_moe(n_exp, k, f, h, group, 0, local)
+    dec.upload_experts(0, w13_q[:local], w13_s[:local], w2_q[:local], w2_s[:local])
+    x = torch.from_numpy(synth.make_acts(t, h, seed=92).view(np.float16).copy()).cuda()
+    lg = torch.from_numpy(synth.make_router_logits(t, n_exp, seed=93)).cuda()
+    assert 7 * n_exp < t * k <= 8 * n_exp
+    dec.set_tuning("moe_gemm", moe_gemm)
+    try:
+        y = dec.moe_ffn_dev_t(0, lg, x, t)
+        assert dec.last_kernel().startswith("gemv_moe_kernel"), dec.last_kernel()
+    finally:
+        dec.set_tuning("moe_gemm", 0)
+    half = t // 2
+    parts = torch.cat([dec.moe_ffn_dev_t(0, lg[:half], x[:half], half), dec.moe_ffn_dev_t(0, lg[half:], x[half:], t - half)])
+    dec.sync()
+    assert float((y - parts).norm()) <= 2e-4 * float(parts.norm())
