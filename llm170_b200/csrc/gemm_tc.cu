@@ -648,6 +648,25 @@ cudaError_t gemm_init_device() {
     return cudaSuccess;
 }
 
+// The line for pairs, which add all of K in one accumulator, in place of token rows that split K: of every tile or of the last wave's.  An accumulator
+// drops what lies below its last bit, so the error grows with the channels that go through one: such a call gives up precision for time, and only
+// those do that gained by it when a stage of 128 channels took a pair 0.317 us and more (groups of 32: 0.445).  The pairs' own estimate, with stages
+// of half that, would send calls here that have had their split all along.  f32 error of the results' size and us, token rows / pairs:
+// 12400 x 20224 at 238 tokens 7.9e-6, 108 / 2.4e-5, 100; 720 x 15424 in groups of 32 at 2005 3.1e-6, 57.5 / 1.8e-5, 41.8; 7168 x 17152 at 1521, a split
+// last wave, 1.89e-5, 274 / 2.01e-5, 256.
+static double one_sum_us(const Lin* l, int t, int sm_count) {
+    const int n_tiles = (l->n + 255) / 256, stages = (l->k + 2 * BK - 1) / (2 * BK), pairs = sm_count / 2;
+    double best = 1e30;
+    for (int cap = 256; cap >= 96; cap -= 32) {
+        const int m_tiles = (t + cap - 1) / cap, tok = ((t + m_tiles - 1) / m_tiles + 31) / 32 * 32;
+        const long long tiles = (long long)m_tiles * n_tiles, waves = (tiles + pairs - 1) / pairs;
+        const double full = std::min(1.0, std::max(0.0, ((double)tiles / (waves * pairs) - 0.41) / 0.52));
+        const double light = std::max(l->group == 128 ? 0.317 : 0.445, 0.00224 * tok), heavy = std::max(l->group == 128 ? 0.439 : 0.470, 0.082 + 0.00254 * tok);
+        best = std::min(best, 5.4 + waves * stages * (light + std::max(0.0, heavy - light) * full) + (waves - 1) * 1.7);
+    }
+    return best;
+}
+
 int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaStream_t st) {
     if (((uintptr_t)x & 15) != 0 || ((uintptr_t)dst & 15) != 0) {
         return fail("w4a16 gemm: x and dst must be 16-byte aligned");
@@ -771,7 +790,8 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                 if (p.ks > 0 && p.cost < (p.ks > 1 ? 1.0 : line) * c.cost) {
                     return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, true, st);
                 }
-            } else if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost)) {
+            } else if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost) &&
+                       (ts || best.ks == 1 || one_sum_us(l, t, sm_count) < 0.98 * best.cost)) {
                 if (out_kind == W4A16_OUT_F16) {
                     return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, false, st);
                 }

@@ -602,3 +602,29 @@ def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form
 @pytest.mark.parametrize("n,k,group,t", [(7168, 5120, 128, 197), (5120, 6144, 32, 197), (4096, 4096, 64, 320)])
 def test_pairs_in_place_of_split_weight_rows(dec, n, k, group, t):
     test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, PAIR, PAIR)
+
+
+# The error of f32 results grows with the channels that go through one accumulator (its sums drop what lies below its last bit).  The form that a call takes
+# adds no more of them than the one whose place it takes: token rows that split K of every tile or of the last wave's (form 1), weight rows that split K
+# over clusters (form 2).  1.05: what the sums' random part leaves between two orders of equal length.
+@pytest.mark.parametrize("n,k,group,t,form", [
+    (12400, 20224, 128, 238, 1), (720, 15424, 32, 2005, 1), (6032, 15104, 32, 184, 1), (144, 18688, 128, 3040, 1), (7168, 17152, 128, 1521, 1),
+    (7168, 5120, 128, 197, 2), (5120, 6144, 32, 197, 2), (4096, 4096, 64, 320, 2), (5120, 6144, 128, 96, 2), (5120, 17408, 128, 72, 2),
+    (3584, 18944, 32, 128, 2), (2560, 9728, 128, 250, 2)])
+def test_sums_are_no_longer_than_in_the_form_that_splits_k(dec, n, k, group, t, form):
+    q, s = synth.make_linear_cuda(n, k, group, 99, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("sums", q, s, n, k, group)
+    x = x_dev(synth.make_acts(t, k, seed=99, scale=1 / np.sqrt(k)))
+    y = dec.lin_forward("sums", x, t)
+    with forced(dec, "gemm_form", form):
+        other = dec.lin_forward("sums", x, t)
+        assert "split" in dec.last_kernel() or "cluster" in dec.last_kernel(), dec.last_kernel()
+    w = dec.dequant_lin("sums", f16=True)
+    dec.sync()
+    dec.drop_lin("sums")
+    err = [0.0, 0.0]
+    for r in range(0, n, 1024):
+        want = x.double() @ w[r:r + 1024].double().T
+        for i, v in enumerate((y, other)):
+            err[i] += float((v[:, r:r + 1024].double() - want).square().sum())
+    assert err[0] ** 0.5 <= 1.05 * err[1] ** 0.5, ((err[0] / err[1]) ** 0.5, dec.last_kernel())
