@@ -102,7 +102,8 @@ W4A16_API const char* w4a16_last_kernel(w4a16_dec* dec);
  *       default 31: the fused all-reduce gives up on its peers after 2^n cycles)
  * Keys of the GEMM above eight rows:
  *   "gemm_form" (0 = automatic, 1 = token rows, 2 = weight rows as the MMA's rows), "gemm_pair" (CTA pairs: 0 = automatic, 1 =
- *       never, 32..256 in steps of 32 = always, with tiles of that many tokens), "gemm_pair_ksplit" (their K splits: 0 = automatic, 1..4), "gemm_ts_tok" (weight rows, most tokens per tile:
+ *       never, 32..256 in steps of 32 = always, with tiles of that many tokens), "gemm_pair_ksplit" (their K splits: 0 = automatic, 1..4),
+ *       "gemm_pair_halves" (1 = with gemm_pair, sums in two halves where a pair has one tile of at most 128 tokens), "gemm_ts_tok" (weight rows, most tokens per tile:
  *       0 = automatic, 64, 96, 128, 192, 256), "gemm_ts_ksplit" (weight rows, K splits: 0 = automatic, 1..8), "gemm_bn" (token
  *       rows, weight rows per tile: 0 = automatic, 128..256 in steps of 32), "gemm_mt" (token rows, 128-token blocks per tile: 0 =
  *       automatic, 1, 2), "gemm_ksplit" (token rows, K splits: 0 = automatic -- all tiles when they are few, the tiles of an

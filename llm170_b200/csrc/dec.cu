@@ -777,6 +777,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
         d.tune_gemm_pair_ks = value;
         return 0;
     }
+    if (!strcmp(key, "gemm_pair_halves")) {
+        if (value != 0 && value != 1) {
+            return d.fail("w4a16 set_tuning: gemm_pair_halves=%d (0 or 1)", value);
+        }
+        d.tune_gemm_pair_halves = value;
+        return 0;
+    }
     if (!strcmp(key, "gemm_pair")) {
         if (value != 0 && value != 1 && (value < 32 || value > 256 || value % 32 != 0)) {
             return d.fail("w4a16 set_tuning: gemm_pair=%d (0, 1 or a multiple of 32 up to 256)", value);

@@ -113,6 +113,7 @@ struct Dec {
     int tune_gemm_tma_store = 1; // dense whole tiles leave through shared memory and TMA stores (0: per-lane stores)
     int tune_gemm_pair = 0;      // CTA pairs (gemm_ts2.cu): 0 = automatic, 1 = never, 32..256 = always, with tiles of that many tokens
     int tune_gemm_pair_ks = 0;   // ... K splits of a tile: 0 = automatic, 1 = never, with gemm_pair 1..4 = that many
+    int tune_gemm_pair_halves = 0;   // ... 1: with gemm_pair, sums in two halves where a pair has one tile of at most 128 tokens
     int tune_moe_gemm = 0;       // MoE prefill: 0 = automatic, 1 = weight rows, 2 = token rows, 128 / 192 / 256 = pairs, tiles of at most that many rows
     int tune_gemm_form = 0;      // above the decode rows: 0 = automatic, 1 = token rows (gemm_tc.cu), 2 = weight rows (gemm_ts.cu)
     int tune_gemm_bn = 0;        // gemm_tc.cu: weight rows per tile (128..256, a multiple of 32), 0 = automatic

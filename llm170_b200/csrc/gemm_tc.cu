@@ -673,7 +673,7 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
     }
     if (tune_gemm_pair > 1) {
         const int ks = std::min(std::max(tune_gemm_pair_ks, 1), (l->k + 2 * TILE_K - 1) / (2 * TILE_K));
-        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, ks, ks > 1, st);
+        return gemm_ts2(l, x, dst, t, out_kind, tune_gemm_pair, ks, ks > 1 || tune_gemm_pair_halves, st);
     }
     // Tile shape and K split are chosen together by a small cost model (microseconds, fitted to measurements on B200).  A
     // k-block takes 0.30 + 0.00105 bn with one 128-token block; with two, 0.295 + 0.00133 bn while at most 100 CTAs run and

@@ -909,7 +909,8 @@ int Dec::gemm_ts2(const Lin* l, const void* x, void* dst, int t, int out_kind, i
     if (e != cudaSuccess) {
         return cuda_fail("launch gemm", e);
     }
-    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(tok) + "-token tiles" + (ks > 1 ? ", ksplit " + std::to_string(ks) : "");
+    last_kernel = "gemm_ts2_kernel<" + std::to_string(l->group) + (l->fma_e >= 0 ? ",fma> " : "> ") + std::to_string(tok) + "-token tiles" + (ks > 1 ? ", ksplit " + std::to_string(ks) : "") +
+                  (a.halves ? ", sums in halves" : "");
     launches++;
     return 0;
 }

@@ -592,9 +592,12 @@ def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form
     dec.sync()
     assert torch.equal(y16, y32.half())
     assert name16.startswith(form16) and name32.startswith(form32), (name16, name32)
-    if n * k <= 1 << 24:
-        want = x.float() @ dec.dequant_lin("both", f16=True).float().T
-        assert (y32 - want).abs().max().item() <= 1e-4 * want.abs().max().item() + 1e-6
+    w = dec.dequant_lin("both", f16=True)
+    top, off = 0.0, 0.0
+    for r in range(0, n, 4096):
+        want = x.float() @ w[r:r + 4096].float().T
+        top, off = max(top, want.abs().max().item()), max(off, (y32[:, r:r + 4096] - want).abs().max().item())
+    assert off <= 1e-4 * top + 1e-6
     dec.drop_lin("both")
 
 
@@ -602,6 +605,7 @@ def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form
 @pytest.mark.parametrize("n,k,group,t", [(7168, 5120, 128, 197), (5120, 6144, 32, 197), (4096, 4096, 64, 320)])
 def test_pairs_in_place_of_split_weight_rows(dec, n, k, group, t):
     test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, PAIR, PAIR)
+    assert "ksplit" in dec.last_kernel() or "halves" in dec.last_kernel()
 
 
 # The error of f32 results grows with the channels that go through one accumulator (its sums drop what lies below its last bit).  The form that a call takes
@@ -628,3 +632,52 @@ def test_sums_are_no_longer_than_in_the_form_that_splits_k(dec, n, k, group, t, 
         for i, v in enumerate((y, other)):
             err[i] += float((v[:, r:r + 1024].double() - want).square().sum())
     assert err[0] ** 0.5 <= 1.05 * err[1] ** 0.5, ((err[0] / err[1]) ** 0.5, dec.last_kernel())
+
+
+# Sums in two halves, an accumulator each: one to ten stages (of one: no halves), odd numbers of them, a last stage of one k-block, ragged rows (also a second
+# half of a tile without any) and tokens, as many tiles as pairs; both expansions of groups of 128
+@pytest.mark.parametrize("t,k,n,group,tok,fma", [(9, 128, 16, 128, 32, True), (9, 256, 16, 128, 32, True), (33, 384, 144, 32, 32, False), (65, 320, 272, 64, 96, False),
+                                                 (128, 1088, 528, 64, 128, False), (97, 1280, 400, 128, 128, True), (97, 1280, 400, 128, 128, False),
+                                                 (200, 640, 784, 128, 128, True), (200, 896, 784, 128, 128, False), (300, 960, 1296, 32, 96, False),
+                                                 (256, 384, 9472, 128, 128, True)])
+@pytest.mark.parametrize("out_f16", [False, True])
+def test_sums_in_halves_pow2_exact(dec, t, k, n, group, tok, fma, out_f16):
+    q, s, x, expect = pow2_case(t, k, n, group)
+    if group == 128 and not fma:                                 # a seventh exponent: still exact, 2^-9 .. 2^14
+        s[0, 0] = 9 << 10
+        nib = (np.arange(128) * 7 % 16).astype(np.float64) - 8
+        expect[:, 0] += ((x[:, :128].view(np.float16).astype(np.float64) * nib).sum(axis=1) * (2.0 ** -6 - 1)).astype(np.float32)
+    dec.upload_lin_g("hv", q, s, n, k, group)
+    guard = torch.full((t + 16, n), 7.0, device="cuda", dtype=torch.float16 if out_f16 else torch.float32)
+    with forced(dec, "gemm_pair", tok), forced(dec, "gemm_pair_halves", 1):
+        for _ in range(2):
+            y = dec.lin_forward("hv", x_dev(x), t, dst=guard[:t], out_f16=out_f16)
+            name = dec.last_kernel()
+            dec.sync()
+            dec.kernel_status()
+    assert name.startswith("gemm_ts2_kernel<%d%s>" % (32 if group == 64 else group, ",fma" if fma else "")) and "halves" in name, name
+    assert np.array_equal(y.cpu().numpy(), expect.astype(np.float16) if out_f16 else expect)
+    assert (guard[t:] == 7.0).all()
+    dec.drop_lin("hv")
+
+
+# ... and on weights as they come: an even number of stages in halves is what two weight-row CTAs of a cluster add, in the same order
+@pytest.mark.parametrize("t,k,n,group,tok,odd", [(197, 5120, 7168, 128, 128, False), (197, 5120, 7168, 128, 128, True), (150, 1024, 2064, 32, 96, False),
+                                                 (250, 1536, 784, 64, 128, False)])
+def test_sums_in_halves_equal_two_weight_row_splits(dec, t, k, n, group, tok, odd):
+    q, s = synth.make_linear_cuda(n, k, group, 41, torch.device("cuda", 0))
+    if odd:
+        s[3, 1] = 0                                              # no multiply-add expansion
+    dec.upload_lin_g_dev("hw", q, s, n, k, group)
+    x = torch.randn((t, k), device="cuda", generator=torch.Generator("cuda").manual_seed(5)).half()
+    with forced(dec, "gemm_form", 2), forced(dec, "gemm_ts_ksplit", 2):
+        want = dec.lin_forward("hw", x, t)
+        assert dec.last_kernel().startswith("gemm_ts_kernel") and "clusters of 2" in dec.last_kernel()
+    for out_f16 in (False, True):
+        with forced(dec, "gemm_pair", tok), forced(dec, "gemm_pair_halves", 1):
+            y = dec.lin_forward("hw", x, t, out_f16=out_f16)
+            assert "halves" in dec.last_kernel() and ("fma" in dec.last_kernel()) == (group == 128 and not odd)
+        dec.sync()
+        assert torch.equal(y, want.half() if out_f16 else want)
+    dec.kernel_status()
+    dec.drop_lin("hw")
