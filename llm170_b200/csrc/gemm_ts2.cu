@@ -642,12 +642,12 @@ __device__ __forceinline__ void pair_gemm(const PairMaps<GROUPED>& maps, const P
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 1, %0;" ::"n"(P_EPI_WARPS * 32) : "memory");
-            const int col = glu ? tl.n0 / 2 : tl.n0, halves = rows_out == 0 ? 0 : glu || rows_out <= TS_MROWS / 2 ? 1 : 2;
+            const int col = glu ? tl.n0 / 2 : tl.n0, boxes = rows_out == 0 ? 0 : glu || rows_out <= TS_MROWS / 2 ? 1 : 2;
             for (int t0 = 0, u = (int)used0; t0 < tl.tok; t0 += n0, ++u) {
                 const int rows = min(min(n0, tl.tok - t0), tl.rows - t0), m0 = tl.m0 + t0;
                 const int whole = GROUPED ? rows & ~(P_OUT_BOX - 1) : rows;           // dense: what lies past the last token is not written
                 if (et == 0) {
-                    for (int hf = 0; hf < halves && ok; ++hf) {
+                    for (int hf = 0; hf < boxes && ok; ++hf) {
                         const uint32_t src = stage + (uint32_t)((u & 1) * P_OUT_STAGE + hf * P_OUT_HALF);
                         for (int r = 0; r < whole; r += P_OUT_BOX) {
                             tma_store_2d(&maps.out[0], src + (uint32_t)(r * 128), col + hf * 64, m0 + r);
