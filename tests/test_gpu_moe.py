@@ -180,15 +180,21 @@ def test_topk_near_ties_order_on_normalised_probabilities(dec, orc):
         assert np.allclose([w for _, w in want], wt[i], rtol=0, atol=2e-7)
 
 
-# prefill-sized batches below 192 rows per expert: weight-row tiles (gemm_ts.cu) over equal shares of an expert's rows
-@pytest.mark.parametrize("t,n_exp,k,f,h,group,local,kernel", [
-    (65, 16, 2, 64, 64, 32, 16, "gemm_ts"),        # just above the GEMV's rows; one 64-channel block, one stage, a half tile
-    (520, 8, 2, 320, 576, 32, 8, "gemm_ts"),       # odd numbers of k-blocks, last tiles of 64 rows, two shares per expert
-    (300, 4, 2, 192, 448, 64, 2, "gemm_ts"),       # half of the experts elsewhere; groups of 64
-    (767, 8, 2, 128, 256, 128, 8, "gemm_ts"),      # the last batch below the line ...
-    (768, 8, 2, 128, 256, 128, 8, "gemm_w4a16_tc"),   # ... and the first above it
+# weight-row tiles (gemm_ts.cu) over equal shares of an expert's rows, and the line to 256-row token tiles; `form`: named by its key where a call of that
+# size has another one by itself
+TS_TILES, TC_TILES, PAIR_TILES = "gemm_ts_grouped_kernel", "gemm_w4a16_tc_kernel", "gemm_ts2_kernel"
+
+
+@pytest.mark.parametrize("t,n_exp,k,f,h,group,local,form,kernel", [
+    (65, 16, 2, 64, 64, 32, 16, 0, TS_TILES),      # just above the GEMV's rows; one 64-channel block, one stage, a half tile
+    (520, 8, 2, 320, 576, 32, 8, 1, TS_TILES),     # odd numbers of k-blocks, last tiles of 64 rows, two shares per expert
+    (520, 8, 2, 320, 576, 32, 8, 0, PAIR_TILES),
+    (300, 4, 2, 192, 448, 64, 2, 1, TS_TILES),     # half of the experts elsewhere; groups of 64
+    (300, 4, 2, 192, 448, 64, 2, 0, PAIR_TILES),
+    (767, 8, 2, 128, 256, 128, 8, 0, TS_TILES),    # the last batch below the line ...
+    (768, 8, 2, 128, 256, 128, 8, 0, TC_TILES),    # ... and the first above it
 ])
-def test_expert_tiles_at_the_edges(dec, orc, t, n_exp, k, f, h, group, local, kernel):
+def test_expert_tiles_at_the_edges(dec, orc, t, n_exp, k, f, h, group, local, form, kernel):
     w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=7 + t)
     x, lg = synth.make_acts(t, h, seed=11 + t), synth.make_router_logits(t, n_exp, seed=13 + t)
     lg[: t // 2, 0] += 4.0                          # one expert with far more rows than the others
@@ -198,8 +204,12 @@ def test_expert_tiles_at_the_edges(dec, orc, t, n_exp, k, f, h, group, local, ke
         dec.set_moe(n_exp, k, f, h, group, e0, local)
         mine = slice(e0, e0 + local)
         dec.upload_experts(0, w13_q[mine], w13_s[mine], w2_q[mine], w2_s[mine])
-        y = dec.moe_ffn_dev_t(0, lgd, xd, t)
-        assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        dec.set_tuning("moe_gemm", form)
+        try:
+            y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+            assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        finally:
+            dec.set_tuning("moe_gemm", 0)
         assert dec.last_kernel().startswith(kernel)
         total = total + y.cpu().numpy()
     want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
@@ -307,8 +317,9 @@ def test_second_matmul_in_the_other_form(dec, orc, t, f, h, group):
 
 
 # MoE prefill on CTA pairs (gemm_ts2.cu): experts of 0, 1, 7, 8, ... rows around the steps of the stores (8, 32), of the accumulators (128), of the tiles
-# that are two MMAs (more than 224) and of the largest tiles; odd numbers of k-blocks, row tiles of 64 and 128 of 256 rows; half of the experts elsewhere
-@pytest.mark.parametrize("tile", [128, 192, 256])
+# that are two MMAs (more than 224) and of the largest tiles; odd numbers of k-blocks, row tiles of 64 and 128 of 256 rows; half of the experts elsewhere.
+# The same on weight rows (1) and token rows (2)
+@pytest.mark.parametrize("tile", [128, 192, 256, 1, 2])
 @pytest.mark.parametrize("f,h,group,local", [(320, 576, 32, 12), (128, 448, 64, 6), (384, 640, 128, 12)])
 def test_expert_tiles_on_pairs(dec, orc, tile, f, h, group, local):
     rows = [0, 33, 1, 129, 7, 225, 8, 257, 31, 300, 224, 96]
@@ -327,7 +338,7 @@ def test_expert_tiles_on_pairs(dec, orc, tile, f, h, group, local):
             dec.set_moe(n_exp, 1, f, h, group, e0, local)
             dec.upload_experts(0, w13_q[mine], w13_s[mine], w2_q[mine], w2_s[mine])
             y = dec.moe_ffn_dev_t(0, lgd, xd, t)
-            assert dec.last_kernel().startswith("gemm_ts2_kernel")
+            assert dec.last_kernel().startswith({1: TS_TILES, 2: TC_TILES}.get(tile, PAIR_TILES))
             assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t))
             total = total + y.cpu().numpy()
     finally:
@@ -383,3 +394,36 @@ def test_eight_rows_per_expert_keep_exact_weights(dec, t, n_exp, k, f, h, group,
     parts = torch.cat([dec.moe_ffn_dev_t(0, lg[:half], x[:half], half), dec.moe_ffn_dev_t(0, lg[half:], x[half:], t - half)])
     dec.sync()
     assert float((y - parts).norm()) <= 2e-4 * float(parts.norm())
+
+
+# Layers whose rings go round more than once, within a tile and from tile to tile (six to ten stages, the last of one k-block; more tiles than CTAs in the
+# first matmul): all prefill forms add the same channels in the same order and round at the same places, so they give the same bits
+@pytest.mark.parametrize("f,h,group,local", [(1216, 1088, 32, 12), (1344, 832, 64, 6), (1280, 1152, 128, 12)])
+def test_prefill_forms_of_the_experts_agree_to_the_bit(dec, f, h, group, local):
+    rows = [0, 33, 1, 129, 7, 225, 8, 257, 31, 300, 224, 96]
+    n_exp, t = len(rows), sum(rows)
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator("cuda").manual_seed(group)
+    lg = torch.randn((t, n_exp), device=dev, generator=gen)
+    lg[torch.arange(t, device=dev), torch.repeat_interleave(torch.arange(n_exp), torch.tensor(rows)).to(dev)[torch.randperm(t, device=dev, generator=gen)]] += 40.0
+    x = torch.randn((t, h), device=dev, generator=gen).half()
+    e0 = n_exp - local
+    dec.set_moe(n_exp, 1, f, h, group, e0, local)
+    q13, s13 = synth.make_linear_cuda(local * 2 * f, h, group, 5, dev)
+    q2, s2 = synth.make_linear_cuda(local * h, f, group, 6, dev)
+    dec.upload_experts(0, q13, s13, q2, s2)
+    ys = {}
+    try:
+        for form in (1, 2, 128, 192, 256):
+            dec.set_tuning("moe_gemm", form)
+            ys[form] = dec.moe_ffn_dev_t(0, lg, x, t)
+            assert dec.last_kernel().startswith({1: TS_TILES, 2: TC_TILES}.get(form, PAIR_TILES))
+            assert torch.equal(ys[form], dec.moe_ffn_dev_t(0, lg, x, t))
+    finally:
+        dec.set_tuning("moe_gemm", 0)
+    dec.sync()
+    dec.kernel_status()
+    here = sum(rows[e0:])
+    assert int((ys[1].abs().amax(dim=1) > 0).sum()) == here              # rows of the experts elsewhere are zero
+    for form in (2, 128, 192, 256):
+        assert torch.equal(ys[form], ys[1]), form
