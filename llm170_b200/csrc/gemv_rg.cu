@@ -219,7 +219,13 @@ const RgKernel& rg_kernel(int group, const RgPlan& p) {
     return rg_kernels[(group == 128 ? 0 : 24) + (p.kw == 4 ? 0 : 12) + (p.nr - 2) * 4 + (p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
 }
 
+// What a plan may take, the padding of the sums aside: it comes from what is left above, so that it costs no ring slot, no warp along K and no second CTA
+// on the SM.  (Counted in, it did: 448 x 12608 in groups of 32 at eight tokens 9.2 -> 14.9 us, with four warps along K; 8352 x 22528 at one token 26.5 ->
+// 31.8, one CTA per SM.)
 constexpr int RG_SMEM_MAX = 224 * 1024, RG_SMEM_TWO = 112 * 1024;
+// What a CTA can have, alone on its SM and beside another one: 227 KB, half of 228 KB less 1 KB, and less the barrier and the flag.
+constexpr int RG_SMEM_MAX_HW = 227 * 1024 - 128, RG_SMEM_TWO_HW = 113 * 1024 - 128, RG_PAD_MAX = RG_WARPS * GEMV_MAX_M * RG_RED_PAD * 4;
+static_assert(RG_SMEM_MAX + RG_PAD_MAX <= RG_SMEM_MAX_HW, "room for the padding");
 // us per k-block of two, three, four row blocks: a CTA alone on its SM, two; groups of 128, of 32
 constexpr double RG_STEP_US[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.437}}, {{0.44, 0.53, 0.64}, {0.49, 0.60, 0.742}}};
 
@@ -249,11 +255,13 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
                 p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
             }
             p.off_red = x_bytes;
-            p.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
+            const int padding = kw * mp * RG_RED_PAD * 4;
+            p.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) - padding + 127) & ~127;
             const double tiles = (double)((ku + kw - 1) / kw * (unit_k / TILE_K) * nr) * (nr == 2 ? 1.3 : nr == 3 ? 1.05 : 1.0);
             for (int per_sm = 1; per_sm <= 2; ++per_sm) {
                 const int room = per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX;
-                if (p.off_ring + 2 * RG_WARPS * slot > room || (per_sm == 2 && p.units <= sm_count)) {
+                const int least = p.off_ring + 2 * RG_WARPS * slot;
+                if (least > room || (per_sm == 2 && (p.units <= sm_count || least + padding > RG_SMEM_TWO_HW))) {
                     continue;
                 }
                 p.ctas = std::min(p.units, per_sm * sm_count);
@@ -264,7 +272,8 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
                     best = p;
                     // alone: as deep a ring as fits; two: two slots (four measured the same)
                     best.depth = per_sm == 2 ? 2 : p.off_ring + 6 * RG_WARPS * slot <= room ? 6 : p.off_ring + 4 * RG_WARPS * slot <= room ? 4 : 2;
-                    best.smem = p.off_ring + best.depth * RG_WARPS * slot;
+                    best.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
+                    best.smem = best.off_ring + best.depth * RG_WARPS * slot;
                     if (per_sm == 1) {
                         best.smem = std::max(best.smem, RG_SMEM_TWO + 2048);      // no second CTA of this launch on the SM
                     }
@@ -286,7 +295,7 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
 
 // Estimated time of a plan, K from 8192 on.
 static double rg_us(const GemvArgs& a, const RgPlan& p, int sm_count) {
-    const bool g32 = a.group == 32, two = p.smem <= RG_SMEM_TWO;
+    const bool g32 = a.group == 32, two = p.smem <= RG_SMEM_TWO_HW;
     const int unit_k = a.group > TILE_K ? a.group : TILE_K, chain = (a.k / unit_k + p.kw - 1) / p.kw * (unit_k / TILE_K);
     const int rounds = (p.units + p.ctas - 1) / p.ctas;
     const double step = RG_STEP_US[two][g32][p.nr - 2] + (!two && p.depth == 2 ? (p.nr == 2 ? 0.085 : 0.04) : 0.0);
@@ -388,7 +397,7 @@ const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(group, p
 
 cudaError_t gemv_rg_init_device() {
     for (const RgKernel& k : rg_kernels) {
-        const cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM_MAX);
+        const cudaError_t e = cudaFuncSetAttribute(k.f, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM_MAX + RG_PAD_MAX);
         if (e != cudaSuccess) {
             return e;
         }

@@ -17,7 +17,8 @@ __host__ __device__ constexpr int rg_slot_bytes(int group, int nr) { return rg_w
 // g + 8 of two tokens -- goes to 32 banks, and consecutive rows come from 32.  As [row][token] every read of eight tokens' sums was an 8-way
 // conflict, 1024 cycles a unit with eight warps along K: eight tokens of 7168 x 5120 7.6 -> 7.1 us, of 5120 x 17408 15.5 -> 14.6, of 2048 x 2048
 // 3.0 -> 2.8; up to six tokens the same.
-__host__ __device__ constexpr int rg_red_pitch(int ur) { return ur * TILE_ROWS + 4; }
+constexpr int RG_RED_PAD = 4;
+__host__ __device__ constexpr int rg_red_pitch(int ur) { return ur * TILE_ROWS + RG_RED_PAD; }
 __host__ __device__ constexpr int rg_red_bytes(int kw, int ur, int tokens) { return kw * tokens * rg_red_pitch(ur) * 4; }
 template <int NR>
 __device__ __forceinline__ void rg_store_sums(float* d, int pitch, const float (&tot)[NR][4], float m0, float m1) {

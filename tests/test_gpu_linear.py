@@ -604,6 +604,31 @@ def test_row_group_form_leaves_what_does_not_fit(dec, orc):
     dec.drop_lin("rgx")
 
 
+# Plans at the edge of shared memory: the padding of the warps' sums costs no warp along K, no ring slot, not the form itself, and no second CTA of an SM
+# (its sums then start past 112 KB a CTA; 12400 x 5312 at seven tokens: as much as two CTAs can have, 113 KB less the barrier)
+@pytest.mark.parametrize("n,k,group,t,plan", [(448, 12608, 32, 8, "32,8,2,2"), (1312, 14464, 32, 7, "32,8,2,2"), (6432, 13952, 128, 6, "128,8,3,4"),
+                                              (2896, 10304, 32, 8, "32,8,2,6"), (16528, 4352, 64, 7, "32,8,4,2"), (12400, 5312, 32, 7, "32,8,3,2")])
+def test_row_group_plans_at_the_edge_of_shared_memory(dec, n, k, group, t, plan):
+    q, s = synth.make_linear_cuda(n, k, group, 960, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("rge", q, s, n, k, group)
+    x = x_dev(synth.make_acts(t, k, seed=961))
+    guard = torch.full((t + 1, n), 7.0, device="cuda", dtype=torch.float32)
+    y = dec.lin_forward("rge", x, t, dst=guard[:t])
+    assert dec.last_kernel() == f"gemv_rg_kernel<{plan}>"
+    dec.set_tuning("gemv_rowgroup", 0)
+    try:
+        other = dec.lin_forward("rge", x, t)
+        assert not dec.last_kernel().startswith("gemv_rg_kernel")
+    finally:
+        dec.set_tuning("gemv_rowgroup", 1)
+    dec.sync()
+    dec.kernel_status()
+    size = (x.float().abs() @ dec.dequant_lin("rge").abs().T).max().item()
+    assert (y - other).abs().max().item() <= 2.0 ** -18 * size                # f32 sums in another order, as in the tests of the corners
+    assert bool((guard[t:] == 7.0).all())
+    dec.drop_lin("rge")
+
+
 # The row-group form over clusters: K that does not divide by the CTAs or their warps (one has no k-blocks), odd numbers of k-blocks, units that the last
 # rows do not fill, more units than clusters, several linears at once, one to eight tokens, every group size -- and x that does not fit, by itself
 @pytest.mark.parametrize("n,k,group,t,cl", [(16, 256, 128, 1, 2), (272, 704, 32, 3, 5), (1040, 1152, 64, 8, 8), (528, 4992, 128, 5, 7), (20000, 512, 128, 2, 3),
