@@ -220,9 +220,12 @@ const RgKernel& rg_kernel(int group, const RgPlan& p) {
 }
 
 // What a plan may take, the padding of the sums aside: it comes from what is left above, so that it costs no ring slot, no warp along K and no second CTA
-// on the SM.  (Counted in, it did: 448 x 12608 in groups of 32 at eight tokens 9.2 -> 14.9 us, with four warps along K; 8352 x 22528 at one token 26.5 ->
-// 31.8, one CTA per SM.)
+// on the SM.  (Counted in, it did: 448 x 12608 in groups of 32 at eight tokens 9.2 -> 14.9 us, with four warps along K; 34032 x 6528 at five 26.3 ->
+// 31.5, with two row blocks a warp.)
 constexpr int RG_SMEM_MAX = 224 * 1024, RG_SMEM_TWO = 112 * 1024;
+// Two CTAs on an SM ask for more than a third of it: kernels of two row blocks a warp have registers for three, and the third place of some SMs went to the
+// next launch's first CTAs, which then ended later than those of the others: 8352 x 22528 in groups of 64 at one token 26.5 us, with three 31.5.
+constexpr int RG_SMEM_NOT_THREE = 77 * 1024;
 // What a CTA can have, alone on its SM and beside another one: 227 KB, half of 228 KB less 1 KB, and less the barrier and the flag.
 constexpr int RG_SMEM_MAX_HW = 227 * 1024 - 128, RG_SMEM_TWO_HW = 113 * 1024 - 128, RG_PAD_MAX = RG_WARPS * GEMV_MAX_M * RG_RED_PAD * 4;
 static_assert(RG_SMEM_MAX + RG_PAD_MAX <= RG_SMEM_MAX_HW, "room for the padding");
@@ -274,9 +277,8 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
                     best.depth = per_sm == 2 ? 2 : p.off_ring + 6 * RG_WARPS * slot <= room ? 6 : p.off_ring + 4 * RG_WARPS * slot <= room ? 4 : 2;
                     best.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
                     best.smem = best.off_ring + best.depth * RG_WARPS * slot;
-                    if (per_sm == 1) {
-                        best.smem = std::max(best.smem, RG_SMEM_TWO + 2048);      // no second CTA of this launch on the SM
-                    }
+                    // no second CTA of this launch on the SM, or no third one
+                    best.smem = std::max(best.smem, per_sm == 1 ? RG_SMEM_TWO + 2048 : RG_SMEM_NOT_THREE);
                 }
             }
         }
@@ -368,7 +370,7 @@ bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& 
                     continue;
                 }
                 p.depth = 2;                                  // (four slots, where they fit, were not faster: 4096 x 14336 11.9 / 11.4 us)
-                p.smem = p.off_ring + p.depth * RG_WARPS * slot;
+                p.smem = std::max(p.off_ring + p.depth * RG_WARPS * slot, RG_SMEM_NOT_THREE);
                 const int at_once = std::min(p.units, room), rounds = (p.units + at_once - 1) / at_once;
                 p.ctas = at_once * cl;
                 // (fitted to 28 launches of 3072 to 24576 rows, 4 % on average: the sums of eight warps take longer)

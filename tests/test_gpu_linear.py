@@ -629,6 +629,34 @@ def test_row_group_plans_at_the_edge_of_shared_memory(dec, n, k, group, t, plan)
     dec.drop_lin("rge")
 
 
+# A plan for two CTAs on an SM gets two: kernels that have registers for three ask for more than a third of the shared memory, or the next launch's first CTAs
+# take the third places of some SMs and keep them busy longer than the others
+@pytest.mark.parametrize("n,k,group", [(8352, 22528, 64), (4816, 512, 32), (9472, 2048, 128)])
+def test_no_third_row_group_cta_on_an_sm(dec, n, k, group):
+    q, s = synth.make_linear_cuda(n, k, group, 970, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("rg3", q, s, n, k, group)
+    x = x_dev(synth.make_acts(1, k, seed=971))
+    y = torch.empty((1, n), device="cuda", dtype=torch.float16)
+    dec.sync()
+    dec.set_tuning("debug_timeline", 1)
+    dec.set_tuning("gemv_rowgroup", 1 + 2 + 16 * 8)
+    try:
+        c0 = dec.launch_count()
+        for _ in range(12):
+            dec.lin_forward("rg3", x, 1, dst=y, out_f16=True)
+        dec.sync()
+        assert dec.last_kernel().startswith("gemv_rg_kernel<%d,8,2," % (128 if group == 128 else 32))
+        tl = dec.debug_timeline().reshape(64, 384, 16)
+    finally:
+        dec.set_tuning("gemv_rowgroup", 1)
+        dec.set_tuning("debug_timeline", 0)
+    units = -(-n // 32)
+    for c in range(c0, c0 + 12):
+        sms = tl[c % 64, :units, 6]
+        assert np.bincount(sms.astype(np.int64)).max() <= 2
+    dec.drop_lin("rg3")
+
+
 # The row-group form over clusters: K that does not divide by the CTAs or their warps (one has no k-blocks), odd numbers of k-blocks, units that the last
 # rows do not fill, more units than clusters, several linears at once, one to eight tokens, every group size -- and x that does not fit, by itself
 @pytest.mark.parametrize("n,k,group,t,cl", [(16, 256, 128, 1, 2), (272, 704, 32, 3, 5), (1040, 1152, 64, 8, 8), (528, 4992, 128, 5, 7), (20000, 512, 128, 2, 3),
