@@ -648,13 +648,10 @@ cudaError_t gemm_init_device() {
     return cudaSuccess;
 }
 
-// The line for pairs, which add all of K in one accumulator, in place of token rows that split K: of every tile or of the last wave's.  An accumulator
-// drops what lies below its last bit, so the error grows with the channels that go through one: such a call gives up precision for time, and only
-// those do that gained by it when a stage of 128 channels took a pair 0.317 us and more (groups of 32: 0.445).  The pairs' own estimate, with stages
-// of half that, would send calls here that have had their split all along.  f32 error of the results' size and us, token rows / pairs:
-// 12400 x 20224 at 238 tokens 7.9e-6, 108 / 2.4e-5, 100; 720 x 15424 in groups of 32 at 2005 3.1e-6, 57.5 / 1.8e-5, 41.8; 7168 x 17152 at 1521, a split
-// last wave, 1.89e-5, 274 / 2.01e-5, 256.
-static double one_sum_us(const Lin* l, int t, int sm_count) {
+// What the pairs without K splits were first estimated to take, when a stage of 128 channels took them 0.317 us and more (groups of 32: 0.445).  The
+// estimate of gemm_ts2_choose has stages of half that.  This one still draws the line where that one is no guide: where pairs give up precision for
+// time, and where calls had been theirs that the other, outside of what it was fitted to, would give away.
+static double pairs_first_us(const Lin* l, int t, int out_kind, int sm_count) {
     const int n_tiles = (l->n + 255) / 256, stages = (l->k + 2 * BK - 1) / (2 * BK), pairs = sm_count / 2;
     double best = 1e30;
     for (int cap = 256; cap >= 96; cap -= 32) {
@@ -662,7 +659,8 @@ static double one_sum_us(const Lin* l, int t, int sm_count) {
         const long long tiles = (long long)m_tiles * n_tiles, waves = (tiles + pairs - 1) / pairs;
         const double full = std::min(1.0, std::max(0.0, ((double)tiles / (waves * pairs) - 0.41) / 0.52));
         const double light = std::max(l->group == 128 ? 0.317 : 0.445, 0.00224 * tok), heavy = std::max(l->group == 128 ? 0.439 : 0.470, 0.082 + 0.00254 * tok);
-        best = std::min(best, 5.4 + waves * stages * (light + std::max(0.0, heavy - light) * full) + (waves - 1) * 1.7);
+        const double f32 = out_kind == W4A16_OUT_F16 ? 0.0 : 0.0263 * tok - 3.23;
+        best = std::min(best, 5.4 + waves * (stages * (light + std::max(0.0, heavy - light) * full) + f32) + (waves - 1) * 1.7);
     }
     return best;
 }
@@ -776,14 +774,19 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // the three adds the channels of a sum in the same order: from the pairs where the weight rows would split K.  Otherwise they keep the
             // form that they have without the pairs, unless that splits tiles: then the token-row form without a split, or the pairs where a nearly
             // empty last wave is what the split was for (its estimate leaves out that the full waves hold the clock down) or where they are ahead
-            // by a clear margin (their estimate for f32 results is good to a tenth).  f32, us with the split / without / pairs: 7168 x 5120 at 4096
-            // tokens 235 / 257 / 230, at 3000 185 / 218 / 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512; 5120 x 6144 at 4096,
-            // 2.92 waves, 206 / 205 / 193.
+            // by a clear margin (their estimate for f32 results is good to a tenth), or were by their first estimate.  f32, us with the split / without /
+            // pairs: 7168 x 5120 at 4096 tokens 235 / 257 / 230, at 3000 185 / 218 / 170; 5120 x 17408 at 2048 269 / 314 / 256, at 4096 524 / 566 / 512;
+            // 5120 x 6144 at 4096, 2.92 waves, 206 / 205 / 193.  Over 140 drawn calls the pairs took 0.36 to 0.93 of the tiles without a split; 12 of
+            // them the margin alone would leave there (5632 x 8064 at 3517 tokens 253 / 225, 11120 x 9472 at 1183 194 / 174).
             const double line = t <= 128 ? 0.8 : !ts ? 0.98 : c.ks > 1 ? 0.84 : t < 256 ? 0.9 : 0.92;
             // In place of weight rows that split K: pairs whose accumulators take no more stages each (gemm_ts2), results of either kind from the
             // same tiles.  Below 256 tokens of more than 2^24 weights these may split K, too: few tiles (101 calls of both kinds take 0.89 of the time).
             // Smaller linears gain little or lose: 1792 x 5120 at 100 tokens 9.4 / 9.2 us, 4096 x 4096 11.1 / 10.8, 1024 x 4096 7.4 / 6.5; from 256
             // tokens on f32 results keep the forms that the tests name.
+            // In place of token rows that split K, of every tile or of the last wave's: an accumulator drops what lies below its last bit, so the error grows
+            // with the channels that go through one, and only the calls give up that split that did so from the first.  f32 error of the results' size
+            // and us, token rows / pairs: 12400 x 20224 at 238 tokens 7.9e-6, 108 / 2.4e-5, 100; 720 x 15424 in groups of 32 at 2005 3.1e-6, 57.5 /
+            // 1.8e-5, 41.8; 7168 x 17152 at 1521, a split last wave, 1.89e-5, 274 / 2.01e-5, 256.
             if (ts && c.ks > 1) {
                 const bool may_split = t < 256 && (long long)l->n * l->k > 16 << 20 && tune_gemm_pair_ks != 1;
                 const TsChoice p = gemm_ts2_choose(l, t, W4A16_OUT_F16, may_split ? 4 : 1, c.ks);
@@ -791,14 +794,15 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
                     return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, true, st);
                 }
             } else if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost) &&
-                       (ts || best.ks == 1 || one_sum_us(l, t, sm_count) < 0.98 * best.cost)) {
+                       (ts || best.ks == 1 || pairs_first_us(l, t, W4A16_OUT_F16, sm_count) < 0.98 * best.cost)) {
                 if (out_kind == W4A16_OUT_F16) {
                     return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, false, st);
                 }
                 if (!ts && best.cost < whole.cost) {
                     const TsChoice p = gemm_ts2_choose(l, t, out_kind, 1);
                     const int rest = (t + BM * whole.mt - 1) / (BM * whole.mt) * ((l->n + whole.bn - 1) / whole.bn) % sm_count;
-                    if (p.cost < whole.cost * (rest > 0 && rest <= 100 ? 1.0 : 0.78)) {
+                    const bool empty = rest > 0 && rest <= 100;
+                    if (p.cost < whole.cost * (empty ? 1.0 : 0.78) || pairs_first_us(l, t, out_kind, sm_count) < whole.cost * (empty ? 1.0 : 0.86)) {
                         return gemm_ts2(l, x, dst, t, out_kind, p.tok, 1, false, st);
                     }
                     best = whole;

@@ -580,7 +580,9 @@ TC, TS, PAIR = "gemm_w4a16_tc_kernel", "gemm_ts_kernel", "gemm_ts2_kernel"
     (34816, 1024, 128, 64, TS, TS), (34816, 1024, 128, 65, TS, TS), (12288, 2048, 128, 197, TS, TS), (7168, 5120, 128, 256, PAIR, TS),
     (5120, 17408, 128, 300, TS, TS), (2144, 16384, 128, 526, TS, TS), (2048, 2048, 128, 1024, PAIR, TS), (7168, 5120, 128, 1500, PAIR, PAIR),
     (7168, 5120, 32, 3000, PAIR, PAIR), (7168, 5120, 128, 4096, PAIR, PAIR), (5120, 6144, 128, 4096, PAIR, TC), (5120, 6144, 128, 4097, TC, TC),
-    (12288, 2048, 64, 2048, PAIR, TC), (8704, 5120, 32, 512, PAIR, TS)])
+    (12288, 2048, 64, 2048, PAIR, TC), (8704, 5120, 32, 512, PAIR, TS),
+    # f32 results whose form without the pairs splits its last wave, and is slower without it than they are
+    (5632, 8064, 128, 3517, PAIR, PAIR), (11120, 9472, 128, 1183, PAIR, PAIR)])
 def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form32):
     q, s = synth.make_linear_cuda(n, k, group, 97, torch.device("cuda", 0))
     dec.upload_lin_g_dev("both", q, s, n, k, group)
