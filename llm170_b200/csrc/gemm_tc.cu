@@ -768,8 +768,9 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // in the median, so the line lies at 0.92 of them, 0.9 below 256 tokens, at 0.84 where they split K over clusters, and at 0.8 up to 128
             // tokens, where a wrong choice costs most.  Over 308 measured calls (22 shapes, 72..3000 tokens) the choice takes 1.0 % more than the
             // best form and tile of each; with a line that ended at split calls, and the estimates before it, it took 7.2 %.  Split calls of
-            // K >= 16384, and up to 320 tokens of linears of up to 2^20 weights, stay with the weight rows, as the tests name them (256 x 5120 x
-            // 17408: 44 us, pairs of 96 tokens 40).  Up to 64 and above 4096 tokens the pairs were not compared.
+            // K >= 16384 from 256 tokens on, and up to 320 tokens of linears of up to 2^20 weights, stay with the weight rows, as the tests name them
+            // (256 x 5120 x 17408: 44 us, pairs of 96 tokens 40; 300 x 1024 x 1024: 5.0, 4.4).  Up to 64 and above 4096 tokens the pairs were not
+            // compared.
             // The f32 results of such a call are what its f16 results are rounded from, so they come from a form without a K split, too -- each of
             // the three adds the channels of a sum in the same order: from the pairs where the weight rows would split K.  Otherwise they keep the
             // form that they have without the pairs, unless that splits tiles: then the token-row form without a split, or the pairs where a nearly
@@ -787,14 +788,24 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // with the channels that go through one, and only the calls give up that split that did so from the first.  f32 error of the results' size
             // and us, token rows / pairs: 12400 x 20224 at 238 tokens 7.9e-6, 108 / 2.4e-5, 100; 720 x 15424 in groups of 32 at 2005 3.1e-6, 57.5 /
             // 1.8e-5, 41.8; 7168 x 17152 at 1521, a split last wave, 1.89e-5, 274 / 2.01e-5, 256.
+            // In place of unsplit weight rows up to 16 stages long the estimates, which were fitted from 12 stages on, are no guide by themselves: their
+            // launches take 2 us less than estimated, those of pairs no less.  us, weight rows / pairs: 11264 x 512 at 315 tokens 7.0 / 8.8, 3808 x 512 at
+            // 250 4.3 / 5.2, 7344 x 896 at 82 5.2 / 5.9, 17664 x 1408 at 126 10.8 / 9.5.  Over 362 such calls the choice takes 1.1 % more than the better
+            // form, without the 2 us 4.5 %.
+            auto unsplit_pairs = [&]() {
+                const double p_us = gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost, first = pairs_first_us(l, t, W4A16_OUT_F16, sm_count);
+                if (!ts) {
+                    return p_us < line * best.cost && (best.ks == 1 || first < 0.98 * best.cost);
+                }
+                return l->k <= 16 * 2 * BK ? p_us < c.cost - 2.0 || first < 0.98 * c.cost : p_us < line * c.cost;
+            };
             if (ts && c.ks > 1) {
                 const bool may_split = t < 256 && (long long)l->n * l->k > 16 << 20 && tune_gemm_pair_ks != 1;
                 const TsChoice p = gemm_ts2_choose(l, t, W4A16_OUT_F16, may_split ? 4 : 1, c.ks);
                 if (p.ks > 0 && p.cost < (p.ks > 1 ? 1.0 : line) * c.cost) {
                     return gemm_ts2(l, x, dst, t, out_kind, p.tok, p.ks, true, st);
                 }
-            } else if (gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost < line * (ts ? c.cost : best.cost) &&
-                       (ts || best.ks == 1 || pairs_first_us(l, t, W4A16_OUT_F16, sm_count) < 0.98 * best.cost)) {
+            } else if (unsplit_pairs()) {
                 if (out_kind == W4A16_OUT_F16) {
                     return gemm_ts2(l, x, dst, t, out_kind, gemm_ts2_choose(l, t, out_kind, 1).tok, 1, false, st);
                 }

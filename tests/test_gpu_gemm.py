@@ -581,6 +581,8 @@ TC, TS, PAIR = "gemm_w4a16_tc_kernel", "gemm_ts_kernel", "gemm_ts2_kernel"
     (5120, 17408, 128, 300, TS, TS), (2144, 16384, 128, 526, TS, TS), (2048, 2048, 128, 1024, PAIR, TS), (7168, 5120, 128, 1500, PAIR, PAIR),
     (7168, 5120, 32, 3000, PAIR, PAIR), (7168, 5120, 128, 4096, PAIR, PAIR), (5120, 6144, 128, 4096, PAIR, TC), (5120, 6144, 128, 4097, TC, TC),
     (12288, 2048, 64, 2048, PAIR, TC), (8704, 5120, 32, 512, PAIR, TS),
+    # launches of few stages, on both sides of their line, and in place of token rows
+    (11264, 512, 128, 315, TS, TS), (3808, 512, 64, 250, TS, TS), (7344, 896, 128, 82, TS, TS), (28544, 1280, 64, 324, PAIR, TS), (19536, 768, 128, 173, PAIR, TC),
     # f32 results whose form without the pairs splits its last wave, and is slower without it than they are
     (5632, 8064, 128, 3517, PAIR, PAIR), (11120, 9472, 128, 1183, PAIR, PAIR)])
 def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form32):
