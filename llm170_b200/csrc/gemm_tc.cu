@@ -791,13 +791,15 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // In place of unsplit weight rows up to 16 stages long the estimates, which were fitted from 12 stages on, are no guide by themselves: their
             // launches take 2 us less than estimated, those of pairs no less.  us, weight rows / pairs: 11264 x 512 at 315 tokens 7.0 / 8.8, 3808 x 512 at
             // 250 4.3 / 5.2, 7344 x 896 at 82 5.2 / 5.9, 17664 x 1408 at 126 10.8 / 9.5.  Over 362 such calls the choice takes 1.1 % more than the better
-            // form, without the 2 us 4.5 %.
+            // form, without the 2 us 4.5 %.  Above 100 us the power limit holds the clock down, which the weight rows' estimate leaves out: 5296 x 6656 at
+            // 2478 tokens 128 / 117, 10720 x 6400 at 1218 124 / 114; where the pairs are estimated at 0.92 to 0.95 of it they took 0.91 to 1.03 there, below
+            // 100 us 0.98 to 1.06.
             auto unsplit_pairs = [&]() {
                 const double p_us = gemm_ts2_choose(l, t, W4A16_OUT_F16, 1).cost, first = pairs_first_us(l, t, W4A16_OUT_F16, sm_count);
                 if (!ts) {
                     return p_us < line * best.cost && (best.ks == 1 || first < 0.98 * best.cost);
                 }
-                return l->k <= 16 * 2 * BK ? p_us < c.cost - 2.0 || first < 0.98 * c.cost : p_us < line * c.cost;
+                return l->k <= 16 * 2 * BK ? p_us < c.cost - 2.0 || first < 0.98 * c.cost : p_us < (c.cost > 100.0 ? 0.98 : line) * c.cost;
             };
             if (ts && c.ks > 1) {
                 const bool may_split = t < 256 && (long long)l->n * l->k > 16 << 20 && tune_gemm_pair_ks != 1;

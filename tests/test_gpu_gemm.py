@@ -583,6 +583,8 @@ TC, TS, PAIR = "gemm_w4a16_tc_kernel", "gemm_ts_kernel", "gemm_ts2_kernel"
     (12288, 2048, 64, 2048, PAIR, TC), (8704, 5120, 32, 512, PAIR, TS),
     # launches of few stages, on both sides of their line, and in place of token rows
     (11264, 512, 128, 315, TS, TS), (3808, 512, 64, 250, TS, TS), (7344, 896, 128, 82, TS, TS), (28544, 1280, 64, 324, PAIR, TS), (19536, 768, 128, 173, PAIR, TC),
+    # long calls near a tie of the estimates
+    (5296, 6656, 128, 2478, PAIR, TS), (10720, 6400, 64, 1218, PAIR, TS),
     # f32 results whose form without the pairs splits its last wave, and is slower without it than they are
     (5632, 8064, 128, 3517, PAIR, PAIR), (11120, 9472, 128, 1183, PAIR, PAIR)])
 def test_automatic_form_of_f16_and_f32_results(dec, n, k, group, t, form16, form32):
