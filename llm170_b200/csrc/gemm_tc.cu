@@ -771,8 +771,9 @@ int Dec::gemm(const Lin* l, const void* x, void* dst, int t, int out_kind, cudaS
             // K >= 16384 from 256 tokens on, and up to 320 tokens of linears of up to 2^20 weights, stay with the weight rows, as the tests name them
             // (256 x 5120 x 17408: 44 us, pairs of 96 tokens 40; 300 x 1024 x 1024: 5.0, 4.4).  Up to 64 and above 4096 tokens the pairs were not
             // compared.
-            // The f32 results of such a call are what its f16 results are rounded from, so they come from a form without a K split, too -- each of
-            // the three adds the channels of a sum in the same order: from the pairs where the weight rows would split K.  Otherwise they keep the
+            // The f32 results of such a call are what its f16 results are rounded from.  Where the weight rows would split K, results of either kind get the same
+            // tiles, K splits and accumulators: the choice is made once, with the estimates for f16 results.  Otherwise f16 results come from pairs
+            // without a K split, and f32 results from any form without one -- each of the three then adds the channels of a sum in the same order: the
             // form that they have without the pairs, unless that splits tiles: then the token-row form without a split, or the pairs where a nearly
             // empty last wave is what the split was for (its estimate leaves out that the full waves hold the clock down) or where they are ahead
             // by a clear margin (their estimate for f32 results is good to a tenth), or were by their first estimate.  f32, us with the split / without /

@@ -163,9 +163,9 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         // <=8-row segment of an expert runs through the GEMV kernel instead of a padded MMA tile.  The line is one of precision, too: the segments
         // multiply by the exact nibbles and keep the scales in f32, the MMA tiles round every weight to f16.  Error against 64 bits, segments / pairs,
         // of 128 experts, top-8, 2048 x 768 at 120 tokens 5.27e-4 / 6.13e-4, of 64 experts (32 here), top-6, 1024 x 576 at 80 5.20e-4 / 6.00e-4.  So the
-        // pairs do not take the calls from 7 rows on, where they would be 4 to 15 % sooner (us per layer, segments / pairs: 128 experts, top-8,
-        // 2048 x 768, 6.9 rows 108 / 110, 8 rows 116 / 111; 64 experts, top-6, 2048 x 1024, 5.6 rows 67 / 81, 8 rows 90 / 82; 8 experts,
-        // 4096 x 2048, 6 rows 43 / 49, 8 rows 59 / 50).
+        // pairs do not take the calls from 7 rows on, where they would be 6 to 21 % sooner (us per layer, segments / pairs: 128 experts, top-8,
+        // 2048 x 768, 6.9 rows 108 / 110, 8 rows 111 / 104; 64 experts, top-6, 2048 x 1024, 5.6 rows 67 / 81, 8 rows 84 / 74; 8 experts, top-2,
+        // 4096 x 2048 in groups of 128, 6 rows 43 / 49, 8 rows 59 / 46).
         // every expert with rows adds at most one partial segment to the ns / 8 full ones: the grid is sized for
         // this bound, and CTAs beyond the actual count leave at once
         const int est_tiles = ns < n_local ? ns : n_local;   // segments expected to be non-empty (split-K sizing)
