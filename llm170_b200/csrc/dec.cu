@@ -136,7 +136,7 @@ int Dec::upload_common(const char* name, const void* q_dev, const void* s_dev, i
     l.glu_f = glu_f;
     const int src_div = group == 64 ? 2 : 1;
     const size_t qb = (size_t)n * (size_t)(k / 2), sb = (size_t)n * (size_t)(k / l.group) * 2;
-    cudaError_t e = cudaMalloc(&l.qt, qb);
+    cudaError_t e = cudaMalloc(&l.qt, qb + TILE_READ_PAD);
     if (e != cudaSuccess) {
         return cuda_fail("alloc weights", e);
     }

@@ -33,7 +33,6 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     __shared__ int s_abort;
     constexpr int RW = RG_WARPS / KW, UR = RW * GM_NR;        // row blocks of a unit
     constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
-    constexpr uint32_t SLOT = rg_slot_bytes(GROUP, GM_NR);
     if (a.tables_fresh) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
@@ -42,7 +41,8 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     const int kw = warp % KW, rw = warp / KW;
     const int nrb = a.seg[0].n / TILE_ROWS, upe = (nrb + UR - 1) / UR;
     const int units = *a.num_tiles * upe;
-    const int u0 = (int)((long long)units * blockIdx.x / gridDim.x), u1 = (int)((long long)units * (blockIdx.x + 1) / gridDim.x);
+    const int per = units / (int)gridDim.x, more = units % (int)gridDim.x;
+    const int u0 = per * (int)blockIdx.x + min(more, (int)blockIdx.x), u1 = u0 + per + ((int)blockIdx.x < more ? 1 : 0);
     if (u0 >= u1) {
         return;
     }
@@ -50,28 +50,18 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks
 
     // ---- weights and scales, in the order of use.  Row blocks past the expert's last one read that one again.
-    const uint32_t ring = smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * SLOT);
-    int fu = u0, fi = 0;
-    int fexp = a.tile_expert[u0 / upe];                       // expert of unit fu
-    uint32_t fdst = 0;
-    RgCursor<GROUP, GM_NR> cur;
+    RgStream<GROUP, GM_NR, D> ring;
+    ring.init(smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * rg_slot_bytes(GROUP, GM_NR)), lane);
+    int fu = u0, fexp = a.tile_expert[u0 / upe];              // expert of unit fu
     auto fetch_unit = [&]() {
-        cur.init(a.seg[0].qt, a.seg[0].st, (fexp - a.expert0) * nrb, fu % upe * UR + rw * GM_NR, nrb, a.nrb_w, ng, kb0, lane);
-        fi = 0;
+        ring.unit(a.seg[0].qt, a.seg[0].st, (fexp - a.expert0) * nrb, fu % upe * UR + rw * GM_NR, nrb, a.nrb_w, ng, kb0, nk, lane);
         if (fu + 1 < u1) {
             fexp = a.tile_expert[(fu + 1) / upe];
         }
     };
-    auto fetch = [&]() {
-        if (fu < u1) {
-            cur.fetch(ring + fdst, lane, (fi & 1) != 0);
-            if (++fi == nk && ++fu < u1) {
-                fetch_unit();
-            }
-        }
-        cp_async_commit();
-        if ((fdst += SLOT) == D * SLOT) {
-            fdst = 0;
+    auto next_unit = [&]() {
+        if (++fu < u1) {
+            fetch_unit();
         }
     };
     if (threadIdx.x == 0) {
@@ -81,9 +71,11 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     }
     if (nk > 0) {
         fetch_unit();
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            fetch();
+        static_assert(D % 2 == 0, "the first and the second k-block of a group in turn");
+#pragma unroll 1
+        for (int d = 0; d < D; d += 2) {
+            ring.template fetch<false>(lane, next_unit);
+            ring.template fetch<true>(lane, next_unit);
         }
     }
     if (!a.tables_fresh) {
@@ -94,7 +86,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
 
     const int xstride = a.k * 2 + RG_XPAD;
     float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][8 tokens]
-    uint32_t rslot = 0, xphase = 0;
+    uint32_t xphase = 0;
     int seg = -1, row0 = 0, m = 0;
     uint32_t xl = 0;
     for (int u = u0; u < u1; ++u) {
@@ -127,7 +119,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
         for (int r = 0; r < GM_NR; ++r) {
             tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
         }
-        rg_multiply<GROUP, GM_NR, D>(tot, xl, nk, ring, rslot, lane, fetch);
+        rg_multiply<GROUP, GM_NR, D>(tot, xl, nk, ring, lane, next_unit);
         // ---- the K warps' sums meet in shared memory
         const int rb0 = u % upe * UR, rows = min(UR, nrb - rb0) * TILE_ROWS;
         if (u > u0) {

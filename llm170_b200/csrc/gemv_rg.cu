@@ -37,7 +37,6 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     __shared__ int s_abort;
     constexpr int RW = RG_WARPS / KW, UR = RW * NR;           // row blocks of a unit
     constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
-    constexpr uint32_t SLOT = rg_slot_bytes(GROUP, NR);
     constexpr int PITCH = rg_red_pitch(UR);
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // optional timeline (diagnostic; a.dbg is null in normal runs): wall-clock stamps of thread 0 in the slots of the other forms
@@ -54,7 +53,7 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     const int kw = warp % KW, rw = warp / KW;
     const int cl = CL ? p.split : 1, rank = CL ? (int)blockIdx.x % cl : 0, cta = (int)blockIdx.x / cl, ctas = (int)gridDim.x / cl;
     // equal contiguous runs of units (row groups over all segments)
-    const int u0 = (int)((long long)p.units * cta / ctas), u1 = (int)((long long)p.units * (cta + 1) / ctas);
+    const int u0 = p.units / ctas * cta + min(p.units % ctas, cta), u1 = u0 + p.units / ctas + (cta < p.units % ctas ? 1 : 0);
     const int ku_all = a.k / (TILE_K * KPU), ng = a.k / GROUP;
     const int ku0 = ku_all * rank / cl, ku = ku_all * (rank + 1) / cl - ku0;   // this CTA's part of K
     const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks, from there
@@ -70,25 +69,16 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     };
 
     // ---- weights and scales, in the order of use
-    const uint32_t ring = smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * SLOT);
-    int fu = u0, fi = 0;
-    uint32_t fdst = 0;
-    RgCursor<GROUP, NR> cur;
+    RgStream<GROUP, NR, D> ring;
+    ring.init(smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * rg_slot_bytes(GROUP, NR)), lane);
+    int fu = u0;
     auto fetch_unit = [&]() {
         const int si = seg_of(fu), nrb = a.seg[si].n / TILE_ROWS;
-        cur.init(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, ku0 * KPU + kb0, lane);
-        fi = 0;
+        ring.unit(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, ku0 * KPU + kb0, nk, lane);
     };
-    auto fetch = [&]() {
-        if (fu < u1) {
-            cur.fetch(ring + fdst, lane, (fi & 1) != 0);
-            if (++fi == nk && ++fu < u1) {
-                fetch_unit();
-            }
-        }
-        cp_async_commit();
-        if ((fdst += SLOT) == D * SLOT) {
-            fdst = 0;
+    auto next_unit = [&]() {
+        if (++fu < u1) {
+            fetch_unit();
         }
     };
     if (threadIdx.x == 0) {
@@ -105,9 +95,10 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     }
     if (nk > 0) {
         fetch_unit();
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-            fetch();
+#pragma unroll 1
+        for (int d = 0; d < D; d += 2) {
+            ring.template fetch<false>(lane, next_unit);
+            ring.template fetch<true>(lane, next_unit);
         }
     }
     stamp_now(8);   // first tiles requested
@@ -136,14 +127,13 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     const uint32_t xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
     const int mp = (m + 1) & ~1;
     float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][mp][PITCH]
-    uint32_t rslot = 0;
     for (int u = u0; u < u1; ++u) {
         float tot[NR][4];
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
             tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
         }
-        rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, rslot, lane, fetch);
+        rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
         stamp_now(4);   // (of the last unit)
         // ---- the K warps' sums meet in shared memory
         const GemvSeg& sg = a.seg[seg_of(u)];

@@ -31,57 +31,63 @@ __device__ __forceinline__ void rg_store_sums(float* d, int pitch, const float (
     }
 }
 
-// Where a warp's next slot comes from: its row blocks (past the matrix: the last one again) and its lane's 16 bytes of scales.
-template <int GROUP, int NR>
-struct RgCursor {
+// A warp's ring and where its next slot comes from.  A slot is refilled as soon as it has been read, so one address serves both sides; a lane
+// copies the weights that it reads itself.  Row blocks past the matrix are whatever lies behind it (the allocation is as much longer,
+// TILE_READ_PAD), their sums are dropped; scales past it are those of the last row block.
+template <int GROUP, int NR, int D>
+struct RgStream {
+    static constexpr uint32_t SLOT = rg_slot_bytes(GROUP, NR), SC = rg_weight_bytes(NR);
     const uint4* q;
     const uint32_t* s;
     size_t pitch;                      // uint4 between k-blocks
-    int step[NR];
+    int left;                          // k-blocks of the unit that are still to be requested
+    uint32_t slot, first;              // this lane's 16 bytes of the slot in turn, of slot 0
 
-    // `rb`: the warp's first row block, `nrb`: row blocks that may be read, both counted from `base` in a matrix of `nrb_all`
-    __device__ __forceinline__ void init(const uint4* qt, const uint32_t* st, int base, int rb, int nrb, int nrb_all, int ng, int kb0, int lane) {
+    __device__ __forceinline__ void init(uint32_t ring, int lane) { slot = first = ring + (uint32_t)lane * 16u; }
+    // `rb`: the warp's first row block, `nrb`: row blocks that it may take, both counted from `base` in a matrix of `nrb_all`; `kbs` k-blocks from kb0
+    __device__ __forceinline__ void unit(const uint4* qt, const uint32_t* st, int base, int rb, int nrb, int nrb_all, int ng, int kb0, int kbs, int lane) {
         constexpr int SP = GROUP == 32 ? 4 : 2;                   // 16-byte pieces of scales per row block and slot
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            step[r] = (base + min(rb + r, nrb - 1)) * 32;
-        }
         pitch = (size_t)nrb_all * 32;
-        q = qt + (size_t)kb0 * pitch + lane;
+        q = qt + (size_t)kb0 * pitch + (size_t)(base + min(rb, nrb - 1)) * 32 + lane;
         s = st + (size_t)(base + min(rb + lane / SP % NR, nrb - 1)) * ng * 8 + (size_t)kb0 * TILE_K / GROUP * 8 + (lane % SP) * 4;
+        left = kbs;
     }
-    // requests the next k-block; `odd`: it is the second one of its group (groups of 128)
-    __device__ __forceinline__ void fetch(uint32_t dst, int lane, bool odd) {
+    // requests the next k-block into the slot in turn; ODD: it is the second one of its group (groups of 128).  `next_unit` is called behind
+    // a unit's last one.
+    template <bool ODD, class Next>
+    __device__ __forceinline__ void fetch(int lane, Next&& next_unit) {
+        if (left > 0) {
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            cp_async_16(dst + (uint32_t)r * 512u + (uint32_t)lane * 16u, q + step[r]);
+            for (int r = 0; r < NR; ++r) {
+                cp_async_16(slot + (uint32_t)r * 512u, q + r * 32);
+            }
+            q += pitch;
+            if (GROUP == 32 || ODD) {
+                if (lane < (GROUP == 32 ? 4 : 2) * NR) {
+                    cp_async_16(slot + SC, s);
+                }
+                s += GROUP == 32 ? 16 : 8;
+            }
+            if (--left == 0) {
+                next_unit();
+            }
         }
-        q += pitch;
-        if (GROUP == 32) {
-            if (lane < 4 * NR) {
-                cp_async_16(dst + rg_weight_bytes(NR) + (uint32_t)lane * 16u, s);
-            }
-            s += 16;
-        } else if (odd) {
-            if (lane < 2 * NR) {
-                cp_async_16(dst + rg_weight_bytes(NR) + (uint32_t)lane * 16u, s);
-            }
-            s += 8;
+        cp_async_commit();
+        if ((slot += SLOT) == first + D * SLOT) {
+            slot = first;
         }
     }
 };
 
 // tot += the warp's NR row blocks times its tokens over nk k-blocks, in nibble units (rows g: 2^-24, rows g + 8: 2^-20).  `xa`: this
-// lane's first activations, `ring`: the warp's ring of D slots, `rslot`: offset of the next slot in it; `fetch()` refills the slot that
-// was just read and commits one group of copies.
+// lane's first activations; `next_unit` as in RgStream::fetch.
 // The zero-point term of a group, -8 * sum(x), is the sum of MMAs whose A operand is the constant -8 in the nibbles' own two scalings: no
 // pass over x, no table.  In groups of 32 it opens the chains of the row blocks as their C operand; in groups of 128, where it is complete
 // only after the group's second k-block, it is added to their sums.
-template <int GROUP, int NR, int D, class Fetch>
-__device__ __forceinline__ void rg_multiply(float (&tot)[NR][4], uint32_t xa, int nk, uint32_t ring, uint32_t& rslot, int lane, Fetch&& fetch) {
-    constexpr uint32_t SLOT = rg_slot_bytes(GROUP, NR), SC = rg_weight_bytes(NR);
+template <int GROUP, int NR, int D, class Next>
+__device__ __forceinline__ void rg_multiply(float (&tot)[NR][4], uint32_t xa, int nk, RgStream<GROUP, NR, D>& ring, int lane, Next&& next_unit) {
     const uint32_t zA[4] = {0x80088008u, 0x80808080u, 0x80088008u, 0x80808080u};
-    const uint32_t wl = ring + (uint32_t)lane * 16u, sl = ring + SC + (uint32_t)(lane >> 2) * 4u;
+    const uint32_t sl = rg_weight_bytes(NR) + (uint32_t)(lane >> 2) * 4u - (uint32_t)lane * 16u;   // from a lane's weights to its scales
     float acc[NR][4] = {};
     auto fold = [&](int r, uint32_t s2) {
         const float2 sf = __half22float2(*reinterpret_cast<const __half2*>(&s2));
@@ -89,13 +95,6 @@ __device__ __forceinline__ void rg_multiply(float (&tot)[NR][4], uint32_t xa, in
         tot[r][1] = fmaf(acc[r][1], sf.x, tot[r][1]);
         tot[r][2] = fmaf(acc[r][2], sf.y, tot[r][2]);
         tot[r][3] = fmaf(acc[r][3], sf.y, tot[r][3]);
-    };
-    auto next_slot = [&]() {
-        __syncwarp();
-        fetch();
-        if ((rslot += SLOT) == D * SLOT) {
-            rslot = 0;
-        }
     };
     if (GROUP == 32) {
         for (int i = 0; i < nk; ++i) {
@@ -111,11 +110,12 @@ __device__ __forceinline__ void rg_multiply(float (&tot)[NR][4], uint32_t xa, in
             uint32_t sc[NR][2];
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
-                wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
-                sc[r][0] = lds32(sl + rslot + (uint32_t)r * 64u);
-                sc[r][1] = lds32(sl + rslot + (uint32_t)r * 64u + 32u);
+                wv[r] = lds128(ring.slot + (uint32_t)r * 512u);
+                sc[r][0] = lds32(ring.slot + sl + (uint32_t)r * 64u);
+                sc[r][1] = lds32(ring.slot + sl + (uint32_t)r * 64u + 32u);
             }
-            next_slot();
+            __syncwarp();
+            ring.template fetch<true>(lane, next_unit);
             float z0[4], z1[4];
             mma16816_z(z0, zA, x[0].x, x[0].y);
             mma16816_z(z1, zA, x[2].x, x[2].y);
@@ -162,16 +162,23 @@ __device__ __forceinline__ void rg_multiply(float (&tot)[NR][4], uint32_t xa, in
                 }
                 xa += TILE_K * 2;
                 cp_async_wait_group<D - 1>();
-                __syncwarp();
+                if (h == 1) {
+                    __syncwarp();                         // the scale words are other lanes' copies
+                }
                 uint4 wv[NR];
 #pragma unroll
                 for (int r = 0; r < NR; ++r) {
-                    wv[r] = lds128(wl + rslot + (uint32_t)r * 512u);
+                    wv[r] = lds128(ring.slot + (uint32_t)r * 512u);
                     if (h == 1) {
-                        sc[r] = lds32(sl + rslot + (uint32_t)r * 32u);
+                        sc[r] = lds32(ring.slot + sl + (uint32_t)r * 32u);
                     }
                 }
-                next_slot();
+                __syncwarp();
+                if (h == 0) {
+                    ring.template fetch<false>(lane, next_unit);
+                } else {
+                    ring.template fetch<true>(lane, next_unit);
+                }
                 uint32_t af[4];
 #pragma unroll
                 for (int w = 0; w < 4; ++w) {

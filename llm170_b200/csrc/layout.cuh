@@ -34,6 +34,9 @@ namespace w4 {
 constexpr int TILE_ROWS = 16;
 constexpr int TILE_K = 64;
 constexpr int TILE_WORDS = 128;  // u32 per tile
+// Allocated behind a matrix's tiles: a warp of the decode GEMVs reads up to four neighbouring tiles of a k-block from one address, also where
+// the matrix ends behind the first of them.
+constexpr int TILE_READ_PAD = 3 * TILE_WORDS * 4;
 
 // Shape contract of the tiled layout (the reference's Marlin path requires k%128==0 && n%64==0,
 // crates/backend-gpu/src/rawcuda/w4a16_dec/kernels/marlin.rs:110; this layout is less strict).

@@ -477,7 +477,7 @@ int Dec::upload_stream(const char* name, int n, int k, int group, int scale_bf16
         }
         pin_cap = 2 * slot;
     }
-    cudaError_t e = cudaMalloc(&l.qt, qb);
+    cudaError_t e = cudaMalloc(&l.qt, qb + w4::TILE_READ_PAD);
     if (e != cudaSuccess) {
         return cuda_fail("alloc weights", e);
     }
@@ -792,7 +792,7 @@ int w4a16_load_lin_cache(w4a16_dec* dec, const char* name, const char* path, uin
     l.group = (int)h.group;
     l.group_src = (int)h.group_src;
     l.out_mul = h.out_mul;
-    cudaError_t e = cudaMalloc(&l.qt, qb);
+    cudaError_t e = cudaMalloc(&l.qt, qb + w4::TILE_READ_PAD);
     if (e == cudaSuccess) {
         e = cudaMalloc(&l.st, sb);
     }
