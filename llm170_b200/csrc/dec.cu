@@ -237,7 +237,7 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
     const bool rowgroup = tune_gemv_rowgroup > 0 && stock && !allreduce;
     auto choose_rowgroup = [&]() {
         const int forced = tune_gemv_rowgroup - 1;
-        const bool fits = rg_make_plan(a, sm_count, forced & 15, forced >> 4, c.rg);
+        const bool fits = rg_make_plan(a, sm_count, forced & 15, forced >> 4, /*digits=*/false, c.rg);
         long long rows = 0;
         for (int i = 0; i < a.nseg; ++i) {
             rows += a.seg[i].n;
@@ -255,6 +255,11 @@ int Dec::gemv_select(GemvArgs& a, bool allreduce, bool own_scratch, bool single,
         if (!clusters && (!fits || leaves)) {
             c.grid_x = gemv_plan_ctas(a);       // the segments' first blocks, which the plan counted in its own units
             return false;
+        }
+        RgPlan dg{};
+        if (!clusters && t <= RG_MAX_DIGIT_TOKENS && (tune_gemv_digits == 2 || (tune_gemv_digits == 1 && rg_digits_pay(a, c.rg))) &&
+            rg_make_plan(a, sm_count, forced & 15, forced >> 4, /*digits=*/true, dg)) {
+            c.rg = dg;
         }
         c.form = GemvChoice::ROWGROUP;
         a.ksplit = 1;
@@ -747,6 +752,13 @@ int w4a16_set_tuning(w4a16_dec* dec, const char* key, int value) {
             return d.fail("w4a16 set_tuning: gemv_rowgroup=%d (0, 1, or 1 + row blocks per warp (2..4) + 16 * warps along K (4, 8))", value);
         }
         d.tune_gemv_rowgroup = value;
+        return 0;
+    }
+    if (!strcmp(key, "gemv_digits")) {
+        if (value < 0 || value > 2) {
+            return d.fail("w4a16 set_tuning: gemv_digits=%d (0..2)", value);
+        }
+        d.tune_gemv_digits = value;
         return 0;
     }
     if (!strcmp(key, "gemv_stages")) {

@@ -13,10 +13,13 @@
 //   * every warp streams its own tiles and scales into its own ring with asynchronous copies, requested before the dependency wait and
 //     refilled across units: no producer, no barrier in the loop, nothing of the copy engine, which takes 60 ns for each copy;
 //   * the warps' sums meet in shared memory once per unit; nothing is shared between CTAs, but where x does not fit beside the rings (five to
-//     eight tokens of long K): there the CTAs of a cluster share K and add up in each other's shared memory (rg_cluster_plan).
-// One token, us per launch, this form against the best of the others: 7168 x 5120 6.6 / 7.2, 5120 x 6144 6.2 / 7.5, 34816 x 5120
-// 17.3 / 21.6 (5.3 TB/s), 5120 x 17408 13.0 / 13.8, 24576 x 4096 12.0 / 15.9; eight tokens: 7.1 / 10.3, 6.6 / 10.2, 20.5 / 26.2;
-// 34816 x 5120 in groups of 32, eight tokens: 21.7 / 48.9.
+//     eight tokens of long K): there the CTAs of a cluster share K and add up in each other's shared memory (rg_cluster_plan);
+//   * one token, and some calls of two, are multiplied as signed digits by integer MMAs (gemv_rg.cuh): with the weights in L2 a launch took as long as
+//     from memory, because a tile cost an SM's scheduler 84 cycles, 40 of MMAs and 48 of masks and shifts among them; as digits it is 53, and
+//     5120 x 17408 streams 7 TB/s once its activations are staged.  Sixteen warps in a CTA were not faster (5120 x 17408 10.8 us, 896 x 5120 4.0).
+// One token, us per launch, this form against the best of the others: 7168 x 5120 5.3 / 7.2, 5120 x 6144 5.0 / 7.5, 34816 x 5120
+// 17.0 / 21.6 (5.4 TB/s), 5120 x 17408 10.2 / 13.8, 24576 x 4096 11.2 / 15.9; eight tokens: 6.8 / 10.3, 6.2 / 10.2, 20.0 / 26.2;
+// 34816 x 5120 in groups of 32, eight tokens: 21.4 / 48.9.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -30,7 +33,7 @@ namespace {
 // KW = warps along K; the other warps of a CTA take further row blocks.  NR = row blocks per warp, D = ring slots per warp.
 // CL: the CTAs of a cluster share K as well, so that a unit's rows are spread over several SMs and each stages its part of x only; their sums
 // meet in distributed shared memory, in the order of their ranks.
-template <int GROUP, int KW, int NR, int D, bool CL>
+template <int GROUP, int KW, int NR, int D, bool CL, bool DIG>
 __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a, const RgPlan p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) unsigned long long s_xbar;
@@ -106,25 +109,37 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
     asm volatile("griddepcontrol.wait;" ::: "memory");        // x and the outputs may be the previous kernel's
     stamp_now(1);
 
-    // ---- activations: one bulk copy per token
-    const int m = a.m, xbytes = ku * (KPU * TILE_K * 2), xstride = CL ? (ku_all + cl - 1) / cl * (KPU * TILE_K * 2) + RG_XPAD : a.k * 2 + RG_XPAD;
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * xbytes));
+    // ---- activations: one bulk copy per token, or digits, every warp its part of K
+    const int m = a.m, xbytes = ku * (KPU * TILE_K * 2);
+    const int xstride = DIG ? rg_digit_stride(a.k) : CL ? (ku_all + cl - 1) / cl * (KPU * TILE_K * 2) + RG_XPAD : a.k * 2 + RG_XPAD;
+    float mul[RG_MAX_DIGIT_TOKENS] = {};
+    if (DIG) {
+        rg_stage_digits(smem_u32(smem), (uint32_t)xstride, smem_u32(smem) + (uint32_t)(p.off_raw + m * (kb0 * RW + rw * nk) * (TILE_K * 2)), a.x, a.k, m, kb0, nk, rw, RW, lane, mul);
+        if (RW > 1) {
+            __syncthreads();
+        } else {
+            __syncwarp();
+        }
+    } else {
+        if (warp == 0) {
+            if (lane == 0) {
+                mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * xbytes));
+            }
+            __syncwarp();
+            if (lane < m) {
+                bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k + ku0 * (KPU * TILE_K), (uint32_t)xbytes, smem_u32(&s_xbar));
+            }
+        }
+        if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
+            mbar_drain(smem_u32(&s_xbar), 0);
         }
         __syncwarp();
-        if (lane < m) {
-            bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k + ku0 * (KPU * TILE_K), (uint32_t)xbytes, smem_u32(&s_xbar));
-        }
     }
-    if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
-        mbar_drain(smem_u32(&s_xbar), 0);
-    }
-    __syncwarp();
     stamp_now(2);   // x staged
     stamp_now(3);
-    // lanes without a token read token 0: their columns are never stored
-    const uint32_t xl = smem_u32(smem) + (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8);
+    // lanes without a token read token 0, those without a digit digit 2: their columns are never stored
+    const uint32_t xl = smem_u32(smem) + (DIG ? (uint32_t)(((g >> 2 < m ? g >> 2 : 0) * 3 + min(g & 3, 2)) * xstride + kb0 * TILE_K + t * 16)
+                                              : (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8));
     const int mp = (m + 1) & ~1;
     float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][mp][PITCH]
     for (int u = u0; u < u1; ++u) {
@@ -133,7 +148,11 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
         for (int r = 0; r < NR; ++r) {
             tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
         }
-        rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
+        if (DIG) {
+            rg_multiply_digits<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
+        } else {
+            rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
+        }
         stamp_now(4);   // (of the last unit)
         // ---- the K warps' sums meet in shared memory
         const GemvSeg& sg = a.seg[seg_of(u)];
@@ -141,7 +160,20 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
         if (u > u0) {
             __syncthreads();
         }
-        if (2 * t < mp) {
+        if (DIG) {
+            // lanes t = 0, 2 have digits 0 and 1 of a token, 1 and 3 digit 2: they put them together, and the first stores row g, the second row g + 8
+            const int tok = t >> 1, odd = t & 1;
+            const float mt = (tok ? mul[1] : mul[0]) * sg.out_mul, w0 = odd ? 65536.f * mt : mt, w1 = odd ? 0.f : 256.f * mt;
+            float* d = red + (kw * mp + tok) * PITCH + rw * NR * TILE_ROWS + g + odd * 8;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const float lo = fmaf(tot[r][1], w1, tot[r][0] * w0), hi = fmaf(tot[r][3], w1, tot[r][2] * w0);
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+                if (tok < m) {
+                    d[r * TILE_ROWS] = (odd ? hi : lo) + other;
+                }
+            }
+        } else if (2 * t < mp) {
             const float m0 = 16777216.f * sg.out_mul, m1 = 1048576.f * sg.out_mul;
             rg_store_sums(red + (kw * mp + 2 * t) * PITCH + rw * NR * TILE_ROWS + g, PITCH, tot, m0, m1);
         }
@@ -193,20 +225,21 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a
 }
 
 struct RgKernel {
-    int group, kw, nr, depth;
-    bool cluster;
     const void* f;
     const char* name;
 };
-#define W4_RG(G, K, N, D, C) {G, K, N, D, C, (const void*)gemv_rg_kernel<G, K, N, D, C>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
-#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2, false), W4_RG(G, K, N, 4, false), W4_RG(G, K, N, 6, false), W4_RG(G, K, N, 2, true)
+#define W4_RG(G, K, N, D, C) {(const void*)gemv_rg_kernel<G, K, N, D, C, false>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
+#define W4_RGD(G, K, N, D) {(const void*)gemv_rg_kernel<G, K, N, D, false, true>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ",digits>"}
+#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2, false), W4_RG(G, K, N, 4, false), W4_RG(G, K, N, 6, false), W4_RG(G, K, N, 2, true), \
+                         W4_RGD(G, K, N, 2), W4_RGD(G, K, N, 4), W4_RGD(G, K, N, 6)
 #define W4_RG_N(G, K) W4_RG_D(G, K, 2), W4_RG_D(G, K, 3), W4_RG_D(G, K, 4)
 const RgKernel rg_kernels[] = {W4_RG_N(128, 4), W4_RG_N(128, 8), W4_RG_N(32, 4), W4_RG_N(32, 8)};
 #undef W4_RG_N
 #undef W4_RG_D
+#undef W4_RGD
 #undef W4_RG
 const RgKernel& rg_kernel(int group, const RgPlan& p) {
-    return rg_kernels[(group == 128 ? 0 : 24) + (p.kw == 4 ? 0 : 12) + (p.nr - 2) * 4 + (p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
+    return rg_kernels[(group == 128 ? 0 : 42) + (p.kw == 4 ? 0 : 21) + (p.nr - 2) * 7 + (p.digits ? 4 : p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
 }
 
 // What a plan may take, the padding of the sums aside: it comes from what is left above, so that it costs no ring slot, no warp along K and no second CTA
@@ -229,10 +262,9 @@ constexpr double RG_STEP_US[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.4
 // share less (two: 1.3, three: 1.05 per tile).  A unit costs about twenty tiles beside its own for its sums.  Best of the twelve ways
 // measured, and the choice: 7168 x 5120 (448 row blocks) 6.6: 4 row blocks, 8 warps, alone; 5120 x 6144 6.2: 3, 8, alone; 12544 x 4224
 // 7.6: 3, 8, two (alone 8.5); 24576 x 4096 12.0: 3, 4, two (4, 8, alone 12.9); 34816 x 5120 17.3: 4, 4, two (4, 8, two 17.7).
-// false: x does not fit in shared memory beside two slots per warp.
-bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& best) {
+// `digits`: one or two tokens as digits, which take more room.  false: x does not fit in shared memory beside two slots per warp.
+bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, bool digits, RgPlan& best) {
     const int unit_k = a.group > TILE_K ? a.group : TILE_K, ku = a.k / unit_k, mp = (a.m + 1) & ~1;
-    const int x_bytes = (a.m * (a.k * 2 + RG_XPAD) + 127) & ~127;
     double cost = -1.0;
     for (int kw : {4, 8}) {
         for (int nr : {4, 3, 2}) {
@@ -244,9 +276,12 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
             p.nr = nr;
             p.kw = kw;
             p.split = 1;
+            p.digits = digits;
             for (int i = 0; i < a.nseg; ++i) {
                 p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
             }
+            p.off_raw = 3 * a.m * rg_digit_stride(a.k);
+            const int x_bytes = ((digits ? p.off_raw + a.m * a.k * 2 * (RG_WARPS / kw) : a.m * (a.k * 2 + RG_XPAD)) + 127) & ~127;
             p.off_red = x_bytes;
             const int padding = kw * mp * RG_RED_PAD * 4;
             p.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) - padding + 127) & ~127;
@@ -283,6 +318,20 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan&
         units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
     }
     return true;
+}
+
+// Whether activations as digits (gemv_rg.cuh) are sooner than as f16, whose plan is `p`: their making takes 0.3 us at 5120 channels of a token and 1.2 at
+// 17408, and every CTA makes its own.  us per launch, f16 / digits: one token 7168 x 5120 6.30 / 5.33, 5120 x 6144 5.68 / 4.98, 5120 x 17408 11.9 / 10.2,
+// 34816 x 5120 17.2 / 17.0, 896 x 5120 3.83 / 3.35, 24576 x 4096 in groups of 32 12.7 / 11.7; two tokens 7168 x 5120 6.34 / 5.85.  Over 430 shapes of
+// 256 to 34816 rows and 512 to 22528 channels digits take 0.92 (groups of 128) and 0.94 of the time of one token where this says so, at most 1.02;
+// shorter K has nothing to win (2048 x 512 2.01 / 2.11), nor have two CTAs on an SM that both stage a long one (34816 x 17408 50.2 / 52.2, 9472 x 14336
+// 14.9 / 15.6).  Two tokens: 0.93 where it says so; 12544 x 5120, two CTAs, 1.08, 1792 x 5120, two row blocks a warp, 1.02.
+bool rg_digits_pay(const GemvArgs& a, const RgPlan& p) {
+    const bool two = p.smem <= RG_SMEM_TWO_HW;
+    if (a.m == 1) {
+        return a.k >= (a.group == 128 ? 2048 : 4096) && !(two && a.k > 8192);
+    }
+    return a.m == 2 && a.group == 128 && !two && p.nr >= 3 && a.k >= 4096 && a.k <= 8192;
 }
 
 // Estimated time of a plan, K from 8192 on.

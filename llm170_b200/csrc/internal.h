@@ -146,16 +146,21 @@ cudaError_t launch_gemv_sk(const GemvArgs& a, const SkPlan& p, cudaStream_t st);
 cudaError_t gemv_sk_init_device();
 cudaError_t gemv_rb_init_device();
 // ---- gemv_rg.cu: the row-group form of the decode GEMV ----
+constexpr int RG_MAX_DIGIT_TOKENS = 2;
 struct RgPlan {
     int nr, kw;              // row blocks per warp, warps along K
     int units;               // row groups over all segments (seg[].cta0 = first of the segment)
     int ctas;                // CTA c takes units [units c / ctas, units (c + 1) / ctas)
     int depth;               // ring slots per warp
     int split;               // CTAs of a cluster that share K (1: none)
+    bool digits;             // activations as digits (gemv_rg.cuh)
+    int off_raw;             // digits: scratch of their making
     int off_red, off_part, off_ring;   // byte offsets in dynamic shared memory: activations first
     int smem;
 };
-bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, RgPlan& p);
+bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, bool digits, RgPlan& p);
+// Whether a call with this plan is sooner with its activations as digits.
+bool rg_digits_pay(const GemvArgs& a, const RgPlan& p);
 // A plan over clusters that is estimated to take less than `us` (false: none); fills seg[].cta0.
 bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& p, double us);
 // Whether another form is estimated to finish the call sooner than this plan; `sk`: the persistent form's plan.

@@ -589,6 +589,69 @@ def test_row_group_form(dec, orc, n, k, group, t, bf16, way):
     dec.drop_lin("rg")
 
 
+# Activations as digits (one and two tokens): fewer k-blocks than warps, odd numbers of k-blocks, units that the last rows do not fill, more units than CTAs,
+# 129 and more pieces of activations (ten loads under way instead of four); inputs of one size, of all sizes that f16 has, zeros, its largest and smallest
+@pytest.mark.parametrize("way", [0, (2, 8), (3, 8), (4, 8), (2, 4), (3, 4), (4, 4)])
+@pytest.mark.parametrize("n,k,group,t,bf16", [(16, 128, 128, 1, False), (48, 192, 32, 2, False), (272, 576, 64, 1, True), (1040, 1152, 128, 2, False),
+                                             (20000, 256, 128, 2, True), (38000, 128, 64, 1, False), (512, 4096, 128, 2, False), (320, 9216, 32, 1, False)])
+def test_row_group_form_with_digits(dec, n, k, group, t, bf16, way):
+    q, s = synth.make_linear_cuda(n, k, group, 920 + n % 97, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("rgd", q, s.to(torch.bfloat16) if bf16 else s, n, k, group, bf16)
+    w = dec.dequant_lin("rgd").double()
+    gen = torch.Generator("cuda").manual_seed(930 + k)
+    x = torch.randn((t, k), device="cuda", generator=gen)
+    wide = x * torch.exp2(torch.randint(-24, 14, (t, k), device="cuda", generator=gen).float())
+    edge = torch.zeros((t, k), device="cuda")
+    edge[0, ::3], edge[0, 1::5], edge[0, k // 2:] = 65504.0, -65504.0, 2.0 ** -24
+    guard = torch.full((t + 1, n), 7.0, device="cuda", dtype=torch.float32)
+    dec.set_tuning("gemv_rowgroup", 1 if way == 0 else 1 + way[0] + 16 * way[1])
+    dec.set_tuning("gemv_digits", 2)
+    try:
+        for xs in (x, wide.clamp(-65504, 65504), edge, torch.zeros_like(x)):
+            xh = xs.half()
+            y = dec.lin_forward("rgd", xh, t, dst=guard[:t]).clone()
+            name = dec.last_kernel()
+            assert name.startswith("gemv_rg_kernel") and name.endswith(",digits>") and (way == 0 or f",{way[1]},{way[0]}," in name), name
+            assert torch.equal(dec.lin_forward("rgd", xh, t, out_f16=True), y.half())
+            outs = dec.sk_multi_dev(["rgd", "rgd"], xh, t=t)
+            assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], y)      # a row's sum does not depend on what is beside it
+            # an activation is rounded by half a unit, at most 2^-21 of the largest; sums and scales in f32, 2^-24 for each of at most 2^6 additions
+            bound = 2.0 ** -21 * xh.double().abs().amax(1, keepdim=True) * w.abs().sum(1) + 2.0 ** -18 * (xh.double().abs() @ w.abs().T)
+            assert bool(((y.double() - xh.double() @ w.T).abs() <= bound).all())
+            assert bool((guard[t:] == 7.0).all())
+        for bad in (float("inf"), float("nan")):
+            xh = x.half()
+            xh[0, k - 1] = bad
+            y = dec.lin_forward("rgd", xh, t)
+            assert bool(y[0].isnan().all()) and (t == 1 or bool(y[1].isfinite().all()))
+    finally:
+        dec.set_tuning("gemv_digits", 1)
+        dec.set_tuning("gemv_rowgroup", 1)
+    dec.drop_lin("rgd")
+
+
+# which calls are multiplied as digits by themselves: both sides of each line (rg_digits_pay)
+@pytest.mark.parametrize("n,k,group,t,digits", [(512, 2048, 128, 1, True), (512, 1920, 128, 1, False), (512, 4096, 32, 1, True), (512, 4032, 64, 1, False),
+                                               (34816, 8192, 128, 1, True), (34816, 8320, 128, 1, False), (7168, 4096, 128, 2, True), (7168, 3968, 128, 2, False),
+                                               (7168, 4096, 32, 2, False), (4096, 4096, 128, 2, False), (512, 4096, 128, 3, False)])
+def test_calls_with_digits(dec, n, k, group, t, digits):
+    q, s = synth.make_linear_cuda(n, k, group, 940, torch.device("cuda", 0))
+    dec.upload_lin_g_dev("rgd", q, s, n, k, group)
+    x = x_dev(synth.make_acts(t, k, seed=941))
+    y = dec.lin_forward("rgd", x, t)
+    name = dec.last_kernel()
+    assert name.startswith("gemv_rg_kernel") and name.endswith(",digits>") == digits, name
+    dec.set_tuning("gemv_digits", 0)
+    try:
+        other = dec.lin_forward("rgd", x, t)
+        assert not dec.last_kernel().endswith(",digits>")
+    finally:
+        dec.set_tuning("gemv_digits", 1)
+    size = (x.float().abs() @ dec.dequant_lin("rgd").abs().T).max().item()
+    assert (y - other).abs().max().item() <= 2.0 ** -18 * size                # f32 sums in another order, as in the tests of the corners
+    dec.drop_lin("rgd")
+
+
 def test_row_group_form_leaves_what_does_not_fit(dec, orc):
     # eight tokens of 17408 channels are 278 KB: the call keeps the form that stages a part of K at a time
     n, k, t = 256, 17408, 8
