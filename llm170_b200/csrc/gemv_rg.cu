@@ -26,220 +26,15 @@
 
 #include "gemv_rg.cuh"
 
+#define RG_TIMELINE false
+#include "gemv_rg_kernel.cuh"
+
 namespace w4 {
 
 namespace {
 
-// KW = warps along K; the other warps of a CTA take further row blocks.  NR = row blocks per warp, D = ring slots per warp.
-// CL: the CTAs of a cluster share K as well, so that a unit's rows are spread over several SMs and each stages its part of x only; their sums
-// meet in distributed shared memory, in the order of their ranks.
-template <int GROUP, int KW, int NR, int D, bool CL, bool DIG>
-__global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a, const RgPlan p) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) unsigned long long s_xbar;
-    __shared__ int s_abort;
-    constexpr int RW = RG_WARPS / KW, UR = RW * NR;           // row blocks of a unit
-    constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
-    constexpr int PITCH = rg_red_pitch(UR);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // optional timeline (diagnostic; a.dbg is null in normal runs): wall-clock stamps of thread 0 in the slots of the other forms
-    auto stamp_now = [&](int j) {
-        if (a.dbg != nullptr && threadIdx.x == 0 && (int)blockIdx.x < DBG_CTAS) {
-            unsigned long long ns;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(ns));
-            a.dbg[((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS + j] = (long long)ns;
-        }
-    };
-    stamp_now(0);
-    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int g = lane >> 2, t = lane & 3;
-    const int kw = warp % KW, rw = warp / KW;
-    const int cl = CL ? p.split : 1, rank = CL ? (int)blockIdx.x % cl : 0, cta = (int)blockIdx.x / cl, ctas = (int)gridDim.x / cl;
-    // equal contiguous runs of units (row groups over all segments)
-    const int u0 = p.units / ctas * cta + min(p.units % ctas, cta), u1 = u0 + p.units / ctas + (cta < p.units % ctas ? 1 : 0);
-    const int ku_all = a.k / (TILE_K * KPU), ng = a.k / GROUP;
-    const int ku0 = ku_all * rank / cl, ku = ku_all * (rank + 1) / cl - ku0;   // this CTA's part of K
-    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks, from there
-    auto seg_of = [&](int u) {
-        int si = 0;
-#pragma unroll
-        for (int i = 1; i < GEMV_MAX_SEG; ++i) {
-            if (i < a.nseg && u >= a.seg[i].cta0) {
-                si = i;
-            }
-        }
-        return si;
-    };
-
-    // ---- weights and scales, in the order of use
-    RgStream<GROUP, NR, D> ring;
-    ring.init(smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * rg_slot_bytes(GROUP, NR)), lane);
-    int fu = u0;
-    auto fetch_unit = [&]() {
-        const int si = seg_of(fu), nrb = a.seg[si].n / TILE_ROWS;
-        ring.unit(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, ku0 * KPU + kb0, nk, lane);
-    };
-    auto next_unit = [&]() {
-        if (++fu < u1) {
-            fetch_unit();
-        }
-    };
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        mbar_init(smem_u32(&s_xbar), 1);
-        mbar_init_fence();
-        if (a.dbg != nullptr && (int)blockIdx.x < DBG_CTAS) {
-            unsigned smid;
-            asm volatile("mov.u32 %0, %smid;" : "=r"(smid));
-            long long* d = a.dbg + ((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS;
-            d[6] = smid;
-            d[7] = u1 - u0;
-        }
-    }
-    if (nk > 0) {
-        fetch_unit();
-#pragma unroll 1
-        for (int d = 0; d < D; d += 2) {
-            ring.template fetch<false>(lane, next_unit);
-            ring.template fetch<true>(lane, next_unit);
-        }
-    }
-    stamp_now(8);   // first tiles requested
-    __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");        // x and the outputs may be the previous kernel's
-    stamp_now(1);
-
-    // ---- activations: one bulk copy per token, or digits, every warp its part of K
-    const int m = a.m, xbytes = ku * (KPU * TILE_K * 2);
-    const int xstride = DIG ? rg_digit_stride(a.k) : CL ? (ku_all + cl - 1) / cl * (KPU * TILE_K * 2) + RG_XPAD : a.k * 2 + RG_XPAD;
-    float mul[RG_MAX_DIGIT_TOKENS] = {};
-    if (DIG) {
-        rg_stage_digits(smem_u32(smem), (uint32_t)xstride, smem_u32(smem) + (uint32_t)(p.off_raw + m * (kb0 * RW + rw * nk) * (TILE_K * 2)), a.x, a.k, m, kb0, nk, rw, RW, lane, mul);
-        if (RW > 1) {
-            __syncthreads();
-        } else {
-            __syncwarp();
-        }
-    } else {
-        if (warp == 0) {
-            if (lane == 0) {
-                mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * xbytes));
-            }
-            __syncwarp();
-            if (lane < m) {
-                bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k + ku0 * (KPU * TILE_K), (uint32_t)xbytes, smem_u32(&s_xbar));
-            }
-        }
-        if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
-            mbar_drain(smem_u32(&s_xbar), 0);
-        }
-        __syncwarp();
-    }
-    stamp_now(2);   // x staged
-    stamp_now(3);
-    // lanes without a token read token 0, those without a digit digit 2: their columns are never stored
-    const uint32_t xl = smem_u32(smem) + (DIG ? (uint32_t)(((g >> 2 < m ? g >> 2 : 0) * 3 + min(g & 3, 2)) * xstride + kb0 * TILE_K + t * 16)
-                                              : (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8));
-    const int mp = (m + 1) & ~1;
-    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][mp][PITCH]
-    for (int u = u0; u < u1; ++u) {
-        float tot[NR][4];
-#pragma unroll
-        for (int r = 0; r < NR; ++r) {
-            tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
-        }
-        if (DIG) {
-            rg_multiply_digits<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
-        } else {
-            rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
-        }
-        stamp_now(4);   // (of the last unit)
-        // ---- the K warps' sums meet in shared memory
-        const GemvSeg& sg = a.seg[seg_of(u)];
-        const int rb0 = (u - sg.cta0) * UR, rows = min(UR, sg.n / TILE_ROWS - rb0) * TILE_ROWS;
-        if (u > u0) {
-            __syncthreads();
-        }
-        if (DIG) {
-            // lanes t = 0, 2 have digits 0 and 1 of a token, 1 and 3 digit 2: they put them together, and the first stores row g, the second row g + 8
-            const int tok = t >> 1, odd = t & 1;
-            const float mt = (tok ? mul[1] : mul[0]) * sg.out_mul, w0 = odd ? 65536.f * mt : mt, w1 = odd ? 0.f : 256.f * mt;
-            float* d = red + (kw * mp + tok) * PITCH + rw * NR * TILE_ROWS + g + odd * 8;
-#pragma unroll
-            for (int r = 0; r < NR; ++r) {
-                const float lo = fmaf(tot[r][1], w1, tot[r][0] * w0), hi = fmaf(tot[r][3], w1, tot[r][2] * w0);
-                const float other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
-                if (tok < m) {
-                    d[r * TILE_ROWS] = (odd ? hi : lo) + other;
-                }
-            }
-        } else if (2 * t < mp) {
-            const float m0 = 16777216.f * sg.out_mul, m1 = 1048576.f * sg.out_mul;
-            rg_store_sums(red + (kw * mp + 2 * t) * PITCH + rw * NR * TILE_ROWS + g, PITCH, tot, m0, m1);
-        }
-        __syncthreads();
-        auto local_sum = [&](int tok, int row) {
-            const float* d = red + tok * PITCH + row;
-            float v = d[0];
-#pragma unroll
-            for (int w = 1; w < KW; ++w) {
-                v += d[w * mp * PITCH];                                  // fixed order: the same bits every run
-            }
-            return v;
-        };
-        int e0 = 0, e1 = rows * m;
-        // a CTA's sums for the others of its cluster, two units in turn: those of the unit before may still be read
-        const uint32_t part = smem_u32(smem) + (uint32_t)p.off_part + (uint32_t)((u - u0) & 1) * (UR * TILE_ROWS * GEMV_MAX_M * 4);
-        if (CL) {
-            for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
-                const int tok = e / rows;
-                asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (uint32_t)e * 4u), "f"(local_sum(tok, e - tok * rows)) : "memory");
-            }
-            cluster_sync_all();
-            e0 = rows * m * rank / cl;
-            e1 = rows * m * (rank + 1) / cl;
-        }
-        for (int e = e0 + (int)threadIdx.x; e < e1; e += RG_THREADS) {
-            const int tok = e / rows, row = e - tok * rows;
-            float v;
-            if (CL) {
-                v = ld_dsmem_f32(part + (uint32_t)e * 4u, 0);
-                for (int c = 1; c < cl; ++c) {
-                    v += ld_dsmem_f32(part + (uint32_t)e * 4u, (unsigned)c);
-                }
-            } else {
-                v = local_sum(tok, row);
-            }
-            const size_t o = (size_t)tok * sg.n + (size_t)rb0 * TILE_ROWS + row;
-            if (a.out_f16) {
-                reinterpret_cast<__half*>(sg.out)[o] = __float2half_rn(v);
-            } else {
-                reinterpret_cast<float*>(sg.out)[o] = v;
-            }
-        }
-    }
-    if (CL) {
-        cluster_sync_all();                                   // nothing of this CTA's shared memory is still read
-    }
-    stamp_now(5);   // sums stored
-}
-
-struct RgKernel {
-    const void* f;
-    const char* name;
-};
-#define W4_RG(G, K, N, D, C) {(const void*)gemv_rg_kernel<G, K, N, D, C, false>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
-#define W4_RGD(G, K, N, D) {(const void*)gemv_rg_kernel<G, K, N, D, false, true>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ",digits>"}
-#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2, false), W4_RG(G, K, N, 4, false), W4_RG(G, K, N, 6, false), W4_RG(G, K, N, 2, true), \
-                         W4_RGD(G, K, N, 2), W4_RGD(G, K, N, 4), W4_RGD(G, K, N, 6)
-#define W4_RG_N(G, K) W4_RG_D(G, K, 2), W4_RG_D(G, K, 3), W4_RG_D(G, K, 4)
-const RgKernel rg_kernels[] = {W4_RG_N(128, 4), W4_RG_N(128, 8), W4_RG_N(32, 4), W4_RG_N(32, 8)};
-#undef W4_RG_N
-#undef W4_RG_D
-#undef W4_RGD
-#undef W4_RG
-const RgKernel& rg_kernel(int group, const RgPlan& p) {
-    return rg_kernels[(group == 128 ? 0 : 42) + (p.kw == 4 ? 0 : 21) + (p.nr - 2) * 7 + (p.digits ? 4 : p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
+const RgKernel& rg_kernel(const RgKernel* kernels, int group, const RgPlan& p) {
+    return kernels[(group == 128 ? 0 : 42) + (p.kw == 4 ? 0 : 21) + (p.nr - 2) * 7 + (p.digits ? 4 : p.split > 1 ? 3 : 0) + p.depth / 2 - 1];
 }
 
 // What a plan may take, the padding of the sums aside: it comes from what is left above, so that it costs no ring slot, no warp along K and no second CTA
@@ -311,6 +106,8 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, bool di
     if (cost < 0.0) {
         return false;
     }
+    best.per = best.units / best.ctas;
+    best.more = best.units % best.ctas;
     int units = 0;
     for (int i = 0; i < a.nseg; ++i) {
         const int ur = RG_WARPS / best.kw * best.nr;
@@ -424,6 +221,8 @@ bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& 
         }
     }
     if (found) {
+        best.per = best.units / (best.ctas / best.split);
+        best.more = best.units % (best.ctas / best.split);
         const int ur = RG_WARPS / best.kw * best.nr;
         int units = 0;
         for (int i = 0; i < a.nseg; ++i) {
@@ -434,7 +233,7 @@ bool rg_cluster_plan(GemvArgs& a, const int* clusters, int force_split, RgPlan& 
     return found;
 }
 
-const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(group, p).name; }
+const char* gemv_rg_name(int group, const RgPlan& p) { return rg_kernel(rg_kernels, group, p).name; }
 
 cudaError_t gemv_rg_init_device() {
     for (const RgKernel& k : rg_kernels) {
@@ -447,6 +246,13 @@ cudaError_t gemv_rg_init_device() {
 }
 
 cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st) {
+    const void* kernel = rg_kernel(a.dbg != nullptr ? rg_timeline_kernels() : rg_kernels, a.group, p).f;
+    if (a.dbg != nullptr) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RG_SMEM_MAX + RG_PAD_MAX);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(p.ctas);
     cfg.blockDim = dim3(RG_THREADS);
@@ -469,7 +275,7 @@ cudaError_t launch_gemv_rg(const GemvArgs& a, const RgPlan& p, cudaStream_t st) 
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     void* args[] = {const_cast<GemvArgs*>(&a), const_cast<RgPlan*>(&p)};
-    return cudaLaunchKernelExC(&cfg, rg_kernel(a.group, p).f, args);
+    return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 }  // namespace w4

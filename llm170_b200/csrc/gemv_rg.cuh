@@ -6,6 +6,12 @@
 
 namespace w4 {
 
+struct RgKernel {
+    const void* f;
+    const char* name;
+};
+const RgKernel* rg_timeline_kernels();   // as rg_kernels of gemv_rg_kernel.cuh
+
 constexpr int RG_WARPS = 8;
 constexpr int RG_THREADS = RG_WARPS * 32;
 constexpr int RG_XPAD = 32;            // bytes added to a token's row of x: 32 mod 128, conflict-free 8-byte reads of eight rows

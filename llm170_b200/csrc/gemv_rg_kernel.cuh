@@ -1,0 +1,223 @@
+// The row-group GEMV kernel (gemv_rg.cu) and its instantiations, with the diagnostic timeline or without: RG_TIMELINE is defined by the source.
+#pragma once
+#include <cuda_fp16.h>
+
+#include "gemv_rg.cuh"
+
+namespace w4 {
+
+namespace {
+
+// KW = warps along K; the other warps of a CTA take further row blocks.  NR = row blocks per warp, D = ring slots per warp.
+// CL: the CTAs of a cluster share K as well, so that a unit's rows are spread over several SMs and each stages its part of x only; their sums
+// meet in distributed shared memory, in the order of their ranks.  DIG: activations as digits.  TL: the diagnostic timeline, in kernels of their own:
+// an SM fetches a launch's code anew, and the stamps' alone took 0.17 us of every launch (7168 x 5120 5.33 -> 5.19, 896 x 5120 3.35 -> 3.18).
+template <int GROUP, int KW, int NR, int D, bool CL, bool DIG, bool TL>
+__global__ void __launch_bounds__(RG_THREADS, 2) gemv_rg_kernel(const GemvArgs a, const RgPlan p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long s_xbar;
+    __shared__ int s_abort;
+    constexpr int RW = RG_WARPS / KW, UR = RW * NR;           // row blocks of a unit
+    constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1; // k-blocks per unit of K: 2 (g128) or 1
+    constexpr int PITCH = rg_red_pitch(UR);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // wall-clock stamps of thread 0 in the slots of the other forms
+    auto stamp_now = [&](int j) {
+        if (TL && threadIdx.x == 0 && (int)blockIdx.x < DBG_CTAS) {
+            unsigned long long ns;
+            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(ns));
+            a.dbg[((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS + j] = (long long)ns;
+        }
+    };
+    stamp_now(0);
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int kw = warp % KW, rw = warp / KW;
+    const int cl = CL ? p.split : 1, rank = CL ? (int)blockIdx.x % cl : 0, cta = CL ? (int)blockIdx.x / cl : (int)blockIdx.x;
+    // equal contiguous runs of units (row groups over all segments)
+    const int u0 = p.per * cta + min(p.more, cta), u1 = u0 + p.per + (cta < p.more ? 1 : 0);
+    const int ku_all = a.k / (TILE_K * KPU), ng = a.k / GROUP;
+    const int ku0 = ku_all * rank / cl, ku = ku_all * (rank + 1) / cl - ku0;   // this CTA's part of K
+    const int kb0 = ku * kw / KW * KPU, nk = ku * (kw + 1) / KW * KPU - kb0;   // this warp's k-blocks, from there
+    auto seg_of = [&](int u) {
+        int si = 0;
+#pragma unroll
+        for (int i = 1; i < GEMV_MAX_SEG; ++i) {
+            if (i < a.nseg && u >= a.seg[i].cta0) {
+                si = i;
+            }
+        }
+        return si;
+    };
+
+    // ---- weights and scales, in the order of use
+    RgStream<GROUP, NR, D> ring;
+    ring.init(smem_u32(smem) + (uint32_t)p.off_ring + (uint32_t)warp * (D * rg_slot_bytes(GROUP, NR)), lane);
+    int fu = u0;
+    auto fetch_unit = [&]() {
+        const int si = seg_of(fu), nrb = a.seg[si].n / TILE_ROWS;
+        ring.unit(a.seg[si].qt, a.seg[si].st, 0, (fu - a.seg[si].cta0) * UR + rw * NR, nrb, nrb, ng, ku0 * KPU + kb0, nk, lane);
+    };
+    auto next_unit = [&]() {
+        if (++fu < u1) {
+            fetch_unit();
+        }
+    };
+    if (threadIdx.x == 0) {
+        s_abort = 0;
+        mbar_init(smem_u32(&s_xbar), 1);
+        mbar_init_fence();
+        if (TL && (int)blockIdx.x < DBG_CTAS) {
+            unsigned smid;
+            asm volatile("mov.u32 %0, %smid;" : "=r"(smid));
+            long long* d = a.dbg + ((size_t)a.dbg_seq * DBG_CTAS + blockIdx.x) * DBG_STAMPS;
+            d[6] = smid;
+            d[7] = u1 - u0;
+        }
+    }
+    if (nk > 0) {
+        fetch_unit();
+#pragma unroll 1
+        for (int d = 0; d < D; d += 2) {
+            ring.template fetch<false>(lane, next_unit);
+            ring.template fetch<true>(lane, next_unit);
+        }
+    }
+    stamp_now(8);   // first tiles requested
+    __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");        // x and the outputs may be the previous kernel's
+    stamp_now(1);
+
+    // ---- activations: one bulk copy per token, or digits, every warp its part of K
+    const int m = a.m, xbytes = ku * (KPU * TILE_K * 2);
+    const int xstride = DIG ? rg_digit_stride(a.k) : CL ? (ku_all + cl - 1) / cl * (KPU * TILE_K * 2) + RG_XPAD : a.k * 2 + RG_XPAD;
+    float mul[RG_MAX_DIGIT_TOKENS] = {};
+    if (DIG) {
+        rg_stage_digits(smem_u32(smem), (uint32_t)xstride, smem_u32(smem) + (uint32_t)(p.off_raw + m * (kb0 * RW + rw * nk) * (TILE_K * 2)), a.x, a.k, m, kb0, nk, rw, RW, lane, mul);
+        if (RW > 1) {
+            __syncthreads();
+        } else {
+            __syncwarp();
+        }
+    } else {
+        if (warp == 0) {
+            if (lane == 0) {
+                mbar_expect_tx(smem_u32(&s_xbar), (uint32_t)(m * xbytes));
+            }
+            __syncwarp();
+            if (lane < m) {
+                bulk_load(smem_u32(smem) + (uint32_t)(lane * xstride), a.x + (size_t)lane * a.k + ku0 * (KPU * TILE_K), (uint32_t)xbytes, smem_u32(&s_xbar));
+            }
+        }
+        if (!mbar_wait(smem_u32(&s_xbar), 0, &s_abort, a.status, (43 << 16))) {
+            mbar_drain(smem_u32(&s_xbar), 0);
+        }
+        __syncwarp();
+    }
+    stamp_now(2);   // x staged
+    stamp_now(3);
+    // lanes without a token read token 0, those without a digit digit 2: their columns are never stored
+    const uint32_t xl = smem_u32(smem) + (DIG ? (uint32_t)(((g >> 2 < m ? g >> 2 : 0) * 3 + min(g & 3, 2)) * xstride + kb0 * TILE_K + t * 16)
+                                              : (uint32_t)((g < m ? g : 0) * xstride + kb0 * (TILE_K * 2) + t * 8));
+    const int mp = (m + 1) & ~1;
+    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][mp][PITCH]
+    for (int u = u0; u < u1; ++u) {
+        float tot[NR][4];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            tot[r][0] = tot[r][1] = tot[r][2] = tot[r][3] = 0.f;
+        }
+        if (DIG) {
+            rg_multiply_digits<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
+        } else {
+            rg_multiply<GROUP, NR, D>(tot, xl, nk, ring, lane, next_unit);
+        }
+        stamp_now(4);   // (of the last unit)
+        // ---- the K warps' sums meet in shared memory
+        const GemvSeg& sg = a.seg[seg_of(u)];
+        const int rb0 = (u - sg.cta0) * UR, rows = min(UR, sg.n / TILE_ROWS - rb0) * TILE_ROWS;
+        if (u > u0) {
+            __syncthreads();
+        }
+        if (DIG) {
+            // lanes t = 0, 2 have digits 0 and 1 of a token, 1 and 3 digit 2: they put them together, and the first stores row g, the second row g + 8
+            const int tok = t >> 1, odd = t & 1;
+            const float mt = (tok ? mul[1] : mul[0]) * sg.out_mul, w0 = odd ? 65536.f * mt : mt, w1 = odd ? 0.f : 256.f * mt;
+            float* d = red + (kw * mp + tok) * PITCH + rw * NR * TILE_ROWS + g + odd * 8;
+#pragma unroll
+            for (int r = 0; r < NR; ++r) {
+                const float lo = fmaf(tot[r][1], w1, tot[r][0] * w0), hi = fmaf(tot[r][3], w1, tot[r][2] * w0);
+                const float other = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
+                if (tok < m) {
+                    d[r * TILE_ROWS] = (odd ? hi : lo) + other;
+                }
+            }
+        } else if (2 * t < mp) {
+            const float m0 = 16777216.f * sg.out_mul, m1 = 1048576.f * sg.out_mul;
+            rg_store_sums(red + (kw * mp + 2 * t) * PITCH + rw * NR * TILE_ROWS + g, PITCH, tot, m0, m1);
+        }
+        __syncthreads();
+        auto local_sum = [&](int tok, int row) {
+            const float* d = red + tok * PITCH + row;
+            float v = d[0];
+#pragma unroll
+            for (int w = 1; w < KW; ++w) {
+                v += d[w * mp * PITCH];                                  // fixed order: the same bits every run
+            }
+            return v;
+        };
+        constexpr int ROWS = UR * TILE_ROWS;
+        auto store = [&](int tok, int row, float v) {
+            const size_t o = (size_t)tok * sg.n + (size_t)rb0 * TILE_ROWS + row;
+            if (a.out_f16) {
+                reinterpret_cast<__half*>(sg.out)[o] = __float2half_rn(v);
+            } else {
+                reinterpret_cast<float*>(sg.out)[o] = v;
+            }
+        };
+        if (CL) {
+            // a CTA's sums for the others of its cluster, two units in turn: those of the unit before may still be read
+            const uint32_t part = smem_u32(smem) + (uint32_t)p.off_part + (uint32_t)((u - u0) & 1) * (ROWS * GEMV_MAX_M * 4);
+            for (int e = threadIdx.x; e < ROWS * m; e += RG_THREADS) {
+                const int tok = e / ROWS;
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(part + (uint32_t)e * 4u), "f"(local_sum(tok, e - tok * ROWS)) : "memory");
+            }
+            cluster_sync_all();
+            for (int e = ROWS * m * rank / cl + (int)threadIdx.x; e < ROWS * m * (rank + 1) / cl; e += RG_THREADS) {
+                const int tok = e / ROWS, row = e - tok * ROWS;
+                float v = ld_dsmem_f32(part + (uint32_t)e * 4u, 0);
+                for (int c = 1; c < cl; ++c) {
+                    v += ld_dsmem_f32(part + (uint32_t)e * 4u, (unsigned)c);
+                }
+                if (row < rows) {
+                    store(tok, row, v);
+                }
+            }
+        } else {
+            for (int e = threadIdx.x; e < ROWS * m; e += RG_THREADS) {
+                const int tok = e / ROWS, row = e - tok * ROWS;
+                if (row < rows) {
+                    store(tok, row, local_sum(tok, row));
+                }
+            }
+        }
+    }
+    if (CL) {
+        cluster_sync_all();                                   // nothing of this CTA's shared memory is still read
+    }
+    stamp_now(5);   // sums stored
+}
+
+#define W4_RG(G, K, N, D, C) {(const void*)gemv_rg_kernel<G, K, N, D, C, false, RG_TIMELINE>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ">"}
+#define W4_RGD(G, K, N, D) {(const void*)gemv_rg_kernel<G, K, N, D, false, true, RG_TIMELINE>, "gemv_rg_kernel<" #G "," #K "," #N "," #D ",digits>"}
+#define W4_RG_D(G, K, N) W4_RG(G, K, N, 2, false), W4_RG(G, K, N, 4, false), W4_RG(G, K, N, 6, false), W4_RG(G, K, N, 2, true), \
+                         W4_RGD(G, K, N, 2), W4_RGD(G, K, N, 4), W4_RGD(G, K, N, 6)
+#define W4_RG_N(G, K) W4_RG_D(G, K, 2), W4_RG_D(G, K, 3), W4_RG_D(G, K, 4)
+const RgKernel rg_kernels[] = {W4_RG_N(128, 4), W4_RG_N(128, 8), W4_RG_N(32, 4), W4_RG_N(32, 8)};
+#undef W4_RG_N
+#undef W4_RG_D
+#undef W4_RGD
+#undef W4_RG
+
+}  // namespace
+}  // namespace w4

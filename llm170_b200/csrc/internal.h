@@ -150,7 +150,7 @@ constexpr int RG_MAX_DIGIT_TOKENS = 2;
 struct RgPlan {
     int nr, kw;              // row blocks per warp, warps along K
     int units;               // row groups over all segments (seg[].cta0 = first of the segment)
-    int ctas;                // CTA c takes units [units c / ctas, units (c + 1) / ctas)
+    int ctas, per, more;     // a CTA, or cluster, takes `per` units in a row, the first `more` of them one more
     int depth;               // ring slots per warp
     int split;               // CTAs of a cluster that share K (1: none)
     bool digits;             // activations as digits (gemv_rg.cuh)
