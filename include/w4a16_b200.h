@@ -98,7 +98,7 @@ W4A16_API const char* w4a16_last_kernel(w4a16_dec* dec);
  *   the (row block, K split) form takes the rest: "gemv_ksplit" (0 = automatic), "gemv_stages" (16 KB weight stages in flight per
  *       CTA, 2..8, default 4), "gemv_warps" (consumer warps per CTA, 8 or 16), "gemv_cluster" (1 = default: 2..8 K splits of a row
  *       block run as a thread-block cluster and reduce through distributed shared memory)
- *   "gemv_subnormal" (1 = default arithmetic, 0 = exact nibble-8 operands), "moe_gemv" (MoE decode: 0 = automatic, 1 = the (row
+ *   "gemv_subnormal" (1 = default arithmetic, 0 = exact nibble-8 operands), "moe_gemv" (MoE decode: 0 = automatic, which takes layers of a few tokens in two launches, 1 = the (row
  *       block, K split) form, 2, 4 or 8 = the row-group form with that many warps along K), "moe_gemm" (MoE prefill: 0 = automatic,
  *       1 = weight rows, 2 = token rows, 128, 192 or 256 = CTA pairs with tiles of at most that many rows), "tp_wait_log2" (16..40,
  *       default 31: the fused all-reduce gives up on its peers after 2^n cycles)

@@ -19,7 +19,7 @@ SO = os.path.join(HERE, "libw4a16_b200.so")
 NATIVE_SO = os.path.join(HERE, "_native.so")
 HASH = SO + ".srchash"
 NATIVE_HASH = NATIVE_SO + ".srchash"
-SOURCES = ["dec.cu", "repack.cu", "gemv.cu", "gemv_sk.cu", "gemv_rb.cu", "gemv_rg.cu", "gemv_rg_timeline.cu", "gemv_moe.cu", "gemm_tc.cu", "gemm_ts.cu", "gemm_ts2.cu", "moe.cu", "moe_host.cu", "gemv_static.cu", "loader.cu", "head.cu"]
+SOURCES = ["dec.cu", "repack.cu", "gemv.cu", "gemv_sk.cu", "gemv_rb.cu", "gemv_rg.cu", "gemv_rg_timeline.cu", "gemv_moe.cu", "gemv_moe_few.cu", "gemm_tc.cu", "gemm_ts.cu", "gemm_ts2.cu", "moe.cu", "moe_host.cu", "gemv_static.cu", "loader.cu", "head.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC,-fvisibility=hidden,-Wall", "--shared", "-cudart", "static",

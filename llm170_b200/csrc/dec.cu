@@ -578,6 +578,9 @@ int w4a16_dec_new(int device, w4a16_dec** out) {
         if (e == cudaSuccess) {
             e = w4::gemv_moe_init_device();
         }
+        if (e == cudaSuccess) {
+            e = w4::gemv_moe_few_init_device();
+        }
     }
     if (e == cudaSuccess) {
         e = w4::gemm_init_device();

@@ -1,0 +1,318 @@
+// A mixture-of-experts layer of a few tokens in two launches: router top-k and first matmul with its activation; second matmul, routing weights
+// and the sum over a token's picks.
+//
+// Takes the place of the reference's routing, grouped GEMV, activation and combine kernels (crates/backend-gpu/src/rawcuda/w4a16_dec/moe/mod.rs:263-447,
+// crates/backend-gpu/src/rawcuda/assets/gptq4.cu:317-374, crates/backend-gpu/src/rawcuda/assets/moe.cu:1649-1674) for up to 32 (token, pick) pairs.
+// Same arithmetic and the same roundings to f16 as the launches for more of them (moe.cu, gemv_moe.cu); activations are multiplied as digits (gemv_rg.cuh).
+//
+// Bound by what surrounds the stream: a token of 128 experts x 768 x 2048 reads 19 MB, 3 us, and took 17.9 us in four launches that wait for one another;
+// 12.4 here.  (Of these the routing takes 2.8, most of it fetching code that runs once; ranking the experts by all threads instead was slower, 13.0.)
+//   * every CTA routes the tokens for itself, a warp per token, while its other warps stage the activations: no routing launch, no tables;
+//   * the second matmul routes once more, while the first one still runs, and has its first weights on the way when that is complete: its CTAs fit on
+//     the SMs beside those of the first (half the registers, less than half the shared memory each);
+//   * its warps take a pick each for the same rows, so a token's picks meet in shared memory, in the order of the picks: no sum kernel.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "gemv_rg.cuh"
+#include "moe_topk.cuh"
+
+namespace w4 {
+
+namespace {
+
+constexpr int FEW_UP_D = 8, FEW_DOWN_D = 8;                   // ring slots per warp
+constexpr int FEW_UP_SMEM = 134 * 1024, FEW_DOWN_SMEM = 92 * 1024;   // both on one SM: 228 KB less 1 KB each
+constexpr int FEW_RED = RG_WARPS * 36;                        // floats: a unit's sums, 32 rows and padding per warp
+
+// Routes the tokens, warp w token w: s_exp / s_wt hold the picks of token i from i * k on.
+__device__ __forceinline__ void few_route(const MoeFewArgs& a, int warp, int lane, int* s_exp, float* s_wt, float* s_stage) {
+    if (warp < a.t) {
+        const float* l = a.logits + (size_t)warp * a.n_exp;
+        if (a.n_exp <= 128) {
+            topk_of_token_n<4>(l, s_exp + warp * a.k, s_wt + warp * a.k, a.n_exp, a.k, lane, s_stage + warp * a.n_exp);
+        } else {
+            topk_of_token_n<8>(l, s_exp + warp * a.k, s_wt + warp * a.k, a.n_exp, a.k, lane, s_stage + warp * a.n_exp);
+        }
+    }
+}
+
+// the token of a pick, t <= 4
+__device__ __forceinline__ int few_token(int slot, int k) { return (slot >= k) + (slot >= 2 * k) + (slot >= 3 * k); }
+
+template <int GROUP>
+__global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_few_up_kernel(const MoeFewArgs a, const MoeFewPlan p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_exp[MOE_FEW_SLOTS], s_list[RG_WARPS][MOE_FEW_SLOTS];
+    __shared__ float s_wt[MOE_FEW_SLOTS], s_mul[RG_WARPS][MOE_FEW_TOKENS];
+    constexpr int NR = 2, KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int ku = a.hidden / (TILE_K * KPU), ng = a.hidden / GROUP;
+    const uint32_t base = smem_u32(smem), stride = (uint32_t)rg_digit_stride(a.hidden);
+    float* red = reinterpret_cast<float*>(smem + p.off_red);
+    RgStream<GROUP, NR, FEW_UP_D> ring;
+    ring.init(base + (uint32_t)p.off_ring + (uint32_t)warp * (FEW_UP_D * rg_slot_bytes(GROUP, NR)), lane);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the second matmul reads the logits before its own wait: only now are they complete
+    few_route(a, warp, lane, s_exp, s_wt, reinterpret_cast<float*>(smem + p.off_stage));
+
+    // the parts of K are dealt to the warps that do not route (t <= 4 of 8)
+    for (int part = warp - a.t; part >= 0 && part < RG_WARPS; part += RG_WARPS - a.t) {
+        const int kb0 = ku * part / RG_WARPS * KPU, nk = ku * (part + 1) / RG_WARPS * KPU - kb0;
+        for (int tok = 0; tok < a.t && nk > 0; tok += RG_MAX_DIGIT_TOKENS) {
+            float mul[RG_MAX_DIGIT_TOKENS] = {};
+            const int m = min(RG_MAX_DIGIT_TOKENS, a.t - tok);
+            rg_stage_digits(base + (uint32_t)(tok * 3) * stride, stride, base + (uint32_t)(p.off_raw + a.t * kb0 * (TILE_K * 2)), a.x + (size_t)tok * a.hidden, a.hidden, m, kb0, nk, 0, 1,
+                            lane, mul);
+            __syncwarp();
+            if (lane < m) {
+                s_mul[part][tok + lane] = lane ? mul[1] : mul[0];
+            }
+        }
+    }
+    __syncthreads();
+    // ---- the picks whose experts are here, and this CTA's units: 16 outputs of a pick (a gate and an up row block)
+    const bool here = lane < a.t * a.k && s_exp[lane] >= a.e0 && s_exp[lane] < a.e1;
+    const unsigned mask = __ballot_sync(0xffffffffu, here);
+    if (here) {
+        s_list[warp][__popc(mask & ((1u << lane) - 1u))] = lane;
+    }
+    __syncwarp();
+    const int ppu = a.ffn / TILE_ROWS, units = __popc(mask) * ppu, per = units / (int)gridDim.x, more = units % (int)gridDim.x;
+    const int u0 = per * (int)blockIdx.x + min(more, (int)blockIdx.x), u1 = u0 + per + ((int)blockIdx.x < more ? 1 : 0);
+    const int kb0 = ku * warp / RG_WARPS * KPU, nk = ku * (warp + 1) / RG_WARPS * KPU - kb0;
+    int li = u0 / ppu, pair = u0 - li * ppu, fu = u0, fli = li, fpair = pair;
+    auto fetch_unit = [&]() { ring.unit(a.qt, a.st, (s_exp[s_list[warp][fli]] - a.e0) * 2 * ppu, fpair * NR, 2 * ppu, a.nrb_all, ng, kb0, nk, lane); };
+    auto next_unit = [&]() {
+        if (++fu < u1) {
+            if (++fpair == ppu) {
+                fpair = 0;
+                ++fli;
+            }
+            fetch_unit();
+        }
+    };
+    ring.left = 0;
+    if (u0 < u1 && nk > 0) {
+        fetch_unit();
+    }
+#pragma unroll 1
+    for (int d = 0; d < FEW_UP_D; d += 2) {
+        ring.template fetch<false>(lane, next_unit);
+        ring.template fetch<true>(lane, next_unit);
+    }
+    for (int u = u0; u < u1; ++u) {
+        const int slot = s_list[warp][li], tok = few_token(slot, a.k);
+        float tot[NR][4] = {};
+        rg_multiply_digits<GROUP, NR, FEW_UP_D>(tot, base + (uint32_t)(tok * 3 + min(g & 3, 2)) * stride + (uint32_t)(kb0 * TILE_K + t * 16), nk, ring, lane, next_unit);
+        // lanes t = 0, 1 have the digits of rows g and g + 8 (2, 3: the same again); the sums of two units in turn
+        float* d = red + ((u - u0) & 1) * FEW_RED;
+        const float mt = nk > 0 ? s_mul[warp][tok] * a.out_mul : 0.f, w0 = t & 1 ? 65536.f * mt : mt, w1 = t & 1 ? 0.f : 256.f * mt;
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const float lo = fmaf(tot[r][1], w1, tot[r][0] * w0), hi = fmaf(tot[r][3], w1, tot[r][2] * w0);
+            const float other = __shfl_xor_sync(0xffffffffu, t & 1 ? lo : hi, 1);
+            if (t < 2) {
+                d[warp * 36 + r * TILE_ROWS + g + t * 8] = (t ? hi : lo) + other;
+            }
+        }
+        __syncthreads();
+        if (warp == 0) {
+            float v = d[lane];
+#pragma unroll
+            for (int w = 1; w < RG_WARPS; ++w) {
+                v += d[w * 36 + lane];                                // fixed order: the same bits every run
+            }
+            const float up = __shfl_down_sync(0xffffffffu, v, 16);
+            if (lane < TILE_ROWS) {
+                reinterpret_cast<__half*>(a.act)[(size_t)slot * a.ffn + pair * TILE_ROWS + lane] = silu_mul_f16(v, up);
+            }
+        }
+        if (++pair == ppu) {
+            pair = 0;
+            ++li;
+        }
+    }
+}
+
+// p.ways warps share the channels of a pick.
+template <int GROUP>
+__global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_few_down_kernel(const MoeFewArgs a, const MoeFewPlan p) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int s_exp[MOE_FEW_SLOTS];
+    __shared__ float s_wt[MOE_FEW_SLOTS], s_red[2][MOE_FEW_SLOTS][TILE_ROWS + 1], s_mul[RG_WARPS][MOE_FEW_PICKS_PER_WARP];
+    constexpr int KPU = GROUP >= TILE_K ? GROUP / TILE_K : 1;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3;
+    const int ku = a.ffn / (TILE_K * KPU), ng = a.ffn / GROUP, nrb = a.hidden / TILE_ROWS;
+    const int ways = p.ways, way = warp % ways, j0 = warp / ways, dj = RG_WARPS / ways;
+    const int kb0 = ku * way / ways * KPU, nk = ku * (way + 1) / ways * KPU - kb0;
+    const uint32_t base = smem_u32(smem), stride = (uint32_t)rg_digit_stride((ku + ways - 1) / ways * KPU * TILE_K);
+    const int per = nrb * a.t / (int)gridDim.x, more = nrb * a.t % (int)gridDim.x;
+    const int u0 = per * (int)blockIdx.x + min(more, (int)blockIdx.x), u1 = u0 + per + ((int)blockIdx.x < more ? 1 : 0);
+    few_route(a, warp, lane, s_exp, s_wt, reinterpret_cast<float*>(smem + p.off_stage));
+    __syncthreads();
+    auto here = [&](int slot) { return s_exp[slot] >= a.e0 && s_exp[slot] < a.e1; };
+    RgStream<GROUP, 1, FEW_DOWN_D> ring;
+    ring.init(base + (uint32_t)p.off_ring + (uint32_t)warp * (FEW_DOWN_D * rg_slot_bytes(GROUP, 1)), lane);
+    ring.left = 0;
+    // this warp's work: for every unit (token, 16 rows) the picks j0, j0 + dj, .. whose experts are here
+    int tok = few_token(u0, nrb), rb = u0 - tok * nrb, fu = u0, fj = j0 - dj, ftok = tok, frb = rb;
+    auto next_unit = [&]() {
+        while (nk > 0 && fu < u1) {
+            if ((fj += dj) >= a.k) {
+                fj = j0 - dj;
+                ++fu;
+                if (++frb == nrb) {
+                    frb = 0;
+                    ++ftok;
+                }
+            } else if (here(ftok * a.k + fj)) {
+                ring.unit(a.qt, a.st, (s_exp[ftok * a.k + fj] - a.e0) * nrb, frb, nrb, a.nrb_all, ng, kb0, nk, lane);
+                break;
+            }
+        }
+    };
+    next_unit();
+#pragma unroll 1
+    for (int d = 0; d < FEW_DOWN_D; d += 2) {
+        ring.template fetch<false>(lane, next_unit);
+        ring.template fetch<true>(lane, next_unit);
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    int staged = -1;
+    for (int u = u0; u < u1; ++u) {
+        const int buf = (u - u0) & 1;
+        if (tok != staged) {
+            staged = tok;
+#pragma unroll 1
+            for (int i = 0, j = j0; j < a.k; ++i, j += dj) {
+                if (nk > 0 && here(tok * a.k + j)) {
+                    float m2[RG_MAX_DIGIT_TOKENS] = {};
+                    rg_stage_digits(base + (uint32_t)((warp * p.picks + i) * 3) * stride - (uint32_t)(kb0 * TILE_K), stride, base + (uint32_t)(p.off_raw + warp * p.raw_bytes),
+                                    reinterpret_cast<const uint16_t*>(a.act) + (size_t)(tok * a.k + j) * a.ffn, a.ffn, 1, kb0, nk, 0, 1, lane, m2);
+                    s_mul[warp][i] = m2[0];
+                    __syncwarp();
+                }
+            }
+        }
+#pragma unroll 1
+        for (int i = 0, j = j0; j < a.k; ++i, j += dj) {
+            if (here(tok * a.k + j)) {
+                float tot[1][4] = {};
+                rg_multiply_digits<GROUP, 1, FEW_DOWN_D>(tot, base + (uint32_t)((warp * p.picks + i) * 3 + min(g & 3, 2)) * stride + (uint32_t)(t * 16), nk, ring, lane, next_unit);
+                const float mt = nk > 0 ? s_mul[warp][i] * a.out_mul : 0.f, w0 = t & 1 ? 65536.f * mt : mt, w1 = t & 1 ? 0.f : 256.f * mt;
+                const float lo = fmaf(tot[0][1], w1, tot[0][0] * w0), hi = fmaf(tot[0][3], w1, tot[0][2] * w0);
+                const float other = __shfl_xor_sync(0xffffffffu, t & 1 ? lo : hi, 1);
+                if (t < 2) {
+                    const float v = (t ? hi : lo) + other;
+                    s_red[buf][j * ways + way][g + t * 8] = ways == 1 ? mul_row_w(v, s_wt[tok * a.k + j]) : v;
+                }
+            } else if (lane < TILE_ROWS) {
+                s_red[buf][j * ways + way][lane] = 0.f;               // the expert lives on another rank
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x < TILE_ROWS) {
+            float sum = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < a.k; ++j) {
+                float v = s_red[buf][j * ways][threadIdx.x];
+                if (ways > 1) {
+                    for (int w = 1; w < ways; ++w) {
+                        v += s_red[buf][j * ways + w][threadIdx.x];
+                    }
+                    v = mul_row_w(v, s_wt[tok * a.k + j]);
+                }
+                sum += v;
+            }
+            const size_t o = (size_t)tok * a.hidden + rb * TILE_ROWS + threadIdx.x;
+            if (a.out_f16) {
+                reinterpret_cast<__half*>(a.out)[o] = __float2half_rn(sum);
+            } else {
+                reinterpret_cast<float*>(a.out)[o] = sum;
+            }
+        }
+        if (++rb == nrb) {
+            rb = 0;
+            ++tok;
+        }
+    }
+}
+
+template <class F>
+cudaError_t launch_few(F* kernel, int grid, int smem, const MoeFewArgs& a, const MoeFewPlan& p, cudaStream_t st) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(RG_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (a.pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelEx(&cfg, kernel, a, p);
+}
+
+}  // namespace
+
+// Plans of both launches; false: the layer takes the launches for more tokens.  Every pick reads its expert for itself here, and a unit's ends are not hidden
+// behind the next one's stream, so the line lies at the bytes: us per layer, the other launches / these, groups of 32, one token and two: 128 experts,
+// top-8, 2048 x 768, all of them here 18.0 / 13.1, 22.2 / 19.5 (three: 25.5 / 26.2), half 17.1 / 10.8, 18.2 / 15.3, a quarter 15.6 / 9.2, 17.0 / 12.7
+// (three, 14 MB: 17.4 / 16.5, four 17.9 / 19.0); 256 experts, 1024 x 384, a quarter 15.0 / 8.0, 15.5 / 9.1, 16.4 / 11.1, 16.3 / 11.7; 8 experts, top-2,
+// 4096 x 2048 in groups of 128 18.8 / 13.9, 23.0 / 20.7; 64 experts, top-8, 3072 x 1024 in groups of 128 21.0 / 18.3.  A rank that less than a
+// pick of a token reaches on average keeps the others, too.
+bool moe_few_plan(int t, int n_exp, int k, int n_local, int hidden, int ffn, int group, MoeFewPlan& up, MoeFewPlan& down) {
+    const double bytes = 1.5 * t * k * n_local / n_exp * hidden * ffn;               // of the picks' weights, on average
+    if (t > MOE_FEW_TOKENS || t * k > MOE_FEW_SLOTS || n_exp > 256 || n_local * k < n_exp || bytes > (t <= 2 ? 40e6 : 8e6)) {
+        return false;
+    }
+    auto round_up = [](int v) { return (v + 127) & ~127; };
+    const int stage = round_up(t * n_exp * 4);
+    up = MoeFewPlan{};
+    up.off_raw = round_up(3 * t * rg_digit_stride(hidden));
+    up.off_red = up.off_raw + round_up(t * hidden * 2);
+    up.off_stage = up.off_red + round_up(2 * FEW_RED * 4);
+    up.off_ring = up.off_stage + stage;
+    up.smem = up.off_ring + RG_WARPS * FEW_UP_D * rg_slot_bytes(group, 2);
+    down = MoeFewPlan{};
+    down.ways = k > 4 ? 1 : k > 2 ? 2 : k > 1 ? 4 : 8;
+    down.picks = (k * down.ways + RG_WARPS - 1) / RG_WARPS;
+    const int unit = group > TILE_K ? group : TILE_K, part = (ffn / unit + down.ways - 1) / down.ways * unit;
+    down.raw_bytes = part * 2;
+    down.off_raw = round_up(RG_WARPS * down.picks * 3 * rg_digit_stride(part));
+    down.off_stage = down.off_raw + round_up(RG_WARPS * down.raw_bytes);
+    down.off_ring = down.off_stage + stage;
+    down.smem = down.off_ring + RG_WARPS * FEW_DOWN_D * rg_slot_bytes(group, 1);
+    return up.smem <= FEW_UP_SMEM && down.smem <= FEW_DOWN_SMEM;
+}
+
+cudaError_t gemv_moe_few_init_device() {
+    for (const void* f : {(const void*)gemv_moe_few_up_kernel<128>, (const void*)gemv_moe_few_up_kernel<32>, (const void*)gemv_moe_few_down_kernel<128>,
+                          (const void*)gemv_moe_few_down_kernel<32>}) {
+        cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_UP_SMEM);
+        if (e == cudaSuccess) {
+            e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);   // room for both on an SM
+        }
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_gemv_moe_few_up(const MoeFewArgs& a, const MoeFewPlan& p, int group, int sm_count, cudaStream_t st) {
+    return launch_few(group == 128 ? gemv_moe_few_up_kernel<128> : gemv_moe_few_up_kernel<32>, sm_count, p.smem, a, p, st);
+}
+
+cudaError_t launch_gemv_moe_few_down(const MoeFewArgs& a, const MoeFewPlan& p, int group, int sm_count, cudaStream_t st) {
+    return launch_few(group == 128 ? gemv_moe_few_down_kernel<128> : gemv_moe_few_down_kernel<32>, std::min(sm_count, a.t * (a.hidden / TILE_ROWS)), p.smem, a, p, st);
+}
+
+}  // namespace w4

@@ -355,6 +355,7 @@ __device__ __forceinline__ void rg_multiply_digits(float (&tot)[NR][4], uint32_t
     };
     if (GROUP == 32) {
         const float z[4] = {-RG_F32_ZERO, -RG_F32_ZERO, -RG_F32_ZERO, -RG_F32_ZERO};
+#pragma unroll(NR == 1 ? 2 : 1)
         for (int i = 0; i < nk; ++i) {
             const uint4 x = lds128(xa);
             xa += TILE_K;

@@ -179,6 +179,29 @@ struct MoeGemvPlan {
 bool moe_gemv_plan(int rows, int k, int group, int sm_count, int segments, int force_kw, MoeGemvPlan& p);
 cudaError_t launch_gemv_moe(const GemvArgs& a, const MoeGemvPlan& p, cudaStream_t st);
 cudaError_t gemv_moe_init_device();
+// ---- gemv_moe_few.cu: a MoE layer of up to 32 (token, pick) pairs in two launches ----
+constexpr int MOE_FEW_TOKENS = 4, MOE_FEW_SLOTS = 32, MOE_FEW_PICKS_PER_WARP = 4;
+struct MoeFewArgs {
+    const float* logits;     // [t][n_exp]
+    const uint16_t* x;       // [t][hidden] f16
+    void* act;               // [t * k][ffn] f16: silu(gate) * up of every pick whose expert is here
+    void* out;               // [t][hidden]
+    const uint4* qt;         // the launch's matrix
+    const uint32_t* st;
+    int nrb_all;             // its 16-row blocks
+    float out_mul;
+    int t, n_exp, k, e0, e1, hidden, ffn, out_f16, pdl;
+};
+struct MoeFewPlan {
+    int ways;                // second matmul: warps that share the channels of a pick
+    int picks;               // and picks per warp
+    int raw_bytes;
+    int off_raw, off_red, off_stage, off_ring, smem;   // byte offsets in dynamic shared memory: digits first
+};
+bool moe_few_plan(int t, int n_exp, int k, int n_local, int hidden, int ffn, int group, MoeFewPlan& up, MoeFewPlan& down);
+cudaError_t launch_gemv_moe_few_up(const MoeFewArgs& a, const MoeFewPlan& p, int group, int sm_count, cudaStream_t st);
+cudaError_t launch_gemv_moe_few_down(const MoeFewArgs& a, const MoeFewPlan& p, int group, int sm_count, cudaStream_t st);
+cudaError_t gemv_moe_few_init_device();
 bool gemv_rb_fits(const GemvArgs& a);
 int gemv_rb_plan(GemvArgs& a, int sm_count, int& rbw);
 cudaError_t launch_gemv_rb(const GemvArgs& a, int total_units, int rbw, int sm_count, cudaStream_t st);

@@ -175,6 +175,27 @@ int Dec::moe_ffn(int layer, const float* logits, const void* x16, void* y, int t
         if (max_tiles > mb.max_tiles) {
             return fail("w4a16 moe_ffn: tile table too small");
         }
+        // a token or a few of them: two launches instead of four (gemv_moe_few.cu)
+        MoeFewPlan up, down;
+        if (t <= MOE_FEW_TOKENS && tune_moe_gemv == 0 && tune_gemv_subnormal && tune_gemv_ksplit == 0 && moe_few_plan(t, moe.n_experts, moe.top_k, n_local, moe.hidden, moe.ffn, i13->second.group, up, down)) {
+            const Lin &l13 = i13->second, &l2 = i2->second;
+            MoeFewArgs a{logits, (const uint16_t*)x16, mb.act, y, (const uint4*)l13.qt, (const uint32_t*)l13.st, l13.n / TILE_ROWS, l13.out_mul,
+                         t, moe.n_experts, moe.top_k, moe.e0, moe.e1, moe.hidden, moe.ffn, out_kind == W4A16_OUT_F16, tune_pdl};
+            e = launch_gemv_moe_few_up(a, up, l13.group, sm_count, st);
+            if (e == cudaSuccess) {
+                a.qt = (const uint4*)l2.qt;
+                a.st = (const uint32_t*)l2.st;
+                a.nrb_all = l2.n / TILE_ROWS;
+                a.out_mul = l2.out_mul;
+                e = launch_gemv_moe_few_down(a, down, l2.group, sm_count, st);
+            }
+            if (e != cudaSuccess) {
+                return cuda_fail("moe_ffn launch", e);
+            }
+            launches += 2;
+            last_kernel = "gemv_moe_kernel<" + std::to_string(l2.group) + ",few>";
+            return 0;
+        }
         bool uneven = false;                         // whether the CTAs of the matmul before end far apart
         if (ns <= 1024) {
             // routing and all dispatch tables in one launch; the first grouped GEMV fetches each row's token itself

@@ -242,6 +242,81 @@ def test_grouped_gemv_forms(dec, orc, t, n_exp, k, f, h, group, way):
     assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # as above
 
 
+# Layers of up to 32 (token, pick) pairs in two launches: one to four tokens, 1 to 32 picks (8, 4, 2 or 1 warps for a pick, picks that a warp takes in
+# turn), fewer k-blocks than warps, odd numbers of them, a part of the experts here, picks that are all elsewhere, equal logits (the lower index first)
+@pytest.mark.parametrize("t,n_exp,k,f,h,group,e0,local", [(1, 8, 1, 64, 64, 32, 0, 8), (2, 8, 2, 128, 320, 64, 0, 8), (4, 16, 3, 192, 448, 32, 0, 16), (1, 16, 5, 320, 576, 32, 8, 8),
+                                                         (4, 32, 8, 256, 1024, 128, 16, 8), (3, 60, 9, 64, 192, 32, 0, 60), (1, 256, 32, 64, 128, 32, 100, 40), (2, 13, 4, 128, 256, 128, 3, 9),
+                                                         (1, 40, 17, 192, 2048, 64, 0, 40)])
+def test_layers_of_few_tokens(dec, orc, t, n_exp, k, f, h, group, e0, local):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, group, seed=101 + k)
+    x, lg = synth.make_acts(t, h, seed=102 + t), synth.make_router_logits(t, n_exp, seed=103 + t)
+    lg[0, n_exp // 2:] = lg[0, n_exp // 2]                          # equal shares for half of the experts
+    if t > 1:
+        lg[1, e0:e0 + local] -= 50.0                                # where experts are elsewhere, this token's picks are
+    if local < n_exp:                                               # an expert elsewhere adds nothing: the oracle gets zeros for it
+        w2_s = w2_s.copy()
+        zeros = w2_s.reshape(n_exp, -1)
+        zeros[:e0] = zeros[e0 + local:] = 0
+    dec.set_moe(n_exp, k, f, h, group, e0, local)
+    here = slice(e0, e0 + local)
+    dec.upload_experts(0, w13_q.reshape(n_exp, -1)[here], w13_s.reshape(n_exp, -1)[here], w2_q.reshape(n_exp, -1)[here], w2_s.reshape(n_exp, -1)[here])
+    xd, lgd = torch.from_numpy(x.view(np.float16).copy()).cuda(), torch.from_numpy(lg).cuda()
+    guard = torch.full((t + 1, h), 7.0, device="cuda", dtype=torch.float32)
+    y = dec.moe_ffn_dev_t(0, lgd, xd, t, out=guard[:t]).clone()
+    assert dec.last_kernel() == f"gemv_moe_kernel<{128 if group == 128 else 32},few>"
+    assert torch.equal(y, dec.moe_ffn_dev_t(0, lgd, xd, t)) and bool((guard[t:] == 7.0).all())
+    dec.set_tuning("moe_gemv", 4)
+    try:
+        other = dec.moe_ffn_dev_t(0, lgd, xd, t)
+        assert dec.last_kernel().endswith(",4>")
+    finally:
+        dec.set_tuning("moe_gemv", 0)
+    dec.sync()
+    # the same roundings to f16 of sums whose f32 terms are added in another order: one falls the other way now and then
+    assert float((y - other).norm()) <= 1e-3 * float(other.norm()) + 1e-6
+    want = orc.moe_ffn(x, lg, w13_q, w13_s, w2_q, w2_s, k, group)
+    err = np.abs(y.cpu().numpy() - want).max()
+    assert err <= TOL and err <= 0.02 * np.abs(want).max() + 1e-6, (err, np.abs(want).max())   # the bounds of the tests above
+    lgd[0, 0] = float("nan")                                        # a NaN makes all of its token's shares NaN: the first k experts, and NaN outputs
+    y = dec.moe_ffn_dev_t(0, lgd, xd, t)
+    assert bool(y[0].isnan().all()) or e0 >= k
+    assert t == 1 or bool(y[1:].isfinite().all())
+
+
+# which layers those are: both sides of the lines (moe_few_plan), and out of a graph that replays the layer over new rows
+@pytest.mark.parametrize("t,n_exp,k,f,h,local,few", [(2, 64, 8, 128, 256, 8, True), (2, 64, 8, 128, 256, 7, False), (4, 32, 8, 128, 256, 32, True), (4, 32, 9, 128, 256, 32, False),
+                                                    (5, 32, 4, 128, 256, 32, False), (3, 32, 8, 448, 448, 32, True), (3, 32, 8, 448, 512, 32, False), (1, 260, 2, 64, 128, 260, False)])
+def test_which_layers_take_two_launches(dec, t, n_exp, k, f, h, local, few):
+    w13_q, w13_s, w2_q, w2_s = synth.make_experts(n_exp, f, h, 32, seed=111)
+    dec.set_moe(n_exp, k, f, h, 32, 0, local)
+    dec.upload_experts(0, w13_q[:local], w13_s[:local], w2_q[:local], w2_s[:local])
+    xd = torch.from_numpy(synth.make_acts(t, h, seed=112).view(np.float16).copy()).cuda()
+    lgd = torch.from_numpy(synth.make_router_logits(t, n_exp, seed=113)).cuda()
+    out = torch.zeros((t, h), device="cuda")
+    c0 = dec.launch_count()
+    dec.moe_ffn_dev_t(0, lgd, xd, t, out=out)
+    assert dec.last_kernel().endswith(",few>") == few and (dec.launch_count() - c0 == 2) == few
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.ExternalStream(dec.stream_ptr())):
+        dec.capture_begin()
+        for _ in range(3):
+            dec.moe_ffn_dev_t(0, lgd, xd, t, out=out)
+        g = dec.capture_end()
+    for seed in range(3):
+        xd.copy_(torch.from_numpy(synth.make_acts(t, h, seed=120 + seed).view(np.float16).copy()))
+        lgd.copy_(torch.from_numpy(synth.make_router_logits(t, n_exp, seed=130 + seed)))
+        torch.cuda.synchronize()
+        dec.graph_launch(g)
+        dec.sync()
+        assert torch.equal(out, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        dec.set_tuning("pdl", 0)
+        try:
+            assert torch.equal(out, dec.moe_ffn_dev_t(0, lgd, xd, t))
+        finally:
+            dec.set_tuning("pdl", 1)
+    dec.graph_destroy(g)
+
+
 # the first call of a scratch counts rows into memory that nothing has written before: on a stream of the caller's, and again after growth
 def test_first_calls_of_a_scratch_on_a_side_stream(dec):
     n_exp, k, f, h, group = 16, 4, 128, 192, 32
