@@ -51,6 +51,12 @@ constexpr int TSG_THREADS = ts_threads(false);  // grouped form (teams: 2 to 6 %
 constexpr int TS_XBOX = 64;                     // grouped form: rows of a token box
 constexpr int TS_STAGE_BYTES = 16 * 1024;       // grouped form: results on their way out
 constexpr int RED_TOK = 64;                     // tokens per round of the cluster's sum
+__host__ __device__ constexpr int ts_push_pitch(int tok) { return tok + 4; }   // floats of a row on their way to its owner: conflict-free 16-byte accesses
+// K splits whose sums are sent to their owners instead of being read there.  Sending costs a 16-byte piece per lane where reading has rows of 128 bytes, and room
+// beside the rings.  Sent against read, us at 16 / 32 / 48 / 64 tokens: 7168 x 5120 in clusters of 4 8.4 / 9.1 / 10.5 / 11.8 against 8.7 / 9.4 / 10.2 / 11.1;
+// 5120 x 17408 in clusters of 6 15.2 / 15.7 / 18.3 / 19.8 against 15.7 / 16.4 / 17.0 / 18.4; 2560 x 2560 in clusters of 7 4.8 / 5.5 / 6.8 / 8.0 against
+// 4.8 / 5.2 / 5.8 / 6.6; 4096 x 4096, 32-channel groups, in clusters of 4 5.9 / 6.6 / 7.2 / 7.9 against 6.3 / 7.1 / 7.4 / 7.9.
+constexpr bool ts_pushes(int tok, int ks) { return ks > 1 && tok <= 32 && tok * ks <= 192; }
 // Shared memory requested per CTA.  The lower bounds keep CTAs whose TMEM does not fit together off one SM: a CTA that
 // waits for TMEM columns would hold up its cluster, and the columns may belong to a CTA that waits for its own cluster.
 // Half the TMEM: two CTAs per SM, never three; all of it: alone, also beside a CTA of the other kind.
@@ -72,6 +78,7 @@ struct TsArgs {
     int tmem_cols;
     int off_x, off_bars; // byte offsets in dynamic shared memory (1024-byte aligned base)
     int off_stage;       // grouped: results of a tile on their way out
+    int off_push;        // where the other splits' sums come in (ts_pushes); 0: the splits read each other's rings
     int pdl;
     float out_mul;
     uint32_t fma_add, fma_mul;   // (20 - E) << 26 | (24 - E) << 10 and the pair (-8 * 2^-E, -8 * 2^-E) (Dec::fma_shift)
@@ -125,7 +132,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 
     // ---- this CTA's tile ----
     const int tile = (int)blockIdx.x, ks = a.ksplit, split = (int)blockIdx.y;
-    const int mtile = tile % a.m_tiles, ntile = tile / a.m_tiles;    // neighbours share the weights
+    const int ntile = a.m_tiles == 1 ? tile : tile / a.m_tiles, mtile = tile - ntile * a.m_tiles;    // neighbours share the weights
     const int n0 = ntile * TS_MROWS;
     const int m0 = mtile * N, rb0 = n0 / TILE_ROWS;
     const int rows_valid = min(N, a.m - m0);
@@ -133,8 +140,8 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     const uint32_t kb_bytes = (uint32_t)nrbv * (TILE_WORDS * 4);
     // K range of this split in stages; the last stage of the matrix may hold one k-block (32-channel groups)
     const int nkb_all = a.k / BK, st_all = (nkb_all + 1) / 2;
-    const int st0 = (int)((long long)st_all * split / ks);
-    const int nst = (int)((long long)st_all * (split + 1) / ks) - st0;
+    const int st0 = (int)((unsigned)(st_all * split) / (unsigned)ks);
+    const int nst = (int)((unsigned)(st_all * (split + 1)) / (unsigned)ks) - st0;
     auto stage_kbs = [&](int it) { return min(2, nkb_all - 2 * (st0 + it)); };
     auto issue_raw = [&](int it, int s) {
         const int kbs = stage_kbs(it);
@@ -147,26 +154,29 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
     };
 
-    if (threadIdx.x == 0) {
-        s_abort = 0;
-        for (int s = 0; s < NR; ++s) {
-            mbar_init(raw_full(s), 1);
-            mbar_init(raw_free(s), ARRIVE);
+    if (warp == 2 + EXP_WARPS) {
+        // The warp that streams the weights makes the barriers, a lane each, and requests its first stages.  By one thread that also did the rest, one after the
+        // other, the first weights were requested 2.3 us after the start (code that runs once is fetched as it runs); 7168 x 5120, 27 tokens, before and now:
+        // 9.9 and 9.4 us, with the sums sent 9.1.
+        if (lane == 0) {
+            s_abort = 0;
         }
-        for (int s = 0; s < NX; ++s) {
-            mbar_init(x_full(s), 1);
-            mbar_init(x_free(s), 1);
+        for (int i = lane; i < 2 * (NR + NX + NA) + 1; i += 32) {
+            const bool all = (i >= NR && i < 2 * NR) || (i >= 2 * (NR + NX) && i < 2 * (NR + NX) + NA);     // raw_free, a_ready
+            mbar_init(bars + 8u * i, all ? ARRIVE : 1);
         }
-        for (int s = 0; s < NA; ++s) {
-            mbar_init(a_ready(s), ARRIVE);
-            mbar_init(a_free(s), 1);
-        }
-        mbar_init(accum_bar, 1);
         mbar_init_fence();
-        // the weights do not depend on the previous kernel of the stream
-        for (int it = 0; it < NR && it < nst; ++it) {
-            issue_raw(it, it);
+        __syncwarp();
+        if (elect_one()) {
+            // the weights do not depend on the previous kernel of the stream
+            for (int it = 0; it < NR && it < nst; ++it) {
+                issue_raw(it, it);
+            }
         }
+        __syncwarp();
+    }
+    if (ks > 1) {
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");      // waited for before the splits' sums: every CTA has started
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem_base)),
@@ -177,11 +187,6 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (a.pdl) {
-        // only now: a CTA of the next kernel that came earlier could take the TMEM this one still has to allocate, and
-        // then wait for this kernel
-        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    }
     const uint32_t tmem = __shfl_sync(0xffffffffu, s_tmem_base, 0);
     const uint32_t tmem_a = tmem + (uint32_t)N;                      // A ring: [stage][64 columns]
     volatile int* abort_flag = &s_abort;
@@ -191,6 +196,10 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // ------------------------------------------------------------------ tokens
         if (a.pdl) {
             asm volatile("griddepcontrol.wait;" ::: "memory");
+            // Only now.  CTAs of the next kernel that came before this one holds its TMEM could take it and then wait for this kernel; and those that come
+            // while the previous kernel still has its SMs pile up on the few that neither holds (68 row tiles in clusters of 2, 5120 channels, 48 tokens, in a
+            // row: 11.5 to 13.2 us a launch, and 10.4).
+            asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         }
         const bool leader = elect_one();
         int sx = 0, px = 1;
@@ -338,11 +347,11 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 } else {
                     ts_expand<FMA>(raw1, sc0, sc1, v);
                 }
+                tmem_st_16x256b_x4(td + BK / 2, v);
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(raw_free(sr));                           // both k-blocks are in registers
+                    mbar_arrive(raw_free(sr));                           // both k-blocks have been used (as in ts_expand_stage)
                 }
-                tmem_st_16x256b_x4(td + BK / 2, v);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -412,7 +421,54 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 }
             }
         }
+    } else if (a.off_push > 0) {
+        // Few tokens: a lane sends its row's sums to the CTA of the cluster that owns the row, into a place of their own beside the rings, and an
+        // owner adds up what it has got, in split order: one barrier, no remote reads to wait for, and nobody to wait for before
+        // leaving.
+        const uint32_t rp = (uint32_t)(TS_MROWS + ks - 1) / (unsigned)ks, pitch = (uint32_t)ts_push_pitch(N);   // rows of an owner, at most; floats of a row
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (dq_warp && ok) {
+            const uint32_t owner = (unsigned)(lrow * ks) / TS_MROWS, first = (owner * TS_MROWS + ks - 1) / (unsigned)ks;
+            uint32_t there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(base + (uint32_t)a.off_push + ((uint32_t)split * rp + lrow - first) * pitch * 4u), "r"(owner));
+            for (int c0 = sub * 16; c0 < rows_valid; c0 += EW * 16) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, v);
+#pragma unroll
+                for (int i = 0; i < 16; i += 4) {
+                    asm volatile("st.shared::cluster.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(there + (uint32_t)(c0 + i) * 4u), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
+                }
+            }
+        }
+        cluster_sync_all();
+        const int r0 = (split * TS_MROWS + ks - 1) / ks, rows = min(((split + 1) * TS_MROWS + ks - 1) / ks, a.n - n0) - r0;
+        for (int tok = warp * 4; tok < rows_valid; tok += ts_threads(TEAMS) / 8) {       // a warp takes four tokens, a lane a row
+            for (int r = lane; r < rows; r += 32) {
+                const uint32_t q = base + (uint32_t)a.off_push + ((uint32_t)r * pitch + tok) * 4u;
+                float4 sum = lds_f32x4(q);
+                for (int i = 1; i < ks; ++i) {
+                    const float4 v = lds_f32x4(q + (uint32_t)i * rp * pitch * 4u);
+                    sum.x += v.x;
+                    sum.y += v.y;
+                    sum.z += v.z;
+                    sum.w += v.w;
+                }
+                const float out[4] = {sum.x * a.out_mul, sum.y * a.out_mul, sum.z * a.out_mul, sum.w * a.out_mul};
+                const size_t o = (size_t)(m0 + tok) * a.n + n0 + r0 + r;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (tok + i < rows_valid) {
+                        if (a.out_f16) {
+                            reinterpret_cast<__half*>(a.out)[o + (size_t)i * a.n] = __float2half_rn(out[i]);
+                        } else {
+                            reinterpret_cast<float*>(a.out)[o + (size_t)i * a.n] = out[i];
+                        }
+                    }
+                }
+            }
+        }
     } else {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         // the splits' accumulators meet in distributed shared memory, RED_TOK tokens at a time: [token][row] f32 over the
         // (idle) rings; every CTA of the cluster adds an equal share of the elements over all splits, in split order
         constexpr int ROWS = TS_MROWS;
@@ -431,7 +487,7 @@ gemm_ts_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             cluster_sync_all();
             const int nr4 = min(ROWS, a.n - n0) / 4;
             const int total = nt * nr4;
-            const int e0 = (int)((long long)total * split / ks), e1 = (int)((long long)total * (split + 1) / ks);
+            const int e0 = (int)((unsigned)(total * split) / (unsigned)ks), e1 = (int)((unsigned)(total * (split + 1)) / (unsigned)ks);
             for (int e = e0 + (int)threadIdx.x; e < e1; e += ts_threads(TEAMS)) {
                 const int tok = e / nr4, r = (e - tok * nr4) * 4;
                 float4 pv[8];
@@ -721,11 +777,11 @@ gemm_ts_grouped_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
                 const uint32_t td = t_st + (uint32_t)(sa * A_COLS);
                 tmem_st_16x256b_x4(td, v);
                 ts_expand<false>(raw1, TsScale<false>(sc[GPS > 2 ? 2 : 0], 0, 0), TsScale<false>(sc[GPS > 2 ? 3 : 0], 0, 0), v);
+                tmem_st_16x256b_x4(td + BK / 2, v);
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(raw_free(sr));                       // both k-blocks are in registers
+                    mbar_arrive(raw_free(sr));                       // both k-blocks have been used (as in ts_expand_stage)
                 }
-                tmem_st_16x256b_x4(td + BK / 2, v);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
@@ -837,16 +893,17 @@ cudaError_t gemm_ts_init_device() {
 // Shared memory and ring depths of a launch with tiles of `tok` tokens.
 namespace {
 struct TsPlan {
-    int tmem_cols, na, nr, nx, off_x, off_bars;
+    int tmem_cols, na, nr, nx, off_x, off_bars, off_push;
     int teams;           // 0: a warp per row block
     size_t smem;
 };
-TsPlan ts_plan(int group, int tok, bool teams) {
+TsPlan ts_plan(int group, int tok, bool teams, int ks) {
     TsPlan p{};
     // TMEM: the accumulator and as many expanded stages as fit in half of it (two CTAs per SM), else in all of it
     p.tmem_cols = tok <= 128 ? 256 : 512;
     p.na = std::min((p.tmem_cols - tok) / A_COLS, 4);
-    const size_t limit = p.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX;
+    const size_t push = ts_pushes(tok, ks) ? (size_t)ks * ((TS_MROWS + ks - 1) / ks) * ts_push_pitch(tok) * 4 + 16 : 0;
+    const size_t limit = (p.tmem_cols == 256 ? TS_SMEM_HALF_MAX : TS_SMEM_FULL_MAX) - push;
     p.teams = !teams ? 0 : p.na % 3 == 0 ? 3 : 2;
     const int step = std::max(1, p.teams);                       // the rings divide by the teams
     p.nx = p.nr = ts_smem(group, tok, 3, 3, p.na, &p.off_x, &p.off_bars) <= limit ? 3 : 2;
@@ -857,7 +914,9 @@ TsPlan ts_plan(int group, int tok, bool teams) {
             ++p.nx;
         }
     }
-    p.smem = std::max(ts_smem(group, tok, p.nr, p.nx, p.na, &p.off_x, &p.off_bars), p.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
+    const size_t used = ts_smem(group, tok, p.nr, p.nx, p.na, &p.off_x, &p.off_bars);
+    p.off_push = push > 0 ? (p.off_bars + (2 * (p.nr + p.nx + p.na) + 1) * 8 + 15) & ~15 : 0;
+    p.smem = std::max(used + push, p.tmem_cols == 256 ? TS_SMEM_HALF_MIN : TS_SMEM_FULL_MIN);
     return p;
 }
 }  // namespace
@@ -946,7 +1005,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     const long long ctas = (long long)((t + c.tok - 1) / c.tok) * ((l->n + TS_MROWS - 1) / TS_MROWS) * c.ks;
     const int nst = ((l->k + SK - 1) / SK + c.ks - 1) / c.ks;
     const bool teams = nst >= 4 && (c.tok <= 64 || (c.tok <= 96 && ctas > sm_count && nst >= 16));
-    const TsPlan p = ts_plan(l->group, c.tok, teams);
+    const TsPlan p = ts_plan(l->group, c.tok, teams, c.ks);
     TsArgs a{};
     a.tok = c.tok;
     a.ksplit = c.ks;
@@ -959,6 +1018,7 @@ int Dec::gemm_ts(const Lin* l, const void* x, void* dst, int t, int out_kind, co
     a.x_stages = p.nx;
     a.off_x = p.off_x;
     a.off_bars = p.off_bars;
+    a.off_push = p.off_push;
     CUtensorMap map;
     const cuuint64_t dims[3] = {(cuuint64_t)BK, (cuuint64_t)t, (cuuint64_t)(l->k / BK)};
     const cuuint64_t strides[2] = {(cuuint64_t)l->k * 2, (cuuint64_t)BK * 2};

@@ -138,13 +138,13 @@ __device__ __forceinline__ bool ts_expand_stage(uint32_t raw, int quad, int nrbv
         if (q == 0) {
             load(1);
         }
-        if (q == 2) {
-            __syncwarp();
-            if (lane == 0) {
-                raw_read();                                          // the stage is in registers
-            }
-        }
         tmem_st_16x256b_x4(td + ((uint32_t)(b * 16) << 16) + (uint32_t)(kb * (BK / 2)), v);
+    }
+    // The stage goes back when the last of what was read of it has been used: an arrival before that could pass loads under way, and the copy
+    // into the stage is not ordered behind them.
+    __syncwarp();
+    if (lane == 0) {
+        raw_read();
     }
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -295,6 +295,30 @@ def test_weight_row_gemm_pow2_exact(dec, t, k, n, group, tok, ks, out_f16):
     assert (guard[t:] == 7.0).all()
 
 
+# the sums of a cluster's splits on both sides of the line between sending and reading them (tokens of a tile x splits <= 192, at most 32 tokens): owners with
+# fewer rows than others, a last row tile of 16 and a ragged token tile; launches in a row, with rings that are filled again after a few stages
+@pytest.mark.parametrize("t,k,n,group,ks", [
+    (9, 256, 400, 128, 2), (16, 2048, 1040, 32, 8), (17, 640, 528, 128, 5), (32, 1536, 784, 32, 6), (31, 1792, 272, 128, 7), (48, 2048, 1536, 32, 4),
+    (48, 1024, 144, 128, 3)])
+def test_cluster_sums_pow2_exact(dec, t, k, n, group, ks):
+    q, s, x, expect = pow2_case(t, k, n, group)
+    dec.upload_lin_g("cs", q, s, n, k, group)
+    xd = x_dev(x)
+    outs = torch.full((12, t + 1, n), 7.0, device="cuda")
+    with forced(dec, "gemm_form", 2), forced(dec, "gemm_ts_ksplit", ks):
+        for o in outs:
+            dec.lin_forward("cs", xd, t, dst=o[:t])
+        name = dec.last_kernel()
+        half = dec.lin_forward("cs", xd, t, out_f16=True)
+    dec.sync()
+    dec.kernel_status()
+    dec.drop_lin("cs")
+    assert name.startswith("gemm_ts_kernel") and f"clusters of {ks}" in name, name
+    assert (outs[:, :t].cpu().numpy() == expect).all()           # sums of powers of two: exact in f32, one rounding to f16
+    assert (outs[:, t] == 7.0).all()
+    assert np.array_equal(half.cpu().numpy(), expect.astype(np.float16))
+
+
 @pytest.mark.parametrize("bn", [128, 160, 192, 224])
 @pytest.mark.parametrize("t,k,n,group,mt,ks", [(130, 256, 272, 128, 2, -1), (300, 768, 496, 32, 2, -1), (200, 512, 448, 64, 1, -1),
                                                (300, 1024, 624, 128, 2, 3)])
