@@ -85,7 +85,10 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const int xstride = a.k * 2 + RG_XPAD;
-    float* red = reinterpret_cast<float*>(smem + p.off_red);  // [KW][rows of a unit][8 tokens]
+    // The K warps' sums, [KW][8 tokens][ROWS], the eights of rows of a token in an order of its own (row ^ 8 (token / 2)): the 32 values of a store, 8 rows
+    // of 4 tokens, and those of a read, neighbouring rows of one, lie in 32 banks.  As [row][token] reads were 8-way conflicts.
+    constexpr int ROWS = UR * TILE_ROWS;
+    float* red = reinterpret_cast<float*>(smem + p.off_red);
     uint32_t xphase = 0;
     int seg = -1, row0 = 0, m = 0;
     uint32_t xl = 0;
@@ -126,40 +129,52 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
             __syncthreads();
         }
         const float m0 = 16777216.f * a.seg[0].out_mul, m1 = 1048576.f * a.seg[0].out_mul;
+        {
+            float* d0 = red + (kw * GEMV_MAX_M + 2 * t) * ROWS;      // (rows of this lane's two tokens: the same turn)
+            const int turn = t << 3;
 #pragma unroll
-        for (int r = 0; r < GM_NR; ++r) {
-            float* d = red + ((size_t)kw * (UR * TILE_ROWS) + (rw * GM_NR + r) * TILE_ROWS + g) * GEMV_MAX_M + 2 * t;
-            *reinterpret_cast<float2*>(d) = make_float2(tot[r][0] * m0, tot[r][1] * m0);
-            *reinterpret_cast<float2*>(d + 8 * GEMV_MAX_M) = make_float2(tot[r][2] * m1, tot[r][3] * m1);
+            for (int r = 0; r < GM_NR; ++r) {
+                const int lo = ((rw * GM_NR + r) * TILE_ROWS + g) ^ turn, hi = ((rw * GM_NR + r) * TILE_ROWS + g + 8) ^ turn;
+                d0[lo] = tot[r][0] * m0;
+                d0[lo + ROWS] = tot[r][1] * m0;
+                d0[hi] = tot[r][2] * m1;
+                d0[hi + ROWS] = tot[r][3] * m1;
+            }
         }
         __syncthreads();
-        auto sum_of = [&](int row, int tok) {
-            float v = red[row * GEMV_MAX_M + tok];
+        // sums of two neighbouring rows of a token
+        auto sums_of = [&](int row, int tok) {
+            const float* p0 = red + tok * ROWS + (row ^ (tok >> 1 << 3));
+            float2 v = *reinterpret_cast<const float2*>(p0);
 #pragma unroll
-            for (int w = 1; w < KW; ++w) {
-                v += red[(w * (UR * TILE_ROWS) + row) * GEMV_MAX_M + tok];      // fixed order: the same bits every run
+            for (int w = 1; w < KW; ++w) {                           // fixed order: the same bits every run
+                const float2 e = *reinterpret_cast<const float2*>(p0 + w * (GEMV_MAX_M * ROWS));
+                v.x += e.x;
+                v.y += e.y;
             }
             return v;
         };
         if (a.glu) {
             // interleaved gate / up row blocks: output o of the unit has its gate sum in row 32 (o / 16) + o % 16, its up sum 16
             // rows further
-            const int nout = rows / 2, nh = a.seg[0].n / 2;
-            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * nh + (size_t)rb0 * (TILE_ROWS / 2);
-            for (int e = threadIdx.x; e < nout * m; e += RG_THREADS) {
-                const int tok = e / nout, o = e - tok * nout;
-                const int lg = (o / TILE_ROWS) * 2 * TILE_ROWS + (o % TILE_ROWS);
-                ob[(size_t)tok * nh + o] = silu_mul_f16(sum_of(lg, tok), sum_of(lg + TILE_ROWS, tok));
+            constexpr int PAIRS = ROWS / 4;
+            const int o = (int)threadIdx.x % PAIRS * 2, lg = (o / TILE_ROWS) * 2 * TILE_ROWS + (o % TILE_ROWS), nh = a.seg[0].n / 2;
+            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * nh + (size_t)rb0 * (TILE_ROWS / 2) + o;
+            for (int tok = (int)threadIdx.x / PAIRS; tok < m && 2 * o < rows; tok += RG_THREADS / PAIRS) {
+                const float2 gate = sums_of(lg, tok), up = sums_of(lg + TILE_ROWS, tok);
+                *reinterpret_cast<__half2*>(ob + (size_t)tok * nh) = __halves2half2(silu_mul_f16(gate.x, up.x), silu_mul_f16(gate.y, up.y));
             }
         } else {
-            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * a.seg[0].n + (size_t)rb0 * TILE_ROWS;
-            for (int e = threadIdx.x; e < rows * m; e += RG_THREADS) {
-                const int tok = e / rows, row = e - tok * rows;
-                float v = sum_of(row, tok);
+            constexpr int PAIRS = ROWS / 2;
+            const int row = (int)threadIdx.x % PAIRS * 2;
+            __half* ob = reinterpret_cast<__half*>(a.seg[0].out) + (size_t)row0 * a.seg[0].n + (size_t)rb0 * TILE_ROWS + row;
+            for (int tok = (int)threadIdx.x / PAIRS; tok < m && row < rows; tok += RG_THREADS / PAIRS) {
+                float2 v = sums_of(row, tok);
                 if (a.row_w != nullptr) {
-                    v = mul_row_w(v, a.row_w[row0 + tok]);
+                    const float w = a.row_w[row0 + tok];
+                    v = make_float2(mul_row_w(v.x, w), mul_row_w(v.y, w));
                 }
-                ob[(size_t)tok * a.seg[0].n + row] = __float2half_rn(v);
+                *reinterpret_cast<__half2*>(ob + (size_t)tok * a.seg[0].n) = __floats2half2_rn(v.x, v.y);
             }
         }
     }
