@@ -23,7 +23,8 @@
 // expanding warps, about 600 cycles a stage, so up to 64 tokens (96 where CTAs queue) teams of four take stages in turn, and three chains
 // overlap: 27 tokens of 34816 x 5120 27.2 -> 25.6 us, of 5120 x 17408 18.7 -> 18.4, in groups of 32 31.0 -> 28.9.  Above that the MMAs
 // of a stage take as long as its chain, with fewer than four stages per CTA a team is idle: eight warps on every stage.
-// 256 rows per CTA were slower (33.5 us).
+// 256 rows per CTA were slower (33.5 us).  With teams a stage takes 550 cycles, the stages of two CTAs on an SM 430 each, 230 of them the MMAs: each of its 32 KB is
+// written to TMEM and read from it once, and the two do not overlap (34816 x 5120, 27 tokens: 22.8 us; with stages handed over in halves 39).
 //
 // The K splits of a tile form a thread-block cluster and sum their f32 accumulators through distributed shared memory in
 // split order (no global scratch, no tickets).

@@ -86,7 +86,8 @@ __global__ void __launch_bounds__(RG_THREADS, 2) gemv_moe_kernel(const GemvArgs 
 
     const int xstride = a.k * 2 + RG_XPAD;
     // The K warps' sums, [KW][8 tokens][ROWS], the eights of rows of a token in an order of its own (row ^ 8 (token / 2)): the 32 values of a store, 8 rows
-    // of 4 tokens, and those of a read, neighbouring rows of one, lie in 32 banks.  As [row][token] reads were 8-way conflicts.
+    // of 4 tokens, and those of a read, neighbouring rows of one, lie in 32 banks.  As [row][token], one value a thread, reads were 8-way conflicts: 128 experts,
+    // top-8, 2048 x 768, us per layer: 64 tokens 86.2 -> 81.1, 100 tokens 95.3 -> 89.1, 16 tokens 59.9 -> 59.3.
     constexpr int ROWS = UR * TILE_ROWS;
     float* red = reinterpret_cast<float*>(smem + p.off_red);
     uint32_t xphase = 0;

@@ -6,7 +6,7 @@
 // Same arithmetic and the same roundings to f16 as the launches for more of them (moe.cu, gemv_moe.cu); activations are multiplied as digits (gemv_rg.cuh).
 //
 // Bound by what surrounds the stream: a token of 128 experts x 768 x 2048 reads 19 MB, 3 us, and took 17.9 us in four launches that wait for one another;
-// 12.4 here.  (Of these the routing takes 2.8, most of it fetching code that runs once; ranking the experts by all threads instead was slower, 13.0.)
+// 11.9 here.  (Of these the routing takes 2.8, most of it fetching code that runs once; ranking the experts by all threads instead was 0.6 slower.)
 //   * every CTA routes the tokens for itself, a warp per token, while its other warps stage the activations: no routing launch, no tables;
 //   * the second matmul routes once more, while the first one still runs, and has its first weights on the way when that is complete: its CTAs fit on
 //     the SMs beside those of the first (half the registers, less than half the shared memory each);

@@ -17,9 +17,8 @@
 //   * one token, and some calls of two, are multiplied as signed digits by integer MMAs (gemv_rg.cuh): with the weights in L2 a launch took as long as
 //     from memory, because a tile cost an SM's scheduler 84 cycles, 40 of MMAs and 48 of masks and shifts among them; as digits it is 53, and
 //     5120 x 17408 streams 7 TB/s once its activations are staged.  Sixteen warps in a CTA were not faster (5120 x 17408 10.8 us, 896 x 5120 4.0).
-// One token, us per launch, this form against the best of the others: 7168 x 5120 5.3 / 7.2, 5120 x 6144 5.0 / 7.5, 34816 x 5120
-// 17.0 / 21.6 (5.4 TB/s), 5120 x 17408 10.2 / 13.8, 24576 x 4096 11.2 / 15.9; eight tokens: 6.8 / 10.3, 6.2 / 10.2, 20.0 / 26.2;
-// 34816 x 5120 in groups of 32, eight tokens: 21.4 / 48.9.
+// One token, us per launch, this form against the best of the others: 7168 x 5120 5.1 / 7.2, 5120 x 6144 4.8 / 7.5, 34816 x 5120
+// 17.1 / 21.6 (5.4 TB/s), 5120 x 17408 10.0 / 13.8; eight tokens: 6.4 / 10.3, 5.9 / 10.2, 18.9 / 26.2.
 #include <cuda_fp16.h>
 
 #include <algorithm>
