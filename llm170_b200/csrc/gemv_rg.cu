@@ -58,46 +58,38 @@ constexpr double RG_STEP_US[2][2][3] = {{{0.245, 0.32, 0.395}, {0.25, 0.352, 0.4
 // 7.6: 3, 8, two (alone 8.5); 24576 x 4096 12.0: 3, 4, two (4, 8, alone 12.9); 34816 x 5120 17.3: 4, 4, two (4, 8, two 17.7).
 // `digits`: one or two tokens as digits, which take more room.  false: x does not fit in shared memory beside two slots per warp.
 bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, bool digits, RgPlan& best) {
-    const int unit_k = a.group > TILE_K ? a.group : TILE_K, ku = a.k / unit_k, mp = (a.m + 1) & ~1;
+    const int unit_k = a.group > TILE_K ? a.group : TILE_K, ku = a.k / unit_k, mp = (a.m + 1) & ~1, stride = rg_digit_stride(a.k);
+    // a call plans on the host, twice where it may take digits: the ways are compared first and the plan is filled in for the best one (0.10 -> 0.05 us each)
     double cost = -1.0;
+    int best_per_sm = 0, best_x = 0;
     for (int kw : {4, 8}) {
+        const int chain = (ku + kw - 1) / kw * (unit_k / TILE_K);
+        const int x_bytes = ((digits ? 3 * a.m * stride + a.m * a.k * 2 * (RG_WARPS / kw) : a.m * (a.k * 2 + RG_XPAD)) + 127) & ~127;
         for (int nr : {4, 3, 2}) {
             if ((force_nr > 0 && nr != force_nr) || (force_kw > 0 && kw != force_kw)) {
                 continue;
             }
-            const int ur = RG_WARPS / kw * nr, slot = rg_slot_bytes(a.group, nr);
-            RgPlan p{};
-            p.nr = nr;
-            p.kw = kw;
-            p.split = 1;
-            p.digits = digits;
+            const int ur = RG_WARPS / kw * nr, padding = kw * mp * RG_RED_PAD * 4;
+            const int ring = (x_bytes + rg_red_bytes(kw, ur, mp) - padding + 127) & ~127, least = ring + 2 * RG_WARPS * rg_slot_bytes(a.group, nr);
+            int units = 0;
             for (int i = 0; i < a.nseg; ++i) {
-                p.units += (a.seg[i].n / TILE_ROWS + ur - 1) / ur;
+                units += (int)((unsigned)(a.seg[i].n / TILE_ROWS + ur - 1) / (unsigned)ur);
             }
-            p.off_raw = 3 * a.m * rg_digit_stride(a.k);
-            const int x_bytes = ((digits ? p.off_raw + a.m * a.k * 2 * (RG_WARPS / kw) : a.m * (a.k * 2 + RG_XPAD)) + 127) & ~127;
-            p.off_red = x_bytes;
-            const int padding = kw * mp * RG_RED_PAD * 4;
-            p.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) - padding + 127) & ~127;
-            const double tiles = (double)((ku + kw - 1) / kw * (unit_k / TILE_K) * nr) * (nr == 2 ? 1.3 : nr == 3 ? 1.05 : 1.0);
+            const double tiles = (double)(chain * nr) * (nr == 2 ? 1.3 : nr == 3 ? 1.05 : 1.0);
             for (int per_sm = 1; per_sm <= 2; ++per_sm) {
-                const int room = per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX;
-                const int least = p.off_ring + 2 * RG_WARPS * slot;
-                if (least > room || (per_sm == 2 && (p.units <= sm_count || least + padding > RG_SMEM_TWO_HW))) {
+                if (least > (per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX) || (per_sm == 2 && (units <= sm_count || least + padding > RG_SMEM_TWO_HW))) {
                     continue;
                 }
-                p.ctas = std::min(p.units, per_sm * sm_count);
-                const int rounds = (p.units + p.ctas - 1) / p.ctas;
+                const int ctas = per_sm * sm_count, rounds = units <= ctas ? 1 : (units + ctas - 1) / ctas;
                 const double c = rounds * (per_sm == 1 ? 1.5 * tiles + 20.0 : 2.0 * (tiles + 20.0));
                 if (cost < 0.0 || c < cost) {
                     cost = c;
-                    best = p;
-                    // alone: as deep a ring as fits; two: two slots (four measured the same)
-                    best.depth = per_sm == 2 ? 2 : p.off_ring + 6 * RG_WARPS * slot <= room ? 6 : p.off_ring + 4 * RG_WARPS * slot <= room ? 4 : 2;
-                    best.off_ring = (x_bytes + rg_red_bytes(kw, ur, mp) + 127) & ~127;
-                    best.smem = best.off_ring + best.depth * RG_WARPS * slot;
-                    // no second CTA of this launch on the SM, or no third one
-                    best.smem = std::max(best.smem, per_sm == 1 ? RG_SMEM_TWO + 2048 : RG_SMEM_NOT_THREE);
+                    best_per_sm = per_sm;
+                    best_x = x_bytes;
+                    best.nr = nr;
+                    best.kw = kw;
+                    best.units = units;
+                    best.off_ring = ring;
                 }
             }
         }
@@ -105,6 +97,18 @@ bool rg_make_plan(GemvArgs& a, int sm_count, int force_nr, int force_kw, bool di
     if (cost < 0.0) {
         return false;
     }
+    const int slot = RG_WARPS * rg_slot_bytes(a.group, best.nr), room = best_per_sm == 2 ? RG_SMEM_TWO : RG_SMEM_MAX;
+    best.split = 1;
+    best.digits = digits;
+    best.off_part = 0;
+    best.off_raw = 3 * a.m * stride;
+    best.off_red = best_x;
+    best.ctas = std::min(best.units, best_per_sm * sm_count);
+    // alone: as deep a ring as fits; two: two slots (four measured the same)
+    best.depth = best_per_sm == 2 ? 2 : best.off_ring + 6 * slot <= room ? 6 : best.off_ring + 4 * slot <= room ? 4 : 2;
+    best.off_ring = (best_x + rg_red_bytes(best.kw, RG_WARPS / best.kw * best.nr, mp) + 127) & ~127;
+    // no second CTA of this launch on the SM, or no third one
+    best.smem = std::max(best.off_ring + best.depth * slot, best_per_sm == 1 ? RG_SMEM_TWO + 2048 : RG_SMEM_NOT_THREE);
     best.per = best.units / best.ctas;
     best.more = best.units % best.ctas;
     int units = 0;
